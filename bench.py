@@ -615,7 +615,7 @@ def main():
             prev = n
         costs = layer_costs(pkg, rows_in, rows_out, pairs)
         pk = peaks()
-        is_conv = lambda n: n.startswith("conv_simt") or n.startswith("conv_umma")  # noqa: E731
+        is_conv = lambda n: n.startswith("conv_")  # noqa: E731
         top = max(per_kernel, key=lambda n: per_kernel[n][1])
         # every conv kernel instance is attributed the layers it ran (same order as the schedule)
         conv_launch_order = [n.strip("()") for n, _ in stages if is_conv(n)]

@@ -2,15 +2,17 @@
 //
 // Replaces the reference's per-offset gather / multiply / atomicAdd kernel, launched kvol times per
 // layer with one thread per rulebook pair and Cout global atomics per pair
-// (submConv3dlayer.cu:479-518, :632-638). Here one launch covers the layer: a thread owns CO_T
-// output channels of one output row, walks the row's kvol neighbour slots, and for each present
-// neighbour accumulates s = sum_ci in[ci]*W[k][ci][co] as one fused-multiply-add chain (ci ascending),
+// (submConv3dlayer.cu:479-518, :632-638). Here one launch covers the layer: a thread owns four
+// output channels of one output row, walks the row's present neighbours, and for each of them
+// accumulates s = sum_ci in[ci]*W[k][ci][co] as one fused-multiply-add chain (ci ascending),
 // then acc += s with k ascending. That is the arithmetic of the reference kernel with the order of
 // the atomic additions fixed, so fp32 results are reproducible bit for bit. BatchNorm scale/shift and
 // ReLU (a separate TensorRT scale + activation layer in the reference, se-ssd-ai-trt.cpp:808-856)
 // run in the epilogue, and the last layer can scatter straight into the dense BEV map.
 //
-// This path serves the memory-bound small-channel layers (4->16, 16->16, 16->32) and every fp32 layer.
+// This path serves the memory-bound small-channel layers (4->16; in fp32 also 16->16 and 16->32) and, with a kernel
+// that takes its channel counts at run time, every pair of channel counts without a kernel of its own. The wide fp32
+// layers are in conv_f32.cu, the wide fp16 layers in conv_umma.cu.
 #include <string>
 
 #include "common.cuh"
@@ -64,25 +66,6 @@ struct RowLoader<__half, N> {
     }
 };
 
-template <typename T, int N>
-__device__ __forceinline__ void store_row(T* __restrict__ p, const float (&y)[N]) {
-    if constexpr (sizeof(T) == 4) {
-        float4* v = reinterpret_cast<float4*>(p);
-#pragma unroll
-        for (int i = 0; i < N / 4; ++i) v[i] = make_float4(y[4 * i], y[4 * i + 1], y[4 * i + 2], y[4 * i + 3]);
-    } else {
-        uint4* v = reinterpret_cast<uint4*>(p);
-#pragma unroll
-        for (int i = 0; i < N / 8; ++i) {
-            uint4 t;
-            __half2* h = reinterpret_cast<__half2*>(&t);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) h[j] = __floats2half2_rn(y[8 * i + 2 * j], y[8 * i + 2 * j + 1]);
-            v[i] = t;
-        }
-    }
-}
-
 template <typename T>
 __device__ __forceinline__ T from_float(float v);
 template <>
@@ -90,104 +73,138 @@ __device__ __forceinline__ float from_float<float>(float v) { return v; }
 template <>
 __device__ __forceinline__ __half from_float<__half>(float v) { return __float2half_rn(v); }
 
-constexpr int CO_T = 16;  // output channels per thread
+__device__ __forceinline__ float to_float(float v) { return v; }
+__device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
+
+__device__ __forceinline__ void store_quad(float* p, const float (&y)[4]) {
+    *reinterpret_cast<float4*>(p) = make_float4(y[0], y[1], y[2], y[3]);
+}
+__device__ __forceinline__ void store_quad(__half* p, const float (&y)[4]) {
+    uint2 t;
+    reinterpret_cast<__half2*>(&t)[0] = __floats2half2_rn(y[0], y[1]);
+    reinterpret_cast<__half2*>(&t)[1] = __floats2half2_rn(y[2], y[3]);
+    *reinterpret_cast<uint2*>(p) = t;
+}
+
+// Narrow layers. Little arithmetic per row (4 to 5 of 27 neighbours at full resolution) behind three dependent reads
+// (row count, map entry, input row), so the kernel lives on rows in flight: COUT / 4 threads share a row, a block takes
+// ROWS rows at a time, reads their map entries side by side (coalesced over rows, all in flight), and every thread
+// then walks its row's present neighbours in ascending k. The weights sit in shared memory as floats, 64 bytes of
+// padding per offset so that rows at different offsets meet in fewer banks. One thread per row with the weights read
+// through L1 (four 16-byte loads per channel and thread) took 45 us for the fp32 16->16 layer of a 20,000-point frame,
+// this takes 22 (timed with events around the launch).
+template <typename T, int CIN, int COUT>
+struct Narrow {
+    static constexpr int TPR = COUT / 4;                 // threads per output row
+    static constexpr int ROWS = kThreads / TPR;
+    static constexpr int KVOL_MAX = 27;                  // 3 x 3 x 3 is the largest kernel the geometry code accepts
+    static constexpr int W_STRIDE = CIN * COUT + 16;     // floats from one offset's weights to the next offset's
+    static constexpr int smem(int kvol) { return (kvol * W_STRIDE + KVOL_MAX * ROWS) * 4; }
+};
 
 template <typename T, int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads)
-conv_simt_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ nbr,
-                 const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
-                 const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
-                 T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
-    constexpr int TPR = COUT / CO_T;          // threads per output row
-    constexpr int ROWS = kThreads / TPR;      // rows per block iteration
-    constexpr int KVOL_MAX = 27;              // 3 x 3 x 3 is the largest kernel the geometry code accepts
-    constexpr bool COMPACT = CIN <= 16;
-    __shared__ int32_t s_idx[COMPACT ? KVOL_MAX : 1][kThreads];
+__global__ void __launch_bounds__(kThreads, 3)
+conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ nbr,
+                   const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
+                   const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
+                   T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
+    using N = Narrow<T, CIN, COUT>;
+    constexpr int TPR = N::TPR, ROWS = N::ROWS;
+    constexpr int LOADS = (N::KVOL_MAX * ROWS + kThreads - 1) / kThreads;   // map entries a thread reads
+    constexpr int NP = 2;                                                   // input rows in flight per thread
+    extern __shared__ __align__(16) float narrow_smem[];
+    float* s_w = narrow_smem;
+    int32_t* s_idx = reinterpret_cast<int32_t*>(narrow_smem + kvol * N::W_STRIDE);   // [KVOL_MAX][ROWS]
+    const int tid = threadIdx.x, r = tid / TPR, cq = tid % TPR;
     const int chunks = (max_voxels + ROWS - 1) / ROWS;
     const int items = batch * chunks;
-    const int cg = threadIdx.x % TPR;
+    bool first = true;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
-        const int o = (it - b * chunks) * ROWS + threadIdx.x / TPR;
+        const int o0 = (it - b * chunks) * ROWS;
         int n = out_num[b];
         n = n > max_voxels ? max_voxels : n;
+        if (o0 >= n) continue;   // uniform over the block
+        // the rows' map entries: entry e = (offset e / ROWS, row e % ROWS)
+        const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b, 0, o0);   // ROWS rows of one 128-row tile
+        int entry[LOADS];
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) {
+            const int e = tid + j * kThreads, k = e / ROWS, row = e % ROWS;
+            entry[j] = k < kvol && o0 + row < n ? __ldg(nb + k * kNbrRun + row) : -1;
+        }
+        if (first) {
+            for (int e = tid; e < kvol * CIN * COUT; e += kThreads) {
+                const int k = e / (CIN * COUT);
+                s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(weights[e]);
+            }
+            first = false;
+        } else {
+            __syncthreads();     // the previous rows' entries have been used
+        }
+#pragma unroll
+        for (int j = 0; j < LOADS; ++j) {
+            const int e = tid + j * kThreads;
+            if (e < N::KVOL_MAX * ROWS) s_idx[e] = entry[j];
+        }
+        __syncthreads();
+        const int o = o0 + r;
+        // the row's present offsets, its threads looking at every TPR-th slot
+        uint32_t present = 0;
+#pragma unroll
+        for (int k0 = 0; k0 < N::KVOL_MAX; k0 += TPR) {
+            const int k = k0 + cq;
+            if (k < N::KVOL_MAX && s_idx[k * ROWS + r] >= 0) present |= 1u << k;
+        }
+#pragma unroll
+        for (int d = 1; d < TPR; d <<= 1) present |= __shfl_xor_sync(0xFFFFFFFFu, present, d);
         if (o >= n) continue;
-        float acc[CO_T];
-#pragma unroll
-        for (int c = 0; c < CO_T; ++c) acc[c] = 0.f;
-        const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b, 0, o);
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
         const T* in_b = in + (size_t)b * max_voxels * CIN;
-        // one neighbour: s = sum_ci x[ci] * W[k][ci][:] as a fused chain, then acc += s
-        auto add_neighbour = [&](int k, const float (&x)[CIN]) {
-            float s[CO_T];
+        while (present) {
+            int ks[NP];
+            float x[NP][CIN];
 #pragma unroll
-            for (int c = 0; c < CO_T; ++c) s[c] = 0.f;
-            const T* wk = weights + (size_t)k * CIN * COUT + cg * CO_T;
-#pragma unroll
-            for (int ci = 0; ci < CIN; ++ci) {
-                float w[CO_T];
-                RowLoader<T, CO_T>::load(wk + ci * COUT, w);
-#pragma unroll
-                for (int c = 0; c < CO_T; ++c) s[c] = fmaf(x[ci], w[c], s[c]);
+            for (int u = 0; u < NP; ++u) {
+                ks[u] = present ? __ffs((int)present) - 1 : -1;
+                present &= present - 1u;          // no-op when nothing is left
+                if (ks[u] >= 0) RowLoader<T, CIN>::load(in_b + (size_t)s_idx[ks[u] * ROWS + r] * CIN, x[u]);
             }
 #pragma unroll
-            for (int c = 0; c < CO_T; ++c) acc[c] = __fadd_rn(acc[c], s[c]);
-        };
-        if constexpr (COMPACT) {
-            // Narrow rows (the full-resolution layers, where a row has 5 of its 27 neighbours on average): all
-            // slots are read first, then every thread walks its own present neighbours in ascending k (two
-            // row loads in flight for the 4-channel input). A warp then runs as many steps as its fullest row has
-            // neighbour pairs, instead of one step for every offset any of its 32 rows has. Same order of additions as below.
-            uint32_t present = 0;
+            for (int u = 0; u < NP; ++u) {
+                if (ks[u] < 0) continue;
+                // one neighbour: sum_ci x[ci] * W[k][ci][:] as a fused chain, then added to the row's sum
+                float s[4] = {0.f, 0.f, 0.f, 0.f};
+                const float* wk = s_w + ks[u] * N::W_STRIDE + cq * 4;
 #pragma unroll
-            for (int k = 0; k < KVOL_MAX; ++k) {
-                const int idx = k < kvol ? __ldg(nb + k * kNbrRun) : -1;
-                s_idx[k][threadIdx.x] = idx;          // read back by this thread only
-                present |= (idx >= 0 ? 1u : 0u) << k;
-            }
-            constexpr int NP = CIN <= 4 ? 2 : 1;      // row loads in flight per thread (four measured no faster than two)
-            while (present) {
-                int ks[NP];
-                float x[NP][CIN];
-#pragma unroll
-                for (int u = 0; u < NP; ++u) {
-                    ks[u] = present ? __ffs((int)present) - 1 : -1;
-                    present &= present - 1u;          // no-op when nothing is left
-                    if (ks[u] >= 0) RowLoader<T, CIN>::load(in_b + (size_t)s_idx[ks[u]][threadIdx.x] * CIN, x[u]);
+                for (int ci = 0; ci < CIN; ++ci) {
+                    const float4 w = *reinterpret_cast<const float4*>(wk + ci * COUT);
+                    s[0] = fmaf(x[u][ci], w.x, s[0]);
+                    s[1] = fmaf(x[u][ci], w.y, s[1]);
+                    s[2] = fmaf(x[u][ci], w.z, s[2]);
+                    s[3] = fmaf(x[u][ci], w.w, s[3]);
                 }
 #pragma unroll
-                for (int u = 0; u < NP; ++u)
-                    if (ks[u] >= 0) add_neighbour(ks[u], x[u]);
-            }
-        } else {
-            for (int k = 0; k < kvol; ++k) {
-                const int idx = __ldg(nb + k * kNbrRun);
-                if (idx < 0) continue;
-                float x[CIN];
-                RowLoader<T, CIN>::load(in_b + (size_t)idx * CIN, x);
-                add_neighbour(k, x);
+                for (int c = 0; c < 4; ++c) acc[c] = __fadd_rn(acc[c], s[c]);
             }
         }
 #pragma unroll
-        for (int c = 0; c < CO_T; ++c) {
+        for (int c = 0; c < 4; ++c) {
             float v = acc[c];
-            if (scale) v = fmaf(v, __ldg(scale + cg * CO_T + c), shift ? __ldg(shift + cg * CO_T + c) : 0.f);
+            if (scale) v = fmaf(v, __ldg(scale + cq * 4 + c), shift ? __ldg(shift + cq * 4 + c) : 0.f);
             if (relu) v = v > 0.f ? v : 0.f;
             acc[c] = v;
         }
-        store_row<T, CO_T>(out + ((size_t)b * max_voxels + o) * COUT + cg * CO_T, acc);
+        store_quad(out + ((size_t)b * max_voxels + o) * COUT + cq * 4, acc);
         if (dense) {
             // Fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x).
             const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + o]);
             T* d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
 #pragma unroll
-            for (int c = 0; c < CO_T; ++c) d[(size_t)(cg * CO_T + c) * D * H * W] = from_float<T>(acc[c]);
+            for (int c = 0; c < 4; ++c) d[(size_t)(cq * 4 + c) * D * H * W] = from_float<T>(acc[c]);
         }
     }
 }
-
-__device__ __forceinline__ float to_float(float v) { return v; }
-__device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 
 // Any channel counts (the reference's kernel takes in_channel and out_channel as run-time values,
 // submConv3dlayer.cu:479-518): one warp per output row, lane = output channel (in rounds of 32), the same order of
@@ -247,27 +264,36 @@ int launch_generic(const ConvLaunch& c, cudaStream_t stream) {
 }
 
 template <typename T, int CIN, int COUT>
-int launch_one(const ConvLaunch& c, cudaStream_t stream) {
-    static const std::string name = std::string("conv_simt<") + (sizeof(T) == 4 ? "f32," : "f16,") +
+int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
+    using N = Narrow<T, CIN, COUT>;
+    static const std::string name = std::string("conv_narrow<") + (sizeof(T) == 4 ? "f32," : "f16,") +
                                     std::to_string(CIN) + "," + std::to_string(COUT) + ">";
-    SESSD_LAUNCH_NAMED(name.c_str(), (conv_simt_kernel<T, CIN, COUT>), persistent_grid(4), kThreads, 0, stream,
-                 static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.out_num,
-                 static_cast<const T*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
-                 static_cast<T*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W);
+    if (N::smem(N::KVOL_MAX) > 48 * 1024) {
+        // the attribute belongs to the device's context: set it once per device (repeating it is harmless)
+        static std::atomic<uint64_t> configured{0};
+        int dev = 0;
+        SESSD_CUDA(cudaGetDevice(&dev));
+        const uint64_t bit = 1ull << (dev & 63);
+        if (!(configured.load(std::memory_order_acquire) & bit)) {
+            SESSD_CUDA(cudaFuncSetAttribute(conv_narrow_kernel<T, CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            N::smem(N::KVOL_MAX)));
+            configured.fetch_or(bit, std::memory_order_release);
+        }
+    }
+    SESSD_LAUNCH_NAMED(name.c_str(), (conv_narrow_kernel<T, CIN, COUT>), persistent_grid(4), kThreads, N::smem(c.kvol),
+                       stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.out_num,
+                       static_cast<const T*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
+                       static_cast<T*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W);
     return SESSD_OK;
 }
 
 template <typename T>
 int dispatch(const ConvLaunch& c, cudaStream_t stream) {
-#define SESSD_CASE(CI, CO) \
-    if (c.cin == CI && c.cout == CO) return launch_one<T, CI, CO>(c, stream);
-    SESSD_CASE(4, 16)
-    SESSD_CASE(16, 16)
-    SESSD_CASE(16, 32)
-    SESSD_CASE(32, 32)
-    SESSD_CASE(32, 64)
-    SESSD_CASE(64, 64)
-#undef SESSD_CASE
+    if (c.cin == 4 && c.cout == 16) return launch_narrow<T, 4, 16>(c, stream);
+    if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these
+        if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16>(c, stream);
+        if (c.cin == 16 && c.cout == 32) return launch_narrow<float, 16, 32>(c, stream);
+    }
     return launch_generic<T>(c, stream);   // any other pair of channel counts
 }
 

@@ -42,7 +42,7 @@
 #include <string>
 #include <vector>
 
-#include "common.cuh"
+#include "mbarrier.cuh"
 
 namespace sessd {
 
@@ -65,7 +65,6 @@ constexpr int KVOL_MAX = 27;
 // take, so that lanes reading different offsets of a stage (32- and 16-channel inputs) use different banks too.
 constexpr int TAP_WORDS = kNbrRun;
 static_assert(kNbrRun == TILE_M + 4, "the map's spacing between offsets is the index block's");
-constexpr long long WAIT_LIMIT_CYCLES = 200000000LL;   // about a tenth of a second; real waits are microseconds
 
 // Gather slots (= gather warps): as many as fit beside the weight ring, the index blocks and the epilogue's staging area.
 // The index ring is deeper than the A ring (index rows come from DRAM, several microseconds away under load):
@@ -76,66 +75,6 @@ struct Ring {
     static constexpr int NIDX = (CIN == 16 ? 2 : 3) * NSLOT;
     static constexpr int THREADS = (FIRST_GATHER_WARP + NSLOT) * 32;
 };
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-// Same, but the hardware may park the thread for up to `ns` nanoseconds while the phase is incomplete,
-// so a waiting warp does not take issue slots from the warps that feed the pipeline.
-__device__ __forceinline__ bool mbar_try_wait_parked(uint32_t bar, uint32_t parity, uint32_t ns) {
-    uint32_t ok;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(ns)
-        : "memory");
-    return ok != 0;
-}
-// Bounded wait: false when the phase did not complete within the clock limit or the CTA is aborting.
-// The polling loop is kept to a handful of instructions (abort flag and clock are looked at every 32
-// polls). RELAXED waits (roles with slack: weight and index prefetch) also sleep between polls. The MMA
-// issuers use the plain limit, every other role one and a half times that: when something upstream is
-// missing, the wait closest to the cause is the one that gets reported.
-template <bool RELAXED = false, bool ISSUER = false>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int where = 0) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const long long t0 = clock64();
-    const long long limit = ISSUER ? WAIT_LIMIT_CYCLES : WAIT_LIMIT_CYCLES + WAIT_LIMIT_CYCLES / 2;
-    for (;;) {
-#pragma unroll 1
-        for (int i = 0; i < 32; ++i) {
-            if (RELAXED) __nanosleep(200);
-            if (mbar_try_wait_parked(bar, parity, 1000u)) return true;
-        }
-        if (*abort_flag) return false;
-        if (clock64() - t0 > limit) {
-            if (*abort_flag == 0) abort_flag[1] = where;   // abort_where follows abort_flag in SharedCtl
-            *abort_flag = 1;
-            return false;
-        }
-    }
-}
 
 __device__ __forceinline__ void cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
@@ -159,12 +98,6 @@ __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-                 "l"(src), "r"(bytes), "r"(bar)
-                 : "memory");
-}
 
 // Shared-memory matrix descriptor, K-major, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024
 // bytes apart (stride byte offset), leading byte offset unused by swizzled K-major layouts (set to 1),
