@@ -1,5 +1,6 @@
 // C ABI of the library: parameter validation, workspace layout and launch sequencing.
-// No kernel lives here; see voxelize.cu, rulebook.cu, conv_simt.cu, conv_umma.cu, sparse2dense.cu.
+// No kernel lives here; see voxelize.cu, rulebook.cu, conv_simt.cu, conv_f32.cu, conv_umma.cu,
+// sparse2dense.cu.
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -133,6 +134,7 @@ size_t esize(int dtype) { return dtype == SESSD_F32 ? 4 : 2; }
 int choose_conv(const ConvLaunch& c_in, cudaStream_t stream) {
     const ConvLaunch& c = c_in;
     if (c.dtype == SESSD_F16 && conv_umma_supported(c.cin, c.cout) && c.umma_weights) return launch_conv_umma(c, stream);
+    if (c.dtype == SESSD_F32 && conv_f32_supported(c.cin, c.cout, c.kvol)) return launch_conv_f32(c, stream);
     return launch_conv_simt(c, stream);
 }
 

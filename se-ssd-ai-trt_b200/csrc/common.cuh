@@ -309,6 +309,10 @@ struct ConvLaunch {
 int launch_conv_simt(const ConvLaunch& c, cudaStream_t stream);
 bool conv_simt_supported(int cin, int cout);
 
+// conv_f32.cu (fp32 storage, a register tile per warp)
+bool conv_f32_supported(int cin, int cout, int kvol);
+int launch_conv_f32(const ConvLaunch& c, cudaStream_t stream);
+
 // conv_umma.cu (tcgen05 implicit GEMM, fp16 storage)
 bool conv_umma_supported(int cin, int cout);
 int conv_umma_pack_weights(const float* weights, int kvol, int cin, int cout, void** device_out);
