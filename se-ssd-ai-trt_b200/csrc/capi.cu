@@ -13,6 +13,7 @@ namespace sessd {
 
 std::atomic<uint64_t> g_launches{0};
 thread_local StageRecorder* g_recorder = nullptr;
+thread_local bool g_overlap_launches = true;
 static thread_local std::string t_last_error;
 
 void set_cuda_error(cudaError_t e, const char* what) {
@@ -973,10 +974,19 @@ void* sessd_pipeline_workspace(sessd_pipeline* pl, int s) {
     return pl->ws[s];
 }
 
+namespace {
+struct OverlapLaunches {   // for the scope of a pipeline run
+    bool before;
+    explicit OverlapLaunches(bool on) : before(g_overlap_launches) { g_overlap_launches = on; }
+    ~OverlapLaunches() { g_overlap_launches = before; }
+};
+}  // namespace
+
 static int pipeline_run(sessd_pipeline* pl, const void* points, const int32_t* sizes, int nframes, bool host,
                         int32_t* host_voxel_num, int32_t* host_status, float* elapsed_ms, void* host_dense = nullptr) {
     if (!pl || !points || !sizes) return SESSD_ERR_NULL;
     if (nframes < 1) return SESSD_ERR_PARAM;
+    const OverlapLaunches overlap_launches(pl->nstreams == 1);
     const sessd_backbone* bb = pl->bb;
     const size_t frame_bytes = (size_t)pl->max_points * 16;
     const int last_layer = (int)bb->layers.size() - 1;

@@ -321,6 +321,7 @@ __device__ __forceinline__ bool f32_short_strips(const F32Args& a) {
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(F32_THREADS, 1) conv_f32_kernel(const __grid_constant__ F32Args a) {
+    pdl_enter();
     extern __shared__ __align__(16) uint8_t f32_smem[];
     F32Shared<CIN, COUT>& s = *reinterpret_cast<F32Shared<CIN, COUT>*>(f32_smem);
     if (threadIdx.x == 0) {

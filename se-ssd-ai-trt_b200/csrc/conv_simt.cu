@@ -108,6 +108,7 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
                    const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                    const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
                    T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
+    pdl_enter();
     using N = Narrow<T, CIN, COUT>;
     constexpr int TPR = N::TPR, ROWS = N::ROWS;
     constexpr int LOADS = (N::KVOL_MAX * ROWS + kThreads - 1) / kThreads;   // map entries a thread reads
@@ -216,6 +217,7 @@ conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t
                     const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                     const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol, int cin, int cout,
                     T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
+    pdl_enter();
     constexpr int ROWS = kThreads / 32;
     const int lane = threadIdx.x & 31, wrow = threadIdx.x >> 5;
     const int chunks = (max_voxels + ROWS - 1) / ROWS;

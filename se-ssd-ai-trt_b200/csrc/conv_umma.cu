@@ -265,6 +265,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                  const uint8_t* __restrict__ wtiles, const __grid_constant__ EpiConst epi, int relu, int batch,
                  int max_voxels, int kvol, __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
                  int W, int32_t* status, int withhold_weights) {
+    pdl_enter();
     // withhold_weights (tests of the time-out path only): the weight streamer stays silent, so the MMA issuers'
     // bounded wait for the first weight block runs out and every CTA with work leaves through the abort path.
     constexpr int KG = 64 / CIN;            // kernel offsets sharing one 128-byte A row

@@ -147,6 +147,7 @@ __device__ __forceinline__ float rank_score(float s) { return s != s ? -INFINITY
 // Kernel 1: rank by (score descending, row ascending) by counting, then the geometry of every ranked box.
 __global__ void __launch_bounds__(kThreads)
 nms_rank_kernel(NmsArgs a) {
+    pdl_enter();
     for (int b = blockIdx.x; b < a.batch; b += gridDim.x) {
         const int n = frame_count(a, b);
         const float* bx = a.boxes + (size_t)b * a.max_box * 9;
@@ -185,6 +186,7 @@ nms_rank_kernel(NmsArgs a) {
 constexpr int kMaskWarps = 8;
 __global__ void __launch_bounds__(kMaskWarps * 32)
 nms_mask_kernel(NmsArgs a) {
+    pdl_enter();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int segs = a.words * 2;
     const int64_t per_frame = (int64_t)a.max_box * segs;
@@ -231,6 +233,7 @@ nms_mask_kernel(NmsArgs a) {
 constexpr int kReduceThreads = 256;
 __global__ void __launch_bounds__(kReduceThreads)
 nms_reduce_kernel(NmsArgs a, int smem_words) {
+    pdl_enter();
     extern __shared__ unsigned long long s_mask[];
     __shared__ unsigned long long s_keep[32];
     __shared__ int s_base[33];

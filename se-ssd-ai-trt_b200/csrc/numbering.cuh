@@ -33,6 +33,7 @@ __device__ __forceinline__ bool numbering_is_owner(const NumberingArgs& a, const
 //   __device__ void operator()(int b, int e, int slot, int id)  once per owner entry
 template <class Emit>
 __global__ void __launch_bounds__(kThreads) emit_owners_kernel(NumberingArgs a, Table t, Emit emit) {
+    pdl_enter();
     const int cpf = a.chunks_per_frame;
     const int items = a.batch * cpf;
     for (int g = blockIdx.x; g < items; g += gridDim.x) {

@@ -64,6 +64,7 @@ __device__ __forceinline__ float sigmoid(float x) { return 1.0f / (1.0f + expf(-
 
 __global__ void __launch_bounds__(kThreads)
 anchor_decode_kernel(const float* __restrict__ box_preds, float* __restrict__ out, AnchorGeom g, int batch) {
+    pdl_enter();
     const int64_t total = (int64_t)batch * g.anchors;
     for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < total; e += (int64_t)gridDim.x * kThreads) {
         const int i = (int)(e % g.anchors);
@@ -96,6 +97,7 @@ struct FilterArgs {
 // them with five memsets, filterBoxByScore.cu:353-371).
 __global__ void __launch_bounds__(kThreads)
 box_count_kernel(FilterArgs a) {
+    pdl_enter();
     const int items = a.batch * a.chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / a.chunks, chunk = it - b * a.chunks;
@@ -120,6 +122,7 @@ box_count_kernel(FilterArgs a) {
 template <bool DECODE>
 __global__ void __launch_bounds__(kThreads)
 box_emit_kernel(FilterArgs a, AnchorGeom g) {
+    pdl_enter();
     const int items = a.batch * a.chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / a.chunks, chunk = it - b * a.chunks;

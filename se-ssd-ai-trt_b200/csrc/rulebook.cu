@@ -31,6 +31,7 @@ namespace {
 __global__ void __launch_bounds__(kThreads)
 table_build_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ voxel_num, int batch, int max_voxels,
                    int Z, int Y, int X, Table t, int32_t* status) {
+    pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
@@ -61,6 +62,7 @@ table_build_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ v
 __global__ void __launch_bounds__(kThreads)
 nbr_build_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__ out_num, int batch, int max_voxels,
                  ConvGeom g, Table in_table, int32_t* __restrict__ nbr) {
+    pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * g.kvol * chunks;
     const int k12 = g.K[1] * g.K[2];
@@ -113,6 +115,7 @@ __device__ __forceinline__ void split_small(int e, int m, int* q, int* r) {   //
 __global__ void __launch_bounds__(kThreads)
 rulebook_export_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int frame, int kvol,
                        int max_voxels, int32_t* __restrict__ pairs, uint32_t* __restrict__ pair_num) {
+    pdl_enter();
     const int k = blockIdx.x;
     int n = out_num[frame];
     n = n > max_voxels ? max_voxels : n;
@@ -138,6 +141,7 @@ rulebook_export_kernel(const int32_t* __restrict__ nbr, const int32_t* __restric
 __global__ void __launch_bounds__(kThreads)
 count_pairs_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels,
                    int kvol, unsigned long long* total) {
+    pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * kvol * chunks;
     int local = 0;
@@ -162,6 +166,7 @@ count_pairs_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ 
 __global__ void __launch_bounds__(kThreads)
 bucket_build_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ voxel_num, int batch, int max_voxels,
                     int Z, int Y, int X, Buckets t, int32_t* status) {
+    pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
@@ -244,6 +249,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 nbr_build_subm_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ voxel_num, int batch,
                       int max_voxels, int Z, int Y, int X, Buckets t, int32_t* __restrict__ nbr,
                       uint32_t* __restrict__ tile_mask, int tiles_per_frame) {
+    pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
@@ -318,6 +324,7 @@ __device__ __forceinline__ unsigned long long rec_bits(const uint4& r) {
 __global__ void __launch_bounds__(kThreads)
 mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict__ in_num, int batch, int max_voxels,
                     ConvGeom g, BitGrid out) {
+    pdl_enter();
     constexpr int MAXS = 3;   // span_max never exceeds the kernel size (<= 3)
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * chunks;
@@ -387,6 +394,7 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
 // Set bits of every 1024-word chunk of every frame.
 __global__ void __launch_bounds__(kThreads)
 count_bits_kernel(BitGrid g, int batch, int32_t* __restrict__ chunk_counts) {
+    pdl_enter();
     const int items = batch * g.chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / g.chunks, c = it - b * g.chunks;
@@ -408,6 +416,7 @@ count_bits_kernel(BitGrid g, int batch, int32_t* __restrict__ chunk_counts) {
 __global__ void __launch_bounds__(kThreads)
 number_outputs_kernel(BitGrid g, int batch, int max_voxels, const int32_t* __restrict__ chunk_counts,
                       int4* __restrict__ out_coors, int32_t* __restrict__ out_num, int32_t* status) {
+    pdl_enter();
     const int items = batch * g.chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / g.chunks, c = it - b * g.chunks;
@@ -513,6 +522,7 @@ __global__ void __launch_bounds__(kThreads, 4)
 map_rows_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__ out_num, int batch, int max_voxels,
                 ConvGeom g, BitsIndex in, int32_t* __restrict__ nbr, uint32_t* __restrict__ tile_mask,
                 int tiles_per_frame) {
+    pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * chunks;
     const int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
@@ -567,6 +577,7 @@ map_rows_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__ 
 // kvol x kNbrRun words is contiguous and 16-byte aligned; the padding words are written too).
 __global__ void __launch_bounds__(kThreads)
 nbr_clear_kernel(int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels, int kvol) {
+    pdl_enter();
     const size_t frame_words = nbr_frame_words(kvol, max_voxels);
     const int chunks = (int)((frame_words / 4 + kThreads - 1) / kThreads);
     const int items = batch * chunks;
@@ -590,6 +601,7 @@ __global__ void __launch_bounds__(kThreads)
 scatter_rows_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict__ in_num, int batch, int max_voxels,
                     ConvGeom g, BitsIndex out, int32_t* __restrict__ nbr, uint32_t* __restrict__ tile_mask,
                     int tiles_per_frame) {
+    pdl_enter();
     const int64_t per_frame = (int64_t)max_voxels * g.ncand;
     const int chunks = (int)((per_frame + kThreads - 1) / kThreads);
     const int items = batch * chunks;
@@ -636,6 +648,7 @@ scatter_rows_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
 __global__ void __launch_bounds__(kThreads)
 tile_mask_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels,
                  int kvol, uint32_t* __restrict__ tile_mask, int tiles_per_frame) {
+    pdl_enter();
     const int warps_per_block = kThreads / 32;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int64_t items = (int64_t)batch * tiles_per_frame * kvol;

@@ -16,6 +16,7 @@ __global__ void __launch_bounds__(kThreads)
 sparse2dense_kernel(const T* __restrict__ feat, const int4* __restrict__ coors, const int32_t* __restrict__ voxel_num,
                     int batch, int max_voxels, int C, int D, int H, int W, int Hp, int Wp, int top, int left,
                     T* __restrict__ dense) {
+    pdl_enter();
     const int64_t per_frame = (int64_t)max_voxels * C;
     const int chunks = (int)((per_frame + kThreads - 1) / kThreads);
     const int items = batch * chunks;
@@ -39,6 +40,7 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads)
 zero_pad2d_kernel(const T* __restrict__ in, T* __restrict__ out, size_t planes, int H, int W, int Hp, int Wp, int top,
                   int left) {
+    pdl_enter();
     const size_t total = planes * H * W, stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < total; i += stride) {
         const size_t plane = i / ((size_t)H * W);

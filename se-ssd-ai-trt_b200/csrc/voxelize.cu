@@ -26,6 +26,7 @@ __global__ void __launch_bounds__(kThreads)
 voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch,
                     int max_points, VoxGeom g, Table t, int max_pts, int32_t* __restrict__ pt_slot,
                     int32_t* status) {
+    pdl_enter();
     const int chunks = (max_points + kThreads - 1) / kThreads;
     const int items = batch * chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
@@ -128,6 +129,7 @@ struct VoxelEmit {
 };
 
 __global__ void __launch_bounds__(kThreads) count_owners_kernel(NumberingArgs a, Table t) {
+    pdl_enter();
     const int cpf = a.chunks_per_frame;
     const int items = a.batch * cpf;
     for (int g = blockIdx.x; g < items; g += gridDim.x) {
@@ -150,6 +152,7 @@ template <typename V>
 __global__ void __launch_bounds__(kThreads)
 zero_tail_kernel(V* __restrict__ tensor, int row_units, const int32_t* __restrict__ voxel_num, int batch,
                  int max_voxels) {
+    pdl_enter();
     const int64_t per_frame = (int64_t)max_voxels * row_units;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
     V zero;
@@ -164,11 +167,13 @@ zero_tail_kernel(V* __restrict__ tensor, int row_units, const int32_t* __restric
 }
 
 __global__ void __launch_bounds__(kThreads) fill_zero_kernel(uint4* __restrict__ p, size_t n16) {
+    pdl_enter();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += stride) p[i] = make_uint4(0, 0, 0, 0);
 }
 
 __global__ void __launch_bounds__(kThreads) fill_ones_kernel(uint4* __restrict__ p, size_t n16) {
+    pdl_enter();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n16; i += stride)
         p[i] = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
@@ -177,6 +182,7 @@ __global__ void __launch_bounds__(kThreads) fill_ones_kernel(uint4* __restrict__
 // Up to four ranges filled by one launch (r = range, 16-byte words; value 0 or kEmpty in every word): the resets a
 // call of the fused front end needs (voxel table and bucket table to 0xFF, grids + masks and the BEV map to 0).
 __global__ void __launch_bounds__(kThreads) fill_ranges_kernel(FillRanges f) {
+    pdl_enter();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t first = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
 #pragma unroll
