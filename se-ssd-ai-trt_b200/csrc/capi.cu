@@ -53,8 +53,6 @@ int launch_count_pairs(const int32_t* nbr, const int32_t* out_num, int batch, in
 
 namespace {
 
-constexpr int kStatusInts = 256;  // status block: 1 KB; word 0 is the status, bytes 256.. hold 64 pair counters
-
 // np.round as the reference mimics it (voxelGenerator.cu:61-68).
 int np_round_f32(float x) {
     const int x2 = (int)(x * 2.0f);
@@ -84,12 +82,22 @@ struct ConvWorkspace {
     Buckets buckets;      // submanifold 3x3x3: x-grouped table of the input coordinates
     Table in_table;       // other submanifold geometries: flat table of the input coordinates
     BitGrid out_bits;     // strided: occupancy grid of the output level
-    void* zero_base;      // occupancy grid + tile masks: zero before use
+    void* zero_base;      // occupancy grid + tile masks + numbering state: zero before use
     size_t zero_bytes;
     uint32_t* tile_mask;  // [B][tiles]
-    int32_t* chunk_counts;
+    ScanState scan;       // strided: numbering of the outputs
     int32_t* nbr;
 };
+
+// Numbering state of one level: a word per chunk and frame and the ticket counter, a multiple of 16 bytes.
+size_t scan_state_bytes(const BitGrid& g, int batch) {
+    return ((size_t)batch * scan_chunks(g.words) + 2) / 2 * 2 * sizeof(unsigned long long);
+}
+ScanState scan_state_at(char* p, const BitGrid& g, int batch) {
+    if (!p) return ScanState{nullptr, nullptr};
+    return ScanState{reinterpret_cast<unsigned long long*>(p),
+                     reinterpret_cast<uint32_t*>(p + scan_state_bytes(g, batch) - sizeof(unsigned long long))};
+}
 
 void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeom& g, int batch, ConvWorkspace* w) {
     *w = ConvWorkspace{};
@@ -109,17 +117,18 @@ void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeo
         w->ones_bytes = per * 2 * sizeof(uint32_t);
     } else {
         w->out_bits = bitgrid_shape(g.out_shape);
-        w->chunk_counts = bump.take<int32_t>((size_t)batch * w->out_bits.chunks);
     }
-    // occupancy grid (strided layers) and tile masks in one block, reset to zero by a single fill
+    // occupancy grid and numbering state (strided layers) and tile masks in one block, reset by the call's first launch
     const size_t tiles = (size_t)(p->max_voxels + 127) / 128;
     const size_t mask_bytes = (batch * tiles * sizeof(uint32_t) + 15) / 16 * 16;
     const size_t grid_bytes = p->subm ? 0 : (size_t)batch * w->out_bits.words * sizeof(uint4);
-    char* zero = bump.take<char>(grid_bytes + mask_bytes);
+    const size_t scan_bytes = p->subm ? 0 : scan_state_bytes(w->out_bits, batch);
+    char* zero = bump.take<char>(grid_bytes + mask_bytes + scan_bytes);
     w->zero_base = zero;
-    w->zero_bytes = grid_bytes + mask_bytes;
+    w->zero_bytes = grid_bytes + mask_bytes + scan_bytes;
     w->out_bits.rec = reinterpret_cast<uint4*>(zero);
     w->tile_mask = reinterpret_cast<uint32_t*>(zero ? zero + grid_bytes : nullptr);
+    if (!p->subm) w->scan = scan_state_at(zero ? zero + grid_bytes + mask_bytes : nullptr, w->out_bits, batch);
     w->nbr = bump.take<int32_t>((size_t)batch * nbr_frame_words(g.kvol, p->max_voxels));
 }
 
@@ -164,8 +173,8 @@ struct sessd_backbone {
     int nlevels;
     std::vector<int> level_shape;  // 3 ints per level
     std::vector<char> level_has_subm;
+    std::vector<char> level_derived;   // the level's occupancy follows from its input level's grid
     int max_voxels;
-    int kvol_strided_max, ncand_max;
 };
 
 namespace {
@@ -184,8 +193,8 @@ struct BackboneWorkspace {
     std::vector<uint32_t*> mask_layer;    // per strided layer (indexed by layer)
     void* zero_base;
     size_t zero_bytes;
-    int32_t* nbr_strided;
-    int32_t* chunk_counts;
+    std::vector<int32_t*> nbr_layer;      // maps of the strided layers (indexed by layer)
+    std::vector<ScanState> scan;          // numbering state of the derived levels
     std::vector<void*> feat;
 };
 
@@ -212,38 +221,44 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
     w->buckets0 = Buckets{block, capb, 32 - ilog2(capb)};
     w->ones_base = block;
     w->ones_bytes = perb * sizeof(uint32_t);
-    // occupancy grids of the derived levels and all tile masks in one block, reset to zero by one fill
+    // What one fill zeroes per call: the occupancy grids that rows mark their outputs in, all tile masks, the numbering
+    // state of the levels and of the voxeliser. A grid that is derived from its input level's grid is written whole.
     const size_t tiles = (size_t)(maxV + 127) / 128;
     const size_t mask_words = (batch * tiles + 3) / 4 * 4;
     size_t nmasks = 0;
     for (int l = 0; l < bb->nlevels; ++l) nmasks += bb->level_has_subm[l] ? 1 : 0;
     for (auto& L : bb->layers) nmasks += L.p.subm ? 0 : 1;
-    size_t grid_recs = 0;
-    int chunks_max = 1;
+    size_t zero_bytes = mask_words * nmasks * sizeof(uint32_t);
+    w->scan.assign(bb->nlevels, ScanState{nullptr, nullptr});
     for (int l = 1; l < bb->nlevels; ++l) {
         w->bits[l] = bitgrid_shape(&bb->level_shape[3 * l]);
-        grid_recs += (size_t)batch * w->bits[l].words;
-        if (w->bits[l].chunks > chunks_max) chunks_max = w->bits[l].chunks;
+        zero_bytes += scan_state_bytes(w->bits[l], batch);
+        if (!bb->level_derived[l]) zero_bytes += (size_t)batch * w->bits[l].words * sizeof(uint4);
     }
-    char* zero = bump.take<char>(grid_recs * sizeof(uint4) + mask_words * nmasks * sizeof(uint32_t) + 16);
+    char* zero = bump.take<char>(zero_bytes + 16);
     w->zero_base = zero;
-    w->zero_bytes = grid_recs * sizeof(uint4) + mask_words * nmasks * sizeof(uint32_t);
+    w->zero_bytes = zero_bytes;
     size_t off = 0;
+    auto carve = [&](size_t bytes) {
+        char* p = zero ? zero + off : nullptr;
+        off += bytes;
+        return p;
+    };
     for (int l = 1; l < bb->nlevels; ++l) {
-        w->bits[l].rec = reinterpret_cast<uint4*>(zero ? zero + off : nullptr);
-        off += (size_t)batch * w->bits[l].words * sizeof(uint4);
+        const size_t bytes = (size_t)batch * w->bits[l].words * sizeof(uint4);
+        w->bits[l].rec = bb->level_derived[l] ? bump.take<uint4>(bytes / sizeof(uint4)) : reinterpret_cast<uint4*>(carve(bytes));
+        w->scan[l] = scan_state_at(carve(scan_state_bytes(w->bits[l], batch)), w->bits[l], batch);
     }
-    uint32_t* masks = reinterpret_cast<uint32_t*>(zero ? zero + off : nullptr);
-    size_t mi = 0;
     for (int l = 0; l < bb->nlevels; ++l)
-        if (bb->level_has_subm[l]) w->mask_subm[l] = masks ? masks + mask_words * mi++ : (mi++, nullptr);
+        if (bb->level_has_subm[l]) w->mask_subm[l] = reinterpret_cast<uint32_t*>(carve(mask_words * sizeof(uint32_t)));
     for (size_t i = 0; i < bb->layers.size(); ++i)
-        if (!bb->layers[i].p.subm) w->mask_layer[i] = masks ? masks + mask_words * mi++ : (mi++, nullptr);
+        if (!bb->layers[i].p.subm) w->mask_layer[i] = reinterpret_cast<uint32_t*>(carve(mask_words * sizeof(uint32_t)));
     for (int l = 0; l < bb->nlevels; ++l)
         if (bb->level_has_subm[l]) w->nbr_subm[l] = bump.take<int32_t>((size_t)batch * nbr_frame_words(27, maxV));
-    w->nbr_strided =
-        bump.take<int32_t>((size_t)batch * nbr_frame_words(bb->kvol_strided_max > 0 ? bb->kvol_strided_max : 1, maxV));
-    w->chunk_counts = bump.take<int32_t>((size_t)batch * chunks_max);
+    w->nbr_layer.assign(bb->layers.size(), nullptr);
+    for (size_t i = 0; i < bb->layers.size(); ++i)
+        if (!bb->layers[i].p.subm)
+            w->nbr_layer[i] = bump.take<int32_t>((size_t)batch * nbr_frame_words(bb->layers[i].g.kvol, maxV));
     w->feat.assign(bb->layers.size(), nullptr);
     for (size_t i = 0; i < bb->layers.size(); ++i)
         w->feat[i] = bump.take<char>((size_t)batch * maxV * bb->layers[i].p.out_channel * esize(bb->dtype));
@@ -347,10 +362,22 @@ int sessd_voxelize_enqueue(const sessd_voxel_params* p, int batch, int max_point
     if (bump.total() > workspace_bytes) return SESSD_ERR_WORKSPACE;
     if (!workspace_aligned(workspace)) return SESSD_ERR_PARAM;
     w.status = status;
-    SESSD_CUDA(cudaMemsetAsync(status, 0, kStatusInts * sizeof(int32_t), stream));
+    FillRanges fills{};
+    fills.ptr[0] = static_cast<uint4*>(w.table_base), fills.n16[0] = w.table_bytes / 16, fills.ones[0] = 1;
+    fills.ptr[1] = static_cast<uint4*>(w.zero_base), fills.n16[1] = w.zero_bytes / 16, fills.ones[1] = 0;
+    fills.status = status;
+    // rows that no point can reach; the rows between the voxel count and the point count are zeroed on the way
+    TailRows tails{};
+    tails.tensor[0] = outputs[0], tails.row_bytes[0] = 4 * (int)esize(out_dtype);
+    tails.tensor[1] = outputs[1], tails.row_bytes[1] = 16;
+    tails.tensor[2] = w.num_points, tails.row_bytes[2] = 4;
+    tails.counts = static_cast<const int32_t*>(inputs[1]);
+    tails.batch = batch, tails.max_rows = p->max_voxels;
+    int rc = launch_prepare(fills, tails, stream);
+    if (rc) return rc;
     return voxelize_run(p, batch, max_points, out_dtype, static_cast<const float*>(inputs[0]),
                         static_cast<const int32_t*>(inputs[1]), outputs[0], static_cast<int32_t*>(outputs[1]),
-                        static_cast<int32_t*>(outputs[2]), w, /*zero_tail=*/true, stream);
+                        static_cast<int32_t*>(outputs[2]), w, /*zero_tail=*/true, VoxelHooks{}, stream);
 }
 
 // ---- sparse convolutions --------------------------------------------------------------------
@@ -453,12 +480,18 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     const int maxV = p->max_voxels;
     const int32_t* in_coors = static_cast<const int32_t*>(inputs[1]);
     const int32_t* in_num = static_cast<const int32_t*>(inputs[2]);
-    SESSD_CUDA(cudaMemsetAsync(ws.status, 0, kStatusInts * sizeof(int32_t), stream));
-    if (ws.ones_bytes) {
-        rc = launch_fill_ones(ws.ones_base, ws.ones_bytes, stream);
-        if (rc) return rc;
-    }
-    rc = launch_fill_zero(ws.zero_base, ws.zero_bytes, stream);
+    // Rows past the active count are zero in the reference (outputs are memset, submConv3dlayer.cu:594): here by the
+    // first launch that knows the count.
+    TailRows tails{};
+    tails.tensor[0] = outputs[0], tails.row_bytes[0] = (int)(p->out_channel * esize(w->impl.dtype));
+    if (!subm) tails.tensor[1] = outputs[1], tails.row_bytes[1] = 16;
+    tails.counts = subm ? in_num : static_cast<const int32_t*>(outputs[2]);
+    tails.batch = batch, tails.max_rows = maxV;
+    FillRanges fills{};
+    fills.ptr[0] = static_cast<uint4*>(ws.ones_base), fills.n16[0] = ws.ones_bytes / 16, fills.ones[0] = 1;
+    fills.ptr[1] = static_cast<uint4*>(ws.zero_base), fills.n16[1] = ws.zero_bytes / 16, fills.ones[1] = 0;
+    fills.status = ws.status;
+    rc = launch_prepare(fills, subm ? tails : TailRows{}, stream);
     if (rc) return rc;
     const int32_t* out_num = in_num;
     if (subm && is_subm_333(g)) {
@@ -476,12 +509,13 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     } else {
         rc = launch_mark_outputs(in_coors, in_num, batch, maxV, g, ws.out_bits, stream);
         if (rc) return rc;
-        rc = launch_number_outputs(ws.out_bits, batch, maxV, ws.chunk_counts, static_cast<int32_t*>(outputs[1]),
+        rc = launch_number_outputs(ws.out_bits, nullptr, g, batch, maxV, ws.scan, static_cast<int32_t*>(outputs[1]),
                                    static_cast<int32_t*>(outputs[2]), ws.status, stream);
         if (rc) return rc;
         out_num = static_cast<const int32_t*>(outputs[2]);
         // the caller's input rows come in any order and have no grid of their own: input-stationary map
-        rc = launch_scatter_rows(in_coors, in_num, out_num, batch, maxV, g, ws.out_bits, ws.nbr, ws.tile_mask, stream);
+        rc = launch_scatter_rows(in_coors, in_num, out_num, batch, maxV, g, ws.out_bits, ws.nbr, ws.tile_mask, tails,
+                                 stream);
         if (rc) return rc;
     }
     ConvLaunch c{};
@@ -505,13 +539,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     c.debug_withhold_weights = w->impl.debug_withhold;
     c.scale_host = w->impl.host_scale;
     c.shift_host = w->impl.host_shift;
-    rc = choose_conv(c, stream);
-    if (rc) return rc;
-    // Rows past the active count are zero in the reference (outputs are memset, submConv3dlayer.cu:594).
-    rc = launch_zero_tail(outputs[0], (int)(p->out_channel * esize(w->impl.dtype)), out_num, batch, maxV, stream);
-    if (rc) return rc;
-    if (!subm) rc = launch_zero_tail(outputs[1], 16, out_num, batch, maxV, stream);
-    return rc;
+    return choose_conv(c, stream);
 }
 
 int sessd_subm_conv_enqueue(const sessd_conv_params* p, const sessd_conv_weights* w, int batch,
@@ -604,9 +632,8 @@ int sessd_backbone_create(const sessd_voxel_params* vp, const sessd_conv_params*
     bb->dtype = dtype;
     bb->max_voxels = vp->max_voxels;
     bb->nlevels = 1;
-    bb->kvol_strided_max = 0;
-    bb->ncand_max = 0;
     bb->level_has_subm.assign(1, 0);
+    bb->level_derived.assign(1, 0);
     int rc = SESSD_OK;
     int cur_c = vp->voxel_feature_num;
     for (int i = 0; i < nlayers && rc == SESSD_OK; ++i) {
@@ -635,8 +662,7 @@ int sessd_backbone_create(const sessd_voxel_params* vp, const sessd_conv_params*
             L.level_out = bb->nlevels++;
             bb->level_shape.insert(bb->level_shape.end(), {L.g.out_shape[0], L.g.out_shape[1], L.g.out_shape[2]});
             bb->level_has_subm.push_back(0);
-            if (L.g.kvol > bb->kvol_strided_max) bb->kvol_strided_max = L.g.kvol;
-            if (L.g.ncand > bb->ncand_max) bb->ncand_max = L.g.ncand;
+            bb->level_derived.push_back(L.level_in > 0 && derivable_in_x(L.g) ? 1 : 0);
         }
         rc = sessd_conv_weights_create(&L.p, weights[i], scale ? scale[i] : nullptr, shift ? shift[i] : nullptr, 1, dtype,
                                        &L.w);
@@ -687,18 +713,16 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
     if (bump.total() > workspace_bytes) return SESSD_ERR_WORKSPACE;
     if (!workspace_aligned(workspace)) return SESSD_ERR_PARAM;
     const int maxV = bb->max_voxels;
-    // keep_status (pipelines): word 0 is left alone, so that it collects the conditions of every group of a run
-    SESSD_CUDA(cudaMemsetAsync(w.status + (keep_status ? 1 : 0), 0, (kStatusInts - (keep_status ? 1 : 0)) * sizeof(int32_t),
-                               stream));
-    // one launch resets everything the call needs: the voxeliser's table and the bucket table (0xFF), the grids and
-    // tile masks (0), and the BEV map (0; by cudaMemsetAsync when its size is not a multiple of 16 bytes)
+    // One launch resets everything the call needs: the voxeliser's table and the bucket table (0xFF), the grids, masks
+    // and numbering state (0), the BEV map (0; by cudaMemsetAsync when its size is not a multiple of 16 bytes) and the
+    // status block. keep_status (pipelines): word 0 is left alone, so that it collects the conditions of every group.
     FillRanges fills{};
-    fills.ptr[0] = static_cast<uint4*>(w.ones_base), fills.n16[0] = w.ones_bytes / 16, fills.ones[0] = 1;
+    fills.ptr[0] = static_cast<uint4*>(w.ones_base), fills.n16[0] = bb->level_has_subm[0] ? w.ones_bytes / 16 : 0, fills.ones[0] = 1;
     fills.ptr[1] = static_cast<uint4*>(w.zero_base), fills.n16[1] = w.zero_bytes / 16, fills.ones[1] = 0;
-    fills.ptr[2] = static_cast<uint4*>(static_cast<void*>(w.vox.table_base)), fills.n16[2] = w.vox.table_bytes / 16,
-    fills.ones[2] = 1;
-    const bool table_in_fill = w.vox.table_bytes % 16 == 0 && reinterpret_cast<uintptr_t>(w.vox.table_base) % 16 == 0;
-    if (!table_in_fill) fills.n16[2] = 0;
+    fills.ptr[2] = static_cast<uint4*>(w.vox.table_base), fills.n16[2] = w.vox.table_bytes / 16, fills.ones[2] = 1;
+    fills.ptr[4] = static_cast<uint4*>(w.vox.zero_base), fills.n16[4] = w.vox.zero_bytes / 16, fills.ones[4] = 0;
+    fills.status = w.status;
+    fills.status_from = keep_status ? 1 : 0;
     if (bb->has_s2d) {
         const size_t bytes = (size_t)batch * bb->s2d.feature_map_channel * bb->s2d.feature_map_size_z *
                              (bb->s2d.feature_map_size_y + bb->pad.top + bb->pad.bottom) *
@@ -708,52 +732,67 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         else
             SESSD_CUDA(cudaMemsetAsync(dense, 0, bytes, stream));
     }
-    int rc = launch_fill_ranges(fills, stream);
+    int rc = launch_prepare(fills, TailRows{}, stream);
     if (rc) return rc;
+    // Coordinates first: voxels, the rows of every level, and all neighbour maps; then the convolutions.
+    VoxelHooks hooks{};
+    if (bb->level_has_subm[0]) hooks.buckets = w.buckets0;
+    const sessd_backbone::Layer* leaving0 = nullptr;   // the strided layer that leaves the voxeliser's level
+    for (auto& L : bb->layers)
+        if (!L.p.subm && L.level_in == 0) leaving0 = &L;
+    if (leaving0) hooks.marks = w.bits[1], hooks.geom = leaving0->g;
     rc = voxelize_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
                       static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vox,
-                      /*zero_tail=*/false, stream, table_in_fill);
+                      /*zero_tail=*/false, hooks, stream);
     if (rc) return rc;
+    if (bb->level_has_subm[0]) {
+        // the voxeliser's rows: one thread per row looks its 27 neighbours up in the x-grouped table
+        rc = launch_nbr_build_subm(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, w.nbr_subm[0],
+                                   w.mask_subm[0], stream);
+        if (rc) return rc;
+    }
+    MapJobs jobs{};
+    auto add_job = [&](const sessd_backbone::Layer& L, int32_t* nbr, uint32_t* mask) {
+        if (jobs.count == MapJobs::kMax) {
+            const int rc_jobs = launch_map_rows(jobs, batch, maxV, stream);
+            if (rc_jobs) return rc_jobs;
+            jobs.count = 0;
+        }
+        jobs.job[jobs.count++] = MapJob{w.coors[L.level_out], w.num[L.level_out], L.g, w.bits[L.level_in], nbr, mask};
+        return (int)SESSD_OK;
+    };
     std::vector<char> nbr_ready(bb->nlevels, 0);
+    for (size_t i = 0; i < bb->layers.size(); ++i) {
+        const sessd_backbone::Layer& L = bb->layers[i];
+        if (L.p.subm) {
+            if (L.level_in == 0 || nbr_ready[L.level_in]) continue;
+            nbr_ready[L.level_in] = 1;
+            rc = add_job(L, w.nbr_subm[L.level_in], w.mask_subm[L.level_in]);
+            if (rc) return rc;
+            continue;
+        }
+        const bool derived = bb->level_derived[L.level_out] != 0;
+        if (L.level_in > 0 && !derived) {
+            rc = launch_mark_outputs(w.coors[L.level_in], w.num[L.level_in], batch, maxV, L.g, w.bits[L.level_out], stream);
+            if (rc) return rc;
+        }
+        rc = launch_number_outputs(w.bits[L.level_out], derived ? &w.bits[L.level_in] : nullptr, L.g, batch, maxV,
+                                   w.scan[L.level_out], w.coors[L.level_out], w.num[L.level_out], w.status, stream);
+        if (rc) return rc;
+        if (L.level_in == 0)   // no grid for the voxeliser's rows: every candidate finds its output row instead
+            rc = launch_scatter_rows(w.coors[0], w.num[0], w.num[L.level_out], batch, maxV, L.g, w.bits[L.level_out],
+                                     w.nbr_layer[i], w.mask_layer[i], TailRows{}, stream);
+        else
+            rc = add_job(L, w.nbr_layer[i], w.mask_layer[i]);
+        if (rc) return rc;
+    }
+    rc = launch_map_rows(jobs, batch, maxV, stream);
+    if (rc) return rc;
     const void* cur = w.voxel_feat;
     for (size_t i = 0; i < bb->layers.size(); ++i) {
         const sessd_backbone::Layer& L = bb->layers[i];
-        const int32_t* nbr;
-        const uint32_t* tile_mask;
-        if (L.p.subm) {
-            if (!nbr_ready[L.level_in]) {
-                if (L.level_in == 0) {
-                    // the voxeliser's rows: x-grouped table, then one thread per row looks its 27 neighbours up
-                    rc = launch_bucket_build(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, w.status,
-                                             stream);
-                    if (rc) return rc;
-                    rc = launch_nbr_build_subm(w.coors[0], w.num[0], batch, maxV, L.g.in_shape, w.buckets0, w.nbr_subm[0],
-                                               w.mask_subm[0], stream);
-                } else {
-                    rc = launch_map_rows(w.coors[L.level_in], w.num[L.level_in], batch, maxV, L.g, w.bits[L.level_in],
-                                         w.nbr_subm[L.level_in], w.mask_subm[L.level_in], stream);
-                }
-                if (rc) return rc;
-                nbr_ready[L.level_in] = 1;
-            }
-            nbr = w.nbr_subm[L.level_in];
-            tile_mask = w.mask_subm[L.level_in];
-        } else {
-            rc = launch_mark_outputs(w.coors[L.level_in], w.num[L.level_in], batch, maxV, L.g, w.bits[L.level_out], stream);
-            if (rc) return rc;
-            rc = launch_number_outputs(w.bits[L.level_out], batch, maxV, w.chunk_counts, w.coors[L.level_out],
-                                       w.num[L.level_out], w.status, stream);
-            if (rc) return rc;
-            if (L.level_in == 0)   // no grid for the voxeliser's rows: every candidate finds its output row instead
-                rc = launch_scatter_rows(w.coors[0], w.num[0], w.num[L.level_out], batch, maxV, L.g, w.bits[L.level_out],
-                                         w.nbr_strided, w.mask_layer[i], stream);
-            else
-                rc = launch_map_rows(w.coors[L.level_out], w.num[L.level_out], batch, maxV, L.g, w.bits[L.level_in],
-                                     w.nbr_strided, w.mask_layer[i], stream);
-            if (rc) return rc;
-            nbr = w.nbr_strided;
-            tile_mask = w.mask_layer[i];
-        }
+        const int32_t* nbr = L.p.subm ? w.nbr_subm[L.level_in] : w.nbr_layer[i];
+        const uint32_t* tile_mask = L.p.subm ? w.mask_subm[L.level_in] : w.mask_layer[i];
         if (count_pairs) {
             auto* counters = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(w.status) + 256);
             rc = launch_count_pairs(nbr, w.num[L.level_out], batch, maxV, L.g.kvol, counters + i, stream);

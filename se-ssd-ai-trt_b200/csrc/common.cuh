@@ -14,7 +14,7 @@ namespace sessd {
 
 constexpr uint32_t kEmpty = 0xFFFFFFFFu;   // empty key / unset rank in a coordinate table
 constexpr size_t kAlign = 256;             // sub-buffer alignment inside a workspace
-constexpr int kChunk = 1024;               // entries per compaction chunk (256 threads x 4)
+constexpr int kStatusInts = 256;           // status block: 1 KB; word 0 is the status, bytes 256.. hold 64 pair counters
 constexpr int kThreads = 256;
 constexpr int kMaxBatch = 4096;
 
@@ -149,14 +149,12 @@ struct BitGrid {
     int Z, Y, X;
     int xw;      // records per x line
     int words;   // records per frame
-    int chunks;  // 1024-record chunks per frame
 };
 inline BitGrid bitgrid_shape(const int shape[3]) {
     BitGrid g{};
     g.Z = shape[0], g.Y = shape[1], g.X = shape[2];
     g.xw = (g.X + 63) / 64;
     g.words = g.Z * g.Y * g.xw;
-    g.chunks = (g.words + kChunk - 1) / kChunk;
     return g;
 }
 
@@ -260,36 +258,35 @@ __device__ __forceinline__ int block_sum(int v) {
 
 // ---- pieces shared between translation units --------------------------------------------
 
-// Ordered-unique numbering. Entry e of frame b (e < entries(b)) points at table slot
-// slot_of[b][e] (or -1). The entry whose index equals the slot's rank owns the slot; owners are
-// numbered 0,1,2,... in entry order. count pass + emit pass, no block waits on another block.
-struct NumberingArgs {
-    const int32_t* slot_of;     // [B][entry_stride]
-    uint32_t slot_mask;         // bits of a non-negative slot_of value that hold the slot (the rest is the caller's)
-    int64_t entry_stride;
-    const int32_t* entry_count; // [B] device counts (points_size or voxel_num)
-    int entry_mul;              // entries(b) = min(entry_count[b], entry_limit) * entry_mul
-    int entry_limit;
-    int32_t* chunk_counts;      // [B][chunks_per_frame]
-    int chunks_per_frame;
-    int batch;
-};
-
-int launch_count_owners(const NumberingArgs& a, const Table& t, cudaStream_t stream);
-
-// Zeroes rows [voxel_num[b], max_voxels) of a [B][max_voxels][row_bytes] tensor (row_bytes % 4 == 0).
-int launch_zero_tail(void* tensor, int row_bytes, const int32_t* voxel_num, int batch, int max_voxels,
-                     cudaStream_t stream);
-int launch_fill_zero(void* ptr, size_t bytes, cudaStream_t stream);  // bytes % 16 == 0, ptr 16-byte aligned
-int launch_fill_ones(void* ptr, size_t bytes, cudaStream_t stream);  // every byte 0xFF; same constraints
-// Several fills as one launch: range r is n16[r] 16-byte words at ptr[r] (16-byte aligned), 0xFF bytes when ones[r]
-// is set, else zeros; unused ranges have n16 = 0.
+// One launch for the resets a call needs. Range r is n16[r] 16-byte words at ptr[r] (16-byte aligned), 0xFF bytes when
+// ones[r] is set, else zeros; unused ranges have n16 = 0. status: words status_from .. kStatusInts - 1 of the status
+// block to zero, or null.
 struct FillRanges {
-    uint4* ptr[4];
-    size_t n16[4];
-    int ones[4];
+    static constexpr int kMax = 5;
+    uint4* ptr[kMax];
+    size_t n16[kMax];
+    int ones[kMax];
+    int32_t* status;
+    int status_from;
 };
-int launch_fill_ranges(const FillRanges& f, cudaStream_t stream);
+// Output tensors [batch][max_rows][row_bytes] whose rows from counts[b] on are to be zero (row_bytes % 2 == 0; null: unused).
+struct TailRows {
+    static constexpr int kMax = 3;
+    void* tensor[kMax];
+    int row_bytes[kMax];
+    const int32_t* counts;
+    int batch, max_rows;
+};
+int launch_prepare(const FillRanges& f, const TailRows& t, cudaStream_t stream);
+int launch_fill_zero(void* ptr, size_t bytes, cudaStream_t stream);  // bytes % 16 == 0, ptr 16-byte aligned
+
+// What a one-pass numbering kernel (scan.cuh) keeps in global memory: a word per chunk of kThreads entries and a ticket
+// counter; all zero before the kernel.
+struct ScanState {
+    unsigned long long* state;   // [batch][scan_chunks(entries)]
+    uint32_t* ticket;
+};
+__host__ __device__ inline int scan_chunks(int entries) { return (entries + kThreads - 1) / kThreads; }
 
 // rulebook.cu
 int conv_geom_from_params(const sessd_conv_params* p, ConvGeom* g);
@@ -297,20 +294,36 @@ int launch_table_build(const int32_t* coors, const int32_t* voxel_num, int batch
                        const Table& t, int32_t* status, cudaStream_t stream);
 int launch_nbr_build(const int32_t* out_coors, const int32_t* out_num, int batch, int max_voxels, const ConvGeom& g,
                      const Table& in_table, int32_t* nbr, cudaStream_t stream);
-// Strided layers: set the bit of every candidate output, then number the set bits in (z, y, x) order.
+// Strided layers: set the bit of every candidate output, then number the set bits in (z, y, x) order. With derive_from
+// the bits are taken from the input level's grid instead (derivable_in_x must hold) and `out` needs no reset.
 int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batch, int max_voxels, const ConvGeom& g,
                         const BitGrid& out, cudaStream_t stream);
-int launch_number_outputs(const BitGrid& out, int batch, int max_voxels, int32_t* chunk_counts, int32_t* out_coors,
-                          int32_t* out_num, int32_t* status, cudaStream_t stream);
-// Neighbour map + tile masks of a layer (any kernel up to 3x3x3, any stride) whose input level has an occupancy
-// grid: output-stationary, one thread per output row.
-int launch_map_rows(const int32_t* out_coors, const int32_t* out_num, int batch, int max_voxels, const ConvGeom& g,
-                    const BitGrid& in, int32_t* nbr, uint32_t* tile_mask, cudaStream_t stream);
+bool derivable_in_x(const ConvGeom& g);
+int launch_number_outputs(const BitGrid& out, const BitGrid* derive_from, const ConvGeom& g, int batch, int max_voxels,
+                          const ScanState& scan, int32_t* out_coors, int32_t* out_num, int32_t* status,
+                          cudaStream_t stream);
+// Neighbour maps + tile masks of layers (any kernel up to 3x3x3, any stride) whose input level has an occupancy grid:
+// output-stationary, one thread per output row; one launch for up to MapJobs::kMax layers.
+struct MapJob {
+    const int32_t* out_coors;
+    const int32_t* out_num;
+    ConvGeom g;
+    BitGrid in;
+    int32_t* nbr;
+    uint32_t* tile_mask;
+};
+struct MapJobs {
+    static constexpr int kMax = 8;
+    MapJob job[kMax];
+    int count;
+};
+int launch_map_rows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream);
 // The same for a strided layer whose input rows have no grid (voxeliser rows, caller's rows): input-stationary,
-// every candidate of every input row finds its output row in the numbered output grid. Clears the map first.
+// every candidate of every input row finds its output row in the numbered output grid. Clears the map first, and with
+// the same launch the tails of the call's outputs.
 int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch,
                         int max_voxels, const ConvGeom& g, const BitGrid& out, int32_t* nbr, uint32_t* tile_mask,
-                        cudaStream_t stream);
+                        const TailRows& tails, cudaStream_t stream);
 int launch_bucket_build(const int32_t* coors, const int32_t* voxel_num, int batch, int max_voxels, const int shape[3],
                         const Buckets& t, int32_t* status, cudaStream_t stream);
 // 3x3x3 / stride 1 / pad 1 neighbour map from a bucket table, plus the per-128-row-tile offset masks.
@@ -366,16 +379,27 @@ struct VoxelWorkspace {
     int32_t* status;
     Table table;          // rank = per-slot sorted point list [cap][max_pts]
     int32_t* pt_slot;     // [B][max_points]
-    int32_t* chunk_counts;// [B][chunks]
+    ScanState scan;       // numbering of the owner points
+    void* zero_base;      // the scan's words, to be zero before a call
+    size_t zero_bytes;
     int32_t* num_points;  // [B][max_voxels]
-    int chunks;
     size_t table_bytes;   // bytes to set to 0xFF before a call (keys + point lists)
     void* table_base;
 };
 void voxel_workspace_layout(Bump& bump, const sessd_voxel_params* p, int batch, int max_points, VoxelWorkspace* w);
+// What the voxeliser can do with a new voxel's row on the way: enter it into the x-grouped table of its level and mark
+// its candidate outputs in the next level's grid.
+struct VoxelHooks {
+    Buckets buckets;      // data == nullptr: none
+    BitGrid marks;        // rec == nullptr: none
+    ConvGeom geom;        // of the strided layer the marks belong to
+};
+// The points of a batch -> rows; the caller has reset the table, the scan's words and the status (and, for a call that
+// returns whole tensors, the rows past each frame's point count). zero_tail: also zero the rows between a frame's voxel
+// count and its point count.
 int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
                  const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelWorkspace& w,
-                 bool zero_tail, cudaStream_t stream, bool table_is_reset = false);   // table_is_reset: the caller has filled w.table_base
+                 bool zero_tail, const VoxelHooks& hooks, cudaStream_t stream);
 
 struct sessd_conv_weights_impl {
     void* w;        // device, [kvol][Cin][Cout] in dtype

@@ -22,7 +22,9 @@
 //     arrival order of an atomic over a dense scan (sparseConv3dlayer.cu:529-541); (z, y, x) order is
 //     deterministic and keeps the rows of a 128-row tile close together in space;
 //   - coordinates handed in by a caller (the stand-alone plugin entry points) go into a flat table.
-#include "numbering.cuh"
+#include "fill.cuh"
+#include "rulebook.cuh"
+#include "scan.cuh"
 
 namespace sessd {
 
@@ -87,27 +89,6 @@ nbr_build_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__
             if (slot >= 0) row = in_table.vals[(size_t)b * in_table.cap + slot];
         }
         nbr[nbr_index(g.kvol, max_voxels, b, k, o)] = row;
-    }
-}
-
-// Integer helpers for the candidate geometry. Strides and candidate spans are 1, 2 or 3; a division by a
-// run-time divisor costs some 25 instructions on the GPU and these kernels are bound by instruction issue,
-// so the common divisors get shifts.
-__device__ __forceinline__ int div_trunc(int a, int s) {   // C division (rounds toward zero)
-    if (s == 1) return a;
-    if (s == 2) return (a + (a < 0 ? 1 : 0)) >> 1;
-    return a / s;
-}
-__device__ __forceinline__ void split_small(int e, int m, int* q, int* r) {   // e = q * m + r, e >= 0
-    if (m == 1) {
-        *q = e;
-        *r = 0;
-    } else if (m == 2) {
-        *q = e >> 1;
-        *r = e & 1;
-    } else {
-        *q = e / m;
-        *r = e - *q * m;
     }
 }
 
@@ -181,21 +162,7 @@ bucket_build_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ 
             continue;
         }
         const uint32_t key = ((uint32_t)c.y * Y + c.z) * X + c.w;
-        const uint32_t gkey = key >> 2;
-        uint32_t* base = t.data + (size_t)b * t.cap * 8;
-        uint32_t h = hash_slot(gkey, t.shift);
-        bool done = false;
-        for (uint32_t probe = 0; probe < t.cap && !done; ++probe) {
-            uint32_t* bk = base + (size_t)h * 8;
-            uint32_t cur = bk[4];
-            if (cur == kEmpty) cur = atomicCAS(&bk[4], kEmpty, gkey);
-            if (cur == kEmpty || cur == gkey) {
-                atomicMax(reinterpret_cast<int32_t*>(&bk[key & 3u]), i);  // duplicates: highest row wins
-                done = true;
-            }
-            h = (h + 1) & (t.cap - 1);
-        }
-        if (!done) atomicOr(status, SESSD_STATUS_HASH_FULL);
+        if (!bucket_insert(t.data + (size_t)b * t.cap * 8, t.cap, t.shift, key, i)) atomicOr(status, SESSD_STATUS_HASH_FULL);
     }
 }
 
@@ -312,154 +279,120 @@ nbr_build_subm_kernel(const int4* __restrict__ coors, const int32_t* __restrict_
 
 // ---- occupancy grids -----------------------------------------------------------------------------
 
-__device__ __forceinline__ unsigned long long rec_bits(const uint4& r) {
-    return (unsigned long long)r.x | ((unsigned long long)r.y << 32);
-}
-
-// Marks the candidate outputs of every input row: the reference's enumeration (sparseConv3dlayer.cu:339-383),
-// one thread per input row. Per axis the row has up to three candidate output positions (one or two for the
-// stride-2 layers); the x candidates of one (z, y) pair are neighbouring bits, mostly of one 64-bit word, so
-// they are tested and set together, and all words are read before any is updated (the reads are independent;
-// most of them find their bits already set by a neighbouring row and nothing is written).
+// Marks the candidate outputs of every input row, one thread per row.
 __global__ void __launch_bounds__(kThreads)
 mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict__ in_num, int batch, int max_voxels,
                     ConvGeom g, BitGrid out) {
     pdl_enter();
-    constexpr int MAXS = 3;   // span_max never exceeds the kernel size (<= 3)
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
     const int items = batch * chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
-        const int i0 = (it - b * chunks) * kThreads;
+        const int i = (it - b * chunks) * kThreads + threadIdx.x;
         int n = in_num[b];
         n = n > max_voxels ? max_voxels : n;
-        if (i0 >= n) continue;   // uniform over the block
-        const int i = i0 + threadIdx.x;
         if (i >= n) continue;
-        const int4 c4 = __ldg(&in_coors[(size_t)b * max_voxels + i]);
-        const int c[3] = {c4.y, c4.z, c4.w};
-        // candidate positions per axis, upper corner downward; pos[j][e] < 0 marks an unusable candidate
-        int pos[3][MAXS];
-        bool in_ok = true;
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-            // C integer division, as in the reference (sparseConv3dlayer.cu:339-348); dilation is 1
-            const int lo = div_trunc(c[j] - (g.K[j] - 1) - 1 + g.S[j] + g.P[j], g.S[j]);
-            const int hi = div_trunc(c[j] + g.P[j], g.S[j]);
-            in_ok = in_ok && c[j] >= 0 && c[j] < g.in_shape[j];
-#pragma unroll
-            for (int e = 0; e < MAXS; ++e) {
-                const int o = hi - e;
-                const int k = c[j] - o * g.S[j] + g.P[j];   // the offset this pair would get (:366)
-                const bool ok = e < g.span_max[j] && e <= hi - lo && o >= 0 && o < g.out_shape[j] && k >= 0 && k < g.K[j];
-                pos[j][e] = ok ? o : -1;
-            }
-        }
-        if (!in_ok) continue;
-        // the x candidates as bits of at most two neighbouring words
-        int w0 = -1;
-        unsigned long long bits0 = 0ull, bits1 = 0ull;
-#pragma unroll
-        for (int e = 0; e < MAXS; ++e) {
-            const int ox = pos[2][e];
-            if (ox < 0) continue;
-            if (w0 < 0) w0 = ox >> 6;            // candidates descend, so the first valid one has the highest word
-            if ((ox >> 6) == w0) bits0 |= 1ull << (ox & 63);
-            else bits1 |= 1ull << (ox & 63);     // the word below (spans are at most three cells)
-        }
-        if (w0 < 0) continue;
-        unsigned long long* base = reinterpret_cast<unsigned long long*>(out.rec + (size_t)b * out.words);
-        unsigned long long cur0[MAXS * MAXS], cur1[MAXS * MAXS];
-        size_t rec[MAXS * MAXS];
-#pragma unroll
-        for (int ez = 0; ez < MAXS; ++ez)
-#pragma unroll
-            for (int ey = 0; ey < MAXS; ++ey) {
-                const int q = ez * MAXS + ey;
-                const bool ok = pos[0][ez] >= 0 && pos[1][ey] >= 0;
-                rec[q] = ok ? ((size_t)pos[0][ez] * out.Y + pos[1][ey]) * out.xw + w0 : (size_t)-1;
-                // a record is 16 bytes: its bits are the first 8
-                cur0[q] = ok ? *reinterpret_cast<volatile unsigned long long*>(base + 2 * rec[q]) : ~0ull;
-                cur1[q] = (ok && bits1) ? *reinterpret_cast<volatile unsigned long long*>(base + 2 * (rec[q] - 1)) : ~0ull;
-            }
-#pragma unroll
-        for (int q = 0; q < MAXS * MAXS; ++q) {
-            if (rec[q] == (size_t)-1) continue;
-            if ((cur0[q] & bits0) != bits0) atomicOr(base + 2 * rec[q], bits0);
-            if (bits1 && (cur1[q] & bits1) != bits1) atomicOr(base + 2 * (rec[q] - 1), bits1);
-        }
+        mark_row(__ldg(&in_coors[(size_t)b * max_voxels + i]), b, g, out);
     }
 }
 
-// Set bits of every 1024-word chunk of every frame.
-__global__ void __launch_bounds__(kThreads)
-count_bits_kernel(BitGrid g, int batch, int32_t* __restrict__ chunk_counts) {
-    pdl_enter();
-    const int items = batch * g.chunks;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int b = it / g.chunks, c = it - b * g.chunks;
-        const uint4* rec = g.rec + (size_t)b * g.words;
-        int cnt = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int w = c * kChunk + threadIdx.x * 4 + j;
-            if (w < g.words) cnt += __popcll(rec_bits(rec[w]));
-        }
-        const int total = block_sum(cnt);
-        if (threadIdx.x == 0) chunk_counts[(size_t)b * g.chunks + c] = total;
-    }
+// The even bits of v, packed into the low half.
+__device__ __forceinline__ uint32_t even_bits(unsigned long long v) {
+    v &= 0x5555555555555555ull;
+    v = (v | (v >> 1)) & 0x3333333333333333ull;
+    v = (v | (v >> 2)) & 0x0F0F0F0F0F0F0F0Full;
+    v = (v | (v >> 4)) & 0x00FF00FF00FF00FFull;
+    v = (v | (v >> 8)) & 0x0000FFFF0000FFFFull;
+    return (uint32_t)(v | (v >> 16));
 }
 
-// Numbers the set bits of a frame in word order (= (z, y, x) order): writes every word's prefix, the output
-// coordinates (sparseConv3dlayer.cu:436-441 writes them per pair) and the frame's row count. Rows past
-// max_voxels are dropped (their bits stay set; look-ups reject ids >= max_voxels) and reported.
+// Output cells of word w of an output level from the occupancy of its input level: a cell is an output when any cell of
+// its receptive field is occupied, which is the set that marking every input row's candidates gives (the truncating
+// divisions of sparseConv3dlayer.cu:339-348 drop no valid candidate). In x the two cases of derivable_in_x; z and y are
+// free. The input words of all lines are read side by side and ORed before the bits are spread.
+__device__ __forceinline__ unsigned long long derive_word(const BitGrid& in, const BitGrid& out, const ConvGeom& g, int b, int w) {
+    const int row = w / out.xw, wx = w - row * out.xw;
+    const int z = row / out.Y, y = row - z * out.Y;
+    const unsigned long long* base = reinterpret_cast<const unsigned long long*>(in.rec + (size_t)b * in.words);
+    const bool same = g.K[2] == 1;                  // kernel 1, stride 1: the word itself; else kernel 3, stride 2, padding 1
+    const int first = same ? wx : 2 * wx;
+    unsigned long long before = 0ull, lo = 0ull, hi = 0ull;
+#pragma unroll
+    for (int kz = 0; kz < 3; ++kz) {
+        const int iz = z * g.S[0] - g.P[0] + kz;
+        if (kz >= g.K[0] || iz < 0 || iz >= in.Z) continue;
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+            const int iy = y * g.S[1] - g.P[1] + ky;
+            if (ky >= g.K[1] || iy < 0 || iy >= in.Y) continue;
+            const unsigned long long* line = base + 2 * ((size_t)iz * in.Y + iy) * in.xw;   // a record is 16 bytes: bits first
+            if (first < in.xw) lo |= __ldg(line + 2 * first);
+            if (!same) {
+                if (first > 0) before |= __ldg(line + 2 * (first - 1));
+                if (first + 1 < in.xw) hi |= __ldg(line + 2 * (first + 1));
+            }
+        }
+    }
+    unsigned long long bits = lo;
+    if (!same) {
+        // output x has the inputs 2x - 1, 2x, 2x + 1
+        const unsigned long long even = (unsigned long long)even_bits(lo) | (unsigned long long)even_bits(hi) << 32;
+        const unsigned long long odd = (unsigned long long)even_bits(lo >> 1) | (unsigned long long)even_bits(hi >> 1) << 32;
+        bits = even | odd | (odd << 1) | (before >> 63);
+    }
+    const int x0 = wx << 6;
+    if (x0 + 64 > out.X) bits &= x0 < out.X ? (1ull << (out.X - x0)) - 1ull : 0ull;   // cells past the line's end
+    return bits;
+}
+
+// Numbers the occupied cells of every frame's output level in word order (= (z, y, x) order): completes the records
+// (bits, rows before the word), writes the output coordinates (sparseConv3dlayer.cu:436-441 writes them per pair) and the
+// frame's row count. The bits come from the records (marked by an earlier kernel) or, with DERIVE, from the input
+// level's records; then the grid needs no reset either. Rows past max_voxels are dropped (their bits too, so that the
+// next level does not see them) and reported. One thread per word; a warp then writes its words' coordinates one word
+// at a time, a lane per cell. Two kernels (count, then prefix and emit with a serial loop over a thread's bits) took 3.5 +
+// 18 us per level of a 20,000-point frame.
+template <bool DERIVE>
 __global__ void __launch_bounds__(kThreads)
-number_outputs_kernel(BitGrid g, int batch, int max_voxels, const int32_t* __restrict__ chunk_counts,
+number_outputs_kernel(BitGrid g, BitGrid in, ConvGeom geom, int batch, int max_voxels, ScanState scan,
                       int4* __restrict__ out_coors, int32_t* __restrict__ out_num, int32_t* status) {
     pdl_enter();
-    const int items = batch * g.chunks;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int b = it / g.chunks, c = it - b * g.chunks;
-        const int32_t* counts = chunk_counts + (size_t)b * g.chunks;
-        if (c == 0) {
-            int partial = 0;
-            for (int j = threadIdx.x; j < g.chunks; j += kThreads) partial += counts[j];
-            const int total = block_sum(partial);
-            if (threadIdx.x == 0) {
-                out_num[b] = total > max_voxels ? max_voxels : total;
-                if (total > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
-            }
-        }
-        int partial = 0;
-        for (int j = threadIdx.x; j < c; j += kThreads) partial += counts[j];
-        const int base = block_sum(partial);
+    const int lane = threadIdx.x & 31;
+    const int chunks = scan_chunks(g.words), items = batch * chunks;
+    for (int t = scan_ticket(scan.ticket, items); t >= 0; t = scan_ticket(scan.ticket, items)) {
+        const int c = t / batch, b = t - c * batch;
+        const int w = c * kThreads + threadIdx.x;
         uint4* rec = g.rec + (size_t)b * g.words;
-        unsigned long long bits[4];
-        int cnt = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int w = c * kChunk + threadIdx.x * 4 + j;
-            bits[j] = w < g.words ? rec_bits(rec[w]) : 0ull;
-            cnt += __popcll(bits[j]);
+        unsigned long long bits = 0ull;
+        if (w < g.words) bits = DERIVE ? derive_word(in, g, geom, b, w) : rec_bits(rec[w]);
+        int end;
+        const int id = scan_position(scan.state + (size_t)b * chunks, c, __popcll(bits), &end, status);
+        if (c == chunks - 1 && threadIdx.x == 0) {
+            out_num[b] = end > max_voxels ? max_voxels : end;
+            if (end > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
         }
-        int unused;
-        int id = base + block_exclusive_scan(cnt, &unused);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int w = c * kChunk + threadIdx.x * 4 + j;
-            if (w >= g.words) continue;
-            rec[w].z = (uint32_t)id;
-            unsigned long long rem = bits[j];
-            if (!rem) continue;
-            const int row = w / g.xw;                 // z * Y + y
-            const int x0 = (w - row * g.xw) << 6;
-            const int z = row / g.Y, y = row - z * g.Y;
-            while (rem) {
-                const int bit = __ffsll((long long)rem) - 1;
+        if (id + __popcll(bits) > max_voxels) {          // keep the first max_voxels - id cells
+            int keep = max_voxels - id > 0 ? max_voxels - id : 0;
+            unsigned long long kept = 0ull;
+            for (unsigned long long rem = bits; rem && keep; --keep) {
+                kept |= rem & (0ull - rem);
                 rem &= rem - 1ull;
-                if (id < max_voxels) out_coors[(size_t)b * max_voxels + id] = make_int4(b, z, y, x0 + bit);
-                ++id;
             }
+            bits = kept;
+        }
+        if (w < g.words) rec[w] = make_uint4((uint32_t)bits, (uint32_t)(bits >> 32), (uint32_t)id, 0u);
+        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, bits != 0ull); todo; todo &= todo - 1u) {
+            const int src = __ffs((int)todo) - 1;
+            const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits, src);
+            const int id0 = __shfl_sync(0xFFFFFFFFu, id, src);
+            const int word = w - lane + src;
+            const int row = word / g.xw;                 // z * Y + y
+            const int x0 = (word - row * g.xw) << 6;
+            const int z = row / g.Y, y = row - z * g.Y;
+            int4* dst = out_coors + (size_t)b * max_voxels + id0;
+            const uint32_t v_lo = (uint32_t)v, v_hi = (uint32_t)(v >> 32), below = (1u << lane) - 1u;
+            if ((v_lo >> lane) & 1u) dst[__popc(v_lo & below)] = make_int4(b, z, y, x0 + lane);
+            if ((v_hi >> lane) & 1u) dst[__popc(v_lo) + __popc(v_hi & below)] = make_int4(b, z, y, x0 + 32 + lane);
         }
     }
 }
@@ -514,22 +447,28 @@ struct BitsIndex {
     }
 };
 
-// Neighbour map of a layer whose input level has an occupancy grid: one thread per output row walks the
+// Neighbour maps of layers whose input level has an occupancy grid: one thread per output row walks the
 // K0 x K1 lines of its receptive field, has the grid reads of a kz plane in flight together, and writes
 // nbr[b][k][o] (coalesced over o) plus the per-128-row-tile offset mask (one ballot per offset, one atomic
 // per warp). in = out*stride - pad + k, the inverse of the offset formula at submConv3dlayer.cu:328.
+// All layers of a call go in one launch (the maps depend on coordinates only): on a 20,000-point frame six launches of
+// 6 to 10 us each kept a fraction of the SMs busy.
 __global__ void __launch_bounds__(kThreads, 4)
-map_rows_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__ out_num, int batch, int max_voxels,
-                ConvGeom g, BitsIndex in, int32_t* __restrict__ nbr, uint32_t* __restrict__ tile_mask,
-                int tiles_per_frame) {
+map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame) {
     pdl_enter();
     const int chunks = (max_voxels + kThreads - 1) / kThreads;
-    const int items = batch * chunks;
-    const int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
+    const int per_job = batch * chunks, items = per_job * jobs.count;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int b = it / chunks;
-        const int o0 = (it - b * chunks) * kThreads;
-        int n = out_num[b];
+        const int j = it / per_job;
+        const MapJob& job = jobs.job[j];
+        const ConvGeom& g = job.g;
+        const BitsIndex in{job.in, max_voxels};
+        const int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
+        const int4* out_coors = reinterpret_cast<const int4*>(job.out_coors);
+        int32_t* nbr = job.nbr;
+        const int b = (it - j * per_job) / chunks;
+        const int o0 = (it - j * per_job - b * chunks) * kThreads;
+        int n = __ldg(job.out_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (o0 >= n) continue;
         const int o = o0 + threadIdx.x;
@@ -569,15 +508,18 @@ map_rows_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__ 
             }
         }
         if ((threadIdx.x & 31) == 0 && bits && live)
-            atomicOr(&tile_mask[(size_t)b * tiles_per_frame + (o >> 7)], bits);
+            atomicOr(&job.tile_mask[(size_t)b * tiles_per_frame + (o >> 7)], bits);
     }
 }
 
 // Fills the map entries of the tiles that hold rows 0 .. out_num[b] with -1, one int4 per thread (a tile's block of
-// kvol x kNbrRun words is contiguous and 16-byte aligned; the padding words are written too).
+// kvol x kNbrRun words is contiguous and 16-byte aligned; the padding words are written too), and zeroes the tails of
+// the call's outputs, whose row counts are known by now.
 __global__ void __launch_bounds__(kThreads)
-nbr_clear_kernel(int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels, int kvol) {
+nbr_clear_kernel(int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels, int kvol,
+                 TailRows tails) {
     pdl_enter();
+    zero_tails(tails);
     const size_t frame_words = nbr_frame_words(kvol, max_voxels);
     const int chunks = (int)((frame_words / 4 + kThreads - 1) / kThreads);
     const int items = batch * chunks;
@@ -751,25 +693,35 @@ int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batc
     return SESSD_OK;
 }
 
-int launch_number_outputs(const BitGrid& out, int batch, int max_voxels, int32_t* chunk_counts, int32_t* out_coors,
-                          int32_t* out_num, int32_t* status, cudaStream_t stream) {
-    SESSD_LAUNCH(count_bits_kernel, persistent_grid(8), kThreads, 0, stream, out, batch, chunk_counts);
-    SESSD_LAUNCH(number_outputs_kernel, persistent_grid(8), kThreads, 0, stream, out, batch, max_voxels, chunk_counts,
-                 reinterpret_cast<int4*>(out_coors), out_num, status);
+// Whether an output level's occupancy can be taken from its input level's grid word by word.
+bool derivable_in_x(const ConvGeom& g) {
+    return (g.K[2] == 3 && g.S[2] == 2 && g.P[2] == 1) || (g.K[2] == 1 && g.S[2] == 1 && g.P[2] == 0);
+}
+
+int launch_number_outputs(const BitGrid& out, const BitGrid* derive_from, const ConvGeom& g, int batch, int max_voxels,
+                          const ScanState& scan, int32_t* out_coors, int32_t* out_num, int32_t* status,
+                          cudaStream_t stream) {
+    const int64_t items = (int64_t)batch * scan_chunks(out.words);
+    const int grid = (int)(items < persistent_grid(8) ? items : persistent_grid(8));
+    if (derive_from)
+        SESSD_LAUNCH(number_outputs_kernel<true>, grid, kThreads, 0, stream, out, *derive_from, g, batch, max_voxels, scan,
+                     reinterpret_cast<int4*>(out_coors), out_num, status);
+    else
+        SESSD_LAUNCH(number_outputs_kernel<false>, grid, kThreads, 0, stream, out, BitGrid{}, g, batch, max_voxels, scan,
+                     reinterpret_cast<int4*>(out_coors), out_num, status);
     return SESSD_OK;
 }
 
-int launch_map_rows(const int32_t* out_coors, const int32_t* out_num, int batch, int max_voxels, const ConvGeom& g,
-                    const BitGrid& in, int32_t* nbr, uint32_t* tile_mask, cudaStream_t stream) {
-    SESSD_LAUNCH(map_rows_kernel, persistent_grid(8), kThreads, 0, stream, reinterpret_cast<const int4*>(out_coors),
-                 out_num, batch, max_voxels, g, BitsIndex{in, max_voxels}, nbr, tile_mask, (max_voxels + 127) / 128);
+int launch_map_rows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream) {
+    if (jobs.count == 0) return SESSD_OK;
+    SESSD_LAUNCH(map_rows_kernel, persistent_grid(8), kThreads, 0, stream, jobs, batch, max_voxels, (max_voxels + 127) / 128);
     return SESSD_OK;
 }
 
 int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch,
                         int max_voxels, const ConvGeom& g, const BitGrid& out, int32_t* nbr, uint32_t* tile_mask,
-                        cudaStream_t stream) {
-    SESSD_LAUNCH(nbr_clear_kernel, persistent_grid(8), kThreads, 0, stream, nbr, out_num, batch, max_voxels, g.kvol);
+                        const TailRows& tails, cudaStream_t stream) {
+    SESSD_LAUNCH(nbr_clear_kernel, persistent_grid(8), kThreads, 0, stream, nbr, out_num, batch, max_voxels, g.kvol, tails);
     SESSD_LAUNCH(scatter_rows_kernel, persistent_grid(8), kThreads, 0, stream, reinterpret_cast<const int4*>(in_coors),
                  in_num, batch, max_voxels, g, BitsIndex{out, max_voxels}, nbr, tile_mask, (max_voxels + 127) / 128);
     return SESSD_OK;

@@ -1,0 +1,111 @@
+// Device pieces of the rulebook that more than one kernel uses: the x-grouped coordinate table and the marking of
+// candidate outputs in an occupancy grid.
+#pragma once
+
+#include "common.cuh"
+
+namespace sessd {
+
+// Integer helpers for the candidate geometry. Strides and candidate spans are 1, 2 or 3; a division by a
+// run-time divisor costs some 25 instructions on the GPU and these kernels are bound by instruction issue,
+// so the common divisors get shifts.
+__device__ __forceinline__ int div_trunc(int a, int s) {   // C division (rounds toward zero)
+    if (s == 1) return a;
+    if (s == 2) return (a + (a < 0 ? 1 : 0)) >> 1;
+    return a / s;
+}
+__device__ __forceinline__ void split_small(int e, int m, int* q, int* r) {   // e = q * m + r, e >= 0
+    if (m == 1) {
+        *q = e;
+        *r = 0;
+    } else if (m == 2) {
+        *q = e >> 1;
+        *r = e & 1;
+    } else {
+        *q = e / m;
+        *r = e - *q * m;
+    }
+}
+
+__device__ __forceinline__ unsigned long long rec_bits(const uint4& r) {
+    return (unsigned long long)r.x | ((unsigned long long)r.y << 32);
+}
+
+// Enters row i of the cell with linear index `key` into a frame's x-grouped table; false when the table is full.
+__device__ __forceinline__ bool bucket_insert(uint32_t* __restrict__ base, uint32_t cap, int shift, uint32_t key, int i) {
+    const uint32_t gkey = key >> 2;
+    uint32_t h = hash_slot(gkey, shift);
+    for (uint32_t probe = 0; probe < cap; ++probe) {
+        uint32_t* bk = base + (size_t)h * 8;
+        uint32_t cur = bk[4];
+        if (cur == kEmpty) cur = atomicCAS(&bk[4], kEmpty, gkey);
+        if (cur == kEmpty || cur == gkey) {
+            atomicMax(reinterpret_cast<int32_t*>(&bk[key & 3u]), i);  // duplicates: highest row wins
+            return true;
+        }
+        h = (h + 1) & (cap - 1);
+    }
+    return false;
+}
+
+// Marks the candidate outputs of the input row at c4 = (b, z, y, x) in frame b's grid: the reference's enumeration
+// (sparseConv3dlayer.cu:339-383). Per axis the row has up to three candidate output positions (one or two for the
+// stride-2 layers); the x candidates of one (z, y) pair are neighbouring bits, mostly of one 64-bit word, so they are
+// tested and set together, and all words are read before any is updated (the reads are independent; most of them find
+// their bits already set by a neighbouring row and nothing is written).
+__device__ __forceinline__ void mark_row(const int4& c4, int b, const ConvGeom& g, const BitGrid& out) {
+    constexpr int MAXS = 3;   // span_max never exceeds the kernel size (<= 3)
+    const int c[3] = {c4.y, c4.z, c4.w};
+    // candidate positions per axis, upper corner downward; pos[j][e] < 0 marks an unusable candidate
+    int pos[3][MAXS];
+    bool in_ok = true;
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+        // C integer division, as in the reference (sparseConv3dlayer.cu:339-348); dilation is 1
+        const int lo = div_trunc(c[j] - (g.K[j] - 1) - 1 + g.S[j] + g.P[j], g.S[j]);
+        const int hi = div_trunc(c[j] + g.P[j], g.S[j]);
+        in_ok = in_ok && c[j] >= 0 && c[j] < g.in_shape[j];
+#pragma unroll
+        for (int e = 0; e < MAXS; ++e) {
+            const int o = hi - e;
+            const int k = c[j] - o * g.S[j] + g.P[j];   // the offset this pair would get (:366)
+            const bool ok = e < g.span_max[j] && e <= hi - lo && o >= 0 && o < g.out_shape[j] && k >= 0 && k < g.K[j];
+            pos[j][e] = ok ? o : -1;
+        }
+    }
+    if (!in_ok) return;
+    // the x candidates as bits of at most two neighbouring words
+    int w0 = -1;
+    unsigned long long bits0 = 0ull, bits1 = 0ull;
+#pragma unroll
+    for (int e = 0; e < MAXS; ++e) {
+        const int ox = pos[2][e];
+        if (ox < 0) continue;
+        if (w0 < 0) w0 = ox >> 6;            // candidates descend, so the first valid one has the highest word
+        if ((ox >> 6) == w0) bits0 |= 1ull << (ox & 63);
+        else bits1 |= 1ull << (ox & 63);     // the word below (spans are at most three cells)
+    }
+    if (w0 < 0) return;
+    unsigned long long* base = reinterpret_cast<unsigned long long*>(out.rec + (size_t)b * out.words);
+    unsigned long long cur0[MAXS * MAXS], cur1[MAXS * MAXS];
+    size_t rec[MAXS * MAXS];
+#pragma unroll
+    for (int ez = 0; ez < MAXS; ++ez)
+#pragma unroll
+        for (int ey = 0; ey < MAXS; ++ey) {
+            const int q = ez * MAXS + ey;
+            const bool ok = pos[0][ez] >= 0 && pos[1][ey] >= 0;
+            rec[q] = ok ? ((size_t)pos[0][ez] * out.Y + pos[1][ey]) * out.xw + w0 : (size_t)-1;
+            // a record is 16 bytes: its bits are the first 8
+            cur0[q] = ok ? *reinterpret_cast<volatile unsigned long long*>(base + 2 * rec[q]) : ~0ull;
+            cur1[q] = (ok && bits1) ? *reinterpret_cast<volatile unsigned long long*>(base + 2 * (rec[q] - 1)) : ~0ull;
+        }
+#pragma unroll
+    for (int q = 0; q < MAXS * MAXS; ++q) {
+        if (rec[q] == (size_t)-1) continue;
+        if ((cur0[q] & bits0) != bits0) atomicOr(base + 2 * rec[q], bits0);
+        if (bits1 && (cur1[q] & bits1) != bits1) atomicOr(base + 2 * (rec[q] - 1), bits1);
+    }
+}
+
+}  // namespace sessd
