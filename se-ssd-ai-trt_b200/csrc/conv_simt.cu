@@ -76,41 +76,52 @@ __device__ __forceinline__ __half from_float<__half>(float v) { return __float2h
 __device__ __forceinline__ float to_float(float v) { return v; }
 __device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 
-__device__ __forceinline__ void store_quad(float* p, const float (&y)[4]) {
-    *reinterpret_cast<float4*>(p) = make_float4(y[0], y[1], y[2], y[3]);
+template <int N>
+__device__ __forceinline__ void store_channels(float* p, const float (&y)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
 }
-__device__ __forceinline__ void store_quad(__half* p, const float (&y)[4]) {
-    uint2 t;
-    reinterpret_cast<__half2*>(&t)[0] = __floats2half2_rn(y[0], y[1]);
-    reinterpret_cast<__half2*>(&t)[1] = __floats2half2_rn(y[2], y[3]);
-    *reinterpret_cast<uint2*>(p) = t;
+template <int N>
+__device__ __forceinline__ void store_channels(__half* p, const float (&y)[N]) {
+    __align__(16) __half2 h[N / 2];
+#pragma unroll
+    for (int i = 0; i < N / 2; ++i) h[i] = __floats2half2_rn(y[2 * i], y[2 * i + 1]);
+    if constexpr (N % 8 == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i += 8) *reinterpret_cast<uint4*>(p + i) = *reinterpret_cast<const uint4*>(h + i / 2);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i += 4) *reinterpret_cast<uint2*>(p + i) = *reinterpret_cast<const uint2*>(h + i / 2);
+    }
 }
 
 // Narrow layers. Little arithmetic per row (4 to 5 of 27 neighbours at full resolution) behind three dependent reads
-// (row count, map entry, input row), so the kernel lives on rows in flight: COUT / 4 threads share a row, a block takes
-// ROWS rows at a time, reads their map entries side by side (coalesced over rows, all in flight), and every thread
-// then walks its row's present neighbours in ascending k. The weights sit in shared memory as floats, 64 bytes of
-// padding per offset so that rows at different offsets meet in fewer banks. One thread per row with the weights read
-// through L1 (four 16-byte loads per channel and thread) took 45 us for the fp32 16->16 layer of a 20,000-point frame,
-// this takes 22 (timed with events around the launch).
+// (row count, map entry, input row), so the kernel lives on rows in flight: COUT / OC threads share a row, a block takes
+// ROWS rows at a time and reads their map entries side by side (coalesced over rows, all in flight, those of its next
+// rows while it works on the present ones); every thread then walks its row's present neighbours in ascending k. The
+// weights sit in shared memory as floats, 16 bytes of padding per offset so that rows at different offsets meet in fewer
+// banks. Four channels per thread for the 16-channel inputs, eight for the 4-channel input, whose rows are small enough
+// to keep six blocks per SM.
 template <typename T, int CIN, int COUT>
 struct Narrow {
-    static constexpr int TPR = COUT / 4;                 // threads per output row
-    static constexpr int ROWS = kThreads / TPR;
+    static constexpr int OC = CIN <= 4 ? 8 : 4;          // output channels per thread
+    static constexpr int TPR = COUT / OC;                // threads per output row
+    static constexpr int ROWS = kThreads / TPR;          // a divisor of the map's 128-row tile
+    static constexpr int BLOCKS = CIN <= 4 ? 5 : 3;      // resident per SM
     static constexpr int KVOL_MAX = 27;                  // 3 x 3 x 3 is the largest kernel the geometry code accepts
-    static constexpr int W_STRIDE = CIN * COUT + 16;     // floats from one offset's weights to the next offset's
+    static constexpr int W_STRIDE = CIN * COUT + 4;      // floats from one offset's weights to the next offset's
     static constexpr int smem(int kvol) { return (kvol * W_STRIDE + KVOL_MAX * ROWS) * 4; }
 };
 
 template <typename T, int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads, 3)
+__global__ void __launch_bounds__(kThreads, (Narrow<T, CIN, COUT>::BLOCKS))
 conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ nbr,
                    const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                    const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
                    T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
     pdl_enter();
     using N = Narrow<T, CIN, COUT>;
-    constexpr int TPR = N::TPR, ROWS = N::ROWS;
+    constexpr int TPR = N::TPR, ROWS = N::ROWS, OC = N::OC;
     constexpr int LOADS = (N::KVOL_MAX * ROWS + kThreads - 1) / kThreads;   // map entries a thread reads
     constexpr int NP = 2;                                                   // input rows in flight per thread
     extern __shared__ __align__(16) float narrow_smem[];
@@ -119,37 +130,42 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
     const int tid = threadIdx.x, r = tid / TPR, cq = tid % TPR;
     const int chunks = (max_voxels + ROWS - 1) / ROWS;
     const int items = batch * chunks;
-    bool first = true;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int b = it / chunks;
-        const int o0 = (it - b * chunks) * ROWS;
-        int n = out_num[b];
-        n = n > max_voxels ? max_voxels : n;
-        if (o0 >= n) continue;   // uniform over the block
-        // the rows' map entries: entry e = (offset e / ROWS, row e % ROWS)
-        const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b, 0, o0);   // ROWS rows of one 128-row tile
-        int entry[LOADS];
+    // the block's next rows: frame, first row, row count of the frame; entry[j] = the map entries this thread reads for
+    // them, entry e = (offset e / ROWS, row e % ROWS)
+    int next = blockIdx.x, b_next = 0, o_next = 0, n_next = 0;
+    int entry[LOADS];
+    auto fetch = [&]() {
+        for (; next < items; next += gridDim.x) {
+            b_next = next / chunks;
+            o_next = (next - b_next * chunks) * ROWS;
+            n_next = __ldg(out_num + b_next);
+            n_next = n_next > max_voxels ? max_voxels : n_next;
+            if (o_next < n_next) break;
+        }
+        if (next >= items) return;
+        const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b_next, 0, o_next);   // ROWS rows of one 128-row tile
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
             const int e = tid + j * kThreads, k = e / ROWS, row = e % ROWS;
-            entry[j] = k < kvol && o0 + row < n ? __ldg(nb + k * kNbrRun + row) : -1;
+            entry[j] = k < kvol && o_next + row < n_next ? __ldg(nb + k * kNbrRun + row) : -1;
         }
-        if (first) {
-            for (int e = tid; e < kvol * CIN * COUT; e += kThreads) {
-                const int k = e / (CIN * COUT);
-                s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(weights[e]);
-            }
-            first = false;
-        } else {
-            __syncthreads();     // the previous rows' entries have been used
-        }
+    };
+    fetch();
+    if (next >= items) return;
+    for (int e = tid; e < kvol * CIN * COUT; e += kThreads) {
+        const int k = e / (CIN * COUT);
+        s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(weights[e]);
+    }
+    while (next < items) {
+        const int b = b_next, o = o_next + r, n = n_next;
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
             const int e = tid + j * kThreads;
             if (e < N::KVOL_MAX * ROWS) s_idx[e] = entry[j];
         }
         __syncthreads();
-        const int o = o0 + r;
+        next += gridDim.x;
+        fetch();
         // the row's present offsets, its threads looking at every TPR-th slot
         uint32_t present = 0;
 #pragma unroll
@@ -159,8 +175,9 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
         }
 #pragma unroll
         for (int d = 1; d < TPR; d <<= 1) present |= __shfl_xor_sync(0xFFFFFFFFu, present, d);
-        if (o >= n) continue;
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+        float acc[OC];
+#pragma unroll
+        for (int c = 0; c < OC; ++c) acc[c] = 0.f;
         const T* in_b = in + (size_t)b * max_voxels * CIN;
         while (present) {
             int ks[NP];
@@ -175,35 +192,43 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
             for (int u = 0; u < NP; ++u) {
                 if (ks[u] < 0) continue;
                 // one neighbour: sum_ci x[ci] * W[k][ci][:] as a fused chain, then added to the row's sum
-                float s[4] = {0.f, 0.f, 0.f, 0.f};
-                const float* wk = s_w + ks[u] * N::W_STRIDE + cq * 4;
+                float s[OC];
+#pragma unroll
+                for (int c = 0; c < OC; ++c) s[c] = 0.f;
+                const float* wk = s_w + ks[u] * N::W_STRIDE + cq * OC;
 #pragma unroll
                 for (int ci = 0; ci < CIN; ++ci) {
-                    const float4 w = *reinterpret_cast<const float4*>(wk + ci * COUT);
-                    s[0] = fmaf(x[u][ci], w.x, s[0]);
-                    s[1] = fmaf(x[u][ci], w.y, s[1]);
-                    s[2] = fmaf(x[u][ci], w.z, s[2]);
-                    s[3] = fmaf(x[u][ci], w.w, s[3]);
+#pragma unroll
+                    for (int c = 0; c < OC; c += 4) {
+                        const float4 w = *reinterpret_cast<const float4*>(wk + ci * COUT + c);
+                        s[c] = fmaf(x[u][ci], w.x, s[c]);
+                        s[c + 1] = fmaf(x[u][ci], w.y, s[c + 1]);
+                        s[c + 2] = fmaf(x[u][ci], w.z, s[c + 2]);
+                        s[c + 3] = fmaf(x[u][ci], w.w, s[c + 3]);
+                    }
                 }
 #pragma unroll
-                for (int c = 0; c < 4; ++c) acc[c] = __fadd_rn(acc[c], s[c]);
+                for (int c = 0; c < OC; ++c) acc[c] = __fadd_rn(acc[c], s[c]);
             }
         }
+        if (o < n) {
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            float v = acc[c];
-            if (scale) v = fmaf(v, __ldg(scale + cq * 4 + c), shift ? __ldg(shift + cq * 4 + c) : 0.f);
-            if (relu) v = v > 0.f ? v : 0.f;
-            acc[c] = v;
-        }
-        store_quad(out + ((size_t)b * max_voxels + o) * COUT + cq * 4, acc);
-        if (dense) {
-            // Fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x).
-            const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + o]);
-            T* d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
+            for (int c = 0; c < OC; ++c) {
+                float v = acc[c];
+                if (scale) v = fmaf(v, __ldg(scale + cq * OC + c), shift ? __ldg(shift + cq * OC + c) : 0.f);
+                if (relu) v = v > 0.f ? v : 0.f;
+                acc[c] = v;
+            }
+            store_channels(out + ((size_t)b * max_voxels + o) * COUT + cq * OC, acc);
+            if (dense) {
+                // Fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x).
+                const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + o]);
+                T* d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
 #pragma unroll
-            for (int c = 0; c < 4; ++c) d[(size_t)(cq * 4 + c) * D * H * W] = from_float<T>(acc[c]);
+                for (int c = 0; c < OC; ++c) d[(size_t)(cq * OC + c) * D * H * W] = from_float<T>(acc[c]);
+            }
         }
+        __syncthreads();     // the rows' entries have been used
     }
 }
 
@@ -282,7 +307,7 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
             configured.fetch_or(bit, std::memory_order_release);
         }
     }
-    SESSD_LAUNCH_NAMED(name.c_str(), (conv_narrow_kernel<T, CIN, COUT>), persistent_grid(4), kThreads, N::smem(c.kvol),
+    SESSD_LAUNCH_NAMED(name.c_str(), (conv_narrow_kernel<T, CIN, COUT>), persistent_grid(N::BLOCKS), kThreads, N::smem(c.kvol),
                        stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.out_num,
                        static_cast<const T*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
                        static_cast<T*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W);
