@@ -373,7 +373,7 @@ int sessd_voxelize_enqueue(const sessd_voxel_params* p, int batch, int max_point
     tails.tensor[2] = w.num_points, tails.row_bytes[2] = 4;
     tails.counts = static_cast<const int32_t*>(inputs[1]);
     tails.batch = batch, tails.max_rows = p->max_voxels;
-    int rc = launch_prepare(fills, tails, stream);
+    int rc = launch_prepare(fills, tails, /*overlap=*/true, stream);
     if (rc) return rc;
     return voxelize_run(p, batch, max_points, out_dtype, static_cast<const float*>(inputs[0]),
                         static_cast<const int32_t*>(inputs[1]), outputs[0], static_cast<int32_t*>(outputs[1]),
@@ -491,7 +491,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     fills.ptr[0] = static_cast<uint4*>(ws.ones_base), fills.n16[0] = ws.ones_bytes / 16, fills.ones[0] = 1;
     fills.ptr[1] = static_cast<uint4*>(ws.zero_base), fills.n16[1] = ws.zero_bytes / 16, fills.ones[1] = 0;
     fills.status = ws.status;
-    rc = launch_prepare(fills, subm ? tails : TailRows{}, stream);
+    rc = launch_prepare(fills, subm ? tails : TailRows{}, w->impl.umma_w == nullptr, stream);
     if (rc) return rc;
     const int32_t* out_num = in_num;
     if (subm && is_subm_333(g)) {
@@ -732,7 +732,7 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         else
             SESSD_CUDA(cudaMemsetAsync(dense, 0, bytes, stream));
     }
-    int rc = launch_prepare(fills, TailRows{}, stream);
+    int rc = launch_prepare(fills, TailRows{}, (int64_t)batch * max_points <= 40000, stream);
     if (rc) return rc;
     // Coordinates first: voxels, the rows of every level, and all neighbour maps; then the convolutions.
     VoxelHooks hooks{};

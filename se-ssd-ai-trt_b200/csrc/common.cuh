@@ -42,9 +42,9 @@ extern thread_local StageRecorder* g_recorder;
         }                                                  \
     } while (0)
 
-// Set while the calling thread enqueues work on one stream only (the default). With several streams in flight the blocks
-// of a waiting kernel would hold registers and shared memory that another stream's running kernel can use: a pipeline
-// of two slots was 9 % slower with overlapping launches, so pipelines with several slots clear this around a run.
+// Cleared for the scope of a pipeline run with several stream slots: the blocks of a waiting kernel would hold registers
+// and shared memory that another slot's running kernel can use (128 frames x 120,000 points on two slots: 40.1 ms with
+// overlapping launches, 37.9 without).
 extern thread_local bool g_overlap_launches;
 
 // Launches `kernel` so that its blocks may start while the stream's previous kernel still runs (programmatic dependent
@@ -52,7 +52,7 @@ extern thread_local bool g_overlap_launches;
 // costs about the same, but a kernel's start-up then overlaps its predecessor's last blocks: of the 40 short kernels
 // of a single 20,000-point frame each used to leave the GPU idle for a microsecond or more.
 template <typename... P, typename... A>
-inline cudaError_t launch_kernel(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A&&... args) {
+inline cudaError_t launch_kernel(bool overlap, void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
@@ -62,21 +62,24 @@ inline cudaError_t launch_kernel(void (*kernel)(P...), int grid, int block, size
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = g_overlap_launches ? 1 : 0;
+    cfg.numAttrs = overlap && g_overlap_launches ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 // Launches `kernel` and accounts for it under `name`; returns from the caller on a launch error.
-#define SESSD_LAUNCH_NAMED(name, kernel, grid, block, smem, stream, ...)      \
-    do {                                                                     \
-        if (::sessd::g_recorder) ::sessd::g_recorder->before(stream);        \
-        const cudaError_t e_launch__ = ::sessd::launch_kernel(kernel, (grid), (block), (smem), (stream), __VA_ARGS__); \
-        ::sessd::g_launches.fetch_add(1, std::memory_order_relaxed);         \
-        if (::sessd::g_recorder) ::sessd::g_recorder->after(name, stream);   \
-        SESSD_CUDA(e_launch__);                                              \
+#define SESSD_LAUNCH_IMPL(overlap, name, kernel, grid, block, smem, stream, ...)                                       \
+    do {                                                                                                               \
+        if (::sessd::g_recorder) ::sessd::g_recorder->before(stream);                                                  \
+        const cudaError_t e_launch__ =                                                                                 \
+            ::sessd::launch_kernel((overlap), kernel, (grid), (block), (smem), (stream), __VA_ARGS__);                 \
+        ::sessd::g_launches.fetch_add(1, std::memory_order_relaxed);                                                   \
+        if (::sessd::g_recorder) ::sessd::g_recorder->after(name, stream);                                             \
+        SESSD_CUDA(e_launch__);                                                                                        \
     } while (0)
+#define SESSD_LAUNCH_NAMED(name, kernel, grid, block, smem, stream, ...) \
+    SESSD_LAUNCH_IMPL(true, name, kernel, grid, block, smem, stream, __VA_ARGS__)
 #define SESSD_LAUNCH(kernel, grid, block, smem, stream, ...) \
-    SESSD_LAUNCH_NAMED(#kernel, kernel, grid, block, smem, stream, __VA_ARGS__)
+    SESSD_LAUNCH_IMPL(true, #kernel, kernel, grid, block, smem, stream, __VA_ARGS__)
 
 // Number of SMs of the current device (cached per device).
 int sm_count();
@@ -277,7 +280,8 @@ struct TailRows {
     const int32_t* counts;
     int batch, max_rows;
 };
-int launch_prepare(const FillRanges& f, const TailRows& t, cudaStream_t stream);
+// overlap: whether the launch may start while the stream's previous kernel runs (see its definition)
+int launch_prepare(const FillRanges& f, const TailRows& t, bool overlap, cudaStream_t stream);
 int launch_fill_zero(void* ptr, size_t bytes, cudaStream_t stream);  // bytes % 16 == 0, ptr 16-byte aligned
 
 // What a one-pass numbering kernel (scan.cuh) keeps in global memory: a word per chunk of kThreads entries and a ticket
