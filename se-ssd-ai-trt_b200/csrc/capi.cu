@@ -89,16 +89,6 @@ struct ConvWorkspace {
     int32_t* nbr;
 };
 
-// Numbering state of one level: a word per chunk and frame and the ticket counter, a multiple of 16 bytes.
-size_t scan_state_bytes(const BitGrid& g, int batch) {
-    return ((size_t)batch * scan_chunks(g.words) + 2) / 2 * 2 * sizeof(unsigned long long);
-}
-ScanState scan_state_at(char* p, const BitGrid& g, int batch) {
-    if (!p) return ScanState{nullptr, nullptr};
-    return ScanState{reinterpret_cast<unsigned long long*>(p),
-                     reinterpret_cast<uint32_t*>(p + scan_state_bytes(g, batch) - sizeof(unsigned long long))};
-}
-
 void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeom& g, int batch, ConvWorkspace* w) {
     *w = ConvWorkspace{};
     w->status = bump.take<int32_t>(kStatusInts);
@@ -122,13 +112,13 @@ void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeo
     const size_t tiles = (size_t)(p->max_voxels + 127) / 128;
     const size_t mask_bytes = (batch * tiles * sizeof(uint32_t) + 15) / 16 * 16;
     const size_t grid_bytes = p->subm ? 0 : (size_t)batch * w->out_bits.words * sizeof(uint4);
-    const size_t scan_bytes = p->subm ? 0 : scan_state_bytes(w->out_bits, batch);
+    const size_t scan_bytes = p->subm ? 0 : scan_state_bytes(w->out_bits.words, batch);
     char* zero = bump.take<char>(grid_bytes + mask_bytes + scan_bytes);
     w->zero_base = zero;
     w->zero_bytes = grid_bytes + mask_bytes + scan_bytes;
     w->out_bits.rec = reinterpret_cast<uint4*>(zero);
     w->tile_mask = reinterpret_cast<uint32_t*>(zero ? zero + grid_bytes : nullptr);
-    if (!p->subm) w->scan = scan_state_at(zero ? zero + grid_bytes + mask_bytes : nullptr, w->out_bits, batch);
+    if (!p->subm) w->scan = scan_state_at(zero ? zero + grid_bytes + mask_bytes : nullptr, w->out_bits.words, batch);
     w->nbr = bump.take<int32_t>((size_t)batch * nbr_frame_words(g.kvol, p->max_voxels));
 }
 
@@ -173,7 +163,6 @@ struct sessd_backbone {
     int nlevels;
     std::vector<int> level_shape;  // 3 ints per level
     std::vector<char> level_has_subm;
-    std::vector<char> level_derived;   // the level's occupancy follows from its input level's grid
     int max_voxels;
 };
 
@@ -181,11 +170,14 @@ namespace {
 
 struct BackboneWorkspace {
     int32_t* status;
-    VoxelWorkspace vox;
+    bool grid0;                      // level 0 has an occupancy grid: voxels numbered in (z, y, x) order (voxel_grid.cu)
+    VoxelGrid vgrid;                 // grid0
+    VoxelWorkspace vox;              // else: voxels in point order,
+    Buckets buckets0;                // and an x-grouped table of their rows
     void* voxel_feat;
     std::vector<int32_t*> coors, num;
-    std::vector<BitGrid> bits;       // occupancy grids of the derived levels (index 0 unused)
-    Buckets buckets0;                // x-grouped table of the voxeliser's rows (level 0)
+    std::vector<BitGrid> bits;       // occupancy grids of the levels
+    std::vector<char> derived;       // the level's occupancy follows from its input level's grid
     void* ones_base;
     size_t ones_bytes;
     std::vector<int32_t*> nbr_subm;
@@ -201,8 +193,26 @@ struct BackboneWorkspace {
 void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_points, BackboneWorkspace* w) {
     const int maxV = bb->max_voxels;
     w->status = bump.take<int32_t>(kStatusInts);
-    voxel_workspace_layout(bump, &bb->vp, batch, max_points, &w->vox);
-    w->vox.status = w->status;
+    w->grid0 = voxel_grid_usable(&bb->vp, max_points, &bb->level_shape[0]);
+    w->vox = VoxelWorkspace{};
+    w->vgrid = VoxelGrid{};
+    w->buckets0 = Buckets{};
+    w->ones_base = nullptr;
+    w->ones_bytes = 0;
+    if (w->grid0) {
+        voxel_grid_layout(bump, &bb->vp, &bb->level_shape[0], batch, max_points, &w->vgrid);
+    } else {
+        voxel_workspace_layout(bump, &bb->vp, batch, max_points, &w->vox);
+        w->vox.status = w->status;
+        if (bb->level_has_subm[0]) {
+            const uint32_t capb = pow2_at_least((uint64_t)maxV);
+            const size_t perb = (size_t)batch * capb * 8;
+            uint32_t* block = bump.take<uint32_t>(perb);
+            w->buckets0 = Buckets{block, capb, 32 - ilog2(capb)};
+            w->ones_base = block;
+            w->ones_bytes = perb * sizeof(uint32_t);
+        }
+    }
     w->voxel_feat = bump.take<char>((size_t)batch * maxV * 4 * esize(bb->dtype));
     w->coors.assign(bb->nlevels, nullptr);
     w->num.assign(bb->nlevels, nullptr);
@@ -214,15 +224,12 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
         w->coors[l] = bump.take<int32_t>((size_t)batch * maxV * 4);
         w->num[l] = bump.take<int32_t>(batch);
     }
-    // the x-grouped table of level 0, reset to 0xFF by one fill (the voxeliser resets its own table)
-    const uint32_t capb = pow2_at_least((uint64_t)maxV);
-    const size_t perb = (size_t)batch * capb * 8;
-    uint32_t* block = bump.take<uint32_t>(perb + 4);
-    w->buckets0 = Buckets{block, capb, 32 - ilog2(capb)};
-    w->ones_base = block;
-    w->ones_bytes = perb * sizeof(uint32_t);
+    w->bits[0] = w->vgrid.grid;
+    w->derived.assign(bb->nlevels, 0);
+    for (auto& L : bb->layers)
+        if (!L.p.subm) w->derived[L.level_out] = (L.level_in > 0 || w->grid0) && derivable_in_x(L.g) ? 1 : 0;
     // What one fill zeroes per call: the occupancy grids that rows mark their outputs in, all tile masks, the numbering
-    // state of the levels and of the voxeliser. A grid that is derived from its input level's grid is written whole.
+    // state of the levels. A grid that is derived from its input level's grid is written whole.
     const size_t tiles = (size_t)(maxV + 127) / 128;
     const size_t mask_words = (batch * tiles + 3) / 4 * 4;
     size_t nmasks = 0;
@@ -232,8 +239,8 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
     w->scan.assign(bb->nlevels, ScanState{nullptr, nullptr});
     for (int l = 1; l < bb->nlevels; ++l) {
         w->bits[l] = bitgrid_shape(&bb->level_shape[3 * l]);
-        zero_bytes += scan_state_bytes(w->bits[l], batch);
-        if (!bb->level_derived[l]) zero_bytes += (size_t)batch * w->bits[l].words * sizeof(uint4);
+        zero_bytes += scan_state_bytes(w->bits[l].words, batch);
+        if (!w->derived[l]) zero_bytes += (size_t)batch * w->bits[l].words * sizeof(uint4);
     }
     char* zero = bump.take<char>(zero_bytes + 16);
     w->zero_base = zero;
@@ -246,8 +253,8 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
     };
     for (int l = 1; l < bb->nlevels; ++l) {
         const size_t bytes = (size_t)batch * w->bits[l].words * sizeof(uint4);
-        w->bits[l].rec = bb->level_derived[l] ? bump.take<uint4>(bytes / sizeof(uint4)) : reinterpret_cast<uint4*>(carve(bytes));
-        w->scan[l] = scan_state_at(carve(scan_state_bytes(w->bits[l], batch)), w->bits[l], batch);
+        w->bits[l].rec = w->derived[l] ? bump.take<uint4>(bytes / sizeof(uint4)) : reinterpret_cast<uint4*>(carve(bytes));
+        w->scan[l] = scan_state_at(carve(scan_state_bytes(w->bits[l].words, batch)), w->bits[l].words, batch);
     }
     for (int l = 0; l < bb->nlevels; ++l)
         if (bb->level_has_subm[l]) w->mask_subm[l] = reinterpret_cast<uint32_t*>(carve(mask_words * sizeof(uint32_t)));
@@ -377,7 +384,7 @@ int sessd_voxelize_enqueue(const sessd_voxel_params* p, int batch, int max_point
     if (rc) return rc;
     return voxelize_run(p, batch, max_points, out_dtype, static_cast<const float*>(inputs[0]),
                         static_cast<const int32_t*>(inputs[1]), outputs[0], static_cast<int32_t*>(outputs[1]),
-                        static_cast<int32_t*>(outputs[2]), w, /*zero_tail=*/true, VoxelHooks{}, stream);
+                        static_cast<int32_t*>(outputs[2]), w, /*zero_tail=*/true, stream);
 }
 
 // ---- sparse convolutions --------------------------------------------------------------------
@@ -633,7 +640,6 @@ int sessd_backbone_create(const sessd_voxel_params* vp, const sessd_conv_params*
     bb->max_voxels = vp->max_voxels;
     bb->nlevels = 1;
     bb->level_has_subm.assign(1, 0);
-    bb->level_derived.assign(1, 0);
     int rc = SESSD_OK;
     int cur_c = vp->voxel_feature_num;
     for (int i = 0; i < nlayers && rc == SESSD_OK; ++i) {
@@ -662,7 +668,6 @@ int sessd_backbone_create(const sessd_voxel_params* vp, const sessd_conv_params*
             L.level_out = bb->nlevels++;
             bb->level_shape.insert(bb->level_shape.end(), {L.g.out_shape[0], L.g.out_shape[1], L.g.out_shape[2]});
             bb->level_has_subm.push_back(0);
-            bb->level_derived.push_back(L.level_in > 0 && derivable_in_x(L.g) ? 1 : 0);
         }
         rc = sessd_conv_weights_create(&L.p, weights[i], scale ? scale[i] : nullptr, shift ? shift[i] : nullptr, 1, dtype,
                                        &L.w);
@@ -713,14 +718,15 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
     if (bump.total() > workspace_bytes) return SESSD_ERR_WORKSPACE;
     if (!workspace_aligned(workspace)) return SESSD_ERR_PARAM;
     const int maxV = bb->max_voxels;
-    // One launch resets everything the call needs: the voxeliser's table and the bucket table (0xFF), the grids, masks
-    // and numbering state (0), the BEV map (0; by cudaMemsetAsync when its size is not a multiple of 16 bytes) and the
+    // One launch resets everything the call needs: the coordinate tables, if any (0xFF), the grids, masks and numbering
+    // state (0), the BEV map (0; by cudaMemsetAsync when its size is not a multiple of 16 bytes) and the
     // status block. keep_status (pipelines): word 0 is left alone, so that it collects the conditions of every group.
     FillRanges fills{};
-    fills.ptr[0] = static_cast<uint4*>(w.ones_base), fills.n16[0] = bb->level_has_subm[0] ? w.ones_bytes / 16 : 0, fills.ones[0] = 1;
+    fills.ptr[0] = static_cast<uint4*>(w.ones_base), fills.n16[0] = w.ones_bytes / 16, fills.ones[0] = 1;
     fills.ptr[1] = static_cast<uint4*>(w.zero_base), fills.n16[1] = w.zero_bytes / 16, fills.ones[1] = 0;
     fills.ptr[2] = static_cast<uint4*>(w.vox.table_base), fills.n16[2] = w.vox.table_bytes / 16, fills.ones[2] = 1;
-    fills.ptr[4] = static_cast<uint4*>(w.vox.zero_base), fills.n16[4] = w.vox.zero_bytes / 16, fills.ones[4] = 0;
+    fills.ptr[4] = static_cast<uint4*>(w.grid0 ? w.vgrid.zero_base : w.vox.zero_base);
+    fills.n16[4] = (w.grid0 ? w.vgrid.zero_bytes : w.vox.zero_bytes) / 16, fills.ones[4] = 0;
     fills.status = w.status;
     fills.status_from = keep_status ? 1 : 0;
     if (bb->has_s2d) {
@@ -735,18 +741,19 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
     int rc = launch_prepare(fills, TailRows{}, (int64_t)batch * max_points <= 40000, stream);
     if (rc) return rc;
     // Coordinates first: voxels, the rows of every level, and all neighbour maps; then the convolutions.
-    VoxelHooks hooks{};
-    if (bb->level_has_subm[0]) hooks.buckets = w.buckets0;
-    const sessd_backbone::Layer* leaving0 = nullptr;   // the strided layer that leaves the voxeliser's level
-    for (auto& L : bb->layers)
-        if (!L.p.subm && L.level_in == 0) leaving0 = &L;
-    if (leaving0) hooks.marks = w.bits[1], hooks.geom = leaving0->g;
-    rc = voxelize_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
-                      static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vox,
-                      /*zero_tail=*/false, hooks, stream);
+    if (w.grid0)
+        rc = voxel_grid_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
+                            static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vgrid, w.status,
+                            stream);
+    else
+        rc = voxelize_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
+                          static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vox,
+                          /*zero_tail=*/false, stream);
     if (rc) return rc;
-    if (bb->level_has_subm[0]) {
-        // the voxeliser's rows: one thread per row looks its 27 neighbours up in the x-grouped table
+    if (bb->level_has_subm[0] && !w.grid0) {
+        // rows in point order: x-grouped table, then one thread per row looks its 27 neighbours up
+        rc = launch_bucket_build(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, w.status, stream);
+        if (rc) return rc;
         rc = launch_nbr_build_subm(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, w.nbr_subm[0],
                                    w.mask_subm[0], stream);
         if (rc) return rc;
@@ -765,21 +772,21 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
     for (size_t i = 0; i < bb->layers.size(); ++i) {
         const sessd_backbone::Layer& L = bb->layers[i];
         if (L.p.subm) {
-            if (L.level_in == 0 || nbr_ready[L.level_in]) continue;
+            if ((L.level_in == 0 && !w.grid0) || nbr_ready[L.level_in]) continue;
             nbr_ready[L.level_in] = 1;
             rc = add_job(L, w.nbr_subm[L.level_in], w.mask_subm[L.level_in]);
             if (rc) return rc;
             continue;
         }
-        const bool derived = bb->level_derived[L.level_out] != 0;
-        if (L.level_in > 0 && !derived) {
+        const bool derived = w.derived[L.level_out] != 0;
+        if (!derived) {
             rc = launch_mark_outputs(w.coors[L.level_in], w.num[L.level_in], batch, maxV, L.g, w.bits[L.level_out], stream);
             if (rc) return rc;
         }
         rc = launch_number_outputs(w.bits[L.level_out], derived ? &w.bits[L.level_in] : nullptr, L.g, batch, maxV,
                                    w.scan[L.level_out], w.coors[L.level_out], w.num[L.level_out], w.status, stream);
         if (rc) return rc;
-        if (L.level_in == 0)   // no grid for the voxeliser's rows: every candidate finds its output row instead
+        if (L.level_in == 0 && !w.grid0)   // no grid for the input rows: every candidate finds its output row instead
             rc = launch_scatter_rows(w.coors[0], w.num[0], w.num[L.level_out], batch, maxV, L.g, w.bits[L.level_out],
                                      w.nbr_layer[i], w.mask_layer[i], TailRows{}, stream);
         else

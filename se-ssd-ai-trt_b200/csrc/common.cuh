@@ -144,14 +144,20 @@ struct Buckets {
     int shift;      // 32 - log2(cap)
 };
 
-// Occupancy grid of one resolution level: frame b owns records [b*words, (b+1)*words); record w covers the 64 cells
-// x = 64*(w % xw) .. +63 of line (z, y) = w / xw and holds {bits lo, bits hi, rows before this word, unused}.
-// Rows are numbered in record order, i.e. in (z, y, x) order.
+// Occupancy grid of one resolution level. Word w of a frame covers the 64 cells x = 64*(w % xw) .. +63 of line
+// (z, y) = w / xw. Rows are numbered in word order, i.e. in (z, y, x) order.
+// One level (top == nullptr): frame b owns records [b*words, (b+1)*words), record w = {bits lo, bits hi, rows before this
+// word, unused} of word w.
+// Two levels (the voxeliser's level, whose words are nearly all empty): top record w / 64 = {bits lo, bits hi, occupied
+// words before, unused} says which of 64 words are occupied, and frame b's records [b*words, ..) hold the occupied words
+// alone, in order: {bits lo, bits hi, rows before this word, w}.
 struct BitGrid {
     uint4* rec;
     int Z, Y, X;
-    int xw;      // records per x line
+    int xw;      // words per x line
     int words;   // records per frame
+    uint4* top;
+    int top_words;   // top records per frame
 };
 inline BitGrid bitgrid_shape(const int shape[3]) {
     BitGrid g{};
@@ -291,6 +297,16 @@ struct ScanState {
     uint32_t* ticket;
 };
 __host__ __device__ inline int scan_chunks(int entries) { return (entries + kThreads - 1) / kThreads; }
+// Bytes of the state of a numbering of `entries` per frame (a multiple of 16; the last word is the ticket counter), and
+// that state at p.
+inline size_t scan_state_bytes(int entries, int batch) {
+    return ((size_t)batch * scan_chunks(entries) + 2) / 2 * 2 * sizeof(unsigned long long);
+}
+inline ScanState scan_state_at(char* p, int entries, int batch) {
+    if (!p) return ScanState{nullptr, nullptr};
+    return ScanState{reinterpret_cast<unsigned long long*>(p),
+                     reinterpret_cast<uint32_t*>(p + scan_state_bytes(entries, batch) - sizeof(unsigned long long))};
+}
 
 // rulebook.cu
 int conv_geom_from_params(const sessd_conv_params* p, ConvGeom* g);
@@ -391,19 +407,29 @@ struct VoxelWorkspace {
     void* table_base;
 };
 void voxel_workspace_layout(Bump& bump, const sessd_voxel_params* p, int batch, int max_points, VoxelWorkspace* w);
-// What the voxeliser can do with a new voxel's row on the way: enter it into the x-grouped table of its level and mark
-// its candidate outputs in the next level's grid.
-struct VoxelHooks {
-    Buckets buckets;      // data == nullptr: none
-    BitGrid marks;        // rec == nullptr: none
-    ConvGeom geom;        // of the strided layer the marks belong to
-};
 // The points of a batch -> rows; the caller has reset the table, the scan's words and the status (and, for a call that
 // returns whole tensors, the rows past each frame's point count). zero_tail: also zero the rows between a frame's voxel
 // count and its point count.
 int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
                  const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelWorkspace& w,
-                 bool zero_tail, const VoxelHooks& hooks, cudaStream_t stream);
+                 bool zero_tail, cudaStream_t stream);
+
+// voxel_grid.cu: rows in (z, y, x) order and an occupancy grid of the level
+struct VoxelGrid {
+    BitGrid grid;
+    uint32_t* pt_key;     // [B][max_points]
+    uint32_t* lists;      // [B][max_points][max_points_per_voxel], by row
+    int32_t* word_num;    // [B] occupied words
+    ScanState scan_words, scan_rows;
+    void* zero_base;      // to be zero before a call
+    size_t zero_bytes;
+};
+bool voxel_grid_usable(const sessd_voxel_params* p, int max_points, const int level_shape[3]);
+void voxel_grid_layout(Bump& bump, const sessd_voxel_params* p, const int level_shape[3], int batch, int max_points,
+                       VoxelGrid* w);
+int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
+                   const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelGrid& w,
+                   int32_t* status, cudaStream_t stream);
 
 struct sessd_conv_weights_impl {
     void* w;        // device, [kvol][Cin][Cout] in dtype

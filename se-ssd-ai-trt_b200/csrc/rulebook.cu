@@ -313,7 +313,6 @@ __device__ __forceinline__ uint32_t even_bits(unsigned long long v) {
 __device__ __forceinline__ unsigned long long derive_word(const BitGrid& in, const BitGrid& out, const ConvGeom& g, int b, int w) {
     const int row = w / out.xw, wx = w - row * out.xw;
     const int z = row / out.Y, y = row - z * out.Y;
-    const unsigned long long* base = reinterpret_cast<const unsigned long long*>(in.rec + (size_t)b * in.words);
     const bool same = g.K[2] == 1;                  // kernel 1, stride 1: the word itself; else kernel 3, stride 2, padding 1
     const int first = same ? wx : 2 * wx;
     unsigned long long before = 0ull, lo = 0ull, hi = 0ull;
@@ -325,11 +324,33 @@ __device__ __forceinline__ unsigned long long derive_word(const BitGrid& in, con
         for (int ky = 0; ky < 3; ++ky) {
             const int iy = y * g.S[1] - g.P[1] + ky;
             if (ky >= g.K[1] || iy < 0 || iy >= in.Y) continue;
-            const unsigned long long* line = base + 2 * ((size_t)iz * in.Y + iy) * in.xw;   // a record is 16 bytes: bits first
-            if (first < in.xw) lo |= __ldg(line + 2 * first);
+            const int line = (iz * in.Y + iy) * in.xw;
+            if (in.top) {
+                // the three words' occupancy first: they are nearly always empty
+                const int w0 = same ? line + first : (first > 0 ? line + first - 1 : line + first);
+                const int w1 = same ? w0 : (first + 1 < in.xw ? line + first + 1 : line + first);
+                const uint4* top = in.top + (size_t)b * in.top_words;
+                const uint4 t0 = __ldg(top + (w0 >> 6));
+                const uint4 t1 = (w1 >> 6) != (w0 >> 6) ? __ldg(top + (w1 >> 6)) : t0;
+                for (int v = w0; v <= w1; ++v) {
+                    const uint4& t = (v >> 6) == (w0 >> 6) ? t0 : t1;
+                    const unsigned long long tb = rec_bits(t), bit = 1ull << (v & 63);
+                    if (!(tb & bit)) continue;
+                    const unsigned long long word =
+                        rec_bits(__ldg(in.rec + (size_t)b * in.words + (int)t.z + __popcll(tb & (bit - 1ull))));
+                    if (v == line + first) lo |= word;
+                    else if (v < line + first) before |= word;
+                    else hi |= word;
+                }
+                continue;
+            }
+            // a record is 16 bytes: bits first
+            const unsigned long long* at =
+                reinterpret_cast<const unsigned long long*>(in.rec + (size_t)b * in.words) + 2 * (size_t)line;
+            if (first < in.xw) lo |= __ldg(at + 2 * first);
             if (!same) {
-                if (first > 0) before |= __ldg(line + 2 * (first - 1));
-                if (first + 1 < in.xw) hi |= __ldg(line + 2 * (first + 1));
+                if (first > 0) before |= __ldg(at + 2 * (first - 1));
+                if (first + 1 < in.xw) hi |= __ldg(at + 2 * (first + 1));
             }
         }
     }
@@ -402,18 +423,45 @@ struct BitsIndex {
     BitGrid g;
     int max_rows;
     struct Probe { uint4 a, b; int w; bool two; };
-    __device__ __forceinline__ void probe(int b, int z, int y, int x0, int count, bool on, Probe* p) const {
+    // Record of word `line + w` of a two-level grid, given its top record; empty (with the right number of rows before
+    // it left open) when the word is.
+    __device__ __forceinline__ uint4 word_record(int b, int word, const uint4& t) const {
+        const unsigned long long tb = rec_bits(t), bit = 1ull << (word & 63);
+        if (!(tb & bit)) return make_uint4(0u, 0u, 0u, 0u);
+        return __ldg(g.rec + (size_t)b * g.words + (int)t.z + __popcll(tb & (bit - 1ull)));
+    }
+    // First reads of a line's probe (the top records of a two-level grid), then the records themselves: kept apart so
+    // that a thread has the reads of several lines in flight.
+    __device__ __forceinline__ void probe_top(int b, int z, int y, int x0, int count, bool on, Probe* p) const {
         p->a = p->b = make_uint4(0u, 0u, 0u, 0u);
         p->two = false;
-        p->w = 0;
+        p->w = -1;
         if (!on) return;
         const int lo = x0 < 0 ? 0 : x0, hi = x0 + count - 1 >= g.X ? g.X - 1 : x0 + count - 1;
         if (lo > hi) return;
-        const uint4* rec = g.rec + (size_t)b * g.words + ((size_t)z * g.Y + y) * g.xw;
         p->w = lo >> 6;
-        p->a = __ldg(rec + p->w);
         p->two = (hi >> 6) != p->w;
-        if (p->two) p->b = __ldg(rec + p->w + 1);
+        if (!g.top) return;
+        const int word = (z * g.Y + y) * g.xw + p->w;
+        p->a = __ldg(g.top + (size_t)b * g.top_words + (word >> 6));
+        if (p->two) p->b = __ldg(g.top + (size_t)b * g.top_words + ((word + 1) >> 6));
+    }
+    __device__ __forceinline__ void probe_rec(int b, int z, int y, Probe* p) const {
+        if (p->w < 0) return;
+        const int word = (z * g.Y + y) * g.xw + p->w;
+        if (g.top) {
+            p->a = word_record(b, word, p->a);
+            if (p->two) p->b = word_record(b, word + 1, p->b);
+            if (rec_bits(p->a) == 0ull) p->a.z = p->b.z;   // the rows of the window are then all of the second word
+        } else {
+            const uint4* rec = g.rec + (size_t)b * g.words + word;
+            p->a = __ldg(rec);
+            if (p->two) p->b = __ldg(rec + 1);
+        }
+    }
+    __device__ __forceinline__ void probe(int b, int z, int y, int x0, int count, bool on, Probe* p) const {
+        probe_top(b, z, y, x0, count, on, p);
+        probe_rec(b, z, y, p);
     }
     __device__ __forceinline__ int finish(const Probe& p, int x) const {
         if (x < 0 || x >= g.X) return -1;
@@ -488,8 +536,11 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
             for (int ky = 0; ky < 3; ++ky) {
                 if (ky >= K1) break;
                 const int y = by + ky;
-                in.probe(b, z, y, bx, K2, z_ok && y >= 0 && y < g.in_shape[1], &pb[ky]);
+                in.probe_top(b, z, y, bx, K2, z_ok && y >= 0 && y < g.in_shape[1], &pb[ky]);
             }
+#pragma unroll
+            for (int ky = 0; ky < 3; ++ky)
+                if (ky < K1) in.probe_rec(b, z, by + ky, &pb[ky]);
 #pragma unroll
             for (int ky = 0; ky < 3; ++ky) {
                 if (ky >= K1) break;

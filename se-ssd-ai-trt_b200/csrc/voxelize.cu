@@ -8,24 +8,18 @@
 //                    (a cascade of atomicMin, so the list content does not depend on timing);
 //   pass 2 (emit)    the owner points (index == smallest index of the slot) are numbered in point order with a
 //                    one-pass scan (scan.cuh); the owner writes coordinates, count and the mean of the listed points,
-//                    summed in ascending index order, and in the fused front end also enters its row into the x-grouped
-//                    table and marks its candidate outputs of the next level.
+//                    summed in ascending index order.
 // Results are therefore bit-reproducible. A single frame is bound by the chain of dependent reads and launches, not by
-// bytes: the passes used to be five to seven launches (reset, insert, count, emit, up to three tails, then table and
-// marks), 46 us for 20,000 points.
+// bytes: as seven launches (reset, insert, count, emit, three tails) 20,000 points took 46 us, as three 19.
+// The fused front end numbers its voxels in space instead where it can (voxel_grid.cu).
 #include "fill.cuh"
 #include "rulebook.cuh"
 #include "scan.cuh"
+#include "voxel.cuh"
 
 namespace sessd {
 
 namespace {
-
-struct VoxGeom {
-    float x_min, x_max, y_min, y_max, z_min, z_max;
-    float vx, vy, vz;
-    int gx, gy, gz;
-};
 
 __global__ void __launch_bounds__(kThreads)
 voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch,
@@ -42,30 +36,12 @@ voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict
         if (p >= n) continue;
         const float4 pt = __ldg(&points[(size_t)b * max_points + p]);
         int slot = -1;
-        // Same tests and fp32 arithmetic as voxelGenerator.cu:363-375.
-        if (pt.x >= g.x_min && pt.x < g.x_max && pt.y >= g.y_min && pt.y < g.y_max && pt.z >= g.z_min &&
-            pt.z < g.z_max) {
-            const int ix = (int)floorf(__fdiv_rn(__fsub_rn(pt.x, g.x_min), g.vx));
-            const int iy = (int)floorf(__fdiv_rn(__fsub_rn(pt.y, g.y_min), g.vy));
-            const int iz = (int)floorf(__fdiv_rn(__fsub_rn(pt.z, g.z_min), g.vz));
-            if (ix >= 0 && ix < g.gx && iy >= 0 && iy < g.gy && iz >= 0 && iz < g.gz) {
-                const uint32_t key = ((uint32_t)iz * g.gy + iy) * g.gx + ix;
-                uint32_t* keys = t.keys + (size_t)b * t.cap;
-                slot = table_insert(keys, t.cap, t.shift, key);
-                if (slot < 0) {
-                    atomicOr(status, SESSD_STATUS_HASH_FULL);
-                } else {
-                    // Keep the max_pts smallest point indices of the cell, ascending: offer the index to
-                    // position 0; whatever loses a position (the larger value) is offered to the next.
-                    uint32_t* list = t.rank + ((size_t)b * t.cap + (uint32_t)slot) * max_pts;
-                    uint32_t carry = (uint32_t)p;
-                    for (int j = 0; j < max_pts; ++j) {
-                        const uint32_t old = atomicMin(&list[j], carry);
-                        if (old == kEmpty) break;
-                        carry = old > carry ? old : carry;
-                    }
-                }
-            }
+        int ix, iy, iz;
+        if (voxel_cell(g, pt, &ix, &iy, &iz)) {
+            const uint32_t key = ((uint32_t)iz * g.gy + iy) * g.gx + ix;
+            slot = table_insert(t.keys + (size_t)b * t.cap, t.cap, t.shift, key);
+            if (slot < 0) atomicOr(status, SESSD_STATUS_HASH_FULL);
+            else list_push(t.rank + ((size_t)b * t.cap + (uint32_t)slot) * max_pts, max_pts, (uint32_t)p);
         }
         pt_slot[(size_t)b * max_points + p] = slot;
     }
@@ -82,24 +58,11 @@ struct VoxelOut {
     int zero_tail;
 };
 
-__device__ __forceinline__ void store_voxel(float* voxels, size_t row, float x, float y, float z, float w) {
-    reinterpret_cast<float4*>(voxels)[row] = make_float4(x, y, z, w);
-}
-__device__ __forceinline__ void store_voxel(__half* voxels, size_t row, float x, float y, float z, float w) {
-    __half2 lo = __floats2half2_rn(x, y), hi = __floats2half2_rn(z, w);
-    uint2 packed;
-    packed.x = *reinterpret_cast<uint32_t*>(&lo);
-    packed.y = *reinterpret_cast<uint32_t*>(&hi);
-    reinterpret_cast<uint2*>(voxels)[row] = packed;
-}
-
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch, int max_points,
-                  VoxGeom g, Table t, int max_pts, const int32_t* __restrict__ pt_slot, ScanState scan, VoxelOut<T> out,
-                  VoxelHooks hooks) {
+                  VoxGeom g, Table t, int max_pts, const int32_t* __restrict__ pt_slot, ScanState scan, VoxelOut<T> out) {
     pdl_enter();
-    constexpr int MAX_PTS = 8;                     // voxel_params_ok
     const int chunks = scan_chunks(max_points), items = batch * chunks;
     for (int ticket = scan_ticket(scan.ticket, items); ticket >= 0; ticket = scan_ticket(scan.ticket, items)) {
         const int c = ticket / batch, b = ticket - c * batch;
@@ -110,14 +73,12 @@ voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__
         const int e = c * kThreads + threadIdx.x;
         const int slot = e < n ? pt_slot[(size_t)b * max_points + e] : -1;
         const size_t gslot = (size_t)b * t.cap + (uint32_t)slot;
-        const uint32_t* list = t.rank + gslot * max_pts;
-        // the cell's points (an ascending list, free places at its end); the first one owns the cell
-        uint32_t pi[MAX_PTS];
+        // the cell's points; the first one owns the cell
+        uint32_t pi[kMaxPointsPerVoxel];
         uint32_t key = 0;
         if (slot >= 0) {
             key = t.keys[gslot];
-#pragma unroll
-            for (int j = 0; j < MAX_PTS; ++j) pi[j] = j < max_pts ? list[j] : kEmpty;
+            list_load(t.rank + gslot * max_pts, max_pts, pi);
         }
         const bool owner = slot >= 0 && pi[0] == (uint32_t)e;
         int end;
@@ -143,39 +104,11 @@ voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__
         const int iz = key / plane, rem = key - iz * plane;
         const int iy = rem / g.gx, ix = rem - iy * g.gx;
         const size_t row = (size_t)b * out.max_voxels + id;
-        const int4 c4 = make_int4(b, iz, iy, ix);
-        reinterpret_cast<int4*>(out.coors)[row] = c4;
-        // Mean as generateAverage_kernel (voxelGenerator.cu:274-296): left-to-right sum over all max_pts slots (unused
-        // slots contribute +0), divided by the clamped count.
-        float4 v[MAX_PTS];
-        int cnt = 0;
-#pragma unroll
-        for (int j = 0; j < MAX_PTS; ++j) {
-            v[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (pi[j] != kEmpty) {
-                v[j] = __ldg(&points[(size_t)b * max_points + pi[j]]);
-                ++cnt;
-            }
-        }
-        float sx = v[0].x, sy = v[0].y, sz = v[0].z, sw = v[0].w;
-#pragma unroll
-        for (int j = 1; j < MAX_PTS; ++j) {
-            if (j >= max_pts) break;
-            sx = __fadd_rn(sx, v[j].x);
-            sy = __fadd_rn(sy, v[j].y);
-            sz = __fadd_rn(sz, v[j].z);
-            sw = __fadd_rn(sw, v[j].w);
-        }
-        const float fn = (float)cnt;
-        store_voxel(out.voxels, row, __fdiv_rn(sx, fn), __fdiv_rn(sy, fn), __fdiv_rn(sz, fn), __fdiv_rn(sw, fn));
+        reinterpret_cast<int4*>(out.coors)[row] = make_int4(b, iz, iy, ix);
+        int cnt;
+        const float4 m = voxel_mean(points + (size_t)b * max_points, max_pts, pi, &cnt);
+        store_voxel(out.voxels, row, m.x, m.y, m.z, m.w);
         out.num_points[row] = cnt;
-        if (hooks.buckets.data) {
-            // (the fused front end's layers share the voxeliser's grid in y and x, so the cell's key is the layer's)
-            if (!bucket_insert(hooks.buckets.data + (size_t)b * hooks.buckets.cap * 8, hooks.buckets.cap, hooks.buckets.shift,
-                               key, id))
-                atomicOr(out.status, SESSD_STATUS_HASH_FULL);
-        }
-        if (hooks.marks.rec) mark_row(c4, b, hooks.geom, hooks.marks);
     }
 }
 
@@ -226,19 +159,17 @@ void voxel_workspace_layout(Bump& bump, const sessd_voxel_params* p, int batch, 
     w->table.rank_stride = p->max_points_per_voxel;
     w->table.key_stride = 1;
     w->pt_slot = bump.take<int32_t>((size_t)batch * max_points);
-    const size_t words = ((size_t)batch * scan_chunks(max_points) + 1 + 1) / 2 * 2;   // one for the ticket; 16-byte multiple
-    w->scan.state = bump.take<unsigned long long>(words);
-    w->scan.ticket = reinterpret_cast<uint32_t*>(w->scan.state ? w->scan.state + (words - 1) : nullptr);
-    w->zero_base = w->scan.state;
-    w->zero_bytes = words * sizeof(unsigned long long);
+    w->zero_bytes = scan_state_bytes(max_points, batch);
+    char* zero = bump.take<char>(w->zero_bytes);
+    w->zero_base = zero;
+    w->scan = scan_state_at(zero, max_points, batch);
     w->num_points = bump.take<int32_t>((size_t)batch * p->max_voxels);
 }
 
 int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
                  const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelWorkspace& w,
-                 bool zero_tail, const VoxelHooks& hooks, cudaStream_t stream) {
-    VoxGeom g{p->x_min, p->x_max, p->y_min, p->y_max, p->z_min, p->z_max, p->voxel_x, p->voxel_y, p->voxel_z,
-              p->grid_x, p->grid_y, p->grid_z};
+                 bool zero_tail, cudaStream_t stream) {
+    const VoxGeom g = voxel_geom(*p);
     const float4* pts = reinterpret_cast<const float4*>(points);
     const int64_t items = (int64_t)batch * scan_chunks(max_points);
     const int grid = (int)(items < persistent_grid(8) ? items : persistent_grid(8));
@@ -247,11 +178,11 @@ int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out
     if (out_dtype == SESSD_F32) {
         VoxelOut<float> o{static_cast<float*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
         SESSD_LAUNCH(voxel_emit_kernel<float>, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                     p->max_points_per_voxel, w.pt_slot, w.scan, o, hooks);
+                     p->max_points_per_voxel, w.pt_slot, w.scan, o);
     } else {
         VoxelOut<__half> o{static_cast<__half*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
         SESSD_LAUNCH(voxel_emit_kernel<__half>, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                     p->max_points_per_voxel, w.pt_slot, w.scan, o, hooks);
+                     p->max_points_per_voxel, w.pt_slot, w.scan, o);
     }
     return SESSD_OK;
 }
