@@ -46,10 +46,10 @@ void StageRecorder::after(const char* name, cudaStream_t s) {
     names.push_back(name);
 }
 
-int launch_rulebook_export(const int32_t* nbr, const int32_t* out_num, int frame, int kvol, int max_voxels,
-                           int32_t* pairs, uint32_t* pair_num, cudaStream_t stream);
-int launch_count_pairs(const int32_t* nbr, const int32_t* out_num, int batch, int max_voxels, int kvol,
-                       unsigned long long* total, cudaStream_t stream);
+int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* order, const int32_t* out_num,
+                           int frame, int kvol, int max_voxels, int32_t* pairs, uint32_t* pair_num, cudaStream_t stream);
+int launch_count_pairs(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* out_num, int batch, int max_voxels,
+                       int kvol, unsigned long long* total, cudaStream_t stream);
 
 namespace {
 
@@ -75,12 +75,18 @@ bool is_subm_333(const ConvGeom& g) {
     return g.kvol == 27 && g.K[0] == 3 && g.K[1] == 3 && g.K[2] == 3 && g.P[0] == 1 && g.P[1] == 1 && g.P[2] == 1;
 }
 
+// Whether the rows of a map are ordered by their neighbours. Pays where tiles would otherwise need most of many offsets;
+// for the three offsets of the last layer there is little to leave out, and rows in spatial order make its scatter into
+// the BEV map coalesced.
+bool sorted_map(const ConvGeom& g) { return g.kvol > 9; }
+
 struct ConvWorkspace {
     int32_t* status;
     void* ones_base;      // tables: every word 0xFFFFFFFF before use
     size_t ones_bytes;
-    Buckets buckets;      // submanifold 3x3x3: x-grouped table of the input coordinates
+    Buckets buckets;      // submanifold 3x3x3 and strided: x-grouped table of the input coordinates
     Table in_table;       // other submanifold geometries: flat table of the input coordinates
+    int32_t* order;       // output row at each position of the map (null: positions are rows)
     BitGrid out_bits;     // strided: occupancy grid of the output level
     void* zero_base;      // occupancy grid + tile masks + numbering state: zero before use
     size_t zero_bytes;
@@ -95,19 +101,20 @@ void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeo
     const uint32_t cap = pow2_at_least(2ull * (uint64_t)p->max_voxels);
     const size_t per = (size_t)batch * cap;
     const int shift = 32 - ilog2(cap);
-    if (p->subm && is_subm_333(g)) {
+    if (!p->subm || is_subm_333(g)) {
         const uint32_t capb = pow2_at_least((uint64_t)p->max_voxels);
         w->buckets = Buckets{bump.take<uint32_t>((size_t)batch * capb * 8), capb, 32 - ilog2(capb)};
         w->ones_base = w->buckets.data;
         w->ones_bytes = (size_t)batch * capb * 8 * sizeof(uint32_t);
-    } else if (p->subm) {
+        w->order = bump.take<int32_t>((size_t)batch * p->max_voxels);
+        if (!sorted_map(g)) w->order = nullptr;
+    } else {
         uint32_t* block = bump.take<uint32_t>(per * 2);
         w->in_table = Table{block, nullptr, reinterpret_cast<int32_t*>(block ? block + per : nullptr), cap, shift, 1, 1};
         w->ones_base = block;
         w->ones_bytes = per * 2 * sizeof(uint32_t);
-    } else {
-        w->out_bits = bitgrid_shape(g.out_shape);
     }
+    if (!p->subm) w->out_bits = bitgrid_shape(g.out_shape);
     // occupancy grid and numbering state (strided layers) and tile masks in one block, reset by the call's first launch
     const size_t tiles = (size_t)(p->max_voxels + 127) / 128;
     const size_t mask_bytes = (batch * tiles * sizeof(uint32_t) + 15) / 16 * 16;
@@ -186,6 +193,7 @@ struct BackboneWorkspace {
     void* zero_base;
     size_t zero_bytes;
     std::vector<int32_t*> nbr_layer;      // maps of the strided layers (indexed by layer)
+    std::vector<int32_t*> order_subm, order_layer;   // output rows at the maps' positions (null: positions are rows)
     std::vector<ScanState> scan;          // numbering state of the derived levels
     std::vector<void*> feat;
 };
@@ -204,14 +212,12 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
     } else {
         voxel_workspace_layout(bump, &bb->vp, batch, max_points, &w->vox);
         w->vox.status = w->status;
-        if (bb->level_has_subm[0]) {
-            const uint32_t capb = pow2_at_least((uint64_t)maxV);
-            const size_t perb = (size_t)batch * capb * 8;
-            uint32_t* block = bump.take<uint32_t>(perb);
-            w->buckets0 = Buckets{block, capb, 32 - ilog2(capb)};
-            w->ones_base = block;
-            w->ones_bytes = perb * sizeof(uint32_t);
-        }
+        const uint32_t capb = pow2_at_least((uint64_t)maxV);
+        const size_t perb = (size_t)batch * capb * 8;
+        uint32_t* block = bump.take<uint32_t>(perb);
+        w->buckets0 = Buckets{block, capb, 32 - ilog2(capb)};
+        w->ones_base = block;
+        w->ones_bytes = perb * sizeof(uint32_t);
     }
     w->voxel_feat = bump.take<char>((size_t)batch * maxV * 4 * esize(bb->dtype));
     w->coors.assign(bb->nlevels, nullptr);
@@ -227,15 +233,12 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
     w->bits[0] = w->vgrid.grid;
     w->derived.assign(bb->nlevels, 0);
     for (auto& L : bb->layers)
-        if (!L.p.subm) w->derived[L.level_out] = (L.level_in > 0 || w->grid0) && derivable_in_x(L.g) ? 1 : 0;
-    // What one fill zeroes per call: the occupancy grids that rows mark their outputs in, all tile masks, the numbering
-    // state of the levels. A grid that is derived from its input level's grid is written whole.
+        if (!L.p.subm) w->derived[L.level_out] = L.level_in > 0 && derivable_in_x(L.g) ? 1 : 0;
+    // What one fill zeroes per call: the occupancy grids that rows mark their outputs in and the numbering state of the
+    // levels. A grid that is derived from its input level's grid is written whole.
     const size_t tiles = (size_t)(maxV + 127) / 128;
-    const size_t mask_words = (batch * tiles + 3) / 4 * 4;
-    size_t nmasks = 0;
-    for (int l = 0; l < bb->nlevels; ++l) nmasks += bb->level_has_subm[l] ? 1 : 0;
-    for (auto& L : bb->layers) nmasks += L.p.subm ? 0 : 1;
-    size_t zero_bytes = mask_words * nmasks * sizeof(uint32_t);
+    const size_t mask_words = batch * tiles;
+    size_t zero_bytes = 0;
     w->scan.assign(bb->nlevels, ScanState{nullptr, nullptr});
     for (int l = 1; l < bb->nlevels; ++l) {
         w->bits[l] = bitgrid_shape(&bb->level_shape[3 * l]);
@@ -256,16 +259,23 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
         w->bits[l].rec = w->derived[l] ? bump.take<uint4>(bytes / sizeof(uint4)) : reinterpret_cast<uint4*>(carve(bytes));
         w->scan[l] = scan_state_at(carve(scan_state_bytes(w->bits[l].words, batch)), w->bits[l].words, batch);
     }
-    for (int l = 0; l < bb->nlevels; ++l)
-        if (bb->level_has_subm[l]) w->mask_subm[l] = reinterpret_cast<uint32_t*>(carve(mask_words * sizeof(uint32_t)));
-    for (size_t i = 0; i < bb->layers.size(); ++i)
-        if (!bb->layers[i].p.subm) w->mask_layer[i] = reinterpret_cast<uint32_t*>(carve(mask_words * sizeof(uint32_t)));
-    for (int l = 0; l < bb->nlevels; ++l)
-        if (bb->level_has_subm[l]) w->nbr_subm[l] = bump.take<int32_t>((size_t)batch * nbr_frame_words(27, maxV));
     w->nbr_layer.assign(bb->layers.size(), nullptr);
-    for (size_t i = 0; i < bb->layers.size(); ++i)
-        if (!bb->layers[i].p.subm)
-            w->nbr_layer[i] = bump.take<int32_t>((size_t)batch * nbr_frame_words(bb->layers[i].g.kvol, maxV));
+    w->order_subm.assign(bb->nlevels, nullptr);
+    w->order_layer.assign(bb->layers.size(), nullptr);
+    const size_t rows = (size_t)batch * maxV;
+    for (int l = 0; l < bb->nlevels; ++l) {
+        if (!bb->level_has_subm[l]) continue;
+        w->mask_subm[l] = bump.take<uint32_t>(mask_words);
+        w->nbr_subm[l] = bump.take<int32_t>((size_t)batch * nbr_frame_words(27, maxV));
+        w->order_subm[l] = bump.take<int32_t>(rows);
+    }
+    for (size_t i = 0; i < bb->layers.size(); ++i) {
+        const sessd_backbone::Layer& L = bb->layers[i];
+        if (L.p.subm) continue;
+        w->mask_layer[i] = bump.take<uint32_t>(mask_words);
+        w->nbr_layer[i] = bump.take<int32_t>((size_t)batch * nbr_frame_words(L.g.kvol, maxV));
+        if (sorted_map(L.g)) w->order_layer[i] = bump.take<int32_t>(rows);
+    }
     w->feat.assign(bb->layers.size(), nullptr);
     for (size_t i = 0; i < bb->layers.size(); ++i)
         w->feat[i] = bump.take<char>((size_t)batch * maxV * bb->layers[i].p.out_channel * esize(bb->dtype));
@@ -501,34 +511,36 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     rc = launch_prepare(fills, subm ? tails : TailRows{}, w->impl.umma_w == nullptr, stream);
     if (rc) return rc;
     const int32_t* out_num = in_num;
-    if (subm && is_subm_333(g)) {
-        rc = launch_bucket_build(in_coors, in_num, batch, maxV, g.in_shape, ws.buckets, ws.status, stream);
+    if (!subm) out_num = static_cast<const int32_t*>(outputs[2]);
+    if (!subm || is_subm_333(g)) {
+        rc = launch_bucket_build(in_coors, in_num, batch, maxV, g.in_shape, ws.buckets, subm ? nullptr : &g, ws.out_bits,
+                                 ws.status, stream);
         if (rc) return rc;
-        rc = launch_nbr_build_subm(in_coors, in_num, batch, maxV, g.in_shape, ws.buckets, ws.nbr, ws.tile_mask, stream);
+        if (!subm) {
+            rc = launch_number_outputs(ws.out_bits, nullptr, g, batch, maxV, ws.scan, static_cast<int32_t*>(outputs[1]),
+                                       static_cast<int32_t*>(outputs[2]), ws.status, stream);
+            if (rc) return rc;
+        }
+        MapJobs jobs{};
+        jobs.count = 1;
+        jobs.job[0] = make_map_job(g, subm ? in_coors : static_cast<const int32_t*>(outputs[1]), out_num, p->in_channel, ws.nbr,
+                                   ws.tile_mask, ws.order);
+        jobs.job[0].table = ws.buckets;
+        rc = launch_map_rows(jobs, batch, maxV, subm ? TailRows{} : tails, stream);
         if (rc) return rc;
-    } else if (subm) {
+    } else {
         rc = launch_table_build(in_coors, in_num, batch, maxV, g.in_shape, ws.in_table, ws.status, stream);
         if (rc) return rc;
         rc = launch_nbr_build(in_coors, in_num, batch, maxV, g, ws.in_table, ws.nbr, stream);
         if (rc) return rc;
         rc = launch_tile_mask(ws.nbr, in_num, batch, maxV, g.kvol, ws.tile_mask, stream);
         if (rc) return rc;
-    } else {
-        rc = launch_mark_outputs(in_coors, in_num, batch, maxV, g, ws.out_bits, stream);
-        if (rc) return rc;
-        rc = launch_number_outputs(ws.out_bits, nullptr, g, batch, maxV, ws.scan, static_cast<int32_t*>(outputs[1]),
-                                   static_cast<int32_t*>(outputs[2]), ws.status, stream);
-        if (rc) return rc;
-        out_num = static_cast<const int32_t*>(outputs[2]);
-        // the caller's input rows come in any order and have no grid of their own: input-stationary map
-        rc = launch_scatter_rows(in_coors, in_num, out_num, batch, maxV, g, ws.out_bits, ws.nbr, ws.tile_mask, tails,
-                                 stream);
-        if (rc) return rc;
     }
     ConvLaunch c{};
     c.in = inputs[0];
     c.out = outputs[0];
     c.nbr = ws.nbr;
+    c.order = ws.order;
     c.tile_mask = ws.tile_mask;
     c.out_num = out_num;
     c.weights = w->impl.w;
@@ -571,8 +583,8 @@ int sessd_conv_rulebook_export(const sessd_conv_params* p, int batch, int frame,
     Bump bump(workspace);
     ConvWorkspace ws;
     conv_workspace_layout(bump, p, g, batch, &ws);
-    return launch_rulebook_export(ws.nbr, static_cast<const int32_t*>(out_voxel_num), frame, g.kvol, p->max_voxels,
-                                  indice_pairs, indice_num, static_cast<cudaStream_t>(stream));
+    return launch_rulebook_export(ws.nbr, ws.tile_mask, ws.order, static_cast<const int32_t*>(out_voxel_num), frame, g.kvol,
+                                  p->max_voxels, indice_pairs, indice_num, static_cast<cudaStream_t>(stream));
 }
 
 // ---- sparse -> dense -------------------------------------------------------------------------
@@ -741,60 +753,67 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
     int rc = launch_prepare(fills, TailRows{}, (int64_t)batch * max_points <= 40000, stream);
     if (rc) return rc;
     // Coordinates first: voxels, the rows of every level, and all neighbour maps; then the convolutions.
+    const sessd_backbone::Layer* leaving0 = nullptr;   // the strided layer that leaves the voxeliser's level, if it can be
+    for (auto& L : bb->layers)                         // marked by the voxeliser
+        if (!L.p.subm && L.level_in == 0 && w.grid0 && derivable_in_x(L.g)) leaving0 = &L;
     if (w.grid0)
         rc = voxel_grid_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
-                            static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vgrid, w.status,
-                            stream);
+                            static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vgrid,
+                            leaving0 ? leaving0->g : ConvGeom{}, leaving0 ? w.bits[1] : BitGrid{}, w.status, stream);
     else
         rc = voxelize_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
                           static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vox,
                           /*zero_tail=*/false, stream);
     if (rc) return rc;
-    if (bb->level_has_subm[0] && !w.grid0) {
-        // rows in point order: x-grouped table, then one thread per row looks its 27 neighbours up
-        rc = launch_bucket_build(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, w.status, stream);
-        if (rc) return rc;
-        rc = launch_nbr_build_subm(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, w.nbr_subm[0],
-                                   w.mask_subm[0], stream);
+    // Maps by the kind of their index: [0] occupancy grids, [1] the table of level-0 rows in point order.
+    MapJobs jobs[2] = {};
+    if (!w.grid0) {
+        rc = launch_bucket_build(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, nullptr, BitGrid{}, w.status,
+                                 stream);
         if (rc) return rc;
     }
-    MapJobs jobs{};
-    auto add_job = [&](const sessd_backbone::Layer& L, int32_t* nbr, uint32_t* mask) {
-        if (jobs.count == MapJobs::kMax) {
-            const int rc_jobs = launch_map_rows(jobs, batch, maxV, stream);
+    auto add_job = [&](const sessd_backbone::Layer& L, int cin, int32_t* nbr, uint32_t* mask, int32_t* order) {
+        const bool table = L.level_in == 0 && !w.grid0;
+        MapJobs& js = jobs[table ? 1 : 0];
+        if (js.count == MapJobs::kMax) {
+            const int rc_jobs = launch_map_rows(js, batch, maxV, TailRows{}, stream);
             if (rc_jobs) return rc_jobs;
-            jobs.count = 0;
+            js.count = 0;
         }
-        jobs.job[jobs.count++] = MapJob{w.coors[L.level_out], w.num[L.level_out], L.g, w.bits[L.level_in], nbr, mask};
+        MapJob j = make_map_job(L.g, w.coors[L.level_out], w.num[L.level_out], cin, nbr, mask, order);
+        j.in = w.bits[L.level_in];
+        if (table) j.table = w.buckets0;
+        js.job[js.count++] = j;
         return (int)SESSD_OK;
     };
     std::vector<char> nbr_ready(bb->nlevels, 0);
     for (size_t i = 0; i < bb->layers.size(); ++i) {
         const sessd_backbone::Layer& L = bb->layers[i];
         if (L.p.subm) {
-            if ((L.level_in == 0 && !w.grid0) || nbr_ready[L.level_in]) continue;
+            if (nbr_ready[L.level_in]) continue;
             nbr_ready[L.level_in] = 1;
-            rc = add_job(L, w.nbr_subm[L.level_in], w.mask_subm[L.level_in]);
+            int cin = L.p.in_channel;
+            for (auto& other : bb->layers)
+                if (other.p.subm && other.level_in == L.level_in && other.p.in_channel < cin) cin = other.p.in_channel;
+            rc = add_job(L, cin, w.nbr_subm[L.level_in], w.mask_subm[L.level_in], w.order_subm[L.level_in]);
             if (rc) return rc;
             continue;
         }
         const bool derived = w.derived[L.level_out] != 0;
-        if (!derived) {
+        if (!derived && &L != leaving0) {
             rc = launch_mark_outputs(w.coors[L.level_in], w.num[L.level_in], batch, maxV, L.g, w.bits[L.level_out], stream);
             if (rc) return rc;
         }
         rc = launch_number_outputs(w.bits[L.level_out], derived ? &w.bits[L.level_in] : nullptr, L.g, batch, maxV,
                                    w.scan[L.level_out], w.coors[L.level_out], w.num[L.level_out], w.status, stream);
         if (rc) return rc;
-        if (L.level_in == 0 && !w.grid0)   // no grid for the input rows: every candidate finds its output row instead
-            rc = launch_scatter_rows(w.coors[0], w.num[0], w.num[L.level_out], batch, maxV, L.g, w.bits[L.level_out],
-                                     w.nbr_layer[i], w.mask_layer[i], TailRows{}, stream);
-        else
-            rc = add_job(L, w.nbr_layer[i], w.mask_layer[i]);
+        rc = add_job(L, L.p.in_channel, w.nbr_layer[i], w.mask_layer[i], w.order_layer[i]);
         if (rc) return rc;
     }
-    rc = launch_map_rows(jobs, batch, maxV, stream);
-    if (rc) return rc;
+    for (const MapJobs& js : jobs) {
+        rc = launch_map_rows(js, batch, maxV, TailRows{}, stream);
+        if (rc) return rc;
+    }
     const void* cur = w.voxel_feat;
     for (size_t i = 0; i < bb->layers.size(); ++i) {
         const sessd_backbone::Layer& L = bb->layers[i];
@@ -802,13 +821,14 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         const uint32_t* tile_mask = L.p.subm ? w.mask_subm[L.level_in] : w.mask_layer[i];
         if (count_pairs) {
             auto* counters = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(w.status) + 256);
-            rc = launch_count_pairs(nbr, w.num[L.level_out], batch, maxV, L.g.kvol, counters + i, stream);
+            rc = launch_count_pairs(nbr, tile_mask, w.num[L.level_out], batch, maxV, L.g.kvol, counters + i, stream);
             if (rc) return rc;
         }
         ConvLaunch c{};
         c.in = cur;
         c.out = w.feat[i];
         c.nbr = nbr;
+        c.order = L.p.subm ? w.order_subm[L.level_in] : w.order_layer[i];
         c.tile_mask = tile_mask;
         c.out_num = w.num[L.level_out];
         c.weights = L.w->impl.w;

@@ -322,40 +322,39 @@ bool derivable_in_x(const ConvGeom& g);
 int launch_number_outputs(const BitGrid& out, const BitGrid* derive_from, const ConvGeom& g, int batch, int max_voxels,
                           const ScanState& scan, int32_t* out_coors, int32_t* out_num, int32_t* status,
                           cudaStream_t stream);
-// Neighbour maps + tile masks of layers (any kernel up to 3x3x3, any stride) whose input level has an occupancy grid:
-// output-stationary, one thread per output row; one launch for up to MapJobs::kMax layers.
+int launch_bucket_build(const int32_t* coors, const int32_t* voxel_num, int batch, int max_voxels, const int shape[3],
+                        const Buckets& t, const ConvGeom* mark, const BitGrid& out, int32_t* status, cudaStream_t stream);
+// map_rows.cu: neighbour maps + tile masks of layers (any kernel up to 3x3x3, any stride) whose input level has an
+// occupancy grid (`in`) or an x-grouped table (`table`), the same kind for all jobs; one launch for up to MapJobs::kMax.
 struct MapJob {
     const int32_t* out_coors;
     const int32_t* out_num;
     ConvGeom g;
     BitGrid in;
+    Buckets table;
     int32_t* nbr;
     uint32_t* tile_mask;
+    int32_t* order;      // [B][max_voxels] output row at each position of the map, or null: positions are rows
+    int group;           // offsets that the map's consumers fetch together
+    uint32_t plane[6];   // offsets of the kernel's outer planes: first and last in z, y, x
 };
 struct MapJobs {
     static constexpr int kMax = 8;
     MapJob job[kMax];
     int count;
 };
-int launch_map_rows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream);
-// The same for a strided layer whose input rows have no grid (voxeliser rows, caller's rows): input-stationary,
-// every candidate of every input row finds its output row in the numbered output grid. Clears the map first, and with
-// the same launch the tails of the call's outputs.
-int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch,
-                        int max_voxels, const ConvGeom& g, const BitGrid& out, int32_t* nbr, uint32_t* tile_mask,
-                        const TailRows& tails, cudaStream_t stream);
-int launch_bucket_build(const int32_t* coors, const int32_t* voxel_num, int batch, int max_voxels, const int shape[3],
-                        const Buckets& t, int32_t* status, cudaStream_t stream);
-// 3x3x3 / stride 1 / pad 1 neighbour map from a bucket table, plus the per-128-row-tile offset masks.
-int launch_nbr_build_subm(const int32_t* coors, const int32_t* voxel_num, int batch, int max_voxels, const int shape[3],
-                          const Buckets& t, int32_t* nbr, uint32_t* tile_mask, cudaStream_t stream);
+// Everything of a job but its index; cin: input channels of the layers that read the map (the smallest).
+MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* out_num, int cin, int32_t* nbr,
+                    uint32_t* tile_mask, int32_t* order);
+int launch_map_rows(const MapJobs& jobs, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream);
 int launch_tile_mask(const int32_t* nbr, const int32_t* out_num, int batch, int max_voxels, int kvol,
                      uint32_t* tile_mask, cudaStream_t stream);
 // conv_simt.cu
 struct ConvLaunch {
     const void* in;        // [B][max_voxels][Cin]
     void* out;             // [B][max_voxels][Cout]
-    const int32_t* nbr;    // neighbour map, tile-major (nbr_index)
+    const int32_t* nbr;    // neighbour map, tile-major (nbr_index); only the offsets that tile_mask names are written
+    const int32_t* order;  // [B][max_voxels] output row at each position of the map, or null: positions are rows
     const int32_t* out_num;// [B]
     const uint32_t* tile_mask; // [B][ceil(max_voxels/128)]: bit k set when offset k has a neighbour in the tile
     const void* weights;   // [kvol][Cin][Cout] in the feature dtype
@@ -424,12 +423,13 @@ struct VoxelGrid {
     void* zero_base;      // to be zero before a call
     size_t zero_bytes;
 };
+// marks (rec != nullptr): the grid of the next level, in which the outputs of the strided layer `geom` are marked
 bool voxel_grid_usable(const sessd_voxel_params* p, int max_points, const int level_shape[3]);
 void voxel_grid_layout(Bump& bump, const sessd_voxel_params* p, const int level_shape[3], int batch, int max_points,
                        VoxelGrid* w);
 int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
                    const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelGrid& w,
-                   int32_t* status, cudaStream_t stream);
+                   const ConvGeom& geom, const BitGrid& marks, int32_t* status, cudaStream_t stream);
 
 struct sessd_conv_weights_impl {
     void* w;        // device, [kvol][Cin][Cout] in dtype

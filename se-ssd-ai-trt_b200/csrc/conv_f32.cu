@@ -54,6 +54,7 @@ struct F32Args {
     const float* in;
     float* out;
     const int32_t* nbr;
+    const int32_t* order;
     const uint32_t* tile_mask;
     const int32_t* out_num;
     const float *weights, *scale, *shift;
@@ -275,12 +276,14 @@ __device__ __forceinline__ void f32_run(F32Shared<CIN, COUT>& s, const F32Args& 
         for (int i = 0; i < RT; ++i) {
             const int r = rg * RT + i;
             if (r >= rows) continue;
-            float* dst = a.out + ((size_t)b * a.max_voxels + row0 + r) * COUT;
+            const size_t pos = (size_t)b * a.max_voxels + row0 + r;
+            const size_t row = a.order ? (size_t)b * a.max_voxels + __ldg(a.order + pos) : pos;
+            float* dst = a.out + row * COUT;
             float* d = nullptr;
             const size_t plane = (size_t)a.D * a.H * a.W;
             if (a.dense) {
                 // fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x)
-                const int4 c4 = __ldg(&a.out_coors[(size_t)b * a.max_voxels + row0 + r]);
+                const int4 c4 = __ldg(&a.out_coors[row]);
                 d = a.dense + (size_t)b * COUT * plane + ((size_t)c4.y * a.H + c4.z) * a.W + c4.w;
             }
 #pragma unroll
@@ -351,7 +354,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
         SESSD_CUDA(cudaFuncSetAttribute(conv_f32_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured.fetch_or(bit, std::memory_order_release);
     }
-    const F32Args a{static_cast<const float*>(c.in), static_cast<float*>(c.out), c.nbr, c.tile_mask, c.out_num,
+    const F32Args a{static_cast<const float*>(c.in), static_cast<float*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                     static_cast<const float*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
                     static_cast<float*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W, c.status};
     SESSD_LAUNCH_NAMED(name.c_str(), (conv_f32_kernel<CIN, COUT>), persistent_grid(1), F32_THREADS, smem, stream, a);

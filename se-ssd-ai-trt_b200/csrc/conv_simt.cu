@@ -116,6 +116,7 @@ struct Narrow {
 template <typename T, int CIN, int COUT>
 __global__ void __launch_bounds__(kThreads, (Narrow<T, CIN, COUT>::BLOCKS))
 conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ nbr,
+                   const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ order,
                    const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                    const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
                    T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
@@ -129,10 +130,10 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
     int32_t* s_idx = reinterpret_cast<int32_t*>(narrow_smem + kvol * N::W_STRIDE);   // [KVOL_MAX][ROWS]
     const int tid = threadIdx.x, r = tid / TPR, cq = tid % TPR;
     const int chunks = (max_voxels + ROWS - 1) / ROWS;
-    const int items = batch * chunks;
+    const int items = batch * chunks, tiles = (max_voxels + 127) / 128;
     // the block's next rows: frame, first row, row count of the frame; entry[j] = the map entries this thread reads for
     // them, entry e = (offset e / ROWS, row e % ROWS)
-    int next = blockIdx.x, b_next = 0, o_next = 0, n_next = 0;
+    int next = blockIdx.x, b_next = 0, o_next = 0, n_next = 0, row_next = 0;
     int entry[LOADS];
     auto fetch = [&]() {
         for (; next < items; next += gridDim.x) {
@@ -143,11 +144,13 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
             if (o_next < n_next) break;
         }
         if (next >= items) return;
+        const uint32_t mask = __ldg(tile_mask + (size_t)b_next * tiles + (o_next >> 7));
+        row_next = order && o_next + r < n_next ? __ldg(order + (size_t)b_next * max_voxels + o_next + r) : o_next + r;
         const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b_next, 0, o_next);   // ROWS rows of one 128-row tile
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
             const int e = tid + j * kThreads, k = e / ROWS, row = e % ROWS;
-            entry[j] = k < kvol && o_next + row < n_next ? __ldg(nb + k * kNbrRun + row) : -1;
+            entry[j] = k < kvol && ((mask >> k) & 1u) && o_next + row < n_next ? __ldg(nb + k * kNbrRun + row) : -1;
         }
     };
     fetch();
@@ -157,7 +160,8 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
         s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(weights[e]);
     }
     while (next < items) {
-        const int b = b_next, o = o_next + r, n = n_next;
+        const int b = b_next, o = row_next;
+        const bool live = o_next + r < n_next;
 #pragma unroll
         for (int j = 0; j < LOADS; ++j) {
             const int e = tid + j * kThreads;
@@ -211,7 +215,7 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
                 for (int c = 0; c < OC; ++c) acc[c] = __fadd_rn(acc[c], s[c]);
             }
         }
-        if (o < n) {
+        if (live) {
 #pragma unroll
             for (int c = 0; c < OC; ++c) {
                 float v = acc[c];
@@ -239,6 +243,7 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ nbr,
+                    const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ order,
                     const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                     const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol, int cin, int cout,
                     T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
@@ -249,11 +254,13 @@ conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t
     const int items = batch * chunks;
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
-        const int o = (it - b * chunks) * ROWS + wrow;
+        const int p = (it - b * chunks) * ROWS + wrow;
         int n = out_num[b];
         n = n > max_voxels ? max_voxels : n;
-        if (o >= n) continue;
-        const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b, 0, o);
+        if (p >= n) continue;
+        const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b, 0, p);
+        const uint32_t mask = __ldg(tile_mask + (size_t)b * ((max_voxels + 127) / 128) + (p >> 7));
+        const int o = order ? __ldg(order + (size_t)b * max_voxels + p) : p;
         const T* in_b = in + (size_t)b * max_voxels * cin;
         T* d = nullptr;
         if (dense) {
@@ -263,7 +270,7 @@ conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t
         for (int co = lane; co < cout; co += 32) {
             float acc = 0.f;
             for (int k = 0; k < kvol; ++k) {
-                const int idx = __ldg(nb + k * kNbrRun);
+                const int idx = (mask >> k) & 1u ? __ldg(nb + k * kNbrRun) : -1;
                 if (idx < 0) continue;
                 const T* x = in_b + (size_t)idx * cin;
                 const T* wk = weights + (size_t)k * cin * cout + co;
@@ -283,7 +290,7 @@ conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t
 template <typename T>
 int launch_generic(const ConvLaunch& c, cudaStream_t stream) {
     SESSD_LAUNCH_NAMED(sizeof(T) == 4 ? "conv_generic<f32>" : "conv_generic<f16>", conv_generic_kernel<T>,
-                       persistent_grid(8), kThreads, 0, stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr,
+                       persistent_grid(8), kThreads, 0, stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.tile_mask, c.order,
                        c.out_num, static_cast<const T*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels,
                        c.kvol, c.cin, c.cout, static_cast<T*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D,
                        c.H, c.W);
@@ -308,7 +315,8 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
         }
     }
     SESSD_LAUNCH_NAMED(name.c_str(), (conv_narrow_kernel<T, CIN, COUT>), persistent_grid(N::BLOCKS), kThreads, N::smem(c.kvol),
-                       stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.out_num,
+                       stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.tile_mask,
+                       c.order, c.out_num,
                        static_cast<const T*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
                        static_cast<T*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W);
     return SESSD_OK;

@@ -261,7 +261,7 @@ __device__ __forceinline__ int items_before_stage(uint32_t bits, int lane, int* 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(Ring<CIN>::THREADS, 1)
 conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const int32_t* __restrict__ nbr,
-                 const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
+                 const int32_t* __restrict__ order, const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
                  const uint8_t* __restrict__ wtiles, const __grid_constant__ EpiConst epi, int relu, int batch,
                  int max_voxels, int kvol, __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
                  int W, int32_t* status, int withhold_weights) {
@@ -548,6 +548,13 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
             }
         } else if (warp < EPI_WARPS) {
             // ---------------- epilogue ----------------
+            // output rows of this thread's positions (the map may hold the rows in another order), requested before the wait
+            int out_row[TILES];
+#pragma unroll
+            for (int t = 0; t < TILES; ++t) {
+                const int pos = row0 + t * TILE_M + tid;
+                out_row[t] = order && t < cnt && pos < n ? __ldg(order + (size_t)b * max_voxels + pos) : pos;
+            }
             bool got = true;
             if (any) {
                 got = mbar_wait<true>(smem_u32(&ctl->acc_full[set]), set_phase, abort_flag, 3 | (int)(acc_it << 4));
@@ -562,10 +569,11 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
             auto stage_swz = [](int r) { return RB == 64 ? (r >> 1) & 3 : (r >> 2) & 1; };
 #pragma unroll 1
             for (int t2 = 0; t2 < cnt; ++t2) {
-                const int row = row0 + t2 * TILE_M + tid;
+                const int pos = row0 + t2 * TILE_M + tid;
+                const int row = t2 == 0 ? out_row[0] : (t2 == 1 ? out_row[1] : (t2 == 2 ? out_row[2] : out_row[3]));
                 const uint32_t m_t2 = t2 == 0 ? m[0] : (t2 == 1 ? m[1] : (t2 == 2 ? m[2] : m[3]));
                 const bool have = any && got && m_t2;
-                const bool store = got && row < n;
+                const bool store = got && pos < n;
                 __half* d = nullptr;
                 if (dense && store) {
                     // fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x)
@@ -627,8 +635,8 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                         for (int i = 0; i < CPR; ++i) {
                             const int rr = lane / CPR + i * (32 / CPR), cc = lane % CPR;
                             const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * RB + ((cc ^ stage_swz(rr)) << 4));
-                            const int grow = row0 + t2 * TILE_M + warp * 32 + rr;
-                            if (grow < n)
+                            const int grow = __shfl_sync(0xFFFFFFFFu, row, rr);
+                            if (row0 + t2 * TILE_M + warp * 32 + rr < n)
                                 *reinterpret_cast<uint4*>(out + ((size_t)b * max_voxels + grow) * COUT + cb + cc * 8) = v;
                         }
                     }
@@ -838,7 +846,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
     memcpy(epi.scale, c.scale_host, sizeof epi.scale);
     memcpy(epi.shift, c.shift_host, sizeof epi.shift);
     SESSD_LAUNCH_NAMED(name.c_str(), (conv_umma_kernel<CIN, COUT>), persistent_grid(1), Ring<CIN>::THREADS, smem, stream,
-                       static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.tile_mask, c.out_num,
+                       static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                        static_cast<const uint8_t*>(c.umma_weights), epi, c.relu, c.batch, c.max_voxels,
                        c.kvol, static_cast<__half*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W,
                        c.status, c.debug_withhold_weights);

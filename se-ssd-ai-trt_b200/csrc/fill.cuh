@@ -24,19 +24,20 @@ __device__ __forceinline__ void zero_rows(void* tensor, int units, const int32_t
                                           int max_rows) {
     constexpr int PER = 4;                              // stores per thread and item
     const int64_t per_frame = (int64_t)max_rows * units;
-    const int chunks = (int)((per_frame + kThreads * PER - 1) / (kThreads * PER));
+    const int threads = (int)blockDim.x;
+    const int chunks = (int)((per_frame + threads * PER - 1) / (threads * PER));
     V zero;
     memset(&zero, 0, sizeof(V));
     for (int64_t it = blockIdx.x; it < (int64_t)batch * chunks; it += gridDim.x) {
         const int b = (int)(it / chunks), c = (int)(it - (int64_t)b * chunks);
         int n = __ldg(counts + b);
         n = n < 0 ? 0 : (n > max_rows ? max_rows : n);
-        const int64_t low = (int64_t)n * units, at = (int64_t)c * kThreads * PER;
-        if (at + kThreads * PER <= low) continue;       // uniform over the block
+        const int64_t low = (int64_t)n * units, at = (int64_t)c * threads * PER;
+        if (at + threads * PER <= low) continue;       // uniform over the block
         V* base = static_cast<V*>(tensor) + (int64_t)b * per_frame;
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            const int64_t i = at + j * kThreads + threadIdx.x;
+            const int64_t i = at + j * threads + threadIdx.x;
             if (i >= low && i < per_frame) base[i] = zero;
         }
     }

@@ -108,4 +108,48 @@ __device__ __forceinline__ void mark_row(const int4& c4, int b, const ConvGeom& 
     }
 }
 
+// The even bits of v, packed into the low half.
+__device__ __forceinline__ uint32_t even_bits(unsigned long long v) {
+    v &= 0x5555555555555555ull;
+    v = (v | (v >> 1)) & 0x3333333333333333ull;
+    v = (v | (v >> 2)) & 0x0F0F0F0F0F0F0F0Full;
+    v = (v | (v >> 4)) & 0x00FF00FF00FF00FFull;
+    v = (v | (v >> 8)) & 0x0000FFFF0000FFFFull;
+    return (uint32_t)(v | (v >> 16));
+}
+
+// Marks the candidate outputs of all cells of word (z, y, wx) of an input level, given its bits: the union of mark_row
+// over them. The layer must be derivable_in_x: kernel 1 and stride 1 in x (outputs are the cells themselves) or kernel 3,
+// stride 2, padding 1 (output x has the inputs 2x - 1, 2x, 2x + 1).
+__device__ __forceinline__ void mark_word(unsigned long long bits, int z, int y, int wx, int b, const ConvGeom& g,
+                                          const BitGrid& out) {
+    unsigned long long m0 = bits, m1 = 0ull;   // bits of output word w0 and of the one after it
+    int w0 = wx;
+    if (g.K[2] == 3) {
+        const unsigned long long even = even_bits(bits), odd = even_bits(bits >> 1);
+        const unsigned long long spread = even | odd | (odd << 1);   // 33 bits, from output 32 wx on
+        w0 = wx >> 1;
+        m0 = wx & 1 ? spread << 32 : spread;
+        m1 = wx & 1 ? spread >> 32 : 0ull;
+    }
+    const int x0 = w0 << 6;
+    if (x0 + 64 > out.X) m0 &= x0 < out.X ? (1ull << (out.X - x0)) - 1ull : 0ull;
+    if (x0 + 64 >= out.X) m1 = 0ull;               // (m1 is at most the next word's first bit)
+    const int c[2] = {z, y};
+#pragma unroll
+    for (int ez = 0; ez < 3; ++ez) {
+        const int oz = div_trunc(c[0] + g.P[0], g.S[0]) - ez, kz = c[0] - oz * g.S[0] + g.P[0];
+        if (ez >= g.span_max[0] || oz < 0 || oz >= out.Z || kz < 0 || kz >= g.K[0]) continue;
+#pragma unroll
+        for (int ey = 0; ey < 3; ++ey) {
+            const int oy = div_trunc(c[1] + g.P[1], g.S[1]) - ey, ky = c[1] - oy * g.S[1] + g.P[1];
+            if (ey >= g.span_max[1] || oy < 0 || oy >= out.Y || ky < 0 || ky >= g.K[1]) continue;
+            unsigned long long* rec = reinterpret_cast<unsigned long long*>(
+                out.rec + (size_t)b * out.words + ((size_t)oz * out.Y + oy) * out.xw + w0);
+            if ((*reinterpret_cast<volatile unsigned long long*>(rec) & m0) != m0) atomicOr(rec, m0);
+            if (m1 && (*reinterpret_cast<volatile unsigned long long*>(rec + 2) & m1) != m1) atomicOr(rec + 2, m1);
+        }
+    }
+}
+
 }  // namespace sessd

@@ -3,9 +3,8 @@
 // voxelize.cu numbers voxels by their first point, which is what the stand-alone voxeliser promises. Inside the front end
 // nobody sees the order of the voxel rows, and (z, y, x) order is the better one: neighbouring rows are neighbouring
 // cells, so the neighbour maps of the full-resolution layers, the gathers of their convolutions and the tiles of the
-// tensor-core kernel all become coherent, and the level gets an occupancy grid like every other one, so that the next
-// level's rows are derived from it and its maps are built like all others (no coordinate table, no input-stationary
-// scatter, no clearing of a map).
+// tensor-core kernel all become coherent, and the level gets an occupancy grid like every other one, so that its maps are
+// built like all others (no coordinate table, no input-stationary scatter, no clearing of a map).
 //
 // A full-resolution grid of a frame has 92 M cells and at most some 100,000 occupied ones, so the grid has two levels:
 // a top record {bits lo, bits hi, words before} per 64 words of 64 x-neighbouring cells (0.36 MB per frame), and a
@@ -13,7 +12,8 @@
 //   1. every point finds its cell and sets its word's bit in the top level;
 //   2. the words are numbered (one-pass scan) and their records cleared;
 //   3. every point sets its cell's bit in its word;
-//   4. the rows are numbered (one-pass scan): coordinates, row count, empty point lists;
+//   4. the rows are numbered (one-pass scan): coordinates, row count, empty point lists; every word marks the outputs of
+//      its cells in the next level's grid, a few atomics for up to 64 cells;
 //   5. every point pushes its index through its row's ascending list of the max_points_per_voxel smallest indices (a
 //      cascade of atomicMin, so the list does not depend on timing);
 //   6. every row averages its listed points, summed in ascending index order.
@@ -111,7 +111,7 @@ point_bits_kernel(const int32_t* __restrict__ points_size, int batch, int max_po
 __global__ void __launch_bounds__(kThreads)
 number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch, int max_voxels, int max_points, int max_pts,
                    ScanState scan, int4* __restrict__ coors, int32_t* __restrict__ voxel_num,
-                   uint32_t* __restrict__ lists, int32_t* status) {
+                   uint32_t* __restrict__ lists, ConvGeom geom, BitGrid marks, int32_t* status) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int chunks = scan_chunks(grid.words), items = batch * chunks;
@@ -128,6 +128,10 @@ number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch
         const int id = scan_position(scan.state + (size_t)b * chunks, c, cnt, &end, status);
         if (c == used - 1 && threadIdx.x == 0) voxel_num[b] = end;   // at most max_points rows, and those fit max_voxels
         if (w < n) rec[w].z = (uint32_t)id;
+        if (w < n && marks.rec) {
+            const int row = (int)r.w / grid.xw;
+            mark_word(bits, row / grid.Y, row % grid.Y, (int)r.w - row * grid.xw, b, geom, marks);
+        }
         // the warp's rows are consecutive: their point lists in one run
         const int first = __shfl_sync(0xFFFFFFFFu, id, 0), last = __shfl_sync(0xFFFFFFFFu, id + cnt, 31);
         uint32_t* list = lists + (size_t)b * max_points * max_pts;
@@ -210,7 +214,7 @@ void voxel_grid_layout(Bump& bump, const sessd_voxel_params* p, const int level_
 
 int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
                    const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelGrid& w,
-                   int32_t* status, cudaStream_t stream) {
+                   const ConvGeom& geom, const BitGrid& marks, int32_t* status, cudaStream_t stream) {
     const VoxGeom g = voxel_geom(*p);
     const float4* pts = reinterpret_cast<const float4*>(points);
     const int max_pts = p->max_points_per_voxel;
@@ -225,7 +229,8 @@ int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int o
                  status);
     SESSD_LAUNCH(point_bits_kernel, blocks(max_points), kThreads, 0, stream, points_size, batch, max_points, w.grid, w.pt_key);
     SESSD_LAUNCH(number_rows_kernel, blocks(w.grid.words), kThreads, 0, stream, w.grid, w.word_num, batch, p->max_voxels,
-                 max_points, max_pts, w.scan_rows, reinterpret_cast<int4*>(coors), voxel_num, w.lists, status);
+                 max_points, max_pts, w.scan_rows, reinterpret_cast<int4*>(coors), voxel_num, w.lists, geom, marks,
+                 status);
     SESSD_LAUNCH(point_list_kernel, blocks(max_points), kThreads, 0, stream, points_size, batch, max_points, w.grid, w.pt_key,
                  max_pts, w.lists);
     if (out_dtype == SESSD_F32)
