@@ -335,6 +335,7 @@ struct MapJob {
     int32_t* nbr;
     uint32_t* tile_mask;
     int32_t* order;      // [B][max_voxels] output row at each position of the map, or null: positions are rows
+    int shape;           // kernel size as K0 K1 K2
     int group;           // offsets that the map's consumers fetch together
     uint32_t plane[6];   // offsets of the kernel's outer planes: first and last in z, y, x
 };

@@ -38,139 +38,190 @@ struct MapShared {
     int warp_sum[kMapThreads / 32];
 };
 
-// Rows of the input level through its occupancy grid. Line probes in two steps, so that a thread has the reads of
-// several lines in flight.
+// An index answers for lines: the rows of the K2 x-neighbours x0 .. x0 + K2 - 1 on line (z, y). What the lines of one
+// output row share (Row) is worked out once; a line is then told by its distance from the row's first line. Reads go in
+// two steps, so that a thread has the reads of several lines in flight.
+
+// Through the level's occupancy grid.
 struct BitsIndex {
-    BitGrid g;
-    struct Probe { uint4 a, b; int w; bool two; };
-    // Record of an occupied word of a two-level grid, given its top record; empty when the word is.
-    __device__ __forceinline__ uint4 word_record(int b, int word, const uint4& t) const {
-        const unsigned long long tb = rec_bits(t), bit = 1ull << (word & 63);
+    const uint4* rec;      // of the frame
+    const uint4* top;      // of the frame, or null (one-level grid)
+    int Y, X, xw;
+    struct Row { int word, sh; bool two, neg; };
+    struct Line { uint4 a, b; };
+    static __device__ __forceinline__ BitsIndex make(const MapJob& j, int b) {
+        const BitGrid& g = j.in;
+        return BitsIndex{g.rec + (size_t)b * g.words, g.top ? g.top + (size_t)b * g.top_words : nullptr, g.Y, g.X, g.xw};
+    }
+    __device__ __forceinline__ Row row(int z, int y, int x0, int count) const {
+        const int lo = max(x0, 0), hi = min(x0 + count, X) - 1;
+        return Row{(z * Y + y) * xw + (lo >> 6), lo & 63, (hi >> 6) > (lo >> 6), x0 < 0};
+    }
+    __device__ __forceinline__ int step(int kz, int ky) const { return (kz * Y + ky) * xw; }
+    // Record of word w of a two-level grid, given its top record; empty when the word is.
+    __device__ __forceinline__ uint4 word_record(int w, const uint4& t) const {
+        const unsigned long long tb = rec_bits(t), bit = 1ull << (w & 63);
         if (!(tb & bit)) return make_uint4(0u, 0u, 0u, 0u);
-        return __ldg(g.rec + (size_t)b * g.words + (int)t.z + __popcll(tb & (bit - 1ull)));
+        return __ldg(rec + ((int)t.z + __popcll(tb & (bit - 1ull))));
     }
-    __device__ __forceinline__ void probe_first(int b, int z, int y, int x0, int count, bool on, Probe* p) const {
-        p->a = p->b = make_uint4(0u, 0u, 0u, 0u);
-        p->two = false;
-        p->w = -1;
+    __device__ __forceinline__ void first(const Row& r, int step, bool on, Line* l) const {
+        l->a = l->b = make_uint4(0u, 0u, 0u, 0u);
         if (!on) return;
-        const int lo = x0 < 0 ? 0 : x0, hi = x0 + count - 1 >= g.X ? g.X - 1 : x0 + count - 1;
-        if (lo > hi) return;
-        p->w = (z * g.Y + y) * g.xw + (lo >> 6);
-        p->two = (hi >> 6) != (lo >> 6);
-        if (!g.top) return;
-        p->a = __ldg(g.top + (size_t)b * g.top_words + (p->w >> 6));
-        if (p->two) p->b = __ldg(g.top + (size_t)b * g.top_words + ((p->w + 1) >> 6));
+        const int w = r.word + step;
+        l->a = __ldg(top ? top + (w >> 6) : rec + w);
+        if (r.two) l->b = __ldg(top ? top + ((w + 1) >> 6) : rec + w + 1);
     }
-    __device__ __forceinline__ void probe_second(int b, Probe* p) const {
-        if (p->w < 0) return;
-        if (g.top) {
-            p->a = word_record(b, p->w, p->a);
-            if (p->two) p->b = word_record(b, p->w + 1, p->b);
-            if (rec_bits(p->a) == 0ull) p->a.z = p->b.z;   // the rows of the window are then all of the second word
-        } else {
-            const uint4* rec = g.rec + (size_t)b * g.words + p->w;
-            p->a = __ldg(rec);
-            if (p->two) p->b = __ldg(rec + 1);
+    __device__ __forceinline__ void second(const Row& r, int step, Line* l) const {
+        if (!top) return;
+        const int w = r.word + step;
+        l->a = word_record(w, l->a);
+        if (r.two) {
+            l->b = word_record(w + 1, l->b);
+            if (rec_bits(l->a) == 0ull) l->a.z = l->b.z;   // the rows of the window are then all of the second word
         }
     }
-    // Rows of the cells x0 .. x0 + count - 1 (count <= 3): neighbouring bits of a window that may straddle two words, and
-    // rows are numbered along the line, so the row of a set cell is the row of the window's first cell plus the set
-    // cells before it.
-    __device__ __forceinline__ void finish(int, int, int, int x0, int count, const Probe& p, int (&rows)[3]) const {
-        const int lo = x0 < 0 ? 0 : x0;
-        const int sh = lo & 63;
-        const unsigned long long a = rec_bits(p.a), b = p.two ? rec_bits(p.b) : 0ull;
-        const unsigned long long window = sh ? (a >> sh) | (b << (64 - sh)) : a;
-        const int base = (int)p.a.z + __popcll(a & ((1ull << sh) - 1ull));
-#pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            const int x = x0 + e, pos = x - lo;
-            const bool set = e < count && x >= 0 && x < g.X && ((window >> pos) & 1ull);
-            rows[e] = set ? base + __popcll(window & ((1ull << pos) - 1ull)) : -1;
-        }
+    // The cells are neighbouring bits of a window that may straddle two words, and rows are numbered along the line, so
+    // the row of a set cell is the row of the window's first cell plus the set cells before it. (Cells past the line's
+    // end are never set.)
+    template <int COUNT>
+    __device__ __forceinline__ uint32_t finish(const Row& r, int, const Line& l, int (&rows)[3]) const {
+        const unsigned long long a = rec_bits(l.a);
+        unsigned long long v = a >> r.sh;
+        if (r.two) v |= rec_bits(l.b) << (64 - r.sh);
+        uint32_t w = (uint32_t)v;
+        if (r.neg) w <<= 1;
+        w &= (1u << COUNT) - 1u;
+        const int base = (int)l.a.z + __popcll(a & ((1ull << r.sh) - 1ull));
+        rows[0] = w & 1u ? base : -1;
+        rows[1] = w & 2u ? base + (int)(w & 1u) : -1;
+        rows[2] = w & 4u ? base + __popc(w & 3u) : -1;
+        return w;
     }
 };
 
-// The same through the x-grouped table: the three x-neighbours lie in at most two 32-byte buckets.
+// Through the x-grouped table: the three x-neighbours lie in at most two 32-byte buckets.
 struct BucketIndex {
-    Buckets t;
-    int Z, Y, X;
-    struct Probe { uint4 lo[2], hi[2]; uint32_t key[2]; };
-    __device__ __forceinline__ uint32_t cell(int z, int y, int x) const { return ((uint32_t)z * Y + y) * X + x; }
-    __device__ __forceinline__ void probe_first(int b, int z, int y, int x0, int count, bool on, Probe* p) const {
-        const int lo = x0 < 0 ? 0 : x0, hi = x0 + count - 1 >= X ? X - 1 : x0 + count - 1;
-        const uint32_t* base = t.data + (size_t)b * t.cap * 8;
+    const uint32_t* data;   // of the frame
+    uint32_t cap;
+    int shift, Y, X;
+    struct Row { uint32_t cell; int lo, hi; };              // cell: key of (z, y, x0); the line's cells are x0 + lo .. x0 + hi
+    struct Line { uint4 lo[2], hi[2]; uint32_t key[2]; };
+    static __device__ __forceinline__ BucketIndex make(const MapJob& j, int b) {
+        return BucketIndex{j.table.data + (size_t)b * j.table.cap * 8, j.table.cap, j.table.shift, j.g.in_shape[1], j.g.in_shape[2]};
+    }
+    __device__ __forceinline__ Row row(int z, int y, int x0, int count) const {
+        return Row{(uint32_t)((z * Y + y) * X + x0), x0 < 0 ? -x0 : 0, min(x0 + count, X) - 1 - x0};
+    }
+    __device__ __forceinline__ int step(int kz, int ky) const { return (kz * Y + ky) * X; }
+    __device__ __forceinline__ void first(const Row& r, int step, bool on, Line* l) const {
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            p->lo[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
-            p->hi[i] = make_uint4(kEmpty, 0u, 0u, 0u);
-            p->key[i] = kEmpty;
-            if (!on || lo > hi) continue;
-            p->key[i] = cell(z, y, i == 0 ? lo : hi) >> 2;
-            if (i == 1 && p->key[1] == p->key[0]) {
-                p->key[1] = kEmpty;
-                continue;
-            }
+            l->lo[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+            l->hi[i] = make_uint4(kEmpty, 0u, 0u, 0u);
+            l->key[i] = kEmpty;
+            if (!on || r.lo > r.hi) continue;
+            const uint32_t key = (r.cell + (uint32_t)step + (uint32_t)(i == 0 ? r.lo : r.hi)) >> 2;
+            if (i == 1 && key == l->key[0]) continue;
+            l->key[i] = key;
             // the whole 32-byte bucket with one 256-bit load (one request to L1 instead of two)
             asm volatile("ld.global.nc.v8.u32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-                         : "=r"(p->lo[i].x), "=r"(p->lo[i].y), "=r"(p->lo[i].z), "=r"(p->lo[i].w), "=r"(p->hi[i].x),
-                           "=r"(p->hi[i].y), "=r"(p->hi[i].z), "=r"(p->hi[i].w)
-                         : "l"(base + (size_t)hash_slot(p->key[i], t.shift) * 8));
+                         : "=r"(l->lo[i].x), "=r"(l->lo[i].y), "=r"(l->lo[i].z), "=r"(l->lo[i].w), "=r"(l->hi[i].x),
+                           "=r"(l->hi[i].y), "=r"(l->hi[i].z), "=r"(l->hi[i].w)
+                         : "l"(data + (size_t)hash_slot(key, shift) * 8));
         }
     }
-    __device__ __forceinline__ void probe_second(int b, Probe* p) const {   // first slot taken by another group: keep probing
-        const uint32_t* base = t.data + (size_t)b * t.cap * 8;
+    __device__ __forceinline__ void second(const Row&, int, Line* l) const {   // first slot taken by another group: keep probing
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            if (p->key[i] == kEmpty || p->hi[i].x == p->key[i]) continue;
-            uint32_t h = hash_slot(p->key[i], t.shift);
+            if (l->key[i] == kEmpty || l->hi[i].x == l->key[i]) continue;
+            uint32_t h = hash_slot(l->key[i], shift);
             uint4 lo = make_uint4(~0u, ~0u, ~0u, ~0u);
-            uint32_t cur = p->hi[i].x;
-            for (uint32_t probe = 1; probe < t.cap && cur != kEmpty; ++probe) {
-                h = (h + 1) & (t.cap - 1);
-                const uint4* bk = reinterpret_cast<const uint4*>(base + (size_t)h * 8);
+            uint32_t cur = l->hi[i].x;
+            for (uint32_t probe = 1; probe < cap && cur != kEmpty; ++probe) {
+                h = (h + 1) & (cap - 1);
+                const uint4* bk = reinterpret_cast<const uint4*>(data + (size_t)h * 8);
                 cur = __ldg(bk + 1).x;
-                if (cur == p->key[i]) {
+                if (cur == l->key[i]) {
                     lo = __ldg(bk);
                     break;
                 }
             }
-            p->lo[i] = lo;
+            l->lo[i] = lo;
         }
     }
     static __device__ __forceinline__ int pick(const uint4& v, uint32_t i) {
         return (int)(i == 0 ? v.x : (i == 1 ? v.y : (i == 2 ? v.z : v.w)));
     }
-    __device__ __forceinline__ void finish(int, int z, int y, int x0, int count, const Probe& p, int (&rows)[3]) const {
+    template <int COUNT>
+    __device__ __forceinline__ uint32_t finish(const Row& r, int step, const Line& l, int (&rows)[3]) const {
+        uint32_t w = 0;
 #pragma unroll
         for (int e = 0; e < 3; ++e) {
-            const int x = x0 + e;
             rows[e] = -1;
-            if (e >= count || x < 0 || x >= X || p.key[0] == kEmpty) continue;
-            const uint32_t key = cell(z, y, x);
-            rows[e] = pick((key >> 2) == p.key[0] ? p.lo[0] : p.lo[1], key & 3u);
+            if (e >= COUNT || e < r.lo || e > r.hi || l.key[0] == kEmpty) continue;
+            const uint32_t key = r.cell + (uint32_t)step + (uint32_t)e;
+            rows[e] = pick((key >> 2) == l.key[0] ? l.lo[0] : l.lo[1], key & 3u);
+            w |= (rows[e] >= 0 ? 1u : 0u) << e;
+        }
+        return w;
+    }
+};
+
+// Entries of row r of a window, whose first input cell is (z, y, x): into s.ids, and as a mask of offsets. KZ, KY, KX: the
+// kernel.
+template <int KZ, int KY, int KX, class Index>
+__device__ __forceinline__ uint32_t map_row(MapShared& s, const Index& in, int Z, int z, int y, int x, bool live, int r) {
+    const typename Index::Row row = in.row(z, y, x, KX);
+    uint32_t bits = 0;
+#pragma unroll
+    for (int kz = 0; kz < KZ; ++kz) {
+        const bool z_ok = live && (unsigned)(z + kz) < (unsigned)Z;
+        typename Index::Line l[KY];
+#pragma unroll
+        for (int ky = 0; ky < KY; ++ky)
+            in.first(row, in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y, &l[ky]);
+#pragma unroll
+        for (int ky = 0; ky < KY; ++ky) in.second(row, in.step(kz, ky), &l[ky]);
+#pragma unroll
+        for (int ky = 0; ky < KY; ++ky) {
+            int rows[3];
+            const int k0 = (kz * KY + ky) * KX;
+            bits |= in.template finish<KX>(row, in.step(kz, ky), l[ky], rows) << k0;
+#pragma unroll
+            for (int kx = 0; kx < KX; ++kx) s.ids[k0 + kx][r] = rows[kx];
         }
     }
-};
+    return bits;
+}
+
+// Any other kernel up to 3 x 3 x 3: one line at a time.
+template <class Index>
+__device__ __noinline__ uint32_t map_row_any(MapShared& s, const Index& in, const ConvGeom& g, int z, int y, int x, bool live,
+                                             int r) {
+    const typename Index::Row row = in.row(z, y, x, g.K[2]);
+    uint32_t bits = 0;
+    for (int kz = 0; kz < g.K[0]; ++kz)
+        for (int ky = 0; ky < g.K[1]; ++ky) {
+            const bool on = live && (unsigned)(z + kz) < (unsigned)g.in_shape[0] && (unsigned)(y + ky) < (unsigned)in.Y;
+            typename Index::Line l;
+            int rows[3];
+            in.first(row, in.step(kz, ky), on, &l);
+            in.second(row, in.step(kz, ky), &l);
+            const uint32_t w = in.template finish<3>(row, in.step(kz, ky), l, rows);
+            const int k0 = (kz * g.K[1] + ky) * g.K[2];
+            for (int kx = 0; kx < g.K[2]; ++kx) s.ids[k0 + kx][r] = rows[kx];
+            bits |= (w & ((1u << g.K[2]) - 1u)) << k0;
+        }
+    return bits;
+}
 
 template <class Index>
-struct MapIndexOf;
+constexpr int map_blocks() { return 2; }
 template <>
-struct MapIndexOf<BitsIndex> {
-    static constexpr int BLOCKS = 2;
-    static __device__ __forceinline__ BitsIndex make(const MapJob& j) { return BitsIndex{j.in}; }
-};
-template <>
-struct MapIndexOf<BucketIndex> {
-    static constexpr int BLOCKS = 1;       // the six buckets of a kz plane need more registers
-    static __device__ __forceinline__ BucketIndex make(const MapJob& j) {
-        return BucketIndex{j.table, j.g.in_shape[0], j.g.in_shape[1], j.g.in_shape[2]};
-    }
-};
+constexpr int map_blocks<BucketIndex>() { return 1; }   // the six buckets of a kz plane need more registers
 
 template <class Index>
-__global__ void __launch_bounds__(kMapThreads, MapIndexOf<Index>::BLOCKS)
+__global__ void __launch_bounds__(kMapThreads, map_blocks<Index>())
 map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame, TailRows tails) {
     pdl_enter();
     zero_tails(tails);
@@ -183,14 +234,13 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
         const int ji = it / per_job;
         const MapJob& job = jobs.job[ji];
         const ConvGeom& g = job.g;
-        const Index in = MapIndexOf<Index>::make(job);
         const int b = (it - ji * per_job) / windows;
+        const Index in = Index::make(job, b);
         const int w0 = (it - ji * per_job - b * windows) * kWindow;
         int n = __ldg(job.out_num + b);
         n = (n > max_voxels ? max_voxels : n) - w0;          // rows of this window
         if (n <= 0) continue;
         n = n > kWindow ? kWindow : n;
-        const int K0 = g.K[0], K1 = g.K[1], K2 = g.K[2];
         __syncthreads();                                     // the previous window has been written out
         for (int e = tid; e < 64 * kGroups / 2; e += kMapThreads) reinterpret_cast<uint32_t*>(s.count)[e] = 0u;
         if (tid < kWindow / 128) s.tile[tid] = 0u;
@@ -204,35 +254,11 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
             int4 c = make_int4(0, 0, 0, 0);
             if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + w0 + r);
             const int bz = c.y * g.S[0] - g.P[0], by = c.z * g.S[1] - g.P[1], bx = c.w * g.S[2] - g.P[2];
-            uint32_t bits = 0;
-#pragma unroll
-            for (int kz = 0; kz < 3; ++kz) {
-                if (kz >= K0) break;
-                const int z = bz + kz;
-                const bool z_ok = live && z >= 0 && z < g.in_shape[0];
-                typename Index::Probe pb[3];
-#pragma unroll
-                for (int ky = 0; ky < 3; ++ky) {
-                    if (ky >= K1) break;
-                    const int y = by + ky;
-                    in.probe_first(b, z, y, bx, K2, z_ok && y >= 0 && y < g.in_shape[1], &pb[ky]);
-                }
-#pragma unroll
-                for (int ky = 0; ky < 3; ++ky)
-                    if (ky < K1) in.probe_second(b, &pb[ky]);
-#pragma unroll
-                for (int ky = 0; ky < 3; ++ky) {
-                    if (ky >= K1) break;
-                    int rows3[3];
-                    in.finish(b, z, by + ky, bx, K2, pb[ky], rows3);
-#pragma unroll
-                    for (int kx = 0; kx < 3; ++kx) {
-                        if (kx >= K2) break;
-                        const int k = (kz * K1 + ky) * K2 + kx;
-                        s.ids[k][r] = rows3[kx];
-                        bits |= (rows3[kx] >= 0 ? 1u : 0u) << k;
-                    }
-                }
+            uint32_t bits;
+            switch (job.shape) {                             // uniform over the block
+                case 333: bits = map_row<3, 3, 3>(s, in, g.in_shape[0], bz, by, bx, live, r); break;
+                case 311: bits = map_row<3, 1, 1>(s, in, g.in_shape[0], bz, by, bx, live, r); break;
+                default: bits = map_row_any(s, in, g, bz, by, bx, live, r);
             }
             uint32_t key = 64u;                              // dead rows (the frame's last window): they stay behind
             if (live) {
@@ -294,18 +320,17 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
             const int r = s.src[p];
             if (job.order && p < n) job.order[(size_t)b * max_voxels + w0 + p] = w0 + r;
             int32_t* out = job.nbr + nbr_index(g.kvol, max_voxels, b, 0, w0 + p);
+            if (g.kvol < kMapKvol) m &= (1u << g.kvol) - 1u;
 #pragma unroll
-            for (int k = 0; k < kMapKvol; ++k) {
-                if (k >= g.kvol) break;
+            for (int k = 0; k < kMapKvol; ++k)
                 if ((m >> k) & 1u) out[k * kNbrRun] = p < n ? s.ids[k][r] : -1;
-            }
         }
     }
 }
 
 template <class Index>
 int launch_maps(const char* name, const MapJobs& jobs, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
-    static_assert(MapIndexOf<BitsIndex>::BLOCKS * (sizeof(MapShared) + 1024) <= 228 * 1024, "two windows per SM");
+    static_assert(map_blocks<BitsIndex>() * (sizeof(MapShared) + 1024) <= 228 * 1024, "two windows per SM");
     // the attribute belongs to the device's context: set it once per device (repeating it is harmless)
     static std::atomic<uint64_t> configured{0};
     int dev = 0;
@@ -317,7 +342,7 @@ int launch_maps(const char* name, const MapJobs& jobs, int batch, int max_voxels
         configured.fetch_or(bit, std::memory_order_release);
     }
     const int64_t items = (int64_t)jobs.count * batch * ((max_voxels + kWindow - 1) / kWindow);
-    const int most = persistent_grid(MapIndexOf<Index>::BLOCKS);
+    const int most = persistent_grid(map_blocks<Index>());
     SESSD_LAUNCH_NAMED(name, map_rows_kernel<Index>, (int)(items < most ? items : most), kMapThreads, sizeof(MapShared), stream,
                        jobs, batch, max_voxels, (max_voxels + 127) / 128, tails);
     return SESSD_OK;
@@ -334,6 +359,7 @@ MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* 
     j.nbr = nbr;
     j.tile_mask = tile_mask;
     j.order = order;
+    j.shape = g.K[0] * 100 + g.K[1] * 10 + g.K[2];
     j.group = cin >= 64 ? 1 : (cin >= 32 ? 2 : 4);       // 64 / cin offsets per stage of the tensor-core kernel
     for (int k = 0; k < g.kvol; ++k) {
         const int at[3] = {k / (g.K[1] * g.K[2]), k / g.K[2] % g.K[1], k % g.K[2]};
