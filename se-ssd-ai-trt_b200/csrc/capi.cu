@@ -86,7 +86,6 @@ struct ConvWorkspace {
     size_t ones_bytes;
     Buckets buckets;      // submanifold 3x3x3 and strided: x-grouped table of the input coordinates
     Table in_table;       // other submanifold geometries: flat table of the input coordinates
-    int32_t* order;       // output row at each position of the map (null: positions are rows)
     BitGrid out_bits;     // strided: occupancy grid of the output level
     void* zero_base;      // occupancy grid + tile masks + numbering state: zero before use
     size_t zero_bytes;
@@ -106,8 +105,6 @@ void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeo
         w->buckets = Buckets{bump.take<uint32_t>((size_t)batch * capb * 8), capb, 32 - ilog2(capb)};
         w->ones_base = w->buckets.data;
         w->ones_bytes = (size_t)batch * capb * 8 * sizeof(uint32_t);
-        w->order = bump.take<int32_t>((size_t)batch * p->max_voxels);
-        if (!sorted_map(g)) w->order = nullptr;
     } else {
         uint32_t* block = bump.take<uint32_t>(per * 2);
         w->in_table = Table{block, nullptr, reinterpret_cast<int32_t*>(block ? block + per : nullptr), cap, shift, 1, 1};
@@ -521,12 +518,10 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
                                        static_cast<int32_t*>(outputs[2]), ws.status, stream);
             if (rc) return rc;
         }
-        MapJobs jobs{};
-        jobs.count = 1;
-        jobs.job[0] = make_map_job(g, subm ? in_coors : static_cast<const int32_t*>(outputs[1]), out_num, p->in_channel, ws.nbr,
-                                   ws.tile_mask, ws.order);
-        jobs.job[0].table = ws.buckets;
-        rc = launch_map_rows(jobs, batch, maxV, subm ? TailRows{} : tails, stream);
+        MapJob job = make_map_job(g, subm ? in_coors : static_cast<const int32_t*>(outputs[1]), out_num, p->in_channel, ws.nbr,
+                                  ws.tile_mask, nullptr);
+        job.table = ws.buckets;
+        rc = launch_map_tiles(job, batch, maxV, subm ? TailRows{} : tails, stream);
         if (rc) return rc;
     } else {
         rc = launch_table_build(in_coors, in_num, batch, maxV, g.in_shape, ws.in_table, ws.status, stream);
@@ -540,7 +535,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     c.in = inputs[0];
     c.out = outputs[0];
     c.nbr = ws.nbr;
-    c.order = ws.order;
+    c.order = nullptr;
     c.tile_mask = ws.tile_mask;
     c.out_num = out_num;
     c.weights = w->impl.w;
@@ -583,7 +578,7 @@ int sessd_conv_rulebook_export(const sessd_conv_params* p, int batch, int frame,
     Bump bump(workspace);
     ConvWorkspace ws;
     conv_workspace_layout(bump, p, g, batch, &ws);
-    return launch_rulebook_export(ws.nbr, ws.tile_mask, ws.order, static_cast<const int32_t*>(out_voxel_num), frame, g.kvol,
+    return launch_rulebook_export(ws.nbr, ws.tile_mask, nullptr, static_cast<const int32_t*>(out_voxel_num), frame, g.kvol,
                                   p->max_voxels, indice_pairs, indice_num, static_cast<cudaStream_t>(stream));
 }
 
@@ -765,25 +760,28 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
                           static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vox,
                           /*zero_tail=*/false, stream);
     if (rc) return rc;
-    // Maps by the kind of their index: [0] occupancy grids, [1] the table of level-0 rows in point order.
-    MapJobs jobs[2] = {};
+    // Maps of the levels with a grid: collected here, one launch. Level-0 rows in point order have a table instead.
+    MapJobs jobs{};
     if (!w.grid0) {
         rc = launch_bucket_build(w.coors[0], w.num[0], batch, maxV, &bb->level_shape[0], w.buckets0, nullptr, BitGrid{}, w.status,
                                  stream);
         if (rc) return rc;
     }
-    auto add_job = [&](const sessd_backbone::Layer& L, int cin, int32_t* nbr, uint32_t* mask, int32_t* order) {
+    auto add_job = [&](const sessd_backbone::Layer& L, int cin, int32_t* nbr, uint32_t* mask, int32_t*& order) {
         const bool table = L.level_in == 0 && !w.grid0;
-        MapJobs& js = jobs[table ? 1 : 0];
-        if (js.count == MapJobs::kMax) {
-            const int rc_jobs = launch_map_rows(js, batch, maxV, TailRows{}, stream);
-            if (rc_jobs) return rc_jobs;
-            js.count = 0;
-        }
+        if (table) order = nullptr;
         MapJob j = make_map_job(L.g, w.coors[L.level_out], w.num[L.level_out], cin, nbr, mask, order);
+        if (table) {
+            j.table = w.buckets0;
+            return launch_map_tiles(j, batch, maxV, TailRows{}, stream);
+        }
         j.in = w.bits[L.level_in];
-        if (table) j.table = w.buckets0;
-        js.job[js.count++] = j;
+        if (jobs.count == MapJobs::kMax) {
+            const int rc_jobs = launch_map_windows(jobs, batch, maxV, stream);
+            if (rc_jobs) return rc_jobs;
+            jobs.count = 0;
+        }
+        jobs.job[jobs.count++] = j;
         return (int)SESSD_OK;
     };
     std::vector<char> nbr_ready(bb->nlevels, 0);
@@ -810,10 +808,8 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         rc = add_job(L, L.p.in_channel, w.nbr_layer[i], w.mask_layer[i], w.order_layer[i]);
         if (rc) return rc;
     }
-    for (const MapJobs& js : jobs) {
-        rc = launch_map_rows(js, batch, maxV, TailRows{}, stream);
-        if (rc) return rc;
-    }
+    rc = launch_map_windows(jobs, batch, maxV, stream);
+    if (rc) return rc;
     const void* cur = w.voxel_feat;
     for (size_t i = 0; i < bb->layers.size(); ++i) {
         const sessd_backbone::Layer& L = bb->layers[i];

@@ -325,7 +325,8 @@ int launch_number_outputs(const BitGrid& out, const BitGrid* derive_from, const 
 int launch_bucket_build(const int32_t* coors, const int32_t* voxel_num, int batch, int max_voxels, const int shape[3],
                         const Buckets& t, const ConvGeom* mark, const BitGrid& out, int32_t* status, cudaStream_t stream);
 // map_rows.cu: neighbour maps + tile masks of layers (any kernel up to 3x3x3, any stride) whose input level has an
-// occupancy grid (`in`) or an x-grouped table (`table`), the same kind for all jobs; one launch for up to MapJobs::kMax.
+// occupancy grid (`in`: launch_map_windows, one launch for up to MapJobs::kMax layers) or an x-grouped table of its rows
+// (`table`: launch_map_tiles).
 struct MapJob {
     const int32_t* out_coors;
     const int32_t* out_num;
@@ -347,7 +348,8 @@ struct MapJobs {
 // Everything of a job but its index; cin: input channels of the layers that read the map (the smallest).
 MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* out_num, int cin, int32_t* nbr,
                     uint32_t* tile_mask, int32_t* order);
-int launch_map_rows(const MapJobs& jobs, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream);
+int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream);
+int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream);
 int launch_tile_mask(const int32_t* nbr, const int32_t* out_num, int batch, int max_voxels, int kvol,
                      uint32_t* tile_mask, cudaStream_t stream);
 // conv_simt.cu

@@ -6,7 +6,7 @@
 // The index is the level's occupancy grid where it has one, else an x-grouped coordinate table (rows handed in by a
 // caller).
 //
-// A block takes a window of 1024 output rows, collects their entries in shared memory, and orders the rows by which of
+// Grids: a block takes a window of 1024 output rows, collects their entries in shared memory, and orders the rows by which of
 // the six outer planes of the kernel (first and last in z, y and x) hold a neighbour: a counting sort with 64 bins.
 // Tiles of such rows need fewer (tile, offset) pairs, which is what the convolutions' time depends on: for the strided
 // layers of the network a third fewer, for the 64-channel submanifold layers a seventh (a full sort by the 27-bit mask
@@ -167,10 +167,10 @@ struct BucketIndex {
     }
 };
 
-// Entries of row r of a window, whose first input cell is (z, y, x): into s.ids, and as a mask of offsets. KZ, KY, KX: the
-// kernel.
-template <int KZ, int KY, int KX, class Index>
-__device__ __forceinline__ uint32_t map_row(MapShared& s, const Index& in, int Z, int z, int y, int x, bool live, int r) {
+// Entries of the row whose first input cell is (z, y, x): put(offset, input row or -1) for every offset, and as a mask of
+// the offsets that have one. KZ, KY, KX: the kernel.
+template <int KZ, int KY, int KX, class Index, class Put>
+__device__ __forceinline__ uint32_t map_row(const Index& in, int Z, int z, int y, int x, bool live, Put put) {
     const typename Index::Row row = in.row(z, y, x, KX);
     uint32_t bits = 0;
 #pragma unroll
@@ -188,16 +188,15 @@ __device__ __forceinline__ uint32_t map_row(MapShared& s, const Index& in, int Z
             const int k0 = (kz * KY + ky) * KX;
             bits |= in.template finish<KX>(row, in.step(kz, ky), l[ky], rows) << k0;
 #pragma unroll
-            for (int kx = 0; kx < KX; ++kx) s.ids[k0 + kx][r] = rows[kx];
+            for (int kx = 0; kx < KX; ++kx) put(k0 + kx, rows[kx]);
         }
     }
     return bits;
 }
 
 // Any other kernel up to 3 x 3 x 3: one line at a time.
-template <class Index>
-__device__ __noinline__ uint32_t map_row_any(MapShared& s, const Index& in, const ConvGeom& g, int z, int y, int x, bool live,
-                                             int r) {
+template <class Index, class Put>
+__device__ __noinline__ uint32_t map_row_any(const Index& in, const ConvGeom& g, int z, int y, int x, bool live, Put put) {
     const typename Index::Row row = in.row(z, y, x, g.K[2]);
     uint32_t bits = 0;
     for (int kz = 0; kz < g.K[0]; ++kz)
@@ -209,38 +208,65 @@ __device__ __noinline__ uint32_t map_row_any(MapShared& s, const Index& in, cons
             in.second(row, in.step(kz, ky), &l);
             const uint32_t w = in.template finish<3>(row, in.step(kz, ky), l, rows);
             const int k0 = (kz * g.K[1] + ky) * g.K[2];
-            for (int kx = 0; kx < g.K[2]; ++kx) s.ids[k0 + kx][r] = rows[kx];
+            for (int kx = 0; kx < g.K[2]; ++kx) put(k0 + kx, rows[kx]);
             bits |= (w & ((1u << g.K[2]) - 1u)) << k0;
         }
     return bits;
 }
 
-template <class Index>
-constexpr int map_blocks() { return 2; }
-template <>
-constexpr int map_blocks<BucketIndex>() { return 1; }   // the six buckets of a kz plane need more registers
+template <class Index, class Put>
+__device__ __forceinline__ uint32_t map_entries(const Index& in, const MapJob& job, const int4& c, bool live, Put put) {
+    const ConvGeom& g = job.g;
+    const int z = c.y * g.S[0] - g.P[0], y = c.z * g.S[1] - g.P[1], x = c.w * g.S[2] - g.P[2];
+    switch (job.shape) {                                     // uniform over the block
+        case 333: return map_row<3, 3, 3>(in, g.in_shape[0], z, y, x, live, put);
+        case 311: return map_row<3, 1, 1>(in, g.in_shape[0], z, y, x, live, put);
+        default: return map_row_any(in, g, z, y, x, live, put);
+    }
+}
 
-template <class Index>
-__global__ void __launch_bounds__(kMapThreads, map_blocks<Index>())
-map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame, TailRows tails) {
+__global__ void __launch_bounds__(kMapThreads, 2)
+map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame) {
     pdl_enter();
-    zero_tails(tails);
     extern __shared__ __align__(16) uint8_t map_smem[];
     MapShared& s = *reinterpret_cast<MapShared*>(map_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int windows = (max_voxels + kWindow - 1) / kWindow;
-    const int per_job = batch * windows, items = per_job * jobs.count;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int ji = it / per_job;
-        const MapJob& job = jobs.job[ji];
-        const ConvGeom& g = job.g;
-        const int b = (it - ji * per_job) / windows;
-        const Index in = Index::make(job, b);
-        const int w0 = (it - ji * per_job - b * windows) * kWindow;
-        int n = __ldg(job.out_num + b);
-        n = (n > max_voxels ? max_voxels : n) - w0;          // rows of this window
-        if (n <= 0) continue;
+    // The windows that hold rows, numbered over (job, frame) pairs: a walk that only moves forward, 32 pairs at a time
+    // (lane = pair), the same in every warp.
+    const int pairs = jobs.count * batch;
+    auto pair_rows = [&](int p) {
+        if (p >= pairs) return 0;
+        const int j = p / batch;
+        const int v = __ldg(jobs.job[j].out_num + (p - j * batch));
+        return v > max_voxels ? max_voxels : (v < 0 ? 0 : v);
+    };
+    int pair0 = 0, before = 0, my_rows = pair_rows(lane), incl = 0;
+    auto running = [&]() {
+        incl = (my_rows + kWindow - 1) / kWindow;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += t;
+        }
+    };
+    running();
+    for (int it = blockIdx.x;; it += gridDim.x) {
+        for (int total = __shfl_sync(0xFFFFFFFFu, incl, 31); it >= before + total && pair0 < pairs;
+             total = __shfl_sync(0xFFFFFFFFu, incl, 31)) {
+            before += total;
+            pair0 += 32;
+            my_rows = pair_rows(pair0 + lane);
+            running();
+        }
+        if (pair0 >= pairs) break;
+        const int src_lane = __ffs((int)__ballot_sync(0xFFFFFFFFu, it < before + incl)) - 1;
+        const int ji = (pair0 + src_lane) / batch, b = pair0 + src_lane - ji * batch;
+        const int first = __shfl_sync(0xFFFFFFFFu, incl - (my_rows + kWindow - 1) / kWindow, src_lane);
+        const int w0 = (it - before - first) * kWindow;
+        int n = __shfl_sync(0xFFFFFFFFu, my_rows, src_lane) - w0;   // rows of this window
         n = n > kWindow ? kWindow : n;
+        const MapJob& job = jobs.job[ji];
+        const BitsIndex in = BitsIndex::make(job, b);
         __syncthreads();                                     // the previous window has been written out
         for (int e = tid; e < 64 * kGroups / 2; e += kMapThreads) reinterpret_cast<uint32_t*>(s.count)[e] = 0u;
         if (tid < kWindow / 128) s.tile[tid] = 0u;
@@ -253,13 +279,7 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
             const bool live = r < n;
             int4 c = make_int4(0, 0, 0, 0);
             if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + w0 + r);
-            const int bz = c.y * g.S[0] - g.P[0], by = c.z * g.S[1] - g.P[1], bx = c.w * g.S[2] - g.P[2];
-            uint32_t bits;
-            switch (job.shape) {                             // uniform over the block
-                case 333: bits = map_row<3, 3, 3>(s, in, g.in_shape[0], bz, by, bx, live, r); break;
-                case 311: bits = map_row<3, 1, 1>(s, in, g.in_shape[0], bz, by, bx, live, r); break;
-                default: bits = map_row_any(s, in, g, bz, by, bx, live, r);
-            }
+            const uint32_t bits = map_entries(in, job, c, live, [&](int k, int v) { s.ids[k][r] = v; });
             uint32_t key = 64u;                              // dead rows (the frame's last window): they stay behind
             if (live) {
                 key = 0u;
@@ -319,8 +339,8 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
             if (job.group >= 4) m |= (m & 0x33333333u) << 2 | ((m >> 2) & 0x33333333u);
             const int r = s.src[p];
             if (job.order && p < n) job.order[(size_t)b * max_voxels + w0 + p] = w0 + r;
-            int32_t* out = job.nbr + nbr_index(g.kvol, max_voxels, b, 0, w0 + p);
-            if (g.kvol < kMapKvol) m &= (1u << g.kvol) - 1u;
+            int32_t* out = job.nbr + nbr_index(job.g.kvol, max_voxels, b, 0, w0 + p);
+            if (job.g.kvol < kMapKvol) m &= (1u << job.g.kvol) - 1u;
 #pragma unroll
             for (int k = 0; k < kMapKvol; ++k)
                 if ((m >> k) & 1u) out[k * kNbrRun] = p < n ? s.ids[k][r] : -1;
@@ -328,24 +348,32 @@ map_rows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels,
     }
 }
 
-template <class Index>
-int launch_maps(const char* name, const MapJobs& jobs, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
-    static_assert(map_blocks<BitsIndex>() * (sizeof(MapShared) + 1024) <= 228 * 1024, "two windows per SM");
-    // the attribute belongs to the device's context: set it once per device (repeating it is harmless)
-    static std::atomic<uint64_t> configured{0};
-    int dev = 0;
-    SESSD_CUDA(cudaGetDevice(&dev));
-    const uint64_t bit = 1ull << (dev & 63);
-    if (!(configured.load(std::memory_order_acquire) & bit)) {
-        SESSD_CUDA(cudaFuncSetAttribute(map_rows_kernel<Index>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)sizeof(MapShared)));
-        configured.fetch_or(bit, std::memory_order_release);
+// Maps through a table: rows as a caller (or the voxeliser, in point order) numbered them. Every line is one or two
+// scattered 32-byte reads, which bounds an SM (a block of 1024 rows took 40 us for its 18 reads per row), so the rows are
+// spread over as many SMs as there are tiles: a block per tile, no ordering. Also zeroes the tails of the call's outputs,
+// whose row counts are known by now.
+__global__ void __launch_bounds__(128)
+map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, int tiles_per_frame, TailRows tails) {
+    pdl_enter();
+    zero_tails(tails);
+    __shared__ uint32_t s_mask[4];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int it = blockIdx.x; it < batch * tiles_per_frame; it += gridDim.x) {
+        const int b = it / tiles_per_frame, p0 = (it - b * tiles_per_frame) * 128;
+        int n = __ldg(job.out_num + b);
+        n = n > max_voxels ? max_voxels : n;
+        if (p0 >= n) continue;
+        const bool live = p0 + tid < n;
+        int4 c = make_int4(0, 0, 0, 0);
+        if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + p0 + tid);
+        int32_t* out = job.nbr + nbr_index(job.g.kvol, max_voxels, b, 0, p0 + tid);
+        const uint32_t bits = map_entries(BucketIndex::make(job, b), job, c, live, [&](int k, int v) { out[k * kNbrRun] = v; });
+        const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, bits);
+        __syncthreads();
+        if (lane == 0) s_mask[warp] = any;
+        __syncthreads();
+        if (tid == 0) job.tile_mask[it] = s_mask[0] | s_mask[1] | s_mask[2] | s_mask[3];
     }
-    const int64_t items = (int64_t)jobs.count * batch * ((max_voxels + kWindow - 1) / kWindow);
-    const int most = persistent_grid(map_blocks<Index>());
-    SESSD_LAUNCH_NAMED(name, map_rows_kernel<Index>, (int)(items < most ? items : most), kMapThreads, sizeof(MapShared), stream,
-                       jobs, batch, max_voxels, (max_voxels + 127) / 128, tails);
-    return SESSD_OK;
 }
 
 }  // namespace
@@ -372,10 +400,31 @@ MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* 
     return j;
 }
 
-int launch_map_rows(const MapJobs& jobs, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
+int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream) {
     if (jobs.count == 0) return SESSD_OK;
-    if (jobs.job[0].table.data) return launch_maps<BucketIndex>("map_rows<table>", jobs, batch, max_voxels, tails, stream);
-    return launch_maps<BitsIndex>("map_rows<grid>", jobs, batch, max_voxels, tails, stream);
+    static_assert(2 * (sizeof(MapShared) + 1024) <= 228 * 1024, "two windows per SM");
+    // the attribute belongs to the device's context: set it once per device (repeating it is harmless)
+    static std::atomic<uint64_t> configured{0};
+    int dev = 0;
+    SESSD_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if (!(configured.load(std::memory_order_acquire) & bit)) {
+        SESSD_CUDA(cudaFuncSetAttribute(map_windows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MapShared)));
+        configured.fetch_or(bit, std::memory_order_release);
+    }
+    const int64_t items = (int64_t)jobs.count * batch * ((max_voxels + kWindow - 1) / kWindow);
+    const int most = persistent_grid(2);
+    SESSD_LAUNCH(map_windows_kernel, (int)(items < most ? items : most), kMapThreads, sizeof(MapShared), stream, jobs, batch,
+                 max_voxels, (max_voxels + 127) / 128);
+    return SESSD_OK;
+}
+
+int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
+    const int tiles = (max_voxels + 127) / 128;
+    const int64_t items = (int64_t)batch * tiles;
+    const int most = persistent_grid(6);
+    SESSD_LAUNCH(map_tiles_kernel, (int)(items < most ? items : most), 128, 0, stream, job, batch, max_voxels, tiles, tails);
+    return SESSD_OK;
 }
 
 }  // namespace sessd
