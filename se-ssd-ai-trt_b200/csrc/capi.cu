@@ -91,6 +91,7 @@ struct ConvWorkspace {
     size_t zero_bytes;
     uint32_t* tile_mask;  // [B][tiles]
     ScanState scan;       // strided: numbering of the outputs
+    int* tile_counter;
     int32_t* nbr;
 };
 
@@ -117,9 +118,11 @@ void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeo
     const size_t mask_bytes = (batch * tiles * sizeof(uint32_t) + 15) / 16 * 16;
     const size_t grid_bytes = p->subm ? 0 : (size_t)batch * w->out_bits.words * sizeof(uint4);
     const size_t scan_bytes = p->subm ? 0 : scan_state_bytes(w->out_bits.words, batch);
-    char* zero = bump.take<char>(grid_bytes + mask_bytes + scan_bytes);
+    const size_t zero_bytes = grid_bytes + mask_bytes + scan_bytes + 16;
+    char* zero = bump.take<char>(zero_bytes);
     w->zero_base = zero;
-    w->zero_bytes = grid_bytes + mask_bytes + scan_bytes;
+    w->zero_bytes = zero_bytes;
+    w->tile_counter = reinterpret_cast<int*>(zero ? zero + zero_bytes - 16 : nullptr);
     w->out_bits.rec = reinterpret_cast<uint4*>(zero);
     w->tile_mask = reinterpret_cast<uint32_t*>(zero ? zero + grid_bytes : nullptr);
     if (!p->subm) w->scan = scan_state_at(zero ? zero + grid_bytes + mask_bytes : nullptr, w->out_bits.words, batch);
@@ -192,6 +195,7 @@ struct BackboneWorkspace {
     std::vector<int32_t*> nbr_layer;      // maps of the strided layers (indexed by layer)
     std::vector<int32_t*> order_subm, order_layer;   // output rows at the maps' positions (null: positions are rows)
     std::vector<ScanState> scan;          // numbering state of the derived levels
+    int* tile_counter;                    // one per layer
     std::vector<void*> feat;
 };
 
@@ -235,7 +239,7 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
     // levels. A grid that is derived from its input level's grid is written whole.
     const size_t tiles = (size_t)(maxV + 127) / 128;
     const size_t mask_words = batch * tiles;
-    size_t zero_bytes = 0;
+    size_t zero_bytes = (bb->layers.size() + 3) / 4 * 4 * sizeof(int);   // tile counters
     w->scan.assign(bb->nlevels, ScanState{nullptr, nullptr});
     for (int l = 1; l < bb->nlevels; ++l) {
         w->bits[l] = bitgrid_shape(&bb->level_shape[3 * l]);
@@ -251,6 +255,7 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
         off += bytes;
         return p;
     };
+    w->tile_counter = reinterpret_cast<int*>(carve((bb->layers.size() + 3) / 4 * 4 * sizeof(int)));
     for (int l = 1; l < bb->nlevels; ++l) {
         const size_t bytes = (size_t)batch * w->bits[l].words * sizeof(uint4);
         w->bits[l].rec = w->derived[l] ? bump.take<uint4>(bytes / sizeof(uint4)) : reinterpret_cast<uint4*>(carve(bytes));
@@ -550,6 +555,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     c.cout = p->out_channel;
     c.dtype = w->impl.dtype;
     c.status = ws.status;
+    c.tile_counter = ws.tile_counter;
     c.debug_withhold_weights = w->impl.debug_withhold;
     c.scale_host = w->impl.host_scale;
     c.shift_host = w->impl.host_shift;
@@ -839,6 +845,8 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         c.cout = L.p.out_channel;
         c.dtype = bb->dtype;
         c.status = w.status;
+        c.tile_counter = w.tile_counter + i;
+        c.maps_ready = i > 0 ? 1 : 0;   // the first layer follows the launch that builds the maps
         c.debug_withhold_weights = L.w->impl.debug_withhold;
         c.scale_host = L.w->impl.host_scale;
         c.shift_host = L.w->impl.host_shift;

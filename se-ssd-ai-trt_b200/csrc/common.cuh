@@ -372,6 +372,8 @@ struct ConvLaunch {
     const int32_t* out_coors;
     int D, H, W;
     int32_t* status;       // device status word (tensor-core path reports wait timeouts there)
+    int* tile_counter;     // tensor-core path: zero before the launch; hands out the tiles of small layers (null: it never does)
+    int maps_ready;        // neighbour map, masks and row counts are older than the kernel launched just before
     int debug_withhold_weights;   // tests only: the tensor-core kernel's weight streamer stays silent (waits run out)
     const float* scale_host;      // [Cout <= 64] host copies of scale / shift (ones / zeros without batch norm), or null
     const float* shift_host;

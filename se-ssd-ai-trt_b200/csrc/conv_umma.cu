@@ -61,6 +61,9 @@ constexpr int B_STAGES = 3;                  // weight ring: a group needs up to
 constexpr int ROW_BYTES = 128;               // 64 halves per A/B row
 constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
+constexpr int FEW_TILES = 2;                 // few-tiles path: up to this many tiles per CTA
+constexpr int FEW_B_FULL = 2;                // where that path keeps its weight barriers among i_full
+constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // Words from one offset's 128 indices to the next offset's inside an index block: 16 bytes more than the indices
 // take, so that lanes reading different offsets of a stage (32- and 16-channel inputs) use different banks too.
 constexpr int TAP_WORDS = kNbrRun;
@@ -258,14 +261,272 @@ __device__ __forceinline__ int items_before_stage(uint32_t bits, int lane, int* 
     return items;
 }
 
+// Epilogue of one tile for one of four warps: rows 32 warp .. + 31 of the tile, lane = position `pos` of the map, output
+// row `row`, accumulators at tensor-memory address taddr (zeros instead when !have).
+template <int COUT>
+__device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiConst& epi, int relu, uint8_t* s_stage, int warp,
+                                           int lane, int pos, int row, int n, int b, int max_voxels, __half* __restrict__ out,
+                                           __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
+                                           int W) {
+    // Column blocks of CB channels keep the register footprint small.
+    constexpr int CB = COUT < 32 ? COUT : 32;
+    constexpr int RB = stage_row_bytes<COUT>();   // bytes of a row's column block
+    constexpr int CPR = RB / 16;                  // 16-byte chunks per row and block: 4 or 2
+    uint8_t* stage = s_stage + warp * (32 * RB);
+    auto stage_swz = [](int r) { return RB == 64 ? (r >> 1) & 3 : (r >> 2) & 1; };
+    __half* d = nullptr;
+    if (dense && pos < n) {
+        // fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x)
+        const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + row]);
+        d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
+    }
+#pragma unroll
+    for (int cb = 0; cb < COUT; cb += CB) {
+        float acc[CB];
+        if (have) {
+            if constexpr (CB == 32) {
+                uint32_t r32[32];
+                tmem_ld32(taddr + cb, r32);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) acc[j] = __uint_as_float(r32[j]);
+            } else {
+                uint32_t r16[16];
+                tmem_ld16(taddr + cb, r16);
+#pragma unroll
+                for (int j = 0; j < 16; ++j) acc[j] = __uint_as_float(r16[j]);
+            }
+            tmem_ld_wait();
+        } else {
+#pragma unroll
+            for (int j = 0; j < CB; ++j) acc[j] = 0.f;
+        }
+        // Every lane packs its row's block into the warp's staging area (16-byte chunks XOR-swizzled by
+        // row so that neither the writes nor the reads below meet in a bank) ...
+#pragma unroll
+        for (int c0 = 0; c0 < CB; c0 += 8) {
+            uint4 pk;
+            __half2* h = reinterpret_cast<__half2*>(&pk);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int ch = cb + c0 + 2 * j;   // a constant after unrolling
+                float v0 = fmaf(acc[c0 + 2 * j], epi.scale[ch], epi.shift[ch]);
+                float v1 = fmaf(acc[c0 + 2 * j + 1], epi.scale[ch + 1], epi.shift[ch + 1]);
+                if (relu) {
+                    v0 = v0 > 0.f ? v0 : 0.f;
+                    v1 = v1 > 0.f ? v1 : 0.f;
+                }
+                h[j] = __floats2half2_rn(v0, v1);
+            }
+            *reinterpret_cast<uint4*>(stage + lane * RB + (((c0 >> 3) ^ stage_swz(lane)) << 4)) = pk;
+            if (d) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    d[(size_t)(cb + c0 + 2 * j) * D * H * W] = __low2half(h[j]);
+                    d[(size_t)(cb + c0 + 2 * j + 1) * D * H * W] = __high2half(h[j]);
+                }
+            }
+        }
+        __syncwarp();
+        // ... and the warp copies the block out with CPR lanes per row: each store instruction writes
+        // 32 / CPR rows as whole runs of RB bytes.
+#pragma unroll
+        for (int i = 0; i < CPR; ++i) {
+            const int rr = lane / CPR + i * (32 / CPR), cc = lane % CPR;
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * RB + ((cc ^ stage_swz(rr)) << 4));
+            const int grow = __shfl_sync(0xFFFFFFFFu, row, rr);
+            if (pos - lane + rr < n)
+                *reinterpret_cast<uint4*>(out + ((size_t)b * max_voxels + grow) * COUT + cb + cc * 8) = v;
+        }
+        __syncwarp();
+    }
+}
+
+// ---- few tiles ----
+// With no more than FEW_TILES tiles per CTA the pipeline above is all latency: one tile's offsets are a serial chain, its
+// weight blocks are used once, so that three of them in flight bound it (390 ns per item on a single 20,000-point frame),
+// and everything before the first gather (5.8 us: work split, masks, index copy) comes on top of every launch. This path
+// takes one tile at a time, with seven A slots and as many weight blocks in flight, all of the tile's indices in one
+// copy, and does what does not depend on the preceding kernel before it waits for that kernel: barriers, tensor memory,
+// tile, indices and the first weight blocks. Tiles are handed out by a counter: a CTA that starts late, because the
+// preceding kernel still held its SM, leaves the tiles to the others. A tile's offsets are added up in the same order as
+// in the other path, so the results are the same bits.
+template <int CIN, int COUT>
+__device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_t* s_idx, uint8_t* s_stage, uint32_t tmem,
+                                         bool leader, const __half* __restrict__ in, __half* __restrict__ out,
+                                         const int32_t* __restrict__ nbr, const int32_t* __restrict__ order,
+                                         const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
+                                         const uint8_t* __restrict__ wtiles, const EpiConst& epi, int relu, int batch,
+                                         int max_voxels, int kvol, __half* __restrict__ dense,
+                                         const int4* __restrict__ out_coors, int D, int H, int W, int* tile_counter,
+                                         bool wait_first, int withhold_weights) {   // returns the weight blocks asked for
+    constexpr int KG = 64 / CIN, CPO = CIN / 8, B_BYTES = COUT * ROW_BYTES;
+    constexpr uint32_t IDESC = umma_idesc(COUT);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tiles_per_frame = (max_voxels + TILE_M - 1) / TILE_M;
+    volatile int* abort_flag = &ctl->abort_flag;
+    uint8_t* sB = sA + FEW_SLOTS * A_BYTES;
+    // barriers and words of the other path with the same arrival counts
+    unsigned long long *a_full = ctl->a_full[0], *empty = ctl->a_empty, *idx_full = &ctl->i_full[0], *acc_full = &ctl->i_full[1],
+                       *b_full = ctl->i_full + FEW_B_FULL;
+    volatile uint32_t* hand = ctl->scan_warp;   // the tile in hand: frame (-1: none left), first row, the frame's rows, mask
+    uint32_t items = 0;                        // items of the tiles so far
+    uint32_t b_issued = 0;
+    bool waited = wait_first;                  // the preceding kernel's writes may be read
+    for (uint32_t round = 0;; ++round) {
+        if (warp == 0) {
+            int t = 0;
+            if (lane == 0) t = atomicAdd(tile_counter, 1);
+            t = __shfl_sync(0xFFFFFFFFu, t, 0);
+            int frame = -1, first = 0, rows = 0;
+            for (int f0 = 0; f0 < batch && frame < 0; f0 += 32) {
+                int n = f0 + lane < batch ? __ldg(out_num + f0 + lane) : 0;
+                n = n > max_voxels ? max_voxels : (n < 0 ? 0 : n);
+                const int tiles = (n + TILE_M - 1) / TILE_M;
+                int incl = tiles;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                    if (lane >= d) incl += v;
+                }
+                const uint32_t hit = __ballot_sync(0xFFFFFFFFu, t < incl);
+                if (hit) {
+                    const int src = __ffs((int)hit) - 1;
+                    frame = f0 + src;
+                    first = (t - __shfl_sync(0xFFFFFFFFu, incl - tiles, src)) * TILE_M;
+                    rows = __shfl_sync(0xFFFFFFFFu, n, src);
+                }
+                t -= __shfl_sync(0xFFFFFFFFu, incl, 31);
+            }
+            if (lane == 0) {
+                hand[0] = (uint32_t)frame, hand[1] = (uint32_t)first, hand[2] = (uint32_t)rows;
+                hand[3] = frame < 0 ? 0u : __ldg(tile_mask + (size_t)frame * tiles_per_frame + first / TILE_M);
+            }
+        }
+        __syncthreads();
+        const int b = (int)hand[0], row0 = (int)hand[1], n = (int)hand[2];
+        const uint32_t mask = hand[3];
+        if (b < 0 || *abort_flag) break;       // (the flag is only ever raised before the barrier below)
+        const uint32_t stages = stage_bits<KG>(mask);        // bit g * KG for stage g
+        const int n_items = __popc(stages);
+        if (warp >= FIRST_GATHER_WARP && warp < FIRST_GATHER_WARP + FEW_SLOTS) {
+            // gather, as in the other path; slot s belongs to this warp
+            const int s = warp - FIRST_GATHER_WARP;
+            const int c = lane & 7, jrow = (lane >> 3) * 8, koff = c / CPO;
+            const __half* lane_base = in + (size_t)b * max_voxels * CIN + (c % CPO) * 8;
+            const uint32_t a_base = smem_u32(sA + s * A_BYTES) + jrow * ROW_BYTES;
+            const int rows_left = n - (row0 + jrow);
+            bool ok = mbar_wait(smem_u32(idx_full), round & 1u, abort_flag, 1 | (int)(items << 4));
+            // this warp's items: every FEW_SLOTS-th stage of the tile
+            int e = (s + FEW_SLOTS - (int)(items % FEW_SLOTS)) % FEW_SLOTS;
+            uint32_t left = stages;
+            for (int i = 0; i < e; ++i) left &= left - 1u;
+            for (; ok && left; e += FEW_SLOTS) {
+                const uint32_t q = items + (uint32_t)e;
+                const int g = (__ffs((int)left) - 1) / KG;
+#pragma unroll
+                for (int i = 0; i < FEW_SLOTS; ++i) left &= left - 1u;
+                const uint32_t idx_base = smem_u32(s_idx + (g * KG + koff) * TAP_WORDS + jrow);
+                const bool k_ok = g * KG + koff < kvol;
+                int vv[32];
+#pragma unroll
+                for (int w4 = 0; w4 < 8; ++w4) {
+                    int4 v;
+                    asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                 : "r"(idx_base + 128 * (w4 >> 1) + 16 * (w4 & 1)));
+                    vv[4 * w4] = v.x, vv[4 * w4 + 1] = v.y, vv[4 * w4 + 2] = v.z, vv[4 * w4 + 3] = v.w;
+                }
+                if (!waited) {
+                    pdl_enter();
+                    waited = true;
+                }
+                ok = mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 2 | (int)(q << 4));
+                if (!ok) break;
+#pragma unroll
+                for (int p = 0; p < 32; ++p) {
+                    const int id = (k_ok && 32 * (p >> 3) + (p & 7) < rows_left) ? vv[p] : -1;
+                    cp_async_16(a_base + (32 * (p >> 3) + (p & 7)) * ROW_BYTES + ((c ^ (p & 7)) << 4),
+                                lane_base + (size_t)(id < 0 ? 0 : id) * CIN, id < 0 ? 0u : 16u);
+                }
+                cp_async_arrive_noinc(smem_u32(a_full + s));
+            }
+        } else if (warp < EPI_WARPS) {
+            const int pos = row0 + tid;
+            const int row = order && pos < n ? __ldg(order + (size_t)b * max_voxels + pos) : pos;
+            if (!waited) {                     // (out is another kernel's input until then)
+                pdl_enter();
+                waited = true;
+            }
+            bool got = true;
+            if (n_items) {
+                got = mbar_wait<true>(smem_u32(acc_full), round & 1u, abort_flag, 3 | (int)(round << 4));
+                got = __all_sync(0xFFFFFFFFu, got);
+                if (got) tc_fence_after();
+            }
+            if (got)
+                store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16), n_items != 0, epi, relu, s_stage, warp, lane, pos, row, n, b,
+                                 max_voxels, out, dense, out_coors, D, H, W);
+            tc_fence_before();
+        } else if (warp == EPI_WARPS) {
+            // issuer
+            bool ok = true;
+            for (int e = 0; e < n_items && ok; ++e) {
+                const uint32_t q = items + (uint32_t)e, s = q % FEW_SLOTS, phase = (q / FEW_SLOTS) & 1u;
+                ok = mbar_wait<false, true>(smem_u32(b_full + s), phase, abort_flag, 5 | (int)(q << 4)) &&
+                     mbar_wait<false, true>(smem_u32(a_full + s), phase, abort_flag, 6 | (int)(q << 4));
+                if (ok && leader) {
+                    fence_proxy_async();       // the gathered rows were written through the generic proxy
+                    tc_fence_after();
+                    const uint64_t adesc = umma_desc(smem_u32(sA + s * A_BYTES));
+                    const uint64_t bdesc = umma_desc(smem_u32(sB + s * B_BYTES));
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_f16(tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (e > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit(smem_u32(empty + s));
+                }
+            }
+            if (ok && leader && n_items) umma_commit(smem_u32(acc_full));
+            __syncwarp();
+        } else if (warp == INDEX_WARP) {
+            if (lane == 0) {
+                mbar_arrive_expect_tx(smem_u32(idx_full), (uint32_t)(kvol * TAP_WORDS * 4));
+                bulk_load(smem_u32(s_idx), nbr + nbr_index(kvol, max_voxels, b, 0, row0), (uint32_t)(kvol * TAP_WORDS * 4),
+                          smem_u32(idx_full));
+                ctl->idx_uses[0] = round + 1u;
+            }
+            __syncwarp();
+        } else if (warp == WEIGHT_WARP) {
+            if (lane == 0 && !withhold_weights) {
+                uint32_t q = items;
+                for (uint32_t left = stages; left; left &= left - 1u, ++q) {
+                    const uint32_t s = q % FEW_SLOTS;
+                    if (!mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 8 | (int)(q << 4))) break;
+                    const uint32_t bar = smem_u32(b_full + s);
+                    mbar_arrive_expect_tx(bar, B_BYTES);
+                    bulk_load(smem_u32(sB + s * B_BYTES), wtiles + (size_t)((__ffs((int)left) - 1) / KG) * B_BYTES, B_BYTES, bar);
+                    b_issued = q + 1u;
+                }
+            }
+            __syncwarp();
+        }
+        items += (uint32_t)n_items;
+        __syncthreads();                       // indices, accumulator and tile may be replaced
+        tc_fence_after();
+    }
+    if (!waited) pdl_enter();                  // every CTA waits: the next kernel counts on what came before this one
+    return b_issued;
+}
+
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(Ring<CIN>::THREADS, 1)
 conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const int32_t* __restrict__ nbr,
                  const int32_t* __restrict__ order, const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
                  const uint8_t* __restrict__ wtiles, const __grid_constant__ EpiConst epi, int relu, int batch,
                  int max_voxels, int kvol, __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
-                 int W, int32_t* status, int withhold_weights) {
-    pdl_enter();
+                 int W, int32_t* status, int* tile_counter, int maps_ready, int withhold_weights) {
+    // Whatever does not depend on the preceding kernel comes before the wait for it. maps_ready: neighbour map, masks and
+    // row counts are older than that kernel.
+    if (!maps_ready) pdl_enter();
     // withhold_weights (tests of the time-out path only): the weight streamer stays silent, so the MMA issuers'
     // bounded wait for the first weight block runs out and every CTA with work leaves through the abort path.
     constexpr int KG = 64 / CIN;            // kernel offsets sharing one 128-byte A row
@@ -348,7 +609,15 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     };
     int total_tiles = 0;
     for (int f = 0; f < batch; ++f) total_tiles += (frame_rows(f) + TILE_M - 1) / TILE_M;
-    {
+    const bool few = tile_counter != nullptr && total_tiles <= FEW_TILES * (int)gridDim.x;
+    if (few) {
+        static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) <= NSLOT * A_BYTES + B_STAGES * B_BYTES &&
+                          KVOL_MAX * TAP_WORDS + 3 * TAP_WORDS <= NIDX * IDX_WORDS,
+                      "the few-tiles path lives in the other path's buffers");
+        b_issued = umma_few<CIN, COUT>(ctl, sA, s_idx, s_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
+                            batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, !maps_ready, withhold_weights);
+    }
+    if (!few) {
         const int per = (total_tiles + THREADS - 1) / THREADS;
         const int first = tid * per, last = first + per < total_tiles ? first + per : total_tiles;
         // a tile costs its items plus its share of the group hand-over and of the epilogue, about eight items' worth
@@ -436,7 +705,8 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         for (int t = 0; t < TILES; ++t)
             nx_m[t] = t < cnt ? __ldg(tile_mask + (size_t)nx_b * tiles_per_frame + nx_tile0 + t) : 0u;
     };
-    fetch_next();
+    if (!few) fetch_next();
+    if (maps_ready && !few) pdl_enter();
 
     while (nx_cnt > 0) {
         const int b = nx_b, n = nx_n, tile0 = nx_tile0, cnt = nx_cnt;
@@ -561,87 +831,14 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 got = __all_sync(0xFFFFFFFFu, got);
                 if (got) tc_fence_after();
             }
-            // Column blocks of CB channels keep the register footprint small.
-            constexpr int CB = COUT < 32 ? COUT : 32;
-            constexpr int RB = stage_row_bytes<COUT>();   // bytes of a row's column block
-            constexpr int CPR = RB / 16;                  // 16-byte chunks per row and block: 4 or 2
-            uint8_t* stage = s_stage + warp * (32 * RB);
-            auto stage_swz = [](int r) { return RB == 64 ? (r >> 1) & 3 : (r >> 2) & 1; };
 #pragma unroll 1
             for (int t2 = 0; t2 < cnt; ++t2) {
                 const int pos = row0 + t2 * TILE_M + tid;
                 const int row = t2 == 0 ? out_row[0] : (t2 == 1 ? out_row[1] : (t2 == 2 ? out_row[2] : out_row[3]));
                 const uint32_t m_t2 = t2 == 0 ? m[0] : (t2 == 1 ? m[1] : (t2 == 2 ? m[2] : m[3]));
-                const bool have = any && got && m_t2;
-                const bool store = got && pos < n;
-                __half* d = nullptr;
-                if (dense && store) {
-                    // fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x)
-                    const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + row]);
-                    d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
-                }
-#pragma unroll
-                for (int cb = 0; cb < COUT; cb += CB) {
-                    float acc[CB];
-                    if (have) {
-                        const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + set * SET_COLS + t2 * COUT + cb;
-                        if constexpr (CB == 32) {
-                            uint32_t r32[32];
-                            tmem_ld32(taddr, r32);
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) acc[j] = __uint_as_float(r32[j]);
-                        } else {
-                            uint32_t r16[16];
-                            tmem_ld16(taddr, r16);
-#pragma unroll
-                            for (int j = 0; j < 16; ++j) acc[j] = __uint_as_float(r16[j]);
-                        }
-                        tmem_ld_wait();
-                    } else {
-#pragma unroll
-                        for (int j = 0; j < CB; ++j) acc[j] = 0.f;
-                    }
-                    // Every lane packs its row's block into the warp's staging area (16-byte chunks XOR-swizzled by
-                    // row so that neither the writes nor the reads below meet in a bank) ...
-#pragma unroll
-                    for (int c0 = 0; c0 < CB; c0 += 8) {
-                        uint4 pk;
-                        __half2* h = reinterpret_cast<__half2*>(&pk);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int ch = cb + c0 + 2 * j;   // a constant after unrolling
-                            float v0 = fmaf(acc[c0 + 2 * j], epi.scale[ch], epi.shift[ch]);
-                            float v1 = fmaf(acc[c0 + 2 * j + 1], epi.scale[ch + 1], epi.shift[ch + 1]);
-                            if (relu) {
-                                v0 = v0 > 0.f ? v0 : 0.f;
-                                v1 = v1 > 0.f ? v1 : 0.f;
-                            }
-                            h[j] = __floats2half2_rn(v0, v1);
-                        }
-                        *reinterpret_cast<uint4*>(stage + lane * RB + (((c0 >> 3) ^ stage_swz(lane)) << 4)) = pk;
-                        if (d) {
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                d[(size_t)(cb + c0 + 2 * j) * D * H * W] = __low2half(h[j]);
-                                d[(size_t)(cb + c0 + 2 * j + 1) * D * H * W] = __high2half(h[j]);
-                            }
-                        }
-                    }
-                    __syncwarp();
-                    // ... and the warp copies the block out with CPR lanes per row: each store instruction writes
-                    // 32 / CPR rows as whole runs of RB bytes.
-                    if (got) {
-#pragma unroll
-                        for (int i = 0; i < CPR; ++i) {
-                            const int rr = lane / CPR + i * (32 / CPR), cc = lane % CPR;
-                            const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * RB + ((cc ^ stage_swz(rr)) << 4));
-                            const int grow = __shfl_sync(0xFFFFFFFFu, row, rr);
-                            if (row0 + t2 * TILE_M + warp * 32 + rr < n)
-                                *reinterpret_cast<uint4*>(out + ((size_t)b * max_voxels + grow) * COUT + cb + cc * 8) = v;
-                        }
-                    }
-                    __syncwarp();
-                }
+                if (got)
+                    store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + set * SET_COLS + t2 * COUT, any && m_t2, epi, relu,
+                                     s_stage, warp, lane, pos, row, n, b, max_voxels, out, dense, out_coors, D, H, W);
             }
             if (any && got) {
                 tc_fence_before();
@@ -796,16 +993,18 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
             for (int j = lane; j < NIDX; j += 32) {
                 const uint32_t uses = ctl->idx_uses[j];
                 if (!uses) continue;
+                const uint32_t bar = smem_u32(&ctl->i_full[j]);
                 const long long t0 = clock64();
-                while (!mbar_try_wait(smem_u32(&ctl->i_full[j]), (uses - 1u) & 1u) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
+                while (!mbar_try_wait(bar, (uses - 1u) & 1u) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
             }
         }
         if (warp == WEIGHT_WARP && lane == 0) {
-            const uint32_t first = b_issued > (uint32_t)B_STAGES ? b_issued - B_STAGES : 0u;
+            const uint32_t ring = few ? FEW_SLOTS : B_STAGES;
+            const uint32_t first = b_issued > ring ? b_issued - ring : 0u;
             for (uint32_t j = first; j < b_issued; ++j) {
-                const uint32_t bar = smem_u32(&ctl->b_full[j % B_STAGES]);
+                const uint32_t bar = smem_u32(few ? &ctl->i_full[FEW_B_FULL + j % ring] : &ctl->b_full[j % ring]);
                 const long long t0 = clock64();
-                while (!mbar_try_wait(bar, (j / B_STAGES) & 1u) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
+                while (!mbar_try_wait(bar, (j / ring) & 1u) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
             }
         }
     }
@@ -849,7 +1048,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
                        static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                        static_cast<const uint8_t*>(c.umma_weights), epi, c.relu, c.batch, c.max_voxels,
                        c.kvol, static_cast<__half*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W,
-                       c.status, c.debug_withhold_weights);
+                       c.status, c.tile_counter, c.maps_ready, c.debug_withhold_weights);
     return SESSD_OK;
 }
 
