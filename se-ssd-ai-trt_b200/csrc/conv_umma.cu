@@ -61,7 +61,7 @@ constexpr int B_STAGES = 3;                  // weight ring: a group needs up to
 constexpr int ROW_BYTES = 128;               // 64 halves per A/B row
 constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
-constexpr int FEW_TILES = 2;                 // few-tiles path: up to this many tiles per CTA
+constexpr int FEW_TILES = 1;                 // few-tiles path: up to this many tiles per CTA
 constexpr int FEW_B_FULL = 2;                // where that path keeps its weight barriers among i_full
 constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // Words from one offset's 128 indices to the next offset's inside an index block: 16 bytes more than the indices
