@@ -107,6 +107,27 @@ def lib():
         L.sessd_launch_count.restype = C.c_uint64
         L.sessd_last_cuda_error.restype = C.c_char_p
         L.sessd_version.restype = C.c_char_p
+        # declared, so that plain ints pass as pointers and sizes
+        p, i, z = C.c_void_p, C.c_int, C.c_size_t
+        L.sessd_read_status.argtypes = [p, p]
+        L.sessd_filter_boxes_workspace_bytes.argtypes = [p, i]
+        L.sessd_filter_boxes_enqueue.argtypes = [p, i, p, p, p, z, p]
+        L.sessd_decode_filter_enqueue.argtypes = [p, p, i, p, p, p, z, p]
+        L.sessd_rotated_nms_workspace_bytes.argtypes = [p, i]
+        L.sessd_rotated_nms_enqueue.argtypes = [p, i, p, p, p, z, p]
+        L.sessd_conv_workspace_bytes.argtypes = [p, i]
+        L.sessd_subm_conv_enqueue.argtypes = [p, p, i, p, p, p, z, p]
+        L.sessd_sparse_conv_enqueue.argtypes = [p, p, i, p, p, p, z, p]
+        L.sessd_voxelize_enqueue.argtypes = [p, i, i, i, p, p, p, z, p]
+        L.sessd_backbone_workspace_bytes.argtypes = [p, i, i]
+        L.sessd_backbone_enqueue.argtypes = [p, i, i, p, p, p, p, z, p]
+        L.sessd_backbone_pair_counts.argtypes = [p, i, i, p, p, p, p, z, p, p]
+        L.sessd_conv_rulebook_export.argtypes = [p, i, i, p, p, p, p, p]
+        L.sessd_sparse2dense_enqueue.argtypes = [p, i, i, i, p, p, p, z, p]
+        L.sessd_sparse2dense_padded_enqueue.argtypes = [p, p, i, i, i, p, p, p]
+        L.sessd_zero_pad2d_enqueue.argtypes = [p, i, i, i, i, i, p, p, p]
+        L.sessd_anchor_decode_enqueue.argtypes = [p, i, p, p, p]
+        L.sessd_profile_end.argtypes = [p, p, z, p, i]
         _lib = L
     return _lib
 
@@ -119,20 +140,34 @@ def _check(rc: int, what: str):
         raise SessdError(f"{what} failed: {names.get(rc, rc)} {extra}")
 
 
-def _torch():
-    import torch
+_torch_module = None
 
-    if not torch.cuda.is_available():
-        raise SessdError("a CUDA device is required (there is no CPU path in this package)")
-    return torch
+
+def _torch():
+    """torch, once a CUDA device has been seen (looked for once: the question costs as much as a kernel launch)."""
+    global _torch_module
+    if _torch_module is None:
+        import torch
+
+        if not torch.cuda.is_available():
+            raise SessdError("a CUDA device is required (there is no CPU path in this package)")
+        _torch_module = torch
+    return _torch_module
 
 
 def _stream():
-    return C.c_void_p(_torch().cuda.current_stream().cuda_stream)
+    """Handle of torch's current stream (an int: the entry points' pointer arguments are declared in lib()). Asked for
+    without building a Stream object, which takes 3 us, where torch offers that."""
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw(torch.cuda.current_device()) if raw else torch.cuda.current_stream().cuda_stream
+
+
+_ARRAYS = tuple(C.c_void_p * n for n in range(8))
 
 
 def _vp(*tensors):
-    return (C.c_void_p * len(tensors))(*[C.c_void_p(t.data_ptr()) if t is not None else None for t in tensors])
+    return _ARRAYS[len(tensors)](*[t.data_ptr() if t is not None else None for t in tensors])
 
 
 def _tdtype(dtype):
@@ -160,7 +195,7 @@ def conv_params(layer: schedule.ConvLayer, max_voxels: int) -> ConvParams:
 
 
 def read_status(workspace) -> int:
-    rc = lib().sessd_read_status(C.c_void_p(workspace.data_ptr()), _stream())
+    rc = lib().sessd_read_status(workspace.data_ptr(), _stream())
     if rc < 0:
         _check(rc, "sessd_read_status")
     return rc
@@ -192,8 +227,8 @@ def voxelize_into(points, points_size, params: VoxelParams, voxels, coors, voxel
     """sessd_voxelize_enqueue into caller-owned outputs and workspace (nothing is allocated, nothing is read back)."""
     B, P = points.shape[0], points.shape[1]
     _check(lib().sessd_voxelize_enqueue(C.byref(params), B, P, out_dtype, _vp(points, points_size),
-                                        _vp(voxels, coors, voxel_num), C.c_void_p(workspace.data_ptr()),
-                                        C.c_size_t(workspace.numel()), _stream()), "sessd_voxelize_enqueue")
+                                        _vp(voxels, coors, voxel_num), workspace.data_ptr(), workspace.numel(),
+                                        _stream()), "sessd_voxelize_enqueue")
 
 
 class ConvWeights:
@@ -256,8 +291,7 @@ def subm_conv(feat, coors, voxel_num, params: ConvParams, weights: ConvWeights, 
 def subm_conv_into(feat, coors, voxel_num, params: ConvParams, weights: ConvWeights, out, workspace):
     """sessd_subm_conv_enqueue into a caller-owned output and workspace (nothing is allocated or read back)."""
     _check(lib().sessd_subm_conv_enqueue(C.byref(params), weights.handle, feat.shape[0], _vp(feat, coors, voxel_num),
-                                         _vp(out), C.c_void_p(workspace.data_ptr()), C.c_size_t(workspace.numel()),
-                                         _stream()), "sessd_subm_conv_enqueue")
+                                         _vp(out), workspace.data_ptr(), workspace.numel(), _stream()), "sessd_subm_conv_enqueue")
 
 
 def sparse_conv(feat, coors, voxel_num, params: ConvParams, weights: ConvWeights, keep_workspace=False):
@@ -268,8 +302,8 @@ def sparse_conv(feat, coors, voxel_num, params: ConvParams, weights: ConvWeights
     ocoors = torch.empty((B, V, 4), dtype=torch.int32, device=feat.device)
     onum = torch.empty((B,), dtype=torch.int32, device=feat.device)
     _check(lib().sessd_sparse_conv_enqueue(C.byref(params), weights.handle, B, _vp(feat, coors, voxel_num),
-                                           _vp(out, ocoors, onum), C.c_void_p(ws.data_ptr()), C.c_size_t(nbytes),
-                                           _stream()), "sessd_sparse_conv_enqueue")
+                                           _vp(out, ocoors, onum), ws.data_ptr(), nbytes, _stream()),
+           "sessd_sparse_conv_enqueue")
     status = read_status(ws)
     r = dict(features=out, coors=ocoors, voxel_num=onum, status=status)
     if keep_workspace:
@@ -347,19 +381,19 @@ def filter_boxes(boxes, cls, iou, dirs, params: FilterParams, anchors: AnchorPar
     read_back_status=False nothing synchronises (stream capture) and `workspace` is returned for read_status."""
     torch = _torch()
     B, M = boxes.shape[0], params.max_box_num
-    f32 = dict(dtype=torch.float32, device=boxes.device)
-    out = dict(box=torch.empty((B, M, 9), **f32), score=torch.empty((B, M), **f32), iou=torch.empty((B, M), **f32),
-               direction=torch.empty((B, M), **f32), valid=torch.empty((B,), dtype=torch.int32, device=boxes.device))
+    like = boxes if boxes.dtype is torch.float32 else torch.empty((0,), dtype=torch.float32, device=boxes.device)
+    out = dict(box=like.new_empty((B, M, 9)), score=like.new_empty((B, M)), iou=like.new_empty((B, M)),
+               direction=like.new_empty((B, M)), valid=like.new_empty((B,), dtype=torch.int32))
     nbytes = lib().sessd_filter_boxes_workspace_bytes(C.byref(params), B)
-    ws = torch.empty((nbytes,), dtype=torch.uint8, device=boxes.device)
+    ws = like.new_empty((nbytes,), dtype=torch.uint8)
     ins = _vp(boxes, cls, iou, dirs)
     outs = _vp(out["box"], out["score"], out["iou"], out["direction"], out["valid"])
     if anchors is None:
-        _check(lib().sessd_filter_boxes_enqueue(C.byref(params), B, ins, outs, C.c_void_p(ws.data_ptr()),
-                                                C.c_size_t(nbytes), _stream()), "sessd_filter_boxes_enqueue")
+        _check(lib().sessd_filter_boxes_enqueue(C.byref(params), B, ins, outs, ws.data_ptr(), nbytes, _stream()),
+               "sessd_filter_boxes_enqueue")
     else:
         _check(lib().sessd_decode_filter_enqueue(C.byref(anchors), C.byref(params), B, ins, outs,
-                                                 C.c_void_p(ws.data_ptr()), C.c_size_t(nbytes), _stream()),
+                                                 ws.data_ptr(), nbytes, _stream()),
                "sessd_decode_filter_enqueue")
     if read_back_status:
         out["status"] = read_status(ws)
@@ -375,12 +409,11 @@ def rotated_nms(boxes, valid, nms_thresh=schedule.NMS_THRESH):
     B, M = boxes.shape[0], boxes.shape[1]
     p = NmsParams(M, nms_thresh)
     kept = torch.empty_like(boxes)
-    kept_num = torch.empty((B,), dtype=torch.int32, device=boxes.device)
+    kept_num = boxes.new_empty((B,), dtype=torch.int32)
     nbytes = lib().sessd_rotated_nms_workspace_bytes(C.byref(p), B)
-    ws = torch.empty((max(nbytes, 1),), dtype=torch.uint8, device=boxes.device)
-    _check(lib().sessd_rotated_nms_enqueue(C.byref(p), B, _vp(boxes, valid), _vp(kept, kept_num),
-                                           C.c_void_p(ws.data_ptr()), C.c_size_t(nbytes), _stream()),
-           "sessd_rotated_nms_enqueue")
+    ws = boxes.new_empty((max(nbytes, 1),), dtype=torch.uint8)
+    _check(lib().sessd_rotated_nms_enqueue(C.byref(p), B, _vp(boxes, valid), _vp(kept, kept_num), ws.data_ptr(), nbytes,
+                                           _stream()), "sessd_rotated_nms_enqueue")
     return kept, kept_num
 
 
@@ -457,15 +490,13 @@ class Backbone:
         """points cuda f32 [B, P, 4], points_size cuda i32 [B] -> (dense, workspace)."""
         torch = _torch()
         B, P = points.shape[0], points.shape[1]
-        nbytes = self.workspace_bytes(B, P)
         if workspace is None:
-            workspace = torch.empty(nbytes, dtype=torch.uint8, device=points.device)
+            workspace = torch.empty(self.workspace_bytes(B, P), dtype=torch.uint8, device=points.device)
         if dense is None and self.s2d is not None:
             dense = torch.empty(self.dense_shape(B), dtype=_tdtype(self.dtype), device=points.device)
-        _check(lib().sessd_backbone_enqueue(self.handle, B, P, C.c_void_p(points.data_ptr()),
-                                            C.c_void_p(points_size.data_ptr()),
-                                            C.c_void_p(dense.data_ptr()) if dense is not None else None,
-                                            C.c_void_p(workspace.data_ptr()), C.c_size_t(workspace.numel()), _stream()),
+        _check(lib().sessd_backbone_enqueue(self.handle, B, P, points.data_ptr(), points_size.data_ptr(),
+                                            dense.data_ptr() if dense is not None else None, workspace.data_ptr(),
+                                            workspace.numel(), _stream()),
                "sessd_backbone_enqueue")
         return dense, workspace
 

@@ -51,6 +51,8 @@ int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const 
 int launch_count_pairs(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* out_num, int batch, int max_voxels,
                        int kvol, unsigned long long* total, cudaStream_t stream);
 
+cudaError_t launch_publish_status(const int32_t* status, unsigned long long* host_word, uint32_t call, cudaStream_t stream);
+
 namespace {
 
 // np.round as the reference mimics it (voxelGenerator.cu:61-68).
@@ -283,6 +285,15 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
         w->feat[i] = bump.take<char>((size_t)batch * maxV * bb->layers[i].p.out_channel * esize(bb->dtype));
 }
 
+// A host thread's place for status words (sessd_read_status).
+struct StatusSlot {
+    unsigned long long* word = nullptr;   // call << 32 | status
+    uint32_t calls = 0;
+    ~StatusSlot() {
+        if (word) cudaFreeHost(word);     // (an error at process exit is of no consequence)
+    }
+};
+
 }  // namespace
 
 extern "C" {
@@ -297,12 +308,35 @@ int sessd_conv_weights_debug_withhold(sessd_conv_weights* w, int on) {
 const char* sessd_last_cuda_error(void) { return t_last_error.c_str(); }
 uint64_t sessd_launch_count(void) { return g_launches.load(); }
 
-int sessd_read_status(const void* workspace, void* stream) {
+// The word comes back through mapped host memory: a one-thread kernel behind the stream's work stores it together with the
+// call's number, and the host polls for that number. A stream synchronisation and a copy of four bytes took some 15 us
+// more. One 8-byte slot per host thread, returned when the thread ends.
+int sessd_read_status(const void* workspace, void* stream_) {
     if (!workspace) return SESSD_ERR_NULL;
-    int32_t v = 0;
-    SESSD_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-    SESSD_CUDA(cudaMemcpy(&v, workspace, sizeof(v), cudaMemcpyDeviceToHost));
-    return v & 0x7FFFFFFF;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+    cudaStreamCaptureStatus capture;
+    SESSD_CUDA(cudaStreamIsCapturing(stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        set_cuda_error(cudaErrorStreamCaptureUnsupported, "sessd_read_status");
+        return SESSD_ERR_CUDA;
+    }
+    static thread_local StatusSlot slot;
+    if (!slot.word)
+        SESSD_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&slot.word), sizeof(*slot.word), cudaHostAllocMapped | cudaHostAllocPortable));
+    const uint32_t call = ++slot.calls;
+    SESSD_CUDA(launch_publish_status(static_cast<const int32_t*>(workspace), slot.word, call, stream));
+    volatile unsigned long long* word = slot.word;
+    unsigned long long v;
+    for (unsigned spins = 0; (uint32_t)((v = *word) >> 32) != call;) {
+        if (++spins < 4096u) continue;
+        spins = 0;
+        const cudaError_t e = cudaStreamQuery(stream);   // an error on the stream would leave the word unwritten
+        if (e != cudaSuccess && e != cudaErrorNotReady) {
+            set_cuda_error(e, "sessd_read_status");
+            return SESSD_ERR_CUDA;
+        }
+    }
+    return (int)(v & 0x7FFFFFFFull);
 }
 
 // ---- profiling hooks ------------------------------------------------------------------------

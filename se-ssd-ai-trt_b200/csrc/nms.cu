@@ -144,24 +144,44 @@ __device__ __forceinline__ int frame_count(const NmsArgs& a, int b) {
 // infinity, so that every box gets a rank of its own and every rank is written.
 __device__ __forceinline__ float rank_score(float s) { return s != s ? -INFINITY : s; }
 
-// Kernel 1: rank by (score descending, row ascending) by counting, then the geometry of every ranked box.
+// Kernel 1: rank by (score descending, row ascending) by counting, a warp per box with the scores in shared memory, then
+// the geometry of every ranked box. Several blocks per frame, each with its share of the boxes. Also resets the
+// status block.
+constexpr int kRankBlocks = 8;
 __global__ void __launch_bounds__(kThreads)
-nms_rank_kernel(NmsArgs a) {
+nms_rank_kernel(NmsArgs a, uint32_t* status) {
     pdl_enter();
-    for (int b = blockIdx.x; b < a.batch; b += gridDim.x) {
+    extern __shared__ float s_score[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0)
+        for (int i = threadIdx.x; i < (int)(kStatusBytes / 4); i += kThreads) status[i] = 0u;
+    const int share = blockIdx.x % kRankBlocks;
+    for (int b = blockIdx.x / kRankBlocks; b < a.batch; b += gridDim.x / kRankBlocks) {
         const int n = frame_count(a, b);
         const float* bx = a.boxes + (size_t)b * a.max_box * 9;
-        for (int i = threadIdx.x; i < n; i += kThreads) {
-            const float si = rank_score(bx[i * 9 + 8]);
-            int rank = 0;
-            for (int j = 0; j < n; ++j) {
-                const float sj = rank_score(bx[j * 9 + 8]);
-                rank += (sj > si || (sj == si && j < i)) ? 1 : 0;
+        __syncthreads();
+        for (int j = threadIdx.x; j < n; j += kThreads) s_score[j] = rank_score(bx[j * 9 + 8]);
+        __syncthreads();
+        // box share + kRankBlocks * (warp + 8 q): a warp counts, 32 of its boxes are then placed by a lane each
+        for (int q0 = 0; share + kRankBlocks * (warp + (kThreads / 32) * q0) < n; q0 += 32) {
+            int my_rank = 0, my_box = -1;
+            for (int q = q0; q < q0 + 32; ++q) {
+                const int i = share + kRankBlocks * (warp + (kThreads / 32) * q);
+                if (i >= n) break;
+                const float si = s_score[i];
+                int ahead = 0;
+                for (int j = lane; j < n; j += 32) {
+                    const float sj = s_score[j];
+                    ahead += (sj > si || (sj == si && j < i)) ? 1 : 0;
+                }
+                ahead = __reduce_add_sync(0xFFFFFFFFu, ahead);
+                if (lane == q - q0) my_rank = ahead, my_box = i;
             }
-            a.order[(size_t)b * a.max_box + rank] = i;
-            const float* p = bx + i * 9;
+            if (my_box < 0) continue;
+            a.order[(size_t)b * a.max_box + my_rank] = my_box;
+            const float* p = bx + my_box * 9;
             const float x = p[0], y = p[1], w = p[3], l = p[4], yaw = p[6];
-            float* g = a.geom + ((size_t)b * a.max_box + rank) * kGeomFloats;
+            float* g = a.geom + ((size_t)b * a.max_box + my_rank) * kGeomFloats;
             g[0] = x, g[1] = y, g[2] = w, g[3] = l;
             g[4] = cosf(-yaw), g[5] = sinf(-yaw);
             g[6] = g[7] = 0.f;
@@ -230,7 +250,7 @@ nms_mask_kernel(NmsArgs a) {
 // lane and resolved with shuffles (no memory access between dependent steps), then the full mask rows of the
 // boxes kept in the block are ORed into the suppressed set with independent loads. All threads write the
 // kept boxes in rank order.
-constexpr int kReduceThreads = 256;
+constexpr int kReduceThreads = 512;
 __global__ void __launch_bounds__(kReduceThreads)
 nms_reduce_kernel(NmsArgs a, int smem_words) {
     pdl_enter();
@@ -265,12 +285,12 @@ nms_reduce_kernel(NmsArgs a, int smem_words) {
                 unsigned long long rem = __shfl_sync(0xFFFFFFFFu, removed, c);
                 unsigned long long keep = 0ull;
                 const int rows = min(64, n - c * 64);
-                for (int r = 0; r < rows; ++r) {           // every quantity here is uniform over the warp
-                    const unsigned long long row = __shfl_sync(0xFFFFFFFFu, r < 32 ? d0 : d1, r & 31);
-                    if (!((rem >> r) & 1ull)) {
-                        keep |= 1ull << r;
-                        rem |= row;
-                    }
+                const unsigned long long all = rows < 64 ? (1ull << rows) - 1ull : ~0ull;
+                // from one kept box to the next (every quantity here is uniform over the warp)
+                for (unsigned long long left = all & ~rem; left; left &= ~rem) {
+                    const int r = __ffsll((long long)left) - 1;
+                    keep |= 1ull << r;
+                    rem |= __shfl_sync(0xFFFFFFFFu, r < 32 ? d0 : d1, r & 31) | (1ull << r);
                 }
                 if (lane == c) keepw = keep;
                 // eight rows per round, so that eight loads are in flight before the first OR waits for one
@@ -368,9 +388,9 @@ int sessd_rotated_nms_enqueue(const sessd_nms_params* p, int batch, const void* 
     a.max_box = p->max_box_num;
     a.words = (int)words;
     a.thresh = p->nms_thresh;
-    SESSD_CUDA(cudaMemsetAsync(workspace, 0, kStatusBytes, stream));
     const int frames_grid = batch < persistent_grid(8) ? batch : persistent_grid(8);
-    SESSD_LAUNCH(nms_rank_kernel, frames_grid, kThreads, 0, stream, a);
+    const int rank_grid = (batch < persistent_grid(1) ? batch : persistent_grid(1)) * kRankBlocks;
+    SESSD_LAUNCH(nms_rank_kernel, rank_grid, kThreads, M * sizeof(float), stream, a, static_cast<uint32_t*>(workspace));
     const int64_t pair_blocks = ((int64_t)batch * M * words * 2 + kMaskWarps - 1) / kMaskWarps;
     const int pair_grid = (int)(pair_blocks < persistent_grid(8) ? pair_blocks : persistent_grid(8));
     SESSD_LAUNCH(nms_mask_kernel, pair_grid, kMaskWarps * 32, 0, stream, a);

@@ -8,7 +8,8 @@
 // writes past its outputs, filterBoxByScore.cu:275); and one entry point fuses both plugins, decoding only
 // the few anchors that pass the score threshold.
 //
-// Ordered compaction without inter-block waits: a count pass stores the number of passing anchors of
+// Ordered compaction: see box_filter_kernel. Frames with more anchors than that kernel takes (131,072) go through two
+// passes without inter-block waits: a count pass stores the number of passing anchors of
 // every 256-anchor chunk, the emit pass sums the counts of the chunks before its own and numbers its
 // rows with a block scan.
 #include "common.cuh"
@@ -93,6 +94,52 @@ struct FilterArgs {
     float threshold, dir_offset;
 };
 
+__device__ __forceinline__ void clear_box(const FilterArgs& a, size_t r) {
+#pragma unroll
+    for (int j = 0; j < 9; ++j) a.out_box[r * 9 + j] = 0.0f;
+    a.out_cls[r] = 0.0f;
+    a.out_iou[r] = 0.0f;
+    a.out_dir[r] = 0.0f;
+}
+
+// Writes row `row` of frame b: the box of anchor i, which passed with `score`. DECODE: `boxes` holds regression outputs
+// and the box is decoded here.
+template <bool DECODE>
+__device__ __forceinline__ void emit_box(const FilterArgs& a, const AnchorGeom& g, int b, int i, int row, float score) {
+    const size_t r = (size_t)b * a.max_box + row, e = (size_t)b * a.anchors + i;
+    const float q = __fmul_rn(__fadd_rn(__ldg(a.iou + e), 1.0f), 0.5f);          // filterBoxByScore.cu:284
+    a.out_iou[r] = q;
+    const float s = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(score, q), q), q), q);   // :288-289
+    a.out_cls[r] = s;
+    int best = 0;
+    float best_v = -1000000.0f;
+    for (int j = 0; j < a.dir_num; ++j) {           // last maximum wins (>=), row stride 2 (:295-302)
+        const float v = __ldg(a.dir + e * 2 + j);
+        if (v >= best_v) {
+            best_v = v;
+            best = j;
+        }
+    }
+    a.out_dir[r] = (float)best;
+    float t[7], bx[7];
+#pragma unroll
+    for (int j = 0; j < 7; ++j) t[j] = __ldg(a.boxes + e * 7 + j);
+    if (DECODE) {
+        decode_box(g, i, t, bx);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 7; ++j) bx[j] = t[j];
+    }
+    float* o = a.out_box + r * 9;
+#pragma unroll
+    for (int j = 0; j < 6; ++j) o[j] = bx[j];
+    const float rel = __fadd_rn(bx[6], -a.dir_offset);
+    const bool flip = (best == 1 && rel < 0.0f) || (best == 0 && rel > 0.0f);   // :307-315
+    o[6] = flip ? __fadd_rn(bx[6], kPiReference) : bx[6];
+    o[7] = 0.0f;
+    o[8] = s;
+}
+
 // Pass 1: passing anchors per chunk; also clears the outputs (FilterBoxByScorePlugin::enqueue clears
 // them with five memsets, filterBoxByScore.cu:353-371).
 __global__ void __launch_bounds__(kThreads)
@@ -109,11 +156,7 @@ box_count_kernel(FilterArgs a) {
     }
     const int64_t rows = (int64_t)a.batch * a.max_box;
     for (int64_t r = (int64_t)blockIdx.x * kThreads + threadIdx.x; r < rows; r += (int64_t)gridDim.x * kThreads) {
-#pragma unroll
-        for (int j = 0; j < 9; ++j) a.out_box[r * 9 + j] = 0.0f;
-        a.out_cls[r] = 0.0f;
-        a.out_iou[r] = 0.0f;
-        a.out_dir[r] = 0.0f;
+        clear_box(a, (size_t)r);
     }
 }
 
@@ -145,39 +188,86 @@ box_emit_kernel(FilterArgs a, AnchorGeom g) {
             if (passed > a.max_box) atomicOr(a.status, SESSD_STATUS_BOX_OVERFLOW);
         }
         if (!keep || idx >= a.max_box) continue;
-        const size_t r = (size_t)b * a.max_box + idx;
-        const float q = __fmul_rn(__fadd_rn(__ldg(a.iou + e), 1.0f), 0.5f);          // filterBoxByScore.cu:284
-        a.out_iou[r] = q;
-        const float s = __fmul_rn(__fmul_rn(__fmul_rn(__fmul_rn(score, q), q), q), q);   // :288-289
-        a.out_cls[r] = s;
-        int best = 0;
-        float best_v = -1000000.0f;
-        for (int j = 0; j < a.dir_num; ++j) {           // last maximum wins (>=), row stride 2 (:295-302)
-            const float v = __ldg(a.dir + e * 2 + j);
-            if (v >= best_v) {
-                best_v = v;
-                best = j;
-            }
-        }
-        a.out_dir[r] = (float)best;
-        float t[7], bx[7];
-#pragma unroll
-        for (int j = 0; j < 7; ++j) t[j] = __ldg(a.boxes + e * 7 + j);
-        if (DECODE) {
-            decode_box(g, i, t, bx);
-        } else {
-#pragma unroll
-            for (int j = 0; j < 7; ++j) bx[j] = t[j];
-        }
-        float* o = a.out_box + r * 9;
-#pragma unroll
-        for (int j = 0; j < 6; ++j) o[j] = bx[j];
-        const float rel = __fadd_rn(bx[6], -a.dir_offset);
-        const bool flip = (best == 1 && rel < 0.0f) || (best == 0 && rel > 0.0f);   // :307-315
-        o[6] = flip ? __fadd_rn(bx[6], kPiReference) : bx[6];
-        o[7] = 0.0f;
-        o[8] = s;
+        emit_box<DECODE>(a, g, b, i, idx, score);
     }
+}
+
+// Both passes in one launch, a cluster of eight blocks per frame: a warp takes consecutive anchors, 32 per step; the blocks exchange their totals through each other's shared memory, so that every passing anchor
+// knows its row. Rows past the count are cleared on the way. One frame of 70,400 anchors: 3.5 +
+// 4.0 us and a reset as separate launches, each a few microseconds of launch away from the next.
+constexpr int kFilterCluster = 8, kFilterThreads = 1024, kFilterSteps = 16;
+constexpr int kFilterMost = kFilterCluster * kFilterThreads * kFilterSteps;   // anchors per frame
+
+template <bool DECODE>
+__global__ void __cluster_dims__(kFilterCluster, 1, 1) __launch_bounds__(kFilterThreads, 1)
+box_filter_kernel(FilterArgs a, AnchorGeom g) {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // this block runs: its shared memory may be written
+    pdl_enter();
+    __shared__ int s_warp[kFilterThreads / 32];
+    __shared__ int s_total[kFilterCluster], s_block_total;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int rank = blockIdx.x % kFilterCluster, b = blockIdx.x / kFilterCluster;
+    const int per_warp = (a.anchors + kFilterCluster * (kFilterThreads / 32) * 32 - 1) /
+                         (kFilterCluster * (kFilterThreads / 32) * 32) * 32;   // consecutive anchors of a warp
+    const int first = (rank * (kFilterThreads / 32) + warp) * per_warp;
+    const float* cls = a.cls + (size_t)b * a.anchors;
+    float logit[kFilterSteps];   // all in flight
+#pragma unroll
+    for (int i = 0; i < kFilterSteps; ++i) {
+        const int e = first + i * 32 + lane;
+        logit[i] = i * 32 < per_warp && e < a.anchors ? __ldg(cls + e) : 0.0f;
+    }
+    int count = 0;
+#pragma unroll
+    for (int i = 0; i < kFilterSteps; ++i) {
+        if (i * 32 >= per_warp) break;
+        const bool in = first + i * 32 + lane < a.anchors;
+        count += __popc(__ballot_sync(0xFFFFFFFFu, in && sigmoid(logit[i]) >= a.threshold));
+    }
+    if (lane == 0) s_warp[warp] = count;
+    __syncthreads();
+    if (warp == 0) {
+        const int total = __reduce_add_sync(0xFFFFFFFFu, s_warp[lane]);
+        s_block_total = total;
+    }
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp == 0) {
+        const int total = s_block_total;
+        if (lane < kFilterCluster) {   // every block of the cluster learns this block's total
+            uint32_t remote;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(remote)
+                         : "r"((uint32_t)__cvta_generic_to_shared(&s_total[rank])), "r"(lane));
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(remote), "r"(total) : "memory");
+        }
+    }
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+    int idx = 0, passed = 0;
+#pragma unroll
+    for (int r = 0; r < kFilterCluster; ++r) {
+        if (r < rank) idx += s_total[r];
+        passed += s_total[r];
+    }
+    for (int w = 0; w < warp; ++w) idx += s_warp[w];
+    const int valid = passed < a.max_box ? passed : a.max_box;
+    if (rank == 0 && tid == 0) {
+        a.valid[b] = (uint32_t)valid;
+        if (a.batch == 1) a.status[0] = passed > a.max_box ? SESSD_STATUS_BOX_OVERFLOW : 0;
+        else if (passed > a.max_box) atomicOr(a.status, SESSD_STATUS_BOX_OVERFLOW);
+    }
+    if (count) {                 // few warps have any: the others are done
+        for (int i = 0; i * 32 < per_warp; ++i) {
+            const int e = first + i * 32 + lane;
+            const float score = e < a.anchors ? sigmoid(__ldg(cls + e)) : 0.0f;
+            const bool keep = e < a.anchors && score >= a.threshold;
+            const uint32_t votes = __ballot_sync(0xFFFFFFFFu, keep);
+            const int row = idx + __popc(votes & ((1u << lane) - 1u));
+            if (keep && row < a.max_box) emit_box<DECODE>(a, g, b, e, row, score);
+            idx += __popc(votes);
+        }
+    }
+    for (int r = valid + rank * kFilterThreads + tid; r < a.max_box; r += kFilterCluster * kFilterThreads)
+        clear_box(a, (size_t)b * a.max_box + r);
 }
 
 bool anchor_params_ok(const sessd_anchor_params* p) {
@@ -232,7 +322,16 @@ int run_filter(const sessd_anchor_params* ap, const sessd_filter_params* p, int 
     a.max_box = p->max_box_num;
     a.threshold = p->score_threshold;
     a.dir_offset = p->direction_offset;
-    SESSD_CUDA(cudaMemsetAsync(workspace, 0, kStatusBytes, stream));
+    // (a single frame's kernel stores the status word itself)
+    if (batch > 1 || a.anchors > kFilterMost) SESSD_CUDA(cudaMemsetAsync(workspace, 0, kStatusBytes, stream));
+    if (a.anchors <= kFilterMost) {
+        if (ap) {
+            SESSD_LAUNCH(box_filter_kernel<true>, batch * kFilterCluster, kFilterThreads, 0, stream, a, anchor_geom(*ap));
+        } else {
+            SESSD_LAUNCH(box_filter_kernel<false>, batch * kFilterCluster, kFilterThreads, 0, stream, a, AnchorGeom{});
+        }
+        return SESSD_OK;
+    }
     const int64_t items = (int64_t)batch * a.chunks;
     const int grid = (int)(items < persistent_grid(8) ? items : persistent_grid(8));
     SESSD_LAUNCH(box_count_kernel, grid, kThreads, 0, stream, a);
