@@ -186,7 +186,7 @@ struct BackboneWorkspace {
     void* voxel_feat;
     std::vector<int32_t*> coors, num;
     std::vector<BitGrid> bits;       // occupancy grids of the levels
-    std::vector<char> derived;       // the level's occupancy follows from its input level's grid
+    LevelChain chain;                // all derived levels, where one kernel can mark and one number them (count 0: it cannot)
     void* ones_base;
     size_t ones_bytes;
     std::vector<int32_t*> nbr_subm;
@@ -234,19 +234,22 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
         w->num[l] = bump.take<int32_t>(batch);
     }
     w->bits[0] = w->vgrid.grid;
-    w->derived.assign(bb->nlevels, 0);
+    w->chain = LevelChain{};
+    std::vector<ConvGeom> geoms;
     for (auto& L : bb->layers)
-        if (!L.p.subm) w->derived[L.level_out] = L.level_in > 0 && derivable_in_x(L.g) ? 1 : 0;
+        if (!L.p.subm) geoms.push_back(L.g);
+    if (w->grid0 && level_chain_usable(geoms.data(), (int)geoms.size())) w->chain.count = (int)geoms.size();
     // What one fill zeroes per call: the occupancy grids that rows mark their outputs in and the numbering state of the
-    // levels. A grid that is derived from its input level's grid is written whole.
+    // levels.
     const size_t tiles = (size_t)(maxV + 127) / 128;
     const size_t mask_words = batch * tiles;
-    size_t zero_bytes = (bb->layers.size() + 3) / 4 * 4 * sizeof(int);   // tile counters
+    const size_t counter_bytes = (bb->layers.size() + 1 + batch + 3) / 4 * 4 * sizeof(int);   // tile counters, chain counters
+    size_t zero_bytes = counter_bytes;
     w->scan.assign(bb->nlevels, ScanState{nullptr, nullptr});
     for (int l = 1; l < bb->nlevels; ++l) {
         w->bits[l] = bitgrid_shape(&bb->level_shape[3 * l]);
         zero_bytes += scan_state_bytes(w->bits[l].words, batch);
-        if (!w->derived[l]) zero_bytes += (size_t)batch * w->bits[l].words * sizeof(uint4);
+        zero_bytes += (size_t)batch * w->bits[l].words * sizeof(uint4);
     }
     char* zero = bump.take<char>(zero_bytes + 16);
     w->zero_base = zero;
@@ -257,11 +260,24 @@ void backbone_layout(Bump& bump, const sessd_backbone* bb, int batch, int max_po
         off += bytes;
         return p;
     };
-    w->tile_counter = reinterpret_cast<int*>(carve((bb->layers.size() + 3) / 4 * 4 * sizeof(int)));
+    w->tile_counter = reinterpret_cast<int*>(carve(counter_bytes));
     for (int l = 1; l < bb->nlevels; ++l) {
         const size_t bytes = (size_t)batch * w->bits[l].words * sizeof(uint4);
-        w->bits[l].rec = w->derived[l] ? bump.take<uint4>(bytes / sizeof(uint4)) : reinterpret_cast<uint4*>(carve(bytes));
+        w->bits[l].rec = reinterpret_cast<uint4*>(carve(bytes));
         w->scan[l] = scan_state_at(carve(scan_state_bytes(w->bits[l].words, batch)), w->bits[l].words, batch);
+    }
+    if (w->chain.count) {
+        LevelChain& ch = w->chain;
+        for (int l = 0; l < ch.count; ++l) {
+            ch.grid[l] = w->bits[l + 1];
+            ch.geom[l] = geoms[l];
+            ch.state[l] = w->scan[l + 1].state;
+            ch.coors[l] = w->coors[l + 1];
+            ch.num[l] = w->num[l + 1];
+        }
+        ch.ticket = reinterpret_cast<uint32_t*>(w->tile_counter ? w->tile_counter + bb->layers.size() : nullptr);
+        ch.done = ch.ticket ? ch.ticket + 1 : nullptr;
+        ch.totals = bump.take<int32_t>((size_t)batch * LevelChain::kMax);
     }
     w->nbr_layer.assign(bb->layers.size(), nullptr);
     w->order_subm.assign(bb->nlevels, nullptr);
@@ -553,7 +569,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
                                  ws.status, stream);
         if (rc) return rc;
         if (!subm) {
-            rc = launch_number_outputs(ws.out_bits, nullptr, g, batch, maxV, ws.scan, static_cast<int32_t*>(outputs[1]),
+            rc = launch_number_outputs(ws.out_bits, batch, maxV, ws.scan, static_cast<int32_t*>(outputs[1]),
                                        static_cast<int32_t*>(outputs[2]), ws.status, stream);
             if (rc) return rc;
         }
@@ -788,13 +804,9 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
     int rc = launch_prepare(fills, TailRows{}, (int64_t)batch * max_points <= 40000, stream);
     if (rc) return rc;
     // Coordinates first: voxels, the rows of every level, and all neighbour maps; then the convolutions.
-    const sessd_backbone::Layer* leaving0 = nullptr;   // the strided layer that leaves the voxeliser's level, if it can be
-    for (auto& L : bb->layers)                         // marked by the voxeliser
-        if (!L.p.subm && L.level_in == 0 && w.grid0 && derivable_in_x(L.g)) leaving0 = &L;
     if (w.grid0)
-        rc = voxel_grid_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
-                            static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vgrid,
-                            leaving0 ? leaving0->g : ConvGeom{}, leaving0 ? w.bits[1] : BitGrid{}, w.status, stream);
+        rc = voxel_grid_run(&bb->vp, batch, max_points, static_cast<const float*>(points),
+                            static_cast<const int32_t*>(points_size), w.coors[0], w.num[0], w.vgrid, w.chain, w.status, stream);
     else
         rc = voxelize_run(&bb->vp, batch, max_points, bb->dtype, static_cast<const float*>(points),
                           static_cast<const int32_t*>(points_size), w.voxel_feat, w.coors[0], w.num[0], w.vox,
@@ -817,7 +829,7 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         }
         j.in = w.bits[L.level_in];
         if (jobs.count == MapJobs::kMax) {
-            const int rc_jobs = launch_map_windows(jobs, batch, maxV, stream);
+            const int rc_jobs = launch_map_windows(jobs, batch, maxV, RowMeans{}, stream);
             if (rc_jobs) return rc_jobs;
             jobs.count = 0;
         }
@@ -837,18 +849,21 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
             if (rc) return rc;
             continue;
         }
-        const bool derived = w.derived[L.level_out] != 0;
-        if (!derived && &L != leaving0) {
+        if (!w.chain.count) {
             rc = launch_mark_outputs(w.coors[L.level_in], w.num[L.level_in], batch, maxV, L.g, w.bits[L.level_out], stream);
             if (rc) return rc;
+            rc = launch_number_outputs(w.bits[L.level_out], batch, maxV, w.scan[L.level_out], w.coors[L.level_out],
+                                       w.num[L.level_out], w.status, stream);
+            if (rc) return rc;
         }
-        rc = launch_number_outputs(w.bits[L.level_out], derived ? &w.bits[L.level_in] : nullptr, L.g, batch, maxV,
-                                   w.scan[L.level_out], w.coors[L.level_out], w.num[L.level_out], w.status, stream);
-        if (rc) return rc;
         rc = add_job(L, L.p.in_channel, w.nbr_layer[i], w.mask_layer[i], w.order_layer[i]);
         if (rc) return rc;
     }
-    rc = launch_map_windows(jobs, batch, maxV, stream);
+    RowMeans means{};
+    if (w.grid0)
+        means = RowMeans{static_cast<const float4*>(points), w.num[0], w.vgrid.lists, w.voxel_feat, max_points,
+                         bb->vp.max_points_per_voxel, bb->dtype == SESSD_F16 ? 1 : 0};
+    rc = launch_map_windows(jobs, batch, maxV, means, stream);
     if (rc) return rc;
     const void* cur = w.voxel_feat;
     for (size_t i = 0; i < bb->layers.size(); ++i) {

@@ -314,14 +314,36 @@ int launch_table_build(const int32_t* coors, const int32_t* voxel_num, int batch
                        const Table& t, int32_t* status, cudaStream_t stream);
 int launch_nbr_build(const int32_t* out_coors, const int32_t* out_num, int batch, int max_voxels, const ConvGeom& g,
                      const Table& in_table, int32_t* nbr, cudaStream_t stream);
-// Strided layers: set the bit of every candidate output, then number the set bits in (z, y, x) order. With derive_from
-// the bits are taken from the input level's grid instead (derivable_in_x must hold) and `out` needs no reset.
+// Strided layers: set the bit of every candidate output, then number the set bits in (z, y, x) order.
 int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batch, int max_voxels, const ConvGeom& g,
                         const BitGrid& out, cudaStream_t stream);
 bool derivable_in_x(const ConvGeom& g);
-int launch_number_outputs(const BitGrid& out, const BitGrid* derive_from, const ConvGeom& g, int batch, int max_voxels,
-                          const ScanState& scan, int32_t* out_coors, int32_t* out_num, int32_t* status,
-                          cudaStream_t stream);
+
+// The levels that a chain of strided layers makes from the voxeliser's level, when the occupancy of all of them follows
+// word by word from the voxeliser's grid (level_chain_usable): marked by one kernel and numbered by one.
+struct LevelChain {
+    static constexpr int kMax = 6;
+    int count;
+    BitGrid grid[kMax];
+    ConvGeom geom[kMax];                 // of the layer that makes the level
+    unsigned long long* state[kMax];     // numbering state
+    int32_t* coors[kMax];
+    int32_t* num[kMax];
+    uint32_t* ticket;
+    int32_t* totals;                     // [B][kMax] rows of a level before the cut at max_voxels
+    uint32_t* done;                      // [B] chunks numbered
+};
+bool level_chain_usable(const ConvGeom* geoms, int count);
+// What the voxeliser's point lists are made from (voxel_grid.cu).
+struct PointLists {
+    const int32_t* points_size;
+    const uint32_t* pt_key;
+    uint32_t* lists;
+    BitGrid grid;
+    int max_points, max_pts;
+};
+int launch_number_levels(const LevelChain& chain, int batch, int max_voxels, const PointLists& lists, int32_t* status,
+                         cudaStream_t stream);
 int launch_bucket_build(const int32_t* coors, const int32_t* voxel_num, int batch, int max_voxels, const int shape[3],
                         const Buckets& t, const ConvGeom* mark, const BitGrid& out, int32_t* status, cudaStream_t stream);
 // map_rows.cu: neighbour maps + tile masks of layers (any kernel up to 3x3x3, any stride) whose input level has an
@@ -348,7 +370,8 @@ struct MapJobs {
 // Everything of a job but its index; cin: input channels of the layers that read the map (the smallest).
 MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* out_num, int cin, int32_t* nbr,
                     uint32_t* tile_mask, int32_t* order);
-int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream);
+struct RowMeans;
+int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const RowMeans& means, cudaStream_t stream);
 int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream);
 int launch_tile_mask(const int32_t* nbr, const int32_t* out_num, int batch, int max_voxels, int kvol,
                      uint32_t* tile_mask, cudaStream_t stream);
@@ -418,6 +441,9 @@ int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out
                  const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelWorkspace& w,
                  bool zero_tail, cudaStream_t stream);
 
+int launch_number_outputs(const BitGrid& out, int batch, int max_voxels, const ScanState& scan, int32_t* out_coors,
+                          int32_t* out_num, int32_t* status, cudaStream_t stream);
+
 // voxel_grid.cu: rows in (z, y, x) order and an occupancy grid of the level
 struct VoxelGrid {
     BitGrid grid;
@@ -428,13 +454,22 @@ struct VoxelGrid {
     void* zero_base;      // to be zero before a call
     size_t zero_bytes;
 };
-// marks (rec != nullptr): the grid of the next level, in which the outputs of the strided layer `geom` are marked
 bool voxel_grid_usable(const sessd_voxel_params* p, int max_points, const int level_shape[3]);
 void voxel_grid_layout(Bump& bump, const sessd_voxel_params* p, const int level_shape[3], int batch, int max_points,
                        VoxelGrid* w);
-int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
-                   const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelGrid& w,
-                   const ConvGeom& geom, const BitGrid& marks, int32_t* status, cudaStream_t stream);
+// Points -> rows, their point lists, and the levels of `chain` (count 0: none). The rows' means follow with
+// launch_map_windows.
+int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, const float* points, const int32_t* points_size,
+                   int32_t* coors, int32_t* voxel_num, const VoxelGrid& w, const LevelChain& chain, int32_t* status,
+                   cudaStream_t stream);
+// What launch_map_windows does besides: the means of the voxeliser's rows (points == nullptr: nothing).
+struct RowMeans {
+    const float4* points;
+    const int32_t* voxel_num;
+    const uint32_t* lists;
+    void* voxels;
+    int max_points, max_pts, half;
+};
 
 struct sessd_conv_weights_impl {
     void* w;        // device, [kvol][Cin][Cout] in dtype

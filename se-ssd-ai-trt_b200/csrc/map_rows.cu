@@ -18,6 +18,7 @@
 // maps another 0.9 through a table and an input-stationary scatter.
 #include "fill.cuh"
 #include "rulebook.cuh"
+#include "voxel.cuh"
 
 namespace sessd {
 
@@ -225,8 +226,23 @@ __device__ __forceinline__ uint32_t map_entries(const Index& in, const MapJob& j
     }
 }
 
+template <typename T>
+__device__ __forceinline__ void row_means(const RowMeans& m, T* voxels, int batch, int max_voxels, int block, int blocks) {
+    const int chunks = (m.max_points + kMapThreads - 1) / kMapThreads;   // rows never outnumber points
+    for (int it = block; it < batch * chunks; it += blocks) {
+        const int b = it / chunks;
+        const int row = (it - b * chunks) * kMapThreads + threadIdx.x;
+        if (row >= __ldg(m.voxel_num + b)) continue;
+        uint32_t pi[kMaxPointsPerVoxel];
+        list_load(m.lists + ((size_t)b * m.max_points + row) * m.max_pts, m.max_pts, pi);
+        int cnt;
+        const float4 v = voxel_mean(m.points + (size_t)b * m.max_points, m.max_pts, pi, &cnt);
+        store_voxel(voxels, (size_t)b * max_voxels + row, v.x, v.y, v.z, v.w);
+    }
+}
+
 __global__ void __launch_bounds__(kMapThreads, 2)
-map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame) {
+map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame, RowMeans means) {
     pdl_enter();
     extern __shared__ __align__(16) uint8_t map_smem[];
     MapShared& s = *reinterpret_cast<MapShared*>(map_smem);
@@ -346,6 +362,12 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
                 if ((m >> k) & 1u) out[k * kNbrRun] = p < n ? s.ids[k][r] : -1;
         }
     }
+    // Beside the maps: the means of the voxeliser's rows. From the last block down, which has the fewest windows.
+    if (means.points) {
+        const int block = (int)(gridDim.x - 1 - blockIdx.x);
+        if (means.half) row_means(means, static_cast<__half*>(means.voxels), batch, max_voxels, block, gridDim.x);
+        else row_means(means, static_cast<float*>(means.voxels), batch, max_voxels, block, gridDim.x);
+    }
 }
 
 // Maps through a table: rows as a caller (or the voxeliser, in point order) numbered them. Every line is one or two
@@ -400,8 +422,8 @@ MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* 
     return j;
 }
 
-int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, cudaStream_t stream) {
-    if (jobs.count == 0) return SESSD_OK;
+int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const RowMeans& means, cudaStream_t stream) {
+    if (jobs.count == 0 && !means.points) return SESSD_OK;
     static_assert(2 * (sizeof(MapShared) + 1024) <= 228 * 1024, "two windows per SM");
     // the attribute belongs to the device's context: set it once per device (repeating it is harmless)
     static std::atomic<uint64_t> configured{0};
@@ -412,10 +434,10 @@ int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, cudaStrea
         SESSD_CUDA(cudaFuncSetAttribute(map_windows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MapShared)));
         configured.fetch_or(bit, std::memory_order_release);
     }
-    const int64_t items = (int64_t)jobs.count * batch * ((max_voxels + kWindow - 1) / kWindow);
+    const int64_t items = (int64_t)(jobs.count > 0 ? jobs.count : 1) * batch * ((max_voxels + kWindow - 1) / kWindow);
     const int most = persistent_grid(2);
     SESSD_LAUNCH(map_windows_kernel, (int)(items < most ? items : most), kMapThreads, sizeof(MapShared), stream, jobs, batch,
-                 max_voxels, (max_voxels + 127) / 128);
+                 max_voxels, (max_voxels + 127) / 128, means);
     return SESSD_OK;
 }
 

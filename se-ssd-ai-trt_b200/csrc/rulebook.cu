@@ -24,6 +24,7 @@
 //   - coordinates handed in by a caller (the stand-alone plugin entry points) go into a flat table.
 #include "rulebook.cuh"
 #include "scan.cuh"
+#include "voxel.cuh"
 
 namespace sessd {
 
@@ -204,87 +205,47 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
     }
 }
 
-// Output cells of word w of an output level from the occupancy of its input level: a cell is an output when any cell of
-// its receptive field is occupied, which is the set that marking every input row's candidates gives (the truncating
-// divisions of sparseConv3dlayer.cu:339-348 drop no valid candidate). In x the two cases of derivable_in_x; z and y are
-// free. The input words of all lines are read side by side and ORed before the bits are spread.
-__device__ __forceinline__ unsigned long long derive_word(const BitGrid& in, const BitGrid& out, const ConvGeom& g, int b, int w) {
-    const int row = w / out.xw, wx = w - row * out.xw;
-    const int z = row / out.Y, y = row - z * out.Y;
-    const bool same = g.K[2] == 1;                  // kernel 1, stride 1: the word itself; else kernel 3, stride 2, padding 1
-    const int first = same ? wx : 2 * wx;
-    unsigned long long before = 0ull, lo = 0ull, hi = 0ull;
-#pragma unroll
-    for (int kz = 0; kz < 3; ++kz) {
-        const int iz = z * g.S[0] - g.P[0] + kz;
-        if (kz >= g.K[0] || iz < 0 || iz >= in.Z) continue;
-#pragma unroll
-        for (int ky = 0; ky < 3; ++ky) {
-            const int iy = y * g.S[1] - g.P[1] + ky;
-            if (ky >= g.K[1] || iy < 0 || iy >= in.Y) continue;
-            // a record is 16 bytes: bits first
-            const unsigned long long* at =
-                reinterpret_cast<const unsigned long long*>(in.rec + (size_t)b * in.words) + 2 * ((size_t)iz * in.Y + iy) * in.xw;
-            if (first < in.xw) lo |= __ldg(at + 2 * first);
-            if (!same) {
-                if (first > 0) before |= __ldg(at + 2 * (first - 1));
-                if (first + 1 < in.xw) hi |= __ldg(at + 2 * (first + 1));
-            }
-        }
-    }
-    unsigned long long bits = lo;
-    if (!same) {
-        // output x has the inputs 2x - 1, 2x, 2x + 1
-        const unsigned long long even = (unsigned long long)even_bits(lo) | (unsigned long long)even_bits(hi) << 32;
-        const unsigned long long odd = (unsigned long long)even_bits(lo >> 1) | (unsigned long long)even_bits(hi >> 1) << 32;
-        bits = even | odd | (odd << 1) | (before >> 63);
-    }
-    const int x0 = wx << 6;
-    if (x0 + 64 > out.X) bits &= x0 < out.X ? (1ull << (out.X - x0)) - 1ull : 0ull;   // cells past the line's end
-    return bits;
-}
-
-// Numbers the occupied cells of every frame's output level in word order (= (z, y, x) order): completes the records
-// (bits, rows before the word), writes the output coordinates (sparseConv3dlayer.cu:436-441 writes them per pair) and the
-// frame's row count. The bits come from the records (marked by an earlier kernel) or, with DERIVE, from the input
-// level's records; then the grid needs no reset either. Rows past max_voxels are dropped (their bits too, so that the
-// next level does not see them) and reported. One thread per word; a warp then writes its words' coordinates one word
-// at a time, a lane per cell. Two kernels (count, then prefix and emit with a serial loop over a thread's bits) took 3.5 +
-// 18 us per level of a 20,000-point frame.
-template <bool DERIVE>
-__global__ void __launch_bounds__(kThreads)
-number_outputs_kernel(BitGrid g, BitGrid in, ConvGeom geom, int batch, int max_voxels, ScanState scan,
-                      int4* __restrict__ out_coors, int32_t* __restrict__ out_num, int32_t* status) {
-    pdl_enter();
+// Numbers one chunk (kThreads x WORDS words) of one frame of a level whose bits are set, in word order (= (z, y, x)
+// order): completes the records (rows before the word), writes the output coordinates (sparseConv3dlayer.cu:436-441 writes
+// them per pair) and, with the last chunk, the row count. Rows past max_voxels are dropped (their bits too, so that the
+// next level does not see them) and reported. A warp writes its words' coordinates one word at a time, a lane per cell.
+// Returns the running total with the chunk.
+template <int WORDS>
+__device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long* state, int b, int c, int chunks, int max_voxels,
+                                            int4* __restrict__ out_coors, int32_t* __restrict__ out_num, int32_t* status) {
     const int lane = threadIdx.x & 31;
-    const int chunks = scan_chunks(g.words), items = batch * chunks;
-    for (int t = scan_ticket(scan.ticket, items); t >= 0; t = scan_ticket(scan.ticket, items)) {
-        const int c = t / batch, b = t - c * batch;
-        const int w = c * kThreads + threadIdx.x;
-        uint4* rec = g.rec + (size_t)b * g.words;
-        unsigned long long bits = 0ull;
-        if (w < g.words) bits = DERIVE ? derive_word(in, g, geom, b, w) : rec_bits(rec[w]);
-        int end;
-        const int id = scan_position(scan.state + (size_t)b * chunks, c, __popcll(bits), &end, status);
-        if (c == chunks - 1 && threadIdx.x == 0) {
-            out_num[b] = end > max_voxels ? max_voxels : end;
-            if (end > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
-        }
-        if (id + __popcll(bits) > max_voxels) {          // keep the first max_voxels - id cells
+    const int w0 = (c * kThreads + threadIdx.x) * WORDS;
+    uint4* rec = g.rec + (size_t)b * g.words;
+    unsigned long long bits[WORDS];
+    int count = 0;
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        bits[i] = w0 + i < g.words ? rec_bits(rec[w0 + i]) : 0ull;
+        count += __popcll(bits[i]);
+    }
+    int end;
+    int id = scan_position(state, c, count, &end, status);
+    if (c == chunks - 1 && threadIdx.x == 0) {
+        out_num[b] = end > max_voxels ? max_voxels : end;
+        if (end > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
+    }
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) {
+        if (id + __popcll(bits[i]) > max_voxels) {       // keep the first max_voxels - id cells
             int keep = max_voxels - id > 0 ? max_voxels - id : 0;
             unsigned long long kept = 0ull;
-            for (unsigned long long rem = bits; rem && keep; --keep) {
+            for (unsigned long long rem = bits[i]; rem && keep; --keep) {
                 kept |= rem & (0ull - rem);
                 rem &= rem - 1ull;
             }
-            bits = kept;
+            bits[i] = kept;
         }
-        if (w < g.words) rec[w] = make_uint4((uint32_t)bits, (uint32_t)(bits >> 32), (uint32_t)id, 0u);
-        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, bits != 0ull); todo; todo &= todo - 1u) {
+        if (w0 + i < g.words) rec[w0 + i] = make_uint4((uint32_t)bits[i], (uint32_t)(bits[i] >> 32), (uint32_t)id, 0u);
+        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, bits[i] != 0ull); todo; todo &= todo - 1u) {
             const int src = __ffs((int)todo) - 1;
-            const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits, src);
+            const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits[i], src);
             const int id0 = __shfl_sync(0xFFFFFFFFu, id, src);
-            const int word = w - lane + src;
+            const int word = w0 + i + (src - lane) * WORDS;
             const int row = word / g.xw;                 // z * Y + y
             const int x0 = (word - row * g.xw) << 6;
             const int z = row / g.Y, y = row - z * g.Y;
@@ -293,6 +254,102 @@ number_outputs_kernel(BitGrid g, BitGrid in, ConvGeom geom, int batch, int max_v
             if ((v_lo >> lane) & 1u) dst[__popc(v_lo & below)] = make_int4(b, z, y, x0 + lane);
             if ((v_hi >> lane) & 1u) dst[__popc(v_lo) + __popc(v_hi & below)] = make_int4(b, z, y, x0 + 32 + lane);
         }
+        id += __popcll(bits[i]);
+    }
+    return end;
+}
+
+__global__ void __launch_bounds__(kThreads)
+number_outputs_kernel(BitGrid g, int batch, int max_voxels, ScanState scan, int4* __restrict__ out_coors,
+                      int32_t* __restrict__ out_num, int32_t* status) {
+    pdl_enter();
+    const int chunks = scan_chunks(g.words), items = batch * chunks;
+    for (int t = scan_first(scan.ticket, items, gridDim.x); t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
+        const int c = t / batch, b = t - c * batch;
+        number_chunk<1>(g, scan.state + (size_t)b * chunks, b, c, chunks, max_voxels, out_coors, out_num, status);
+    }
+}
+
+// The levels below a level that had more rows than max_voxels must not see the rows it dropped: their grids are marked and
+// numbered again from the rows that are left. By one block, for a frame that has lost rows anyway.
+__device__ __noinline__ void renumber_levels(const LevelChain& chain, int b, int l0, int max_voxels, int32_t* status) {
+    for (int l = l0; l < chain.count; ++l) {
+        const BitGrid& g = chain.grid[l];
+        uint4* rec = g.rec + (size_t)b * g.words;
+        for (int w = threadIdx.x; w < g.words; w += kThreads) __stcg(rec + w, make_uint4(0u, 0u, 0u, 0u));
+        __threadfence();
+        __syncthreads();
+        const int4* in = reinterpret_cast<const int4*>(chain.coors[l - 1]) + (size_t)b * max_voxels;
+        const int n = __ldcg(chain.num[l - 1] + b);
+        for (int i = threadIdx.x; i < n; i += kThreads) mark_row(__ldcg(in + i), b, chain.geom[l], g);
+        __threadfence();
+        __syncthreads();
+        int4* out = reinterpret_cast<int4*>(chain.coors[l]) + (size_t)b * max_voxels;
+        int base = 0;
+        for (int w0 = 0; w0 < g.words; w0 += kThreads) {
+            const int w = w0 + threadIdx.x;
+            unsigned long long v = w < g.words ? rec_bits(__ldcg(rec + w)) : 0ull;
+            int total;
+            int id = base + block_exclusive_scan(__popcll(v), &total);
+            const int id0 = id;
+            unsigned long long kept = 0ull;
+            const int row = w / g.xw, z = row / g.Y;
+            for (; v && id < max_voxels; ++id) {
+                const int bit = __ffsll((long long)v) - 1;
+                v &= v - 1ull;
+                kept |= 1ull << bit;
+                __stcg(out + id, make_int4(b, z, row - z * g.Y, ((w - row * g.xw) << 6) + bit));
+            }
+            if (w < g.words) __stcg(rec + w, make_uint4((uint32_t)kept, (uint32_t)(kept >> 32), (uint32_t)id0, 0u));
+            base += total;
+        }
+        if (threadIdx.x == 0) {
+            __stcg(chain.num[l] + b, base > max_voxels ? max_voxels : base);
+            if (base > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
+        }
+        __threadfence();
+        __syncthreads();
+    }
+}
+
+// All levels of a chain in one launch (blocks 0 .. number_blocks - 1), and beside it the point lists of the voxeliser's
+// rows (the other blocks), which depend on the same kernel and on nothing here.
+template <int WORDS>
+__global__ void __launch_bounds__(kThreads, 5)   // (renumber_levels would take 104 registers; it may spill)
+number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int max_voxels, int number_blocks, PointLists lists,
+                     int32_t* status) {
+    pdl_enter();
+    if ((int)blockIdx.x >= number_blocks) {
+        push_points(lists, batch, blockIdx.x - number_blocks, gridDim.x - number_blocks);
+        return;
+    }
+    __shared__ int s_last;
+    int per_frame = 0;
+    for (int l = 0; l < chain.count; ++l) per_frame += scan_chunks((chain.grid[l].words + WORDS - 1) / WORDS);
+    const int items = batch * per_frame;
+    for (int t = scan_first(chain.ticket, items, number_blocks); t >= 0; t = scan_next(chain.ticket, items, number_blocks)) {
+        const int b = t % batch;
+        int c = t / batch, l = 0, chunks = 0;
+        for (;; ++l) {
+            chunks = scan_chunks((chain.grid[l].words + WORDS - 1) / WORDS);
+            if (c < chunks) break;
+            c -= chunks;
+        }
+        const int end = number_chunk<WORDS>(chain.grid[l], chain.state[l] + (size_t)b * chunks, b, c, chunks, max_voxels,
+                                            reinterpret_cast<int4*>(chain.coors[l]), chain.num[l], status);
+        if (c == chunks - 1 && threadIdx.x == 0) chain.totals[b * LevelChain::kMax + l] = end;
+        // the frame's last block looks whether a level lost rows
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) s_last = atomicAdd(chain.done + b, 1u) == (uint32_t)(per_frame - 1);
+        __syncthreads();
+        if (!s_last) continue;
+        __threadfence();
+        for (int k = 0; k + 1 < chain.count; ++k)
+            if (__ldcg(chain.totals + b * LevelChain::kMax + k) > max_voxels) {
+                renumber_levels(chain, b, k + 1, max_voxels, status);
+                break;
+            }
     }
 }
 
@@ -405,17 +462,40 @@ bool derivable_in_x(const ConvGeom& g) {
     return (g.K[2] == 3 && g.S[2] == 2 && g.P[2] == 1) || (g.K[2] == 1 && g.S[2] == 1 && g.P[2] == 0);
 }
 
-int launch_number_outputs(const BitGrid& out, const BitGrid* derive_from, const ConvGeom& g, int batch, int max_voxels,
-                          const ScanState& scan, int32_t* out_coors, int32_t* out_num, int32_t* status,
-                          cudaStream_t stream) {
+bool level_chain_usable(const ConvGeom* geoms, int count) {
+    int halvings = 0;
+    for (int l = 0; l < count; ++l) {
+        if (!derivable_in_x(geoms[l])) return false;
+        halvings += geoms[l].K[2] == 3 ? 1 : 0;
+    }
+    return count >= 1 && count <= LevelChain::kMax && halvings <= 6;   // a word's first cell stays even before each of them
+}
+
+int launch_number_outputs(const BitGrid& out, int batch, int max_voxels, const ScanState& scan, int32_t* out_coors,
+                          int32_t* out_num, int32_t* status, cudaStream_t stream) {
     const int64_t items = (int64_t)batch * scan_chunks(out.words);
     const int grid = (int)(items < persistent_grid(8) ? items : persistent_grid(8));
-    if (derive_from)
-        SESSD_LAUNCH(number_outputs_kernel<true>, grid, kThreads, 0, stream, out, *derive_from, g, batch, max_voxels, scan,
-                     reinterpret_cast<int4*>(out_coors), out_num, status);
-    else
-        SESSD_LAUNCH(number_outputs_kernel<false>, grid, kThreads, 0, stream, out, BitGrid{}, g, batch, max_voxels, scan,
-                     reinterpret_cast<int4*>(out_coors), out_num, status);
+    SESSD_LAUNCH(number_outputs_kernel, grid, kThreads, 0, stream, out, batch, max_voxels, scan,
+                 reinterpret_cast<int4*>(out_coors), out_num, status);
+    return SESSD_OK;
+}
+
+// One word per thread while there is a block for every chunk (a single frame: short chains), four above (fewer rounds of
+// a persistent grid).
+int launch_number_levels(const LevelChain& chain, int batch, int max_voxels, const PointLists& lists, int32_t* status,
+                         cudaStream_t stream) {
+    int64_t items = 0;
+    for (int l = 0; l < chain.count; ++l) items += (int64_t)batch * scan_chunks(chain.grid[l].words);
+    const int most = persistent_grid(6);
+    const int64_t point_chunks = (int64_t)batch * scan_chunks(lists.max_points);
+    const int list_blocks = (int)(point_chunks < persistent_grid(2) ? point_chunks : persistent_grid(2));
+    if (items <= most) {
+        SESSD_LAUNCH(number_levels_kernel<1>, (int)items + list_blocks, kThreads, 0, stream, chain, batch, max_voxels, (int)items,
+                     lists, status);
+    } else {
+        SESSD_LAUNCH(number_levels_kernel<4>, most + list_blocks, kThreads, 0, stream, chain, batch, max_voxels, most, lists,
+                     status);
+    }
     return SESSD_OK;
 }
 

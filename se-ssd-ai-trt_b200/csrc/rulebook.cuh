@@ -118,37 +118,37 @@ __device__ __forceinline__ uint32_t even_bits(unsigned long long v) {
     return (uint32_t)(v | (v >> 16));
 }
 
-// Marks the candidate outputs of all cells of word (z, y, wx) of an input level, given its bits: the union of mark_row
-// over them. The layer must be derivable_in_x: kernel 1 and stride 1 in x (outputs are the cells themselves) or kernel 3,
-// stride 2, padding 1 (output x has the inputs 2x - 1, 2x, 2x + 1).
-__device__ __forceinline__ void mark_word(unsigned long long bits, int z, int y, int wx, int b, const ConvGeom& g,
-                                          const BitGrid& out) {
-    unsigned long long m0 = bits, m1 = 0ull;   // bits of output word w0 and of the one after it
-    int w0 = wx;
-    if (g.K[2] == 3) {
-        const unsigned long long even = even_bits(bits), odd = even_bits(bits >> 1);
-        const unsigned long long spread = even | odd | (odd << 1);   // 33 bits, from output 32 wx on
-        w0 = wx >> 1;
-        m0 = wx & 1 ? spread << 32 : spread;
-        m1 = wx & 1 ? spread >> 32 : 0ull;
-    }
-    const int x0 = w0 << 6;
-    if (x0 + 64 > out.X) m0 &= x0 < out.X ? (1ull << (out.X - x0)) - 1ull : 0ull;
-    if (x0 + 64 >= out.X) m1 = 0ull;               // (m1 is at most the next word's first bit)
-    const int c[2] = {z, y};
-#pragma unroll
-    for (int ez = 0; ez < 3; ++ez) {
-        const int oz = div_trunc(c[0] + g.P[0], g.S[0]) - ez, kz = c[0] - oz * g.S[0] + g.P[0];
-        if (ez >= g.span_max[0] || oz < 0 || oz >= out.Z || kz < 0 || kz >= g.K[0]) continue;
-#pragma unroll
-        for (int ey = 0; ey < 3; ++ey) {
-            const int oy = div_trunc(c[1] + g.P[1], g.S[1]) - ey, ky = c[1] - oy * g.S[1] + g.P[1];
-            if (ey >= g.span_max[1] || oy < 0 || oy >= out.Y || ky < 0 || ky >= g.K[1]) continue;
-            unsigned long long* rec = reinterpret_cast<unsigned long long*>(
-                out.rec + (size_t)b * out.words + ((size_t)oz * out.Y + oy) * out.xw + w0);
-            if ((*reinterpret_cast<volatile unsigned long long*>(rec) & m0) != m0) atomicOr(rec, m0);
-            if (m1 && (*reinterpret_cast<volatile unsigned long long*>(rec + 2) & m1) != m1) atomicOr(rec + 2, m1);
+// Sets the bits `lo` of the grid word at rec and `hi` of the next one. The words are read first, through L1: a stale copy
+// only costs an atomic that changes nothing, and most bits have been set by a neighbouring word long before.
+__device__ __forceinline__ void set_bits(uint4* rec, unsigned long long lo, unsigned long long hi) {
+    unsigned long long* p = reinterpret_cast<unsigned long long*>(rec);
+    if ((*p & lo) != lo) atomicOr(p, lo);
+    if (hi && (p[2] & hi) != hi) atomicOr(p + 2, hi);
+}
+
+// Marks, in the grids of all levels of a chain, the outputs of the cells of word (z, y, wx) of the voxeliser's level,
+// given its bits. Per axis the outputs of a range of input cells are a range of output cells (sparseConv3dlayer.cu:339-348
+// enumerates the same cells), so a word reaches at most two or three lines per axis of every level; in x the layers are
+// those of derivable_in_x: kernel 1 and stride 1 (outputs are the cells themselves) or kernel 3, stride 2, padding 1
+// (output x has the inputs 2x - 1, 2x, 2x + 1).
+__device__ __forceinline__ void mark_levels(unsigned long long bits, int z, int y, int wx, int b, const LevelChain& chain) {
+    int z0 = z, z1 = z, y0 = y, y1 = y, off = wx << 6;   // lines, and the cell of the lowest bit (even before every halving)
+    for (int l = 0; l < chain.count && bits; ++l) {
+        const ConvGeom& g = chain.geom[l];
+        const BitGrid& out = chain.grid[l];
+        z0 = max(z0 + g.P[0] - g.K[0] + g.S[0], 0) / g.S[0], z1 = min((z1 + g.P[0]) / g.S[0], out.Z - 1);
+        y0 = max(y0 + g.P[1] - g.K[1] + g.S[1], 0) / g.S[1], y1 = min((y1 + g.P[1]) / g.S[1], out.Y - 1);
+        if (g.K[2] == 3) {
+            const unsigned long long even = even_bits(bits), odd = even_bits(bits >> 1);
+            bits = even | odd | (odd << 1);
+            off >>= 1;
         }
+        if (off + 64 > out.X) bits &= off < out.X ? (1ull << (out.X - off)) - 1ull : 0ull;
+        const int sh = off & 63;
+        const unsigned long long lo = bits << sh, hi = sh ? bits >> (64 - sh) : 0ull;
+        uint4* rec = out.rec + (size_t)b * out.words + (off >> 6);
+        for (int oz = z0; oz <= z1; ++oz)
+            for (int oy = y0; oy <= y1; ++oy) set_bits(rec + (oz * out.Y + oy) * out.xw, lo, hi);
     }
 }
 

@@ -12,13 +12,13 @@
 //   1. every point finds its cell and sets its word's bit in the top level;
 //   2. the words are numbered (one-pass scan) and their records cleared;
 //   3. every point sets its cell's bit in its word;
-//   4. the rows are numbered (one-pass scan): coordinates, row count, empty point lists; every word marks the outputs of
-//      its cells in the next level's grid, a few atomics for up to 64 cells;
-//   5. every point pushes its index through its row's ascending list of the max_points_per_voxel smallest indices (a
+//   4. the rows are numbered (one-pass scan): coordinates, row count, empty point lists; every word also marks the cells
+//      that it reaches in the grids of all further levels, a few atomics for up to 64 cells;
+//   5. (one launch with the numbering of the further levels) every point pushes its index through its row's ascending list of the max_points_per_voxel smallest indices (a
 //      cascade of atomicMin, so the list does not depend on timing);
-//   6. every row averages its listed points, summed in ascending index order.
-// What bounds it: the chain of dependent L2 reads of six short kernels for one frame, the random 16-byte point reads of
-// pass 6 and the atomics of pass 5 for a batch.
+//   6. (one launch with the neighbour maps) every row averages its listed points, summed in ascending index order.
+// What bounds it: the chain of dependent L2 reads of short kernels for one frame, the atomics of pass 5 and the random
+// 16-byte point reads of pass 6 for a batch.
 #include "rulebook.cuh"
 #include "scan.cuh"
 #include "voxel.cuh"
@@ -27,20 +27,7 @@ namespace sessd {
 
 namespace {
 
-// Calls fn(frame, point) for every point of the batch. A point's key is word << 6 | bit of its cell, kEmpty outside the
-// range.
-template <class Fn>
-__device__ __forceinline__ void for_points(const int32_t* __restrict__ points_size, int batch, int max_points, Fn fn) {
-    const int chunks = (max_points + kThreads - 1) / kThreads;
-    const int items = batch * chunks;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int b = it / chunks;
-        const int p = (it - b * chunks) * kThreads + threadIdx.x;
-        int n = __ldg(points_size + b);
-        n = n > max_points ? max_points : n;
-        if (p < n) fn(b, p);
-    }
-}
+// A point's key is word << 6 | bit of its cell, kEmpty outside the range.
 
 __device__ __forceinline__ void set_bit(uint4* rec, int bit) {   // of a record's first 8 bytes
     unsigned long long* word = reinterpret_cast<unsigned long long*>(rec);
@@ -52,7 +39,7 @@ __global__ void __launch_bounds__(kThreads)
 point_mark_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch, int max_points,
                   VoxGeom g, BitGrid grid, uint32_t* __restrict__ pt_key) {
     pdl_enter();
-    for_points(points_size, batch, max_points, [&](int b, int p) {
+    for_points(points_size, batch, max_points, blockIdx.x, gridDim.x, [&](int b, int p) {
         const float4 pt = __ldg(&points[(size_t)b * max_points + p]);
         int ix, iy, iz;
         uint32_t key = kEmpty;
@@ -70,7 +57,7 @@ number_words_kernel(BitGrid grid, int batch, ScanState scan, int32_t* __restrict
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int chunks = scan_chunks(grid.top_words), items = batch * chunks;
-    for (int t = scan_ticket(scan.ticket, items); t >= 0; t = scan_ticket(scan.ticket, items)) {
+    for (int t = scan_first(scan.ticket, items, gridDim.x); t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = t / batch, b = t - c * batch;
         const int w = c * kThreads + threadIdx.x;
         uint4* top = grid.top + (size_t)b * grid.top_words;
@@ -92,17 +79,11 @@ number_words_kernel(BitGrid grid, int batch, ScanState scan, int32_t* __restrict
     }
 }
 
-// Number of the record of an occupied word.
-__device__ __forceinline__ int word_id(const BitGrid& grid, int b, uint32_t word) {
-    const uint4 t = __ldg(grid.top + (size_t)b * grid.top_words + (word >> 6));
-    return (int)t.z + __popcll(rec_bits(t) & ((1ull << (word & 63)) - 1ull));
-}
-
 __global__ void __launch_bounds__(kThreads)
 point_bits_kernel(const int32_t* __restrict__ points_size, int batch, int max_points, BitGrid grid,
                   const uint32_t* __restrict__ pt_key) {
     pdl_enter();
-    for_points(points_size, batch, max_points, [&](int b, int p) {
+    for_points(points_size, batch, max_points, blockIdx.x, gridDim.x, [&](int b, int p) {
         const uint32_t key = __ldg(pt_key + (size_t)b * max_points + p);
         if (key != kEmpty) set_bit(grid.rec + (size_t)b * grid.words + word_id(grid, b, key >> 6), key & 63);
     });
@@ -111,11 +92,11 @@ point_bits_kernel(const int32_t* __restrict__ points_size, int batch, int max_po
 __global__ void __launch_bounds__(kThreads)
 number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch, int max_voxels, int max_points, int max_pts,
                    ScanState scan, int4* __restrict__ coors, int32_t* __restrict__ voxel_num,
-                   uint32_t* __restrict__ lists, ConvGeom geom, BitGrid marks, int32_t* status) {
+                   uint32_t* __restrict__ lists, const __grid_constant__ LevelChain chain, int32_t* status) {
     pdl_enter();
     const int lane = threadIdx.x & 31;
     const int chunks = scan_chunks(grid.words), items = batch * chunks;
-    for (int t = scan_ticket(scan.ticket, items); t >= 0; t = scan_ticket(scan.ticket, items)) {
+    for (int t = scan_first(scan.ticket, items, gridDim.x); t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = t / batch, b = t - c * batch;
         const int n = __ldg(word_num + b), used = n > 0 ? scan_chunks(n) : 1;
         if (c >= used) continue;                   // uniform over the block
@@ -128,9 +109,9 @@ number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch
         const int id = scan_position(scan.state + (size_t)b * chunks, c, cnt, &end, status);
         if (c == used - 1 && threadIdx.x == 0) voxel_num[b] = end;   // at most max_points rows, and those fit max_voxels
         if (w < n) rec[w].z = (uint32_t)id;
-        if (w < n && marks.rec) {
+        if (w < n && chain.count) {
             const int row = (int)r.w / grid.xw;
-            mark_word(bits, row / grid.Y, row % grid.Y, (int)r.w - row * grid.xw, b, geom, marks);
+            mark_levels(bits, row / grid.Y, row % grid.Y, (int)r.w - row * grid.xw, b, chain);
         }
         // the warp's rows are consecutive: their point lists in one run
         const int first = __shfl_sync(0xFFFFFFFFu, id, 0), last = __shfl_sync(0xFFFFFFFFu, id + cnt, 31);
@@ -151,36 +132,9 @@ number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch
     }
 }
 
-__global__ void __launch_bounds__(kThreads)
-point_list_kernel(const int32_t* __restrict__ points_size, int batch, int max_points, BitGrid grid,
-                  const uint32_t* __restrict__ pt_key, int max_pts, uint32_t* __restrict__ lists) {
+__global__ void __launch_bounds__(kThreads) point_list_kernel(PointLists lists, int batch) {
     pdl_enter();
-    for_points(points_size, batch, max_points, [&](int b, int p) {
-        const uint32_t key = __ldg(pt_key + (size_t)b * max_points + p);
-        if (key == kEmpty) return;
-        const uint4 r = __ldg(grid.rec + (size_t)b * grid.words + word_id(grid, b, key >> 6));
-        const int row = (int)r.z + __popcll(rec_bits(r) & ((1ull << (key & 63)) - 1ull));
-        list_push(lists + ((size_t)b * max_points + row) * max_pts, max_pts, (uint32_t)p);
-    });
-}
-
-template <typename T>
-__global__ void __launch_bounds__(kThreads)
-row_mean_kernel(const float4* __restrict__ points, const int32_t* __restrict__ voxel_num, int batch, int max_voxels,
-                int max_points, int max_pts, const uint32_t* __restrict__ lists, T* __restrict__ voxels) {
-    pdl_enter();
-    const int chunks = (max_points + kThreads - 1) / kThreads;   // rows never outnumber points
-    const int items = batch * chunks;
-    for (int it = blockIdx.x; it < items; it += gridDim.x) {
-        const int b = it / chunks;
-        const int row = (it - b * chunks) * kThreads + threadIdx.x;
-        if (row >= __ldg(voxel_num + b)) continue;
-        uint32_t pi[kMaxPointsPerVoxel];
-        list_load(lists + ((size_t)b * max_points + row) * max_pts, max_pts, pi);
-        int cnt;
-        const float4 m = voxel_mean(points + (size_t)b * max_points, max_pts, pi, &cnt);
-        store_voxel(voxels, (size_t)b * max_voxels + row, m.x, m.y, m.z, m.w);
-    }
+    push_points(lists, batch, blockIdx.x, gridDim.x);
 }
 
 }  // namespace
@@ -212,9 +166,9 @@ void voxel_grid_layout(Bump& bump, const sessd_voxel_params* p, const int level_
     w->scan_rows = scan_state_at(zero ? zero + top_bytes + words_bytes : nullptr, w->grid.words, batch);
 }
 
-int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int out_dtype, const float* points,
-                   const int32_t* points_size, void* voxels, int32_t* coors, int32_t* voxel_num, const VoxelGrid& w,
-                   const ConvGeom& geom, const BitGrid& marks, int32_t* status, cudaStream_t stream) {
+int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, const float* points, const int32_t* points_size,
+                   int32_t* coors, int32_t* voxel_num, const VoxelGrid& w, const LevelChain& chain, int32_t* status,
+                   cudaStream_t stream) {
     const VoxGeom g = voxel_geom(*p);
     const float4* pts = reinterpret_cast<const float4*>(points);
     const int max_pts = p->max_points_per_voxel;
@@ -229,16 +183,10 @@ int voxel_grid_run(const sessd_voxel_params* p, int batch, int max_points, int o
                  status);
     SESSD_LAUNCH(point_bits_kernel, blocks(max_points), kThreads, 0, stream, points_size, batch, max_points, w.grid, w.pt_key);
     SESSD_LAUNCH(number_rows_kernel, blocks(w.grid.words), kThreads, 0, stream, w.grid, w.word_num, batch, p->max_voxels,
-                 max_points, max_pts, w.scan_rows, reinterpret_cast<int4*>(coors), voxel_num, w.lists, geom, marks,
-                 status);
-    SESSD_LAUNCH(point_list_kernel, blocks(max_points), kThreads, 0, stream, points_size, batch, max_points, w.grid, w.pt_key,
-                 max_pts, w.lists);
-    if (out_dtype == SESSD_F32)
-        SESSD_LAUNCH(row_mean_kernel<float>, blocks(max_points), kThreads, 0, stream, pts, voxel_num, batch, p->max_voxels,
-                     max_points, max_pts, w.lists, static_cast<float*>(voxels));
-    else
-        SESSD_LAUNCH(row_mean_kernel<__half>, blocks(max_points), kThreads, 0, stream, pts, voxel_num, batch, p->max_voxels,
-                     max_points, max_pts, w.lists, static_cast<__half*>(voxels));
+                 max_points, max_pts, w.scan_rows, reinterpret_cast<int4*>(coors), voxel_num, w.lists, chain, status);
+    const PointLists lists{points_size, w.pt_key, w.lists, w.grid, max_points, max_pts};
+    if (chain.count) return launch_number_levels(chain, batch, p->max_voxels, lists, status, stream);
+    SESSD_LAUNCH(point_list_kernel, blocks(max_points), kThreads, 0, stream, lists, batch);
     return SESSD_OK;
 }
 

@@ -64,7 +64,8 @@ voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__
                   VoxGeom g, Table t, int max_pts, const int32_t* __restrict__ pt_slot, ScanState scan, VoxelOut<T> out) {
     pdl_enter();
     const int chunks = scan_chunks(max_points), items = batch * chunks;
-    for (int ticket = scan_ticket(scan.ticket, items); ticket >= 0; ticket = scan_ticket(scan.ticket, items)) {
+    for (int ticket = scan_first(scan.ticket, items, gridDim.x); ticket >= 0;
+         ticket = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = ticket / batch, b = ticket - c * batch;
         int n = points_size[b];
         n = n < 0 ? 0 : (n > max_points ? max_points : n);
