@@ -208,53 +208,66 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
 // Numbers one chunk (kThreads x WORDS words) of one frame of a level whose bits are set, in word order (= (z, y, x)
 // order): completes the records (rows before the word), writes the output coordinates (sparseConv3dlayer.cu:436-441 writes
 // them per pair) and, with the last chunk, the row count. Rows past max_voxels are dropped (their bits too, so that the
-// next level does not see them) and reported. A warp writes its words' coordinates one word at a time, a lane per cell.
-// Returns the running total with the chunk.
+// next level does not see them) and reported. Returns the running total with the chunk.
 template <int WORDS>
 __device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long* state, int b, int c, int chunks, int max_voxels,
                                             int4* __restrict__ out_coors, int32_t* __restrict__ out_num, int32_t* status) {
-    const int lane = threadIdx.x & 31;
-    const int w0 = (c * kThreads + threadIdx.x) * WORDS;
+    // word i of a thread: c * kThreads * WORDS + i * kThreads + threadIdx.x, so that a warp's words of a step are neighbours.
+    // Counts of the steps travel through one block scan, 16 bits each (a step has at most 256 x 64 cells).
+    static_assert(WORDS <= 4, "four steps to a 64-bit scan");
+    __shared__ unsigned long long s_sum[kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int w0 = c * kThreads * WORDS + threadIdx.x;
     uint4* rec = g.rec + (size_t)b * g.words;
-    unsigned long long bits[WORDS];
-    int count = 0;
+    unsigned long long bits[WORDS], mine = 0ull;
 #pragma unroll
     for (int i = 0; i < WORDS; ++i) {
-        bits[i] = w0 + i < g.words ? rec_bits(rec[w0 + i]) : 0ull;
-        count += __popcll(bits[i]);
+        const int w = w0 + i * kThreads;
+        bits[i] = w < g.words ? rec_bits(rec[w]) : 0ull;
+        mine |= (unsigned long long)__popcll(bits[i]) << (16 * i);
     }
-    int end;
-    int id = scan_position(state, c, count, &end, status);
+    unsigned long long incl = mine;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= d) incl += t;
+    }
+    __syncthreads();                                     // s_sum has been read by the previous chunk
+    if (lane == 31) s_sum[warp] = incl;
+    __syncthreads();
+    unsigned long long before = incl - mine, all = 0ull;
+#pragma unroll
+    for (int i = 0; i < kThreads / 32; ++i) {
+        if (i < warp) before += s_sum[i];
+        all += s_sum[i];
+    }
+    int total = 0;
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i) total += (int)(all >> (16 * i) & 0xFFFFull);
+    const int prefix = scan_prefix(state, c, total, status), end = prefix + total;
     if (c == chunks - 1 && threadIdx.x == 0) {
         out_num[b] = end > max_voxels ? max_voxels : end;
         if (end > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
     }
+    int step0 = prefix;                                  // rows before the step
 #pragma unroll
     for (int i = 0; i < WORDS; ++i) {
-        if (id + __popcll(bits[i]) > max_voxels) {       // keep the first max_voxels - id cells
+        const int w = w0 + i * kThreads;
+        const int id = step0 + (int)(before >> (16 * i) & 0xFFFFull);
+        step0 += (int)(all >> (16 * i) & 0xFFFFull);
+        unsigned long long v = bits[i];
+        if (id + __popcll(v) > max_voxels) {             // keep the first max_voxels - id cells
             int keep = max_voxels - id > 0 ? max_voxels - id : 0;
             unsigned long long kept = 0ull;
-            for (unsigned long long rem = bits[i]; rem && keep; --keep) {
-                kept |= rem & (0ull - rem);
-                rem &= rem - 1ull;
+            for (; v && keep; --keep) {
+                kept |= v & (0ull - v);
+                v &= v - 1ull;
             }
-            bits[i] = kept;
+            v = kept;
         }
-        if (w0 + i < g.words) rec[w0 + i] = make_uint4((uint32_t)bits[i], (uint32_t)(bits[i] >> 32), (uint32_t)id, 0u);
-        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, bits[i] != 0ull); todo; todo &= todo - 1u) {
-            const int src = __ffs((int)todo) - 1;
-            const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits[i], src);
-            const int id0 = __shfl_sync(0xFFFFFFFFu, id, src);
-            const int word = w0 + i + (src - lane) * WORDS;
-            const int row = word / g.xw;                 // z * Y + y
-            const int x0 = (word - row * g.xw) << 6;
-            const int z = row / g.Y, y = row - z * g.Y;
-            int4* dst = out_coors + (size_t)b * max_voxels + id0;
-            const uint32_t v_lo = (uint32_t)v, v_hi = (uint32_t)(v >> 32), below = (1u << lane) - 1u;
-            if ((v_lo >> lane) & 1u) dst[__popc(v_lo & below)] = make_int4(b, z, y, x0 + lane);
-            if ((v_hi >> lane) & 1u) dst[__popc(v_lo) + __popc(v_hi & below)] = make_int4(b, z, y, x0 + 32 + lane);
-        }
-        id += __popcll(bits[i]);
+        if (w < g.words) rec[w] = make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)id, 0u);
+        if (__any_sync(0xFFFFFFFFu, v != 0ull))
+            write_cells(out_coors + (size_t)b * max_voxels, b, g.xw, g.Y, w, v, min(id, max_voxels));
     }
     return end;
 }

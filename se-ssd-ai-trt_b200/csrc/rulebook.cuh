@@ -31,6 +31,43 @@ __device__ __forceinline__ unsigned long long rec_bits(const uint4& r) {
     return (unsigned long long)r.x | ((unsigned long long)r.y << 32);
 }
 
+// Position of the n-th set bit of v (n < popcount).
+__device__ __forceinline__ int nth_bit(unsigned long long v, int n) {
+    uint32_t x = (uint32_t)v;
+    int pos = 0, c = __popc(x);
+    if (n >= c) n -= c, x = (uint32_t)(v >> 32), pos = 32;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+        c = __popc(x & ((1u << s) - 1u));
+        if (n >= c) n -= c, x >>= s, pos += s;
+    }
+    return pos;
+}
+
+// Writes the coordinates of the cells of a warp's 32 words: lane's word `word` (of a grid with xw words per line and Y lines
+// per plane) has `bits`, its cells the rows id, id + 1, .. of frame b, consecutive over the lanes. A lane per cell: it finds
+// its word by bisection over the lanes. (A lane per cell of one word at a time keeps most lanes idle: words have some four
+// cells.)
+__device__ __forceinline__ void write_cells(int4* __restrict__ coors, int b, int xw, int Y, int word, unsigned long long bits,
+                                            int id) {
+    const int lane = threadIdx.x & 31;
+    const int first = __shfl_sync(0xFFFFFFFFu, id, 0);
+    const int end = __shfl_sync(0xFFFFFFFFu, id + __popcll(bits), 31);
+    for (int r0 = first; r0 < end; r0 += 32) {
+        const int r = r0 + lane;
+        int src = 0;                                     // the last lane whose rows start at or before r
+#pragma unroll
+        for (int s = 16; s; s >>= 1)
+            if (__shfl_sync(0xFFFFFFFFu, id, src + s) <= r) src += s;
+        const int id0 = __shfl_sync(0xFFFFFFFFu, id, src);
+        const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits, src);
+        const int w = __shfl_sync(0xFFFFFFFFu, word, src);
+        if (r >= end) continue;
+        const int line = w / xw, z = line / Y;
+        coors[r] = make_int4(b, z, line - z * Y, ((w - line * xw) << 6) + nth_bit(v, r - id0));
+    }
+}
+
 // Enters row i of the cell with linear index `key` into a frame's x-grouped table; false when the table is full.
 __device__ __forceinline__ bool bucket_insert(uint32_t* __restrict__ base, uint32_t cap, int shift, uint32_t key, int i) {
     const uint32_t gkey = key >> 2;
@@ -118,12 +155,20 @@ __device__ __forceinline__ uint32_t even_bits(unsigned long long v) {
     return (uint32_t)(v | (v >> 16));
 }
 
-// Sets the bits `lo` of the grid word at rec and `hi` of the next one. The words are read first, through L1: a stale copy
-// only costs an atomic that changes nothing, and most bits have been set by a neighbouring word long before.
-__device__ __forceinline__ void set_bits(uint4* rec, unsigned long long lo, unsigned long long hi) {
-    unsigned long long* p = reinterpret_cast<unsigned long long*>(rec);
-    if ((*p & lo) != lo) atomicOr(p, lo);
-    if (hi && (p[2] & hi) != hi) atomicOr(p + 2, hi);
+// Sets the bits `lo` of the grid word at rec[0] and `hi` of the next one, for up to four words. The words are read first,
+// side by side and through L1: a stale copy only costs an atomic that changes nothing, and most bits have been set by a
+// neighbouring word long before.
+__device__ __forceinline__ void set_bits(uint4* const (&rec)[4], unsigned long long lo, unsigned long long hi) {
+    unsigned long long cur[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) cur[i] = rec[i] ? *reinterpret_cast<const unsigned long long*>(rec[i]) : ~0ull;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if ((cur[i] & lo) != lo) atomicOr(reinterpret_cast<unsigned long long*>(rec[i]), lo);
+    if (!hi) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (rec[i]) atomicOr(reinterpret_cast<unsigned long long*>(rec[i] + 1), hi);
 }
 
 // Marks, in the grids of all levels of a chain, the outputs of the cells of word (z, y, wx) of the voxeliser's level,
@@ -136,8 +181,8 @@ __device__ __forceinline__ void mark_levels(unsigned long long bits, int z, int 
     for (int l = 0; l < chain.count && bits; ++l) {
         const ConvGeom& g = chain.geom[l];
         const BitGrid& out = chain.grid[l];
-        z0 = max(z0 + g.P[0] - g.K[0] + g.S[0], 0) / g.S[0], z1 = min((z1 + g.P[0]) / g.S[0], out.Z - 1);
-        y0 = max(y0 + g.P[1] - g.K[1] + g.S[1], 0) / g.S[1], y1 = min((y1 + g.P[1]) / g.S[1], out.Y - 1);
+        z0 = div_trunc(max(z0 + g.P[0] - g.K[0] + g.S[0], 0), g.S[0]), z1 = min(div_trunc(z1 + g.P[0], g.S[0]), out.Z - 1);
+        y0 = div_trunc(max(y0 + g.P[1] - g.K[1] + g.S[1], 0), g.S[1]), y1 = min(div_trunc(y1 + g.P[1], g.S[1]), out.Y - 1);
         if (g.K[2] == 3) {
             const unsigned long long even = even_bits(bits), odd = even_bits(bits >> 1);
             bits = even | odd | (odd << 1);
@@ -147,8 +192,14 @@ __device__ __forceinline__ void mark_levels(unsigned long long bits, int z, int 
         const int sh = off & 63;
         const unsigned long long lo = bits << sh, hi = sh ? bits >> (64 - sh) : 0ull;
         uint4* rec = out.rec + (size_t)b * out.words + (off >> 6);
-        for (int oz = z0; oz <= z1; ++oz)
-            for (int oy = y0; oy <= y1; ++oy) set_bits(rec + (oz * out.Y + oy) * out.xw, lo, hi);
+        for (int oz = z0; oz <= z1; oz += 2)             // (rarely more than 2 x 2 lines)
+            for (int oy = y0; oy <= y1; oy += 2) {
+                uint4* at = rec + (oz * out.Y + oy) * out.xw;
+                const bool z2 = oz < z1, y2 = oy < y1;
+                uint4* const lines[4] = {at, y2 ? at + out.xw : nullptr, z2 ? at + out.Y * out.xw : nullptr,
+                                         z2 && y2 ? at + (out.Y + 1) * out.xw : nullptr};
+                set_bits(lines, lo, hi);
+            }
     }
 }
 

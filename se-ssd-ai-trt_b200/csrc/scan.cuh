@@ -36,12 +36,9 @@ __device__ __forceinline__ int scan_await(const unsigned long long* p, unsigned 
     return (int)(unsigned)v;
 }
 
-// Exclusive position of the calling thread's `count` things among those of all chunks before chunk c of the frame whose
-// state words start at `state` (zero before the kernel) and of its own block (kThreads threads); *chunk_end gets the
-// running total including the chunk. The whole block calls it.
-__device__ __forceinline__ int scan_position(unsigned long long* state, int c, int count, int* chunk_end, int32_t* status) {
-    int total;
-    const int before = block_exclusive_scan(count, &total);
+// Sum of the totals of the chunks before chunk c of the frame whose state words start at `state` (zero before the kernel);
+// `total` is chunk c's own. The whole block (kThreads threads) calls it.
+__device__ __forceinline__ int scan_prefix(unsigned long long* state, int c, int total, int32_t* status) {
     const bool closes_group = c % kScanGroup == kScanGroup - 1;
     if (threadIdx.x == 0 && !closes_group) scan_publish(state + c, total);
     int prefix = 0;
@@ -63,6 +60,15 @@ __device__ __forceinline__ int scan_position(unsigned long long* state, int c, i
         prefix = block_sum(sum);
     }
     if (threadIdx.x == 0 && closes_group) scan_publish(state + c, prefix + total);
+    return prefix;
+}
+
+// Exclusive position of the calling thread's `count` things among those of all chunks before chunk c and of its own block;
+// *chunk_end gets the running total including the chunk.
+__device__ __forceinline__ int scan_position(unsigned long long* state, int c, int count, int* chunk_end, int32_t* status) {
+    int total;
+    const int before = block_exclusive_scan(count, &total);
+    const int prefix = scan_prefix(state, c, total, status);
     *chunk_end = prefix + total;
     return prefix + before;
 }

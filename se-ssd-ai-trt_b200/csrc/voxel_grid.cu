@@ -117,18 +117,7 @@ number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch
         const int first = __shfl_sync(0xFFFFFFFFu, id, 0), last = __shfl_sync(0xFFFFFFFFu, id + cnt, 31);
         uint32_t* list = lists + (size_t)b * max_points * max_pts;
         for (int e = first * max_pts + lane; e < last * max_pts; e += 32) list[e] = kEmpty;
-        for (uint32_t todo = __ballot_sync(0xFFFFFFFFu, bits != 0ull); todo; todo &= todo - 1u) {
-            const int src = __ffs((int)todo) - 1;
-            const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits, src);
-            const int word = (int)__shfl_sync(0xFFFFFFFFu, r.w, src);
-            int4* dst = coors + (size_t)b * max_voxels + __shfl_sync(0xFFFFFFFFu, id, src);
-            const int row = word / grid.xw;                 // z * Y + y
-            const int x0 = (word - row * grid.xw) << 6;
-            const int z = row / grid.Y, y = row - z * grid.Y;
-            const uint32_t v_lo = (uint32_t)v, v_hi = (uint32_t)(v >> 32), below = (1u << lane) - 1u;
-            if ((v_lo >> lane) & 1u) dst[__popc(v_lo & below)] = make_int4(b, z, y, x0 + lane);
-            if ((v_hi >> lane) & 1u) dst[__popc(v_lo) + __popc(v_hi & below)] = make_int4(b, z, y, x0 + 32 + lane);
-        }
+        if (first < last) write_cells(coors + (size_t)b * max_voxels, b, grid.xw, grid.Y, (int)r.w, bits, id);
     }
 }
 
