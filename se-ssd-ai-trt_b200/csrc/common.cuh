@@ -147,7 +147,7 @@ struct Buckets {
 // Occupancy grid of one resolution level. Word w of a frame covers the 64 cells x = 64*(w % xw) .. +63 of line
 // (z, y) = w / xw. Rows are numbered in word order, i.e. in (z, y, x) order.
 // One level (top == nullptr): frame b owns records [b*words, (b+1)*words), record w = {bits lo, bits hi, rows before this
-// word, unused} of word w.
+// word, first two cells of the line's next word} of word w.
 // Two levels (the voxeliser's level, whose words are nearly all empty): top record w / 64 = {bits lo, bits hi, occupied
 // words before, unused} says which of 64 words are occupied, and frame b's records [b*words, ..) hold the occupied words
 // alone, in order: {bits lo, bits hi, rows before this word, w}.

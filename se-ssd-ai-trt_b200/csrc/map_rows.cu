@@ -25,12 +25,14 @@ namespace sessd {
 namespace {
 
 constexpr int kWindow = 1024;              // rows of a window (eight tiles)
-constexpr int kMapThreads = 512;           // two rows per thread; two blocks per SM
+constexpr int kMapThreads = 512;           // two rows per thread
+constexpr int kMapBlocks = 2;              // per SM: 64 registers (three blocks with 40 spill, and are an eighth slower)
 constexpr int kMapKvol = 27;
 constexpr int kGroups = kWindow / 32;      // groups of 32 rows, one per warp and step
 
 struct MapShared {
-    int32_t ids[kMapKvol][kWindow];
+    int32_t base[9][kWindow];              // per line of the receptive field: the input row of its first neighbour
+    uint32_t bits[kWindow];                // which offsets have a neighbour
     union {
         uint16_t count[64][kGroups];       // rows per bin and group of 32 rows; then where they start
         uint16_t src[kWindow];             // row of the window at each position
@@ -39,68 +41,133 @@ struct MapShared {
     int warp_sum[kMapThreads / 32];
 };
 
-// An index answers for lines: the rows of the K2 x-neighbours x0 .. x0 + K2 - 1 on line (z, y). What the lines of one
-// output row share (Row) is worked out once; a line is then told by its distance from the row's first line. Reads go in
-// two steps, so that a thread has the reads of several lines in flight.
-
-// Through the level's occupancy grid.
+// Through a level's occupancy grid. The K2 x-neighbours x0 .. x0 + K2 - 1 of a line (z, y) are neighbouring bits that may
+// straddle two words, and rows are numbered along the line, so a line is told by its bits and the row of its first
+// neighbour: all that the window keeps of it. What the lines of one output row share (Row) is worked out once; a line is
+// then told by its distance from the row's first line. Reads go in two steps, so that a thread has the reads of several lines in
+// flight.
 struct BitsIndex {
     const uint4* rec;      // of the frame
     const uint4* top;      // of the frame, or null (one-level grid)
     int Y, X, xw;
-    struct Row { int word, sh; bool two, neg; };
-    struct Line { uint4 a, b; };
+    struct Row {
+        int word;
+        uint32_t sh, below_lo, below_hi;   // first bit of the window (mod 32), bits of the word before it
+        bool upper, neg, two;              // window starts in the word's upper half; at x = -1; goes on in the next word
+    };
     static __device__ __forceinline__ BitsIndex make(const MapJob& j, int b) {
         const BitGrid& g = j.in;
         return BitsIndex{g.rec + (size_t)b * g.words, g.top ? g.top + (size_t)b * g.top_words : nullptr, g.Y, g.X, g.xw};
     }
     __device__ __forceinline__ Row row(int z, int y, int x0, int count) const {
         const int lo = max(x0, 0), hi = min(x0 + count, X) - 1;
-        return Row{(z * Y + y) * xw + (lo >> 6), lo & 63, (hi >> 6) > (lo >> 6), x0 < 0};
+        const uint32_t sh = lo & 31, below = (1u << sh) - 1u;
+        const bool upper = lo & 32;
+        return Row{(z * Y + y) * xw + (lo >> 6), sh, upper ? ~0u : below, upper ? below : 0u, upper, x0 < 0, (hi >> 6) > (lo >> 6)};
     }
     __device__ __forceinline__ int step(int kz, int ky) const { return (kz * Y + ky) * xw; }
+    __device__ __forceinline__ uint4 first(int w, bool on) const {
+        return on ? __ldg(top ? top + (w >> 6) : rec + w) : make_uint4(0u, 0u, 0u, 0u);
+    }
     // Record of word w of a two-level grid, given its top record; empty when the word is.
     __device__ __forceinline__ uint4 word_record(int w, const uint4& t) const {
-        const unsigned long long tb = rec_bits(t), bit = 1ull << (w & 63);
-        if (!(tb & bit)) return make_uint4(0u, 0u, 0u, 0u);
-        return __ldg(rec + ((int)t.z + __popcll(tb & (bit - 1ull))));
+        const uint32_t bit = 1u << (w & 31);
+        const bool upper = w & 32;
+        if (!((upper ? t.y : t.x) & bit)) return make_uint4(0u, 0u, 0u, 0u);
+        return __ldg(rec + ((int)t.z + __popc(upper ? t.x : 0u) + __popc((upper ? t.y : t.x) & (bit - 1u))));
     }
-    __device__ __forceinline__ void first(const Row& r, int step, bool on, Line* l) const {
-        l->a = l->b = make_uint4(0u, 0u, 0u, 0u);
-        if (!on) return;
-        const int w = r.word + step;
-        l->a = __ldg(top ? top + (w >> 6) : rec + w);
-        if (r.two) l->b = __ldg(top ? top + ((w + 1) >> 6) : rec + w + 1);
-    }
-    __device__ __forceinline__ void second(const Row& r, int step, Line* l) const {
+    __device__ __forceinline__ void second(const Row& r, int w, bool on, uint4* l) const {
         if (!top) return;
-        const int w = r.word + step;
-        l->a = word_record(w, l->a);
-        if (r.two) {
-            l->b = word_record(w + 1, l->b);
-            if (rec_bits(l->a) == 0ull) l->a.z = l->b.z;   // the rows of the window are then all of the second word
+        *l = word_record(w, *l);
+        l->w = 0u;
+        if (r.two && on) {
+            const uint4 next = word_record(w + 1, __ldg(top + ((w + 1) >> 6)));
+            if (!(l->x | l->y)) l->z = next.z;   // the rows of the window are then all of the second word
+            l->w = next.x & 3u;
         }
     }
-    // The cells are neighbouring bits of a window that may straddle two words, and rows are numbered along the line, so
-    // the row of a set cell is the row of the window's first cell plus the set cells before it. (Cells past the line's
-    // end are never set.)
+    // Neighbours of a line as bits, and the row of the first.
     template <int COUNT>
-    __device__ __forceinline__ uint32_t finish(const Row& r, int, const Line& l, int (&rows)[3]) const {
-        const unsigned long long a = rec_bits(l.a);
-        unsigned long long v = a >> r.sh;
-        if (r.two) v |= rec_bits(l.b) << (64 - r.sh);
-        uint32_t w = (uint32_t)v;
-        if (r.neg) w <<= 1;
-        w &= (1u << COUNT) - 1u;
-        const int base = (int)l.a.z + __popcll(a & ((1ull << r.sh) - 1ull));
-        rows[0] = w & 1u ? base : -1;
-        rows[1] = w & 2u ? base + (int)(w & 1u) : -1;
-        rows[2] = w & 4u ? base + __popc(w & 3u) : -1;
-        return w;
+    __device__ __forceinline__ uint32_t finish(const Row& r, const uint4& l, int* base) const {
+        const uint32_t w = __funnelshift_r(r.upper ? l.y : l.x, r.upper ? l.w : l.y, r.sh) << (r.neg ? 1 : 0);
+        *base = (int)l.z + __popc(l.x & r.below_lo) + __popc(l.y & r.below_hi);
+        return w & ((1u << COUNT) - 1u);
     }
 };
 
+// Neighbours of the row whose first input cell is (z, y, x), as a mask of offsets; put(line, row of its first neighbour).
+// KZ, KY, KX: the kernel.
+template <int KZ, int KY, int KX, class Put>
+__device__ __forceinline__ uint32_t grid_row(const BitsIndex& in, int Z, int z, int y, int x, bool live, Put put) {
+    const BitsIndex::Row row = in.row(z, y, x, KX);
+    uint32_t bits = 0;
+#pragma unroll
+    for (int kz = 0; kz < KZ; ++kz) {
+        const bool z_ok = live && (unsigned)(z + kz) < (unsigned)Z;
+        uint4 l[KY];
+#pragma unroll
+        for (int ky = 0; ky < KY; ++ky) l[ky] = in.first(row.word + in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y);
+#pragma unroll
+        for (int ky = 0; ky < KY; ++ky)
+            in.second(row, row.word + in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y, &l[ky]);
+#pragma unroll
+        for (int ky = 0; ky < KY; ++ky) {
+            int base;
+            bits |= in.template finish<KX>(row, l[ky], &base) << ((kz * KY + ky) * KX);
+            put(kz * KY + ky, base);
+        }
+    }
+    return bits;
+}
+
+// Any other kernel up to 3 x 3 x 3: one line at a time.
+template <class Put>
+__device__ __noinline__ uint32_t grid_row_any(const BitsIndex& in, const ConvGeom& g, int z, int y, int x, bool live, Put put) {
+    const BitsIndex::Row row = in.row(z, y, x, g.K[2]);
+    uint32_t bits = 0;
+    for (int kz = 0; kz < g.K[0]; ++kz)
+        for (int ky = 0; ky < g.K[1]; ++ky) {
+            const bool on = live && (unsigned)(z + kz) < (unsigned)g.in_shape[0] && (unsigned)(y + ky) < (unsigned)in.Y;
+            const int w = row.word + in.step(kz, ky), line = kz * g.K[1] + ky;
+            uint4 l = in.first(w, on);
+            in.second(row, w, on, &l);
+            int base;
+            bits |= (in.template finish<3>(row, l, &base) & ((1u << g.K[2]) - 1u)) << (line * g.K[2]);
+            put(line, base);
+        }
+    return bits;
+}
+
+template <class Put>
+__device__ __forceinline__ uint32_t grid_entries(const BitsIndex& in, const MapJob& job, const int4& c, bool live, Put put) {
+    const ConvGeom& g = job.g;
+    const int z = c.y * g.S[0] - g.P[0], y = c.z * g.S[1] - g.P[1], x = c.w * g.S[2] - g.P[2];
+    switch (job.shape) {                                     // uniform over the block
+        case 333: return grid_row<3, 3, 3>(in, g.in_shape[0], z, y, x, live, put);
+        case 311: return grid_row<3, 1, 1>(in, g.in_shape[0], z, y, x, live, put);
+        default: return grid_row_any(in, g, z, y, x, live, put);
+    }
+}
+
+// The entries of one position, whose row of the window is r (none: r < 0), for the offsets in m.
+template <int KX>
+__device__ __forceinline__ void write_entries(const MapShared& s, int r, uint32_t m, int lines, int32_t* out) {
+    uint32_t w = r >= 0 ? s.bits[r] : 0u;
+#pragma unroll
+    for (int line = 0; line < 9; ++line, w >>= KX) {
+        if (line >= lines) break;
+        const uint32_t t = m >> (line * KX);
+        if (!(t & ((1u << KX) - 1u))) continue;              // uniform over the warp
+        const int base = s.base[line][r < 0 ? 0 : r];
+#pragma unroll
+        for (int k = 0; k < KX; ++k)
+            if ((t >> k) & 1u)
+                out[(line * KX + k) * kNbrRun] = (w >> k) & 1u ? base + __popc(w & ((1u << k) - 1u)) : -1;
+    }
+}
+
 // Through the x-grouped table: the three x-neighbours lie in at most two 32-byte buckets.
+// Same division of the work as above, but the rows are in no order: a line is its three rows.
 struct BucketIndex {
     const uint32_t* data;   // of the frame
     uint32_t cap;
@@ -169,7 +236,7 @@ struct BucketIndex {
 };
 
 // Entries of the row whose first input cell is (z, y, x): put(offset, input row or -1) for every offset, and as a mask of
-// the offsets that have one. KZ, KY, KX: the kernel.
+// the offsets that have one.
 template <int KZ, int KY, int KX, class Index, class Put>
 __device__ __forceinline__ uint32_t map_row(const Index& in, int Z, int z, int y, int x, bool live, Put put) {
     const typename Index::Row row = in.row(z, y, x, KX);
@@ -241,7 +308,7 @@ __device__ __forceinline__ void row_means(const RowMeans& m, T* voxels, int batc
     }
 }
 
-__global__ void __launch_bounds__(kMapThreads, 2)
+__global__ void __launch_bounds__(kMapThreads, kMapBlocks)
 map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxels, int tiles_per_frame, RowMeans means) {
     pdl_enter();
     extern __shared__ __align__(16) uint8_t map_smem[];
@@ -295,7 +362,8 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
             const bool live = r < n;
             int4 c = make_int4(0, 0, 0, 0);
             if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + w0 + r);
-            const uint32_t bits = map_entries(in, job, c, live, [&](int k, int v) { s.ids[k][r] = v; });
+            const uint32_t bits = grid_entries(in, job, c, live, [&](int line, int base) { s.base[line][r] = base; });
+            s.bits[r] = bits;
             uint32_t key = 64u;                              // dead rows (the frame's last window): they stay behind
             if (live) {
                 key = 0u;
@@ -357,9 +425,12 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
             if (job.order && p < n) job.order[(size_t)b * max_voxels + w0 + p] = w0 + r;
             int32_t* out = job.nbr + nbr_index(job.g.kvol, max_voxels, b, 0, w0 + p);
             if (job.g.kvol < kMapKvol) m &= (1u << job.g.kvol) - 1u;
-#pragma unroll
-            for (int k = 0; k < kMapKvol; ++k)
-                if ((m >> k) & 1u) out[k * kNbrRun] = p < n ? s.ids[k][r] : -1;
+            const int from = p < n ? r : -1, lines = job.g.K[0] * job.g.K[1];
+            switch (job.g.K[2]) {                            // uniform over the block
+                case 3: write_entries<3>(s, from, m, lines, out); break;
+                case 2: write_entries<2>(s, from, m, lines, out); break;
+                default: write_entries<1>(s, from, m, lines, out);
+            }
         }
     }
     // Beside the maps: the means of the voxeliser's rows. From the last block down, which has the fewest windows.
@@ -435,7 +506,7 @@ int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const Row
         configured.fetch_or(bit, std::memory_order_release);
     }
     const int64_t items = (int64_t)(jobs.count > 0 ? jobs.count : 1) * batch * ((max_voxels + kWindow - 1) / kWindow);
-    const int most = persistent_grid(2);
+    const int most = persistent_grid(kMapBlocks);
     SESSD_LAUNCH(map_windows_kernel, (int)(items < most ? items : most), kMapThreads, sizeof(MapShared), stream, jobs, batch,
                  max_voxels, (max_voxels + 127) / 128, means);
     return SESSD_OK;

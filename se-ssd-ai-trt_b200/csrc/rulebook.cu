@@ -256,6 +256,9 @@ __device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long
         const int id = step0 + (int)(before >> (16 * i) & 0xFFFFull);
         step0 += (int)(all >> (16 * i) & 0xFFFFull);
         unsigned long long v = bits[i];
+        uint32_t next = __shfl_down_sync(0xFFFFFFFFu, (uint32_t)v, 1);
+        if (lane == 31 && w + 1 < g.words) next = rec[w + 1].x;
+        next = next_cells(next, w, g, id + __popcll(v), max_voxels);
         if (id + __popcll(v) > max_voxels) {             // keep the first max_voxels - id cells
             int keep = max_voxels - id > 0 ? max_voxels - id : 0;
             unsigned long long kept = 0ull;
@@ -265,7 +268,7 @@ __device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long
             }
             v = kept;
         }
-        if (w < g.words) rec[w] = make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)id, 0u);
+        if (w < g.words) rec[w] = make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)id, next);
         if (__any_sync(0xFFFFFFFFu, v != 0ull))
             write_cells(out_coors + (size_t)b * max_voxels, b, g.xw, g.Y, w, v, min(id, max_voxels));
     }
@@ -305,6 +308,7 @@ __device__ __noinline__ void renumber_levels(const LevelChain& chain, int b, int
             int total;
             int id = base + block_exclusive_scan(__popcll(v), &total);
             const int id0 = id;
+            const uint32_t next = next_cells(w + 1 < g.words ? __ldcg(rec + w + 1).x : 0u, w, g, id + __popcll(v), max_voxels);
             unsigned long long kept = 0ull;
             const int row = w / g.xw, z = row / g.Y;
             for (; v && id < max_voxels; ++id) {
@@ -313,7 +317,7 @@ __device__ __noinline__ void renumber_levels(const LevelChain& chain, int b, int
                 kept |= 1ull << bit;
                 __stcg(out + id, make_int4(b, z, row - z * g.Y, ((w - row * g.xw) << 6) + bit));
             }
-            if (w < g.words) __stcg(rec + w, make_uint4((uint32_t)kept, (uint32_t)(kept >> 32), (uint32_t)id0, 0u));
+            if (w < g.words) __stcg(rec + w, make_uint4((uint32_t)kept, (uint32_t)(kept >> 32), (uint32_t)id0, next));
             base += total;
         }
         if (threadIdx.x == 0) {

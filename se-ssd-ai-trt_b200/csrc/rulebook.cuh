@@ -155,6 +155,14 @@ __device__ __forceinline__ uint32_t even_bits(unsigned long long v) {
     return (uint32_t)(v | (v >> 16));
 }
 
+// Last word of word w's record: the first two cells of the next word of the line, whose low bits (before any row is dropped)
+// are `low` and whose rows begin at next_row.
+__device__ __forceinline__ uint32_t next_cells(uint32_t low, int w, const BitGrid& g, int next_row, int max_voxels) {
+    uint32_t c = low & 3u;
+    if (next_row + 2 > max_voxels) c = next_row < max_voxels ? c & (0u - c) : 0u;
+    return c && w + 1 < g.words && (w + 1) % g.xw != 0 ? c : 0u;
+}
+
 // Sets the bits `lo` of the grid word at rec[0] and `hi` of the next one, for up to four words. The words are read first,
 // side by side and through L1: a stale copy only costs an atomic that changes nothing, and most bits have been set by a
 // neighbouring word long before.
