@@ -32,12 +32,12 @@ constexpr int kGroups = kWindow / 32;      // groups of 32 rows, one per warp an
 
 struct MapShared {
     int32_t base[9][kWindow];              // per line of the receptive field: the input row of its first neighbour
-    uint32_t bits[kWindow];                // which offsets have a neighbour
+    uint32_t bits[kWindow];                // which offsets have a neighbour (none for rows past the frame's)
     union {
         uint16_t count[64][kGroups];       // rows per bin and group of 32 rows; then where they start
         uint16_t src[kWindow];             // row of the window at each position
     };
-    uint32_t tile[kWindow / 128];
+    alignas(16) uint32_t group_bits[kGroups];          // offsets that 32 positions have any neighbour under
     int warp_sum[kMapThreads / 32];
 };
 
@@ -66,8 +66,9 @@ struct BitsIndex {
         return Row{(z * Y + y) * xw + (lo >> 6), sh, upper ? ~0u : below, upper ? below : 0u, upper, x0 < 0, (hi >> 6) > (lo >> 6)};
     }
     __device__ __forceinline__ int step(int kz, int ky) const { return (kz * Y + ky) * xw; }
-    __device__ __forceinline__ uint4 first(int w, bool on) const {
-        return on ? __ldg(top ? top + (w >> 6) : rec + w) : make_uint4(0u, 0u, 0u, 0u);
+    template <bool TOP>
+    __device__ __forceinline__ uint4 first(int w, bool on) const {   // (off: some record, which finish() then ignores)
+        return __ldg(TOP ? top + (on ? w >> 6 : 0) : rec + (on ? w : 0));
     }
     // Record of word w of a two-level grid, given its top record; empty when the word is.
     __device__ __forceinline__ uint4 word_record(int w, const uint4& t) const {
@@ -76,9 +77,10 @@ struct BitsIndex {
         if (!((upper ? t.y : t.x) & bit)) return make_uint4(0u, 0u, 0u, 0u);
         return __ldg(rec + ((int)t.z + __popc(upper ? t.x : 0u) + __popc((upper ? t.y : t.x) & (bit - 1u))));
     }
+    template <bool TOP>
     __device__ __forceinline__ void second(const Row& r, int w, bool on, uint4* l) const {
-        if (!top) return;
-        *l = word_record(w, *l);
+        if (!TOP) return;
+        if (on) *l = word_record(w, *l);
         l->w = 0u;
         if (r.two && on) {
             const uint4 next = word_record(w + 1, __ldg(top + ((w + 1) >> 6)));
@@ -88,33 +90,40 @@ struct BitsIndex {
     }
     // Neighbours of a line as bits, and the row of the first.
     template <int COUNT>
-    __device__ __forceinline__ uint32_t finish(const Row& r, const uint4& l, int* base) const {
+    __device__ __forceinline__ uint32_t finish(const Row& r, const uint4& l, bool on, int* base) const {
         const uint32_t w = __funnelshift_r(r.upper ? l.y : l.x, r.upper ? l.w : l.y, r.sh) << (r.neg ? 1 : 0);
         *base = (int)l.z + __popc(l.x & r.below_lo) + __popc(l.y & r.below_hi);
-        return w & ((1u << COUNT) - 1u);
+        return w & (on ? (1u << COUNT) - 1u : 0u);
     }
 };
 
 // Neighbours of the row whose first input cell is (z, y, x), as a mask of offsets; put(line, row of its first neighbour).
 // KZ, KY, KX: the kernel.
-template <int KZ, int KY, int KX, class Put>
+template <int KZ, int KY, int KX, bool TOP, class Put>
 __device__ __forceinline__ uint32_t grid_row(const BitsIndex& in, int Z, int z, int y, int x, bool live, Put put) {
+    constexpr int BATCH = TOP ? 1 : KZ;                      // planes whose reads are in flight together
     const BitsIndex::Row row = in.row(z, y, x, KX);
+    bool y_ok[KY];
+#pragma unroll
+    for (int ky = 0; ky < KY; ++ky) y_ok[ky] = live && (unsigned)(y + ky) < (unsigned)in.Y;
     uint32_t bits = 0;
 #pragma unroll
-    for (int kz = 0; kz < KZ; ++kz) {
-        const bool z_ok = live && (unsigned)(z + kz) < (unsigned)Z;
-        uint4 l[KY];
+    for (int kz0 = 0; kz0 < KZ; kz0 += BATCH) {
+        uint4 l[BATCH * KY];
+        bool on[BATCH * KY];
 #pragma unroll
-        for (int ky = 0; ky < KY; ++ky) l[ky] = in.first(row.word + in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y);
+        for (int i = 0; i < BATCH * KY; ++i) {
+            const int kz = kz0 + i / KY, ky = i % KY;
+            on[i] = y_ok[ky] && (unsigned)(z + kz) < (unsigned)Z;
+            l[i] = in.template first<TOP>(row.word + in.step(kz, ky), on[i]);
+        }
 #pragma unroll
-        for (int ky = 0; ky < KY; ++ky)
-            in.second(row, row.word + in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y, &l[ky]);
+        for (int i = 0; i < BATCH * KY; ++i) in.template second<TOP>(row, row.word + in.step(kz0 + i / KY, i % KY), on[i], &l[i]);
 #pragma unroll
-        for (int ky = 0; ky < KY; ++ky) {
+        for (int i = 0; i < BATCH * KY; ++i) {
             int base;
-            bits |= in.template finish<KX>(row, l[ky], &base) << ((kz * KY + ky) * KX);
-            put(kz * KY + ky, base);
+            bits |= in.template finish<KX>(row, l[i], on[i], &base) << ((kz0 * KY + i) * KX);
+            put(kz0 * KY + i, base);
         }
     }
     return bits;
@@ -129,10 +138,10 @@ __device__ __noinline__ uint32_t grid_row_any(const BitsIndex& in, const ConvGeo
         for (int ky = 0; ky < g.K[1]; ++ky) {
             const bool on = live && (unsigned)(z + kz) < (unsigned)g.in_shape[0] && (unsigned)(y + ky) < (unsigned)in.Y;
             const int w = row.word + in.step(kz, ky), line = kz * g.K[1] + ky;
-            uint4 l = in.first(w, on);
-            in.second(row, w, on, &l);
+            uint4 l = in.top ? in.first<true>(w, on) : in.first<false>(w, on);
+            if (in.top) in.second<true>(row, w, on, &l);
             int base;
-            bits |= (in.template finish<3>(row, l, &base) & ((1u << g.K[2]) - 1u)) << (line * g.K[2]);
+            bits |= (in.finish<3>(row, l, on, &base) & ((1u << g.K[2]) - 1u)) << (line * g.K[2]);
             put(line, base);
         }
     return bits;
@@ -143,22 +152,25 @@ __device__ __forceinline__ uint32_t grid_entries(const BitsIndex& in, const MapJ
     const ConvGeom& g = job.g;
     const int z = c.y * g.S[0] - g.P[0], y = c.z * g.S[1] - g.P[1], x = c.w * g.S[2] - g.P[2];
     switch (job.shape) {                                     // uniform over the block
-        case 333: return grid_row<3, 3, 3>(in, g.in_shape[0], z, y, x, live, put);
-        case 311: return grid_row<3, 1, 1>(in, g.in_shape[0], z, y, x, live, put);
+        case 333:
+            if (in.top) return grid_row<3, 3, 3, true>(in, g.in_shape[0], z, y, x, live, put);
+            return grid_row<3, 3, 3, false>(in, g.in_shape[0], z, y, x, live, put);
+        case 311:
+            if (!in.top) return grid_row<3, 1, 1, false>(in, g.in_shape[0], z, y, x, live, put);
+            [[fallthrough]];
         default: return grid_row_any(in, g, z, y, x, live, put);
     }
 }
 
-// The entries of one position, whose row of the window is r (none: r < 0), for the offsets in m.
+// The entries of one position for the offsets in m; its row of the window is r, with neighbours w.
 template <int KX>
-__device__ __forceinline__ void write_entries(const MapShared& s, int r, uint32_t m, int lines, int32_t* out) {
-    uint32_t w = r >= 0 ? s.bits[r] : 0u;
+__device__ __forceinline__ void write_entries(const MapShared& s, int r, uint32_t w, uint32_t m, int lines, int32_t* out) {
 #pragma unroll
     for (int line = 0; line < 9; ++line, w >>= KX) {
         if (line >= lines) break;
         const uint32_t t = m >> (line * KX);
         if (!(t & ((1u << KX) - 1u))) continue;              // uniform over the warp
-        const int base = s.base[line][r < 0 ? 0 : r];
+        const int base = s.base[line][r];
 #pragma unroll
         for (int k = 0; k < KX; ++k)
             if ((t >> k) & 1u)
@@ -333,7 +345,8 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
         }
     };
     running();
-    for (int it = blockIdx.x;; it += gridDim.x) {
+    struct Window { int job, frame, first, rows; };
+    auto locate = [&](int it) {                              // the it-th window (rows = 0: there is none)
         for (int total = __shfl_sync(0xFFFFFFFFu, incl, 31); it >= before + total && pair0 < pairs;
              total = __shfl_sync(0xFFFFFFFFu, incl, 31)) {
             before += total;
@@ -341,18 +354,32 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
             my_rows = pair_rows(pair0 + lane);
             running();
         }
-        if (pair0 >= pairs) break;
+        if (pair0 >= pairs) return Window{0, 0, 0, 0};
         const int src_lane = __ffs((int)__ballot_sync(0xFFFFFFFFu, it < before + incl)) - 1;
-        const int ji = (pair0 + src_lane) / batch, b = pair0 + src_lane - ji * batch;
-        const int first = __shfl_sync(0xFFFFFFFFu, incl - (my_rows + kWindow - 1) / kWindow, src_lane);
-        const int w0 = (it - before - first) * kWindow;
-        int n = __shfl_sync(0xFFFFFFFFu, my_rows, src_lane) - w0;   // rows of this window
-        n = n > kWindow ? kWindow : n;
-        const MapJob& job = jobs.job[ji];
+        const int ji = (pair0 + src_lane) / batch;
+        const int first = (it - before - __shfl_sync(0xFFFFFFFFu, incl - (my_rows + kWindow - 1) / kWindow, src_lane)) * kWindow;
+        return Window{ji, pair0 + src_lane - ji * batch, first, min(__shfl_sync(0xFFFFFFFFu, my_rows, src_lane) - first, kWindow)};
+    };
+    // The coordinates of a window's rows are requested a window ahead: two blocks per SM do not hide that latency.
+    int4 coor[2];
+    auto fetch = [&](const Window& w) {
+        const int4* c = reinterpret_cast<const int4*>(jobs.job[w.job].out_coors) + (size_t)w.frame * max_voxels + w.first;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            coor[i] = make_int4(0, 0, 0, 0);
+            if (tid + i * kMapThreads < w.rows) coor[i] = __ldg(c + tid + i * kMapThreads);
+        }
+    };
+    Window next = locate(blockIdx.x);
+    fetch(next);
+    for (int it = blockIdx.x; next.rows > 0;) {
+        const int b = next.frame, w0 = next.first, n = next.rows;   // (rows of this window)
+        const MapJob& job = jobs.job[next.job];
         const BitsIndex in = BitsIndex::make(job, b);
+        it += gridDim.x;
+        next = locate(it);
         __syncthreads();                                     // the previous window has been written out
         for (int e = tid; e < 64 * kGroups / 2; e += kMapThreads) reinterpret_cast<uint32_t*>(s.count)[e] = 0u;
-        if (tid < kWindow / 128) s.tile[tid] = 0u;
         __syncthreads();
         // entries of this thread's rows, and the rows' offsets
         uint32_t mask[2], rank[2], bin[2];
@@ -360,9 +387,7 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
         for (int i = 0; i < 2; ++i) {
             const int r = tid + i * kMapThreads;
             const bool live = r < n;
-            int4 c = make_int4(0, 0, 0, 0);
-            if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + w0 + r);
-            const uint32_t bits = grid_entries(in, job, c, live, [&](int line, int base) { s.base[line][r] = base; });
+            const uint32_t bits = grid_entries(in, job, i == 0 ? coor[0] : coor[1], live, [&](int line, int base) { s.base[line][r] = base; });
             s.bits[r] = bits;
             uint32_t key = 64u;                              // dead rows (the frame's last window): they stay behind
             if (live) {
@@ -377,6 +402,7 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
             if (i == 0) mask[0] = bits, rank[0] = before, bin[0] = key;
             else mask[1] = bits, rank[1] = before, bin[1] = key;
         }
+        fetch(next);
         __syncthreads();
         {   // running totals over (bin, group), four entries per thread
             uint2* at = reinterpret_cast<uint2*>(s.count) + tid;
@@ -405,31 +431,38 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
         }
         __syncthreads();                                     // src takes the counts' place
 #pragma unroll
+        for (int i = 0; i < 2; ++i) s.src[pos[i]] = (uint16_t)(tid + i * kMapThreads);
+        __syncthreads();
+        // a warp takes 32 positions of a tile, and again 32
+        int from[2];
+#pragma unroll
         for (int i = 0; i < 2; ++i) {
-            s.src[pos[i]] = (uint16_t)(tid + i * kMapThreads);
-            if (mask[i]) atomicOr(&s.tile[pos[i] >> 7], mask[i]);
+            const int p = tid + i * kMapThreads;
+            from[i] = s.src[p];
+            mask[i] = s.bits[from[i]];                       // of the position from here on (dead rows: none)
+            const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, mask[i]);
+            if (lane == 0) s.group_bits[p >> 5] = any;
         }
         __syncthreads();
-        // write-out: a warp takes 32 positions of a tile
-#pragma unroll 1
+#pragma unroll
         for (int i = 0; i < 2; ++i) {
             const int p = tid + i * kMapThreads;
             const int tile0 = p & ~127;
             if (tile0 >= n) break;                           // a tile without rows (uniform over the warp)
-            uint32_t m = s.tile[p >> 7];
+            const uint4 g = *reinterpret_cast<const uint4*>(&s.group_bits[tile0 >> 5]);
+            uint32_t m = g.x | g.y | g.z | g.w;
             if ((p & 127) == 0) job.tile_mask[(size_t)b * tiles_per_frame + ((w0 + p) >> 7)] = m;
             // a consumer that fetches `group` offsets at a time wants all of them as soon as it wants one
             if (job.group >= 2) m |= (m & 0x55555555u) << 1 | ((m >> 1) & 0x55555555u);
             if (job.group >= 4) m |= (m & 0x33333333u) << 2 | ((m >> 2) & 0x33333333u);
-            const int r = s.src[p];
-            if (job.order && p < n) job.order[(size_t)b * max_voxels + w0 + p] = w0 + r;
+            if (job.order && p < n) job.order[(size_t)b * max_voxels + w0 + p] = w0 + from[i];
             int32_t* out = job.nbr + nbr_index(job.g.kvol, max_voxels, b, 0, w0 + p);
             if (job.g.kvol < kMapKvol) m &= (1u << job.g.kvol) - 1u;
-            const int from = p < n ? r : -1, lines = job.g.K[0] * job.g.K[1];
+            const int lines = job.g.K[0] * job.g.K[1];
             switch (job.g.K[2]) {                            // uniform over the block
-                case 3: write_entries<3>(s, from, m, lines, out); break;
-                case 2: write_entries<2>(s, from, m, lines, out); break;
-                default: write_entries<1>(s, from, m, lines, out);
+                case 3: write_entries<3>(s, from[i], mask[i], m, lines, out); break;
+                case 2: write_entries<2>(s, from[i], mask[i], m, lines, out); break;
+                default: write_entries<1>(s, from[i], mask[i], m, lines, out);
             }
         }
     }
