@@ -213,6 +213,18 @@ int sessd_sparse2dense_padded_enqueue(const sessd_s2d_params* p, const sessd_pad
                                       void* stream);
 
 /* ------------------------------------------------------------------------------------------
+ * Around the dense convolutions of the 2D neck and head (se-ssd-ai-trt.cpp:1262-1440); fp16 maps. 16-byte aligned.
+ * ---------------------------------------------------------------------------------------- */
+/* out [batch][pixels][channels] = in [batch][channels][pixels]; channels a multiple of 8. */
+int sessd_channels_last_enqueue(const void* in, void* out, int batch, int channels, int pixels, void* stream);
+/* y [pixels][channels] = relu(y + bias) (+ add, unless null), in place; channels 8, 16, 32 .. 2048. */
+int sessd_bias_relu_enqueue(void* y, const void* bias, const void* add, long long pixels, int channels, void* stream);
+/* inputs = { branch 0, branch 1 [pixels][128], attention weights [2][128], biases [2], head weights [22][128], biases [22] };
+ * outputs = { features [pixels][128] fp16 or null, box [pixels][14], cls [pixels][2], iou [pixels][2], dir [pixels][4] fp32
+ * or all four null }: the softmax-weighted sum of the branches, and the 1x1 heads of it. */
+int sessd_neck_tail_enqueue(const void* const* inputs, void* const* outputs, long long pixels, void* stream);
+
+/* ------------------------------------------------------------------------------------------
  * Whole front end: voxelise -> conv stack (BN + ReLU folded) -> dense BEV, the layer sequence
  * wired at se-ssd-ai-trt.cpp:1138-1252, as one call. Coordinate tables and neighbour maps are built
  * once per resolution and shared by the layers that use them (the reference rebuilds the rulebook
@@ -372,6 +384,8 @@ uint64_t sessd_launch_count(void);
 /* Synchronises `stream`, copies the status word of `workspace` to the host and returns it (>= 0),
  * or a negative sessd_error. */
 int sessd_read_status(const void* workspace, void* stream);
+/* The status words of two workspaces OR-ed together, for the price of one wait. */
+int sessd_read_status2(const void* workspace, const void* other, void* stream);
 /* Text of the last CUDA error seen by this thread inside the library ("" if none). */
 const char* sessd_last_cuda_error(void);
 /* Library version string. */

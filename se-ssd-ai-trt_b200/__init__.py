@@ -31,11 +31,12 @@ EXPORTS = (
     "sessd_backbone_final_level", "sessd_pipeline_create", "sessd_pipeline_destroy", "sessd_pipeline_run_host",
     "sessd_pipeline_run_device", "sessd_pipeline_run_host_bev", "sessd_pipeline_dense", "sessd_pipeline_workspace", "sessd_pipeline_use_graphs",
     "sessd_launch_count",
-    "sessd_profile_begin", "sessd_profile_end", "sessd_read_status", "sessd_last_cuda_error", "sessd_version",
+    "sessd_profile_begin", "sessd_profile_end", "sessd_read_status", "sessd_read_status2", "sessd_last_cuda_error", "sessd_version",
     "sessd_anchor_decode_enqueue", "sessd_filter_boxes_workspace_bytes", "sessd_filter_boxes_enqueue",
     "sessd_decode_filter_enqueue", "sessd_rotated_nms_workspace_bytes", "sessd_rotated_nms_enqueue",
     "sessd_wts_load", "sessd_wts_destroy", "sessd_wts_count", "sessd_wts_entry", "sessd_wts_find", "sessd_wts_save",
     "sessd_fold_batchnorm", "sessd_backbone_create_from_wts", "sessd_points_load", "sessd_conv_weights_debug_withhold",
+    "sessd_channels_last_enqueue", "sessd_bias_relu_enqueue", "sessd_neck_tail_enqueue",
 )
 
 
@@ -110,6 +111,7 @@ def lib():
         # declared, so that plain ints pass as pointers and sizes
         p, i, z = C.c_void_p, C.c_int, C.c_size_t
         L.sessd_read_status.argtypes = [p, p]
+        L.sessd_read_status2.argtypes = [p, p, p]
         L.sessd_filter_boxes_workspace_bytes.argtypes = [p, i]
         L.sessd_filter_boxes_enqueue.argtypes = [p, i, p, p, p, z, p]
         L.sessd_decode_filter_enqueue.argtypes = [p, p, i, p, p, p, z, p]
@@ -127,6 +129,9 @@ def lib():
         L.sessd_sparse2dense_padded_enqueue.argtypes = [p, p, i, i, i, p, p, p]
         L.sessd_zero_pad2d_enqueue.argtypes = [p, i, i, i, i, i, p, p, p]
         L.sessd_anchor_decode_enqueue.argtypes = [p, i, p, p, p]
+        L.sessd_channels_last_enqueue.argtypes = [p, p, i, i, i, p]
+        L.sessd_bias_relu_enqueue.argtypes = [p, p, p, C.c_longlong, i, p]
+        L.sessd_neck_tail_enqueue.argtypes = [p, p, C.c_longlong, p]
         L.sessd_profile_end.argtypes = [p, p, z, p, i]
         _lib = L
     return _lib
@@ -194,8 +199,9 @@ def conv_params(layer: schedule.ConvLayer, max_voxels: int) -> ConvParams:
     return p
 
 
-def read_status(workspace) -> int:
-    rc = lib().sessd_read_status(workspace.data_ptr(), _stream())
+def read_status(workspace, other=None) -> int:
+    """Status word of a workspace once the stream's work is done; of two workspaces, both words OR-ed."""
+    rc = lib().sessd_read_status2(workspace.data_ptr(), (workspace if other is None else other).data_ptr(), _stream())
     if rc < 0:
         _check(rc, "sessd_read_status")
     return rc

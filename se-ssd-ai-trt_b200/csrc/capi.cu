@@ -51,7 +51,8 @@ int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const 
 int launch_count_pairs(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* out_num, int batch, int max_voxels,
                        int kvol, unsigned long long* total, cudaStream_t stream);
 
-cudaError_t launch_publish_status(const int32_t* status, unsigned long long* host_word, uint32_t call, cudaStream_t stream);
+cudaError_t launch_publish_status(const int32_t* status, const int32_t* other, unsigned long long* host_word, uint32_t call,
+                                  cudaStream_t stream);
 
 namespace {
 
@@ -327,8 +328,10 @@ uint64_t sessd_launch_count(void) { return g_launches.load(); }
 // The word comes back through mapped host memory: a one-thread kernel behind the stream's work stores it together with the
 // call's number, and the host polls for that number. A stream synchronisation and a copy of four bytes took some 15 us
 // more. One 8-byte slot per host thread, returned when the thread ends.
-int sessd_read_status(const void* workspace, void* stream_) {
-    if (!workspace) return SESSD_ERR_NULL;
+int sessd_read_status(const void* workspace, void* stream) { return sessd_read_status2(workspace, workspace, stream); }
+
+int sessd_read_status2(const void* workspace, const void* other, void* stream_) {
+    if (!workspace || !other) return SESSD_ERR_NULL;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_);
     cudaStreamCaptureStatus capture;
     SESSD_CUDA(cudaStreamIsCapturing(stream, &capture));
@@ -340,7 +343,7 @@ int sessd_read_status(const void* workspace, void* stream_) {
     if (!slot.word)
         SESSD_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&slot.word), sizeof(*slot.word), cudaHostAllocMapped | cudaHostAllocPortable));
     const uint32_t call = ++slot.calls;
-    SESSD_CUDA(launch_publish_status(static_cast<const int32_t*>(workspace), slot.word, call, stream));
+    SESSD_CUDA(launch_publish_status(static_cast<const int32_t*>(workspace), static_cast<const int32_t*>(other), slot.word, call, stream));
     volatile unsigned long long* word = slot.word;
     unsigned long long v;
     for (unsigned spins = 0; (uint32_t)((v = *word) >> 32) != call;) {

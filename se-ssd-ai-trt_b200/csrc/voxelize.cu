@@ -125,18 +125,19 @@ __global__ void __launch_bounds__(kThreads) prepare_kernel(FillRanges f, TailRow
     zero_tails(t);
 }
 
-__global__ void publish_status_kernel(const int32_t* status, unsigned long long* host_word, uint32_t call) {
+__global__ void publish_status_kernel(const int32_t* status, const int32_t* other, unsigned long long* host_word, uint32_t call) {
     pdl_enter();
-    const unsigned long long v = (unsigned long long)call << 32 | (uint32_t)*status;
+    const unsigned long long v = (unsigned long long)call << 32 | (uint32_t)(*status | *other);
     asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(host_word), "l"(v) : "memory");
 }
 
 }  // namespace
 
-// Stores `call` << 32 | *status to mapped host memory behind the stream's work (sessd_read_status; not counted as a launch
+// Stores `call` << 32 | *status | *other to mapped host memory behind the stream's work (sessd_read_status; not counted as a launch
 // of the library's work).
-cudaError_t launch_publish_status(const int32_t* status, unsigned long long* host_word, uint32_t call, cudaStream_t stream) {
-    return launch_kernel(true, publish_status_kernel, 1, 1, 0, stream, status, host_word, call);
+cudaError_t launch_publish_status(const int32_t* status, const int32_t* other, unsigned long long* host_word, uint32_t call,
+                                  cudaStream_t stream) {
+    return launch_kernel(true, publish_status_kernel, 1, 1, 0, stream, status, other, host_word, call);
 }
 
 // The first launch of a call. A call that ends with tensor-core convolutions leaves the SMs set up for 200 KB of shared

@@ -4,7 +4,8 @@ The sparse front end (voxelise, 14 sparse layers, dense BEV map with its zero bo
 (anchor decoding, score filter, rotated NMS) are the library's CUDA kernels. The 2D neck and head between them
 are plain dense convolutions, which the reference leaves to TensorRT's own layers (`addConvolutionNd`,
 `addDeconvolutionNd`, `addScale`, `addSoftMax`, :1262-1374); here they are torch's convolution calls in fp16
-with the batch norms folded in: library glue, as in the reference. Needs a CUDA device."""
+with the batch norms folded in: library glue, as in the reference. What lies between the convolutions (layout, bias, ReLU,
+the attention over the two branches, the 1x1 heads) is the library's. Needs a CUDA device."""
 from __future__ import annotations
 
 import numpy as np
@@ -80,47 +81,71 @@ class Neck2D:
             w = w * (scale[None, :, None, None] if transposed else scale[:, None, None, None])
             self.w[name] = torch.from_numpy(np.ascontiguousarray(w)).to(device).half().contiguous(memory_format=torch.channels_last)
             self.b[name] = torch.from_numpy(shift).to(device).half()
-        # the four heads read the same map: one convolution with 22 output channels
-        hw = np.concatenate([np.asarray(blobs[p + ".weight"], np.float32).reshape(c, 128, 1, 1) for _, p, c in HEAD_LAYERS])
+        # the attention's two 1x1 convolutions to one channel, and the four heads, which read the same map
+        self.gate_w = torch.cat([self.w.pop(n).reshape(1, 128) for n in ("w_0", "w_1")]).contiguous()
+        self.gate_b = torch.cat([self.b.pop(n).reshape(1) for n in ("w_0", "w_1")])
+        hw = np.concatenate([np.asarray(blobs[p + ".weight"], np.float32).reshape(c, 128) for _, p, c in HEAD_LAYERS])
         hb = np.concatenate([np.asarray(blobs[p + ".bias"], np.float32).reshape(c) for _, p, c in HEAD_LAYERS])
-        self.head_w = torch.from_numpy(hw).to(device).half().contiguous(memory_format=torch.channels_last)
+        self.head_w = torch.from_numpy(hw).to(device).half()
         self.head_b = torch.from_numpy(hb).to(device).half()
 
-    def _conv(self, x, name, relu=True):
-        F = self.torch.nn.functional
-        _n, _c, _b, _cin, _cout, _k, s, p = next(l for l in NECK_LAYERS if l[0] == name)
-        if name.startswith("deconv"):
-            y = F.conv_transpose2d(x, self.w[name], self.b[name], stride=s, padding=p, output_padding=1)
-        else:
-            y = F.conv2d(x, self.w[name], self.b[name], stride=s, padding=p)
-        return F.relu_(y) if relu else y
+    def _channels_last(self, x):
+        """x [B, C, H, W] with its channels last in memory."""
+        from . import _check, _stream, lib
 
-    def features(self, bev_padded):
-        """[B, 128, 202, 178] fp16 (the zero-padded BEV map) -> fused neck output [B, 128, 200, 176]."""
         torch = self.torch
-        x = bev_padded.contiguous(memory_format=torch.channels_last)
+        if x.is_contiguous(memory_format=torch.channels_last) or not x.is_contiguous():
+            return x.contiguous(memory_format=torch.channels_last)
+        B, C, H, W = x.shape
+        y = torch.empty_like(x, memory_format=torch.channels_last)
+        _check(lib().sessd_channels_last_enqueue(x.data_ptr(), y.data_ptr(), B, C, H * W, _stream()), "sessd_channels_last_enqueue")
+        return y
+
+    def _conv(self, x, name, add=None):
+        """relu(convolution + bias) (+ add)."""
+        from . import _check, _stream, lib
+
+        torch, F = self.torch, self.torch.nn.functional
+        _n, _c, _b, _cin, cout, _k, s, p = next(l for l in NECK_LAYERS if l[0] == name)
+        if name.startswith("deconv"):
+            y = F.conv_transpose2d(x, self.w[name], None, stride=s, padding=p, output_padding=1)
+        else:
+            y = F.conv2d(x, self.w[name], None, stride=s, padding=p)
+        y = y.contiguous(memory_format=torch.channels_last)
+        _check(lib().sessd_bias_relu_enqueue(y.data_ptr(), self.b[name].data_ptr(), None if add is None else add.data_ptr(),
+                                             y.numel() // cout, cout, _stream()), "sessd_bias_relu_enqueue")
+        return y
+
+    def _branches(self, bev_padded):
+        x = self._channels_last(bev_padded.half())
         for n in ("bu0_0", "bu0_1", "bu0_2"):
             x = self._conv(x, n)
         x0 = x
         for n in ("bu1_0", "bu1_1", "bu1_2"):
             x = self._conv(x, n)
         t0, t1 = self._conv(x0, "trans_0"), self._conv(x, "trans_1")
-        o0 = self._conv(self._conv(t1, "deconv_0") + t0, "conv_0")
-        o1 = self._conv(self._conv(t1, "deconv_1"), "conv_1")
-        w = torch.softmax(torch.cat([self._conv(o0, "w_0", relu=False), self._conv(o1, "w_1", relu=False)], dim=1).float(),
-                          dim=1).half()
-        return o0 * w[:, 0:1] + o1 * w[:, 1:2]
+        return self._conv(self._conv(t1, "deconv_0", add=t0), "conv_0"), self._conv(self._conv(t1, "deconv_1"), "conv_1")
+
+    def _tail(self, o0, o1, features=None, heads=(None,) * 4):
+        from . import _check, _stream, _vp, lib
+
+        _check(lib().sessd_neck_tail_enqueue(_vp(o0, o1, self.gate_w, self.gate_b, self.head_w, self.head_b),
+                                             _vp(features, *heads), o0.numel() // 128, _stream()), "sessd_neck_tail_enqueue")
+
+    def features(self, bev_padded):
+        """[B, 128, 202, 178] fp16 (the zero-padded BEV map) -> fused neck output [B, 128, 200, 176]."""
+        o0, o1 = self._branches(bev_padded)
+        out = self.torch.empty_like(o0)
+        self._tail(o0, o1, features=out)
+        return out
 
     def __call__(self, bev_padded):
         """-> dict of fp32 head outputs in the layout the post-processing plugins take:
         box [B, 70400, 7], cls [B, 70400, 1], iou [B, 70400, 1], dir [B, 70400, 2] (anchor = (y*W + x)*2 + a)."""
-        F = self.torch.nn.functional
-        y = F.conv2d(self.features(bev_padded), self.head_w, self.head_b).permute(0, 2, 3, 1).float()   # [B, H, W, 22]
-        B = y.shape[0]
-        out, c0 = {}, 0
-        for name, _p, c in HEAD_LAYERS:
-            out[name] = y[..., c0:c0 + c].reshape(B, -1, c // 2).contiguous()
-            c0 += c
+        o0, o1 = self._branches(bev_padded)
+        B, _, H, W = o0.shape
+        out = {name: self.torch.empty((B, H * W * 2, c // 2), device=o0.device) for name, _p, c in HEAD_LAYERS}
+        self._tail(o0, o1, heads=out.values())
         return out
 
 
@@ -180,7 +205,7 @@ class Detector:
         self._graph.replay()
         out = dict(self._out)
         if read_back_status:
-            out["status"] = read_status(self._ws) | read_status(self._out["filtered"]["workspace"])
+            out["status"] = read_status(self._ws, self._out["filtered"]["workspace"])
         return out
 
     def __call__(self, points, sizes):

@@ -1,0 +1,64 @@
+"""GPU: the kernels between the dense convolutions of the 2D neck, at the edges of their tiles, against torch in fp32.
+
+Layout and bias + ReLU (+ sum) round where separate fp16 operations round: bit for bit. The attention and the heads sum 128
+products in fp32, in another order than torch (128 * 2^-24 of the sum of magnitudes), and then round to fp16 (2^-11 of the
+value) after the sum, after the bias, the attention's weights, its two products and their sum."""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("batch,channels,pixels", [(1, 8, 1), (2, 64, 63), (1, 72, 65), (3, 128, 129), (1, 128, 202 * 178)])
+def test_channels_last(gpu, batch, channels, pixels):
+    import torch
+
+    x = torch.randn((batch, channels, pixels), device="cuda").half()
+    y = torch.empty((batch, pixels, channels), device="cuda", dtype=torch.float16)
+    assert gpu.lib().sessd_channels_last_enqueue(x.data_ptr(), y.data_ptr(), batch, channels, pixels, gpu._stream()) == 0
+    assert torch.equal(y, x.transpose(1, 2))
+
+
+@pytest.mark.parametrize("add", [False, True])
+@pytest.mark.parametrize("pixels,channels", [(1, 8), (33, 128), (100 * 88, 256), (200 * 176 * 3 + 1, 128)])
+def test_bias_relu(gpu, pixels, channels, add):
+    import torch
+
+    y = torch.randn((pixels, channels), device="cuda").half()
+    bias = torch.randn(channels, device="cuda").half()
+    other = torch.randn((pixels, channels), device="cuda").half() if add else None
+    want = torch.relu(y + bias)
+    want = want + other if add else want
+    assert gpu.lib().sessd_bias_relu_enqueue(y.data_ptr(), bias.data_ptr(), other.data_ptr() if add else None, pixels, channels,
+                                             gpu._stream()) == 0
+    assert torch.equal(y, want)
+    assert gpu.lib().sessd_bias_relu_enqueue(y.data_ptr(), bias.data_ptr(), None, pixels, 24, gpu._stream()) != 0
+
+
+@pytest.mark.parametrize("pixels", [1, 63, 64, 65, 2 * 200 * 176 + 7])
+def test_neck_tail(gpu, pixels):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(pixels)
+    rnd = lambda *s: torch.randn(s, generator=g, device="cuda").half()
+    o0, o1, gw, gb, hw, hb = rnd(pixels, 128), rnd(pixels, 128), rnd(2, 128) * 0.1, rnd(2), rnd(22, 128) * 0.1, rnd(22)
+    feat = torch.empty_like(o0)
+    heads = [torch.empty((pixels, c), device="cuda") for c in (14, 2, 2, 4)]
+    run = lambda f, h: gpu.lib().sessd_neck_tail_enqueue(gpu._vp(o0, o1, gw, gb, hw, hb), gpu._vp(f, *h), pixels, gpu._stream())
+    assert run(feat, heads) == 0
+    d = lambda t: t.double()
+    logit = torch.stack([(d(o0) * d(gw[0])).sum(1) + d(gb[0]), (d(o1) * d(gw[1])).sum(1) + d(gb[1])], 1)
+    w = torch.softmax(logit, 1)
+    want = d(o0) * w[:, :1] + d(o1) * w[:, 1:]
+    # a logit: its sum's error, two roundings; a weight moves by at most a quarter of the logits' errors, and is rounded
+    mag = lambda o, w, b: (d(o).abs() @ d(w).abs().T + d(b).abs())
+    slack = (128 * 2.0 ** -24 + 2 * 2.0 ** -11) * (mag(o0, gw[:1], gb[:1]) + mag(o1, gw[1:], gb[1:]))
+    tol = (d(o0).abs() + d(o1).abs()) * (slack / 4 + 2.0 ** -11 + 2 * 2.0 ** -11) + 2.0 ** -23
+    assert ((d(feat) - want).abs() <= tol).all()
+    out = d(feat) @ d(hw).T + d(hb)
+    tol = (129 * 2.0 ** -24 + 2 * 2.0 ** -11) * mag(feat, hw, hb) + 2.0 ** -23
+    assert ((d(torch.cat(heads, 1)) - out).abs() <= tol).all()
+    only = [torch.empty_like(h) for h in heads]
+    assert run(None, only) == 0 and all(torch.equal(a, b) for a, b in zip(only, heads))
+    only_feat = torch.empty_like(feat)
+    assert run(only_feat, [None] * 4) == 0 and torch.equal(only_feat, feat)
+    assert run(None, [None] * 4) != 0
