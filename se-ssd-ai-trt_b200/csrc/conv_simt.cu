@@ -120,7 +120,6 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
                    const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                    const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
                    T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
-    pdl_enter();
     using N = Narrow<T, CIN, COUT>;
     constexpr int TPR = N::TPR, ROWS = N::ROWS, OC = N::OC;
     constexpr int LOADS = (N::KVOL_MAX * ROWS + kThreads - 1) / kThreads;   // map entries a thread reads
@@ -153,12 +152,13 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
             entry[j] = k < kvol && ((mask >> k) & 1u) && o_next + row < n_next ? __ldg(nb + k * kNbrRun + row) : -1;
         }
     };
-    fetch();
-    if (next >= items) return;
+    // the weights are older than any preceding kernel
     for (int e = tid; e < kvol * CIN * COUT; e += kThreads) {
         const int k = e / (CIN * COUT);
-        s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(weights[e]);
+        s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(__ldg(weights + e));
     }
+    pdl_enter();
+    fetch();
     while (next < items) {
         const int b = b_next, o = row_next;
         const bool live = o_next + r < n_next;

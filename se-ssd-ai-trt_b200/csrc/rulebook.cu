@@ -331,8 +331,9 @@ __device__ __noinline__ void renumber_levels(const LevelChain& chain, int b, int
 
 // All levels of a chain in one launch (blocks 0 .. number_blocks - 1), and beside it the point lists of the voxeliser's
 // rows (the other blocks), which depend on the same kernel and on nothing here.
+constexpr int kLevelBlocks = 5;
 template <int WORDS>
-__global__ void __launch_bounds__(kThreads, 5)   // (renumber_levels would take 104 registers; it may spill)
+__global__ void __launch_bounds__(kThreads, kLevelBlocks)   // (renumber_levels would take 104 registers; it may spill)
 number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int max_voxels, int number_blocks, PointLists lists,
                      int32_t* status) {
     pdl_enter();
@@ -497,22 +498,29 @@ int launch_number_outputs(const BitGrid& out, int batch, int max_voxels, const S
     return SESSD_OK;
 }
 
-// One word per thread while there is a block for every chunk (a single frame: short chains), four above (fewer rounds of
-// a persistent grid).
+// As few words per thread (short chains) as let every chunk and the point lists have a resident block; else four, and
+// rounds of a persistent grid. (One frame of the network's levels: 843 chunks of one word per thread took two waves of blocks, 22 us.)
 int launch_number_levels(const LevelChain& chain, int batch, int max_voxels, const PointLists& lists, int32_t* status,
                          cudaStream_t stream) {
-    int64_t items = 0;
-    for (int l = 0; l < chain.count; ++l) items += (int64_t)batch * scan_chunks(chain.grid[l].words);
-    const int most = persistent_grid(6);
+    const int resident = persistent_grid(kLevelBlocks);
     const int64_t point_chunks = (int64_t)batch * scan_chunks(lists.max_points);
     const int list_blocks = (int)(point_chunks < persistent_grid(2) ? point_chunks : persistent_grid(2));
-    if (items <= most) {
-        SESSD_LAUNCH(number_levels_kernel<1>, (int)items + list_blocks, kThreads, 0, stream, chain, batch, max_voxels, (int)items,
-                     lists, status);
+    auto items = [&](int words) {
+        int64_t n = 0;
+        for (int l = 0; l < chain.count; ++l) n += (int64_t)batch * scan_chunks((chain.grid[l].words + words - 1) / words);
+        return n;
+    };
+#define SESSD_LEVELS(WORDS, BLOCKS)                                                                                            \
+    SESSD_LAUNCH(number_levels_kernel<WORDS>, (BLOCKS) + list_blocks, kThreads, 0, stream, chain, batch, max_voxels, (BLOCKS), lists, status)
+    if (items(1) + list_blocks <= resident) {
+        SESSD_LEVELS(1, (int)items(1));
+    } else if (items(2) + list_blocks <= resident) {
+        SESSD_LEVELS(2, (int)items(2));
     } else {
-        SESSD_LAUNCH(number_levels_kernel<4>, most + list_blocks, kThreads, 0, stream, chain, batch, max_voxels, most, lists,
-                     status);
+        const int64_t n = items(4);
+        SESSD_LEVELS(4, (int)(n < resident ? n : resident));
     }
+#undef SESSD_LEVELS
     return SESSD_OK;
 }
 
