@@ -330,8 +330,10 @@ __device__ __noinline__ void renumber_levels(const LevelChain& chain, int b, int
 }
 
 // All levels of a chain in one launch (blocks 0 .. number_blocks - 1), and beside it the point lists of the voxeliser's
-// rows (the other blocks), which depend on the same kernel and on nothing here.
-constexpr int kLevelBlocks = 5;
+// rows, which depend on the same kernel and on nothing here: by the other blocks, or where there are none by every block that
+// finds no more chunks (both parts are chains of dependent reads; blocks of their own for the lists only start when a
+// numbering block is through, and took two thirds of the kernel's 408 us on 32 frames x 120,000 points).
+constexpr int kLevelBlocks = 6;
 template <int WORDS>
 __global__ void __launch_bounds__(kThreads, kLevelBlocks)   // (renumber_levels would take 104 registers; it may spill)
 number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int max_voxels, int number_blocks, PointLists lists,
@@ -369,6 +371,7 @@ number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int ma
                 break;
             }
     }
+    if (number_blocks == (int)gridDim.x) push_points(lists, batch, blockIdx.x, gridDim.x);
 }
 
 // Generic variant of the tile mask for maps built by nbr_build_kernel: one warp per (tile, k).
@@ -510,15 +513,15 @@ int launch_number_levels(const LevelChain& chain, int batch, int max_voxels, con
         for (int l = 0; l < chain.count; ++l) n += (int64_t)batch * scan_chunks((chain.grid[l].words + words - 1) / words);
         return n;
     };
-#define SESSD_LEVELS(WORDS, BLOCKS)                                                                                            \
-    SESSD_LAUNCH(number_levels_kernel<WORDS>, (BLOCKS) + list_blocks, kThreads, 0, stream, chain, batch, max_voxels, (BLOCKS), lists, status)
+#define SESSD_LEVELS(WORDS, BLOCKS, LIST_BLOCKS)                                                                          \
+    SESSD_LAUNCH(number_levels_kernel<WORDS>, (BLOCKS) + (LIST_BLOCKS), kThreads, 0, stream, chain, batch, max_voxels, (BLOCKS), \
+                 lists, status)
     if (items(1) + list_blocks <= resident) {
-        SESSD_LEVELS(1, (int)items(1));
+        SESSD_LEVELS(1, (int)items(1), list_blocks);
     } else if (items(2) + list_blocks <= resident) {
-        SESSD_LEVELS(2, (int)items(2));
+        SESSD_LEVELS(2, (int)items(2), list_blocks);
     } else {
-        const int64_t n = items(4);
-        SESSD_LEVELS(4, (int)(n < resident ? n : resident));
+        SESSD_LEVELS(4, resident, 0);
     }
 #undef SESSD_LEVELS
     return SESSD_OK;
