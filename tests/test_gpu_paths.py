@@ -1,0 +1,125 @@
+"""GPU: the sizes at which a kernel changes its way of working, against the oracle (same tolerances as the tests whose helpers
+are used here: fp32 identical, fp16 1e-2 per layer)."""
+import numpy as np
+import pytest
+
+import make_golden_inputs as mk
+from test_gpu_backbone import _check_fp32_layers, _gpu_run, _oracle_layers
+from test_gpu_conv import _check_layer, _layer, _random_coords
+from test_gpu_postprocess import _check_filter
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("cin,cout,rows", [(64, 32, 300), (32, 64, 17760), (32, 64, 17761)])
+def test_fp32_register_tiles(gpu, oracle, cin, cout, rows):
+    """64 -> 32 channels; strips of 8 rows while every warp of the GPU gets one (148 SMs x 15 warps x 8 rows), of 16 above."""
+    rs = np.random.RandomState(rows)
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
+    c = _random_coords(rs, rows, layer.in_shape)
+    f = rs.randn(rows, cin).astype(np.float32)
+    _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, cin, cout) * 0.05).astype(np.float32), maxV=rows + 5)
+
+
+@pytest.mark.parametrize("rows", [148 * 128, 148 * 128 + 1])
+def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
+    rs = np.random.RandomState(rows)
+    layer = _layer(gpu, True, 32, 32, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
+    c = _random_coords(rs, rows, layer.in_shape)
+    f = rs.randn(rows, 32).astype(np.float32)
+    _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, 32, 32) * 0.05).astype(np.float32), dtype=1, maxV=rows + 200)
+
+
+def test_numbering_of_more_chunks_than_one_scan_group(gpu, oracle):
+    """41 x 1600 x 1408 output cells: 5,638 chunks of 256 words; running totals pass from group to group of 1024."""
+    rs = np.random.RandomState(5)
+    layer = _layer(gpu, False, 16, 32, (1, 1, 3), (1, 1, 1), (0, 0, 1), (41, 1600, 1408))
+    c = _random_coords(rs, 400, layer.in_shape)
+    f = rs.randn(len(c), 16).astype(np.float32)
+    _check_layer(gpu, oracle, layer, [(c, f), (c[:77], f[:77])], (rs.randn(3, 16, 32) * 0.05).astype(np.float32), maxV=1300)
+
+
+def test_filter_beyond_the_clustered_pass(gpu, oracle):
+    """133,120 anchors: more than a cluster holds (131,072), so two passes."""
+    _check_filter(gpu, oracle, 2, 260, 256, 500, -4.0, True, 11)
+
+
+def _case(gpu, layers, points, max_voxels, seed=3):
+    small = mk.small_case(gpu)
+    w, sc, sh = gpu.random_weights(seed=seed, layers=layers)
+    return dict(small, layers=layers, weights=w, scale=sc, shift=sh, points=np.ascontiguousarray(points), max_voxels=max_voxels)
+
+
+@pytest.mark.parametrize("K0,K1", [((1, 3, 3), (3, 3, 1)), ((2, 2, 2), (3, 1, 1)), ((3, 2, 1), (2, 3, 3))])
+def test_map_windows_of_other_kernels(gpu, oracle, K0, K1):
+    """Kernels other than 3x3x3 over the voxeliser's two-level grid (K0) and over a one-level grid (K1)."""
+    layers, shape = [], (41, 80, 64)
+    for i, (cin, cout, K) in enumerate(((4, 16, K0), (16, 32, K1))):
+        layers.append(_layer(gpu, False, cin, cout, K, tuple(min(k, 2) for k in K), tuple(k // 2 for k in K), shape))
+        shape = layers[-1].out_shape
+    layers.append(_layer(gpu, True, 32, 32, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape))
+    case = _case(gpu, tuple(layers), mk.small_case(gpu)["points"][:700], 16000)
+    _, views = _gpu_run(gpu, case, 0, frames=[case["points"]])
+    _check_fp32_layers(_oracle_layers(oracle, case, False), views)
+
+
+def test_front_end_with_more_points_than_rows(gpu, oracle):
+    """More points than max_voxels: voxels are numbered in point order, through a table, instead of in the grid's order."""
+    points = np.tile(mk.small_case(gpu)["points"][:90], (30, 1))
+    case = _case(gpu, mk.small_layers(gpu), points, 1200)
+    assert len(points) > case["max_voxels"]
+    _, views = _gpu_run(gpu, case, 0)
+    _check_fp32_layers(_oracle_layers(oracle, case, False), views)
+
+
+@pytest.mark.parametrize("max_voxels", [1500, 1537])
+def test_levels_that_lose_rows(gpu, max_voxels):
+    """A level with more rows than max_voxels keeps the first in (z, y, x) order, and the levels below see only those: what a
+    chain of strided plugin calls with the same max_voxels gives. Two frames, the second of which loses none."""
+    import torch
+
+    small = mk.small_case(gpu)
+    layers = mk.small_layers(gpu)
+    frames = [small["points"], small["points"][:60]]
+    pts = torch.zeros((2, 1500, 4))
+    for b, f in enumerate(frames):
+        pts[b, :len(f)] = torch.from_numpy(f)
+    sizes = torch.tensor([len(f) for f in frames], dtype=torch.int32).cuda()
+    bb = gpu.Backbone(max_voxels, small["weights"], small["scale"], small["shift"], dtype=0, layers=layers,
+                      point_range=small["range"], voxel_size=small["voxel"])
+    _, ws = bb.run(pts.cuda(), sizes)
+    assert gpu.read_status(ws) & gpu.STATUS_VOXEL_OVERFLOW
+    view = lambda i: [t.clone() for t in bb.layer_view(ws, 2, 1500, i)]
+    lost = 0
+    for i, l in enumerate(layers):
+        if l.subm:
+            continue
+        f, c, n = view(i - 1)
+        p = gpu.conv_params(l, max_voxels)
+        w = gpu.ConvWeights(p, small["weights"][i], small["scale"][i], small["shift"][i], True, 0)
+        r = gpu.sparse_conv(f, c, n, p, w)
+        gf, gc, gn = view(i)
+        lost += bool(r["status"] & gpu.STATUS_VOXEL_OVERFLOW)
+        assert torch.equal(gn, r["voxel_num"]) and int(gn[0]) <= max_voxels
+        for b in range(2):
+            m = int(gn[b])
+            assert torch.equal(gc[b, :m], r["coors"][b, :m]) and torch.equal(gf[b, :m], r["features"][b, :m])
+        w.close()
+    assert lost
+    bb.close()
+
+
+def test_status_is_not_read_during_capture(gpu):
+    import torch
+
+    ws = torch.zeros(1024, dtype=torch.uint8, device="cuda")
+    other = ws.clone()
+    other[0] = 4
+    assert gpu.read_status(ws) == 0 and gpu.read_status(ws, other) == 4
+    g, x = torch.cuda.CUDAGraph(), torch.zeros(8, device="cuda")
+    with torch.cuda.graph(g):
+        x += 1
+        with pytest.raises(gpu.SessdError):
+            gpu.read_status(ws)
+    g.replay()
+    assert gpu.read_status(ws) == 0 and float(x[0]) == 1.0
