@@ -1,13 +1,13 @@
 // Rotated non-maximum suppression in the bird's-eye view on the GPU.
 //
 // Replaces the host functions nms_cpu / box_overlap of the reference (se-ssd-ai-trt.cpp:97-273), which run
-// after the score filter on at most max_box_num boxes per frame. Three small kernels per call:
+// after the score filter on at most max_box_num boxes per frame. Two small kernels per call:
 //   1. per frame: rank the boxes by descending score (equal scores: lower row first; the reference's
 //      std::sort leaves that open) and store every box's rotated corners and the cos/sin of -yaw once
 //      (the reference recomputes them for every pair);
 //   2. pairs: one thread per (box i, later box j) computes the IoU by the reference's polygon rule; a warp
-//      covers 32 consecutive j and packs its "i suppresses j" bits with a ballot;
-//   3. per frame: one warp walks the boxes in rank order, 64 at a time, keeps the ones not yet suppressed,
+//      covers 32 consecutive j and packs its "i suppresses j" bits with a ballot,
+//      and the last block of a frame walks the boxes in rank order, 64 at a time, keeps the ones not yet suppressed,
 //      ORs their bit rows into the suppressed set, and writes the kept boxes in that order.
 // Arithmetic is fp32 with explicit round-to-nearest operations (no contraction), in the reference's order.
 #include "common.cuh"
@@ -131,6 +131,7 @@ struct NmsArgs {
     int32_t* order;           // [B][M]  rank -> input row
     float* geom;              // [B][M][16]
     unsigned long long* mask; // [B][M][words]
+    uint32_t* done;           // [B] blocks of the second kernel that are through with the frame
     int batch, max_box, words;
     float thresh;
 };
@@ -158,6 +159,7 @@ nms_rank_kernel(NmsArgs a, uint32_t* status) {
     const int share = blockIdx.x % kRankBlocks;
     for (int b = blockIdx.x / kRankBlocks; b < a.batch; b += gridDim.x / kRankBlocks) {
         const int n = frame_count(a, b);
+        if (share == 0 && threadIdx.x == 0) a.done[b] = 0u;
         const float* bx = a.boxes + (size_t)b * a.max_box * 9;
         __syncthreads();
         for (int j = threadIdx.x; j < n; j += kThreads) s_score[j] = rank_score(bx[j * 9 + 8]);
@@ -199,24 +201,115 @@ nms_rank_kernel(NmsArgs a, uint32_t* status) {
     }
 }
 
+// The greedy pass over a frame in rank order, by one block. When the frame's part of the mask fits the
+// block's shared memory all threads stage it there first; warp 0 then walks the boxes 64 at a time (lane w
+// holds word w of the suppressed set): the 64 x 64 diagonal block of the mask is fetched with one load per
+// lane and resolved with shuffles (no memory access between dependent steps), then the full mask rows of the
+// boxes kept in the block are ORed into the suppressed set with independent loads. All threads write the
+// kept boxes in rank order.
+constexpr int kMaskWarps = 8, kMaskThreads = kMaskWarps * 32;
+__device__ void greedy_pass(const NmsArgs& a, int b, int n, unsigned long long* s_mask, int smem_words) {
+    __shared__ unsigned long long s_keep[32];
+    __shared__ int s_base[33];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int words_n = (n + 63) >> 6;
+    const float* bx = a.boxes + (size_t)b * a.max_box * 9;
+    float* out = a.kept + (size_t)b * a.max_box * 9;
+    const unsigned long long* mask = a.mask + (size_t)b * a.max_box * a.words;
+    int stride = a.words;
+    if (n * words_n <= smem_words) {
+        // only words from the one that holds the row itself onward are ever written or read
+        for (int e = threadIdx.x; e < n * words_n; e += kMaskThreads) {
+            const int i = e / words_n, w = e - i * words_n;
+            s_mask[e] = w >= (i >> 6) ? mask[(size_t)i * a.words + w] : 0ull;
+        }
+        mask = s_mask;
+        stride = words_n;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        unsigned long long removed = 0ull, keepw = 0ull;
+        for (int c = 0; c < words_n; ++c) {
+            const int i0 = c * 64 + lane, i1 = i0 + 32;
+            const unsigned long long d0 = i0 < n ? mask[(size_t)i0 * stride + c] : 0ull;
+            const unsigned long long d1 = i1 < n ? mask[(size_t)i1 * stride + c] : 0ull;
+            unsigned long long rem = __shfl_sync(0xFFFFFFFFu, removed, c);
+            unsigned long long keep = 0ull;
+            const int rows = min(64, n - c * 64);
+            const unsigned long long all = rows < 64 ? (1ull << rows) - 1ull : ~0ull;
+            // from one kept box to the next (every quantity here is uniform over the warp)
+            for (unsigned long long left = all & ~rem; left; left &= ~rem) {
+                const int r = __ffsll((long long)left) - 1;
+                keep |= 1ull << r;
+                rem |= __shfl_sync(0xFFFFFFFFu, r < 32 ? d0 : d1, r & 31) | (1ull << r);
+            }
+            if (lane == c) keepw = keep;
+            // eight rows per round, so that eight loads are in flight before the first OR waits for one
+            unsigned long long acc = 0ull;
+            const bool mine = lane > c && lane < words_n;
+            for (unsigned long long kk = keep; kk;) {
+                unsigned long long v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    v[u] = 0ull;
+                    if (kk) {
+                        const int r = __ffsll((long long)kk) - 1;
+                        kk &= kk - 1ull;
+                        if (mine) v[u] = mask[(size_t)(c * 64 + r) * stride + lane];
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc |= v[u];
+            }
+            removed |= acc;
+        }
+        const int cnt = __popcll(keepw);
+        int incl = cnt;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        s_keep[lane] = keepw;
+        s_base[lane] = incl - cnt;
+        if (lane == 31) s_base[32] = incl;
+    }
+    __syncthreads();
+    // output rows: kept boxes in rank order
+    const int total = s_base[32];
+    for (int i = threadIdx.x; i < n; i += kMaskThreads) {
+        const int c = i >> 6, r = i & 63;
+        const unsigned long long kw = s_keep[c];
+        if ((kw >> r) & 1ull) {
+            const int pos = s_base[c] + __popcll(kw & ((1ull << r) - 1ull));
+            const int src = a.order[(size_t)b * a.max_box + i];
+            if ((unsigned)src >= (unsigned)n) continue;   // cannot happen with a total order; never read out of bounds
+#pragma unroll
+            for (int e = 0; e < 9; ++e) out[(size_t)pos * 9 + e] = bx[(size_t)src * 9 + e];
+        }
+    }
+    for (int e = total * 9 + threadIdx.x; e < a.max_box * 9; e += kMaskThreads) out[e] = 0.f;   // rows after the count
+    if (threadIdx.x == 0) a.kept_num[b] = (uint32_t)total;
+}
+
 // Kernel 2: bit j of mask[b][i][w] = ranked box i suppresses ranked box w*64 + j (only j > i matter).
 // One warp per (box i, 32-box column segment): lane = column, one IoU per thread, the 32 decisions packed
 // by a ballot into half of a 64-bit mask word. Segments from the word that holds i itself up to the last
 // word in use are always written (zeros where j <= i or j >= n), so the greedy pass never reads stale bits.
-constexpr int kMaskWarps = 8;
-__global__ void __launch_bounds__(kMaskWarps * 32)
-nms_mask_kernel(NmsArgs a) {
+// A frame has blocks_per_frame blocks; the last of them to finish then makes the greedy pass (as a kernel of its own it cost
+// the host a launch, 5 us of a call that is host time for the most part, and the GPU the wait for it).
+__global__ void __launch_bounds__(kMaskThreads, 4)
+nms_mask_kernel(NmsArgs a, int blocks_per_frame, int smem_words) {
     pdl_enter();
+    extern __shared__ unsigned long long s_mask[];
+    __shared__ bool s_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int segs = a.words * 2;
-    const int64_t per_frame = (int64_t)a.max_box * segs;
-    const int64_t items = (int64_t)a.batch * per_frame;
-    for (int64_t it = (int64_t)blockIdx.x * kMaskWarps + warp; it < items; it += (int64_t)gridDim.x * kMaskWarps) {
-        const int b = (int)(it / per_frame);
-        const int r = (int)(it - (int64_t)b * per_frame);
+    const int b = blockIdx.x / blocks_per_frame, block = blockIdx.x - b * blocks_per_frame;
+    const int n = frame_count(a, b);
+    const int segs = ((n + 63) >> 6) * 2;
+    for (int r = block * kMaskWarps + warp; r < n * segs; r += blocks_per_frame * kMaskWarps) {
         const int i = r / segs, seg = r - i * segs;
-        const int n = frame_count(a, b);
-        if (i >= n || seg < (i >> 6) * 2 || seg >= ((n + 63) >> 6) * 2) continue;   // uniform over the warp
+        if (seg < (i >> 6) * 2) continue;                    // uniform over the warp
         const int j = seg * 32 + lane;
         bool hit = false;
         if (j > i && j < n) {
@@ -242,104 +335,13 @@ nms_mask_kernel(NmsArgs a) {
         if (lane == 0)   // little-endian halves of the 64-bit word: even segment = low half
             reinterpret_cast<uint32_t*>(a.mask + ((size_t)b * a.max_box + i) * a.words)[seg] = bits;
     }
-}
-
-// Kernel 3: greedy pass in rank order, one block per frame. When the frame's part of the mask fits the
-// block's shared memory all threads stage it there first; warp 0 then walks the boxes 64 at a time (lane w
-// holds word w of the suppressed set): the 64 x 64 diagonal block of the mask is fetched with one load per
-// lane and resolved with shuffles (no memory access between dependent steps), then the full mask rows of the
-// boxes kept in the block are ORed into the suppressed set with independent loads. All threads write the
-// kept boxes in rank order.
-constexpr int kReduceThreads = 512;
-__global__ void __launch_bounds__(kReduceThreads)
-nms_reduce_kernel(NmsArgs a, int smem_words) {
-    pdl_enter();
-    extern __shared__ unsigned long long s_mask[];
-    __shared__ unsigned long long s_keep[32];
-    __shared__ int s_base[33];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int b = blockIdx.x; b < a.batch; b += gridDim.x) {
-        const int n = frame_count(a, b);
-        const int words_n = (n + 63) >> 6;
-        const float* bx = a.boxes + (size_t)b * a.max_box * 9;
-        float* out = a.kept + (size_t)b * a.max_box * 9;
-        const unsigned long long* mask = a.mask + (size_t)b * a.max_box * a.words;
-        int stride = a.words;
-        __syncthreads();   // the previous frame is done with the shared arrays
-        if (n * words_n <= smem_words) {
-            // only words from the one that holds the row itself onward are ever written or read
-            for (int e = threadIdx.x; e < n * words_n; e += kReduceThreads) {
-                const int i = e / words_n, w = e - i * words_n;
-                s_mask[e] = w >= (i >> 6) ? mask[(size_t)i * a.words + w] : 0ull;
-            }
-            mask = s_mask;
-            stride = words_n;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long removed = 0ull, keepw = 0ull;
-            for (int c = 0; c < words_n; ++c) {
-                const int i0 = c * 64 + lane, i1 = i0 + 32;
-                const unsigned long long d0 = i0 < n ? mask[(size_t)i0 * stride + c] : 0ull;
-                const unsigned long long d1 = i1 < n ? mask[(size_t)i1 * stride + c] : 0ull;
-                unsigned long long rem = __shfl_sync(0xFFFFFFFFu, removed, c);
-                unsigned long long keep = 0ull;
-                const int rows = min(64, n - c * 64);
-                const unsigned long long all = rows < 64 ? (1ull << rows) - 1ull : ~0ull;
-                // from one kept box to the next (every quantity here is uniform over the warp)
-                for (unsigned long long left = all & ~rem; left; left &= ~rem) {
-                    const int r = __ffsll((long long)left) - 1;
-                    keep |= 1ull << r;
-                    rem |= __shfl_sync(0xFFFFFFFFu, r < 32 ? d0 : d1, r & 31) | (1ull << r);
-                }
-                if (lane == c) keepw = keep;
-                // eight rows per round, so that eight loads are in flight before the first OR waits for one
-                unsigned long long acc = 0ull;
-                const bool mine = lane > c && lane < words_n;
-                for (unsigned long long kk = keep; kk;) {
-                    unsigned long long v[8];
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) {
-                        v[u] = 0ull;
-                        if (kk) {
-                            const int r = __ffsll((long long)kk) - 1;
-                            kk &= kk - 1ull;
-                            if (mine) v[u] = mask[(size_t)(c * 64 + r) * stride + lane];
-                        }
-                    }
-#pragma unroll
-                    for (int u = 0; u < 8; ++u) acc |= v[u];
-                }
-                removed |= acc;
-            }
-            const int cnt = __popcll(keepw);
-            int incl = cnt;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const int v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-                if (lane >= d) incl += v;
-            }
-            s_keep[lane] = keepw;
-            s_base[lane] = incl - cnt;
-            if (lane == 31) s_base[32] = incl;
-        }
-        __syncthreads();
-        // output rows: kept boxes in rank order
-        const int total = s_base[32];
-        for (int i = threadIdx.x; i < n; i += kReduceThreads) {
-            const int c = i >> 6, r = i & 63;
-            const unsigned long long kw = s_keep[c];
-            if ((kw >> r) & 1ull) {
-                const int pos = s_base[c] + __popcll(kw & ((1ull << r) - 1ull));
-                const int src = a.order[(size_t)b * a.max_box + i];
-                if ((unsigned)src >= (unsigned)n) continue;   // cannot happen with a total order; never read out of bounds
-#pragma unroll
-                for (int e = 0; e < 9; ++e) out[(size_t)pos * 9 + e] = bx[(size_t)src * 9 + e];
-            }
-        }
-        for (int e = total * 9 + threadIdx.x; e < a.max_box * 9; e += kReduceThreads) out[e] = 0.f;   // rows after the count
-        if (threadIdx.x == 0) a.kept_num[b] = (uint32_t)total;
-    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(a.done + b, 1u) == (uint32_t)(blocks_per_frame - 1);
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    greedy_pass(a, b, n, s_mask, smem_words);
 }
 
 bool nms_params_ok(const sessd_nms_params* p, int batch) {
@@ -362,6 +364,7 @@ size_t sessd_rotated_nms_workspace_bytes(const sessd_nms_params* p, int batch) {
     bump.take<int32_t>((size_t)batch * M);
     bump.take<float>((size_t)batch * M * kGeomFloats);
     bump.take<unsigned long long>((size_t)batch * M * words);
+    bump.take<uint32_t>(batch);
     return bump.total();
 }
 
@@ -384,21 +387,22 @@ int sessd_rotated_nms_enqueue(const sessd_nms_params* p, int batch, const void* 
     a.order = bump.take<int32_t>((size_t)batch * M);
     a.geom = bump.take<float>((size_t)batch * M * kGeomFloats);
     a.mask = bump.take<unsigned long long>((size_t)batch * M * words);
+    a.done = bump.take<uint32_t>(batch);
     a.batch = batch;
     a.max_box = p->max_box_num;
     a.words = (int)words;
     a.thresh = p->nms_thresh;
-    const int frames_grid = batch < persistent_grid(8) ? batch : persistent_grid(8);
     const int rank_grid = (batch < persistent_grid(1) ? batch : persistent_grid(1)) * kRankBlocks;
     SESSD_LAUNCH(nms_rank_kernel, rank_grid, kThreads, M * sizeof(float), stream, a, static_cast<uint32_t*>(workspace));
-    const int64_t pair_blocks = ((int64_t)batch * M * words * 2 + kMaskWarps - 1) / kMaskWarps;
-    const int pair_grid = (int)(pair_blocks < persistent_grid(8) ? pair_blocks : persistent_grid(8));
-    SESSD_LAUNCH(nms_mask_kernel, pair_grid, kMaskWarps * 32, 0, stream, a);
     // the staged copy of a frame's mask must fit the 48 KB a block gets without opting in; larger tables are read in place
     const size_t stage_bytes = M * words * sizeof(unsigned long long);
     const int smem_words = stage_bytes <= 40 * 1024 ? (int)(M * words) : 0;
-    SESSD_LAUNCH(nms_reduce_kernel, frames_grid, kReduceThreads, (size_t)smem_words * sizeof(unsigned long long), stream, a,
-                 smem_words);
+    // a warp per (box, segment) of a full frame, unless the frames of the batch have to share the GPU
+    const int most = persistent_grid(4) / batch > 1 ? persistent_grid(4) / batch : 1;
+    const int full = (int)((M * words * 2 + kMaskWarps - 1) / kMaskWarps);
+    const int blocks_per_frame = full < most ? full : most;
+    SESSD_LAUNCH(nms_mask_kernel, batch * blocks_per_frame, kMaskThreads, (size_t)smem_words * sizeof(unsigned long long), stream,
+                 a, blocks_per_frame, smem_words);
     return SESSD_OK;
 }
 
