@@ -111,7 +111,7 @@ void conv_workspace_layout(Bump& bump, const sessd_conv_params* p, const ConvGeo
         w->ones_bytes = (size_t)batch * capb * 8 * sizeof(uint32_t);
     } else {
         uint32_t* block = bump.take<uint32_t>(per * 2);
-        w->in_table = Table{block, nullptr, reinterpret_cast<int32_t*>(block ? block + per : nullptr), cap, shift, 1, 1};
+        w->in_table = Table{block, reinterpret_cast<int32_t*>(block ? block + per : nullptr), cap, shift};
         w->ones_base = block;
         w->ones_bytes = per * 2 * sizeof(uint32_t);
     }

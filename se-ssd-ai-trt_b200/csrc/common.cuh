@@ -118,21 +118,22 @@ inline int ilog2(uint32_t v) {
 
 // One open-addressing coordinate table per frame: frame b owns slots [b*cap, (b+1)*cap).
 // keys: linear cell index inside the frame's grid, kEmpty when free.
-// rank: smallest producer index seen for the key (drives deterministic numbering); stride
-//       `rank_stride` between consecutive slots so that the voxeliser's per-slot point lists
-//       (whose first element is that minimum) can serve as the rank array.
 // vals: row index of the key, -1 when the key has no row.
-// Output tables of strided layers pack key and rank into one 64-bit slot (key in the high word), so that
-// claiming a cell and lowering its rank is a single atomic; keys/rank then point into that array with
-// stride 2.
 struct Table {
     uint32_t* keys;
-    uint32_t* rank;
     int32_t* vals;
     uint32_t cap;       // power of two
     int shift;          // 32 - log2(cap)
-    int rank_stride;
-    int key_stride;     // 1 for separate key / rank arrays; 2 when a slot is one 64-bit word (key << 32 | rank)
+};
+
+// The voxeliser's table. A slot is (point that claimed the cell) << 32 | key, ~0 when free; the cell's other points are listed
+// under the claiming point. Most cells have one point, so that little beside the slots is touched at random, and what
+// belongs to a point lies in point order.
+struct VoxelTable {
+    unsigned long long* slots;   // [B][cap]
+    uint32_t* lists;             // [B][max_points][max_points_per_voxel], ascending, kEmpty when free
+    uint32_t cap;                // power of two
+    int shift;                   // 32 - log2(cap)
 };
 
 // x-grouped coordinate table of one resolution level: frame b owns buckets [b*cap, (b+1)*cap), a
@@ -424,13 +425,13 @@ int launch_zero_pad2d(const void* in, void* out, size_t planes, int H, int W, in
 // voxelize.cu
 struct VoxelWorkspace {
     int32_t* status;
-    Table table;          // rank = per-slot sorted point list [cap][max_pts]
-    int32_t* pt_slot;     // [B][max_points]
+    VoxelTable table;
+    int32_t* pt_claim;    // [B][max_points] the point that claimed the point's cell, -1 outside the range
     ScanState scan;       // numbering of the owner points
     void* zero_base;      // the scan's words, to be zero before a call
     size_t zero_bytes;
     int32_t* num_points;  // [B][max_voxels]
-    size_t table_bytes;   // bytes to set to 0xFF before a call (keys + point lists)
+    size_t table_bytes;   // bytes to set to 0xFF before a call (slots and lists)
     void* table_base;
 };
 void voxel_workspace_layout(Bump& bump, const sessd_voxel_params* p, int batch, int max_points, VoxelWorkspace* w);

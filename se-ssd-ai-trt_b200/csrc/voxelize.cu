@@ -3,14 +3,16 @@
 // Replaces the reference's dense-grid voxeliser (voxelGenerator.cu:348-451, 255-321), which zeroes
 // a 739 MB coordinate table every frame and lets a thread spin until another thread has published a
 // voxel id. Here each frame owns a small open-addressing table keyed by the linear cell index:
-//   pass 1 (insert)  every point claims/finds its cell's slot and pushes its index through the
-//                    slot's ascending list of the max_points_per_voxel smallest point indices
-//                    (a cascade of atomicMin, so the list content does not depend on timing);
-//   pass 2 (emit)    the owner points (index == smallest index of the slot) are numbered in point order with a
+//   pass 1 (insert)  every point claims its cell's slot, or finds the point that has and pushes its index through that
+//                    one's ascending list of the max_points_per_voxel smallest other points (a cascade of atomicMin;
+//                    which point claims a cell depends on timing, the cell's points do not);
+//   pass 2 (emit)    the owner points (the smallest index of their cell) are numbered in point order with a
 //                    one-pass scan (scan.cuh); the owner writes coordinates, count and the mean of the listed points,
 //                    summed in ascending index order.
 // Results are therefore bit-reproducible. A single frame is bound by the chain of dependent reads and launches, not by
-// bytes: as seven launches (reset, insert, count, emit, three tails) 20,000 points took 46 us, as three 19.
+// bytes: as seven launches (reset, insert, count, emit, three tails) 20,000 points took 46 us, as three 18. A batch is bound by
+// the random accesses of pass 1: with the lists in the slots (24 or 32 bytes each) the table of 64 frames x 20,000 points
+// did not fit L2 and the call took 133 - 136 us.
 // The fused front end numbers its voxels in space instead where it can (voxel_grid.cu).
 #include "fill.cuh"
 #include "rulebook.cuh"
@@ -23,7 +25,7 @@ namespace {
 
 __global__ void __launch_bounds__(kThreads)
 voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch,
-                    int max_points, VoxGeom g, Table t, int max_pts, int32_t* __restrict__ pt_slot,
+                    int max_points, VoxGeom g, VoxelTable t, int max_pts, int32_t* __restrict__ pt_claim,
                     int32_t* status) {
     pdl_enter();
     const int chunks = (max_points + kThreads - 1) / kThreads;
@@ -35,15 +37,23 @@ voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict
         n = n > max_points ? max_points : n;
         if (p >= n) continue;
         const float4 pt = __ldg(&points[(size_t)b * max_points + p]);
-        int slot = -1;
+        int claim = -1;
         int ix, iy, iz;
         if (voxel_cell(g, pt, &ix, &iy, &iz)) {
             const uint32_t key = ((uint32_t)iz * g.gy + iy) * g.gx + ix;
-            slot = table_insert(t.keys + (size_t)b * t.cap, t.cap, t.shift, key);
-            if (slot < 0) atomicOr(status, SESSD_STATUS_HASH_FULL);
-            else list_push(t.rank + ((size_t)b * t.cap + (uint32_t)slot) * max_pts, max_pts, (uint32_t)p);
+            // most cells have one point: a free slot takes it with one swap, made without looking first
+            unsigned long long* slots = t.slots + (size_t)b * t.cap;
+            uint32_t h = hash_slot(key, t.shift);
+            for (uint32_t probe = 0; probe < t.cap; ++probe, h = (h + 1) & (t.cap - 1)) {
+                const unsigned long long old = atomicCAS(slots + h, ~0ull, (unsigned long long)p << 32 | key);
+                if (old != ~0ull && (uint32_t)old != key) continue;
+                claim = old == ~0ull ? p : (int)(old >> 32);
+                break;
+            }
+            if (claim < 0) atomicOr(status, SESSD_STATUS_HASH_FULL);
+            else if (claim != p) list_push(t.lists + ((size_t)b * max_points + claim) * max_pts, max_pts, (uint32_t)p);
         }
-        pt_slot[(size_t)b * max_points + p] = slot;
+        pt_claim[(size_t)b * max_points + p] = claim;
     }
 }
 
@@ -61,7 +71,7 @@ struct VoxelOut {
 template <typename T>
 __global__ void __launch_bounds__(kThreads)
 voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch, int max_points,
-                  VoxGeom g, Table t, int max_pts, const int32_t* __restrict__ pt_slot, ScanState scan, VoxelOut<T> out) {
+                  VoxGeom g, VoxelTable t, int max_pts, const int32_t* __restrict__ pt_claim, ScanState scan, VoxelOut<T> out) {
     pdl_enter();
     const int chunks = scan_chunks(max_points), items = batch * chunks;
     for (int ticket = scan_first(scan.ticket, items, gridDim.x); ticket >= 0;
@@ -72,16 +82,21 @@ voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__
         const int used = n > 0 ? scan_chunks(n) : 1;
         if (c >= used) continue;                   // uniform over the block
         const int e = c * kThreads + threadIdx.x;
-        const int slot = e < n ? pt_slot[(size_t)b * max_points + e] : -1;
-        const size_t gslot = (size_t)b * t.cap + (uint32_t)slot;
-        // the cell's points; the first one owns the cell
+        const int claim = e < n ? pt_claim[(size_t)b * max_points + e] : -1;
+        // the cell's points, the claiming one among its list; the first of them owns the cell
         uint32_t pi[kMaxPointsPerVoxel];
-        uint32_t key = 0;
-        if (slot >= 0) {
-            key = t.keys[gslot];
-            list_load(t.rank + gslot * max_pts, max_pts, pi);
+        bool owner = false;
+        if (claim >= 0) {
+            list_load(t.lists + ((size_t)b * max_points + claim) * max_pts, max_pts, pi);
+            uint32_t carry = (uint32_t)claim;
+#pragma unroll
+            for (int j = 0; j < kMaxPointsPerVoxel; ++j) {
+                if (j >= max_pts) break;
+                const uint32_t v = pi[j];
+                pi[j] = min(v, carry), carry = max(v, carry);
+            }
+            owner = pi[0] == (uint32_t)e;
         }
-        const bool owner = slot >= 0 && pi[0] == (uint32_t)e;
         int end;
         const int id = scan_position(scan.state + (size_t)b * chunks, c, owner ? 1 : 0, &end, out.status);
         if (c == used - 1 && threadIdx.x == 0) {
@@ -101,9 +116,8 @@ voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__
             continue;
         }
         if (id >= out.max_voxels) continue;
-        const int plane = g.gy * g.gx;
-        const int iz = key / plane, rem = key - iz * plane;
-        const int iy = rem / g.gx, ix = rem - iy * g.gx;
+        int ix, iy, iz;
+        voxel_cell(g, __ldg(points + (size_t)b * max_points + e), &ix, &iy, &iz);
         const size_t row = (size_t)b * out.max_voxels + id;
         reinterpret_cast<int4*>(out.coors)[row] = make_int4(b, iz, iy, ix);
         int cnt;
@@ -159,20 +173,13 @@ int launch_fill_zero(void* ptr, size_t bytes, cudaStream_t stream) {
 
 void voxel_workspace_layout(Bump& bump, const sessd_voxel_params* p, int batch, int max_points, VoxelWorkspace* w) {
     const uint32_t cap = pow2_at_least(2ull * (uint64_t)max_points);
-    // keys and point lists are contiguous so that one fill resets both.
-    const size_t key_elems = (size_t)batch * cap;
-    const size_t list_elems = key_elems * p->max_points_per_voxel;
-    uint32_t* block = bump.take<uint32_t>(key_elems + list_elems);
+    const size_t slots = (size_t)batch * cap;
+    const size_t lists = ((size_t)batch * max_points * p->max_points_per_voxel + 3) / 4 * 4;   // (filled 16 bytes at a time)
+    uint32_t* block = bump.take<uint32_t>(2 * slots + lists);   // contiguous, so that one fill resets both
+    w->table = VoxelTable{reinterpret_cast<unsigned long long*>(block), block ? block + 2 * slots : nullptr, cap, 32 - ilog2(cap)};
     w->table_base = block;
-    w->table_bytes = (key_elems + list_elems) * sizeof(uint32_t);
-    w->table.keys = block;
-    w->table.rank = block ? block + key_elems : nullptr;
-    w->table.vals = nullptr;
-    w->table.cap = cap;
-    w->table.shift = 32 - ilog2(cap);
-    w->table.rank_stride = p->max_points_per_voxel;
-    w->table.key_stride = 1;
-    w->pt_slot = bump.take<int32_t>((size_t)batch * max_points);
+    w->table_bytes = (2 * slots + lists) * sizeof(uint32_t);
+    w->pt_claim = bump.take<int32_t>((size_t)batch * max_points);
     w->zero_bytes = scan_state_bytes(max_points, batch);
     char* zero = bump.take<char>(w->zero_bytes);
     w->zero_base = zero;
@@ -188,15 +195,15 @@ int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out
     const int64_t items = (int64_t)batch * scan_chunks(max_points);
     const int grid = (int)(items < persistent_grid(8) ? items : persistent_grid(8));
     SESSD_LAUNCH(voxel_insert_kernel, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                 p->max_points_per_voxel, w.pt_slot, w.status);
+                 p->max_points_per_voxel, w.pt_claim, w.status);
     if (out_dtype == SESSD_F32) {
         VoxelOut<float> o{static_cast<float*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
         SESSD_LAUNCH(voxel_emit_kernel<float>, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                     p->max_points_per_voxel, w.pt_slot, w.scan, o);
+                     p->max_points_per_voxel, w.pt_claim, w.scan, o);
     } else {
         VoxelOut<__half> o{static_cast<__half*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
         SESSD_LAUNCH(voxel_emit_kernel<__half>, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                     p->max_points_per_voxel, w.pt_slot, w.scan, o);
+                     p->max_points_per_voxel, w.pt_claim, w.scan, o);
     }
     return SESSD_OK;
 }
