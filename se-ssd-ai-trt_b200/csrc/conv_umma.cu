@@ -552,28 +552,31 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = (kvol + KG - 1) / KG;
 
-    if (tid == 0) {
-        for (int s = 0; s < NSLOT; ++s) {
+    if (tid < THREADS / 2) {   // side by side: one thread would take half a microsecond for the hundred and more barriers
+        if (tid < NSLOT) {
             for (int i = 0; i < MMA_WARPS; ++i)
-                mbar_init(smem_u32(&ctl->a_full[i][s]), 32);   // the lanes of the gather warp that owns the slot
-            mbar_init(smem_u32(&ctl->a_empty[s]), 1);
+                mbar_init(smem_u32(&ctl->a_full[i][tid]), 32);   // the lanes of the gather warp that owns the slot
+            mbar_init(smem_u32(&ctl->a_empty[tid]), 1);
         }
-        for (int j = 0; j < NIDX; ++j) {
+        if (tid >= 32 && tid < 32 + NIDX) {
+            const int j = tid - 32;
             ctl->idx_uses[j] = 0;
-            mbar_init(smem_u32(&ctl->i_full[j]), 1);           // the lane of the index warp that issues the block's copy
-            mbar_init(smem_u32(&ctl->i_empty[j]), 32);         // the lanes of the gather warp
+            mbar_init(smem_u32(&ctl->i_full[j]), 1);             // the lane of the index warp that issues the block's copy
+            mbar_init(smem_u32(&ctl->i_empty[j]), 32);           // the lanes of the gather warp
         }
-        for (int s = 0; s < B_STAGES; ++s) {
-            mbar_init(smem_u32(&ctl->b_full[s]), 1);
-            mbar_init(smem_u32(&ctl->b_empty[s]), MMA_WARPS);
+        if (tid >= 96 && tid < 96 + B_STAGES) {
+            mbar_init(smem_u32(&ctl->b_full[tid - 96]), 1);
+            mbar_init(smem_u32(&ctl->b_empty[tid - 96]), MMA_WARPS);
         }
-        for (int s = 0; s < 2; ++s) {
-            mbar_init(smem_u32(&ctl->acc_full[s]), MMA_WARPS);          // every MMA issuer reports its tile
-            mbar_init(smem_u32(&ctl->acc_empty[s]), EPI_WARPS * 32);    // every epilogue thread
+        if (tid >= 128 && tid < 130) {
+            mbar_init(smem_u32(&ctl->acc_full[tid - 128]), MMA_WARPS);          // every MMA issuer reports its tile
+            mbar_init(smem_u32(&ctl->acc_empty[tid - 128]), EPI_WARPS * 32);    // every epilogue thread
         }
-        mbar_init(smem_u32(&ctl->mma_drain), MMA_WARPS);
-        ctl->abort_flag = 0;
-        ctl->abort_where = 0;
+        if (tid == 160) {
+            mbar_init(smem_u32(&ctl->mma_drain), MMA_WARPS);
+            ctl->abort_flag = 0;
+            ctl->abort_where = 0;
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     const int tiles_per_frame = (max_voxels + TILE_M - 1) / TILE_M;
@@ -607,8 +610,36 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         const int v = __ldg(out_num + f);
         return v > max_voxels ? max_voxels : (v < 0 ? 0 : v);
     };
+    // Tiles before every frame, in shared memory that nothing uses yet. (Row counts and masks are read side by side: one
+    // after the other they were most of the 15 to 19 us that a launch over 32 frames cost beside its work.) With few frames
+    // every thread adds and walks by itself: those launches are all latency, and the hand-over takes half a microsecond.
+    int* first_tile = reinterpret_cast<int*>(sA);             // [batch]
+    static_assert(kMaxBatch * 4 <= NSLOT * A_BYTES, "a word per frame");
+    constexpr int FEW_FRAMES = 8;
     int total_tiles = 0;
-    for (int f = 0; f < batch; ++f) total_tiles += (frame_rows(f) + TILE_M - 1) / TILE_M;
+    if (batch <= FEW_FRAMES) {
+        for (int f = 0; f < batch; ++f) total_tiles += (frame_rows(f) + TILE_M - 1) / TILE_M;
+    } else {
+        for (int f = tid; f < batch; f += THREADS) first_tile[f] = (frame_rows(f) + TILE_M - 1) / TILE_M;
+        __syncthreads();
+        if (warp == 0) {
+            int before = 0;
+            for (int f0 = 0; f0 < batch; f0 += 32) {
+                const int v = f0 + lane < batch ? first_tile[f0 + lane] : 0;
+                int incl = v;
+#pragma unroll
+                for (int d = 1; d < 32; d <<= 1) {
+                    const int u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                    if (lane >= d) incl += u;
+                }
+                if (f0 + lane < batch) first_tile[f0 + lane] = before + incl - v;
+                before += __shfl_sync(0xFFFFFFFFu, incl, 31);
+            }
+            if (lane == 0) ctl->range_hi = before;
+        }
+        __syncthreads();
+        total_tiles = ctl->range_hi;
+    }
     const bool few = tile_counter != nullptr && total_tiles <= FEW_TILES * (int)gridDim.x;
     if (few) {
         static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) <= NSLOT * A_BYTES + B_STAGES * B_BYTES &&
@@ -618,59 +649,82 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                             batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, !maps_ready, withhold_weights);
     }
     if (!few) {
+        if (tid == 0) ctl->range_lo = 0, ctl->range_hi = total_tiles;   // (the next barrier comes before anyone's cut point)
         const int per = (total_tiles + THREADS - 1) / THREADS;
         const int first = tid * per, last = first + per < total_tiles ? first + per : total_tiles;
         // a tile costs its items plus its share of the group hand-over and of the epilogue, about eight items' worth
         // (fitted to the CTA lifetimes of 1/4-resolution launches)
         auto tile_weight = [&](uint32_t mask) { return (uint32_t)(__popc(stage_bits<KG>(mask)) + 8); };
-        int f = 0, f_first = 0, f_tiles = batch > 0 ? (frame_rows(0) + TILE_M - 1) / TILE_M : 0;
-        auto seek = [&](int tile) {   // frame of a tile of the sequence (tiles are visited in ascending order)
-            while (f < batch && tile >= f_first + f_tiles) {
-                f_first += f_tiles;
-                ++f;
-                f_tiles = f < batch ? (frame_rows(f) + TILE_M - 1) / TILE_M : 0;
+        // Pass 0: the weight of this thread's slice, and the weights before it. Passes 1 and 2: cut points c and c + 1, each the
+        // first tile whose running total (inclusive) exceeds grand * c / gridDim.x; a thread whose slice holds one walks the
+        // slice again. (One copy of the walk: a kernel's first launch in a while fetches its code from L2, and two
+        // copies cost a single frame 1 %.)
+        uint32_t mine = 0, excl = 0, grand = 0;
+#pragma unroll 1
+        for (int pass = 0; pass < 3; ++pass) {
+            uint32_t run = excl, target = ~0u;
+            if (pass > 0) {
+                const unsigned long long c = blockIdx.x + pass - 1;
+                if (c == 0 || c >= gridDim.x) continue;   // 0 and total_tiles are preset
+                target = (uint32_t)((unsigned long long)grand * c / gridDim.x);
+                if (mine == 0 || target < excl || target >= excl + mine) continue;
             }
-        };
-        uint32_t mine = 0;
-        for (int i = first; i < last; ++i) {
-            seek(i);
-            mine += tile_weight(__ldg(tile_mask + (size_t)f * tiles_per_frame + (i - f_first)));
-        }
-        uint32_t incl = mine;   // inclusive block scan of `mine`
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-            if (lane >= d) incl += v;
-        }
-        if (lane == 31) ctl->scan_warp[warp] = incl;
-        if (tid == 0) ctl->range_lo = 0, ctl->range_hi = total_tiles;
-        __syncthreads();
-        uint32_t before = 0, grand = 0;
-        for (int w = 0; w < THREADS / 32; ++w) {
-            const uint32_t v = ctl->scan_warp[w];
-            if (w < warp) before += v;
-            grand += v;
-        }
-        const uint32_t excl = before + incl - mine;   // weight of all tiles before this thread's slice
-        // cut point c: the first tile whose running total (inclusive) exceeds grand * c / gridDim.x
-        for (int side = 0; side < 2; ++side) {
-            const unsigned long long c = blockIdx.x + side;
-            if (c == 0 || c >= gridDim.x) continue;   // 0 and total_tiles are preset
-            const uint32_t target = (uint32_t)((unsigned long long)grand * c / gridDim.x);
-            if (mine == 0 || target < excl || target >= excl + mine) continue;
-            f = 0, f_first = 0, f_tiles = batch > 0 ? (frame_rows(0) + TILE_M - 1) / TILE_M : 0;
-            uint32_t run = excl;
             int cut = last;
-            for (int i = first; i < last; ++i) {
-                seek(i);
-                run += tile_weight(__ldg(tile_mask + (size_t)f * tiles_per_frame + (i - f_first)));
-                if (run > target) {
-                    cut = i;
-                    break;
+            if (batch <= FEW_FRAMES) {
+                int f = 0, start = 0, tiles = (frame_rows(0) + TILE_M - 1) / TILE_M;
+                for (int i = first; i < last; ++i) {
+                    while (i >= start + tiles) {
+                        start += tiles;
+                        tiles = (frame_rows(++f) + TILE_M - 1) / TILE_M;
+                    }
+                    run += tile_weight(__ldg(tile_mask + (size_t)f * tiles_per_frame + (i - start)));
+                    if (run > target) {
+                        cut = i;
+                        break;
+                    }
+                }
+            } else if (first < last) {
+                int f = 0;                                    // frame of the slice's first tile: the last that starts at or before it
+                for (int n = batch; n > 1;) {
+                    const int half = n / 2;
+                    if (first_tile[f + half] <= first) f += half;
+                    n -= half;
+                }
+                for (int i0 = first; i0 < last && cut == last; i0 += 4) {   // the masks of four tiles requested together
+                    uint32_t w[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        while (i0 + u < last && f + 1 < batch && first_tile[f + 1] <= i0 + u) ++f;
+                        w[u] = i0 + u < last ? tile_weight(__ldg(tile_mask + (size_t)f * tiles_per_frame + (i0 + u - first_tile[f]))) : 0u;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        run += w[u];
+                        if (run > target && cut == last) cut = i0 + u;
+                    }
                 }
             }
-            if (side == 0) ctl->range_lo = cut;
-            else ctl->range_hi = cut;
+            if (pass > 0) {
+                if (pass == 1) ctl->range_lo = cut;
+                else ctl->range_hi = cut;
+                continue;
+            }
+            mine = run;
+            uint32_t incl = mine;   // inclusive block scan of `mine`
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+                if (lane >= d) incl += v;
+            }
+            if (lane == 31) ctl->scan_warp[warp] = incl;
+            __syncthreads();
+            uint32_t before = 0;
+            for (int w = 0; w < THREADS / 32; ++w) {
+                const uint32_t v = ctl->scan_warp[w];
+                if (w < warp) before += v;
+                grand += v;
+            }
+            excl = before + incl - mine;   // weight of all tiles before this thread's slice
         }
     }
     __syncthreads();

@@ -69,7 +69,7 @@ struct VoxelOut {
 };
 
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 5)
 voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch, int max_points,
                   VoxGeom g, VoxelTable t, int max_pts, const int32_t* __restrict__ pt_claim, ScanState scan, VoxelOut<T> out) {
     pdl_enter();
