@@ -95,22 +95,46 @@ __device__ __forceinline__ void store_channels(__half* p, const float (&y)[N]) {
     }
 }
 
+// N weights from shared memory.
+template <int N>
+__device__ __forceinline__ void load_weights(const float* p, float (&w)[N]) {
+#pragma unroll
+    for (int c = 0; c < N; c += 4) {
+        const float4 t = *reinterpret_cast<const float4*>(p + c);
+        w[c] = t.x, w[c + 1] = t.y, w[c + 2] = t.z, w[c + 3] = t.w;
+    }
+}
+template <int N>
+__device__ __forceinline__ void load_weights(const __half* p, float (&w)[N]) {
+    static_assert(N % 8 == 0, "eight halves per read");
+#pragma unroll
+    for (int c = 0; c < N; c += 8) {
+        const uint4 t = *reinterpret_cast<const uint4*>(p + c);
+        const __half2* h = reinterpret_cast<const __half2*>(&t);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const float2 f = __half22float2(h[j]);
+            w[c + 2 * j] = f.x, w[c + 2 * j + 1] = f.y;
+        }
+    }
+}
+
 // Narrow layers. Little arithmetic per row (4 to 5 of 27 neighbours at full resolution) behind three dependent reads
 // (row count, map entry, input row), so the kernel lives on rows in flight: COUT / OC threads share a row, a block takes
 // ROWS rows at a time and reads their map entries side by side (coalesced over rows, all in flight, those of its next
 // rows while it works on the present ones); every thread then walks its row's present neighbours in ascending k. The
-// weights sit in shared memory as floats, 16 bytes of padding per offset so that rows at different offsets meet in fewer
-// banks. Four channels per thread for the 16-channel inputs, eight for the 4-channel input, whose rows are small enough
-// to keep six blocks per SM.
+// weights sit in shared memory as they come (a warp's rows are at different offsets, so that their reads are what the
+// multiply-adds wait for), 16 bytes of padding per offset so that rows at different offsets meet in fewer banks. Four channels per thread for the 16-channel inputs, eight for the 4-channel input, whose rows are small enough
+// to keep four blocks per SM.
 template <typename T, int CIN, int COUT>
 struct Narrow {
     static constexpr int OC = CIN <= 4 ? 8 : 4;          // output channels per thread
     static constexpr int TPR = COUT / OC;                // threads per output row
     static constexpr int ROWS = kThreads / TPR;          // a divisor of the map's 128-row tile
-    static constexpr int BLOCKS = CIN <= 4 ? 5 : 3;      // resident per SM
+    static constexpr int BLOCKS = CIN <= 4 ? 4 : 3;      // resident per SM
     static constexpr int KVOL_MAX = 27;                  // 3 x 3 x 3 is the largest kernel the geometry code accepts
-    static constexpr int W_STRIDE = CIN * COUT + 4;      // floats from one offset's weights to the next offset's
-    static constexpr int smem(int kvol) { return (kvol * W_STRIDE + KVOL_MAX * ROWS) * 4; }
+    static constexpr int W_STRIDE = CIN * COUT + 16 / (int)sizeof(T);   // elements from one offset's weights to the next offset's
+    static constexpr int smem(int kvol) { return kvol * W_STRIDE * (int)sizeof(T) + KVOL_MAX * ROWS * 4; }
 };
 
 template <typename T, int CIN, int COUT>
@@ -124,9 +148,9 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
     constexpr int TPR = N::TPR, ROWS = N::ROWS, OC = N::OC;
     constexpr int LOADS = (N::KVOL_MAX * ROWS + kThreads - 1) / kThreads;   // map entries a thread reads
     constexpr int NP = 2;                                                   // input rows in flight per thread
-    extern __shared__ __align__(16) float narrow_smem[];
-    float* s_w = narrow_smem;
-    int32_t* s_idx = reinterpret_cast<int32_t*>(narrow_smem + kvol * N::W_STRIDE);   // [KVOL_MAX][ROWS]
+    extern __shared__ __align__(16) uint8_t narrow_smem[];
+    T* s_w = reinterpret_cast<T*>(narrow_smem);
+    int32_t* s_idx = reinterpret_cast<int32_t*>(s_w + kvol * N::W_STRIDE);           // [KVOL_MAX][ROWS]
     const int tid = threadIdx.x, r = tid / TPR, cq = tid % TPR;
     const int chunks = (max_voxels + ROWS - 1) / ROWS;
     const int items = batch * chunks, tiles = (max_voxels + 127) / 128;
@@ -155,7 +179,7 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
     // the weights are older than any preceding kernel
     for (int e = tid; e < kvol * CIN * COUT; e += kThreads) {
         const int k = e / (CIN * COUT);
-        s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = to_float(__ldg(weights + e));
+        s_w[k * N::W_STRIDE + (e - k * (CIN * COUT))] = __ldg(weights + e);
     }
     pdl_enter();
     fetch();
@@ -199,17 +223,13 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
                 float s[OC];
 #pragma unroll
                 for (int c = 0; c < OC; ++c) s[c] = 0.f;
-                const float* wk = s_w + ks[u] * N::W_STRIDE + cq * OC;
+                const T* wk = s_w + ks[u] * N::W_STRIDE + cq * OC;
 #pragma unroll
                 for (int ci = 0; ci < CIN; ++ci) {
+                    float w[OC];
+                    load_weights(wk + ci * COUT, w);
 #pragma unroll
-                    for (int c = 0; c < OC; c += 4) {
-                        const float4 w = *reinterpret_cast<const float4*>(wk + ci * COUT + c);
-                        s[c] = fmaf(x[u][ci], w.x, s[c]);
-                        s[c + 1] = fmaf(x[u][ci], w.y, s[c + 1]);
-                        s[c + 2] = fmaf(x[u][ci], w.z, s[c + 2]);
-                        s[c + 3] = fmaf(x[u][ci], w.w, s[c + 3]);
-                    }
+                    for (int c = 0; c < OC; ++c) s[c] = fmaf(x[u][ci], w[c], s[c]);
                 }
 #pragma unroll
                 for (int c = 0; c < OC; ++c) acc[c] = __fadd_rn(acc[c], s[c]);
