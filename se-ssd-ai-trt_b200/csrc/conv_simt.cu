@@ -14,6 +14,7 @@
 // that takes its channel counts at run time, every pair of channel counts without a kernel of its own. The wide fp32
 // layers are in conv_f32.cu, the wide fp16 layers in conv_umma.cu.
 #include <string>
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -106,13 +107,14 @@ __device__ __forceinline__ void load_weights(const float* p, float (&w)[N]) {
 }
 template <int N>
 __device__ __forceinline__ void load_weights(const __half* p, float (&w)[N]) {
-    static_assert(N % 8 == 0, "eight halves per read");
+    using V = typename std::conditional<N % 8 == 0, uint4, uint2>::type;
+    constexpr int E = sizeof(V) / 2;                     // halves per read
 #pragma unroll
-    for (int c = 0; c < N; c += 8) {
-        const uint4 t = *reinterpret_cast<const uint4*>(p + c);
+    for (int c = 0; c < N; c += E) {
+        const V t = *reinterpret_cast<const V*>(p + c);
         const __half2* h = reinterpret_cast<const __half2*>(&t);
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < E / 2; ++j) {
             const float2 f = __half22float2(h[j]);
             w[c + 2 * j] = f.x, w[c + 2 * j + 1] = f.y;
         }
@@ -124,11 +126,12 @@ __device__ __forceinline__ void load_weights(const __half* p, float (&w)[N]) {
 // ROWS rows at a time and reads their map entries side by side (coalesced over rows, all in flight, those of its next
 // rows while it works on the present ones); every thread then walks its row's present neighbours in ascending k. The
 // weights sit in shared memory as they come (a warp's rows are at different offsets, so that their reads are what the
-// multiply-adds wait for), 16 bytes of padding per offset so that rows at different offsets meet in fewer banks. Four channels per thread for the 16-channel inputs, eight for the 4-channel input, whose rows are small enough
-// to keep four blocks per SM.
-template <typename T, int CIN, int COUT>
+// multiply-adds wait for: as halves instead of floats a frame of 20,000 points took 257 instead of 262 us), 16 bytes of
+// padding per offset so that rows at different offsets meet in fewer banks. Four channels per thread for the 16-channel
+// inputs, four or eight for the 4-channel input (dispatch).
+template <typename T, int CIN, int COUT, int OC_>
 struct Narrow {
-    static constexpr int OC = CIN <= 4 ? 8 : 4;          // output channels per thread
+    static constexpr int OC = OC_;                       // output channels per thread
     static constexpr int TPR = COUT / OC;                // threads per output row
     static constexpr int ROWS = kThreads / TPR;          // a divisor of the map's 128-row tile
     static constexpr int BLOCKS = CIN <= 4 ? 4 : 3;      // resident per SM
@@ -137,14 +140,14 @@ struct Narrow {
     static constexpr int smem(int kvol) { return kvol * W_STRIDE * (int)sizeof(T) + KVOL_MAX * ROWS * 4; }
 };
 
-template <typename T, int CIN, int COUT>
-__global__ void __launch_bounds__(kThreads, (Narrow<T, CIN, COUT>::BLOCKS))
+template <typename T, int CIN, int COUT, int OC_>
+__global__ void __launch_bounds__(kThreads, (Narrow<T, CIN, COUT, OC_>::BLOCKS))
 conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t* __restrict__ nbr,
                    const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ order,
                    const int32_t* __restrict__ out_num, const T* __restrict__ weights, const float* __restrict__ scale,
                    const float* __restrict__ shift, int relu, int batch, int max_voxels, int kvol,
                    T* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H, int W) {
-    using N = Narrow<T, CIN, COUT>;
+    using N = Narrow<T, CIN, COUT, OC_>;
     constexpr int TPR = N::TPR, ROWS = N::ROWS, OC = N::OC;
     constexpr int LOADS = (N::KVOL_MAX * ROWS + kThreads - 1) / kThreads;   // map entries a thread reads
     constexpr int NP = 2;                                                   // input rows in flight per thread
@@ -317,9 +320,9 @@ int launch_generic(const ConvLaunch& c, cudaStream_t stream) {
     return SESSD_OK;
 }
 
-template <typename T, int CIN, int COUT>
+template <typename T, int CIN, int COUT, int OC>
 int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
-    using N = Narrow<T, CIN, COUT>;
+    using N = Narrow<T, CIN, COUT, OC>;
     static const std::string name = std::string("conv_narrow<") + (sizeof(T) == 4 ? "f32," : "f16,") +
                                     std::to_string(CIN) + "," + std::to_string(COUT) + ">";
     if (N::smem(N::KVOL_MAX) > 48 * 1024) {
@@ -329,12 +332,12 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
         SESSD_CUDA(cudaGetDevice(&dev));
         const uint64_t bit = 1ull << (dev & 63);
         if (!(configured.load(std::memory_order_acquire) & bit)) {
-            SESSD_CUDA(cudaFuncSetAttribute(conv_narrow_kernel<T, CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            SESSD_CUDA(cudaFuncSetAttribute(conv_narrow_kernel<T, CIN, COUT, OC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                             N::smem(N::KVOL_MAX)));
             configured.fetch_or(bit, std::memory_order_release);
         }
     }
-    SESSD_LAUNCH_NAMED(name.c_str(), (conv_narrow_kernel<T, CIN, COUT>), persistent_grid(N::BLOCKS), kThreads, N::smem(c.kvol),
+    SESSD_LAUNCH_NAMED(name.c_str(), (conv_narrow_kernel<T, CIN, COUT, OC>), persistent_grid(N::BLOCKS), kThreads, N::smem(c.kvol),
                        stream, static_cast<const T*>(c.in), static_cast<T*>(c.out), c.nbr, c.tile_mask,
                        c.order, c.out_num,
                        static_cast<const T*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
@@ -344,10 +347,17 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
 
 template <typename T>
 int dispatch(const ConvLaunch& c, cudaStream_t stream) {
-    if (c.cin == 4 && c.cout == 16) return launch_narrow<T, 4, 16>(c, stream);
+    if (c.cin == 4 && c.cout == 16) {
+        // Room for a million rows is what a few frames have. Those are latency: a thread with four channels is through its
+        // row's neighbours sooner, and twice as many blocks share out the rows with the longest lists (one frame of
+        // 20,000 points 258 -> 253 us, four of 120,000 1057 -> 1053). Larger batches are throughput: eight channels per
+        // thread walk half as many lists (32 frames of 120,000 points: the layer 290 us, 338 with four).
+        if ((int64_t)c.batch * c.max_voxels <= 1000000) return launch_narrow<T, 4, 16, 4>(c, stream);
+        return launch_narrow<T, 4, 16, 8>(c, stream);
+    }
     if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these
-        if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16>(c, stream);
-        if (c.cin == 16 && c.cout == 32) return launch_narrow<float, 16, 32>(c, stream);
+        if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16, 4>(c, stream);
+        if (c.cin == 16 && c.cout == 32) return launch_narrow<float, 16, 32, 4>(c, stream);
     }
     return launch_generic<T>(c, stream);   // any other pair of channel counts
 }
