@@ -79,8 +79,13 @@ __device__ __forceinline__ float to_float(__half v) { return __half2float(v); }
 
 template <int N>
 __device__ __forceinline__ void store_channels(float* p, const float (&y)[N]) {
+    if constexpr (N % 4 == 0) {
 #pragma unroll
-    for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
+        for (int i = 0; i < N; i += 4) *reinterpret_cast<float4*>(p + i) = make_float4(y[i], y[i + 1], y[i + 2], y[i + 3]);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; i += 2) *reinterpret_cast<float2*>(p + i) = make_float2(y[i], y[i + 1]);
+    }
 }
 template <int N>
 __device__ __forceinline__ void store_channels(__half* p, const float (&y)[N]) {
@@ -99,10 +104,18 @@ __device__ __forceinline__ void store_channels(__half* p, const float (&y)[N]) {
 // N weights from shared memory.
 template <int N>
 __device__ __forceinline__ void load_weights(const float* p, float (&w)[N]) {
+    if constexpr (N % 4 == 0) {
 #pragma unroll
-    for (int c = 0; c < N; c += 4) {
-        const float4 t = *reinterpret_cast<const float4*>(p + c);
-        w[c] = t.x, w[c + 1] = t.y, w[c + 2] = t.z, w[c + 3] = t.w;
+        for (int c = 0; c < N; c += 4) {
+            const float4 t = *reinterpret_cast<const float4*>(p + c);
+            w[c] = t.x, w[c + 1] = t.y, w[c + 2] = t.z, w[c + 3] = t.w;
+        }
+    } else {
+#pragma unroll
+        for (int c = 0; c < N; c += 2) {
+            const float2 t = *reinterpret_cast<const float2*>(p + c);
+            w[c] = t.x, w[c + 1] = t.y;
+        }
     }
 }
 template <int N>
@@ -127,8 +140,8 @@ __device__ __forceinline__ void load_weights(const __half* p, float (&w)[N]) {
 // rows while it works on the present ones); every thread then walks its row's present neighbours in ascending k. The
 // weights sit in shared memory as they come (a warp's rows are at different offsets, so that their reads are what the
 // multiply-adds wait for: as halves instead of floats a frame of 20,000 points took 257 instead of 262 us), 16 bytes of
-// padding per offset so that rows at different offsets meet in fewer banks. Four channels per thread for the 16-channel
-// inputs, four or eight for the 4-channel input (dispatch).
+// padding per offset so that rows at different offsets meet in fewer banks. How many channels a thread has is the
+// dispatch's choice.
 template <typename T, int CIN, int COUT, int OC_>
 struct Narrow {
     static constexpr int OC = OC_;                       // output channels per thread
@@ -347,17 +360,16 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
 
 template <typename T>
 int dispatch(const ConvLaunch& c, cudaStream_t stream) {
-    if (c.cin == 4 && c.cout == 16) {
-        // Room for a million rows is what a few frames have. Those are latency: a thread with four channels is through its
-        // row's neighbours sooner, and twice as many blocks share out the rows with the longest lists (one frame of
-        // 20,000 points 258 -> 253 us, four of 120,000 1057 -> 1053). Larger batches are throughput: eight channels per
-        // thread walk half as many lists (32 frames of 120,000 points: the layer 290 us, 338 with four).
-        if ((int64_t)c.batch * c.max_voxels <= 1000000) return launch_narrow<T, 4, 16, 4>(c, stream);
-        return launch_narrow<T, 4, 16, 8>(c, stream);
-    }
+    // Room for a million rows is what a few frames have. Those are latency: a thread with half the channels is through its
+    // row's neighbours sooner, and twice as many blocks share out the rows with the longest lists (4 -> 16: one frame of
+    // 20,000 points 258 -> 253 us, four of 120,000 1057 -> 1054; fp32 16 -> 16 and 16 -> 32: 1008 -> 1000 us). Larger batches
+    // are throughput: with twice the channels half as many threads walk a list (32 frames of 120,000 points: 290 us for
+    // 4 -> 16, 338 with four channels).
+    const bool few = (int64_t)c.batch * c.max_voxels <= 1000000;
+    if (c.cin == 4 && c.cout == 16) return few ? launch_narrow<T, 4, 16, 4>(c, stream) : launch_narrow<T, 4, 16, 8>(c, stream);
     if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these
-        if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16, 4>(c, stream);
-        if (c.cin == 16 && c.cout == 32) return launch_narrow<float, 16, 32, 4>(c, stream);
+        if (c.cin == 16 && c.cout == 16) return few ? launch_narrow<float, 16, 16, 2>(c, stream) : launch_narrow<float, 16, 16, 4>(c, stream);
+        if (c.cin == 16 && c.cout == 32) return few ? launch_narrow<float, 16, 32, 2>(c, stream) : launch_narrow<float, 16, 32, 4>(c, stream);
     }
     return launch_generic<T>(c, stream);   // any other pair of channel counts
 }

@@ -30,15 +30,15 @@ def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, 32, 32) * 0.05).astype(np.float32), dtype=1, maxV=rows + 200)
 
 
-@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("cin,cout,dtype", [(4, 16, 0), (4, 16, 1), (16, 16, 0), (16, 32, 0)])
 @pytest.mark.parametrize("max_voxels", [1000000, 1000001])
-def test_first_layer_with_four_or_eight_channels_per_thread(gpu, oracle, max_voxels, dtype):
-    """Room for a million rows is where the 4 -> 16 kernel changes its split; 129 rows: one more than a tile."""
+def test_narrow_layers_around_a_million_rows(gpu, oracle, max_voxels, cin, cout, dtype):
+    """Room for a million rows is where the narrow kernels change their split; 129 rows: one more than a tile."""
     rs = np.random.RandomState(dtype)
-    layer = _layer(gpu, True, 4, 16, (3, 3, 3), (1, 1, 1), (1, 1, 1), (6, 9, 66))
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (6, 9, 66))
     c = _random_coords(rs, 129, layer.in_shape)
-    f = rs.randn(129, 4).astype(np.float32)
-    _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, 4, 16) * 0.1).astype(np.float32), dtype=dtype, maxV=max_voxels)
+    f = rs.randn(129, cin).astype(np.float32)
+    _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, cin, cout) * 0.1).astype(np.float32), dtype=dtype, maxV=max_voxels)
 
 
 def test_numbering_of_more_chunks_than_one_scan_group(gpu, oracle):
