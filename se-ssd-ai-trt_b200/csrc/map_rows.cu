@@ -57,7 +57,8 @@ struct BitsIndex {
     struct Row {
         int word;
         uint32_t sh, below_lo, below_hi;   // first bit of the window (mod 32), bits of the word before it
-        bool upper, neg, two;              // window starts in the word's upper half; at x = -1; goes on in the next word
+        uint32_t lead;                     // cells of the window before the line (x < 0; up to the padding, 2)
+        bool upper, two;                   // window starts in the word's upper half; goes on in the next word
     };
     static __device__ __forceinline__ BitsIndex make(const MapJob& j, int b) {
         const BitGrid& g = j.in;
@@ -67,7 +68,8 @@ struct BitsIndex {
         const int lo = max(x0, 0), hi = min(x0 + count, X) - 1;
         const uint32_t sh = lo & 31, below = (1u << sh) - 1u;
         const bool upper = lo & 32;
-        return Row{(z * Y + y) * xw + (lo >> 6), sh, upper ? ~0u : below, upper ? below : 0u, upper, x0 < 0, (hi >> 6) > (lo >> 6)};
+        return Row{(z * Y + y) * xw + (lo >> 6), sh, upper ? ~0u : below, upper ? below : 0u, (uint32_t)(lo - x0), upper,
+                   (hi >> 6) > (lo >> 6)};
     }
     __device__ __forceinline__ int step(int kz, int ky) const { return (kz * Y + ky) * xw; }
     template <bool TOP>
@@ -95,7 +97,7 @@ struct BitsIndex {
     // Neighbours of a line as bits, and the row of the first.
     template <int COUNT>
     __device__ __forceinline__ uint32_t finish(const Row& r, const uint4& l, bool on, int* base) const {
-        const uint32_t w = __funnelshift_r(r.upper ? l.y : l.x, r.upper ? l.w : l.y, r.sh) << (r.neg ? 1 : 0);
+        const uint32_t w = __funnelshift_r(r.upper ? l.y : l.x, r.upper ? l.w : l.y, r.sh) << r.lead;
         *base = (int)l.z + __popc(l.x & r.below_lo) + __popc(l.y & r.below_hi);
         return w & (on ? (1u << COUNT) - 1u : 0u);
     }

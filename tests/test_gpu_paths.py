@@ -74,6 +74,31 @@ def test_map_windows_of_other_kernels(gpu, oracle, K0, K1):
     _check_fp32_layers(_oracle_layers(oracle, case, False), views)
 
 
+def _scattered_points(n, seed, edge=()):
+    """n points all over the 64 x 80 x 40 cell range of the small case, so that most cells have no neighbour; edge: x cells
+    that get 40 points each besides."""
+    rs = np.random.RandomState(seed)
+    cells = rs.randint(0, (64, 80, 40), (n + 40 * len(edge), 3))
+    for i, x in enumerate(edge):
+        cells[n + 40 * i:n + 40 * (i + 1), 0] = x
+    xyz = np.array([0.0, 0.0, -3.0]) + (cells + 0.5) * np.array([0.05, 0.05, 0.1])
+    return np.concatenate([xyz, rs.rand(len(xyz), 1)], 1).astype(np.float32)
+
+
+@pytest.mark.parametrize("K", [(3, 3, 3), (1, 3, 3)])
+def test_map_windows_with_two_cells_of_x_padding(gpu, oracle, K):
+    """Output x = 0 then looks at x = -2 .. 0: over the voxeliser's two-level grid and over a one-level grid, by the kernel for
+    3x3x3 and by the one for any size."""
+    layers, shape = [], (41, 80, 64)
+    for cin, cout in ((4, 16), (16, 32)):
+        layers.append(_layer(gpu, False, cin, cout, K, (2, 2, 2), (K[0] // 2, 2, 2), shape))
+        shape = layers[-1].out_shape
+    layers.append(_layer(gpu, True, 32, 32, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape))
+    case = _case(gpu, tuple(layers), _scattered_points(300, 1, edge=(0, 1, 2)), 16000)
+    _, views = _gpu_run(gpu, case, 0)
+    _check_fp32_layers(_oracle_layers(oracle, case, False), views)
+
+
 def test_front_end_with_more_points_than_rows(gpu, oracle):
     """More points than max_voxels: voxels are numbered in point order, through a table, instead of in the grid's order."""
     points = np.tile(mk.small_case(gpu)["points"][:90], (30, 1))
