@@ -191,6 +191,7 @@ __device__ __forceinline__ void mark_levels(unsigned long long bits, int z, int 
         const BitGrid& out = chain.grid[l];
         z0 = div_trunc(max(z0 + g.P[0] - g.K[0] + g.S[0], 0), g.S[0]), z1 = min(div_trunc(z1 + g.P[0], g.S[0]), out.Z - 1);
         y0 = div_trunc(max(y0 + g.P[1] - g.K[1] + g.S[1], 0), g.S[1]), y1 = min(div_trunc(y1 + g.P[1], g.S[1]), out.Y - 1);
+        if (z0 > z1 || y0 > y1) return;   // no output of this level, so none of the levels below (which an empty range would not say)
         if (g.K[2] == 3) {
             const unsigned long long even = even_bits(bits), odd = even_bits(bits >> 1);
             bits = even | odd | (odd << 1);

@@ -99,6 +99,20 @@ def test_map_windows_with_two_cells_of_x_padding(gpu, oracle, K):
     _check_fp32_layers(_oracle_layers(oracle, case, False), views)
 
 
+@pytest.mark.parametrize("K,S,P", [((3, 3, 3), (2, 2, 2), (0, 0, 1)),
+                                   ((1, 1, 3), (2, 2, 2), (0, 0, 1)), ((1, 2, 1), (3, 3, 1), (0, 0, 0))])
+def test_levels_below_lines_that_reach_no_output(gpu, oracle, K, S, P):
+    """Lines in z and y that a layer without padding or with gaps between its windows leaves out (the last of an even
+    number, every second or third one): the padded layers after it must not see them."""
+    layers, shape = [], (41, 80, 64)
+    for cin, cout, k, s, p in ((4, 16, K, S, P), (16, 32, (3, 3, 3), (2, 2, 2), (1, 1, 1)), (32, 64, (3, 3, 3), (2, 2, 2), (1, 1, 1))):
+        layers.append(_layer(gpu, False, cin, cout, k, s, p, shape))
+        shape = layers[-1].out_shape
+    case = _case(gpu, tuple(layers), _scattered_points(200, 2), 16000)
+    _, views = _gpu_run(gpu, case, 0)
+    _check_fp32_layers(_oracle_layers(oracle, case, False), views)
+
+
 def test_front_end_with_more_points_than_rows(gpu, oracle):
     """More points than max_voxels: voxels are numbered in point order, through a table, instead of in the grid's order."""
     points = np.tile(mk.small_case(gpu)["points"][:90], (30, 1))
