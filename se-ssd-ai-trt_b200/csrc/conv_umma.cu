@@ -370,6 +370,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                        *b_full = ctl->i_full + FEW_B_FULL;
     volatile uint32_t* hand = ctl->scan_warp;   // the tile in hand: frame (-1: none left), first row, the frame's rows, mask
     uint32_t items = 0;                        // items of the tiles so far
+    uint32_t sums = 0;                         // tiles so far that had any: acc_full completes a phase for those alone
     uint32_t b_issued = 0;
     bool waited = wait_first;                  // the preceding kernel's writes may be read
     for (uint32_t round = 0;; ++round) {
@@ -459,7 +460,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             }
             bool got = true;
             if (n_items) {
-                got = mbar_wait<true>(smem_u32(acc_full), round & 1u, abort_flag, 3 | (int)(round << 4));
+                got = mbar_wait<true>(smem_u32(acc_full), sums & 1u, abort_flag, 3 | (int)(round << 4));
                 got = __all_sync(0xFFFFFFFFu, got);
                 if (got) tc_fence_after();
             }
@@ -510,6 +511,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             __syncwarp();
         }
         items += (uint32_t)n_items;
+        sums += n_items ? 1u : 0u;
         __syncthreads();                       // indices, accumulator and tile may be replaced
         tc_fence_after();
     }

@@ -30,6 +30,60 @@ def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, 32, 32) * 0.05).astype(np.float32), dtype=1, maxV=rows + 200)
 
 
+def test_few_fp16_tiles_some_without_neighbours(gpu):
+    """Every second tile has rows outside the grid alone, hence no neighbour. A layer on another stream keeps 48 SMs, so that
+    the blocks on the others take several tiles each. Rows inside the grid have the bits of a call on them alone."""
+    import torch
+
+    rs = np.random.RandomState(9)
+    layer = _layer(gpu, True, 32, 32, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
+    tiles = 73
+    inside = _random_coords(rs, tiles * 128, layer.in_shape)
+    both = np.full((tiles, 2, 128, 4), -9, np.int32)
+    both[..., 0] = 0
+    both[:, 1] = inside.reshape(tiles, 128, 4)
+    feat = torch.from_numpy(rs.randn(tiles * 128, 32).astype(np.float16)).cuda()
+    spread = torch.zeros((tiles, 2, 128, 32), dtype=torch.float16, device="cuda")
+    spread[:, 1] = feat.view(tiles, 128, 32)
+    scale, shift = (1 + 0.1 * rs.randn(32)).astype(np.float32), rs.randn(32).astype(np.float32)
+
+    def call(coors, f):
+        rows = len(coors)
+        p = gpu.conv_params(layer, rows)
+        w = gpu.ConvWeights(p, (np.random.RandomState(4).randn(27, 32, 32) * 0.05).astype(np.float32), scale, shift, True, 1)
+        args = (f.reshape(1, rows, 32), torch.from_numpy(coors)[None].cuda(), torch.tensor([rows], dtype=torch.int32).cuda(), p, w)
+        r = gpu.subm_conv(*args, keep_workspace=True)
+        return args, r["features"], r["workspace"], r["status"]
+
+    _, want, _, status = call(inside, feat)
+    assert status == 0
+    args, out, ws, status = call(both.reshape(-1, 4), spread)
+    assert status == gpu.STATUS_BAD_COORD
+    # 48 strips of 8 rows: a block each, the other blocks end at once
+    busy = _layer(gpu, True, 64, 64, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
+    bp = gpu.conv_params(busy, 384)
+    bw = gpu.ConvWeights(bp, (rs.randn(27, 64, 64) * 0.05).astype(np.float32), None, None, True, 0)
+    near = np.zeros((384, 4), np.int32)
+    near[:, 1:] = np.stack(np.unravel_index(np.arange(384), (6, 8, 8)), 1)
+    bargs = (torch.randn((1, 384, 64), device="cuda"), torch.from_numpy(near)[None].cuda(),
+             torch.tensor([384], dtype=torch.int32).cuda(), bp, bw)
+    bws = gpu.subm_conv(*bargs, keep_workspace=True)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(10):
+        with torch.cuda.stream(side):
+            for _ in range(6):
+                gpu.subm_conv_into(*bargs, bws["features"], bws["workspace"])
+        for _ in range(6):
+            out.zero_()
+            gpu.subm_conv_into(*args, out, ws)
+            got = out.view(tiles, 2, 128, 32)
+            assert torch.equal(got[:, 1].reshape(-1, 32), want[0])
+            assert (got[:, 0] == torch.from_numpy(shift).cuda().clamp_min(0).half()).all()
+    torch.cuda.synchronize()
+    args[-1].close(), bw.close()
+
+
 @pytest.mark.parametrize("cin,cout,dtype", [(4, 16, 0), (4, 16, 1), (16, 16, 0), (16, 32, 0)])
 @pytest.mark.parametrize("max_voxels", [1000000, 1000001])
 def test_narrow_layers_around_a_million_rows(gpu, oracle, max_voxels, cin, cout, dtype):
