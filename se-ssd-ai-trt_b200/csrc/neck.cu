@@ -59,7 +59,7 @@ channels_last_kernel(const __half* __restrict__ in, __half* __restrict__ out, in
     }
 }
 
-// y = relu(y + bias) (+ add), in place; rounded where the separate operations round. A thread's vectors of eight channels
+// y = relu(y + bias) (+ add), in place; rounded where the separate operations round, and a NaN stays one as with them. A thread's vectors of eight channels
 // are whole blocks apart, and 8 * kThreads is a multiple of `channels`, so its bias stays in registers.
 __global__ void __launch_bounds__(kThreads)
 bias_relu_kernel(__half* __restrict__ y, const __half* __restrict__ bias, const __half* __restrict__ add, int64_t vectors,
@@ -86,7 +86,7 @@ bias_relu_kernel(__half* __restrict__ y, const __half* __restrict__ bias, const 
             __half2* h = reinterpret_cast<__half2*>(&o);
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                h[j] = __hmax2(__floats2half2_rn(x[2 * j] + bv[2 * j], x[2 * j + 1] + bv[2 * j + 1]), __half2(0.f, 0.f));
+                h[j] = __hmax2_nan(__floats2half2_rn(x[2 * j] + bv[2 * j], x[2 * j + 1] + bv[2 * j + 1]), __half2(0.f, 0.f));
                 if (add) {
                     const float2 f = __half22float2(h[j]);
                     h[j] = __floats2half2_rn(f.x + r[2 * j], f.y + r[2 * j + 1]);

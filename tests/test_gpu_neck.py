@@ -34,6 +34,22 @@ def test_bias_relu(gpu, pixels, channels, add):
     assert gpu.lib().sessd_bias_relu_enqueue(y.data_ptr(), bias.data_ptr(), None, pixels, 24, gpu._stream()) != 0
 
 
+def test_bias_relu_keeps_what_is_not_a_number(gpu):
+    import torch
+
+    inf, nan = float("inf"), float("nan")
+    row = torch.tensor([nan, inf, -inf, 1.0, -1.0, 65504.0, -65504.0, 0.0], device="cuda").half()
+    bias = torch.tensor([[0.0] * 8, [inf] * 8, [-inf] * 8, [nan] * 8, [65504.0] * 8], device="cuda").half()
+    for b in bias:
+        for add in (None, row.flip(0).expand(8, 8).contiguous()):
+            y = row.expand(8, 8).contiguous()
+            want = torch.relu(y + b)
+            want = want if add is None else want + add
+            assert gpu.lib().sessd_bias_relu_enqueue(y.data_ptr(), b.clone().data_ptr(), None if add is None else add.data_ptr(), 8, 8,
+                                                     gpu._stream()) == 0
+            assert torch.equal(y.isnan(), want.isnan()) and torch.equal(y.nan_to_num(7.0), want.nan_to_num(7.0))
+
+
 @pytest.mark.parametrize("pixels", [1, 63, 64, 65, 2 * 200 * 176 + 7])
 def test_neck_tail(gpu, pixels):
     import torch
