@@ -144,7 +144,7 @@ class Neck2D:
         box [B, 70400, 7], cls [B, 70400, 1], iou [B, 70400, 1], dir [B, 70400, 2] (anchor = (y*W + x)*2 + a)."""
         o0, o1 = self._branches(bev_padded)
         B, _, H, W = o0.shape
-        out = {name: self.torch.empty((B, H * W * 2, c // 2), device=o0.device) for name, _p, c in HEAD_LAYERS}
+        out = {name: self.torch.empty((B, H * W * 2, c // 2), dtype=self.torch.float32, device=o0.device) for name, _p, c in HEAD_LAYERS}
         self._tail(o0, o1, heads=out.values())
         return out
 

@@ -78,3 +78,29 @@ def test_neck_tail(gpu, pixels):
     only_feat = torch.empty_like(feat)
     assert run(only_feat, [None] * 4) == 0 and torch.equal(only_feat, feat)
     assert run(None, [None] * 4) != 0
+
+
+@pytest.fixture(scope="module")
+def neck(gpu):
+    return gpu.detector.Neck2D(gpu.detector.random_neck_weights())
+
+
+def _bev(batch, height, width, seed=3):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn((batch, 128, height, width), generator=g, device="cuda").relu().half()
+
+
+def test_heads_are_fp32_whatever_the_default_type(gpu, neck):
+    import torch
+
+    x = _bev(2, 18, 26)
+    want = neck(x)
+    try:
+        torch.set_default_dtype(torch.float64)
+        got = neck(x)
+    finally:
+        torch.set_default_dtype(torch.float32)
+    for k, v in want.items():
+        assert v.dtype == got[k].dtype == torch.float32 and torch.equal(v, got[k])
