@@ -64,9 +64,9 @@ channels_last_kernel(const __half* __restrict__ in, __half* __restrict__ out, in
 __global__ void __launch_bounds__(kThreads)
 bias_relu_kernel(__half* __restrict__ y, const __half* __restrict__ bias, const __half* __restrict__ add, int64_t vectors,
                  int channels) {
+    pdl_enter();                               // (the bias, too, may be the preceding kernel's work)
     float bv[8];
     unpack8(__ldg(reinterpret_cast<const uint4*>(bias) + threadIdx.x % (channels / 8)), bv);
-    pdl_enter();
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < vectors; e += 2 * stride) {
         uint4 v[2], a[2];
@@ -118,6 +118,7 @@ neck_tail_kernel(const __half* __restrict__ o0, const __half* __restrict__ o1, c
     __shared__ float s_out[kTilePixels * kHeadChannels];
     const int tid = threadIdx.x, l16 = tid & 15, lane = tid & 31, warp = tid >> 5;
     const bool want_heads = heads.out[0] != nullptr;
+    pdl_enter();                               // (the weights are arguments: they, too, may be the preceding kernel's work)
     float g0[8], g1[8];
     unpack8(__ldg(reinterpret_cast<const uint4*>(gate_w) + l16), g0);
     unpack8(__ldg(reinterpret_cast<const uint4*>(gate_w + C) + l16), g1);
@@ -128,7 +129,6 @@ neck_tail_kernel(const __half* __restrict__ o0, const __half* __restrict__ o1, c
             *reinterpret_cast<uint4*>(s_w + o * STRIDE + c) =
                 o < kHeadChannels ? __ldg(reinterpret_cast<const uint4*>(head_w + o * C + c)) : make_uint4(0u, 0u, 0u, 0u);
         }
-    pdl_enter();
     const int64_t tiles = (pixels + kTilePixels - 1) / kTilePixels;
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const int64_t p0 = t * kTilePixels;

@@ -104,3 +104,34 @@ def test_heads_are_fp32_whatever_the_default_type(gpu, neck):
         torch.set_default_dtype(torch.float32)
     for k, v in want.items():
         assert v.dtype == got[k].dtype == torch.float32 and torch.equal(v, got[k])
+
+
+def test_weights_written_just_before_the_call(gpu):
+    """Bias and weights that the kernel launched just before writes (its blocks let the next kernel start early)."""
+    import torch
+
+    lib, s = gpu.lib(), gpu._stream()
+    zero = torch.zeros(128, dtype=torch.float16, device="cuda")
+    big = torch.zeros((300000, 128), dtype=torch.float16, device="cuda")
+    g = torch.Generator(device="cuda").manual_seed(1)
+    o0, o1 = (torch.randn((64, 128), generator=g, device="cuda").half() for _ in range(2))
+    for i in range(1, 20):
+        params = torch.full((26, 128), i / 64.0, dtype=torch.float16, device="cuda")     # 2 gate rows, gate and head bias, 22 head rows
+        big.zero_()
+        big[-26:].fill_(-1.0)
+        y = torch.zeros((64, 128), dtype=torch.float16, device="cuda")
+        heads = [torch.empty((64, c), device="cuda") for c in (14, 2, 2, 4)]
+        want = [torch.empty_like(h) for h in heads]
+        run = lambda w, out: lib.sessd_neck_tail_enqueue(gpu._vp(o0, o1, w[:2], w[2], w[4:], w[3]), gpu._vp(None, *out), 64, s)
+        assert run(params, want) == 0
+        tail = big[-26:]
+        add = torch.zeros_like(big)
+        add[-26:] = params
+        torch.cuda.synchronize()
+        assert lib.sessd_bias_relu_enqueue(big.data_ptr(), zero.data_ptr(), add.data_ptr(), len(big), 128, s) == 0
+        assert lib.sessd_bias_relu_enqueue(y.data_ptr(), tail[5].data_ptr(), None, 64, 128, s) == 0
+        assert (y == i / 64.0).all()
+        tail.fill_(-1.0)
+        assert lib.sessd_bias_relu_enqueue(big.data_ptr(), zero.data_ptr(), add.data_ptr(), len(big), 128, s) == 0
+        assert run(tail, heads) == 0
+        assert all(torch.equal(a, b) for a, b in zip(heads, want))
