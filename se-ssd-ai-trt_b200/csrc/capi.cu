@@ -444,7 +444,7 @@ int sessd_voxelize_enqueue(const sessd_voxel_params* p, int batch, int max_point
     tails.tensor[1] = outputs[1], tails.row_bytes[1] = 16;
     tails.tensor[2] = w.num_points, tails.row_bytes[2] = 4;
     tails.counts = static_cast<const int32_t*>(inputs[1]);
-    tails.batch = batch, tails.max_rows = p->max_voxels;
+    tails.batch = batch, tails.max_rows = p->max_voxels, tails.most = max_points;   // (a count above max_points means max_points)
     int rc = launch_prepare(fills, tails, /*overlap=*/true, stream);
     if (rc) return rc;
     return voxelize_run(p, batch, max_points, out_dtype, static_cast<const float*>(inputs[0]),
@@ -558,7 +558,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     tails.tensor[0] = outputs[0], tails.row_bytes[0] = (int)(p->out_channel * esize(w->impl.dtype));
     if (!subm) tails.tensor[1] = outputs[1], tails.row_bytes[1] = 16;
     tails.counts = subm ? in_num : static_cast<const int32_t*>(outputs[2]);
-    tails.batch = batch, tails.max_rows = maxV;
+    tails.batch = batch, tails.max_rows = tails.most = maxV;
     FillRanges fills{};
     fills.ptr[0] = static_cast<uint4*>(ws.ones_base), fills.n16[0] = ws.ones_bytes / 16, fills.ones[0] = 1;
     fills.ptr[1] = static_cast<uint4*>(ws.zero_base), fills.n16[1] = ws.zero_bytes / 16, fills.ones[1] = 0;

@@ -279,13 +279,14 @@ struct FillRanges {
     int32_t* status;
     int status_from;
 };
-// Output tensors [batch][max_rows][row_bytes] whose rows from counts[b] on are to be zero (row_bytes % 2 == 0; null: unused).
+// Output tensors [batch][max_rows][row_bytes] whose rows from min(counts[b], most) on are to be zero (row_bytes % 2 == 0;
+// null: unused).
 struct TailRows {
     static constexpr int kMax = 3;
     void* tensor[kMax];
     int row_bytes[kMax];
     const int32_t* counts;
-    int batch, max_rows;
+    int batch, max_rows, most;
 };
 // overlap: whether the launch may start while the stream's previous kernel runs (see its definition)
 int launch_prepare(const FillRanges& f, const TailRows& t, bool overlap, cudaStream_t stream);

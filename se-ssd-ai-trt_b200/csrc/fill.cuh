@@ -20,18 +20,16 @@ __device__ __forceinline__ void fill_ranges(const FillRanges& f) {
 }
 
 template <typename V>
-__device__ __forceinline__ void zero_rows(void* tensor, int units, const int32_t* __restrict__ counts, int batch,
-                                          int max_rows) {
+__device__ __forceinline__ void zero_rows(void* tensor, int units, const TailRows& t) {
     constexpr int PER = 4;                              // stores per thread and item
-    const int64_t per_frame = (int64_t)max_rows * units;
+    const int64_t per_frame = (int64_t)t.max_rows * units;
     const int threads = (int)blockDim.x;
     const int chunks = (int)((per_frame + threads * PER - 1) / (threads * PER));
     V zero;
     memset(&zero, 0, sizeof(V));
-    for (int64_t it = blockIdx.x; it < (int64_t)batch * chunks; it += gridDim.x) {
+    for (int64_t it = blockIdx.x; it < (int64_t)t.batch * chunks; it += gridDim.x) {
         const int b = (int)(it / chunks), c = (int)(it - (int64_t)b * chunks);
-        int n = __ldg(counts + b);
-        n = n < 0 ? 0 : (n > max_rows ? max_rows : n);
+        const int most = min(t.most, t.max_rows), n = max(0, min(__ldg(t.counts + b), most));
         const int64_t low = (int64_t)n * units, at = (int64_t)c * threads * PER;
         if (at + threads * PER <= low) continue;       // uniform over the block
         V* base = static_cast<V*>(tensor) + (int64_t)b * per_frame;
@@ -43,16 +41,16 @@ __device__ __forceinline__ void zero_rows(void* tensor, int units, const int32_t
     }
 }
 
-// Rows counts[b] .. max_rows - 1 of up to three [batch][max_rows][row_bytes] tensors to zero (row_bytes % 2 == 0).
+// The rows of `t`.
 __device__ __forceinline__ void zero_tails(const TailRows& t) {
 #pragma unroll
     for (int i = 0; i < TailRows::kMax; ++i) {
         if (!t.tensor[i]) continue;
         const int rb = t.row_bytes[i];
-        if (rb % 16 == 0) zero_rows<uint4>(t.tensor[i], rb / 16, t.counts, t.batch, t.max_rows);
-        else if (rb % 8 == 0) zero_rows<uint2>(t.tensor[i], rb / 8, t.counts, t.batch, t.max_rows);
-        else if (rb % 4 == 0) zero_rows<uint32_t>(t.tensor[i], rb / 4, t.counts, t.batch, t.max_rows);
-        else zero_rows<uint16_t>(t.tensor[i], rb / 2, t.counts, t.batch, t.max_rows);
+        if (rb % 16 == 0) zero_rows<uint4>(t.tensor[i], rb / 16, t);
+        else if (rb % 8 == 0) zero_rows<uint2>(t.tensor[i], rb / 8, t);
+        else if (rb % 4 == 0) zero_rows<uint32_t>(t.tensor[i], rb / 4, t);
+        else zero_rows<uint16_t>(t.tensor[i], rb / 2, t);
     }
 }
 

@@ -99,3 +99,25 @@ def test_repeat_runs_are_bitwise_identical(gpu):
     b, _ = _run(gpu, f, 65536)
     for k in ("voxels", "coors", "voxel_num", "num_points"):
         np.testing.assert_array_equal(a[k], b[k])
+
+
+def test_point_count_beyond_the_buffer_counts_as_full(gpu, oracle):
+    """Rows past the buffer's points are zero, also where a frame's count claims more points than the buffer holds."""
+    import ctypes
+
+    import torch
+
+    frame = gpu.synth.lidar_frame(7, n_points=300, n_boxes=3)
+    pts = torch.from_numpy(np.stack([frame, frame])).cuda()
+    sizes = torch.tensor([700, 300], dtype=torch.int32, device="cuda")
+    params = gpu.voxel_params(1000, gpu.synth.POINT_RANGE, gpu.synth.VOXEL_SIZE, 5)
+    vox, coors = torch.full((2, 1000, 4), 9.0, device="cuda"), torch.full((2, 1000, 4), 9, dtype=torch.int32, device="cuda")
+    num = torch.empty(2, dtype=torch.int32, device="cuda")
+    ws = torch.full((gpu.lib().sessd_voxelize_workspace_bytes(ctypes.byref(params), 2, 300),), 9, dtype=torch.uint8, device="cuda")
+    gpu.voxelize_into(pts, sizes, params, vox, coors, num, ws, 0)
+    want, want_coors, _, n, _ = oracle.voxelize(frame, gpu.synth.POINT_RANGE, gpu.synth.VOXEL_SIZE, 1000)
+    assert num.tolist() == [n, n] and gpu.read_status(ws) == 0
+    for b in range(2):
+        want_coors[:n, 0] = b
+        np.testing.assert_array_equal(vox[b].cpu().numpy(), want)
+        np.testing.assert_array_equal(coors[b].cpu().numpy(), want_coors)
