@@ -144,7 +144,10 @@ size_t esize(int dtype) { return dtype == SESSD_F32 ? 4 : 2; }
 int choose_conv(const ConvLaunch& c_in, cudaStream_t stream) {
     const ConvLaunch& c = c_in;
     if (c.dtype == SESSD_F16 && conv_umma_supported(c.cin, c.cout) && c.umma_weights) return launch_conv_umma(c, stream);
-    if (c.dtype == SESSD_F32 && conv_f32_supported(c.cin, c.cout, c.kvol)) return launch_conv_f32(c, stream);
+    // conv_f32.cu copies rows 16 bytes at a time; 64 -> 32 channels had no vector accesses before it had a kernel there, so that
+    // buffers at any multiple of four bytes are still taken
+    const bool aligned = (reinterpret_cast<uintptr_t>(c.in) | reinterpret_cast<uintptr_t>(c.out)) % 16 == 0;
+    if (c.dtype == SESSD_F32 && aligned && conv_f32_supported(c.cin, c.cout, c.kvol)) return launch_conv_f32(c, stream);
     return launch_conv_simt(c, stream);
 }
 

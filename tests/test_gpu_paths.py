@@ -21,6 +21,29 @@ def test_fp32_register_tiles(gpu, oracle, cin, cout, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, cin, cout) * 0.05).astype(np.float32), maxV=rows + 5)
 
 
+@pytest.mark.parametrize("skip_in,skip_out", [(1, 0), (0, 2), (3, 1)])
+def test_fp32_rows_off_the_vector_alignment(gpu, skip_in, skip_out):
+    """64 -> 32 channels from and to buffers that start a few floats off a 16-byte boundary: the bits of aligned ones. (All rows
+    are in use: the zeros behind them are stored 16 bytes at a time.)"""
+    import torch
+
+    rs = np.random.RandomState(5)
+    layer = _layer(gpu, True, 64, 32, (3, 3, 3), (1, 1, 1), (1, 1, 1), (6, 20, 30))
+    rows = 700
+    coors = torch.from_numpy(_random_coords(rs, rows, layer.in_shape))[None].cuda()
+    num = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, rows)
+    w = gpu.ConvWeights(p, (rs.randn(27, 64, 32) * 0.05).astype(np.float32), None, None, True, 0)
+    feat = torch.randn((1, rows, 64), device="cuda")
+    r = gpu.subm_conv(feat, coors, num, p, w, keep_workspace=True)
+    shifted = lambda n, off: torch.empty(n + off, device="cuda")[off:]
+    x, out = shifted(rows * 64, skip_in).view(1, rows, 64), shifted(rows * 32, skip_out).view(1, rows, 32)
+    x.copy_(feat)
+    gpu.subm_conv_into(x, coors, num, p, w, out, r["workspace"])
+    assert torch.equal(out, r["features"])
+    w.close()
+
+
 @pytest.mark.parametrize("rows", [148 * 128, 148 * 128 + 1])
 def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     rs = np.random.RandomState(rows)
