@@ -381,8 +381,9 @@ int sessd_profile_end(void* stream, char* names, size_t names_cap, float* ms, in
 /* Number of kernel launches issued by this library since process start (for launch accounting). */
 uint64_t sessd_launch_count(void);
 
-/* Synchronises `stream`, copies the status word of `workspace` to the host and returns it (>= 0),
- * or a negative sessd_error. */
+/* Waits for the work on `stream`, brings the status word of `workspace` to the host and returns it (>= 0), or a negative
+ * sessd_error. Launches a one-thread kernel where stream and workspace belong to the thread's current device, and
+ * synchronises and copies where not. Not for a stream that is being captured. */
 int sessd_read_status(const void* workspace, void* stream);
 /* The status words of two workspaces OR-ed together, for the price of one wait. */
 int sessd_read_status2(const void* workspace, const void* other, void* stream);

@@ -328,9 +328,28 @@ int sessd_conv_weights_debug_withhold(sessd_conv_weights* w, int on) {
 const char* sessd_last_cuda_error(void) { return t_last_error.c_str(); }
 uint64_t sessd_launch_count(void) { return g_launches.load(); }
 
+// Whether a kernel on `stream` can be launched from the thread's current device and reads both workspaces there. Asked where
+// there is more than one device.
+static cudaError_t on_current_device(const void* workspace, const void* other, cudaStream_t stream, bool* yes) {
+    int count = 0, current = 0, device = 0;
+    *yes = true;
+    cudaError_t e = cudaGetDeviceCount(&count);
+    if (e != cudaSuccess || count < 2) return e;
+    if ((e = cudaGetDevice(&current)) != cudaSuccess) return e;
+    if ((e = cudaStreamGetDevice(stream, &device)) != cudaSuccess) return e;
+    *yes = device == current;
+    for (const void* p : {workspace, other}) {
+        cudaPointerAttributes a;
+        if ((e = cudaPointerGetAttributes(&a, p)) != cudaSuccess) return e;
+        *yes = *yes && a.type == cudaMemoryTypeDevice && a.device == current;
+    }
+    return cudaSuccess;
+}
+
 // The word comes back through mapped host memory: a one-thread kernel behind the stream's work stores it together with the
-// call's number, and the host polls for that number. A stream synchronisation and a copy of four bytes took some 15 us
-// more. One 8-byte slot per host thread, returned when the thread ends.
+// call's number, and the host polls for that number. A stream synchronisation and a copy of four bytes take some 15 us
+// more; that is the way for a stream or a workspace of another device than the thread's current one. One 8-byte slot per
+// host thread, returned when the thread ends.
 int sessd_read_status(const void* workspace, void* stream) { return sessd_read_status2(workspace, workspace, stream); }
 
 int sessd_read_status2(const void* workspace, const void* other, void* stream_) {
@@ -341,6 +360,15 @@ int sessd_read_status2(const void* workspace, const void* other, void* stream_) 
     if (capture != cudaStreamCaptureStatusNone) {
         set_cuda_error(cudaErrorStreamCaptureUnsupported, "sessd_read_status");
         return SESSD_ERR_CUDA;
+    }
+    bool here;
+    SESSD_CUDA(on_current_device(workspace, other, stream, &here));
+    if (!here) {
+        int32_t v[2];
+        SESSD_CUDA(cudaStreamSynchronize(stream));
+        SESSD_CUDA(cudaMemcpy(&v[0], workspace, sizeof(v[0]), cudaMemcpyDeviceToHost));
+        SESSD_CUDA(cudaMemcpy(&v[1], other, sizeof(v[1]), cudaMemcpyDeviceToHost));
+        return (v[0] | v[1]) & 0x7FFFFFFF;
     }
     static thread_local StatusSlot slot;
     if (!slot.word)

@@ -250,3 +250,19 @@ def test_status_is_not_read_during_capture(gpu):
             gpu.read_status(ws)
     g.replay()
     assert gpu.read_status(ws) == 0 and float(x[0]) == 1.0
+
+
+def test_status_of_another_device(gpu):
+    """The workspace of one device, read by a thread whose current device is another one."""
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    ws = torch.zeros(1024, dtype=torch.uint8, device="cuda:1")
+    ws[0] = 4
+    torch.cuda.synchronize(1)
+    with torch.cuda.device(0):
+        assert gpu.read_status(ws) == 4
+        assert gpu.lib().sessd_read_status(ws.data_ptr(), torch.cuda.current_stream(1).cuda_stream) == 4
+        stream = torch.cuda.Stream(1)
+        assert gpu.lib().sessd_read_status(ws.data_ptr(), stream.cuda_stream) == 4
