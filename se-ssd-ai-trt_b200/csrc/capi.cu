@@ -371,8 +371,10 @@ int sessd_read_status2(const void* workspace, const void* other, void* stream_) 
         return (v[0] | v[1]) & 0x7FFFFFFF;
     }
     static thread_local StatusSlot slot;
-    if (!slot.word)
+    if (!slot.word) {
         SESSD_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&slot.word), sizeof(*slot.word), cudaHostAllocMapped | cudaHostAllocPortable));
+        *slot.word = 0;   // no call's number
+    }
     const uint32_t call = ++slot.calls;
     SESSD_CUDA(launch_publish_status(static_cast<const int32_t*>(workspace), static_cast<const int32_t*>(other), slot.word, call, stream));
     volatile unsigned long long* word = slot.word;
