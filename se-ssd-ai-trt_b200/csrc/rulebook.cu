@@ -278,9 +278,10 @@ __device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long
 __global__ void __launch_bounds__(kThreads)
 number_outputs_kernel(BitGrid g, int batch, int max_voxels, ScanState scan, int4* __restrict__ out_coors,
                       int32_t* __restrict__ out_num, int32_t* status) {
-    pdl_enter();
     const int chunks = scan_chunks(g.words), items = batch * chunks;
-    for (int t = scan_first(scan.ticket, items, gridDim.x); t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
+    int t = scan_first(scan.ticket, items);
+    pdl_enter();
+    for (; t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = t / batch, b = t - c * batch;
         number_chunk<1>(g, scan.state + (size_t)b * chunks, b, c, chunks, max_voxels, out_coors, out_num, status);
     }
@@ -338,8 +339,8 @@ template <int WORDS>
 __global__ void __launch_bounds__(kThreads, kLevelBlocks)   // (renumber_levels would take 104 registers; it may spill)
 number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int max_voxels, int number_blocks, PointLists lists,
                      int32_t* status) {
-    pdl_enter();
     if ((int)blockIdx.x >= number_blocks) {
+        pdl_enter();
         push_points(lists, batch, blockIdx.x - number_blocks, gridDim.x - number_blocks);
         return;
     }
@@ -347,7 +348,9 @@ number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int ma
     int per_frame = 0;
     for (int l = 0; l < chain.count; ++l) per_frame += scan_chunks((chain.grid[l].words + WORDS - 1) / WORDS);
     const int items = batch * per_frame;
-    for (int t = scan_first(chain.ticket, items, number_blocks); t >= 0; t = scan_next(chain.ticket, items, number_blocks)) {
+    int t = scan_first(chain.ticket, items);
+    pdl_enter();
+    for (; t >= 0; t = scan_next(chain.ticket, items, number_blocks)) {
         const int b = t % batch;
         int c = t / batch, l = 0, chunks = 0;
         for (;; ++l) {

@@ -4,9 +4,9 @@
 // A block publishes its chunk's total and adds up the totals of all chunks before it: every thread polls up to four of
 // them, so that the sum is one round trip once the slowest has published (a chain of running totals, 32 chunks a step,
 // took 10 us for the levels of a single frame). Chunks come in groups of 1024; the last chunk of a group publishes the
-// running total instead, which the next groups start from. A chunk's predecessors belong to blocks that are already
-// running: blocks take chunks by their index when there is a block for each, else from a ticket counter. The wait for a
-// predecessor is bounded by a clock limit, after which the call reports SESSD_STATUS_TIMEOUT.
+// running total instead, which the next groups start from. Blocks take their chunks from a ticket counter, so that a chunk's
+// predecessors belong to blocks that are already running, whatever order the blocks start in and however many are
+// resident. The wait for a predecessor is bounded by a clock limit, after which the call reports SESSD_STATUS_TIMEOUT.
 #pragma once
 
 #include "common.cuh"
@@ -73,8 +73,9 @@ __device__ __forceinline__ int scan_position(unsigned long long* state, int c, i
     return prefix + before;
 }
 
-// The chunks of a block, out of `items` over all blocks that number (blocks 0 .. blocks - 1 of the grid): for (int t =
-// scan_first(..); t >= 0; t = scan_next(..)).
+// The chunks of a block, out of `items` over all `blocks` blocks that number: for (int t = scan_first(..); t >= 0; t =
+// scan_next(..)). The first ticket may be taken before pdl_wait() where the counter is older than the preceding kernel: the
+// trip to the counter is then over by the time that kernel is.
 __device__ __forceinline__ int scan_ticket(uint32_t* counter, int items) {
     __shared__ int s_ticket;
     __syncthreads();                 // the previous ticket has been read
@@ -82,10 +83,7 @@ __device__ __forceinline__ int scan_ticket(uint32_t* counter, int items) {
     __syncthreads();
     return s_ticket < items ? s_ticket : -1;
 }
-__device__ __forceinline__ int scan_first(uint32_t* counter, int items, int blocks) {
-    if (items <= blocks) return (int)blockIdx.x < items ? (int)blockIdx.x : -1;
-    return scan_ticket(counter, items);
-}
+__device__ __forceinline__ int scan_first(uint32_t* counter, int items) { return scan_ticket(counter, items); }
 __device__ __forceinline__ int scan_next(uint32_t* counter, int items, int blocks) {
     return items <= blocks ? -1 : scan_ticket(counter, items);
 }

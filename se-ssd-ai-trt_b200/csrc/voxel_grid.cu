@@ -54,10 +54,11 @@ point_mark_kernel(const float4* __restrict__ points, const int32_t* __restrict__
 
 __global__ void __launch_bounds__(kThreads)
 number_words_kernel(BitGrid grid, int batch, ScanState scan, int32_t* __restrict__ word_num, int32_t* status) {
-    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int chunks = scan_chunks(grid.top_words), items = batch * chunks;
-    for (int t = scan_first(scan.ticket, items, gridDim.x); t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
+    int t = scan_first(scan.ticket, items);
+    pdl_enter();
+    for (; t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = t / batch, b = t - c * batch;
         const int w = c * kThreads + threadIdx.x;
         uint4* top = grid.top + (size_t)b * grid.top_words;
@@ -93,10 +94,11 @@ __global__ void __launch_bounds__(kThreads)
 number_rows_kernel(BitGrid grid, const int32_t* __restrict__ word_num, int batch, int max_voxels, int max_points, int max_pts,
                    ScanState scan, int4* __restrict__ coors, int32_t* __restrict__ voxel_num,
                    uint32_t* __restrict__ lists, const __grid_constant__ LevelChain chain, int32_t* status) {
-    pdl_enter();
     const int lane = threadIdx.x & 31;
     const int chunks = scan_chunks(grid.words), items = batch * chunks;
-    for (int t = scan_first(scan.ticket, items, gridDim.x); t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
+    int t = scan_first(scan.ticket, items);
+    pdl_enter();
+    for (; t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = t / batch, b = t - c * batch;
         const int n = __ldg(word_num + b), used = n > 0 ? scan_chunks(n) : 1;
         if (c >= used) continue;                   // uniform over the block

@@ -72,10 +72,10 @@ template <typename T>
 __global__ void __launch_bounds__(kThreads, 5)
 voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch, int max_points,
                   VoxGeom g, VoxelTable t, int max_pts, const int32_t* __restrict__ pt_claim, ScanState scan, VoxelOut<T> out) {
-    pdl_enter();
     const int chunks = scan_chunks(max_points), items = batch * chunks;
-    for (int ticket = scan_first(scan.ticket, items, gridDim.x); ticket >= 0;
-         ticket = scan_next(scan.ticket, items, gridDim.x)) {
+    int ticket = scan_first(scan.ticket, items);
+    pdl_enter();
+    for (; ticket >= 0; ticket = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = ticket / batch, b = ticket - c * batch;
         int n = points_size[b];
         n = n < 0 ? 0 : (n > max_points ? max_points : n);

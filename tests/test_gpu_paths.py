@@ -7,6 +7,7 @@ import make_golden_inputs as mk
 from test_gpu_backbone import _check_fp32_layers, _gpu_run, _oracle_layers
 from test_gpu_conv import _check_layer, _layer, _random_coords
 from test_gpu_postprocess import _check_filter
+from test_gpu_voxelize import _compare
 
 pytestmark = pytest.mark.gpu
 
@@ -125,6 +126,13 @@ def test_numbering_of_more_chunks_than_one_scan_group(gpu, oracle):
     c = _random_coords(rs, 400, layer.in_shape)
     f = rs.randn(len(c), 16).astype(np.float32)
     _check_layer(gpu, oracle, layer, [(c, f), (c[:77], f[:77])], (rs.randn(3, 16, 32) * 0.05).astype(np.float32), maxV=1300)
+
+
+def test_numbering_with_more_chunks_than_resident_blocks(gpu, oracle):
+    """Two frames of 120,000 points: 938 chunks of points, occupied words and top words each, where 592 to 888 blocks of the
+    numbering kernels are resident."""
+    points = [gpu.synth.lidar_frame(11 + i, n_points=120000, n_boxes=40) for i in range(2)]
+    _compare(gpu, oracle, points, 100000)
 
 
 def test_filter_beyond_the_clustered_pass(gpu, oracle):
