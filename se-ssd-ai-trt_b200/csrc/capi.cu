@@ -46,8 +46,8 @@ void StageRecorder::after(const char* name, cudaStream_t s) {
     names.push_back(name);
 }
 
-int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* order, const int32_t* out_num,
-                           int frame, int kvol, int max_voxels, int32_t* pairs, uint32_t* pair_num, cudaStream_t stream);
+int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* out_num, int frame, int kvol,
+                           int max_voxels, int32_t* pairs, uint32_t* pair_num, cudaStream_t stream);
 int launch_count_pairs(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* out_num, int batch, int max_voxels,
                        int kvol, unsigned long long* total, cudaStream_t stream);
 
@@ -670,7 +670,7 @@ int sessd_conv_rulebook_export(const sessd_conv_params* p, int batch, int frame,
     Bump bump(workspace);
     ConvWorkspace ws;
     conv_workspace_layout(bump, p, g, batch, &ws);
-    return launch_rulebook_export(ws.nbr, ws.tile_mask, nullptr, static_cast<const int32_t*>(out_voxel_num), frame, g.kvol,
+    return launch_rulebook_export(ws.nbr, ws.tile_mask, static_cast<const int32_t*>(out_voxel_num), frame, g.kvol,
                                   p->max_voxels, indice_pairs, indice_num, static_cast<cudaStream_t>(stream));
 }
 

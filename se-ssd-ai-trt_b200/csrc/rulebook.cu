@@ -92,43 +92,31 @@ nbr_build_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__
     }
 }
 
-// One block per kernel offset: compacts nbr[frame][k][*] into the reference's pair columns, in ascending output row. The
-// positions of the map are brought back into row order 1024 at a time (order keeps rows within their window).
+// One block per kernel offset: compacts nbr[frame][k][*] of a map in row order into the reference's pair columns, in ascending
+// output row.
 __global__ void __launch_bounds__(kThreads)
 rulebook_export_kernel(const int32_t* __restrict__ nbr, const uint32_t* __restrict__ tile_mask,
-                       const int32_t* __restrict__ order, const int32_t* __restrict__ out_num, int frame, int kvol,
-                       int max_voxels, int32_t* __restrict__ pairs, uint32_t* __restrict__ pair_num) {
+                       const int32_t* __restrict__ out_num, int frame, int kvol, int max_voxels, int32_t* __restrict__ pairs,
+                       uint32_t* __restrict__ pair_num) {
     pdl_enter();
-    constexpr int WINDOW = 1024;
-    __shared__ int32_t s_row[WINDOW];
     const int k = blockIdx.x;
     int n = out_num[frame];
     n = n > max_voxels ? max_voxels : n;
-    const int32_t* col = nbr + nbr_index(kvol, max_voxels, frame, k, 0);   // entry p of the column: col[(p >> 7) * kvol * kNbrRun + (p & 127)]
+    const int32_t* col = nbr + nbr_index(kvol, max_voxels, frame, k, 0);   // entry o of the column: col[(o >> 7) * kvol * kNbrRun + (o & 127)]
     const uint32_t* mask = tile_mask + (size_t)frame * ((max_voxels + 127) / 128);
     int32_t* pin = pairs + ((size_t)k * 2 + 0) * max_voxels;
     int32_t* pout = pairs + ((size_t)k * 2 + 1) * max_voxels;
     int base = 0;
-    for (int w0 = 0; w0 < n; w0 += WINDOW) {
-        __syncthreads();
-        for (int e = threadIdx.x; e < WINDOW; e += kThreads) {
-            const int p = w0 + e;
-            if (p >= n) continue;
-            const int o = order ? order[(size_t)frame * max_voxels + p] : p;
-            s_row[o - w0] = (mask[p >> 7] >> k) & 1u ? col[(size_t)(p >> 7) * kvol * kNbrRun + (p & 127)] : -1;
+    for (int o0 = 0; o0 < n; o0 += kThreads) {
+        const int o = o0 + threadIdx.x;
+        const int v = o < n && (mask[o >> 7] >> k) & 1u ? col[(size_t)(o >> 7) * kvol * kNbrRun + (o & 127)] : -1;
+        int total;
+        const int pos = base + block_exclusive_scan(v >= 0 ? 1 : 0, &total);
+        if (v >= 0) {
+            pin[pos] = v;
+            pout[pos] = o;
         }
-        __syncthreads();
-        for (int e0 = 0; e0 < WINDOW && w0 + e0 < n; e0 += kThreads) {
-            const int o = w0 + e0 + threadIdx.x;
-            const int v = o < n ? s_row[e0 + threadIdx.x] : -1;
-            int total;
-            const int pos = base + block_exclusive_scan(v >= 0 ? 1 : 0, &total);
-            if (v >= 0) {
-                pin[pos] = v;
-                pout[pos] = o;
-            }
-            base += total;
-        }
+        base += total;
     }
     if (threadIdx.x == 0) pair_num[k] = (uint32_t)base;
 }
@@ -530,10 +518,10 @@ int launch_number_levels(const LevelChain& chain, int batch, int max_voxels, con
     return SESSD_OK;
 }
 
-int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* order, const int32_t* out_num,
-                           int frame, int kvol, int max_voxels, int32_t* pairs, uint32_t* pair_num, cudaStream_t stream) {
+int launch_rulebook_export(const int32_t* nbr, const uint32_t* tile_mask, const int32_t* out_num, int frame, int kvol,
+                           int max_voxels, int32_t* pairs, uint32_t* pair_num, cudaStream_t stream) {
     SESSD_CUDA(cudaMemsetAsync(pairs, 0xFF, sizeof(int32_t) * 2 * (size_t)kvol * max_voxels, stream));
-    SESSD_LAUNCH(rulebook_export_kernel, kvol, kThreads, 0, stream, nbr, tile_mask, order, out_num, frame, kvol, max_voxels,
+    SESSD_LAUNCH(rulebook_export_kernel, kvol, kThreads, 0, stream, nbr, tile_mask, out_num, frame, kvol, max_voxels,
                  pairs, pair_num);
     return SESSD_OK;
 }
