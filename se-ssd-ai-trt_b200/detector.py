@@ -81,13 +81,31 @@ class Neck2D:
             w = w * (scale[None, :, None, None] if transposed else scale[:, None, None, None])
             self.w[name] = torch.from_numpy(np.ascontiguousarray(w)).to(device).half().contiguous(memory_format=torch.channels_last)
             self.b[name] = torch.from_numpy(shift).to(device).half()
-        # the attention's two 1x1 convolutions to one channel, and the four heads, which read the same map
-        self.gate_w = torch.cat([self.w.pop(n).reshape(1, 128) for n in ("w_0", "w_1")]).contiguous()
-        self.gate_b = torch.cat([self.b.pop(n).reshape(1) for n in ("w_0", "w_1")])
-        hw = np.concatenate([np.asarray(blobs[p + ".weight"], np.float32).reshape(c, 128) for _, p, c in HEAD_LAYERS])
+        # the attention's two 1x1 convolutions to one channel lie side by side
+        gates = ("w_0", "w_1")
+        self.gate_w = torch.cat([self.w[n].reshape(1, 128) for n in gates]).contiguous()
+        self.gate_b = torch.cat([self.b[n].reshape(1) for n in gates])
+        for i, n in enumerate(gates):
+            self.w[n], self.b[n] = self.gate_w[i].view(1, 128, 1, 1), self.gate_b[i:i + 1]
+        # the four heads read the same map: one convolution with 22 output channels
+        hw = np.concatenate([np.asarray(blobs[p + ".weight"], np.float32).reshape(c, 128, 1, 1) for _, p, c in HEAD_LAYERS])
         hb = np.concatenate([np.asarray(blobs[p + ".bias"], np.float32).reshape(c) for _, p, c in HEAD_LAYERS])
-        self.head_w = torch.from_numpy(hw).to(device).half()
+        self.head_w = torch.from_numpy(hw).to(device).half().contiguous(memory_format=torch.channels_last)
         self.head_b = torch.from_numpy(hb).to(device).half()
+
+    def _by_kernels(self, x):
+        """Whether the library's kernels take x: a half map in a GPU's memory that nothing looks over the shoulder of (gradients,
+        forward mode, function transforms, tracing, autocast, dispatch modes). Any other input takes torch's operations."""
+        torch = self.torch
+        if type(x) not in (torch.Tensor, torch.nn.Parameter) or torch.compiler.is_compiling() or torch.jit.is_tracing():
+            return False
+        if x.dim() != 4 or x.shape[1] != 128 or x.dtype is not torch.float16 or not x.is_cuda or x.numel() == 0:
+            return False
+        if torch.is_grad_enabled() and (x.requires_grad or self.head_w.requires_grad or self.head_b.requires_grad or
+                                        any(t.requires_grad for d in (self.w, self.b) for t in d.values())):
+            return False
+        return (not torch.is_autocast_enabled("cuda") and torch.autograd.forward_ad._current_level < 0 and
+                torch._C._functorch.maybe_current_level() is None and torch._C._len_torch_dispatch_stack() == 0)
 
     def _channels_last(self, x):
         """x [B, C, H, W] with its channels last in memory."""
@@ -116,8 +134,39 @@ class Neck2D:
                                              y.numel() // cout, cout, _stream()), "sessd_bias_relu_enqueue")
         return y
 
+    def _torch_features(self, bev_padded):
+        torch, F = self.torch, self.torch.nn.functional
+
+        def conv(x, name, relu=True):
+            _n, _c, _b, _cin, _cout, _k, s, p = next(l for l in NECK_LAYERS if l[0] == name)
+            if name.startswith("deconv"):
+                y = F.conv_transpose2d(x, self.w[name], self.b[name], stride=s, padding=p, output_padding=1)
+            else:
+                y = F.conv2d(x, self.w[name], self.b[name], stride=s, padding=p)
+            return F.relu_(y) if relu else y
+
+        x = bev_padded.contiguous(memory_format=torch.channels_last)
+        for n in ("bu0_0", "bu0_1", "bu0_2"):
+            x = conv(x, n)
+        x0 = x
+        for n in ("bu1_0", "bu1_1", "bu1_2"):
+            x = conv(x, n)
+        t0, t1 = conv(x0, "trans_0"), conv(x, "trans_1")
+        o0, o1 = conv(conv(t1, "deconv_0") + t0, "conv_0"), conv(conv(t1, "deconv_1"), "conv_1")
+        w = torch.softmax(torch.cat([conv(o0, "w_0", relu=False), conv(o1, "w_1", relu=False)], dim=1).float(), dim=1).half()
+        return o0 * w[:, 0:1] + o1 * w[:, 1:2]
+
+    def _torch_heads(self, bev_padded):
+        y = self.torch.nn.functional.conv2d(self._torch_features(bev_padded), self.head_w, self.head_b)
+        y = y.permute(0, 2, 3, 1).float()                     # [B, H, W, 22]
+        out, c0 = {}, 0
+        for name, _p, c in HEAD_LAYERS:
+            out[name] = y[..., c0:c0 + c].reshape(y.shape[0], y.shape[1] * y.shape[2] * 2, c // 2).contiguous()
+            c0 += c
+        return out
+
     def _branches(self, bev_padded):
-        x = self._channels_last(bev_padded.half())
+        x = self._channels_last(bev_padded)
         for n in ("bu0_0", "bu0_1", "bu0_2"):
             x = self._conv(x, n)
         x0 = x
@@ -134,18 +183,25 @@ class Neck2D:
 
     def features(self, bev_padded):
         """[B, 128, 202, 178] fp16 (the zero-padded BEV map) -> fused neck output [B, 128, 200, 176]."""
-        o0, o1 = self._branches(bev_padded)
-        out = self.torch.empty_like(o0)
-        self._tail(o0, o1, features=out)
+        if not self._by_kernels(bev_padded):
+            return self._torch_features(bev_padded)
+        with self.torch.cuda.device(bev_padded.device):
+            o0, o1 = self._branches(bev_padded)
+            out = self.torch.empty_like(o0)
+            self._tail(o0, o1, features=out)
         return out
 
     def __call__(self, bev_padded):
         """-> dict of fp32 head outputs in the layout the post-processing plugins take:
         box [B, 70400, 7], cls [B, 70400, 1], iou [B, 70400, 1], dir [B, 70400, 2] (anchor = (y*W + x)*2 + a)."""
-        o0, o1 = self._branches(bev_padded)
-        B, _, H, W = o0.shape
-        out = {name: self.torch.empty((B, H * W * 2, c // 2), dtype=self.torch.float32, device=o0.device) for name, _p, c in HEAD_LAYERS}
-        self._tail(o0, o1, heads=out.values())
+        torch = self.torch
+        if not self._by_kernels(bev_padded):
+            return self._torch_heads(bev_padded)
+        with torch.cuda.device(bev_padded.device):
+            o0, o1 = self._branches(bev_padded)
+            B, _, H, W = o0.shape
+            out = {name: torch.empty((B, H * W * 2, c // 2), dtype=torch.float32, device=o0.device) for name, _p, c in HEAD_LAYERS}
+            self._tail(o0, o1, heads=out.values())
         return out
 
 

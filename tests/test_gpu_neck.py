@@ -135,3 +135,70 @@ def test_weights_written_just_before_the_call(gpu):
         assert lib.sessd_bias_relu_enqueue(big.data_ptr(), zero.data_ptr(), add.data_ptr(), len(big), 128, s) == 0
         assert run(tail, heads) == 0
         assert all(torch.equal(a, b) for a, b in zip(heads, want))
+
+
+def _close(got, want, tol=2.0 ** -8):
+    """Kernels and separate operations round to fp16 at the same points; the attention's and the heads' sums may fall on the other
+    side of a rounding (2^-11 of a weight, of its products, of a head's sum): a few of those."""
+    assert got.dtype == want.dtype and got.shape == want.shape
+    assert float((got - want).abs().max()) <= tol * float(want.abs().max())
+
+
+def test_inputs_that_the_kernels_do_not_take(gpu, neck):
+    """Gradients, forward mode, autocast, function transforms, an empty batch, the CPU, another type: as torch's operations do."""
+    import torch
+
+    D = gpu.detector
+    x = _bev(2, 10, 14)
+    want, heads = neck.features(x), neck(x)
+    leaf = x.clone().requires_grad_()
+    got = neck.features(leaf)
+    _close(got.detach(), want)
+    for k, v in neck(leaf).items():
+        _close(v.detach(), heads[k])
+    v = torch.randn(want.shape, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda").half()
+    grad, = torch.autograd.grad(got, leaf, v)
+    d = torch.randn(x.shape, generator=torch.Generator(device="cuda").manual_seed(3), device="cuda").half()
+    with torch.no_grad():
+        assert torch.equal(neck.features(leaf), want)          # nothing records it: the kernels
+    with torch.autograd.forward_ad.dual_level():
+        out = torch.autograd.forward_ad.unpack_dual(neck.features(torch.autograd.forward_ad.make_dual(x, d)))
+    _close(out.primal, want)
+    # the same derivative from both sides; fourteen fp16 layers either way (2e-2 of the sum of magnitudes)
+    a, b = float((grad.double() * d.double()).sum()), float((out.tangent.double() * v.double()).sum())
+    assert abs(a - b) <= 2e-2 * float((out.tangent.double() * v.double()).abs().sum()) and out.tangent.abs().max() > 0
+    neck.w["bu0_0"].requires_grad_()
+    try:
+        assert neck.features(x).requires_grad
+    finally:
+        neck.w["bu0_0"].requires_grad_(False)
+    _, tangent = torch.func.jvp(neck.features, (x,), (d,))
+    assert torch.equal(tangent, out.tangent)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        y = neck.features(x)
+    assert float((y.float() - want.float()).abs().max()) <= 0.1 * float(want.abs().max())   # fourteen layers of 2^-8
+    traced = torch.jit.trace(neck.features, (x,))
+    x2 = _bev(2, 10, 14, seed=8)
+    _close(traced(x2), neck.features(x2))
+    empty = neck(x[:0])
+    assert [tuple(empty[k].shape) for k in ("box", "cls", "iou", "dir")] == [(0, 8 * 12 * 2, c) for c in (7, 1, 1, 2)]
+    assert neck.features(x[:0]).shape == (0, 128, 8, 12)
+    for bad in (x.float(), x[:, :64], x[0]):
+        with pytest.raises(RuntimeError):
+            neck.features(bad)
+    host = D.Neck2D(D.random_neck_weights(), device="cpu")
+    _close(host.features(x.cpu()).float(), want.float().cpu(), 2e-2)
+    strided = x.transpose(2, 3)                                # neither layout
+    _close(neck.features(strided), neck.features(strided.contiguous()))
+
+
+def test_map_on_another_device(gpu):
+    import torch
+
+    if torch.cuda.device_count() < 2:
+        pytest.skip("needs two devices")
+    D, x = gpu.detector, _bev(1, 10, 14)
+    want = D.Neck2D(D.random_neck_weights())(x)
+    got = D.Neck2D(D.random_neck_weights(), device="cuda:1")(x.to("cuda:1"))
+    for k, v in want.items():
+        _close(got[k].cpu(), v.cpu())
