@@ -108,6 +108,44 @@ def test_few_fp16_tiles_some_without_neighbours(gpu):
     args[-1].close(), bw.close()
 
 
+@pytest.mark.parametrize("cin,cout", [(16, 32), (64, 64)])
+@pytest.mark.parametrize("frames", [8, 9, 40, 130])
+def test_fp16_work_split_over_frames(gpu, oracle, frames, cin, cout):
+    """More than one tile per SM in up to eight frames, and in more (the work is then cut with the frames' first tiles in shared
+    memory): one, two and seven tiles per thread of the cut, with empty frames at the ends and in between. Every frame has the
+    bits of a call on it alone, and the first has the oracle's values."""
+    import torch
+
+    rs = np.random.RandomState(frames + cin)
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
+    W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
+    rows, maxV = [6000, 1, 6000, 128, 5800, 6301], 6301
+    coors = [_random_coords(rs, n, layer.in_shape) for n in rows]
+    feats = [rs.randn(n, cin).astype(np.float32) for n in rows]
+    _check_layer(gpu, oracle, layer, [(coors[0], feats[0])], W, dtype=1, maxV=maxV)
+    use = [None if f in (0, 3, frames - 1) else f % len(rows) for f in range(frames)]
+    p = gpu.conv_params(layer, maxV)
+    w = gpu.ConvWeights(p, W, None, None, False, 1)
+
+    def call(which):
+        c, x, n = np.zeros((len(which), maxV, 4), np.int32), np.zeros((len(which), maxV, cin), np.float16), []
+        for b, i in enumerate(which):
+            n.append(0 if i is None else rows[i])
+            if i is not None:
+                c[b, :rows[i]], x[b, :rows[i]] = coors[i], feats[i]
+                c[b, :rows[i], 0] = b
+        r = gpu.subm_conv(torch.from_numpy(x).cuda(), torch.from_numpy(c).cuda(), torch.tensor(n, dtype=torch.int32).cuda(), p, w)
+        assert r["status"] == 0
+        return r["features"], sum((v + 127) // 128 for v in n)
+
+    got, tiles = call(use)
+    assert tiles > 148
+    alone = [call([i])[0][0] for i in range(len(rows))]
+    for b, i in enumerate(use):
+        assert not got[b].any() if i is None else torch.equal(got[b], alone[i]), b
+    w.close()
+
+
 @pytest.mark.parametrize("cin,cout,dtype", [(4, 16, 0), (4, 16, 1), (16, 16, 0), (16, 32, 0)])
 @pytest.mark.parametrize("max_voxels", [1000000, 1000001])
 def test_narrow_layers_around_a_million_rows(gpu, oracle, max_voxels, cin, cout, dtype):
