@@ -196,10 +196,12 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
 // Numbers one chunk (kThreads x WORDS words) of one frame of a level whose bits are set, in word order (= (z, y, x)
 // order): completes the records (rows before the word), writes the output coordinates (sparseConv3dlayer.cu:436-441 writes
 // them per pair) and, with the last chunk, the row count. Rows past max_voxels are dropped (their bits too, so that the
-// next level does not see them) and reported. Returns the running total with the chunk.
-template <int WORDS>
-__device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long* state, int b, int c, int chunks, int max_voxels,
-                                            int4* __restrict__ out_coors, int32_t* __restrict__ out_num, int32_t* status) {
+// next level does not see them; the record of a word that lost all of them gets kLostCells in its third word) and
+// reported. before_chunk(total): rows before the chunk, which has `total`. Returns the running total with the chunk.
+constexpr uint32_t kLostCells = 0x80000000u;
+template <int WORDS, bool WRITE = true, class Before>
+__device__ __forceinline__ int number_chunk(const BitGrid& g, int b, int c, int chunks, int max_voxels, int4* __restrict__ out_coors,
+                                            int32_t* __restrict__ out_num, int32_t* status, Before before_chunk) {
     // word i of a thread: c * kThreads * WORDS + i * kThreads + threadIdx.x, so that a warp's words of a step are neighbours.
     // Counts of the steps travel through one block scan, 16 bits each (a step has at most 256 x 64 cells).
     static_assert(WORDS <= 4, "four steps to a 64-bit scan");
@@ -232,7 +234,7 @@ __device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long
     int total = 0;
 #pragma unroll
     for (int i = 0; i < WORDS; ++i) total += (int)(all >> (16 * i) & 0xFFFFull);
-    const int prefix = scan_prefix(state, c, total, status), end = prefix + total;
+    const int prefix = before_chunk(total), end = prefix + total;
     if (c == chunks - 1 && threadIdx.x == 0) {
         out_num[b] = end > max_voxels ? max_voxels : end;
         if (end > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
@@ -256,8 +258,9 @@ __device__ __forceinline__ int number_chunk(const BitGrid& g, unsigned long long
             }
             v = kept;
         }
-        if (w < g.words) rec[w] = make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)id, next);
-        if (__any_sync(0xFFFFFFFFu, v != 0ull))
+        const uint32_t lost = v == 0ull && bits[i] != 0ull ? kLostCells : 0u;
+        if (w < g.words) rec[w] = make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)id | lost, next);
+        if (WRITE && __any_sync(0xFFFFFFFFu, v != 0ull))
             write_cells(out_coors + (size_t)b * max_voxels, b, g.xw, g.Y, w, v, min(id, max_voxels));
     }
     return end;
@@ -271,50 +274,90 @@ number_outputs_kernel(BitGrid g, int batch, int max_voxels, ScanState scan, int4
     pdl_enter();
     for (; t >= 0; t = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = t / batch, b = t - c * batch;
-        number_chunk<1>(g, scan.state + (size_t)b * chunks, b, c, chunks, max_voxels, out_coors, out_num, status);
+        number_chunk<1>(g, b, c, chunks, max_voxels, out_coors, out_num, status,
+                        [&](int total) { return scan_prefix(scan.state + (size_t)b * chunks, c, total, status); });
     }
 }
 
-// The levels below a level that had more rows than max_voxels must not see the rows it dropped: their grids are marked and
-// numbered again from the rows that are left. By one block, for a frame that has lost rows anyway.
+// Cells of word w of a level's grid that have an input cell in frame b's grid `in` of the level before: the marks of
+// mark_levels, collected from the output's side. The words of the lines that a word's cells look at are OR-ed first; what x does
+// to them (the layers of derivable_in_x) is the same for all.
+__device__ __forceinline__ unsigned long long word_outputs(const BitGrid& in, const ConvGeom& geom, const BitGrid& g, int b, int w) {
+    const int line = w / g.xw, wx = w - line * g.xw, z = line / g.Y;
+    const int z0 = z * geom.S[0] - geom.P[0], y0 = (line - z * g.Y) * geom.S[1] - geom.P[1];
+    const bool half = geom.K[2] == 3;                    // the word's cells lie over two words of `in`, and one cell before them
+    const int w0 = half ? 2 * wx : wx;
+    const uint4* rec = in.rec + (size_t)b * in.words;
+    unsigned long long lo = 0ull, hi = 0ull, left = 0ull;
+    for (int kz = 0; kz < geom.K[0]; ++kz) {
+        if ((unsigned)(z0 + kz) >= (unsigned)in.Z) continue;
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+            if (ky >= geom.K[1] || (unsigned)(y0 + ky) >= (unsigned)in.Y) continue;
+            const uint4* at = rec + ((z0 + kz) * in.Y + y0 + ky) * in.xw + w0;
+            if (w0 < in.xw) lo |= *reinterpret_cast<const unsigned long long*>(at);
+            if (half && w0 + 1 < in.xw) hi |= *reinterpret_cast<const unsigned long long*>(at + 1);
+            if (half && w0 > 0 && w0 <= in.xw) left |= *reinterpret_cast<const unsigned long long*>(at - 1) >> 63;
+        }
+    }
+    if (half) {
+        const unsigned long long odd = even_bits(lo >> 1) | (unsigned long long)even_bits(hi >> 1) << 32;
+        lo = even_bits(lo) | (unsigned long long)even_bits(hi) << 32 | odd | odd << 1 | left;
+    }
+    const int cells = g.X - (wx << 6);
+    return cells < 64 ? lo & ((1ull << cells) - 1ull) : lo;
+}
+
+// The levels below a level that had more rows than max_voxels must not see the rows it dropped: their cells are taken from the
+// rows that are left, and numbered again. By one block, for a frame that has lost rows anyway, so that what counts is that few
+// reads depend on one another: every row of the level before marking its outputs once more took 1.4 ms (one frame of 45,000 points
+// in 60,000 rows: 1762 us, now 416; 20,000 points in 20,000 rows: 922 and 432).
 __device__ __noinline__ void renumber_levels(const LevelChain& chain, int b, int l0, int max_voxels, int32_t* status) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto last_z = [&](int l) {                           // plane of the last row of a level that dropped some: they lie there or above
+        return __ldcg(reinterpret_cast<const int4*>(chain.coors[l]) + (size_t)b * max_voxels + max_voxels - 1).y;
+    };
+    int z_in = last_z(l0 - 1);                           // first plane of the level before that may have changed
     for (int l = l0; l < chain.count; ++l) {
-        const BitGrid& g = chain.grid[l];
+        const BitGrid &g = chain.grid[l], &in = chain.grid[l - 1];
+        const ConvGeom& geom = chain.geom[l];
         uint4* rec = g.rec + (size_t)b * g.words;
-        for (int w = threadIdx.x; w < g.words; w += kThreads) __stcg(rec + w, make_uint4(0u, 0u, 0u, 0u));
-        __threadfence();
-        __syncthreads();
-        const int4* in = reinterpret_cast<const int4*>(chain.coors[l - 1]) + (size_t)b * max_voxels;
-        const int n = __ldcg(chain.num[l - 1] + b);
-        for (int i = threadIdx.x; i < n; i += kThreads) mark_row(__ldcg(in + i), b, chain.geom[l], g);
-        __threadfence();
-        __syncthreads();
-        int4* out = reinterpret_cast<int4*>(chain.coors[l]) + (size_t)b * max_voxels;
-        int base = 0;
-        for (int w0 = 0; w0 < g.words; w0 += kThreads) {
-            const int w = w0 + threadIdx.x;
-            unsigned long long v = w < g.words ? rec_bits(__ldcg(rec + w)) : 0ull;
-            int total;
-            int id = base + block_exclusive_scan(__popcll(v), &total);
-            const int id0 = id;
-            const uint32_t next = next_cells(w + 1 < g.words ? __ldcg(rec + w + 1).x : 0u, w, g, id + __popcll(v), max_voxels);
-            unsigned long long kept = 0ull;
-            const int row = w / g.xw, z = row / g.Y;
-            for (; v && id < max_voxels; ++id) {
-                const int bit = __ffsll((long long)v) - 1;
-                v &= v - 1ull;
-                kept |= 1ull << bit;
-                __stcg(out + id, make_int4(b, z, row - z * g.Y, ((w - row * g.xw) << 6) + bit));
+        // planes below this one look at unchanged ones alone: their words and rows stay as they are
+        const int z0 = (max(z_in + geom.P[0] - geom.K[0] + 1, 0) + geom.S[0] - 1) / geom.S[0];
+        const int chunks = scan_chunks((g.words + 3) / 4), first = min(z0, g.Z) * g.Y * g.xw / (kThreads * 4) * (kThreads * 4);
+        int rows = first < g.words ? (int)(rec[first].z & ~kLostCells) : __ldcg(chain.totals + b * LevelChain::kMax + l);
+        // (words without a mark stay empty; marks that the first numbering removed have left kLostCells)
+        for (int w0 = first + warp * 128; w0 < g.words; w0 += kThreads * 4) {   // 128 words to a warp, a lane to each that needs it
+            unsigned long long todo[2] = {0ull, 0ull};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int w = w0 + i * 32 + lane;
+                const uint4 r = w < g.words ? rec[w] : make_uint4(0u, 0u, 0u, 0u);
+                const bool need = w < g.words && (r.x | r.y | (r.z & kLostCells)) != 0u;
+                todo[i >> 1] |= (unsigned long long)__ballot_sync(0xFFFFFFFFu, need) << (32 * (i & 1));
             }
-            if (w < g.words) __stcg(rec + w, make_uint4((uint32_t)kept, (uint32_t)(kept >> 32), (uint32_t)id0, next));
-            base += total;
+            const int n0 = __popcll(todo[0]), n = n0 + __popcll(todo[1]);
+            for (int e = lane; e < n; e += 32) {
+                const int w = w0 + (e < n0 ? nth_bit(todo[0], e) : 64 + nth_bit(todo[1], e - n0));
+                *reinterpret_cast<unsigned long long*>(rec + w) = word_outputs(in, geom, g, b, w);
+            }
         }
-        if (threadIdx.x == 0) {
-            __stcg(chain.num[l] + b, base > max_voxels ? max_voxels : base);
-            if (base > max_voxels) atomicOr(status, SESSD_STATUS_VOXEL_OVERFLOW);
-        }
-        __threadfence();
         __syncthreads();
+        for (int c = first / (kThreads * 4); c < chunks; ++c)
+            rows = number_chunk<4, false>(g, b, c, chunks, max_voxels, nullptr, chain.num[l], status, [&](int) { return rows; });
+        __syncthreads();
+        // the coordinates, by warps that need not wait for one another
+        int4* coors = reinterpret_cast<int4*>(chain.coors[l]) + (size_t)b * max_voxels;
+        auto fetch = [&](int w0) { return w0 + lane < g.words ? rec[w0 + lane] : make_uint4(0u, 0u, (uint32_t)rows, 0u); };
+        uint4 next = fetch(first + warp * 32);
+        for (int w0 = first + warp * 32; w0 < g.words; w0 += kThreads) {
+            const uint4 r = next;
+            next = fetch(w0 + kThreads);
+            if (__any_sync(0xFFFFFFFFu, (r.x | r.y) != 0u))
+                write_cells(coors, b, g.xw, g.Y, w0 + lane, rec_bits(r), min((int)(r.z & ~kLostCells), max_voxels));
+        }
+        __syncthreads();
+        z_in = rows > max_voxels ? min(z0, last_z(l)) : z0;
     }
 }
 
@@ -346,8 +389,10 @@ number_levels_kernel(const __grid_constant__ LevelChain chain, int batch, int ma
             if (c < chunks) break;
             c -= chunks;
         }
-        const int end = number_chunk<WORDS>(chain.grid[l], chain.state[l] + (size_t)b * chunks, b, c, chunks, max_voxels,
-                                            reinterpret_cast<int4*>(chain.coors[l]), chain.num[l], status);
+        const int end = number_chunk<WORDS>(chain.grid[l], b, c, chunks, max_voxels, reinterpret_cast<int4*>(chain.coors[l]), chain.num[l],
+                                            status, [&](int total) {
+                                                return scan_prefix(chain.state[l] + (size_t)b * chunks, c, total, status);
+                                            });
         if (c == chunks - 1 && threadIdx.x == 0) chain.totals[b * LevelChain::kMax + l] = end;
         // the frame's last block looks whether a level lost rows
         __threadfence();

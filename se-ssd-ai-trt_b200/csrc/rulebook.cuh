@@ -51,6 +51,7 @@ __device__ __forceinline__ int nth_bit(unsigned long long v, int n) {
 __device__ __forceinline__ void write_cells(int4* __restrict__ coors, int b, int xw, int Y, int word, unsigned long long bits,
                                             int id) {
     const int lane = threadIdx.x & 31;
+    const int line = word / xw, z0 = line / Y, y0 = line - z0 * Y, x0 = (word - line * xw) << 6;   // of the word's first cell
     const int first = __shfl_sync(0xFFFFFFFFu, id, 0);
     const int end = __shfl_sync(0xFFFFFFFFu, id + __popcll(bits), 31);
     for (int r0 = first; r0 < end; r0 += 32) {
@@ -61,10 +62,8 @@ __device__ __forceinline__ void write_cells(int4* __restrict__ coors, int b, int
             if (__shfl_sync(0xFFFFFFFFu, id, src + s) <= r) src += s;
         const int id0 = __shfl_sync(0xFFFFFFFFu, id, src);
         const unsigned long long v = __shfl_sync(0xFFFFFFFFu, bits, src);
-        const int w = __shfl_sync(0xFFFFFFFFu, word, src);
-        if (r >= end) continue;
-        const int line = w / xw, z = line / Y;
-        coors[r] = make_int4(b, z, line - z * Y, ((w - line * xw) << 6) + nth_bit(v, r - id0));
+        const int z = __shfl_sync(0xFFFFFFFFu, z0, src), y = __shfl_sync(0xFFFFFFFFu, y0, src), x = __shfl_sync(0xFFFFFFFFu, x0, src);
+        if (r < end) coors[r] = make_int4(b, z, y, x + nth_bit(v, r - id0));
     }
 }
 

@@ -245,6 +245,65 @@ def test_front_end_with_more_points_than_rows(gpu, oracle):
     _check_fp32_layers(_oracle_layers(oracle, case, False), views)
 
 
+def _levels_against_calls(gpu, layers, W, sc, sh, pts, sizes, max_voxels, **where):
+    """Front end of pts [B, P, 4]: every strided layer against its plugin call on the layer before, bit for bit. Returns how many
+    of them lost rows."""
+    import torch
+
+    B, P = pts.shape[:2]
+    bb = gpu.Backbone(max_voxels, W, sc, sh, dtype=0, layers=layers, with_dense=False, **where)
+    _, ws = bb.run(pts.cuda(), sizes)
+    assert gpu.read_status(ws) & gpu.STATUS_VOXEL_OVERFLOW
+    view = lambda i: [t.clone() for t in bb.layer_view(ws, B, P, i)]
+    lost = 0
+    for i, l in enumerate(layers):
+        if l.subm:
+            continue
+        f, c, n = view(i - 1)
+        p = gpu.conv_params(l, max_voxels)
+        w = gpu.ConvWeights(p, W[i], sc[i], sh[i], True, 0)
+        r = gpu.sparse_conv(f, c, n, p, w)
+        gf, gc, gn = view(i)
+        lost += bool(r["status"] & gpu.STATUS_VOXEL_OVERFLOW)
+        assert torch.equal(gn, r["voxel_num"]) and int(gn.max()) <= max_voxels, i
+        for b in range(B):
+            m = int(gn[b])
+            assert torch.equal(gc[b, :m], r["coors"][b, :m]) and torch.equal(gf[b, :m], r["features"][b, :m]), (i, b)
+        w.close()
+    bb.close()
+    return lost
+
+
+@pytest.mark.parametrize("points,max_voxels", [(20000, 20000), (8000, 8000), (45000, 60000)])
+def test_full_size_levels_that_lose_rows(gpu, points, max_voxels):
+    """The network's levels, with lines of several words: the first derived level of one of two frames has more rows than
+    max_voxels; so has the next one as first marked, except for 45,000 points."""
+    import torch
+
+    pts = torch.zeros((2, points, 4))
+    pts[0] = torch.from_numpy(gpu.synth.lidar_frame(5, n_points=points, n_boxes=20))
+    pts[1, :2000] = torch.from_numpy(gpu.synth.lidar_frame(6, n_points=2000, n_boxes=5))
+    sizes = torch.tensor([points, 2000], dtype=torch.int32).cuda()
+    assert _levels_against_calls(gpu, gpu.schedule.LAYERS, *gpu.random_weights(), pts, sizes, max_voxels)
+
+
+@pytest.mark.parametrize("K,S,P", [((1, 2, 3), (1, 1, 2), (0, 0, 1)), ((2, 1, 1), (3, 2, 1), (1, 0, 0)), ((3, 3, 3), (1, 2, 2), (2, 2, 1))])
+def test_levels_of_other_layers_that_lose_rows(gpu, K, S, P):
+    """Below a level that loses rows: other kernels, strides and paddings (in x those that levels can be marked with)."""
+    import torch
+
+    layers, shape = [], (41, 80, 192)
+    for cin, cout, k, s, p in ((4, 16, (3, 3, 1), (1, 1, 1), (1, 1, 0)), (16, 32, K, S, P), (32, 32, (3, 3, 3), (2, 2, 2), (1, 1, 1)), (32, 64, K, S, P)):
+        layers.append(_layer(gpu, False, cin, cout, k, s, p, shape))
+        shape = layers[-1].out_shape
+    points = np.concatenate([_scattered_points(2000, 7 + i) + np.array([3.2 * i, 0, 0, 0], np.float32) for i in range(3)])
+    points = points[np.random.RandomState(1).permutation(len(points))]
+    sizes = torch.tensor([6000, 300], dtype=torch.int32).cuda()
+    pts = torch.from_numpy(np.stack([points, points]))
+    assert _levels_against_calls(gpu, tuple(layers), *gpu.random_weights(layers=tuple(layers)), pts, sizes, 6100,
+                                 point_range=(0.0, 0.0, -3.0, 9.6, 4.0, 1.0), voxel_size=gpu.synth.VOXEL_SIZE)
+
+
 @pytest.mark.parametrize("max_voxels", [1500, 1537])
 def test_levels_that_lose_rows(gpu, max_voxels):
     """A level with more rows than max_voxels keeps the first in (z, y, x) order, and the levels below see only those: what a
@@ -258,28 +317,8 @@ def test_levels_that_lose_rows(gpu, max_voxels):
     for b, f in enumerate(frames):
         pts[b, :len(f)] = torch.from_numpy(f)
     sizes = torch.tensor([len(f) for f in frames], dtype=torch.int32).cuda()
-    bb = gpu.Backbone(max_voxels, small["weights"], small["scale"], small["shift"], dtype=0, layers=layers,
-                      point_range=small["range"], voxel_size=small["voxel"])
-    _, ws = bb.run(pts.cuda(), sizes)
-    assert gpu.read_status(ws) & gpu.STATUS_VOXEL_OVERFLOW
-    view = lambda i: [t.clone() for t in bb.layer_view(ws, 2, 1500, i)]
-    lost = 0
-    for i, l in enumerate(layers):
-        if l.subm:
-            continue
-        f, c, n = view(i - 1)
-        p = gpu.conv_params(l, max_voxels)
-        w = gpu.ConvWeights(p, small["weights"][i], small["scale"][i], small["shift"][i], True, 0)
-        r = gpu.sparse_conv(f, c, n, p, w)
-        gf, gc, gn = view(i)
-        lost += bool(r["status"] & gpu.STATUS_VOXEL_OVERFLOW)
-        assert torch.equal(gn, r["voxel_num"]) and int(gn[0]) <= max_voxels
-        for b in range(2):
-            m = int(gn[b])
-            assert torch.equal(gc[b, :m], r["coors"][b, :m]) and torch.equal(gf[b, :m], r["features"][b, :m])
-        w.close()
-    assert lost
-    bb.close()
+    assert _levels_against_calls(gpu, layers, small["weights"], small["scale"], small["shift"], pts, sizes, max_voxels,
+                                 point_range=small["range"], voxel_size=small["voxel"])
 
 
 def test_status_is_not_read_during_capture(gpu):
