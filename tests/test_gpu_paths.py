@@ -173,6 +173,23 @@ def test_numbering_with_more_chunks_than_resident_blocks(gpu, oracle):
     _compare(gpu, oracle, points, 100000)
 
 
+@pytest.mark.parametrize("rows", [64, 1024, 16384])
+@pytest.mark.parametrize("subm", [True, False])
+def test_tables_with_every_row_in_use(gpu, oracle, rows, subm):
+    """max_voxels rows of power-of-two size, all of them cells of x groups of their own."""
+    rs = np.random.RandomState(rows)
+    K, S = (3, 3, 3), (1, 1, 1) if subm else (2, 2, 2)
+    layer = _layer(gpu, subm, 16, 16 if subm else 32, K, S, (1, 1, 1), (12, 96, 128))
+    c = _random_coords(rs, rows, (12, 96, 32))
+    c[:, 3] = c[:, 3] * 4 + 1
+    f = rs.randn(rows, 16).astype(np.float32)
+    W = (rs.randn(27, 16, layer.cout) * 0.1).astype(np.float32)
+    if not subm:                                   # outputs must fit the rows: every input reaches one alone
+        layer = _layer(gpu, False, 16, 32, (2, 2, 2), (2, 2, 2), (0, 0, 0), (12, 96, 128))
+        W = W[:8]
+    _check_layer(gpu, oracle, layer, [(c, f)], W, maxV=rows)
+
+
 def test_filter_beyond_the_clustered_pass(gpu, oracle):
     """133,120 anchors: more than a cluster holds (131,072), so two passes."""
     _check_filter(gpu, oracle, 2, 260, 256, 500, -4.0, True, 11)
