@@ -598,7 +598,8 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     tails.counts = subm ? in_num : static_cast<const int32_t*>(outputs[2]);
     tails.batch = batch, tails.max_rows = tails.most = maxV;
     FillRanges fills{};
-    fills.ptr[0] = static_cast<uint4*>(ws.ones_base), fills.n16[0] = ws.ones_bytes / 16, fills.ones[0] = 1;
+    const bool by_inputs = !subm && scatter_rows_usable(g);   // (no table then)
+    if (!by_inputs) fills.ptr[0] = static_cast<uint4*>(ws.ones_base), fills.n16[0] = ws.ones_bytes / 16, fills.ones[0] = 1;
     fills.ptr[1] = static_cast<uint4*>(ws.zero_base), fills.n16[1] = ws.zero_bytes / 16, fills.ones[1] = 0;
     fills.status = ws.status;
     rc = launch_prepare(fills, subm ? tails : TailRows{}, w->impl.umma_w == nullptr, stream);
@@ -606,18 +607,23 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     const int32_t* out_num = in_num;
     if (!subm) out_num = static_cast<const int32_t*>(outputs[2]);
     if (!subm || is_subm_333(g)) {
-        rc = launch_bucket_build(in_coors, in_num, batch, maxV, g.in_shape, ws.buckets, subm ? nullptr : &g, ws.out_bits,
-                                 ws.status, stream);
+        rc = by_inputs ? launch_mark_outputs(in_coors, in_num, batch, maxV, g, ws.out_bits, stream)
+                       : launch_bucket_build(in_coors, in_num, batch, maxV, g.in_shape, ws.buckets, subm ? nullptr : &g, ws.out_bits,
+                                             ws.status, stream);
         if (rc) return rc;
         if (!subm) {
             rc = launch_number_outputs(ws.out_bits, batch, maxV, ws.scan, static_cast<int32_t*>(outputs[1]),
                                        static_cast<int32_t*>(outputs[2]), ws.status, stream);
             if (rc) return rc;
         }
-        MapJob job = make_map_job(g, subm ? in_coors : static_cast<const int32_t*>(outputs[1]), out_num, p->in_channel, ws.nbr,
-                                  ws.tile_mask, nullptr);
-        job.table = ws.buckets;
-        rc = launch_map_tiles(job, batch, maxV, subm ? TailRows{} : tails, stream);
+        if (by_inputs) {
+            rc = launch_scatter_rows(in_coors, in_num, out_num, batch, maxV, g, ws.out_bits, ws.nbr, ws.tile_mask, tails, stream);
+        } else {
+            MapJob job = make_map_job(g, subm ? in_coors : static_cast<const int32_t*>(outputs[1]), out_num, p->in_channel, ws.nbr,
+                                      ws.tile_mask, nullptr);
+            job.table = ws.buckets;
+            rc = launch_map_tiles(job, batch, maxV, subm ? TailRows{} : tails, stream);
+        }
         if (rc) return rc;
     } else {
         rc = launch_table_build(in_coors, in_num, batch, maxV, g.in_shape, ws.in_table, ws.status, stream);

@@ -189,7 +189,6 @@ struct ConvGeom {
     int kvol;
     int span_max[3];  // most candidate outputs one input can have per axis
     int ncand;        // product of span_max
-    int cand_shift;   // log2(ncand) when ncand is a power of two, else -1
 };
 
 // ---- device side -------------------------------------------------------------------------
@@ -320,6 +319,11 @@ int launch_nbr_build(const int32_t* out_coors, const int32_t* out_num, int batch
 int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batch, int max_voxels, const ConvGeom& g,
                         const BitGrid& out, cudaStream_t stream);
 bool derivable_in_x(const ConvGeom& g);
+// Their maps by input rows, once the outputs are numbered; tile_mask zero before. Where the rule says so.
+bool scatter_rows_usable(const ConvGeom& g);
+int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch, int max_voxels,
+                        const ConvGeom& g, const BitGrid& out, int32_t* nbr, uint32_t* tile_mask, const TailRows& tails,
+                        cudaStream_t stream);
 
 // The levels that a chain of strided layers makes from the voxeliser's level, when the occupancy of all of them follows
 // word by word from the voxeliser's grid (level_chain_usable): marked by one kernel and numbered by one.

@@ -22,6 +22,7 @@
 //     arrival order of an atomic over a dense scan (sparseConv3dlayer.cu:529-541); (z, y, x) order is
 //     deterministic and keeps the rows of a 128-row tile close together in space;
 //   - coordinates handed in by a caller (the stand-alone plugin entry points) go into a flat table.
+#include "fill.cuh"
 #include "rulebook.cuh"
 #include "scan.cuh"
 #include "voxel.cuh"
@@ -190,6 +191,73 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
         n = n > max_voxels ? max_voxels : n;
         if (i >= n) continue;
         mark_row(__ldg(&in_coors[(size_t)b * max_voxels + i]), b, g, out);
+    }
+}
+
+// ---- maps of strided layers by input rows ----------------------------------------------------------
+// No table: every candidate output of an input row is looked up in the numbered output grid, and the pair lands as
+// nbr[b][k][out] = row. Pays where the grid is fine (scatter_rows_usable): rows then have few neighbours and there are more
+// outputs than inputs.
+
+// Fills the map entries of the tiles that hold rows 0 .. out_num[b] with -1, 16 bytes per thread (a tile's kvol x kNbrRun words
+// are contiguous; the padding is written too), and zeroes the tails of the call's outputs.
+__global__ void __launch_bounds__(kThreads)
+nbr_clear_kernel(int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels, int kvol,
+                 TailRows tails) {
+    pdl_enter();
+    zero_tails(tails);
+    const size_t frame_words = nbr_frame_words(kvol, max_voxels);
+    const int chunks = (int)((frame_words / 4 + kThreads - 1) / kThreads);
+    const int64_t items = (int64_t)batch * chunks;
+    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+        const int b = (int)(it / chunks);
+        const int n = min(__ldg(out_num + b), max_voxels);
+        const size_t w = ((size_t)(it - (int64_t)b * chunks) * kThreads + threadIdx.x) * 4;
+        if (w < (size_t)((n + 127) / 128) * kvol * kNbrRun)
+            *reinterpret_cast<int4*>(nbr + (size_t)b * frame_words + w) = make_int4(-1, -1, -1, -1);
+    }
+}
+
+// Thread = (input row, candidate output) as in mark_row, k = in - out*stride + pad per axis (sparseConv3dlayer.cu:366). Rows of
+// the same cell: the highest wins, as in a table.
+__global__ void __launch_bounds__(kThreads)
+scatter_rows_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict__ in_num, int batch, int max_voxels,
+                    ConvGeom g, BitGrid out, int32_t* __restrict__ nbr, uint32_t* __restrict__ tile_mask) {
+    pdl_enter();
+    const int tiles = (max_voxels + 127) / 128;
+    const int chunks = (int)(((int64_t)max_voxels * g.ncand + kThreads - 1) / kThreads);
+    const int64_t items = (int64_t)batch * chunks;
+    for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
+        const int b = (int)(it / chunks);
+        const int t = (int)(it - (int64_t)b * chunks) * kThreads + threadIdx.x;
+        const int n = min(__ldg(in_num + b), max_voxels);
+        if (t >= n * g.ncand) continue;
+        int i, e[3], rest;
+        split_small(t, g.span_max[2], &rest, &e[2]);
+        split_small(rest, g.span_max[1], &rest, &e[1]);
+        split_small(rest, g.span_max[0], &i, &e[0]);
+        const int4 c4 = __ldg(&in_coors[(size_t)b * max_voxels + i]);
+        const int c[3] = {c4.y, c4.z, c4.w};
+        int o[3], k = 0;
+        bool ok = true;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            const int lo = div_trunc(c[j] - (g.K[j] - 1) - 1 + g.S[j] + g.P[j], g.S[j]);
+            const int hi = div_trunc(c[j] + g.P[j], g.S[j]);
+            o[j] = hi - e[j];
+            const int kj = c[j] - o[j] * g.S[j] + g.P[j];
+            ok = ok && e[j] <= hi - lo && o[j] >= 0 && o[j] < g.out_shape[j] && kj >= 0 && kj < g.K[j] && c[j] >= 0 &&
+                 c[j] < g.in_shape[j];
+            k = k * g.K[j] + kj;
+        }
+        if (!ok) continue;
+        const uint4 r = __ldg(out.rec + (size_t)b * out.words + ((size_t)o[0] * out.Y + o[1]) * out.xw + (o[2] >> 6));
+        const unsigned long long bits = rec_bits(r), bit = 1ull << (o[2] & 63);
+        if (!(bits & bit)) continue;                     // dropped: past max_voxels
+        const int row = (int)r.z + __popcll(bits & (bit - 1ull));
+        atomicMax(nbr + nbr_index(g.kvol, max_voxels, b, k, row), i);
+        uint32_t* m = tile_mask + (size_t)b * tiles + (row >> 7);
+        if (!((*reinterpret_cast<volatile uint32_t*>(m) >> k) & 1u)) atomicOr(m, 1u << k);
     }
 }
 
@@ -484,9 +552,6 @@ int conv_geom_from_params(const sessd_conv_params* p, ConvGeom* g) {
         g->span_max[j] = (g->K[j] - 1) / g->S[j] + 1;
         g->ncand *= g->span_max[j];
     }
-    g->cand_shift = -1;
-    for (int sh = 0; sh < 6; ++sh)
-        if (g->ncand == (1 << sh)) g->cand_shift = sh;
     const uint64_t vin = (uint64_t)g->in_shape[0] * g->in_shape[1] * g->in_shape[2];
     const uint64_t vout = (uint64_t)g->out_shape[0] * g->out_shape[1] * g->out_shape[2];
     if (vin >= 0xFFFFFFFFull || vout >= 0xFFFFFFFFull) return SESSD_ERR_PARAM;  // keys are 32-bit cell indices
@@ -511,6 +576,23 @@ int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batc
                         const BitGrid& out, cudaStream_t stream) {
     SESSD_LAUNCH(mark_outputs_kernel, persistent_grid(8), kThreads, 0, stream, reinterpret_cast<const int4*>(in_coors),
                  in_num, batch, max_voxels, g, out);
+    return SESSD_OK;
+}
+
+// Fine grids: a row of the network's full resolution (92 M cells) has 3.4 candidate outputs and there are twice as many outputs as
+// inputs, so that going by inputs touches less; one level down (12 M cells) there are fewer outputs than inputs. Strided calls, by
+// inputs and through a table: full resolution, 1 x 20,000 points 53 and 58 us, 16 x 20,000 222 and 247, 1 x 120,000 94 and 86,
+// 8 x 120,000 366 and 423; one level down 68 and 67, 267 and 248, 142 and 96, 466 and 373. The line lies between the two.
+bool scatter_rows_usable(const ConvGeom& g) {
+    return (uint64_t)g.in_shape[0] * g.in_shape[1] * g.in_shape[2] >= 1ull << 25;
+}
+
+int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch, int max_voxels,
+                        const ConvGeom& g, const BitGrid& out, int32_t* nbr, uint32_t* tile_mask, const TailRows& tails,
+                        cudaStream_t stream) {
+    SESSD_LAUNCH(nbr_clear_kernel, persistent_grid(8), kThreads, 0, stream, nbr, out_num, batch, max_voxels, g.kvol, tails);
+    SESSD_LAUNCH(scatter_rows_kernel, persistent_grid(8), kThreads, 0, stream, reinterpret_cast<const int4*>(in_coors), in_num,
+                 batch, max_voxels, g, out, nbr, tile_mask);
     return SESSD_OK;
 }
 

@@ -190,6 +190,49 @@ def test_tables_with_every_row_in_use(gpu, oracle, rows, subm):
     _check_layer(gpu, oracle, layer, [(c, f)], W, maxV=rows)
 
 
+@pytest.mark.parametrize("K,S,P", [((3, 3, 3), (2, 2, 2), (1, 1, 1)), ((3, 3, 3), (2, 2, 2), (0, 2, 2)), ((3, 1, 1), (2, 1, 1), (0, 0, 0)),
+                                   ((1, 2, 3), (1, 1, 1), (0, 1, 2)), ((2, 3, 1), (3, 2, 3), (1, 2, 0)), ((3, 3, 3), (1, 3, 2), (1, 0, 2))])
+@pytest.mark.parametrize("edge", [1448, 1449])
+def test_strided_maps_by_inputs_and_through_a_table(gpu, oracle, edge, K, S, P):
+    """Grids of 16 x 1448 x 1448 cells (just under 2^25) and 16 x 1449 x 1449 (just over): maps through a table, and by input rows."""
+    rs = np.random.RandomState(3)
+    layer = _layer(gpu, False, 16, 32, K, S, P, (16, edge, edge))
+    c = np.concatenate([_random_coords(rs, 200, (16, 20, 30)), _random_coords(rs, 150, layer.in_shape)])
+    c = np.unique(np.concatenate([c, [[0, 15, edge - 1, edge - 1], [0, 0, edge - 1, 0], [0, 15, 0, edge - 2]]]).astype(np.int32), axis=0)
+    c = rs.permutation(c)
+    f = rs.randn(len(c), 16).astype(np.float32)
+    W = (rs.randn(int(np.prod(K)), 16, 32) * 0.1).astype(np.float32)
+    _check_layer(gpu, oracle, layer, [(c, f), (c[:131], f[:131]), (c[:0], f[:0])], W, maxV=len(c) * 27)
+
+
+@pytest.mark.parametrize("edge", [1448, 1449])
+def test_strided_rows_outside_the_grid_and_of_the_same_cell(gpu, edge):
+    """Rows outside reach nothing; of two rows of a cell the later one counts. Both ways of making the map."""
+    import torch
+
+    rs = np.random.RandomState(8)
+    layer = _layer(gpu, False, 16, 32, (3, 3, 3), (2, 2, 2), (1, 1, 1), (16, edge, edge))
+    c = _random_coords(rs, 300, (16, 20, 30))
+    f = rs.randn(300, 16).astype(np.float32)
+    extra = np.array([[0, -1, 3, 3], [0, 16, 3, 3], [0, 3, -2, 3], [0, 3, edge, 3], [0, 3, 3, -1], [0, 3, 3, edge + 5]], np.int32)
+    stale = rs.randn(300 + len(extra), 16).astype(np.float32)
+    W = (rs.randn(27, 16, 32) * 0.1).astype(np.float32)
+    p = gpu.conv_params(layer, 3000)
+    w = gpu.ConvWeights(p, W, None, None, False, 0)
+
+    def call(coors, feat):
+        x, co = np.zeros((1, 3000, 16), np.float32), np.zeros((1, 3000, 4), np.int32)
+        x[0, :len(feat)], co[0, :len(coors)] = feat, coors
+        r = gpu.sparse_conv(torch.from_numpy(x).cuda(), torch.from_numpy(co).cuda(), torch.tensor([len(coors)], dtype=torch.int32).cuda(), p, w)
+        assert r["status"] == 0
+        return r
+    want = call(c, f)
+    got = call(np.concatenate([c, extra, c]), np.concatenate([stale, f]))
+    for k in ("voxel_num", "coors", "features"):
+        assert torch.equal(want[k], got[k]), k
+    w.close()
+
+
 def test_filter_beyond_the_clustered_pass(gpu, oracle):
     """133,120 anchors: more than a cluster holds (131,072), so two passes."""
     _check_filter(gpu, oracle, 2, 260, 256, 500, -4.0, True, 11)
