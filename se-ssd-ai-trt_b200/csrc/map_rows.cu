@@ -555,7 +555,10 @@ int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const Row
 int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
     const int tiles = (max_voxels + 127) / 128;
     const int64_t items = (int64_t)batch * tiles;
-    const int most = persistent_grid(6);
+    // four rounds of the nine blocks that are resident: with six per SM the reads in flight did not cover their latency, and in few
+    // rounds the blocks whose tiles are empty leave SMs idle (calls of 8 x 120,000 points, 4 -> 16 channels: six 334 us, nine 318,
+    // eighteen 307, thirty-six 304; 4 x 20,000 points, 16 -> 16: 54, 53, 44, 44)
+    const int most = persistent_grid(36);
     SESSD_LAUNCH(map_tiles_kernel, (int)(items < most ? items : most), 128, 0, stream, job, batch, max_voxels, tiles, tails);
     return SESSD_OK;
 }
