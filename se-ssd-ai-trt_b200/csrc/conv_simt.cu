@@ -306,7 +306,9 @@ conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t
         for (int co = lane; co < cout; co += 32) {
             float acc = 0.f;
             for (int k = 0; k < kvol; ++k) {
-                const int idx = (mask >> k) & 1u ? __ldg(nb + k * kNbrRun) : -1;
+                // the entry is read whether the mask has the offset or not, so that reads run ahead of the loop (behind the mask:
+                // 4 x 120,000 points, 8 -> 24 channels 670 us instead of 640); what it holds counts only where the mask has it
+                const int entry = __ldg(nb + k * kNbrRun), idx = (mask >> k) & 1u ? entry : -1;
                 if (idx < 0) continue;
                 const T* x = in_b + (size_t)idx * cin;
                 const T* wk = weights + (size_t)k * cin * cout + co;
