@@ -397,10 +397,14 @@ int sessd_rotated_nms_enqueue(const sessd_nms_params* p, int batch, const void* 
     // the staged copy of a frame's mask must fit the 48 KB a block gets without opting in; larger tables are read in place
     const size_t stage_bytes = M * words * sizeof(unsigned long long);
     const int smem_words = stage_bytes <= 40 * 1024 ? (int)(M * words) : 0;
-    // a warp per (box, segment) of a full frame, unless the frames of the batch have to share the GPU
-    const int most = persistent_grid(4) / batch > 1 ? persistent_grid(4) / batch : 1;
-    const int full = (int)((M * words * 2 + kMaskWarps - 1) / kMaskWarps);
-    const int blocks_per_frame = full < most ? full : most;
+    // A warp per (box, segment) of a full frame, unless the frames of the batch have to share the GPU: then a frame's part of the
+    // blocks that are resident. Where that is a few blocks with much to do, the parts do not fill the GPU and frames differ: four
+    // times as many blocks then (500 boxes, random and all overlapping, us: 16 frames 128 and 329 with one round of blocks, 136 and
+    // 345 with four; 128 frames 723 and 3835, 576 and 2635; 100 boxes, 512 frames 158, 166).
+    const int full = (int)((M * words * 2 + kMaskWarps - 1) / kMaskWarps), resident = persistent_grid(4);
+    int blocks_per_frame = resident / batch > 1 ? resident / batch : 1;
+    if (blocks_per_frame < 16 && full / blocks_per_frame >= 64) blocks_per_frame = 4 * resident / batch > 1 ? 4 * resident / batch : 1;
+    if (blocks_per_frame > full) blocks_per_frame = full;
     SESSD_LAUNCH(nms_mask_kernel, batch * blocks_per_frame, kMaskThreads, (size_t)smem_words * sizeof(unsigned long long), stream,
                  a, blocks_per_frame, smem_words);
     return SESSD_OK;

@@ -228,3 +228,22 @@ def test_rotated_nms_after_score_filter(gpu, oracle):
         want, _ = oracle.rotated_nms(src, S.NMS_THRESH)
         assert int(kept_num[b]) == len(want) and len(want) > 0
         np.testing.assert_array_equal(kept[b, :len(want)].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("frames", [37, 38, 300])
+def test_nms_of_many_frames_equals_that_of_each(gpu, frames):
+    """500 boxes a frame, most of them overlapping: at 37 frames (16 blocks each on 148 SMs) and 38 the frames' share of the GPU
+    changes; 300 frames have more blocks than are resident."""
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(frames)
+    boxes = torch.rand((frames, 500, 9), generator=g, device="cuda")
+    boxes[..., 0] *= 20
+    boxes[..., 1] *= 20
+    boxes[..., 3], boxes[..., 4] = 1.6, 3.9
+    valid = torch.randint(0, 501, (frames,), generator=g, device="cuda").int()
+    valid[0], valid[-1] = 500, 0
+    kept, num = gpu.rotated_nms(boxes, valid)
+    for b in list(range(0, frames, 13)) + [frames - 1]:
+        k, n = gpu.rotated_nms(boxes[b:b + 1].contiguous(), valid[b:b + 1].contiguous())
+        assert int(n[0]) == int(num[b]) and torch.equal(k[0], kept[b])
