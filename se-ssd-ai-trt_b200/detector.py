@@ -8,6 +8,8 @@ with the batch norms folded in: library glue, as in the reference. What lies bet
 the attention over the two branches, the 1x1 heads) is the library's. Needs a CUDA device."""
 from __future__ import annotations
 
+import contextlib
+
 import numpy as np
 
 from . import schedule, synth
@@ -102,7 +104,8 @@ class Neck2D:
         if x.dim() != 4 or x.shape[1] != 128 or x.dtype is not torch.float16 or not x.is_cuda or x.numel() == 0:
             return False
         if torch.is_grad_enabled() and (x.requires_grad or self.head_w.requires_grad or self.head_b.requires_grad or
-                                        any(t.requires_grad for d in (self.w, self.b) for t in d.values())):
+                                        True in [t.requires_grad for t in self.w.values()] or
+                                        True in [t.requires_grad for t in self.b.values()]):
             return False
         return (not torch.is_autocast_enabled("cuda") and torch.autograd.forward_ad._current_level < 0 and
                 torch._C._functorch.maybe_current_level() is None and torch._C._len_torch_dispatch_stack() == 0)
@@ -133,6 +136,10 @@ class Neck2D:
         _check(lib().sessd_bias_relu_enqueue(y.data_ptr(), self.b[name].data_ptr(), None if add is None else add.data_ptr(),
                                              y.numel() // cout, cout, _stream()), "sessd_bias_relu_enqueue")
         return y
+
+    def _on_device_of(self, x):
+        cuda = self.torch.cuda
+        return contextlib.nullcontext() if x.device.index == cuda.current_device() else cuda.device(x.device)
 
     def _torch_features(self, bev_padded):
         torch, F = self.torch, self.torch.nn.functional
@@ -185,7 +192,7 @@ class Neck2D:
         """[B, 128, 202, 178] fp16 (the zero-padded BEV map) -> fused neck output [B, 128, 200, 176]."""
         if not self._by_kernels(bev_padded):
             return self._torch_features(bev_padded)
-        with self.torch.cuda.device(bev_padded.device):
+        with self._on_device_of(bev_padded):
             o0, o1 = self._branches(bev_padded)
             out = self.torch.empty_like(o0)
             self._tail(o0, o1, features=out)
@@ -197,7 +204,7 @@ class Neck2D:
         torch = self.torch
         if not self._by_kernels(bev_padded):
             return self._torch_heads(bev_padded)
-        with torch.cuda.device(bev_padded.device):
+        with self._on_device_of(bev_padded):
             o0, o1 = self._branches(bev_padded)
             B, _, H, W = o0.shape
             out = {name: torch.empty((B, H * W * 2, c // 2), dtype=torch.float32, device=o0.device) for name, _p, c in HEAD_LAYERS}
