@@ -32,6 +32,13 @@ int sm_count() {
     return cached[dev];
 }
 
+int copy_status(const void* workspace, cudaStream_t stream) {
+    int32_t v = 0;
+    SESSD_CUDA(cudaStreamSynchronize(stream));
+    SESSD_CUDA(cudaMemcpy(&v, workspace, sizeof(v), cudaMemcpyDeviceToHost));
+    return v & 0x7FFFFFFF;
+}
+
 void StageRecorder::before(cudaStream_t s) {
     cudaEvent_t e;
     cudaEventCreate(&e);
@@ -369,11 +376,10 @@ int sessd_read_status2(const void* workspace, const void* other, void* stream_) 
     bool here;
     SESSD_CUDA(on_current_device(workspace, other, stream, &here));
     if (!here) {
-        int32_t v[2];
-        SESSD_CUDA(cudaStreamSynchronize(stream));
-        SESSD_CUDA(cudaMemcpy(&v[0], workspace, sizeof(v[0]), cudaMemcpyDeviceToHost));
-        SESSD_CUDA(cudaMemcpy(&v[1], other, sizeof(v[1]), cudaMemcpyDeviceToHost));
-        return (v[0] | v[1]) & 0x7FFFFFFF;
+        const int first = copy_status(workspace, stream);
+        if (first < 0 || other == workspace) return first;
+        const int second = copy_status(other, stream);
+        return second < 0 ? second : first | second;
     }
     static thread_local StatusSlot slot;
     if (!slot.word) {

@@ -81,6 +81,9 @@ inline cudaError_t launch_kernel(bool overlap, void (*kernel)(P...), int grid, i
 #define SESSD_LAUNCH(kernel, grid, block, smem, stream, ...) \
     SESSD_LAUNCH_IMPL(true, #kernel, kernel, grid, block, smem, stream, __VA_ARGS__)
 
+// A workspace's status word by synchronisation and copy: allocates nothing (sessd_read_status: pinned memory for a thread's first call).
+int copy_status(const void* workspace, cudaStream_t stream);
+
 // Number of SMs of the current device (cached per device).
 int sm_count();
 // Grid for a persistent grid-stride kernel: `per_sm` blocks on every SM.

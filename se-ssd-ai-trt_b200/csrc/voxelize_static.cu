@@ -69,5 +69,5 @@ extern "C" int sessd_voxelize_static_status(void* stream) {
         scratch = g_scratch_addr[dev];
     }
     if (!scratch) return SESSD_ERR_PARAM;
-    return sessd_read_status(scratch, stream);
+    return sessd::copy_status(scratch, static_cast<cudaStream_t>(stream));
 }

@@ -84,3 +84,24 @@ def test_static_scratch_reports_lost_voxels_through_its_status_reader(gpu):
     assert st >= 0 and st & gpu.STATUS_VOXEL_OVERFLOW
     rc, voxels, coors, num = _call_static(gpu, gpu.voxel_params(20000), pts, sizes)
     assert rc == 0 and gpu.lib().sessd_voxelize_static_status(None) == 0
+
+
+def test_static_status_allocates_no_host_memory(gpu):
+    """The first status of a thread that uses nothing but the static entry point: no call that allocates."""
+    import threading
+
+    import torch
+
+    params = gpu.voxel_params(2000)
+    pts = torch.from_numpy(gpu.synth.lidar_frame(3, n_points=1000, n_boxes=3)[None]).cuda()
+    sizes = torch.tensor([1000], dtype=torch.int32, device="cuda")
+    assert _call_static(gpu, params, pts, sizes)[0] == 0
+    stream, got = C.c_void_p(torch.cuda.current_stream().cuda_stream), []
+    worker = threading.Thread(target=lambda: got.append(gpu.lib().sessd_voxelize_static_status(stream)))
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA]) as prof:
+        worker.start()
+        worker.join()
+        torch.cuda.synchronize()
+    names = {e.key for e in prof.key_averages()}
+    assert got == [0] and "cudaStreamSynchronize" in names
+    assert not [n for n in names if "Alloc" in n or "Malloc" in n], names
