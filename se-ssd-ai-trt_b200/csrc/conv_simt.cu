@@ -2,7 +2,7 @@
 //
 // Replaces the reference's per-offset gather / multiply / atomicAdd kernel, launched kvol times per
 // layer with one thread per rulebook pair and Cout global atomics per pair
-// (submConv3dlayer.cu:479-518, :632-638). Here one launch covers the layer: a thread owns four
+// (submConv3dlayer.cu:479-518, :632-638). Here one launch covers the layer: a thread owns two, four or eight
 // output channels of one output row, walks the row's present neighbours, and for each of them
 // accumulates s = sum_ci in[ci]*W[k][ci][co] as one fused-multiply-add chain (ci ascending),
 // then acc += s with k ascending. That is the arithmetic of the reference kernel with the order of
@@ -363,10 +363,14 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
 template <typename T>
 int dispatch(const ConvLaunch& c, cudaStream_t stream) {
     // Room for a million rows is what a few frames have. Those are latency: a thread with half the channels is through its
-    // row's neighbours sooner, and twice as many blocks share out the rows with the longest lists (4 -> 16: one frame of
-    // 20,000 points 258 -> 253 us, four of 120,000 1057 -> 1054; fp32 16 -> 16 and 16 -> 32: 1008 -> 1000 us). Larger batches
-    // are throughput: with twice the channels half as many threads walk a list (32 frames of 120,000 points: 290 us for
-    // 4 -> 16, 338 with four channels).
+    // row's neighbours sooner, and twice as many blocks share out the rows with the longest lists. Larger batches are
+    // throughput: with twice the channels half as many threads walk a list. The line is a capacity, because row counts are on the
+    // device. Half the channels and all of them, in us: fp16 front end (4 -> 16) 1 x 20,000 points 254 and 258, 4 x 120,000
+    // (800,000 rows) 1047 and 1055, 16 x 20,000 (960,000) 1208 and 1208, 32 x 20,000 2199 and 2190, 32 x 120,000 6920 and 6896; fp32
+    // front end (all three) 1 x 20,000 992 and 1000, 4 x 120,000 9407 and 9408, 8 x 120,000 18097 and 18062. Single calls: 4 -> 16
+    // 8 x 20,000 103 and 106, 16 x 20,000 152 and 149; fp32 16 -> 16 half is better at every size (16 x 120,000: 1189 and
+    // 1227); a submanifold fp32 16 -> 32, which the network has none of, would cross between 4 and 8 x 20,000 (4 x 120,000: 523
+    // and 460).
     const bool few = (int64_t)c.batch * c.max_voxels <= 1000000;
     if (c.cin == 4 && c.cout == 16) return few ? launch_narrow<T, 4, 16, 4>(c, stream) : launch_narrow<T, 4, 16, 8>(c, stream);
     if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these

@@ -366,7 +366,7 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
         const int first = (it - before - __shfl_sync(0xFFFFFFFFu, incl - (my_rows + kWindow - 1) / kWindow, src_lane)) * kWindow;
         return Window{ji, pair0 + src_lane - ji * batch, first, min(__shfl_sync(0xFFFFFFFFu, my_rows, src_lane) - first, kWindow)};
     };
-    // The coordinates of a window's rows are requested a window ahead: two blocks per SM do not hide that latency.
+    // The coordinates of a window's rows are requested a window ahead: one block per SM does not hide that latency.
     int4 coor[2];
     auto fetch = [&](const Window& w) {
         const int4* c = reinterpret_cast<const int4*>(jobs.job[w.job].out_coors) + (size_t)w.frame * max_voxels + w.first;
@@ -535,7 +535,7 @@ MapJob make_map_job(const ConvGeom& g, const int32_t* out_coors, const int32_t* 
 
 int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const RowMeans& means, cudaStream_t stream) {
     if (jobs.count == 0 && !means.points) return SESSD_OK;
-    static_assert(2 * (sizeof(MapShared) + 1024) <= 228 * 1024, "two windows per SM");
+    static_assert(sizeof(MapShared) <= 227 * 1024, "a window does not fit the shared memory of one SM");
     // the attribute belongs to the device's context: set it once per device (repeating it is harmless)
     static std::atomic<uint64_t> configured{0};
     int dev = 0;

@@ -10,18 +10,18 @@
 // 128-row tile side by side), so that the tensor-core kernel fetches a tile's offsets with one copy.
 //
 // Where the rows of a frame come from decides how a coordinate is turned back into its row:
-//   - the voxeliser's rows (full resolution, 92 M cells, 80 K of them active) sit in an x-grouped
-//     open-addressing table (32-byte buckets of four x-neighbours);
-//   - the rows a strided layer produces are numbered through an occupancy grid of the output level: one
-//     bit per cell, 64 x-neighbours per word, each word followed by the number of rows before it. Every
-//     candidate output of every input row sets its bit (sparseConv3dlayer.cu:310-386 with the truncating
-//     divisions kept); a count and a scan/emit pass then number the set bits in (z, y, x) order and write
-//     the output coordinates. A cell's row is prefix + popcount(bits below), one 16-byte read, and the
-//     three x-neighbours of a 3x3x3 kernel share that read. The grids are small (3 MB per frame at half
-//     resolution, 0.4 MB at quarter resolution) and stay in L2. The reference numbers outputs in the
-//     arrival order of an atomic over a dense scan (sparseConv3dlayer.cu:529-541); (z, y, x) order is
-//     deterministic and keeps the rows of a 128-row tile close together in space;
-//   - coordinates handed in by a caller (the stand-alone plugin entry points) go into a flat table.
+//   - the front end's own rows are numbered through an occupancy grid of their level, 64 x-neighbouring cells to a word, each
+//     word followed by the number of rows before it: a cell's row is prefix + popcount(bits below), one 16-byte read that the
+//     three x-neighbours of a 3x3x3 kernel share. The voxeliser's level (92 M cells, 80 K of them active) has a grid of two levels
+//     (voxel_grid.cu), the derived ones (3 MB per frame at half resolution, 0.4 MB at quarter) one. A strided layer's
+//     candidate outputs (sparseConv3dlayer.cu:310-386, truncating divisions kept) are set as bits; a one-pass scan (scan.cuh)
+//     numbers them in (z, y, x) order and writes the output coordinates. The reference numbers outputs in the arrival
+//     order of an atomic over a dense scan (sparseConv3dlayer.cu:529-541); (z, y, x) order is deterministic and keeps the
+//     rows of a 128-row tile close together in space;
+//   - rows in an order of their own (a caller's, or the voxeliser's where rows may have to be dropped) sit in an x-grouped
+//     open-addressing table (32-byte buckets of four x-neighbours). Strided calls on fine grids go without: their input rows
+//     look up their outputs in the numbered grid (scatter_rows_kernel);
+//   - submanifold kernels other than 3x3x3 use a flat table.
 #include "fill.cuh"
 #include "rulebook.cuh"
 #include "scan.cuh"

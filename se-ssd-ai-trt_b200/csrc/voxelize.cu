@@ -158,8 +158,9 @@ cudaError_t launch_publish_status(const int32_t* status, const int32_t* other, u
 // memory and a small L1; an SM changes that only when it is empty, and with overlapping launches throughout it never
 // is: the table kernels that follow would run on the small L1 (32 frames x 120,000 points: insert 196 -> 453 us, emit
 // 509 -> 737, neighbour map 551 -> 958). So there this launch waits for its predecessor to leave the SMs. It overlaps
-// where that costs more than it gives: after calls that end otherwise, and with tables so small that L1 hardly matters
-// (one 20,000-point frame: 377 us overlapping, 381 not; one 120,000-point frame: 588 and 566).
+// where that costs more than it gives: after calls that end otherwise, and for front ends of so few points that L1 hardly matters
+// (overlapping and not: 20,000 points 251 and 255 us, two such frames 340 and 343, three 398 and 398, four 459 and 458, eight 727 and
+// 712; one frame of 60,000 points 345 and 347, of 120,000 431 and 429: the line at 40,000 points could lie at 60,000 as well).
 int launch_prepare(const FillRanges& f, const TailRows& t, bool overlap, cudaStream_t stream) {
     SESSD_LAUNCH_IMPL(overlap, "prepare_kernel", prepare_kernel, persistent_grid(8), kThreads, 0, stream, f, t);
     return SESSD_OK;

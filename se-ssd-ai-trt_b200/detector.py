@@ -228,7 +228,7 @@ class Detector:
     def capture(self, max_points, batch=1):
         """Records the whole chain for `batch` frames of up to `max_points` points into one CUDA graph (every
         enqueue call of the library is capturable: no allocation, no synchronisation, all counts read on the
-        device). Afterwards replay(points, sizes) costs one graph launch instead of some sixty kernel launches."""
+        device). Afterwards replay(points, sizes) costs one graph launch instead of some fifty kernel launches."""
         import torch
 
         from . import filter_boxes, rotated_nms
