@@ -411,3 +411,26 @@ def test_status_of_another_device(gpu):
         assert gpu.lib().sessd_read_status(ws.data_ptr(), torch.cuda.current_stream(1).cuda_stream) == 4
         stream = torch.cuda.Stream(1)
         assert gpu.lib().sessd_read_status(ws.data_ptr(), stream.cuda_stream) == 4
+
+
+def test_repeated_passes_give_the_same_bits(gpu):
+    """150 passes over the same four 120,000-point frames, every layer's rows bit for bit."""
+    import torch
+
+    w, sc, sh = gpu.random_weights()
+    bb = gpu.Backbone(200000, w, sc, sh, dtype=1)
+    pts = torch.stack([torch.from_numpy(gpu.synth.sweep_frame(i)) for i in range(4)]).cuda()
+    sizes = torch.full((4,), pts.shape[1], dtype=torch.int32, device="cuda")
+    dense, ws = bb.run(pts, sizes)
+    views = [bb.layer_view(ws, 4, pts.shape[1], i) for i in range(-1, len(bb.layers))]
+    rows = [n.tolist() for _, _, n in views]
+    want = [[f[b, :n[b]].clone() for b in range(4)] for (f, _, _), n in zip(views, rows)]
+    first = dense.clone()
+    for _ in range(150):
+        bb.run(pts, sizes, ws, dense)
+        assert torch.equal(dense, first)
+        for (f, _, num), n, layer in zip(views, rows, want):
+            assert num.tolist() == n
+            assert all(torch.equal(f[b, :n[b]], layer[b]) for b in range(4))
+    assert gpu.read_status(ws) == 0
+    bb.close()
