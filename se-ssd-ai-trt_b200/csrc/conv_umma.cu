@@ -64,7 +64,6 @@ constexpr int KVOL_MAX = 27;
 // with two 196 tiles would take 49.5 instead of 47.0, 207 of 64 -> 64 50.0 instead of 47.7: the second tile waits for the first.
 // Front end of 5,000 points without the path, with one, with two: 239, 195, 195 us; 20,000 points 269, 251, 257.
 constexpr int FEW_TILES = 1;
-constexpr int FEW_B_FULL = 2;                // where that path keeps its weight barriers among i_full
 constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // Words from one offset's 128 indices to the next offset's inside an index block: 16 bytes more than the indices
 // take, so that lanes reading different offsets of a stage (32- and 16-channel inputs) use different banks too.
@@ -360,7 +359,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                                          const uint8_t* __restrict__ wtiles, const EpiConst& epi, int relu, int batch,
                                          int max_voxels, int kvol, __half* __restrict__ dense,
                                          const int4* __restrict__ out_coors, int D, int H, int W, int* tile_counter,
-                                         bool wait_first, int withhold_weights) {   // returns the weight blocks asked for
+                                         bool wait_first, int withhold_weights) {   // returns a gather warp's uses of its slot
     constexpr int KG = 64 / CIN, CPO = CIN / 8, B_BYTES = COUT * ROW_BYTES;
     constexpr uint32_t IDESC = umma_idesc(COUT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -368,12 +367,11 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     volatile int* abort_flag = &ctl->abort_flag;
     uint8_t* sB = sA + FEW_SLOTS * A_BYTES;
     // barriers and words of the other path with the same arrival counts
-    unsigned long long *a_full = ctl->a_full[0], *empty = ctl->a_empty, *idx_full = &ctl->i_full[0], *acc_full = &ctl->i_full[1],
-                       *b_full = ctl->i_full + FEW_B_FULL;
+    unsigned long long *full = ctl->a_full[0], *empty = ctl->a_empty, *idx_full = &ctl->i_full[0], *acc_full = &ctl->i_full[1];
     volatile uint32_t* hand = ctl->scan_warp;   // the tile in hand: frame (-1: none left), first row, the frame's rows, mask
     uint32_t items = 0;                        // items of the tiles so far
     uint32_t sums = 0;                         // tiles so far that had any: acc_full completes a phase for those alone
-    uint32_t b_issued = 0;
+    uint32_t uses = 0;                         // gather warps: times that the slot has been filled
     bool waited = wait_first;                  // the preceding kernel's writes may be read
     for (uint32_t round = 0;; ++round) {
         if (warp == 0) {
@@ -439,19 +437,27 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                                  : "r"(idx_base + 128 * (w4 >> 1) + 16 * (w4 & 1)));
                     vv[4 * w4] = v.x, vv[4 * w4 + 1] = v.y, vv[4 * w4 + 2] = v.z, vv[4 * w4 + 3] = v.w;
                 }
+                ok = mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 2 | (int)(q << 4));
+                if (!ok) break;
+                if (lane == 0) {               // (this lane's arrival for the phase comes with its copies below)
+                    mbar_expect_tx(smem_u32(full + s), B_BYTES);
+                    if (!withhold_weights) {
+                        bulk_load(smem_u32(sB + s * B_BYTES), wtiles + (size_t)g * B_BYTES, B_BYTES, smem_u32(full + s));
+                        ++uses;
+                    }
+                }
+                __syncwarp();
                 if (!waited) {
                     pdl_enter();
                     waited = true;
                 }
-                ok = mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 2 | (int)(q << 4));
-                if (!ok) break;
 #pragma unroll
                 for (int p = 0; p < 32; ++p) {
                     const int id = (k_ok && 32 * (p >> 3) + (p & 7) < rows_left) ? vv[p] : -1;
                     cp_async_16(a_base + (32 * (p >> 3) + (p & 7)) * ROW_BYTES + ((c ^ (p & 7)) << 4),
                                 lane_base + (size_t)(id < 0 ? 0 : id) * CIN, id < 0 ? 0u : 16u);
                 }
-                cp_async_arrive_noinc(smem_u32(a_full + s));
+                cp_async_arrive_noinc(smem_u32(full + s));
             }
         } else if (warp < EPI_WARPS) {
             const int pos = row0 + tid;
@@ -471,24 +477,30 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                                  max_voxels, out, dense, out_coors, D, H, W);
             tc_fence_before();
         } else if (warp == EPI_WARPS) {
-            // issuer
-            bool ok = true;
-            for (int e = 0; e < n_items && ok; ++e) {
-                const uint32_t q = items + (uint32_t)e, s = q % FEW_SLOTS, phase = (q / FEW_SLOTS) & 1u;
-                ok = mbar_wait<false, true>(smem_u32(b_full + s), phase, abort_flag, 5 | (int)(q << 4)) &&
-                     mbar_wait<false, true>(smem_u32(a_full + s), phase, abort_flag, 6 | (int)(q << 4));
-                if (ok && leader) {
+            // Issuer: what bounds the chain of a tile's items, whose rows and weights are there long before. One thread, so that
+            // nothing holds the lanes together, one barrier per slot for both operands (each wait is some 80 cycles), and the next
+            // item's looked at before this item's instructions go out. (As a warp, with a barrier for each operand, an item took
+            // some 500 cycles: front end of a 20,000-point frame 250.1 us, now 240.2.)
+            if (leader) {
+                bool ok = true, ready = false;
+                uint32_t s = items % FEW_SLOTS, phase = (items / FEW_SLOTS) & 1u;
+                for (int e = 0; e < n_items; ++e) {
+                    if (!ready) ok = mbar_wait<false, true>(smem_u32(full + s), phase, abort_flag, 5 | (int)((items + e) << 4));
+                    if (!ok) break;
                     fence_proxy_async();       // the gathered rows were written through the generic proxy
                     tc_fence_after();
-                    const uint64_t adesc = umma_desc(smem_u32(sA + s * A_BYTES));
-                    const uint64_t bdesc = umma_desc(smem_u32(sB + s * B_BYTES));
+                    const uint32_t at = s;
+                    if (++s == FEW_SLOTS) s = 0, phase ^= 1u;
+                    ready = mbar_test(smem_u32(full + s), phase);
+                    const uint64_t adesc = umma_desc(smem_u32(sA + at * A_BYTES));
+                    const uint64_t bdesc = umma_desc(smem_u32(sB + at * B_BYTES));
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
                         umma_f16(tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (e > 0 || kk > 0) ? 1u : 0u);
-                    umma_commit(smem_u32(empty + s));
+                    umma_commit(smem_u32(empty + at));
                 }
+                if (ok && n_items) umma_commit(smem_u32(acc_full));
             }
-            if (ok && leader && n_items) umma_commit(smem_u32(acc_full));
             __syncwarp();
         } else if (warp == INDEX_WARP) {
             if (lane == 0) {
@@ -498,19 +510,6 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 ctl->idx_uses[0] = round + 1u;
             }
             __syncwarp();
-        } else if (warp == WEIGHT_WARP) {
-            if (lane == 0 && !withhold_weights) {
-                uint32_t q = items;
-                for (uint32_t left = stages; left; left &= left - 1u, ++q) {
-                    const uint32_t s = q % FEW_SLOTS;
-                    if (!mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 8 | (int)(q << 4))) break;
-                    const uint32_t bar = smem_u32(b_full + s);
-                    mbar_arrive_expect_tx(bar, B_BYTES);
-                    bulk_load(smem_u32(sB + s * B_BYTES), wtiles + (size_t)((__ffs((int)left) - 1) / KG) * B_BYTES, B_BYTES, bar);
-                    b_issued = q + 1u;
-                }
-            }
-            __syncwarp();
         }
         items += (uint32_t)n_items;
         sums += n_items ? 1u : 0u;
@@ -518,7 +517,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
         tc_fence_after();
     }
     if (!waited) pdl_enter();                  // every CTA waits: the next kernel counts on what came before this one
-    return b_issued;
+    return uses;
 }
 
 template <int CIN, int COUT>
@@ -600,6 +599,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     uint32_t a_it = 0, b_it = 0, acc_it = 0;  // items, weight blocks and accumulator sets used so far; every role advances them identically
     uint32_t full_phase = 0;                  // MMA issuers: bit s = parity of the next phase of their a_full[t][s]
     uint32_t b_issued = 0;                    // weight streamer: blocks whose bulk copy has been started
+    uint32_t few_uses = 0;                    // few-tiles path, gather warps (lane 0): weight blocks asked for
     uint32_t zero_rows = 0;                   // gather warps: bit p = this lane's chunk of row p of its slot holds zeros
 
     // Balanced split: the occupied 128-row tiles of all frames, laid end to end, are cut into gridDim.x
@@ -651,7 +651,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) <= NSLOT * A_BYTES + B_STAGES * B_BYTES &&
                           KVOL_MAX * TAP_WORDS + 3 * TAP_WORDS <= NIDX * IDX_WORDS,
                       "the few-tiles path lives in the other path's buffers");
-        b_issued = umma_few<CIN, COUT>(ctl, sA, s_idx, s_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
+        few_uses = umma_few<CIN, COUT>(ctl, sA, s_idx, s_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
                             batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, !maps_ready, withhold_weights);
     }
     if (!few) {
@@ -1058,15 +1058,14 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 while (!mbar_try_wait(bar, (uses - 1u) & 1u) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
             }
         }
-        if (warp == WEIGHT_WARP && lane == 0) {
-            const uint32_t ring = few ? FEW_SLOTS : B_STAGES;
-            const uint32_t first = b_issued > ring ? b_issued - ring : 0u;
-            for (uint32_t j = first; j < b_issued; ++j) {
-                const uint32_t bar = smem_u32(few ? &ctl->i_full[FEW_B_FULL + j % ring] : &ctl->b_full[j % ring]);
-                const long long t0 = clock64();
-                while (!mbar_try_wait(bar, (j / ring) & 1u) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
-            }
-        }
+        auto settle = [&](const unsigned long long* bar, uint32_t parity) {
+            const long long t0 = clock64();
+            while (!mbar_try_wait(smem_u32(bar), parity) && clock64() - t0 < WAIT_LIMIT_CYCLES) {}
+        };
+        if (warp == WEIGHT_WARP && lane == 0)
+            for (uint32_t j = b_issued > B_STAGES ? b_issued - B_STAGES : 0u; j < b_issued; ++j)
+                settle(&ctl->b_full[j % B_STAGES], (j / B_STAGES) & 1u);
+        if (few_uses) settle(&ctl->a_full[0][warp - FIRST_GATHER_WARP], (few_uses - 1u) & 1u);
     }
     __syncthreads();
     if (tid == 0 && *abort_flag) {
