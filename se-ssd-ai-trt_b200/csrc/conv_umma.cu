@@ -54,17 +54,20 @@ constexpr int MMA_WARPS = TILES;             // warps 4-7: issuer t owns tile t
 constexpr int WEIGHT_WARP = EPI_WARPS + MMA_WARPS;
 constexpr int INDEX_WARP = WEIGHT_WARP + 1;
 constexpr int FIRST_GATHER_WARP = INDEX_WARP + 1;
-constexpr int NSLOT_MAX = 12;
-constexpr int NIDX_MAX = 36;
+constexpr int NSLOT_MAX = 10;
+constexpr int NIDX_MAX = 30;
 constexpr int B_STAGES = 3;                  // weight ring: a group needs up to 27 blocks, each an L2 round trip away
 constexpr int ROW_BYTES = 128;               // 64 halves per A/B row
 constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
-// Few-tiles path: up to this many tiles per CTA. With one a layer of 141 tiles on 148 SMs takes 39.4 us as a call (41.5 without the path),
-// with two 196 tiles would take 49.5 instead of 47.0, 207 of 64 -> 64 50.0 instead of 47.7: the second tile waits for the first.
-// Front end of 5,000 points without the path, with one, with two: 239, 195, 195 us; 20,000 points 269, 251, 257.
-constexpr int FEW_TILES = 1;
+// Few-tiles path: up to this many tiles per CTA. It fetches a weight block per item instead of one for up to four tiles, but is
+// through sooner and shares the tiles out by a counter. In us, without the path / with one tile per CTA, three, six, ten, any number:
+// front end of 1 x 20,000 points 250 (239 at one), 227 from three on; 3 x 20,000 389, 385, 369, 365, 365; 5 x 77,000 721, 725, 705, 708,
+// 714; 3 x 120,000 824, -, 805, 805, 840; 8 x 120,000 1858, -, 1857, 1856, 1933. Calls of 64 -> 64 channels: 8 tiles per CTA 87.2 and
+// with the path 84.5, 16 tiles 151.0 and 154.4.
+constexpr int FEW_TILES = 10;
 constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
+constexpr int FEW_IDX = 28;                  // offsets of a tile's index block there (27, and those of the last stage past them)
 // Words from one offset's 128 indices to the next offset's inside an index block: 16 bytes more than the indices
 // take, so that lanes reading different offsets of a stage (32- and 16-channel inputs) use different banks too.
 constexpr int TAP_WORDS = kNbrRun;
@@ -184,6 +187,8 @@ struct SharedCtl {
     // steps straight to the items it owns
     uint8_t stage_list[NSLOT_MAX][TILES * 32];
     uint8_t idx_list[TILES * 32];            // the same list for the index warp
+    unsigned long long tile_free[2];         // few-tiles path: every role is through with the tile's indices and its entry below
+    int tile[2][4];                          // few-tiles path: frame (-1: none left), first row, the frame's rows, mask
     uint32_t scan_warp[32];                  // work split: per-warp totals of the block scan
     int range_lo, range_hi;                  // work split: this CTA's tiles
     uint32_t idx_uses[NIDX_MAX];             // bulk copies issued into index block j so far (for the abort path)
@@ -343,14 +348,15 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
 }
 
 // ---- few tiles ----
-// With no more than FEW_TILES tiles per CTA the pipeline above is all latency: one tile's offsets are a serial chain, its
-// weight blocks are used once, so that three of them in flight bound it (390 ns per item on a single 20,000-point frame),
-// and everything before the first gather (5.8 us: work split, masks, index copy) comes on top of every launch. This path
-// takes one tile at a time, with seven A slots and as many weight blocks in flight, all of the tile's indices in one
-// copy, and does what does not depend on the preceding kernel before it waits for that kernel: barriers, tensor memory,
-// tile, indices and the first weight blocks. Tiles are handed out by a counter: a CTA that starts late, because the
-// preceding kernel still held its SM, leaves the tiles to the others. A tile's offsets are added up in the same order as
-// in the other path, so the results are the same bits.
+// With few tiles per CTA the pipeline below is latency in good part: a group of one or two tiles uses a weight block once or
+// twice, so that three of them in flight bound it (390 ns per item on a single 20,000-point frame), everything before
+// the first gather (5.8 us: work split, masks, index copy) comes on top of every launch, and whole groups divide badly. This path takes one tile at a time,
+// with seven slots in flight that hold a stage's rows and its weight block, and all of a tile's indices in one copy. What does not
+// depend on the preceding kernel comes before the wait for that kernel: barriers, tensor memory, tile, indices and the
+// first weight blocks. Tiles are handed out by a counter, one ahead of the tile in work (two index blocks, two accumulators: the
+// next tile's gathers run while this one is stored): a CTA that starts late, because the preceding kernel still held its
+// SM, leaves the tiles to the others. A tile's offsets are added up in the same order as in the other path, so the results are
+// the same bits.
 template <int CIN, int COUT>
 __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_t* s_idx, uint8_t* s_stage, uint32_t tmem,
                                          bool leader, const __half* __restrict__ in, __half* __restrict__ out,
@@ -359,22 +365,161 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                                          const uint8_t* __restrict__ wtiles, const EpiConst& epi, int relu, int batch,
                                          int max_voxels, int kvol, __half* __restrict__ dense,
                                          const int4* __restrict__ out_coors, int D, int H, int W, int* tile_counter,
-                                         bool wait_first, int withhold_weights) {   // returns a gather warp's uses of its slot
+                                         bool ahead, bool wait_first, int withhold_weights) {   // returns a gather warp's uses of its slot
     constexpr int KG = 64 / CIN, CPO = CIN / 8, B_BYTES = COUT * ROW_BYTES;
     constexpr uint32_t IDESC = umma_idesc(COUT);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int tiles_per_frame = (max_voxels + TILE_M - 1) / TILE_M;
     volatile int* abort_flag = &ctl->abort_flag;
     uint8_t* sB = sA + FEW_SLOTS * A_BYTES;
-    // barriers and words of the other path with the same arrival counts
-    unsigned long long *full = ctl->a_full[0], *empty = ctl->a_empty, *idx_full = &ctl->i_full[0], *acc_full = &ctl->i_full[1];
-    volatile uint32_t* hand = ctl->scan_warp;   // the tile in hand: frame (-1: none left), first row, the frame's rows, mask
+    // barriers of the other path with the same arrival counts
+    unsigned long long *full = ctl->a_full[0], *empty = ctl->a_empty, *tile_full = ctl->i_full, *tile_free = ctl->tile_free,
+                       *acc_full = ctl->i_full + 2, *acc_empty = ctl->acc_empty;
+    volatile int(*tile)[4] = ctl->tile;
     uint32_t items = 0;                        // items of the tiles so far
-    uint32_t sums = 0;                         // tiles so far that had any: acc_full completes a phase for those alone
+    uint32_t sums = 0;                         // tiles so far that had any: accumulator sets are used for those alone
     uint32_t uses = 0;                         // gather warps: times that the slot has been filled
     bool waited = wait_first;                  // the preceding kernel's writes may be read
-    for (uint32_t round = 0;; ++round) {
-        if (warp == 0) {
+    // Every role goes through the CTA's tiles in the same order; entry and index block `round & 1`.
+    if (warp >= FIRST_GATHER_WARP && warp < FIRST_GATHER_WARP + FEW_SLOTS) {
+        // gather, as in the other path; slot s belongs to this warp
+        const int s = warp - FIRST_GATHER_WARP;
+        const int c = lane & 7, jrow = (lane >> 3) * 8, koff = c / CPO;
+        const uint32_t a_base = smem_u32(sA + s * A_BYTES) + jrow * ROW_BYTES;
+        bool ok = true;
+        for (uint32_t round = 0; ok; ++round) {
+            const uint32_t r = round & 1u;
+            ok = mbar_wait(smem_u32(tile_full + r), (round >> 1) & 1u, abort_flag, 1 | (int)(items << 4));
+            if (!ok) break;
+            const int b = tile[r][0], row0 = tile[r][1], n = tile[r][2];
+            if (b < 0) break;
+            const uint32_t stages = stage_bits<KG>((uint32_t)tile[r][3]);   // bit g * KG for stage g
+            const __half* lane_base = in + (size_t)b * max_voxels * CIN + (c % CPO) * 8;
+            const int rows_left = n - (row0 + jrow);
+            // this warp's items: every FEW_SLOTS-th stage of the tile
+            int e = (s + FEW_SLOTS - (int)(items % FEW_SLOTS)) % FEW_SLOTS;
+            uint32_t left = stages;
+            for (int i = 0; i < e; ++i) left &= left - 1u;
+            for (; left; e += FEW_SLOTS) {
+                const uint32_t q = items + (uint32_t)e;
+                const int g = (__ffs((int)left) - 1) / KG;
+#pragma unroll
+                for (int i = 0; i < FEW_SLOTS; ++i) left &= left - 1u;
+                const uint32_t idx_base = smem_u32(s_idx + r * (FEW_IDX * TAP_WORDS) + (g * KG + koff) * TAP_WORDS + jrow);
+                const bool k_ok = g * KG + koff < kvol;
+                int vv[32];
+#pragma unroll
+                for (int w4 = 0; w4 < 8; ++w4) {
+                    int4 v;
+                    asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];"
+                                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                                 : "r"(idx_base + 128 * (w4 >> 1) + 16 * (w4 & 1)));
+                    vv[4 * w4] = v.x, vv[4 * w4 + 1] = v.y, vv[4 * w4 + 2] = v.z, vv[4 * w4 + 3] = v.w;
+                }
+                ok = mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 2 | (int)(q << 4));
+                if (!ok) break;
+                if (lane == 0) {               // (this lane's arrival for the phase comes with its copies below)
+                    mbar_expect_tx(smem_u32(full + s), B_BYTES);
+                    if (!withhold_weights) {
+                        bulk_load(smem_u32(sB + s * B_BYTES), wtiles + (size_t)g * B_BYTES, B_BYTES, smem_u32(full + s));
+                        ++uses;
+                    }
+                }
+                if (!waited) {
+                    pdl_enter();
+                    waited = true;
+                }
+#pragma unroll
+                for (int p = 0; p < 32; ++p) {
+                    const int id = (k_ok && 32 * (p >> 3) + (p & 7) < rows_left) ? vv[p] : -1;
+                    cp_async_16(a_base + (32 * (p >> 3) + (p & 7)) * ROW_BYTES + ((c ^ (p & 7)) << 4),
+                                lane_base + (size_t)(id < 0 ? 0 : id) * CIN, id < 0 ? 0u : 16u);
+                }
+                cp_async_arrive_noinc(smem_u32(full + s));
+            }
+            items += (uint32_t)__popc(stages);
+            mbar_arrive(smem_u32(tile_free + r));   // (behind the copies, which have consumed the indices)
+        }
+    } else if (warp < EPI_WARPS) {
+        for (uint32_t round = 0;; ++round) {
+            const uint32_t r = round & 1u;
+            bool ok = mbar_wait(smem_u32(tile_full + r), (round >> 1) & 1u, abort_flag, 3 | (int)(round << 4));
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (!ok) break;
+            const int b = tile[r][0], row0 = tile[r][1], n = tile[r][2];
+            const bool have = tile[r][3] != 0;
+            if (b < 0) break;
+            const int pos = row0 + tid;
+            const int row = order && pos < n ? __ldg(order + (size_t)b * max_voxels + pos) : pos;
+            mbar_arrive(smem_u32(tile_free + r));
+            if (!waited) {                     // (out is another kernel's input until then)
+                pdl_enter();
+                waited = true;
+            }
+            const uint32_t set = sums & 1u;
+            if (have) {
+                ok = mbar_wait(smem_u32(acc_full + set), (sums >> 1) & 1u, abort_flag, 3 | (int)(round << 4));
+                ok = __all_sync(0xFFFFFFFFu, ok);
+                if (!ok) break;
+                tc_fence_after();
+            }
+            store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + set * COUT, have, epi, relu, s_stage, warp, lane, pos, row, n, b,
+                             max_voxels, out, dense, out_coors, D, H, W);
+            if (have) {
+                tc_fence_before();
+                mbar_arrive(smem_u32(acc_empty + set));
+                ++sums;
+            }
+        }
+    } else if (warp == EPI_WARPS) {
+        // Issuer: what bounds the chain of a tile's items, whose rows and weights are there long before. One thread, so that
+        // nothing holds the lanes together, one barrier per slot for both operands (each wait is some 80 cycles), and the next
+        // item's looked at before this item's instructions go out. (As a warp, with a barrier for each operand, an item took
+        // some 500 cycles: front end of a 20,000-point frame 250.1 us, then 240.2.)
+        if (leader) {
+            bool ok = true;
+            uint32_t s = 0, phase = 0;
+            for (uint32_t round = 0; ok; ++round) {
+                const uint32_t r = round & 1u;
+                ok = mbar_wait<false, true>(smem_u32(tile_full + r), (round >> 1) & 1u, abort_flag, 4 | (int)(round << 4));
+                if (!ok || tile[r][0] < 0) break;
+                const int n_items = __popc(stage_bits<KG>((uint32_t)tile[r][3]));
+                mbar_arrive(smem_u32(tile_free + r));
+                if (!n_items) continue;
+                const uint32_t set = sums & 1u, d_tmem = tmem + set * COUT;
+                // the epilogue must have read this set's previous contents (two tiles back)
+                ok = mbar_wait<false, true>(smem_u32(acc_empty + set), ((sums >> 1) & 1u) ^ 1u, abort_flag, 4 | (int)(round << 4));
+                bool ready = false;
+                for (int e = 0; e < n_items && ok; ++e) {
+                    if (!ready) ok = mbar_wait<false, true>(smem_u32(full + s), phase, abort_flag, 5 | (int)((items + e) << 4));
+                    if (!ok) break;
+                    fence_proxy_async();       // the gathered rows were written through the generic proxy
+                    tc_fence_after();
+                    const uint32_t at = s;
+                    if (++s == FEW_SLOTS) s = 0, phase ^= 1u;
+                    ready = mbar_test(smem_u32(full + s), phase);
+                    const uint64_t adesc = umma_desc(smem_u32(sA + at * A_BYTES));
+                    const uint64_t bdesc = umma_desc(smem_u32(sB + at * B_BYTES));
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_f16(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (e > 0 || kk > 0) ? 1u : 0u);
+                    umma_commit(smem_u32(empty + at));
+                }
+                if (ok) umma_commit(smem_u32(acc_full + set));
+                items += (uint32_t)n_items;
+                ++sums;
+            }
+        }
+        __syncwarp();
+    } else if (warp == INDEX_WARP) {
+        // the CTA's tiles and their indices. ahead: the next tile is taken while the last one is in work; where there is no more
+        // than a tile per CTA, those that start first would take two.
+        for (uint32_t round = 0;; ++round) {
+            const uint32_t r = round & 1u;
+            if (!ahead && round > 0) {
+                const bool ok = mbar_wait(smem_u32(tile_free + (r ^ 1u)), ((round - 1u) >> 1) & 1u, abort_flag, 7 | (int)(round << 4));
+                if (!__all_sync(0xFFFFFFFFu, ok)) break;
+            }
             int t = 0;
             if (lane == 0) t = atomicAdd(tile_counter, 1);
             t = __shfl_sync(0xFFFFFFFFu, t, 0);
@@ -398,123 +543,23 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 }
                 t -= __shfl_sync(0xFFFFFFFFu, incl, 31);
             }
+            const int mask = frame < 0 ? 0 : (int)__ldg(tile_mask + (size_t)frame * tiles_per_frame + first / TILE_M);
+            bool ok = mbar_wait(smem_u32(tile_free + r), ((round >> 1) & 1u) ^ 1u, abort_flag, 7 | (int)(round << 4));
+            ok = __all_sync(0xFFFFFFFFu, ok);
+            if (!ok) break;
             if (lane == 0) {
-                hand[0] = (uint32_t)frame, hand[1] = (uint32_t)first, hand[2] = (uint32_t)rows;
-                hand[3] = frame < 0 ? 0u : __ldg(tile_mask + (size_t)frame * tiles_per_frame + first / TILE_M);
+                tile[r][0] = frame, tile[r][1] = first, tile[r][2] = rows, tile[r][3] = mask;
+                ctl->idx_uses[r] = (round >> 1) + 1u;
+                if (frame < 0) {
+                    mbar_arrive(smem_u32(tile_full + r));
+                } else {
+                    mbar_arrive_expect_tx(smem_u32(tile_full + r), (uint32_t)(kvol * TAP_WORDS * 4));
+                    bulk_load(smem_u32(s_idx + r * (FEW_IDX * TAP_WORDS)), nbr + nbr_index(kvol, max_voxels, frame, 0, first),
+                              (uint32_t)(kvol * TAP_WORDS * 4), smem_u32(tile_full + r));
+                }
             }
+            if (frame < 0) break;
         }
-        __syncthreads();
-        const int b = (int)hand[0], row0 = (int)hand[1], n = (int)hand[2];
-        const uint32_t mask = hand[3];
-        if (b < 0 || *abort_flag) break;       // (the flag is only ever raised before the barrier below)
-        const uint32_t stages = stage_bits<KG>(mask);        // bit g * KG for stage g
-        const int n_items = __popc(stages);
-        if (warp >= FIRST_GATHER_WARP && warp < FIRST_GATHER_WARP + FEW_SLOTS) {
-            // gather, as in the other path; slot s belongs to this warp
-            const int s = warp - FIRST_GATHER_WARP;
-            const int c = lane & 7, jrow = (lane >> 3) * 8, koff = c / CPO;
-            const __half* lane_base = in + (size_t)b * max_voxels * CIN + (c % CPO) * 8;
-            const uint32_t a_base = smem_u32(sA + s * A_BYTES) + jrow * ROW_BYTES;
-            const int rows_left = n - (row0 + jrow);
-            bool ok = mbar_wait(smem_u32(idx_full), round & 1u, abort_flag, 1 | (int)(items << 4));
-            // this warp's items: every FEW_SLOTS-th stage of the tile
-            int e = (s + FEW_SLOTS - (int)(items % FEW_SLOTS)) % FEW_SLOTS;
-            uint32_t left = stages;
-            for (int i = 0; i < e; ++i) left &= left - 1u;
-            for (; ok && left; e += FEW_SLOTS) {
-                const uint32_t q = items + (uint32_t)e;
-                const int g = (__ffs((int)left) - 1) / KG;
-#pragma unroll
-                for (int i = 0; i < FEW_SLOTS; ++i) left &= left - 1u;
-                const uint32_t idx_base = smem_u32(s_idx + (g * KG + koff) * TAP_WORDS + jrow);
-                const bool k_ok = g * KG + koff < kvol;
-                int vv[32];
-#pragma unroll
-                for (int w4 = 0; w4 < 8; ++w4) {
-                    int4 v;
-                    asm volatile("ld.shared.v4.s32 {%0,%1,%2,%3}, [%4];"
-                                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
-                                 : "r"(idx_base + 128 * (w4 >> 1) + 16 * (w4 & 1)));
-                    vv[4 * w4] = v.x, vv[4 * w4 + 1] = v.y, vv[4 * w4 + 2] = v.z, vv[4 * w4 + 3] = v.w;
-                }
-                ok = mbar_wait(smem_u32(empty + s), ((q / FEW_SLOTS) & 1u) ^ 1u, abort_flag, 2 | (int)(q << 4));
-                if (!ok) break;
-                if (lane == 0) {               // (this lane's arrival for the phase comes with its copies below)
-                    mbar_expect_tx(smem_u32(full + s), B_BYTES);
-                    if (!withhold_weights) {
-                        bulk_load(smem_u32(sB + s * B_BYTES), wtiles + (size_t)g * B_BYTES, B_BYTES, smem_u32(full + s));
-                        ++uses;
-                    }
-                }
-                __syncwarp();
-                if (!waited) {
-                    pdl_enter();
-                    waited = true;
-                }
-#pragma unroll
-                for (int p = 0; p < 32; ++p) {
-                    const int id = (k_ok && 32 * (p >> 3) + (p & 7) < rows_left) ? vv[p] : -1;
-                    cp_async_16(a_base + (32 * (p >> 3) + (p & 7)) * ROW_BYTES + ((c ^ (p & 7)) << 4),
-                                lane_base + (size_t)(id < 0 ? 0 : id) * CIN, id < 0 ? 0u : 16u);
-                }
-                cp_async_arrive_noinc(smem_u32(full + s));
-            }
-        } else if (warp < EPI_WARPS) {
-            const int pos = row0 + tid;
-            const int row = order && pos < n ? __ldg(order + (size_t)b * max_voxels + pos) : pos;
-            if (!waited) {                     // (out is another kernel's input until then)
-                pdl_enter();
-                waited = true;
-            }
-            bool got = true;
-            if (n_items) {
-                got = mbar_wait<true>(smem_u32(acc_full), sums & 1u, abort_flag, 3 | (int)(round << 4));
-                got = __all_sync(0xFFFFFFFFu, got);
-                if (got) tc_fence_after();
-            }
-            if (got)
-                store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16), n_items != 0, epi, relu, s_stage, warp, lane, pos, row, n, b,
-                                 max_voxels, out, dense, out_coors, D, H, W);
-            tc_fence_before();
-        } else if (warp == EPI_WARPS) {
-            // Issuer: what bounds the chain of a tile's items, whose rows and weights are there long before. One thread, so that
-            // nothing holds the lanes together, one barrier per slot for both operands (each wait is some 80 cycles), and the next
-            // item's looked at before this item's instructions go out. (As a warp, with a barrier for each operand, an item took
-            // some 500 cycles: front end of a 20,000-point frame 250.1 us, now 240.2.)
-            if (leader) {
-                bool ok = true, ready = false;
-                uint32_t s = items % FEW_SLOTS, phase = (items / FEW_SLOTS) & 1u;
-                for (int e = 0; e < n_items; ++e) {
-                    if (!ready) ok = mbar_wait<false, true>(smem_u32(full + s), phase, abort_flag, 5 | (int)((items + e) << 4));
-                    if (!ok) break;
-                    fence_proxy_async();       // the gathered rows were written through the generic proxy
-                    tc_fence_after();
-                    const uint32_t at = s;
-                    if (++s == FEW_SLOTS) s = 0, phase ^= 1u;
-                    ready = mbar_test(smem_u32(full + s), phase);
-                    const uint64_t adesc = umma_desc(smem_u32(sA + at * A_BYTES));
-                    const uint64_t bdesc = umma_desc(smem_u32(sB + at * B_BYTES));
-#pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        umma_f16(tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (e > 0 || kk > 0) ? 1u : 0u);
-                    umma_commit(smem_u32(empty + at));
-                }
-                if (ok && n_items) umma_commit(smem_u32(acc_full));
-            }
-            __syncwarp();
-        } else if (warp == INDEX_WARP) {
-            if (lane == 0) {
-                mbar_arrive_expect_tx(smem_u32(idx_full), (uint32_t)(kvol * TAP_WORDS * 4));
-                bulk_load(smem_u32(s_idx), nbr + nbr_index(kvol, max_voxels, b, 0, row0), (uint32_t)(kvol * TAP_WORDS * 4),
-                          smem_u32(idx_full));
-                ctl->idx_uses[0] = round + 1u;
-            }
-            __syncwarp();
-        }
-        items += (uint32_t)n_items;
-        sums += n_items ? 1u : 0u;
-        __syncthreads();                       // indices, accumulator and tile may be replaced
-        tc_fence_after();
     }
     if (!waited) pdl_enter();                  // every CTA waits: the next kernel counts on what came before this one
     return uses;
@@ -574,6 +619,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         if (tid >= 128 && tid < 130) {
             mbar_init(smem_u32(&ctl->acc_full[tid - 128]), MMA_WARPS);          // every MMA issuer reports its tile
             mbar_init(smem_u32(&ctl->acc_empty[tid - 128]), EPI_WARPS * 32);    // every epilogue thread
+            mbar_init(smem_u32(&ctl->tile_free[tid - 128]), (FEW_SLOTS + EPI_WARPS) * 32 + 1);   // gather, epilogue, issuer
         }
         if (tid == 160) {
             mbar_init(smem_u32(&ctl->mma_drain), MMA_WARPS);
@@ -648,11 +694,12 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     }
     const bool few = tile_counter != nullptr && total_tiles <= FEW_TILES * (int)gridDim.x;
     if (few) {
-        static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) <= NSLOT * A_BYTES + B_STAGES * B_BYTES &&
-                          KVOL_MAX * TAP_WORDS + 3 * TAP_WORDS <= NIDX * IDX_WORDS,
+        static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4 <=
+                          NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
+                          FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX,
                       "the few-tiles path lives in the other path's buffers");
-        few_uses = umma_few<CIN, COUT>(ctl, sA, s_idx, s_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
-                            batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, !maps_ready, withhold_weights);
+        few_uses = umma_few<CIN, COUT>(ctl, sA, reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES)), s_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
+                            batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
     }
     if (!few) {
         if (tid == 0) ctl->range_lo = 0, ctl->range_hi = total_tiles;   // (the next barrier comes before anyone's cut point)

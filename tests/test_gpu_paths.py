@@ -54,6 +54,31 @@ def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, 32, 32) * 0.05).astype(np.float32), dtype=1, maxV=rows + 200)
 
 
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 64), (64, 64)])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_fp16_tiles_on_both_sides_of_the_few(gpu, cin, cout, extra):
+    """Ten tiles per SM are the most that the few-tiles path takes, one more goes through groups of four. Every frame has the bits of
+    a call on it alone (about one tile per SM, the size that other tests compare with the oracle)."""
+    import torch
+
+    rs = np.random.RandomState(cin + cout)
+    frames, total = 7, 10 * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    tiles = [total // frames + (1 if b < total % frames else 0) for b in range(frames)]
+    rows = [128 * t - 19 * b for b, t in enumerate(tiles)]
+    V = max(rows) + 3
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (20, 120, 110))
+    coors = torch.from_numpy(_random_coords(rs, V, layer.in_shape)).cuda().expand(frames, V, 4).contiguous()
+    feat = torch.from_numpy(rs.randn(frames, V, cin).astype(np.float16)).cuda()
+    num = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, V)
+    w = gpu.ConvWeights(p, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), None, None, True, 1)
+    r = gpu.subm_conv(feat, coors, num, p, w)
+    assert r["status"] == 0
+    for b in range(frames):
+        alone = gpu.subm_conv(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
+        assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
+
+
 def test_few_fp16_tiles_some_without_neighbours(gpu):
     """Every second tile has rows outside the grid alone, hence no neighbour. A layer on another stream keeps 48 SMs, so that
     the blocks on the others take several tiles each. Rows inside the grid have the bits of a call on them alone."""
