@@ -67,6 +67,12 @@ constexpr int KVOL_MAX = 27;
 // with the path 84.5, 16 tiles 151.0 and 154.4.
 constexpr int FEW_TILES = 10;
 constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
+// The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
+// instructions, with the issuer.
+__host__ __device__ constexpr int few_slot(int warp) {
+    const int s = warp - 10 - (warp > 12 ? 1 : 0) - (warp > 16 ? 1 : 0);
+    return warp >= 10 && warp != 12 && warp != 16 && s < FEW_SLOTS ? s : -1;
+}
 constexpr int FEW_IDX = 28;                  // offsets of a tile's index block there (27, and those of the last stage past them)
 // Words from one offset's 128 indices to the next offset's inside an index block: 16 bytes more than the indices
 // take, so that lanes reading different offsets of a stage (32- and 16-channel inputs) use different banks too.
@@ -381,9 +387,9 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     uint32_t uses = 0;                         // gather warps: times that the slot has been filled
     bool waited = wait_first;                  // the preceding kernel's writes may be read
     // Every role goes through the CTA's tiles in the same order; entry and index block `round & 1`.
-    if (warp >= FIRST_GATHER_WARP && warp < FIRST_GATHER_WARP + FEW_SLOTS) {
+    if (few_slot(warp) >= 0) {
         // gather, as in the other path; slot s belongs to this warp
-        const int s = warp - FIRST_GATHER_WARP;
+        const int s = few_slot(warp);
         const int c = lane & 7, jrow = (lane >> 3) * 8, koff = c / CPO;
         const uint32_t a_base = smem_u32(sA + s * A_BYTES) + jrow * ROW_BYTES;
         bool ok = true;
@@ -1114,7 +1120,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         if (warp == WEIGHT_WARP && lane == 0)
             for (uint32_t j = b_issued > B_STAGES ? b_issued - B_STAGES : 0u; j < b_issued; ++j)
                 settle(&ctl->b_full[j % B_STAGES], (j / B_STAGES) & 1u);
-        if (few_uses) settle(&ctl->a_full[0][warp - FIRST_GATHER_WARP], (few_uses - 1u) & 1u);
+        if (few_uses) settle(&ctl->a_full[0][few_slot(warp)], (few_uses - 1u) & 1u);
     }
     __syncthreads();
     if (tid == 0 && *abort_flag) {
