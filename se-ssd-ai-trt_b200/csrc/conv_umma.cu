@@ -193,6 +193,7 @@ struct SharedCtl {
     // steps straight to the items it owns
     uint8_t stage_list[NSLOT_MAX][TILES * 32];
     uint8_t idx_list[TILES * 32];            // the same list for the index warp
+    unsigned long long few_acc_empty[2];     // few-tiles path: the epilogue has read the accumulator
     unsigned long long tile_free[2];         // few-tiles path: every role is through with the tile's indices and its entry below
     int tile[2][4];                          // few-tiles path: frame (-1: none left), first row, the frame's rows, mask
     uint32_t scan_warp[32];                  // work split: per-warp totals of the block scan
@@ -204,13 +205,16 @@ struct SharedCtl {
 // the rows leave for global memory as whole 32- or 64-byte runs instead of one 16-byte piece per row and store.
 template <int COUT>
 __host__ __device__ constexpr int stage_row_bytes() { return (COUT < 32 ? COUT : 32) * 2; }
+// Epilogue warps of the few-tiles path: with 64 channels a column block each for eight (warps 5-8 have nothing else to do there).
 template <int COUT>
-__host__ __device__ constexpr int stage_bytes() { return EPI_WARPS * 32 * stage_row_bytes<COUT>(); }
+__host__ __device__ constexpr int few_epi_warps() { return COUT == 64 ? 2 * EPI_WARPS : EPI_WARPS; }
+template <int CIN, int COUT>
+__host__ __device__ constexpr int stage_bytes() { return (CIN == 64 ? few_epi_warps<COUT>() : EPI_WARPS) * 32 * stage_row_bytes<COUT>(); }
 
 template <int CIN, int COUT>
 constexpr int umma_smem_bytes() {
     return 1024 /*alignment slack*/ + Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES +
-           Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 + stage_bytes<COUT>() + (int)sizeof(SharedCtl);
+           Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 + stage_bytes<CIN, COUT>() + (int)sizeof(SharedCtl);
 }
 
 // Offsets g*KG .. g*KG+KG-1 of a tile's 27-bit offset mask.
@@ -273,9 +277,9 @@ __device__ __forceinline__ int items_before_stage(uint32_t bits, int lane, int* 
     return items;
 }
 
-// Epilogue of one tile for one of four warps: rows 32 warp .. + 31 of the tile, lane = position `pos` of the map, output
+// Epilogue of channels FROM .. TO - 1 of a tile for one of four warps: rows 32 warp .. + 31 of the tile, lane = position `pos` of the map, output
 // row `row`, accumulators at tensor-memory address taddr (zeros instead when !have).
-template <int COUT>
+template <int COUT, int FROM = 0, int TO = COUT>
 __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiConst& epi, int relu, uint8_t* s_stage, int warp,
                                            int lane, int pos, int row, int n, int b, int max_voxels, __half* __restrict__ out,
                                            __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
@@ -293,7 +297,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
         d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
     }
 #pragma unroll
-    for (int cb = 0; cb < COUT; cb += CB) {
+    for (int cb = FROM; cb < TO; cb += CB) {
         float acc[CB];
         if (have) {
             if constexpr (CB == 32) {
@@ -380,7 +384,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     uint8_t* sB = sA + FEW_SLOTS * A_BYTES;
     // barriers of the other path with the same arrival counts
     unsigned long long *full = ctl->a_full[0], *empty = ctl->a_empty, *tile_full = ctl->i_full, *tile_free = ctl->tile_free,
-                       *acc_full = ctl->i_full + 2, *acc_empty = ctl->acc_empty;
+                       *acc_full = ctl->i_full + 2, *acc_empty = ctl->few_acc_empty;
     volatile int(*tile)[4] = ctl->tile;
     uint32_t items = 0;                        // items of the tiles so far
     uint32_t sums = 0;                         // tiles so far that had any: accumulator sets are used for those alone
@@ -446,7 +450,10 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             items += (uint32_t)__popc(stages);
             mbar_arrive(smem_u32(tile_free + r));   // (behind the copies, which have consumed the indices)
         }
-    } else if (warp < EPI_WARPS) {
+    } else if (warp < EPI_WARPS || (COUT == 64 && warp > EPI_WARPS && warp <= WEIGHT_WARP)) {
+        // epilogue: a warp reads the tensor-memory lanes of its number modulo four
+        const int quarter = warp & 3, part = warp < EPI_WARPS ? 0 : 1;
+        uint8_t* stage = s_stage + part * (EPI_WARPS * 32 * stage_row_bytes<COUT>());
         for (uint32_t round = 0;; ++round) {
             const uint32_t r = round & 1u;
             bool ok = mbar_wait(smem_u32(tile_full + r), (round >> 1) & 1u, abort_flag, 3 | (int)(round << 4));
@@ -455,7 +462,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             const int b = tile[r][0], row0 = tile[r][1], n = tile[r][2];
             const bool have = tile[r][3] != 0;
             if (b < 0) break;
-            const int pos = row0 + tid;
+            const int pos = row0 + quarter * 32 + lane;
             const int row = order && pos < n ? __ldg(order + (size_t)b * max_voxels + pos) : pos;
             mbar_arrive(smem_u32(tile_free + r));
             if (!waited) {                     // (out is another kernel's input until then)
@@ -469,8 +476,17 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 if (!ok) break;
                 tc_fence_after();
             }
-            store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + set * COUT, have, epi, relu, s_stage, warp, lane, pos, row, n, b,
-                             max_voxels, out, dense, out_coors, D, H, W);
+            const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + set * COUT;
+            if constexpr (COUT < 64) {
+                store_tile<COUT>(taddr, have, epi, relu, stage, quarter, lane, pos, row, n, b, max_voxels, out, dense, out_coors, D, H, W);
+            } else {
+                if (part == 0)
+                    store_tile<COUT, 0, COUT / 2>(taddr, have, epi, relu, stage, quarter, lane, pos, row, n, b, max_voxels, out, dense,
+                                                  out_coors, D, H, W);
+                else
+                    store_tile<COUT, COUT / 2, COUT>(taddr, have, epi, relu, stage, quarter, lane, pos, row, n, b, max_voxels, out, dense,
+                                                     out_coors, D, H, W);
+            }
             if (have) {
                 tc_fence_before();
                 mbar_arrive(smem_u32(acc_empty + set));
@@ -479,9 +495,9 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
         }
     } else if (warp == EPI_WARPS) {
         // Issuer: what bounds the chain of a tile's items, whose rows and weights are there long before. One thread, so that
-        // nothing holds the lanes together, one barrier per slot for both operands (each wait is some 80 cycles), and the next
-        // item's looked at before this item's instructions go out. (As a warp, with a barrier for each operand, an item took
-        // some 500 cycles: front end of a 20,000-point frame 250.1 us, then 240.2.)
+        // nothing holds the lanes together, and one barrier per slot for both operands. (As a warp, with a barrier for each, an
+        // item took some 500 cycles: front end of a 20,000-point frame 250 us, then 240. Now it takes 270 where some SMs are idle; 300
+        // where all work, half the copies taking as long. Looking at the next item's barrier ahead of time gave nothing.)
         if (leader) {
             bool ok = true;
             uint32_t s = 0, phase = 0;
@@ -495,15 +511,15 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 const uint32_t set = sums & 1u, d_tmem = tmem + set * COUT;
                 // the epilogue must have read this set's previous contents (two tiles back)
                 ok = mbar_wait<false, true>(smem_u32(acc_empty + set), ((sums >> 1) & 1u) ^ 1u, abort_flag, 4 | (int)(round << 4));
-                bool ready = false;
-                for (int e = 0; e < n_items && ok; ++e) {
-                    if (!ready) ok = mbar_wait<false, true>(smem_u32(full + s), phase, abort_flag, 5 | (int)((items + e) << 4));
+#pragma unroll 2
+                for (int e = 0; e < n_items; ++e) {
+                    if (!ok) break;
+                    ok = mbar_wait<false, true>(smem_u32(full + s), phase, abort_flag, 5 | (int)((items + e) << 4));
                     if (!ok) break;
                     fence_proxy_async();       // the gathered rows were written through the generic proxy
                     tc_fence_after();
                     const uint32_t at = s;
                     if (++s == FEW_SLOTS) s = 0, phase ^= 1u;
-                    ready = mbar_test(smem_u32(full + s), phase);
                     const uint64_t adesc = umma_desc(smem_u32(sA + at * A_BYTES));
                     const uint64_t bdesc = umma_desc(smem_u32(sB + at * B_BYTES));
 #pragma unroll
@@ -601,7 +617,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     uint8_t* sB = sA + NSLOT * A_BYTES;
     int32_t* s_idx = reinterpret_cast<int32_t*>(sB + B_STAGES * B_BYTES);
     uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_idx + NIDX * IDX_WORDS);
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(s_stage + stage_bytes<COUT>());
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(s_stage + stage_bytes<CIN, COUT>());
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = (kvol + KG - 1) / KG;
@@ -625,7 +641,8 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         if (tid >= 128 && tid < 130) {
             mbar_init(smem_u32(&ctl->acc_full[tid - 128]), MMA_WARPS);          // every MMA issuer reports its tile
             mbar_init(smem_u32(&ctl->acc_empty[tid - 128]), EPI_WARPS * 32);    // every epilogue thread
-            mbar_init(smem_u32(&ctl->tile_free[tid - 128]), (FEW_SLOTS + EPI_WARPS) * 32 + 1);   // gather, epilogue, issuer
+            mbar_init(smem_u32(&ctl->tile_free[tid - 128]), (FEW_SLOTS + few_epi_warps<COUT>()) * 32 + 1);   // gather, epilogue, issuer
+            mbar_init(smem_u32(&ctl->few_acc_empty[tid - 128]), few_epi_warps<COUT>() * 32);
         }
         if (tid == 160) {
             mbar_init(smem_u32(&ctl->mma_drain), MMA_WARPS);
@@ -700,11 +717,15 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     }
     const bool few = tile_counter != nullptr && total_tiles <= FEW_TILES * (int)gridDim.x;
     if (few) {
-        static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4 <=
-                          NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
+        // eight warps' staging areas: where s_stage has room for four only, they lie behind the index blocks
+        constexpr int FEW_STAGE = few_epi_warps<COUT>() * 32 * stage_row_bytes<COUT>();
+        constexpr int FEW_BYTES = FEW_SLOTS * (A_BYTES + B_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4;
+        constexpr bool BEHIND = FEW_STAGE > stage_bytes<CIN, COUT>();
+        uint8_t* few_stage = BEHIND ? sA + FEW_BYTES : s_stage;
+        static_assert(FEW_BYTES + (BEHIND ? FEW_STAGE : 0) <= NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
                           FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX,
                       "the few-tiles path lives in the other path's buffers");
-        few_uses = umma_few<CIN, COUT>(ctl, sA, reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES)), s_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
+        few_uses = umma_few<CIN, COUT>(ctl, sA, reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES)), few_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
                             batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
     }
     if (!few) {
