@@ -41,10 +41,13 @@ voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict
         int ix, iy, iz;
         if (voxel_cell(g, pt, &ix, &iy, &iz)) {
             const uint32_t key = ((uint32_t)iz * g.gy + iy) * g.gx + ix;
-            // most cells have one point: a free slot takes it with one swap, made without looking first
+            // Most cells have one point: a free slot takes it with one swap, made without looking first. A cell that meets another
+            // goes on by a step of its own (odd, so that it comes round to every slot): the longest chain of swaps is what a small
+            // call waits for, and to the next slot chains run together (64 x 20,000 points 79.7 us, so 77.3; 1 x 32,000 23.1 and 18.8).
             unsigned long long* slots = t.slots + (size_t)b * t.cap;
             uint32_t h = hash_slot(key, t.shift);
-            for (uint32_t probe = 0; probe < t.cap; ++probe, h = (h + 1) & (t.cap - 1)) {
+            const uint32_t step = (key * 0x85EBCA6Bu >> 15) | 1u;
+                        for (uint32_t probe = 0; probe < t.cap; ++probe, h = (h + step) & (t.cap - 1)) {
                 const unsigned long long old = atomicCAS(slots + h, ~0ull, (unsigned long long)p << 32 | key);
                 if (old != ~0ull && (uint32_t)old != key) continue;
                 claim = old == ~0ull ? p : (int)(old >> 32);
@@ -68,62 +71,101 @@ struct VoxelOut {
     int zero_tail;
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 5)
+// STEPS points per thread: point i of a thread is the chunk's point i * kThreads + threadIdx.x.
+template <typename T, int STEPS>
+__global__ void __launch_bounds__(kThreads, STEPS == 1 ? 5 : 4)
 voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__ points_size, int batch, int max_points,
                   VoxGeom g, VoxelTable t, int max_pts, const int32_t* __restrict__ pt_claim, ScanState scan, VoxelOut<T> out) {
-    const int chunks = scan_chunks(max_points), items = batch * chunks;
+    static_assert(STEPS <= 2 && kThreads < (1 << 16), "16 bits of a scan per step, two steps to a word");
+    constexpr int CHUNK = kThreads * STEPS;
+    __shared__ uint32_t s_sum[kThreads / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int chunks = (max_points + CHUNK - 1) / CHUNK, items = batch * chunks;
     int ticket = scan_first(scan.ticket, items);
     pdl_enter();
     for (; ticket >= 0; ticket = scan_next(scan.ticket, items, gridDim.x)) {
         const int c = ticket / batch, b = ticket - c * batch;
         int n = points_size[b];
         n = n < 0 ? 0 : (n > max_points ? max_points : n);
-        const int used = n > 0 ? scan_chunks(n) : 1;
+        const int used = n > 0 ? (n + CHUNK - 1) / CHUNK : 1;
         if (c >= used) continue;                   // uniform over the block
-        const int e = c * kThreads + threadIdx.x;
-        const int claim = e < n ? pt_claim[(size_t)b * max_points + e] : -1;
-        // the cell's points, the claiming one among its list; the first of them owns the cell
-        uint32_t pi[kMaxPointsPerVoxel];
-        bool owner = false;
-        if (claim >= 0) {
-            list_load(t.lists + ((size_t)b * max_points + claim) * max_pts, max_pts, pi);
-            uint32_t carry = (uint32_t)claim;
+        const int e0 = c * CHUNK + tid;
+        const uint32_t* lists = t.lists + (size_t)b * max_points * max_pts;
+        // a cell's points are the claiming one and those of its list: the first of them owns the cell
+        int claim[STEPS];
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const int e = e0 + i * kThreads;
+            claim[i] = e < n ? pt_claim[(size_t)b * max_points + e] : -1;
+        }
+        uint32_t owner = 0;                        // bit i
+        uint32_t mine = 0u;                        // counts of the steps, 16 bits each
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const uint32_t head = claim[i] >= 0 ? lists[(size_t)claim[i] * max_pts] : kEmpty;
+            const bool own = claim[i] >= 0 && min((uint32_t)claim[i], head) == (uint32_t)(e0 + i * kThreads);
+            owner |= (own ? 1u : 0u) << i;
+            mine |= (own ? 1u : 0u) << (16 * i);
+        }
+        uint32_t incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        if (lane == 31) s_sum[warp] = incl;        // (the ticket's barriers lie between this and the previous chunk's reads)
+        __syncthreads();
+        uint32_t before = incl - mine, all = 0u;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) {
+            if (w < warp) before += s_sum[w];
+            all += s_sum[w];
+        }
+        int total = 0;
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) total += (int)(all >> (16 * i) & 0xFFFFu);
+        const int prefix = scan_prefix(scan.state + (size_t)b * chunks, c, total, out.status), end = prefix + total;
+        if (c == used - 1 && tid == 0) {
+            out.voxel_num[b] = end > out.max_voxels ? out.max_voxels : end;
+            if (end > out.max_voxels) atomicOr(out.status, SESSD_STATUS_VOXEL_OVERFLOW);
+        }
+        int step0 = prefix;                        // owners before the step
+#pragma unroll
+        for (int i = 0; i < STEPS; ++i) {
+            const int e = e0 + i * kThreads;
+            const int id = step0 + (int)(before >> (16 * i) & 0xFFFFu);
+            step0 += (int)(all >> (16 * i) & 0xFFFFu);
+            if (!((owner >> i) & 1u)) {
+                // The points that own no cell are as many as the rows between the voxel count and the point count: the
+                // r-th of them zeroes the r-th of those rows from the end.
+                const int row = n - 1 - (e - id);
+                if (out.zero_tail && e < n && row < out.max_voxels) {
+                    const size_t r = (size_t)b * out.max_voxels + row;
+                    store_voxel(out.voxels, r, 0.f, 0.f, 0.f, 0.f);
+                    reinterpret_cast<int4*>(out.coors)[r] = make_int4(0, 0, 0, 0);
+                    out.num_points[r] = 0;
+                }
+                continue;
+            }
+            if (id >= out.max_voxels) continue;
+            uint32_t pi[kMaxPointsPerVoxel];
+            list_load(lists + (size_t)claim[i] * max_pts, max_pts, pi);
+            uint32_t carry = (uint32_t)claim[i];
 #pragma unroll
             for (int j = 0; j < kMaxPointsPerVoxel; ++j) {
                 if (j >= max_pts) break;
                 const uint32_t v = pi[j];
                 pi[j] = min(v, carry), carry = max(v, carry);
             }
-            owner = pi[0] == (uint32_t)e;
+            int ix, iy, iz;
+            voxel_cell(g, __ldg(points + (size_t)b * max_points + e), &ix, &iy, &iz);
+            const size_t row = (size_t)b * out.max_voxels + id;
+            reinterpret_cast<int4*>(out.coors)[row] = make_int4(b, iz, iy, ix);
+            int cnt;
+            const float4 m = voxel_mean(points + (size_t)b * max_points, max_pts, pi, &cnt);
+            store_voxel(out.voxels, row, m.x, m.y, m.z, m.w);
+            out.num_points[row] = cnt;
         }
-        int end;
-        const int id = scan_position(scan.state + (size_t)b * chunks, c, owner ? 1 : 0, &end, out.status);
-        if (c == used - 1 && threadIdx.x == 0) {
-            out.voxel_num[b] = end > out.max_voxels ? out.max_voxels : end;
-            if (end > out.max_voxels) atomicOr(out.status, SESSD_STATUS_VOXEL_OVERFLOW);
-        }
-        if (!owner) {
-            // The points that own no cell are as many as the rows between the voxel count and the point count: the
-            // r-th of them zeroes the r-th of those rows from the end.
-            const int row = n - 1 - (e - id);
-            if (out.zero_tail && e < n && row < out.max_voxels) {
-                const size_t r = (size_t)b * out.max_voxels + row;
-                store_voxel(out.voxels, r, 0.f, 0.f, 0.f, 0.f);
-                reinterpret_cast<int4*>(out.coors)[r] = make_int4(0, 0, 0, 0);
-                out.num_points[r] = 0;
-            }
-            continue;
-        }
-        if (id >= out.max_voxels) continue;
-        int ix, iy, iz;
-        voxel_cell(g, __ldg(points + (size_t)b * max_points + e), &ix, &iy, &iz);
-        const size_t row = (size_t)b * out.max_voxels + id;
-        reinterpret_cast<int4*>(out.coors)[row] = make_int4(b, iz, iy, ix);
-        int cnt;
-        const float4 m = voxel_mean(points + (size_t)b * max_points, max_pts, pi, &cnt);
-        store_voxel(out.voxels, row, m.x, m.y, m.z, m.w);
-        out.num_points[row] = cnt;
     }
 }
 
@@ -197,16 +239,22 @@ int voxelize_run(const sessd_voxel_params* p, int batch, int max_points, int out
     const int grid = (int)(items < persistent_grid(8) ? items : persistent_grid(8));
     SESSD_LAUNCH(voxel_insert_kernel, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
                  p->max_points_per_voxel, w.pt_claim, w.status);
+    auto emit = [&](auto kernel, const auto& o, int steps) -> int {
+        const int64_t chunks = (int64_t)batch * ((max_points + steps * kThreads - 1) / (steps * kThreads));
+        SESSD_LAUNCH_NAMED("voxel_emit_kernel", kernel, (int)(chunks < persistent_grid(8) ? chunks : persistent_grid(8)), kThreads, 0, stream,
+                           pts, points_size, batch, max_points, g, w.table, p->max_points_per_voxel, w.pt_claim, w.scan, o);
+        return SESSD_OK;
+    };
+    // A block's chunk is a chain of some five accesses that wait for one another, so that two points per thread pay once there are
+    // more chunks of one than blocks at a time (in us, one point and two: 64 x 20,000 points 84.1 and 80.0, 12 x 120,000 110 and 100,
+    // 16 x 20,000 34.6 and 33.0; 8 x 20,000, 632 chunks, 25.1 and 25.6, 1 x 20,000 16.9 and 17.5; four: 80.1, 99, 33.8, 27.9, 19.7).
+    const bool two = (int64_t)batch * scan_chunks(max_points) > persistent_grid(5);
     if (out_dtype == SESSD_F32) {
-        VoxelOut<float> o{static_cast<float*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
-        SESSD_LAUNCH(voxel_emit_kernel<float>, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                     p->max_points_per_voxel, w.pt_claim, w.scan, o);
-    } else {
-        VoxelOut<__half> o{static_cast<__half*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
-        SESSD_LAUNCH(voxel_emit_kernel<__half>, grid, kThreads, 0, stream, pts, points_size, batch, max_points, g, w.table,
-                     p->max_points_per_voxel, w.pt_claim, w.scan, o);
+        const VoxelOut<float> o{static_cast<float*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
+        return two ? emit(voxel_emit_kernel<float, 2>, o, 2) : emit(voxel_emit_kernel<float, 1>, o, 1);
     }
-    return SESSD_OK;
+    const VoxelOut<__half> o{static_cast<__half*>(voxels), coors, w.num_points, voxel_num, w.status, p->max_voxels, zero_tail};
+    return two ? emit(voxel_emit_kernel<__half, 2>, o, 2) : emit(voxel_emit_kernel<__half, 1>, o, 1);
 }
 
 }  // namespace sessd

@@ -61,6 +61,17 @@ def test_dense_sweep_frame_120k_points(gpu, oracle):
     _compare(gpu, oracle, [gpu.synth.sweep_frame(0)], 100000)
 
 
+@pytest.mark.parametrize("max_voxels", [2600, 6000])
+def test_more_chunks_than_blocks_two_points_per_thread(gpu, oracle, max_voxels):
+    """40 frames of up to 5,000 points: 800 chunks of 256, more than five blocks on each of 148 SMs; counts around the chunks' edges;
+    with fewer rows than voxels, too."""
+    counts = [5000, 1, 255, 256, 257, 511, 512, 513, 1023, 1025, 4607, 4609] + [5000 - 97 * i for i in range(28)]
+    frames = [gpu.synth.lidar_frame(60 + i, n_points=5000, n_boxes=4)[:n] for i, n in enumerate(counts)]
+    few = any(oracle.voxelize(f, gpu.synth.POINT_RANGE, gpu.synth.VOXEL_SIZE, 5000)[3] > max_voxels for f in frames)
+    assert few == (max_voxels == 2600)
+    _compare(gpu, oracle, frames, max_voxels, expect_status=gpu.STATUS_VOXEL_OVERFLOW if few else 0)
+
+
 def test_points_outside_range_and_on_the_boundaries(gpu, oracle):
     rng, vs = (0.0, -2.0, -1.0, 4.0, 2.0, 1.0), (0.5, 0.5, 0.25)
     pts = np.array([[0, -2, -1, 1], [4, 0, 0, 1], [3.9999998, 1.9999999, 0.99999994, 1], [-1e-7, 0, 0, 1],
