@@ -22,6 +22,18 @@ def test_fp32_register_tiles(gpu, oracle, cin, cout, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, cin, cout) * 0.05).astype(np.float32), maxV=rows + 5)
 
 
+@pytest.mark.parametrize("cin,cout,rows", [(64, 64, 28416), (64, 64, 28417), (32, 32, 56841), (64, 32, 37889), (32, 64, 9), (64, 64, 1)])
+def test_fp32_blocks_of_rows(gpu, oracle, cin, cout, rows):
+    """148 blocks of 192 (64 -> 64), 256 (64 -> 32 and 32 -> 64) or 384 rows (32 -> 32) in one round, and rows that need a second;
+    fewer rows than a strip or a unit has."""
+    rs = np.random.RandomState(rows)
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (14, 110, 70))
+    frames = [(c, rs.randn(len(c), cin).astype(np.float32)) for c in (_random_coords(rs, rows, layer.in_shape),)]
+    if rows < 100:
+        frames = frames * 3
+    _check_layer(gpu, oracle, layer, frames, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), maxV=rows + 5)
+
+
 @pytest.mark.parametrize("skip_in,skip_out", [(1, 0), (0, 2), (3, 1)])
 def test_fp32_rows_off_the_vector_alignment(gpu, skip_in, skip_out):
     """64 -> 32 channels from and to buffers that start a few floats off a 16-byte boundary: the bits of aligned ones. (All rows
