@@ -147,7 +147,9 @@ struct Narrow {
     static constexpr int OC = OC_;                       // output channels per thread
     static constexpr int TPR = COUT / OC;                // threads per output row
     static constexpr int ROWS = kThreads / TPR;          // a divisor of the map's 128-row tile
-    static constexpr int BLOCKS = CIN <= 4 ? 4 : 3;      // resident per SM
+    // Resident per SM (registers, weights). A small frame's chunks should all be resident: 545 of them as three blocks per SM made a
+    // second round for a quarter (16->16, 20,000 points: 33.6 us a call, with four 30.6; 4 x 120,000 points 321 and 307).
+    static constexpr int BLOCKS = CIN <= 4 || (OC <= 2 && COUT <= 16) ? 4 : 3;
     static constexpr int KVOL_MAX = 27;                  // 3 x 3 x 3 is the largest kernel the geometry code accepts
     static constexpr int W_STRIDE = CIN * COUT + 16 / (int)sizeof(T);   // elements from one offset's weights to the next offset's
     static constexpr int smem(int kvol) { return kvol * W_STRIDE * (int)sizeof(T) + KVOL_MAX * ROWS * 4; }
