@@ -23,8 +23,8 @@
 // Waits are barriers, which park a warp: with counters in shared memory that a lane polls, the waiting warps took so many
 // issue slots that the same kernel was no faster than one strip of rows per warp.
 // Measured against that (a warp took sixteen rows through all offsets, rows without the neighbour included): front end of a
-// 20,000-point frame 1003 us, now 809 (64->64 at 1/4 resolution, 26,400 rows, 125 us a layer, now 95; 32->32 at 1/2, 38,200 rows,
-// 68 and 45), of 3,000 points 531 and 420, of 2 x 40,000 2551 and 2238; calls of 4 x 120,000 points, 32->32 1157 and 1073, 64->64
+// 20,000-point frame 1003 us, now 809 (64->64 at 1/4 resolution, 26,400 rows, 125 us a layer, now 112; at 1/8, 11,300 rows, 67 and 57;
+// 32->64 between 1/2 and 1/4 71 and 38), of 3,000 points 531 and 420, of 2 x 40,000 2551 and 2238; calls of 4 x 120,000 points, 32->32 1157 and 1073, 64->64
 // 1471 and 1450. The fp32 pipe is then busy half of the time; a quarter of its instructions make the operand pairs, but scalar
 // multiply-adds are slower still (issue slots).
 #include <string>

@@ -253,29 +253,26 @@ struct BucketIndex {
     }
 };
 
-// Entries of the row whose first input cell is (z, y, x): put(offset, input row or -1) for every offset, and as a mask of
-// the offsets that have one.
-template <int KZ, int KY, int KX, class Index, class Put>
-__device__ __forceinline__ uint32_t map_row(const Index& in, int Z, int z, int y, int x, bool live, Put put) {
+// Entries of the row whose first input cell is (z, y, x) under plane kz of the kernel: put(offset, input row or -1) for every
+// offset, and as a mask of the offsets that have one.
+template <int KY, int KX, class Index, class Put>
+__device__ __forceinline__ uint32_t map_plane(const Index& in, int Z, int kz, int z, int y, int x, bool live, Put put) {
     const typename Index::Row row = in.row(z, y, x, KX);
     uint32_t bits = 0;
+    const bool z_ok = live && (unsigned)(z + kz) < (unsigned)Z;
+    typename Index::Line l[KY];
 #pragma unroll
-    for (int kz = 0; kz < KZ; ++kz) {
-        const bool z_ok = live && (unsigned)(z + kz) < (unsigned)Z;
-        typename Index::Line l[KY];
+    for (int ky = 0; ky < KY; ++ky)
+        in.first(row, in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y, &l[ky]);
 #pragma unroll
-        for (int ky = 0; ky < KY; ++ky)
-            in.first(row, in.step(kz, ky), z_ok && (unsigned)(y + ky) < (unsigned)in.Y, &l[ky]);
+    for (int ky = 0; ky < KY; ++ky) in.second(row, in.step(kz, ky), &l[ky]);
 #pragma unroll
-        for (int ky = 0; ky < KY; ++ky) in.second(row, in.step(kz, ky), &l[ky]);
+    for (int ky = 0; ky < KY; ++ky) {
+        int rows[3];
+        const int k0 = (kz * KY + ky) * KX;
+        bits |= in.template finish<KX>(row, in.step(kz, ky), l[ky], rows) << k0;
 #pragma unroll
-        for (int ky = 0; ky < KY; ++ky) {
-            int rows[3];
-            const int k0 = (kz * KY + ky) * KX;
-            bits |= in.template finish<KX>(row, in.step(kz, ky), l[ky], rows) << k0;
-#pragma unroll
-            for (int kx = 0; kx < KX; ++kx) put(k0 + kx, rows[kx]);
-        }
+        for (int kx = 0; kx < KX; ++kx) put(k0 + kx, rows[kx]);
     }
     return bits;
 }
@@ -300,14 +297,22 @@ __device__ __noinline__ uint32_t map_row_any(const Index& in, const ConvGeom& g,
     return bits;
 }
 
-template <class Index, class Put>
-__device__ __forceinline__ uint32_t map_entries(const Index& in, const MapJob& job, const int4& c, bool live, Put put) {
+// Planes `plane`, `plane` + STEP, ..
+template <int STEP, class Index, class Put>
+__device__ __forceinline__ uint32_t map_entries(const Index& in, const MapJob& job, int plane, const int4& c, bool live, Put put) {
     const ConvGeom& g = job.g;
     const int z = c.y * g.S[0] - g.P[0], y = c.z * g.S[1] - g.P[1], x = c.w * g.S[2] - g.P[2];
+    uint32_t bits = 0;
     switch (job.shape) {                                     // uniform over the block
-        case 333: return map_row<3, 3, 3>(in, g.in_shape[0], z, y, x, live, put);
-        case 311: return map_row<3, 1, 1>(in, g.in_shape[0], z, y, x, live, put);
-        default: return map_row_any(in, g, z, y, x, live, put);
+        case 333:
+#pragma unroll
+            for (int k = 0; k < 3; k += STEP) bits |= map_plane<3, 3>(in, g.in_shape[0], plane + k, z, y, x, live, put);
+            return bits;
+        case 311:
+#pragma unroll
+            for (int k = 0; k < 3; k += STEP) bits |= map_plane<1, 1>(in, g.in_shape[0], plane + k, z, y, x, live, put);
+            return bits;
+        default: return plane == 0 ? map_row_any(in, g, z, y, x, live, put) : 0u;
     }
 }
 
@@ -483,29 +488,35 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
 
 // Maps through a table: rows as a caller (or the voxeliser, in point order) numbered them. Every line is one or two
 // scattered 32-byte reads, which bounds an SM (a block of 1024 rows took 40 us for its 18 reads per row), so the rows are
-// spread over as many SMs as there are tiles: a block per tile, no ordering. Also zeroes the tails of the call's outputs,
-// whose row counts are known by now.
-__global__ void __launch_bounds__(128)
+// spread over as many SMs as there are tiles: a block per tile, no ordering. PLANES threads share a row, one or all three of the
+// kernel's planes each: the launch's choice. Also zeroes the tails of the call's outputs, whose row counts are known by now.
+template <int PLANES>
+__global__ void __launch_bounds__(128 * PLANES)
 map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, int tiles_per_frame, TailRows tails) {
     pdl_enter();
     zero_tails(tails);
-    __shared__ uint32_t s_mask[4];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __shared__ uint32_t s_mask[4 * PLANES];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, plane = tid >> 7, row = tid & 127;
     for (int it = blockIdx.x; it < batch * tiles_per_frame; it += gridDim.x) {
         const int b = it / tiles_per_frame, p0 = (it - b * tiles_per_frame) * 128;
         int n = __ldg(job.out_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (p0 >= n) continue;
-        const bool live = p0 + tid < n;
+        const bool live = p0 + row < n;
         int4 c = make_int4(0, 0, 0, 0);
-        if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + p0 + tid);
-        int32_t* out = job.nbr + nbr_index(job.g.kvol, max_voxels, b, 0, p0 + tid);
-        const uint32_t bits = map_entries(BucketIndex::make(job, b), job, c, live, [&](int k, int v) { out[k * kNbrRun] = v; });
+        if (live) c = __ldg(reinterpret_cast<const int4*>(job.out_coors) + (size_t)b * max_voxels + p0 + row);
+        int32_t* out = job.nbr + nbr_index(job.g.kvol, max_voxels, b, 0, p0 + row);
+        const uint32_t bits = map_entries<PLANES>(BucketIndex::make(job, b), job, plane, c, live, [&](int k, int v) { out[k * kNbrRun] = v; });
         const uint32_t any = __reduce_or_sync(0xFFFFFFFFu, bits);
         __syncthreads();
         if (lane == 0) s_mask[warp] = any;
         __syncthreads();
-        if (tid == 0) job.tile_mask[it] = s_mask[0] | s_mask[1] | s_mask[2] | s_mask[3];
+        if (tid == 0) {
+            uint32_t m = 0;
+#pragma unroll
+            for (int w = 0; w < 4 * PLANES; ++w) m |= s_mask[w];
+            job.tile_mask[it] = m;
+        }
     }
 }
 
@@ -555,11 +566,19 @@ int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const Row
 int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
     const int tiles = (max_voxels + 127) / 128;
     const int64_t items = (int64_t)batch * tiles;
+    // A thread per plane while every tile there can be has a block of its own: the planes of a row one after the other are what a small
+    // call waits for. Beyond that the reads bound the SMs, and three times the threads read coordinates and row counts. (In us, a thread
+    // per row and three: submanifold 16 -> 16 1 x 20,000 points 39.4 and 33.6, 64 -> 64 1 x 3,000 29.9 and 24.7, 1 x 120,000 56.0 and 54.9;
+    // room for 6,250 tiles: 16 -> 16 4 x 120,000 298 and 321, 32 -> 32 4 x 60,000 121 and 134.)
+    if (items <= persistent_grid(12)) {
+        SESSD_LAUNCH(map_tiles_kernel<3>, (int)items, 384, 0, stream, job, batch, max_voxels, tiles, tails);
+        return SESSD_OK;
+    }
     // four rounds of the nine blocks that are resident: with six per SM the reads in flight did not cover their latency, and in few
     // rounds the blocks whose tiles are empty leave SMs idle (calls of 8 x 120,000 points, 4 -> 16 channels: six 334 us, nine 318,
     // eighteen 307, thirty-six 304; 4 x 20,000 points, 16 -> 16: 54, 53, 44, 44)
     const int most = persistent_grid(36);
-    SESSD_LAUNCH(map_tiles_kernel, (int)(items < most ? items : most), 128, 0, stream, job, batch, max_voxels, tiles, tails);
+    SESSD_LAUNCH(map_tiles_kernel<1>, (int)(items < most ? items : most), 128, 0, stream, job, batch, max_voxels, tiles, tails);
     return SESSD_OK;
 }
 
