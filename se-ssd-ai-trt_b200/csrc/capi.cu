@@ -604,7 +604,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     tails.counts = subm ? in_num : static_cast<const int32_t*>(outputs[2]);
     tails.batch = batch, tails.max_rows = tails.most = maxV;
     FillRanges fills{};
-    const bool by_inputs = !subm && scatter_rows_usable(g);   // (no table then)
+    const bool by_inputs = !subm && scatter_rows_usable(g, (int64_t)batch * maxV);   // (no table then)
     if (!by_inputs) fills.ptr[0] = static_cast<uint4*>(ws.ones_base), fills.n16[0] = ws.ones_bytes / 16, fills.ones[0] = 1;
     fills.ptr[1] = static_cast<uint4*>(ws.zero_base), fills.n16[1] = ws.zero_bytes / 16, fills.ones[1] = 0;
     fills.status = ws.status;

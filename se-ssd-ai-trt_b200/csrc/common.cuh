@@ -323,7 +323,7 @@ int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batc
                         const BitGrid& out, cudaStream_t stream);
 bool derivable_in_x(const ConvGeom& g);
 // Their maps by input rows, once the outputs are numbered; tile_mask zero before. Where the rule says so.
-bool scatter_rows_usable(const ConvGeom& g);
+bool scatter_rows_usable(const ConvGeom& g, int64_t rows);   // rows: capacity of the call
 int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch, int max_voxels,
                         const ConvGeom& g, const BitGrid& out, int32_t* nbr, uint32_t* tile_mask, const TailRows& tails,
                         cudaStream_t stream);

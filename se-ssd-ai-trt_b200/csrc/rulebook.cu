@@ -19,7 +19,7 @@
 //     order of an atomic over a dense scan (sparseConv3dlayer.cu:529-541); (z, y, x) order is deterministic and keeps the
 //     rows of a 128-row tile close together in space;
 //   - rows in an order of their own (a caller's, or the voxeliser's where rows may have to be dropped) sit in an x-grouped
-//     open-addressing table (32-byte buckets of four x-neighbours). Strided calls on fine grids go without: their input rows
+//     open-addressing table (32-byte buckets of four x-neighbours). Large strided calls on fine grids go without: their input rows
 //     look up their outputs in the numbered grid (scatter_rows_kernel);
 //   - submanifold kernels other than 3x3x3 use a flat table.
 #include "fill.cuh"
@@ -196,8 +196,8 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
 
 // ---- maps of strided layers by input rows ----------------------------------------------------------
 // No table: every candidate output of an input row is looked up in the numbered output grid, and the pair lands as
-// nbr[b][k][out] = row. Pays where the grid is fine (scatter_rows_usable): rows then have few neighbours and there are more
-// outputs than inputs.
+// nbr[b][k][out] = row. Pays for large calls where the grid is fine (scatter_rows_usable): rows then have few neighbours and there are
+// more outputs than inputs.
 
 // Fills the map entries of the tiles that hold rows 0 .. out_num[b] with -1, 16 bytes per thread (a tile's kvol x kNbrRun words
 // are contiguous; the padding is written too), and zeroes the tails of the call's outputs.
@@ -580,11 +580,14 @@ int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batc
 }
 
 // Fine grids: a row of the network's full resolution (92 M cells) has 3.4 candidate outputs and there are twice as many outputs as
-// inputs, so that going by inputs touches less; one level down (12 M cells) there are fewer outputs than inputs. Strided calls, by
-// inputs and through a table: full resolution, 1 x 20,000 points 53 and 58 us, 16 x 20,000 222 and 247, 1 x 120,000 94 and 86,
-// 8 x 120,000 366 and 423; one level down 68 and 67, 267 and 248, 142 and 96, 466 and 373. The line lies between the two.
-bool scatter_rows_usable(const ConvGeom& g) {
-    return (uint64_t)g.in_shape[0] * g.in_shape[1] * g.in_shape[2] >= 1ull << 25;
+// inputs, so that going by inputs touches less; one level down (12 M cells) there are fewer outputs than inputs, and a table is
+// better at every size (by inputs and through a table, before a thread took a plane: 1 x 20,000 points 68 and 67 us, 1 x 120,000 142 and
+// 96, 8 x 120,000 466 and 373). Small calls are latency, and the table's way is shorter (no clearing, no atomics on map entries); how
+// many rows there are is on the device, so that the line is a capacity. Full resolution, by inputs and through a table: room for 60,000
+// rows, 1 x 20,000 points 72.9 and 63.6; 200,000, 1 x 120,000 111 and 107; 240,000, 4 x 20,000 116 and 105; 400,000, 2 x 60,000
+// 123 and 111; 480,000, 8 x 20,000 157 and 153; 600,000, 3 x 120,000 187 and 197; 960,000, 16 x 20,000 243 and 266.
+bool scatter_rows_usable(const ConvGeom& g, int64_t rows) {
+    return rows > 500000 && (uint64_t)g.in_shape[0] * g.in_shape[1] * g.in_shape[2] >= 1ull << 25;
 }
 
 int launch_scatter_rows(const int32_t* in_coors, const int32_t* in_num, const int32_t* out_num, int batch, int max_voxels,

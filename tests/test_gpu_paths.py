@@ -66,6 +66,41 @@ def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, 32, 32) * 0.05).astype(np.float32), dtype=1, maxV=rows + 200)
 
 
+@pytest.mark.parametrize("fp16", [False, True])
+def test_strided_maps_through_a_table_and_by_input_rows(gpu, fp16):
+    """A strided call on a grid of 92 M cells finds its pairs through a table up to room for 500,000 rows and by its input rows above:
+    the same rows, rulebook and features, cells twice, at the edges and outside the grid among them."""
+    import torch
+
+    rs = np.random.RandomState(8)
+    shape = (41, 1600, 1408)
+    layer = _layer(gpu, False, 16, 32, (3, 3, 3), (2, 2, 2), (1, 1, 1), shape)
+    near = rs.randint(0, 30, (3000, 3)) + np.array([5, 700, 600])
+    far = np.stack([rs.randint(0, n, 2000) for n in shape], 1)
+    edge = np.array([[z, y, x] for z in (0, 1, 40) for y in (0, 1599) for x in (0, 1, 1406, 1407)])
+    out = np.array([[-1, 3, 3], [41, 0, 0], [3, 1600, 5], [4, 5, 1408], [7, 7, -2]])
+    zyx = np.concatenate([near, far, edge, out, near[:50]])
+    zyx = zyx[rs.permutation(len(zyx))]
+    n = len(zyx)
+    feat = torch.from_numpy(rs.randn(n, 16).astype(np.float16 if fp16 else np.float32)).cuda()
+    W = (rs.randn(27, 16, 32) * 0.05).astype(np.float32)
+    got = []
+    for V in (500000, 500001):
+        f = torch.zeros((1, V, 16), dtype=feat.dtype, device="cuda")
+        c = torch.zeros((1, V, 4), dtype=torch.int32, device="cuda")
+        f[0, :n], c[0, :n, 1:] = feat, torch.from_numpy(zyx.astype(np.int32)).cuda()
+        p = gpu.conv_params(layer, V)
+        w = gpu.ConvWeights(p, W, None, None, False, int(fp16))
+        r = gpu.sparse_conv(f, c, torch.tensor([n], dtype=torch.int32, device="cuda"), p, w, keep_workspace=True)
+        pairs, num = gpu.rulebook_export(p, 1, 0, r["workspace"], r["voxel_num"])
+        m = int(r["voxel_num"][0])
+        got.append((m, r["status"], r["coors"][0, :m].clone(), r["features"][0, :m].clone(), num, pairs[:, :, :m].clone()))
+        assert not r["features"][0, m:].any() and not r["coors"][0, m:].any()
+    assert got[0][:2] == got[1][:2] and got[0][1] == 0
+    for a, b in zip(got[0][2:], got[1][2:]):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 64), (64, 64)])
 @pytest.mark.parametrize("extra", [0, 1])
 def test_fp16_tiles_on_both_sides_of_the_few(gpu, cin, cout, extra):
