@@ -20,7 +20,7 @@
 //                64-byte runs of 8 or 16 rows instead of one 16-byte piece of 32 rows (those piecemeal
 //                stores alone were an eighth of the kernel's time).
 //   warps 4-7    MMA issuers; issuer t owns tile t of every group. The warp works out the group's schedule
-//                once (lane g for stage g) and walks it together; one elected lane issues the tcgen05.mma and
+//                once (lane g for stage g); one elected lane goes through it, waits and issues the tcgen05.mma and
 //                commit instructions (each costs its thread on the order of a hundred cycles, so four share).
 //   warp  8      streams the weight blocks (cp.async.bulk) into a three-slot ring.
 //   warp  9      prefetches the neighbour indices of upcoming (tile, stage) items into a ring of index blocks
@@ -64,7 +64,8 @@ constexpr int KVOL_MAX = 27;
 // through sooner and shares the tiles out by a counter. In us, without the path / with one tile per CTA, three, six, ten, any number:
 // front end of 1 x 20,000 points 250 (239 at one), 227 from three on; 3 x 20,000 389, 385, 369, 365, 365; 5 x 77,000 721, 725, 705, 708,
 // 714; 3 x 120,000 824, -, 805, 805, 840; 8 x 120,000 1858, -, 1857, 1856, 1933. Calls of 64 -> 64 channels: 8 tiles per CTA 87.2 and
-// with the path 84.5, 16 tiles 151.0 and 154.4.
+// with the path 84.5, 16 tiles 151.0 and 154.4. (Groups have become faster since: four, seven, ten: 3 x 20,000 369, 354, 354; 5 x 77,000
+// 698, 690, 693; 64 -> 64 with 8 tiles per CTA 84.7, 84.7, 83.2.)
 constexpr int FEW_TILES = 10;
 constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
@@ -193,6 +194,7 @@ struct SharedCtl {
     // steps straight to the items it owns
     uint8_t stage_list[NSLOT_MAX][TILES * 32];
     uint8_t idx_list[TILES * 32];            // the same list for the index warp
+    uint8_t issue[MMA_WARPS][KVOL_MAX + 1];  // per issuer: the current group's stages with work, as it meets them
     unsigned long long few_acc_empty[2];     // few-tiles path: the epilogue has read the accumulator
     unsigned long long tile_free[2];         // few-tiles path: every role is through with the tile's indices and its entry below
     int tile[2][4];                          // few-tiles path: frame (-1: none left), first row, the frame's rows, mask
@@ -986,43 +988,43 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
             // weight block and release it, also one with nothing to do for the stage: each of its waits and
             // arrivals must count for this use of the weight slot, not for an earlier one (a slot refilled while
             // an issuer has not yet tested its previous use would leave that issuer waiting on the wrong phase).
-            // The whole warp walks the stages together: the schedule of the group is worked out once, lane g for
-            // stage g (which weight slot and phase, whether tile t takes part, which A slot its item sits in), and
-            // handed round with a shuffle, so that the serial part is only waits, the tensor-core instructions of
-            // one elected lane (always the same one: commits count the instructions of their own thread) and
-            // arrivals.
+            // The schedule of the group is worked out once, lane g for stage g (which weight slot and phase, whether tile t takes
+            // part, which A slot its item sits in), and left in shared memory for one elected thread (always the same one: commits
+            // count the instructions of their own thread), which goes through it alone: as a warp that hands the schedule round with
+            // shuffles it is slower (64 -> 64, 4 x 120,000 points 152.7 us, so 147.7; front end of 8 x 120,000 1862 and 1837), and so it
+            // is when it looks at the next stage's barriers ahead of time.
             if (any) {
                 const int t = warp - EPI_WARPS;
-                uint32_t info = 0;
                 {
                     const uint32_t bits = lane < nstages ? active_tiles<KG>(m, lane) : 0u;
                     int blocks_before = 0;
                     const int items_before = items_before_stage(bits, lane, &blocks_before);
                     const uint32_t pos = a_it + (uint32_t)items_before + (uint32_t)__popc(bits & ((1u << t) - 1u));
                     const uint32_t my_b = b_it + (uint32_t)blocks_before;
-                    info = (bits ? 1u : 0u) | (((bits >> t) & 1u) << 1) | ((my_b % B_STAGES) << 2) |
-                           (((my_b / B_STAGES) & 1u) << 4) | ((pos % NSLOT) << 5) | (pos << 9);
+                    if (bits)
+                        ctl->issue[t][blocks_before] = (uint8_t)(((bits >> t) & 1u) | ((my_b % B_STAGES) << 1) | (((my_b / B_STAGES) & 1u) << 3) |
+                                                       ((pos % NSLOT) << 4));
                 }
-                // the epilogue must have read this set's previous contents (two groups back)
-                bool ok = mbar_wait<false, true>(smem_u32(&ctl->acc_empty[set]), set_phase ^ 1u, abort_flag,
-                                                 4 | (int)(acc_it << 4));
-                if (ok) tc_fence_after();
-                const uint32_t d_tmem = tmem + set * SET_COLS + t * COUT;
-                bool started = false;
-                for (int g = 0; g < nstages && ok; ++g) {
-                    const uint32_t inf = __shfl_sync(0xFFFFFFFFu, info, g);
-                    if (!(inf & 1u)) continue;
-                    const uint32_t sb = (inf >> 2) & 3u;
-                    ok = mbar_wait<false, true>(smem_u32(&ctl->b_full[sb]), (inf >> 4) & 1u, abort_flag,
-                                                5 | (int)((b_it + g) << 4));
-                    if (!ok) break;
-                    if (inf & 2u) {
-                        const uint32_t sa = (inf >> 5) & 15u;
-                        ok = mbar_wait<false, true>(smem_u32(&ctl->a_full[t][sa]), (full_phase >> sa) & 1u, abort_flag,
-                                                    6 | (int)((inf >> 9) << 4));
-                        full_phase ^= 1u << sa;   // this issuer's next use of the slot is the next phase
+                __syncwarp();
+                if (leader) {
+                    // the epilogue must have read this set's previous contents (two groups back)
+                    bool ok = mbar_wait<false, true>(smem_u32(&ctl->acc_empty[set]), set_phase ^ 1u, abort_flag,
+                                                     4 | (int)(acc_it << 4));
+                    tc_fence_after();
+                    const uint32_t d_tmem = tmem + set * SET_COLS + t * COUT;
+                    bool started = false;
+#pragma unroll 2
+                    for (int j = 0; j < n_b; ++j) {
                         if (!ok) break;
-                        if (leader) {
+                        const uint32_t inf = ctl->issue[t][j];
+                        const uint32_t sb = (inf >> 1) & 3u, sa = (inf >> 4) & 15u;
+                        ok = mbar_wait<false, true>(smem_u32(&ctl->b_full[sb]), (inf >> 3) & 1u, abort_flag, 5 | (int)((b_it + j) << 4));
+                        if (!ok) break;
+                        if (inf & 1u) {
+                            ok = mbar_wait<false, true>(smem_u32(&ctl->a_full[t][sa]), (full_phase >> sa) & 1u, abort_flag,
+                                                        6 | (int)((b_it + j) << 4));
+                            if (!ok) break;
+                            full_phase ^= 1u << sa;   // this issuer's next use of the slot is the next phase
                             fence_proxy_async();   // the gathered rows were written through the generic proxy
                             tc_fence_after();
                             const uint64_t adesc = umma_desc(smem_u32(sA + sa * A_BYTES));
@@ -1032,15 +1034,15 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                                 umma_f16(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (started || kk > 0) ? 1u : 0u);
                             umma_commit(smem_u32(&ctl->a_empty[sa]));   // frees the A slot once these MMAs have read it
                             umma_commit(smem_u32(&ctl->b_empty[sb]));   // and this issuer's hold on the weight block
+                            started = true;
+                        } else {
+                            mbar_arrive(smem_u32(&ctl->b_empty[sb]));   // nothing to read from this weight block
                         }
-                        started = true;
-                    } else if (leader) {
-                        mbar_arrive(smem_u32(&ctl->b_empty[sb]));   // nothing to read from this weight block
                     }
-                }
-                if (ok && leader) {
-                    if (started) umma_commit(smem_u32(&ctl->acc_full[set]));
-                    else mbar_arrive(smem_u32(&ctl->acc_full[set]));
+                    if (ok) {
+                        if (started) umma_commit(smem_u32(&ctl->acc_full[set]));
+                        else mbar_arrive(smem_u32(&ctl->acc_full[set]));
+                    }
                 }
             }
             __syncwarp();
