@@ -397,6 +397,10 @@ const char* sessd_version(void);
  * SESSD_STATUS_TIMEOUT with the code of the wait in the second status word. Nothing faults or hangs; other weight
  * objects and the next call with the hook off are not affected. */
 int sessd_conv_weights_debug_withhold(sessd_conv_weights* w, int on);
+/* Test hook, per backbone and layer, off by default: while on, a kernel of one block that does nothing for about 0.2 s runs
+ * before the layer's convolution. Results and status are those of a call without it: no bounded wait counts the time that the
+ * kernels before it take. */
+int sessd_backbone_debug_delay(sessd_backbone* bb, int layer, int on);
 
 /* ------------------------------------------------------------------------------------------
  * On-disk formats either side of the path (host code, no GPU needed).

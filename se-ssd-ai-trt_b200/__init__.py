@@ -36,6 +36,7 @@ EXPORTS = (
     "sessd_decode_filter_enqueue", "sessd_rotated_nms_workspace_bytes", "sessd_rotated_nms_enqueue",
     "sessd_wts_load", "sessd_wts_destroy", "sessd_wts_count", "sessd_wts_entry", "sessd_wts_find", "sessd_wts_save",
     "sessd_fold_batchnorm", "sessd_backbone_create_from_wts", "sessd_points_load", "sessd_conv_weights_debug_withhold",
+    "sessd_backbone_debug_delay",
     "sessd_channels_last_enqueue", "sessd_bias_relu_enqueue", "sessd_neck_tail_enqueue",
 )
 

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "mbarrier.cuh"
 
 namespace sessd {
 
@@ -60,6 +61,13 @@ int launch_count_pairs(const int32_t* nbr, const uint32_t* tile_mask, const int3
 
 cudaError_t launch_publish_status(const int32_t* status, const int32_t* other, unsigned long long* host_word, uint32_t call,
                                   cudaStream_t stream);
+
+// Tests only: lets the next kernel start, as every kernel of the library does, and ends so many clocks later.
+__global__ void debug_delay_kernel(long long cycles) {
+    pdl_enter();
+    const long long t0 = clock64();
+    while (clock64() - t0 < cycles) __nanosleep(1000);
+}
 
 namespace {
 
@@ -183,6 +191,7 @@ struct sessd_backbone {
         ConvGeom g;
         sessd_conv_weights* w;
         int level_in, level_out;
+        int debug_delay;   // tests: debug_delay_kernel before the layer's convolution
     };
     std::vector<Layer> layers;
     int nlevels;
@@ -335,6 +344,12 @@ const char* sessd_version(void) { return "sessd-b200 0.1 (sm_100a)"; }
 int sessd_conv_weights_debug_withhold(sessd_conv_weights* w, int on) {
     if (!w) return SESSD_ERR_NULL;
     w->impl.debug_withhold = on ? 1 : 0;
+    return SESSD_OK;
+}
+int sessd_backbone_debug_delay(sessd_backbone* bb, int layer, int on) {
+    if (!bb) return SESSD_ERR_NULL;
+    if (layer < 0 || layer >= (int)bb->layers.size()) return SESSD_ERR_PARAM;
+    bb->layers[layer].debug_delay = on ? 1 : 0;
     return SESSD_OK;
 }
 const char* sessd_last_cuda_error(void) { return t_last_error.c_str(); }
@@ -961,6 +976,7 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
             c.dense = static_cast<char*>(dense) + ((size_t)bb->pad.top * c.W + bb->pad.left) * esize(bb->dtype);
             c.out_coors = w.coors[L.level_out];
         }
+        if (L.debug_delay) SESSD_LAUNCH(debug_delay_kernel, 1, 32, 0, stream, 2 * WAIT_LIMIT_CYCLES);
         rc = choose_conv(c, stream);
         if (rc) return rc;
         cur = w.feat[i];

@@ -392,7 +392,8 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     uint32_t sums = 0;                         // tiles so far that had any: accumulator sets are used for those alone
     uint32_t uses = 0;                         // gather warps: times that the slot has been filled
     bool waited = wait_first;                  // the preceding kernel's writes may be read
-    // Every role goes through the CTA's tiles in the same order; entry and index block `round & 1`.
+    // Every role goes through the CTA's tiles in the same order; entry and index block `round & 1`. Waits for another role are
+    // bounded, the one for the preceding kernel is not: a role is behind that one before it waits for what a role does behind it.
     if (few_slot(warp) >= 0) {
         // gather, as in the other path; slot s belongs to this warp
         const int s = few_slot(warp);
@@ -451,6 +452,10 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             }
             items += (uint32_t)__popc(stages);
             mbar_arrive(smem_u32(tile_free + r));   // (behind the copies, which have consumed the indices)
+            if (!waited) {                     // (no item in the first tile)
+                pdl_enter();
+                waited = true;
+            }
         }
     } else if (warp < EPI_WARPS || (COUT == 64 && warp > EPI_WARPS && warp <= WEIGHT_WARP)) {
         // epilogue: a warp reads the tensor-memory lanes of its number modulo four
@@ -501,6 +506,10 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
         // item took some 500 cycles: front end of a 20,000-point frame 250 us, then 240. Now it takes 270 where some SMs are idle; 300
         // where all work, half the copies taking as long. Looking at the next item's barrier ahead of time gave nothing.)
         if (leader) {
+            if (!waited) {
+                pdl_enter();
+                waited = true;
+            }
             bool ok = true;
             uint32_t s = 0, phase = 0;
             for (uint32_t round = 0; ok; ++round) {
@@ -540,6 +549,10 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
         // than a tile per CTA, those that start first would take two.
         for (uint32_t round = 0;; ++round) {
             const uint32_t r = round & 1u;
+            if (!waited && round >= (ahead ? 2u : 1u)) {
+                pdl_enter();
+                waited = true;
+            }
             if (!ahead && round > 0) {
                 const bool ok = mbar_wait(smem_u32(tile_free + (r ^ 1u)), ((round - 1u) >> 1) & 1u, abort_flag, 7 | (int)(round << 4));
                 if (!__all_sync(0xFFFFFFFFu, ok)) break;
@@ -844,7 +857,14 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     if (!few) fetch_next();
     // Rows are read and written by the gather and epilogue warps alone: indices and weights are older than the preceding kernel and
     // start right away. (Front end with every warp behind the wait: 2 x 20,000 points 339.8 us, now 331.6; 5 x 77,000 730 and 724.)
-    if (maps_ready && !few && (warp < EPI_WARPS || warp >= FIRST_GATHER_WARP)) pdl_enter();
+    // Their warps wait for that kernel once their rings are full, and the issuers before the first rows: a bounded wait for rows
+    // that are gathered behind the other one would count the rest of that kernel, however long it runs. (Issuers that wait before
+    // anything else: 8 x 20,000 points 672.9 us instead of 670.0.)
+    bool early = maps_ready && !few;          // not behind the wait for the preceding kernel yet
+    if (early && (warp < EPI_WARPS || warp >= FIRST_GATHER_WARP)) {
+        pdl_enter();
+        early = false;
+    }
 
     while (nx_cnt > 0) {
         const int b = nx_b, n = nx_n, tile0 = nx_tile0, cnt = nx_cnt;
@@ -1010,6 +1030,10 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                     // the epilogue must have read this set's previous contents (two groups back)
                     bool ok = mbar_wait<false, true>(smem_u32(&ctl->acc_empty[set]), set_phase ^ 1u, abort_flag,
                                                      4 | (int)(acc_it << 4));
+                    if (early) {
+                        pdl_enter();
+                        early = false;
+                    }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem + set * SET_COLS + t * COUT;
                     bool started = false;
@@ -1076,6 +1100,10 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                         const uint32_t j = q % NIDX;
                         const int code = list[e];
                         const int g = code >> 2, t = code & 3;
+                        if (early && q >= (uint32_t)NIDX) {
+                            pdl_enter();
+                            early = false;
+                        }
                         live = mbar_wait(smem_u32(&ctl->i_empty[j]), ((q / NIDX) & 1u) ^ 1u, abort_flag, 7 | (int)(q << 4));
                         if (live) {
                             // the map is tile-major with the block's own spacing between offsets: the stage's
@@ -1101,6 +1129,10 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 for (int g = 0; g < nstages; ++g) {
                     if (!active_tiles<KG>(m, g)) continue;
                     const uint32_t sb = my_b % B_STAGES;
+                    if (early && my_b >= B_STAGES) {
+                        pdl_enter();
+                        early = false;
+                    }
                     if (!mbar_wait(smem_u32(&ctl->b_empty[sb]), ((my_b / B_STAGES) & 1u) ^ 1u, abort_flag,
                                    8 | (int)(my_b << 4)))
                         break;

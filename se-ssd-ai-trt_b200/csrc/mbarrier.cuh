@@ -5,7 +5,9 @@
 
 namespace sessd {
 
-constexpr long long WAIT_LIMIT_CYCLES = 200000000LL;   // about a tenth of a second; real waits are microseconds
+// About a tenth of a second. Waits are microseconds: whoever waits for another role of its block is behind the wait for the
+// preceding kernel (which may run for any time) where that role is.
+constexpr long long WAIT_LIMIT_CYCLES = 200000000LL;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 

@@ -516,3 +516,30 @@ def test_empty_and_out_of_range_frames_inside_a_batch(gpu):
     # row counts), numbered differently
     assert dense[3].any()
     bb.close()
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("frames", [1, 8])
+def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dtype):
+    """Layers start while the kernel before them runs. One that takes twice the limit of their bounded waits (about 0.2 s) is put
+    before one layer after the other: no wait runs out, and the outputs are those of a call without it. In fp16 one frame goes
+    through the few-tiles path, and eight through groups of tiles in the layers at 1/2 and 1/4 resolution."""
+    import torch
+
+    w, sc, sh = gpu.random_weights()
+    bb = gpu.Backbone(60000, w, sc, sh, dtype=dtype)
+    pts = torch.stack([torch.from_numpy(gpu.synth.lidar_frame(40 + i, n_points=20000, n_boxes=15)) for i in range(frames)]).cuda()
+    sizes = torch.full((frames,), pts.shape[1], dtype=torch.int32, device="cuda")
+    dense, ws = bb.run(pts, sizes)
+    assert gpu.read_status(ws) == 0
+    want = dense.clone()
+    delay = gpu.lib().sessd_backbone_debug_delay
+    wide = [i for i, l in enumerate(bb.layers) if i > 0 and l.cin >= (32 if dtype == 0 else 16)]
+    for i in (wide[0], wide[2], wide[4], wide[-1]):
+        assert delay(bb.handle, i, 1) == 0
+        bb.run(pts, sizes, ws, dense)
+        assert delay(bb.handle, i, 0) == 0
+        assert gpu.read_status(ws) == 0, i
+        assert torch.equal(dense, want), i
+    assert delay(bb.handle, len(bb.layers), 1) < 0 and delay(None, 0, 1) < 0
+    bb.close()
