@@ -41,6 +41,7 @@ constexpr int F32_KVOL_MAX = 27;
 constexpr int F32_UNIT = 16;                 // rows of a register tile
 constexpr int F32_RT = F32_UNIT / 4;         // rows per thread
 constexpr int F32_STRIP = 8;                 // rows that are dealt out together (of one tile)
+constexpr int F32_FEW_FRAMES = 8;            // up to here a strip's frame is looked for frame by frame
 
 template <int CIN, int COUT>
 struct F32Shared {
@@ -127,8 +128,9 @@ __global__ void __launch_bounds__(F32_THREADS, 1) conv_f32_kernel(const __grid_c
     }
     if (warp == 0) {
         int strips = 0;
-        for (int f0 = 0; f0 < a.batch; f0 += 32)
-            strips += __reduce_add_sync(0xFFFFFFFFu, (f32_frame_rows(a, f0 + lane) + F32_STRIP - 1) / F32_STRIP);
+#pragma unroll 8
+        for (int f = lane; f < a.batch; f += 32) strips += (f32_frame_rows(a, f) + F32_STRIP - 1) / F32_STRIP;
+        strips = __reduce_add_sync(0xFFFFFFFFu, strips);
         if (lane == 0) s.strips = strips;
     }
     __syncthreads();
@@ -138,6 +140,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1) conv_f32_kernel(const __grid_c
     const int per_round = rounds > 0 ? (strips + grid * rounds - 1) / (grid * rounds) : 0;   // strips of a block
     const int rows_here = per_round * F32_STRIP;
     const int tiles_per_frame = (a.max_voxels + 127) / 128;
+    int at_frame = 0, at_strip = 0;                  // where the look-up of the present round's strips starts, and the strips before
     uint32_t used = 0;                               // weight blocks of the rounds so far
     uint32_t issued = 0;                             // weight streamer: blocks whose copy has been started
     for (int round = 0; round < rounds; ++round) {
@@ -147,14 +150,41 @@ __global__ void __launch_bounds__(F32_THREADS, 1) conv_f32_kernel(const __grid_c
         if (warp < S::STRIPS / 32 + (S::STRIPS % 32 ? 1 : 0)) {
             const int i = warp * 32 + lane;
             const int want = i < per_round ? (round * per_round + i) * grid + (int)blockIdx.x : INT32_MAX;
-            int frame = 0, row0 = 0, rows = 0, before = 0;
-            for (int f0 = 0; f0 < a.batch; f0 += 32) {
-                const int n = f32_frame_rows(a, f0 + lane);
-                for (int f = 0; f < 32 && f0 + f < a.batch; ++f) {
+            int frame = 0, row0 = 0, rows = 0;
+            if (a.batch <= F32_FEW_FRAMES) {
+                const int n = f32_frame_rows(a, lane);
+                int before = 0;
+                for (int f = 0; f < a.batch; ++f) {
                     const int nf = __shfl_sync(0xFFFFFFFFu, n, f), mine = (nf + F32_STRIP - 1) / F32_STRIP;
                     if (want >= before && want - before < mine)
-                        frame = f0 + f, row0 = (want - before) * F32_STRIP, rows = min(nf - row0, F32_STRIP);
+                        frame = f, row0 = (want - before) * F32_STRIP, rows = min(nf - row0, F32_STRIP);
                     before += mine;
+                }
+            } else if (warp * 32 < per_round) {
+                // 32 frames at a time, from where the round before found its last strip. (All frames one after the other, in every
+                // round: calls of 4,096 frames of 200 rows 4427 us, now 1381 (32 -> 32), and 8811 and 2697 (64 -> 64).)
+                const int last = __shfl_sync(0xFFFFFFFFu, want, min(per_round - warp * 32, 32) - 1);
+                int ahead = f32_frame_rows(a, at_frame + lane);
+                for (;;) {
+                    const int n = ahead, mine = (n + F32_STRIP - 1) / F32_STRIP;
+                    ahead = f32_frame_rows(a, at_frame + 32 + lane);
+                    int start = mine;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int v = __shfl_up_sync(0xFFFFFFFFu, start, d);
+                        if (lane >= d) start += v;
+                    }
+                    const int end = at_strip + __shfl_sync(0xFFFFFFFFu, start, 31);
+                    start += at_strip - mine;
+                    int src = 0;                     // the last of the frames that starts at or before the strip
+#pragma unroll
+                    for (int d = 16; d; d >>= 1)
+                        if (__shfl_sync(0xFFFFFFFFu, start, src + d) <= want) src += d;
+                    const int from = __shfl_sync(0xFFFFFFFFu, start, src), nf = __shfl_sync(0xFFFFFFFFu, n, src);
+                    if (want >= at_strip && want < end)
+                        frame = at_frame + src, row0 = (want - from) * F32_STRIP, rows = min(nf - row0, F32_STRIP);
+                    if (last < end || at_frame + 32 >= a.batch) break;
+                    at_frame += 32, at_strip = end;
                 }
             }
             if (i < S::STRIPS) {

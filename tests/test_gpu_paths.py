@@ -34,6 +34,71 @@ def test_fp32_blocks_of_rows(gpu, oracle, cin, cout, rows):
     _check_layer(gpu, oracle, layer, frames, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), maxV=rows + 5)
 
 
+@pytest.mark.parametrize("cin,cout", [(32, 32), (32, 64), (64, 64)])
+@pytest.mark.parametrize("frames", [8, 9, 33, 700])
+def test_fp32_rows_of_many_frames(gpu, oracle, frames, cin, cout):
+    """Up to eight frames a block looks its rows up frame by frame, beyond that 32 frames at a time, going on in each round (700
+    frames have two to four) where the last one ended. Frames of a few kinds, empty ones at the ends and in between: each has the
+    bits of a call on it alone, and two have the oracle's values."""
+    import torch
+
+    rs = np.random.RandomState(frames + cin + cout)
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (5, 16, 12))
+    W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
+    rows, maxV = [0, 1, 7, 8, 9, 130, 513, 257], 515
+    coors = [_random_coords(rs, n, layer.in_shape) for n in rows]
+    feats = [rs.randn(n, cin).astype(np.float32) for n in rows]
+    _check_layer(gpu, oracle, layer, [(coors[i], feats[i]) for i in (5, 6)], W, maxV=maxV)
+    p = gpu.conv_params(layer, maxV)
+    w = gpu.ConvWeights(p, W, None, None, False, 0)
+
+    def call(which):
+        c, x = np.zeros((len(which), maxV, 4), np.int32), np.zeros((len(which), maxV, cin), np.float32)
+        for b, i in enumerate(which):
+            c[b, :rows[i]], x[b, :rows[i]] = coors[i], feats[i]
+        r = gpu.subm_conv(torch.from_numpy(x).cuda(), torch.from_numpy(c).cuda(),
+                          torch.tensor([rows[i] for i in which], dtype=torch.int32).cuda(), p, w)
+        assert r["status"] == 0
+        return r["features"]
+
+    use = [0 if f in (0, frames - 1) else int(rs.randint(len(rows))) for f in range(frames)]
+    if frames == 700:
+        use[300:400] = [0] * 100          # more than 32 empty frames in a row
+    got, alone = call(use), [call([i])[0] for i in range(len(rows))]
+    for b, i in enumerate(use):
+        assert torch.equal(got[b], alone[i]), b
+    w.close()
+
+
+def test_fp32_rows_of_many_frames_cost_what_those_of_few_do(gpu):
+    """4,096 frames of a cluster of 40 rows and 5 frames of the same clusters far from one another: the same rows and pairs for
+    the convolution, which should take about as long (it took 4.4 times as long when every block looked its rows up
+    frame by frame)."""
+    import torch
+
+    rs = np.random.RandomState(2)
+    layer = _layer(gpu, True, 32, 32, (3, 3, 3), (1, 1, 1), (1, 1, 1), (5, 200, 200))
+    cluster = _random_coords(rs, 40, (5, 4, 4))
+    cluster = cluster[np.lexsort(cluster.T[::-1])]
+    at = np.stack(np.unravel_index(np.arange(820), (33, 33)), 1) * 6
+    field = np.repeat(cluster[None], 820, 0)
+    field[:, :, 2:] += at[:, None].astype(np.int32)
+    W = (rs.randn(27, 32, 32) * 0.05).astype(np.float32)
+    took = []
+    for frames, coors in ((4096, cluster), (5, field.reshape(-1, 4))):
+        n = len(coors)
+        p = gpu.conv_params(layer, n)
+        w = gpu.ConvWeights(p, W, None, None, False, 0)
+        args = (torch.randn((frames, n, 32), device="cuda"), torch.from_numpy(coors)[None].repeat(frames, 1, 1).cuda(),
+                torch.full((frames,), n, dtype=torch.int32, device="cuda"), p, w)
+        first = gpu.subm_conv(*args, keep_workspace=True)
+        assert first["status"] == 0
+        runs = [gpu.profile(lambda: gpu.subm_conv_into(*args, first["features"], first["workspace"])) for _ in range(8)]
+        took.append(min(ms for run in runs for name, ms in run if name.startswith("conv_f32")))
+        w.close()
+    assert took[0] < 1.4 * took[1] + 0.01, took
+
+
 @pytest.mark.parametrize("skip_in,skip_out", [(1, 0), (0, 2), (3, 1)])
 def test_fp32_rows_off_the_vector_alignment(gpu, skip_in, skip_out):
     """64 -> 32 channels from and to buffers that start a few floats off a 16-byte boundary: the bits of aligned ones. (All rows
