@@ -1009,64 +1009,100 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
             // arrivals must count for this use of the weight slot, not for an earlier one (a slot refilled while
             // an issuer has not yet tested its previous use would leave that issuer waiting on the wrong phase).
             // The schedule of the group is worked out once, lane g for stage g (which weight slot and phase, whether tile t takes
-            // part, which A slot its item sits in), and left in shared memory for one elected thread (always the same one: commits
-            // count the instructions of their own thread), which goes through it alone: as a warp that hands the schedule round with
-            // shuffles it is slower (64 -> 64, 4 x 120,000 points 152.7 us, so 147.7; front end of 8 x 120,000 1862 and 1837), and so it
-            // is when it looks at the next stage's barriers ahead of time.
+            // part, which A slot its item sits in). With 64 input channels it is left in shared memory for one elected thread, which
+            // goes through it alone; with fewer the warp goes through it together and hands it round with shuffles, and the elected
+            // lane issues (always the same one: commits count the instructions of their own thread). Calls, warp and thread, in us:
+            // 64 -> 64 32 x 120,000 points 1008 and 989, 32 x 20,000 378 and 369; 16 -> 32 1262 and 1295, 417 and 425; 32 -> 64
+            // 1327 and 1347, 411 and 417. Looking at the next stage's barriers ahead of time is slower for either.
             if (any) {
                 const int t = warp - EPI_WARPS;
-                {
-                    const uint32_t bits = lane < nstages ? active_tiles<KG>(m, lane) : 0u;
-                    int blocks_before = 0;
-                    const int items_before = items_before_stage(bits, lane, &blocks_before);
-                    const uint32_t pos = a_it + (uint32_t)items_before + (uint32_t)__popc(bits & ((1u << t) - 1u));
-                    const uint32_t my_b = b_it + (uint32_t)blocks_before;
-                    if (bits)
-                        ctl->issue[t][blocks_before] = (uint8_t)(((bits >> t) & 1u) | ((my_b % B_STAGES) << 1) | (((my_b / B_STAGES) & 1u) << 3) |
-                                                       ((pos % NSLOT) << 4));
-                }
-                __syncwarp();
-                if (leader) {
-                    // the epilogue must have read this set's previous contents (two groups back)
-                    bool ok = mbar_wait<false, true>(smem_u32(&ctl->acc_empty[set]), set_phase ^ 1u, abort_flag,
-                                                     4 | (int)(acc_it << 4));
+                const uint32_t bits = lane < nstages ? active_tiles<KG>(m, lane) : 0u;
+                int blocks_before = 0;
+                const int items_before = items_before_stage(bits, lane, &blocks_before);
+                const uint32_t pos = a_it + (uint32_t)items_before + (uint32_t)__popc(bits & ((1u << t) - 1u));
+                const uint32_t my_b = b_it + (uint32_t)blocks_before;
+                const uint32_t info = ((bits >> t) & 1u) | ((my_b % B_STAGES) << 1) | (((my_b / B_STAGES) & 1u) << 3) | ((pos % NSLOT) << 4);
+                const uint32_t d_tmem = tmem + set * SET_COLS + t * COUT;
+                bool started = false;
+                auto weights_landed = [&](uint32_t inf, int j) {
+                    return mbar_wait<false, true>(smem_u32(&ctl->b_full[(inf >> 1) & 3u]), (inf >> 3) & 1u, abort_flag,
+                                                  5 | (int)((b_it + j) << 4));
+                };
+                auto rows_landed = [&](uint32_t inf, int j) {   // the issuer's next use of the slot is the next phase
+                    const uint32_t sa = (inf >> 4) & 15u, phase = (full_phase >> sa) & 1u;
+                    full_phase ^= 1u << sa;
+                    return mbar_wait<false, true>(smem_u32(&ctl->a_full[t][sa]), phase, abort_flag, 6 | (int)((b_it + j) << 4));
+                };
+                auto issue = [&](uint32_t inf) {
+                    const uint32_t sb = (inf >> 1) & 3u, sa = (inf >> 4) & 15u;
+                    fence_proxy_async();       // the gathered rows were written through the generic proxy
+                    tc_fence_after();
+                    const uint64_t adesc = umma_desc(smem_u32(sA + sa * A_BYTES));
+                    const uint64_t bdesc = umma_desc(smem_u32(sB + sb * B_BYTES));
+#pragma unroll
+                    for (int kk = 0; kk < 4; ++kk)
+                        umma_f16(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (started || kk > 0) ? 1u : 0u);
+                    umma_commit(smem_u32(&ctl->a_empty[sa]));   // frees the A slot once these MMAs have read it
+                    umma_commit(smem_u32(&ctl->b_empty[sb]));   // and this issuer's hold on the weight block
+                };
+                auto pass = [&](uint32_t inf) { mbar_arrive(smem_u32(&ctl->b_empty[(inf >> 1) & 3u])); };   // nothing to read from this block
+                // the epilogue must have read this set's previous contents (two groups back)
+                auto set_free = [&]() {
+                    return mbar_wait<false, true>(smem_u32(&ctl->acc_empty[set]), set_phase ^ 1u, abort_flag, 4 | (int)(acc_it << 4));
+                };
+                auto report = [&]() {
+                    if (started) umma_commit(smem_u32(&ctl->acc_full[set]));
+                    else mbar_arrive(smem_u32(&ctl->acc_full[set]));
+                };
+                if constexpr (CIN == 64) {
+                    if (bits) ctl->issue[t][blocks_before] = (uint8_t)info;
+                    __syncwarp();
+                    if (leader) {
+                        bool ok = set_free();
+                        if (early) {
+                            pdl_enter();
+                            early = false;
+                        }
+                        tc_fence_after();
+#pragma unroll 2
+                        for (int j = 0; j < n_b; ++j) {
+                            if (!ok) break;
+                            const uint32_t inf = ctl->issue[t][j];
+                            ok = weights_landed(inf, j);
+                            if (!ok) break;
+                            if (inf & 1u) {
+                                ok = rows_landed(inf, j);
+                                if (!ok) break;
+                                issue(inf);
+                                started = true;
+                            } else {
+                                pass(inf);
+                            }
+                        }
+                        if (ok) report();
+                    }
+                } else {
+                    bool ok = __all_sync(0xFFFFFFFFu, set_free());
                     if (early) {
                         pdl_enter();
                         early = false;
                     }
                     tc_fence_after();
-                    const uint32_t d_tmem = tmem + set * SET_COLS + t * COUT;
-                    bool started = false;
-#pragma unroll 2
-                    for (int j = 0; j < n_b; ++j) {
-                        if (!ok) break;
-                        const uint32_t inf = ctl->issue[t][j];
-                        const uint32_t sb = (inf >> 1) & 3u, sa = (inf >> 4) & 15u;
-                        ok = mbar_wait<false, true>(smem_u32(&ctl->b_full[sb]), (inf >> 3) & 1u, abort_flag, 5 | (int)((b_it + j) << 4));
+                    uint32_t left = __ballot_sync(0xFFFFFFFFu, bits != 0u);
+                    for (int j = 0; left && ok; ++j, left &= left - 1u) {
+                        const uint32_t inf = __shfl_sync(0xFFFFFFFFu, info, __ffs((int)left) - 1);
+                        ok = weights_landed(inf, j);
+                        if (inf & 1u) ok = ok && rows_landed(inf, j);
+                        ok = __all_sync(0xFFFFFFFFu, ok);
                         if (!ok) break;
                         if (inf & 1u) {
-                            ok = mbar_wait<false, true>(smem_u32(&ctl->a_full[t][sa]), (full_phase >> sa) & 1u, abort_flag,
-                                                        6 | (int)((b_it + j) << 4));
-                            if (!ok) break;
-                            full_phase ^= 1u << sa;   // this issuer's next use of the slot is the next phase
-                            fence_proxy_async();   // the gathered rows were written through the generic proxy
-                            tc_fence_after();
-                            const uint64_t adesc = umma_desc(smem_u32(sA + sa * A_BYTES));
-                            const uint64_t bdesc = umma_desc(smem_u32(sB + sb * B_BYTES));
-#pragma unroll
-                            for (int kk = 0; kk < 4; ++kk)
-                                umma_f16(d_tmem, adesc + 2 * kk, bdesc + 2 * kk, IDESC, (started || kk > 0) ? 1u : 0u);
-                            umma_commit(smem_u32(&ctl->a_empty[sa]));   // frees the A slot once these MMAs have read it
-                            umma_commit(smem_u32(&ctl->b_empty[sb]));   // and this issuer's hold on the weight block
+                            if (leader) issue(inf);
                             started = true;
-                        } else {
-                            mbar_arrive(smem_u32(&ctl->b_empty[sb]));   // nothing to read from this weight block
+                        } else if (leader) {
+                            pass(inf);
                         }
                     }
-                    if (ok) {
-                        if (started) umma_commit(smem_u32(&ctl->acc_full[set]));
-                        else mbar_arrive(smem_u32(&ctl->acc_full[set]));
-                    }
+                    if (ok && leader) report();
                 }
             }
             __syncwarp();
