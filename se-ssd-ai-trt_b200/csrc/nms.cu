@@ -210,11 +210,15 @@ nms_rank_kernel(NmsArgs a, uint32_t* status) {
 // loads. All threads write the kept boxes in rank order, a float each, and the zeros after them. (From every kept box to the next, rows
 // fetched and copied by a thread per box: 20 us for both parts of this kernel on a frame of 300 boxes, now 18; filter and NMS of
 // 4 frames 71.1 us and 68.2, the detector's graph 446.8 and 444.1. The pass is half of the kernel.)
+// Beside a staged mask the ranks' input rows wait in registers until the walk is over and the mask's memory free: with 4 KB of their
+// own the blocks leave the pairs' local arrays less L1 (16 frames of 500 boxes on 10 objects 246 us, so 228).
 constexpr int kMaskWarps = 8, kMaskThreads = kMaskWarps * 32;
+constexpr int kStagedBoxes = 568;   // per frame, whose mask is staged: 40 KB
 __device__ void greedy_pass(const NmsArgs& a, int b, int n, unsigned long long* s_mask, int smem_words) {
     __shared__ unsigned long long s_keep[32];
     __shared__ int s_base[33];
-    __shared__ uint16_t s_order[kMaxBoxes];      // input row of a rank, then of a kept row
+    uint16_t* s_order = reinterpret_cast<uint16_t*>(s_mask);   // where no mask is staged, or no more: input row of a rank, then of a kept row
+    const bool staged = smem_words > 0;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int words_n = (n + 63) >> 6;
     const float* bx = a.boxes + (size_t)b * a.max_box * 9;
@@ -222,14 +226,22 @@ __device__ void greedy_pass(const NmsArgs& a, int b, int n, unsigned long long* 
     const unsigned long long* mask = a.mask + (size_t)b * a.max_box * a.words;
     int stride = a.words;
     // (requested together: the input rows of a thread's ranks and their part of the mask)
+    int held[kStagedBoxes / kMaskThreads + 1];
+#pragma unroll
+    for (int q = 0; q <= kStagedBoxes / kMaskThreads; ++q) {
+        const int i = q * kMaskThreads + threadIdx.x;
+        held[q] = staged && i < n ? a.order[(size_t)b * a.max_box + i] : 0;
+    }
     for (int i = threadIdx.x; i < n; i += kMaskThreads) {
-        s_order[i] = (uint16_t)a.order[(size_t)b * a.max_box + i];
-        if (n * words_n > smem_words) continue;
+        if (!staged) {
+            s_order[i] = (uint16_t)a.order[(size_t)b * a.max_box + i];
+            continue;
+        }
         // only words from the one that holds the row itself onward are ever written or read
 #pragma unroll 4
         for (int w = i >> 6; w < words_n; ++w) s_mask[i * words_n + w] = mask[(size_t)i * a.words + w];
     }
-    if (n * words_n <= smem_words) {
+    if (staged) {
         mask = s_mask;
         stride = words_n;
     }
@@ -290,7 +302,8 @@ __device__ void greedy_pass(const NmsArgs& a, int b, int n, unsigned long long* 
 #pragma unroll
     for (int q = 0; q < kMaxBoxes / kMaskThreads; ++q) {
         const int i = q * kMaskThreads + threadIdx.x;
-        src[q] = i < n ? s_order[i] : 0;
+        src[q] = i < n && !staged ? s_order[i] : 0;
+        if (staged && q <= kStagedBoxes / kMaskThreads) src[q] = held[q];
     }
     __syncthreads();
 #pragma unroll
@@ -301,10 +314,11 @@ __device__ void greedy_pass(const NmsArgs& a, int b, int n, unsigned long long* 
         if ((kw >> (i & 63)) & 1ull) s_order[s_base[i >> 6] + __popcll(kw & ((1ull << (i & 63)) - 1ull))] = (uint16_t)min(src[q], n - 1);
     }
     __syncthreads();
-    for (int e = threadIdx.x; e < a.max_box * 9; e += kMaskThreads) {
+    for (int e = threadIdx.x; e < total * 9; e += kMaskThreads) {
         const int pos = e / 9;
-        out[e] = pos < total ? bx[(size_t)s_order[pos] * 9 + (e - pos * 9)] : 0.f;
+        out[e] = bx[(size_t)s_order[pos] * 9 + (e - pos * 9)];
     }
+    for (int e = total * 9 + threadIdx.x; e < a.max_box * 9; e += kMaskThreads) out[e] = 0.f;
     if (threadIdx.x == 0) a.kept_num[b] = (uint32_t)total;
 }
 
@@ -411,8 +425,8 @@ int sessd_rotated_nms_enqueue(const sessd_nms_params* p, int batch, const void* 
     const int rank_grid = (batch < persistent_grid(1) ? batch : persistent_grid(1)) * kRankBlocks;
     SESSD_LAUNCH(nms_rank_kernel, rank_grid, kThreads, M * sizeof(float), stream, a, static_cast<uint32_t*>(workspace));
     // the staged copy of a frame's mask must fit the 48 KB a block gets without opting in; larger tables are read in place
-    const size_t stage_bytes = M * words * sizeof(unsigned long long);
-    const int smem_words = stage_bytes <= 40 * 1024 ? (int)(M * words) : 0;
+    const int smem_words = M <= kStagedBoxes ? (int)(M * words) : 0;
+    const size_t smem_bytes = smem_words ? smem_words * sizeof(unsigned long long) : M * sizeof(uint16_t);
     // A warp per (box, segment) of a full frame, unless the frames of the batch have to share the GPU: then a frame's part of the
     // blocks that are resident. Where that is a few blocks with much to do, the parts do not fill the GPU and frames differ: four
     // times as many blocks then (500 boxes, random and all overlapping, us: 16 frames 128 and 329 with one round of blocks, 136 and
@@ -421,8 +435,7 @@ int sessd_rotated_nms_enqueue(const sessd_nms_params* p, int batch, const void* 
     int blocks_per_frame = resident / batch > 1 ? resident / batch : 1;
     if (blocks_per_frame < 16 && full / blocks_per_frame >= 64) blocks_per_frame = 4 * resident / batch > 1 ? 4 * resident / batch : 1;
     if (blocks_per_frame > full) blocks_per_frame = full;
-    SESSD_LAUNCH(nms_mask_kernel, batch * blocks_per_frame, kMaskThreads, (size_t)smem_words * sizeof(unsigned long long), stream,
-                 a, blocks_per_frame, smem_words);
+    SESSD_LAUNCH(nms_mask_kernel, batch * blocks_per_frame, kMaskThreads, smem_bytes, stream, a, blocks_per_frame, smem_words);
     return SESSD_OK;
 }
 

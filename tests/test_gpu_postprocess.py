@@ -214,6 +214,29 @@ def test_rotated_nms_table_larger_than_the_staged_copy(gpu, oracle):
         assert not kept[b, len(want):].any()
 
 
+@pytest.mark.parametrize("max_box,n", [(1, 1), (64, 64), (65, 65), (568, 568), (569, 569), (2048, 2048), (2048, 3), (2048, 0)])
+def test_rotated_nms_kept_rows_and_the_zeros_after_them(gpu, max_box, n):
+    """Up to 568 boxes the mask is staged. Boxes apart from one another, every second one twice in the same place: of those the
+    one with the lower score goes, the others come in the order of their scores, the rest of the table is zero."""
+    import torch
+
+    rs = np.random.RandomState(max_box + n)
+    boxes = np.full((2, max_box, 9), 3.0, np.float32)
+    for b in range(2):
+        spot = np.arange(n) // 2
+        boxes[b, :n, 0], boxes[b, :n, 1] = spot % 40 * 9, spot // 40 * 9
+        boxes[b, :n, 2:8] = np.array([-1, 1.6, 3.9, 1.5, 0.3, 0], np.float32)
+        boxes[b, :n, 8] = rs.permutation(n)
+        boxes[b, :n] = boxes[b, rs.permutation(n)]
+    kept, num = gpu.rotated_nms(torch.from_numpy(boxes).cuda(), torch.full((2,), n, dtype=torch.int32, device="cuda"), 0.1)
+    for b in range(2):
+        ranked = boxes[b, :n][np.argsort(-boxes[b, :n, 8], kind="stable")]
+        first = np.sort(np.unique(ranked[:, :2], axis=0, return_index=True)[1]) if n else np.zeros(0, int)
+        assert int(num[b]) == len(first) == (n + 1) // 2
+        np.testing.assert_array_equal(kept[b, :len(first)].cpu().numpy(), ranked[first])
+        assert not kept[b, len(first):].any()
+
+
 def test_rotated_nms_after_score_filter(gpu, oracle):
     """Score filter -> NMS on the device, the reference's post-processing chain (se-ssd-ai-trt.cpp:1868-1892)."""
     S = gpu.schedule
