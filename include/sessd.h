@@ -391,10 +391,10 @@ int sessd_read_status2(const void* workspace, const void* other, void* stream);
 const char* sessd_last_cuda_error(void);
 /* Library version string. */
 const char* sessd_version(void);
-/* Test hook for the time-out path, per weight object, off by default: while on, the tensor-core convolution
- * kernel launched with these weights keeps its weight streamer silent, so the kernel's bounded waits run out (about
- * 0.1 s), every block leaves through its abort path, the call returns SESSD_OK and the status word carries
- * SESSD_STATUS_TIMEOUT with the code of the wait in the second status word. Nothing faults or hangs; other weight
+/* Test hook for the time-out path, per weight object, off by default: while on, a convolution kernel that streams its
+ * weights (fp16 with 16, 32 or 64 channels, fp32 with 32 or 64) and is launched with these does not ask for them, so that its
+ * bounded waits run out (about 0.1 s), every block leaves through its abort path, the call returns SESSD_OK and the status word
+ * carries SESSD_STATUS_TIMEOUT with the code of the wait in the second status word. Nothing faults or hangs; other weight
  * objects and the next call with the hook off are not affected. */
 int sessd_conv_weights_debug_withhold(sessd_conv_weights* w, int on);
 /* Test hook, per backbone and layer, off by default: while on, a kernel of one block that does nothing for about 0.2 s runs

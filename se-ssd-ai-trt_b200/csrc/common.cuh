@@ -406,7 +406,7 @@ struct ConvLaunch {
     int32_t* status;       // device status word (tensor-core path reports wait timeouts there)
     int* tile_counter;     // tensor-core path: zero before the launch; hands out the tiles of small layers (null: it never does)
     int maps_ready;        // neighbour map, masks and row counts are older than the kernel launched just before
-    int debug_withhold_weights;   // tests only: the tensor-core kernel's weight streamer stays silent (waits run out)
+    int debug_withhold_weights;   // tests only: whoever streams the weights stays silent (waits run out)
     const float* scale_host;      // [Cout <= 64] host copies of scale / shift (ones / zeros without batch norm), or null
     const float* shift_host;
 };
@@ -486,7 +486,7 @@ struct sessd_conv_weights_impl {
     float* scale;   // device or null
     float* shift;   // device or null
     int relu, dtype, kvol, cin, cout;
-    int debug_withhold;   // tests of the time-out path: the tensor-core kernel's weight streamer stays silent
+    int debug_withhold;   // tests of the time-out path: whoever streams the weights stays silent
     // host copies of scale and shift (ones and zeros without batch norm) for kernels that take them as launch
     // parameters; filled for out_channel <= 64
     float host_scale[64], host_shift[64];

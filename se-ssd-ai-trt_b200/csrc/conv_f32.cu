@@ -77,7 +77,7 @@ struct F32Args {
     const int4* out_coors;
     int D, H, W;
     int32_t* status;
-    int maps_ready;
+    int maps_ready, withhold_weights;   // withhold_weights: tests of the time-out path only
 };
 
 __device__ __forceinline__ void copy_16(void* dst, const void* src) {
@@ -248,7 +248,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1) conv_f32_kernel(const __grid_c
 
         if (warp == F32_WARPS) {
             // ---- weight streamer ----
-            uint32_t m = present, old = present;     // old: the offset whose block a stage held
+            uint32_t m = a.withhold_weights ? 0u : present, old = present;   // old: the offset whose block a stage held
             for (int q = 0; m; m &= m - 1u, ++q) {
                 const uint32_t at = used + (uint32_t)q, st = at % STAGES;
                 if (q >= STAGES) {
@@ -415,7 +415,8 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
     }
     const F32Args a{static_cast<const float*>(c.in), static_cast<float*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                     static_cast<const float*>(c.weights), c.scale, c.shift, c.relu, c.batch, c.max_voxels, c.kvol,
-                    static_cast<float*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W, c.status, c.maps_ready};
+                    static_cast<float*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W, c.status, c.maps_ready,
+                    c.debug_withhold_weights};
     SESSD_LAUNCH_NAMED(name.c_str(), (conv_f32_kernel<CIN, COUT>), persistent_grid(1), F32_THREADS, smem, stream, a);
     return SESSD_OK;
 }

@@ -612,8 +612,9 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     // Whatever does not depend on the preceding kernel comes before the wait for it. maps_ready: neighbour map, masks and
     // row counts are older than that kernel.
     if (!maps_ready) pdl_enter();
-    // withhold_weights (tests of the time-out path only): the weight streamer stays silent, so the MMA issuers'
-    // bounded wait for the first weight block runs out and every CTA with work leaves through the abort path.
+    // withhold_weights (tests of the time-out path only): the weight streamer stays silent, or the gather warps that ask for the
+    // weights in the few-tiles path do, so the MMA issuers' bounded wait for the first weight block runs out and every CTA
+    // with work leaves through the abort path.
     constexpr int KG = 64 / CIN;            // kernel offsets sharing one 128-byte A row
     constexpr int CPO = CIN / 8;            // 16-byte chunks per offset
     constexpr int B_BYTES = COUT * ROW_BYTES;

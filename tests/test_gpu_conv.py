@@ -248,40 +248,46 @@ def test_bad_coordinate_is_reported_not_dereferenced(gpu):
     assert res[0]["status"] & gpu.STATUS_BAD_COORD
 
 
-@pytest.mark.parametrize("cin,cout", [(32, 32), (64, 64)])
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 64), (64, 64)])
 def test_more_row_groups_than_resident_blocks_fp16(gpu, oracle, cin, cout):
-    """4 frames x 45,000 rows: 352 groups of 512 rows, more than a persistent grid holds at once, so blocks
-    walk through several groups and their staging rings wrap many times."""
+    """5 frames of 30,001 to 50,000 rows: more than ten tiles per SM, so that the kernel works in groups of four tiles; blocks walk
+    through several groups and their staging rings wrap many times."""
+    import torch
+
     rs = np.random.RandomState(77 + cin)
     shape = (10, 200, 176)
     frames = []
-    for n in (45000, 44000, 45000, 30001):
+    for n in (50000, 44000, 45000, 30001, 45000):
         c = _random_coords(rs, n, shape)
         frames.append((c, rs.randn(len(c), cin).astype(np.float32)))
+    assert sum((len(c) + 127) // 128 for c, _ in frames) > 10 * torch.cuda.get_device_properties(0).multi_processor_count
     W = (rs.randn(27, cin, cout) / np.sqrt(5 * cin)).astype(np.float32)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
-    _check_layer(gpu, oracle, layer, frames, W, dtype=gpu.F16, maxV=45056)
+    _check_layer(gpu, oracle, layer, frames, W, dtype=gpu.F16, maxV=50048)
 
 
-def test_bounded_waits_run_out_report_and_leave_the_context_usable(gpu):
-    """Time-out path of the tensor-core kernel, made on the host: with the library's test hook on, the kernel's
-    weight streamer stays silent, the MMA issuers' bounded wait for the first weight block runs out, every block
-    leaves through its abort path and the call reports SESSD_STATUS_TIMEOUT with the code of that wait. Nothing
-    faults; the same call with the hook off then gives the result it gave before."""
+@pytest.mark.parametrize("dtype,cin,cout,n", [(1, 32, 32, 3000), (1, 32, 32, 195000), (1, 64, 64, 195000), (0, 32, 32, 3000), (0, 64, 64, 60000)])
+def test_bounded_waits_run_out_report_and_leave_the_context_usable(gpu, dtype, cin, cout, n):
+    """Time-out path of the kernels that stream their weights, made on the host: with the library's test hook on, nobody asks
+    for weights, the bounded waits for the first block run out, every block leaves through its abort path and the call
+    reports SESSD_STATUS_TIMEOUT with the code of that wait. Nothing faults; the same call with the hook off then gives the
+    result it gave before. fp16: the few-tiles path, and groups (more than ten tiles per SM) with either kind of issuer; fp32: one
+    round of rows, and three."""
     import torch
 
     rs = np.random.RandomState(5)
-    shape, cin, cout, n, maxV = (10, 60, 60), 32, 32, 3000, 4096
+    shape = (10, 60, 60) if n < 36000 else (10, 200, 176)
+    maxV = n + 1096
     c = _random_coords(rs, n, shape)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
-    feat = np.zeros((1, maxV, cin), np.float16)
+    feat = np.zeros((1, maxV, cin), np.float16 if dtype else np.float32)
     coors = np.zeros((1, maxV, 4), np.int32)
-    feat[0, :len(c)] = rs.randn(len(c), cin).astype(np.float16)
+    feat[0, :len(c)] = rs.randn(len(c), cin)
     coors[0, :len(c)] = c
     coors[0, :, 0] = 0
     W = (rs.randn(27, cin, cout) / np.sqrt(5 * cin)).astype(np.float32)
     p = gpu.conv_params(layer, maxV)
-    w = gpu.ConvWeights(p, W, None, None, False, gpu.F16)
+    w = gpu.ConvWeights(p, W, None, None, False, dtype)
     tf, tc = torch.from_numpy(feat).cuda(), torch.from_numpy(coors).cuda()
     tn = torch.tensor([len(c)], dtype=torch.int32, device="cuda")
     good = gpu.subm_conv(tf, tc, tn, p, w)
@@ -294,7 +300,7 @@ def test_bounded_waits_run_out_report_and_leave_the_context_usable(gpu):
         gpu.lib().sessd_conv_weights_debug_withhold(w.handle, 0)
     assert r["status"] & gpu.STATUS_TIMEOUT
     where = int(r["workspace"][4:8].view(torch.int32)[0])
-    assert where & 15 == 5                    # an MMA issuer waiting for a weight block
+    assert where & 15 == (5 if dtype else 10)   # an MMA issuer, or a warp with a unit of rows, waiting for a weight block
     again = gpu.subm_conv(tf, tc, tn, p, w)
     assert again["status"] == 0 and torch.equal(again["features"], want)
     w.close()

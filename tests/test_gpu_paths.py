@@ -14,7 +14,8 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("cin,cout,rows", [(64, 32, 300), (32, 64, 17760), (32, 64, 17761)])
 def test_fp32_register_tiles(gpu, oracle, cin, cout, rows):
-    """64 -> 32 channels; strips of 8 rows while every warp of the GPU gets one (148 SMs x 15 warps x 8 rows), of 16 above."""
+    """64 -> 32 channels with a few strips for the whole GPU; 32 -> 64 with half a round of rows, and one row more than whole tiles
+    and strips."""
     rs = np.random.RandomState(rows)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
     c = _random_coords(rs, rows, layer.in_shape)
@@ -22,10 +23,11 @@ def test_fp32_register_tiles(gpu, oracle, cin, cout, rows):
     _check_layer(gpu, oracle, layer, [(c, f)], (rs.randn(27, cin, cout) * 0.05).astype(np.float32), maxV=rows + 5)
 
 
-@pytest.mark.parametrize("cin,cout,rows", [(64, 64, 28416), (64, 64, 28417), (32, 32, 56841), (64, 32, 37889), (32, 64, 9), (64, 64, 1)])
+@pytest.mark.parametrize("cin,cout,rows", [(64, 64, 28416), (64, 64, 28417), (64, 64, 56833), (32, 32, 56841), (64, 32, 37889),
+                                           (32, 64, 37888), (32, 64, 37889), (32, 64, 9), (64, 64, 1)])
 def test_fp32_blocks_of_rows(gpu, oracle, cin, cout, rows):
-    """148 blocks of 192 (64 -> 64), 256 (64 -> 32 and 32 -> 64) or 384 rows (32 -> 32) in one round, and rows that need a second;
-    fewer rows than a strip or a unit has."""
+    """148 blocks of 192 (64 -> 64), 256 (64 -> 32 and 32 -> 64) or 384 rows (32 -> 32) in one round, and rows that need a second,
+    or a third, in which the offsets' barriers are back at their first parity; fewer rows than a strip or a unit has."""
     rs = np.random.RandomState(rows)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (14, 110, 70))
     frames = [(c, rs.randn(len(c), cin).astype(np.float32)) for c in (_random_coords(rs, rows, layer.in_shape),)]
@@ -168,9 +170,9 @@ def test_strided_maps_through_a_table_and_by_input_rows(gpu, fp16):
 
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 64), (64, 64)])
 @pytest.mark.parametrize("extra", [0, 1])
-def test_fp16_tiles_on_both_sides_of_the_few(gpu, cin, cout, extra):
+def test_fp16_tiles_on_both_sides_of_the_few(gpu, oracle, cin, cout, extra):
     """Ten tiles per SM are the most that the few-tiles path takes, one more goes through groups of four. Every frame has the bits of
-    a call on it alone (about one tile per SM, the size that other tests compare with the oracle)."""
+    a call on it alone (211 or 212 tiles, through the few-tiles path), and the first of those has the oracle's values."""
     import torch
 
     rs = np.random.RandomState(cin + cout)
@@ -183,9 +185,13 @@ def test_fp16_tiles_on_both_sides_of_the_few(gpu, cin, cout, extra):
     feat = torch.from_numpy(rs.randn(frames, V, cin).astype(np.float16)).cuda()
     num = torch.tensor(rows, dtype=torch.int32, device="cuda")
     p = gpu.conv_params(layer, V)
-    w = gpu.ConvWeights(p, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), None, None, True, 1)
+    W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
+    w = gpu.ConvWeights(p, W, None, None, True, 1)
     r = gpu.subm_conv(feat, coors, num, p, w)
     assert r["status"] == 0
+    if extra == 0:
+        first = coors[0, :rows[0]].cpu().numpy(), feat[0, :rows[0]].float().cpu().numpy()
+        _check_layer(gpu, oracle, layer, [first], W, relu=True, dtype=1, maxV=V)
     for b in range(frames):
         alone = gpu.subm_conv(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
         assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
@@ -246,17 +252,17 @@ def test_few_fp16_tiles_some_without_neighbours(gpu):
 
 
 @pytest.mark.parametrize("cin,cout", [(16, 32), (64, 64)])
-@pytest.mark.parametrize("frames", [8, 9, 40, 130])
-def test_fp16_work_split_over_frames(gpu, oracle, frames, cin, cout):
-    """More than one tile per SM in up to eight frames, and in more (the work is then cut with the frames' first tiles in shared
-    memory): one, two and seven tiles per thread of the cut, with empty frames at the ends and in between. Every frame has the
+@pytest.mark.parametrize("frames,most", [(8, 56301), (9, 56301), (40, 9301), (130, 6301)])
+def test_fp16_work_split_over_frames(gpu, oracle, frames, most, cin, cout):
+    """More than ten tiles per SM in up to eight frames, and in more (the work is then cut with the frames' first tiles in shared
+    memory): three to seven tiles per thread of the cut, with empty frames at the ends and in between. Every frame has the
     bits of a call on it alone, and the first has the oracle's values."""
     import torch
 
     rs = np.random.RandomState(frames + cin)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
     W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
-    rows, maxV = [6000, 1, 6000, 128, 5800, 6301], 6301
+    rows, maxV = [most - 301, 1, most - 301, 128, most - 501, most], most
     coors = [_random_coords(rs, n, layer.in_shape) for n in rows]
     feats = [rs.randn(n, cin).astype(np.float32) for n in rows]
     _check_layer(gpu, oracle, layer, [(coors[0], feats[0])], W, dtype=1, maxV=maxV)
@@ -276,7 +282,7 @@ def test_fp16_work_split_over_frames(gpu, oracle, frames, cin, cout):
         return r["features"], sum((v + 127) // 128 for v in n)
 
     got, tiles = call(use)
-    assert tiles > 148
+    assert tiles > 10 * torch.cuda.get_device_properties(0).multi_processor_count
     alone = [call([i])[0][0] for i in range(len(rows))]
     for b, i in enumerate(use):
         assert not got[b].any() if i is None else torch.equal(got[b], alone[i]), b
@@ -329,9 +335,10 @@ def test_tables_with_every_row_in_use(gpu, oracle, rows, subm):
 
 @pytest.mark.parametrize("K,S,P", [((3, 3, 3), (2, 2, 2), (1, 1, 1)), ((3, 3, 3), (2, 2, 2), (0, 2, 2)), ((3, 1, 1), (2, 1, 1), (0, 0, 0)),
                                    ((1, 2, 3), (1, 1, 1), (0, 1, 2)), ((2, 3, 1), (3, 2, 3), (1, 2, 0)), ((3, 3, 3), (1, 3, 2), (1, 0, 2))])
-@pytest.mark.parametrize("edge", [1448, 1449])
-def test_strided_maps_by_inputs_and_through_a_table(gpu, oracle, edge, K, S, P):
-    """Grids of 16 x 1448 x 1448 cells (just under 2^25) and 16 x 1449 x 1449 (just over): maps through a table, and by input rows."""
+@pytest.mark.parametrize("edge,room", [(1448, 166667), (1449, 0), (1449, 166667)])
+def test_strided_maps_by_inputs_and_through_a_table(gpu, oracle, edge, room, K, S, P):
+    """Grids of 16 x 1448 x 1448 cells (just under 2^25) and 16 x 1449 x 1449 (just over): maps through a table, and on the finer
+    grid by input rows where three frames have room for more than 500,000 rows."""
     rs = np.random.RandomState(3)
     layer = _layer(gpu, False, 16, 32, K, S, P, (16, edge, edge))
     c = np.concatenate([_random_coords(rs, 200, (16, 20, 30)), _random_coords(rs, 150, layer.in_shape)])
@@ -339,12 +346,13 @@ def test_strided_maps_by_inputs_and_through_a_table(gpu, oracle, edge, K, S, P):
     c = rs.permutation(c)
     f = rs.randn(len(c), 16).astype(np.float32)
     W = (rs.randn(int(np.prod(K)), 16, 32) * 0.1).astype(np.float32)
-    _check_layer(gpu, oracle, layer, [(c, f), (c[:131], f[:131]), (c[:0], f[:0])], W, maxV=len(c) * 27)
+    _check_layer(gpu, oracle, layer, [(c, f), (c[:131], f[:131]), (c[:0], f[:0])], W, maxV=max(room, len(c) * 27))
 
 
-@pytest.mark.parametrize("edge", [1448, 1449])
-def test_strided_rows_outside_the_grid_and_of_the_same_cell(gpu, edge):
-    """Rows outside reach nothing; of two rows of a cell the later one counts. Both ways of making the map."""
+@pytest.mark.parametrize("edge,room", [(1448, 500001), (1449, 3000), (1449, 500001)])
+def test_strided_rows_outside_the_grid_and_of_the_same_cell(gpu, edge, room):
+    """Rows outside reach nothing; of two rows of a cell the later one counts. Both ways of making the map: by input rows on the
+    finer grid with room for more than 500,000 rows."""
     import torch
 
     rs = np.random.RandomState(8)
@@ -354,11 +362,11 @@ def test_strided_rows_outside_the_grid_and_of_the_same_cell(gpu, edge):
     extra = np.array([[0, -1, 3, 3], [0, 16, 3, 3], [0, 3, -2, 3], [0, 3, edge, 3], [0, 3, 3, -1], [0, 3, 3, edge + 5]], np.int32)
     stale = rs.randn(300 + len(extra), 16).astype(np.float32)
     W = (rs.randn(27, 16, 32) * 0.1).astype(np.float32)
-    p = gpu.conv_params(layer, 3000)
+    p = gpu.conv_params(layer, room)
     w = gpu.ConvWeights(p, W, None, None, False, 0)
 
     def call(coors, feat):
-        x, co = np.zeros((1, 3000, 16), np.float32), np.zeros((1, 3000, 4), np.int32)
+        x, co = np.zeros((1, room, 16), np.float32), np.zeros((1, room, 4), np.int32)
         x[0, :len(feat)], co[0, :len(coors)] = feat, coors
         r = gpu.sparse_conv(torch.from_numpy(x).cuda(), torch.from_numpy(co).cuda(), torch.tensor([len(coors)], dtype=torch.int32).cuda(), p, w)
         assert r["status"] == 0
