@@ -8,9 +8,9 @@
 // shared memory hands to registers. A thread that owns one output row and reads a weight vector per channel and row is
 // bound by those reads (3 TFLOP/s). Hence this shape:
 //   - a block (one per SM) owns up to ROWS output rows, eight by eight from all over the map, so that blocks get alike shares
-//     although the map's rows are ordered by their neighbours. Per offset it lists the rows that have the neighbour, and its warps
-//     take sixteen of a list at a time, offset by offset, each warp the next sixteen that nobody has: rows without the neighbour cost
-//     nothing, and every warp is busy whatever the offsets' lists look like;
+//     although the map's rows are ordered by their neighbours. Per offset it lists the rows that have the neighbour, and sixteen of a
+//     list at a time, offset by offset, go to its warps in turn: rows without the neighbour cost nothing, and a warp that is early
+//     waits to add its sums until the offset before has all of its own;
 //   - sixteen rows are a register tile, 4 rows x 8 (or 4) channels per thread; their sums under the offset are added to the rows'
 //     sums in shared memory once all of the offset before have been: ascending offsets, whichever warps they fall to;
 //   - the input rows of a warp's next sixteen are copied in while the current ones are worked on;
@@ -24,9 +24,11 @@
 // issue slots that the same kernel was no faster than one strip of rows per warp.
 // Measured against that (a warp took sixteen rows through all offsets, rows without the neighbour included): front end of a
 // 20,000-point frame 1003 us, now 809 (64->64 at 1/4 resolution, 26,400 rows, 125 us a layer, now 112; at 1/8, 11,300 rows, 67 and 57;
-// 32->64 between 1/2 and 1/4 71 and 38), of 3,000 points 531 and 420, of 2 x 40,000 2551 and 2238; calls of 4 x 120,000 points, 32->32 1157 and 1073, 64->64
-// 1471 and 1450. The fp32 pipe is then busy half of the time; a quarter of its instructions make the operand pairs, but scalar
-// multiply-adds are slower still (issue slots).
+// 32->64 between 1/2 and 1/4 71 and 38), of 3,000 points 531 and 420, of 2 x 40,000 2551 and 2238; calls of 4 x 120,000 points,
+// 32->32 1157 and 1073, 64->64 1471 and 1450. Dense maps have few rows to leave out: 4 x 30,000 rows with 18 of 27 neighbours, 32->32
+// 227 and 237, 64->64 580 and 486. On one 120,000-point frame the 64->64 kernel keeps the fp32 pipe active 53 % of the time and the
+// shared-memory data path 68 %; about a fifth of the pipe's 111 M instructions are no multiply-adds (they make operand pairs,
+// among other things), but scalar multiply-adds are slower still (issue slots).
 #include <string>
 
 #include "mbarrier.cuh"

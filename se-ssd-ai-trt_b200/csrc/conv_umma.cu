@@ -20,8 +20,9 @@
 //                64-byte runs of 8 or 16 rows instead of one 16-byte piece of 32 rows (those piecemeal
 //                stores alone were an eighth of the kernel's time).
 //   warps 4-7    MMA issuers; issuer t owns tile t of every group. The warp works out the group's schedule
-//                once (lane g for stage g); one elected lane goes through it, waits and issues the tcgen05.mma and
-//                commit instructions (each costs its thread on the order of a hundred cycles, so four share).
+//                once (lane g for stage g); it goes through it together, or with 64 input channels one elected lane alone,
+//                and that lane issues the tcgen05.mma and commit instructions (each costs its thread on the order of a
+//                hundred cycles, so four share).
 //   warp  8      streams the weight blocks (cp.async.bulk) into a three-slot ring.
 //   warp  9      prefetches the neighbour indices of upcoming (tile, stage) items into a ring of index blocks
 //                with bulk copies, sixteen items side by side (one lane each), two to three slot cycles ahead.
@@ -362,8 +363,9 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
 // ---- few tiles ----
 // With few tiles per CTA the pipeline below is latency in good part: a group of one or two tiles uses a weight block once or
 // twice, so that three of them in flight bound it (390 ns per item on a single 20,000-point frame), everything before
-// the first gather (5.8 us: work split, masks, index copy) comes on top of every launch, and whole groups divide badly. This path takes one tile at a time,
-// with seven slots in flight that hold a stage's rows and its weight block, and all of a tile's indices in one copy. What does not
+// the first gather (5.8 us: work split, masks, index copy) comes on top of every launch, and whole groups divide badly. This path
+// takes one tile at a time, with seven slots in flight that hold a stage's rows and its weight block, and all of a tile's indices in one
+// copy. What does not
 // depend on the preceding kernel comes before the wait for that kernel: barriers, tensor memory, tile, indices and the
 // first weight blocks. Tiles are handed out by a counter, one ahead of the tile in work (two index blocks, two accumulators: the
 // next tile's gathers run while this one is stored): a CTA that starts late, because the preceding kernel still held its
@@ -501,10 +503,11 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             }
         }
     } else if (warp == EPI_WARPS) {
-        // Issuer: what bounds the chain of a tile's items, whose rows and weights are there long before. One thread, so that
-        // nothing holds the lanes together, and one barrier per slot for both operands. (As a warp, with a barrier for each, an
-        // item took some 500 cycles: front end of a 20,000-point frame 250 us, then 240. Now it takes 270 where some SMs are idle; 300
-        // where all work, half the copies taking as long. Looking at the next item's barrier ahead of time gave nothing.)
+        // Issuer. One thread, so that nothing holds the lanes together, and one barrier per slot for both operands. (As a warp, with
+        // a barrier for each, an item took some 500 cycles and the issuer was what bound the chain of a tile's items: front end of a
+        // 20,000-point frame 250 us, then 240. Looking at the next item's barrier ahead of time gave nothing.) An item now takes 270
+        // cycles where some SMs are idle and 300 where all work, and what it takes is a slot's round trip, some 1,900 cycles, over the
+        // slots in flight: 320 with six of them, 372 with five, while half of the tcgen05.mma (270) or of the copies (303) change nothing.
         if (leader) {
             if (!waited) {
                 pdl_enter();
@@ -741,8 +744,10 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         static_assert(FEW_BYTES + (BEHIND ? FEW_STAGE : 0) <= NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
                           FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX,
                       "the few-tiles path lives in the other path's buffers");
-        few_uses = umma_few<CIN, COUT>(ctl, sA, reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES)), few_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi, relu,
-                            batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter, total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
+        int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));
+        few_uses = umma_few<CIN, COUT>(ctl, sA, few_idx, few_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi,
+                                       relu, batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter,
+                                       total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
     }
     if (!few) {
         if (tid == 0) ctl->range_lo = 0, ctl->range_hi = total_tiles;   // (the next barrier comes before anyone's cut point)

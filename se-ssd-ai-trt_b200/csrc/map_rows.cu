@@ -566,10 +566,13 @@ int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const Row
 int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
     const int tiles = (max_voxels + 127) / 128;
     const int64_t items = (int64_t)batch * tiles;
-    // A thread per plane while every tile there can be has a block of its own: the planes of a row one after the other are what a small
-    // call waits for. Beyond that the reads bound the SMs, and three times the threads read coordinates and row counts. (In us, a thread
-    // per row and three: submanifold 16 -> 16 1 x 20,000 points 39.4 and 33.6, 64 -> 64 1 x 3,000 29.9 and 24.7, 1 x 120,000 56.0 and 54.9;
-    // room for 6,250 tiles: 16 -> 16 4 x 120,000 298 and 321, 32 -> 32 4 x 60,000 121 and 134.)
+    // A thread per plane up to room for twelve tiles per SM: the planes of a row one after the other are what a small call waits for.
+    // Beyond that the reads bound the SMs, and three times the threads read coordinates and row counts. (This kernel in us, a thread
+    // per row and three, 4 -> 16, 32 -> 32 and 64 -> 64 channels: room for 469 tiles, 1 x 20,000 points 17.1 and 11.3, 19.1 and 13.0,
+    // 9.8 and 6.3; 1,563, 1 x 120,000 30.8 and 28.8, 35.9 and 37.4, 10.1 and 8.0; 1,876, 2 x 60,000 24.3 and 24.0, 34.9 and 32.8, 11.0
+    // and 9.8; 1,876, 4 x 20,000 23.0 and 21.5, 27.4 and 28.2, 11.7 and 12.0; 2,345, 5 x 20,000 24.3 and 24.0, 31.8 and 33.4, 12.7 and
+    // 13.2; 2,814, 3 x 60,000 28.5 and 31.7, 41.4 and 44.8, 13.1 and 14.2; 3,126, 2 x 120,000 36.2 and 44.0, 55.0 and 62.3, 12.6 and
+    // 13.2; 5,628, 12 x 20,000 45.4 and 51.0, 62.4 and 74.1, 25.2 and 30.0.)
     if (items <= persistent_grid(12)) {
         SESSD_LAUNCH(map_tiles_kernel<3>, (int)items, 384, 0, stream, job, batch, max_voxels, tiles, tails);
         return SESSD_OK;

@@ -586,6 +586,10 @@ int launch_mark_outputs(const int32_t* in_coors, const int32_t* in_num, int batc
 // many rows there are is on the device, so that the line is a capacity. Full resolution, by inputs and through a table: room for 60,000
 // rows, 1 x 20,000 points 72.9 and 63.6; 200,000, 1 x 120,000 111 and 107; 240,000, 4 x 20,000 116 and 105; 400,000, 2 x 60,000
 // 123 and 111; 480,000, 8 x 20,000 157 and 153; 600,000, 3 x 120,000 187 and 197; 960,000, 16 x 20,000 243 and 266.
+// Between 200,000 and 500,000 the fill decides, which the host does not know. fp16 16 -> 32, room for half to four fifths (60,000 rows for
+// 20,000 points, 200,000 for 120,000): 300,000 101 and 105, 360,000 119 and 115, 400,000 132 and 133, 480,000 136 and 135; room for
+// hardly more than there is: 164,000 95 and 90, 205,000 102 and 111, 328,000 131 and 137, 410,000 152 and 169; room for five times as
+// much: 400,000 89 and 67. The line is where the usual room breaks even.
 bool scatter_rows_usable(const ConvGeom& g, int64_t rows) {
     return rows > 500000 && (uint64_t)g.in_shape[0] * g.in_shape[1] * g.in_shape[2] >= 1ull << 25;
 }

@@ -43,11 +43,13 @@ voxel_insert_kernel(const float4* __restrict__ points, const int32_t* __restrict
             const uint32_t key = ((uint32_t)iz * g.gy + iy) * g.gx + ix;
             // Most cells have one point: a free slot takes it with one swap, made without looking first. A cell that meets another
             // goes on by a step of its own (odd, so that it comes round to every slot): the longest chain of swaps is what a small
-            // call waits for, and to the next slot chains run together (64 x 20,000 points 79.7 us, so 77.3; 1 x 32,000 23.1 and 18.8).
+            // call waits for, and to the next slot chains run together (64 x 20,000 points 79.7 us, so 77.3; 1 x 32,000 23.1 and 18.8. How
+            // long the longest chain is depends on the frame: over eight frames in turn this kernel takes 9.7 and 8.9 us at
+            // 1 x 20,000, 13.1 and 10.8 at 1 x 32,000, 13.2 and 12.0 at 1 x 120,000).
             unsigned long long* slots = t.slots + (size_t)b * t.cap;
             uint32_t h = hash_slot(key, t.shift);
-            const uint32_t step = (key * 0x85EBCA6Bu >> 15) | 1u;
-                        for (uint32_t probe = 0; probe < t.cap; ++probe, h = (h + step) & (t.cap - 1)) {
+            const uint32_t step = (key * 0x85EBCA6Bu >> 15) | 1u;   // (a multiplier of MurmurHash3's finaliser; any odd one that mixes)
+            for (uint32_t probe = 0; probe < t.cap; ++probe, h = (h + step) & (t.cap - 1)) {
                 const unsigned long long old = atomicCAS(slots + h, ~0ull, (unsigned long long)p << 32 | key);
                 if (old != ~0ull && (uint32_t)old != key) continue;
                 claim = old == ~0ull ? p : (int)(old >> 32);
