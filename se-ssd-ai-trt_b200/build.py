@@ -10,7 +10,7 @@ _ROOT = os.path.dirname(_HERE)
 _CSRC = os.path.join(_HERE, "csrc")
 LIB_PATH = os.path.join(_HERE, "libsessd.so")
 
-SOURCES = ["capi.cu", "voxelize.cu", "voxel_grid.cu", "rulebook.cu", "map_rows.cu", "conv_simt.cu", "conv_f32.cu", "conv_umma.cu", "sparse2dense.cu", "neck.cu", "voxelize_static.cu",
+SOURCES = ["capi.cu", "voxelize.cu", "voxel_grid.cu", "rulebook.cu", "map_rows.cu", "conv_simt.cu", "conv_f32.cu", "conv_rows.cu", "conv_umma.cu", "sparse2dense.cu", "neck.cu", "voxelize_static.cu",
            "postprocess.cu", "nms.cu", "plugins.cu", "formats.cu", "trt_shim.cpp"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",

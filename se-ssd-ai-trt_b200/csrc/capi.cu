@@ -168,7 +168,7 @@ int choose_conv(const ConvLaunch& c_in, cudaStream_t stream) {
     // buffers at any multiple of four bytes are still taken
     const bool aligned = (reinterpret_cast<uintptr_t>(c.in) | reinterpret_cast<uintptr_t>(c.out)) % 16 == 0;
     if (c.dtype == SESSD_F32 && aligned && conv_f32_supported(c.cin, c.cout, c.kvol)) return launch_conv_f32(c, stream);
-    return launch_conv_simt(c, stream);
+    return conv_rows_takes(c) ? launch_conv_rows(c, stream) : launch_conv_simt(c, stream);
 }
 
 }  // namespace
@@ -557,6 +557,9 @@ int sessd_conv_weights_create(const sessd_conv_params* p, const float* weights, 
             e = cudaMemset(w->impl.shift, 0, p->out_channel * 4);
         if (e != cudaSuccess) return fail(e, "cudaMemcpy(shift)");
     }
+    w->impl.finite = 1;                      // (asked of the narrow layers alone)
+    for (size_t i = 0; i < count && w->impl.finite && p->in_channel <= 16 && p->out_channel <= 16; ++i)
+        w->impl.finite = std::isfinite(dtype == SESSD_F32 ? weights[i] : __half2float(__float2half_rn(weights[i])));
     for (int c = 0; c < 64; ++c) {
         w->impl.host_scale[c] = (scale && c < p->out_channel) ? scale[c] : 1.f;
         w->impl.host_shift[c] = (scale && shift && c < p->out_channel) ? shift[c] : 0.f;
@@ -675,6 +678,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     c.status = ws.status;
     c.tile_counter = ws.tile_counter;
     c.debug_withhold_weights = w->impl.debug_withhold;
+    c.weights_finite = w->impl.finite;
     c.scale_host = w->impl.host_scale;
     c.shift_host = w->impl.host_shift;
     return choose_conv(c, stream);
@@ -965,6 +969,7 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         c.tile_counter = w.tile_counter + i;
         c.maps_ready = i > 0 ? 1 : 0;   // the first layer follows the launch that builds the maps
         c.debug_withhold_weights = L.w->impl.debug_withhold;
+        c.weights_finite = L.w->impl.finite;
         c.scale_host = L.w->impl.host_scale;
         c.shift_host = L.w->impl.host_shift;
         if (bb->has_s2d && i + 1 == bb->layers.size()) {

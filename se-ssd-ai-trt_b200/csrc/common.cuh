@@ -182,6 +182,11 @@ __host__ __device__ inline size_t nbr_frame_words(int kvol, int max_voxels) {
 __host__ __device__ inline size_t nbr_index(int kvol, int max_voxels, int b, int k, int o) {
     return (size_t)b * nbr_frame_words(kvol, max_voxels) + ((size_t)(o >> 7) * kvol + k) * kNbrRun + (o & 127);
 }
+// The padding behind a tile's first offset holds four words, for each 32 of its rows a mask of offsets: at least those that any of
+// the 32 has a neighbour under (all ones where a map's builder does not say; bits that the tile's mask lacks mean nothing).
+__host__ __device__ inline size_t nbr_runs_index(int kvol, int max_voxels, int b, int o) {
+    return nbr_index(kvol, max_voxels, b, 0, o & ~127) + 128 + ((o >> 5) & 3);
+}
 
 // Geometry of one sparse convolution (z, y, x order everywhere).
 struct ConvGeom {
@@ -407,11 +412,16 @@ struct ConvLaunch {
     int* tile_counter;     // tensor-core path: zero before the launch; hands out the tiles of small layers (null: it never does)
     int maps_ready;        // neighbour map, masks and row counts are older than the kernel launched just before
     int debug_withhold_weights;   // tests only: whoever streams the weights stays silent (waits run out)
+    int weights_finite;           // every weight is a finite number of the feature dtype
     const float* scale_host;      // [Cout <= 64] host copies of scale / shift (ones / zeros without batch norm), or null
     const float* shift_host;
 };
 int launch_conv_simt(const ConvLaunch& c, cudaStream_t stream);
 bool conv_simt_supported(int cin, int cout);
+
+// conv_rows.cu (narrow layers: a warp per 32 rows)
+bool conv_rows_takes(const ConvLaunch& c);
+int launch_conv_rows(const ConvLaunch& c, cudaStream_t stream);
 
 // conv_f32.cu (fp32 storage, a register tile per warp)
 bool conv_f32_supported(int cin, int cout, int kvol);
@@ -486,6 +496,7 @@ struct sessd_conv_weights_impl {
     float* scale;   // device or null
     float* shift;   // device or null
     int relu, dtype, kvol, cin, cout;
+    int finite;           // every weight is a finite number of dtype
     int debug_withhold;   // tests of the time-out path: whoever streams the weights stays silent
     // host copies of scale and shift (ones and zeros without batch norm) for kernels that take them as launch
     // parameters; filled for out_channel <= 64

@@ -10,9 +10,9 @@
 // ReLU (a separate TensorRT scale + activation layer in the reference, se-ssd-ai-trt.cpp:808-856)
 // run in the epilogue, and the last layer can scatter straight into the dense BEV map.
 //
-// This path serves the memory-bound small-channel layers (4->16; in fp32 also 16->16 and 16->32) and, with a kernel
-// that takes its channel counts at run time, every pair of channel counts without a kernel of its own. The wide fp32
-// layers are in conv_f32.cu, the wide fp16 layers in conv_umma.cu.
+// This path serves the memory-bound small-channel layers (4->16; in fp32 also 16->16 and 16->32) in calls of few rows (larger ones,
+// but for 16->32, are in conv_rows.cu) and, with a kernel that takes its channel counts at run time, every pair of channel counts
+// without a kernel of its own. The wide fp32 layers are in conv_f32.cu, the wide fp16 layers in conv_umma.cu.
 #include <string>
 #include <type_traits>
 
@@ -364,19 +364,15 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
 
 template <typename T>
 int dispatch(const ConvLaunch& c, cudaStream_t stream) {
-    // Room for a million rows is what a few frames have. Those are latency: a thread with half the channels is through its
-    // row's neighbours sooner, and twice as many blocks share out the rows with the longest lists. Larger batches are
-    // throughput: with twice the channels half as many threads walk a list. The line is a capacity, because row counts are on the
-    // device. Half the channels and all of them, in us: fp16 front end (4 -> 16) 1 x 20,000 points 254 and 258, 4 x 120,000
-    // (800,000 rows) 1047 and 1055, 16 x 20,000 (960,000) 1208 and 1208, 32 x 20,000 2199 and 2190, 32 x 120,000 6920 and 6896; fp32
-    // front end (all three) 1 x 20,000 992 and 1000, 4 x 120,000 9407 and 9408, 8 x 120,000 18097 and 18062. Single calls: 4 -> 16
-    // 8 x 20,000 103 and 106, 16 x 20,000 152 and 149; fp32 16 -> 16 half is better at every size (16 x 120,000: 1189 and
-    // 1227); a submanifold fp32 16 -> 32, which the network has none of, would cross between 4 and 8 x 20,000 (4 x 120,000: 523
-    // and 460).
+    // Half the channels per thread (a thread is through its row's neighbours sooner, and twice as many blocks share out the rows with
+    // the longest lists) is the faster way for the calls that conv_rows.cu leaves here: front end of 1 x 20,000 points, fp16 254 us
+    // and 258 with all of them, fp32 992 and 1000. fp32 16 -> 32 stays here at every size; with all the channels half as many threads
+    // walk a list, which a submanifold layer (the network has none of these) gains from between 4 and 8 x 20,000 points (4 x 120,000:
+    // 523 and 460), the network's strided one from a million rows on (8 x 120,000 18097 and 18062, the whole front end).
     const bool few = (int64_t)c.batch * c.max_voxels <= 1000000;
-    if (c.cin == 4 && c.cout == 16) return few ? launch_narrow<T, 4, 16, 4>(c, stream) : launch_narrow<T, 4, 16, 8>(c, stream);
+    if (c.cin == 4 && c.cout == 16) return launch_narrow<T, 4, 16, 4>(c, stream);
     if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these
-        if (c.cin == 16 && c.cout == 16) return few ? launch_narrow<float, 16, 16, 2>(c, stream) : launch_narrow<float, 16, 16, 4>(c, stream);
+        if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16, 2>(c, stream);
         if (c.cin == 16 && c.cout == 32) return few ? launch_narrow<float, 16, 32, 2>(c, stream) : launch_narrow<float, 16, 32, 4>(c, stream);
     }
     return launch_generic<T>(c, stream);   // any other pair of channel counts

@@ -463,7 +463,10 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
             if (tile0 >= n) break;                           // a tile without rows (uniform over the warp)
             const uint4 g = *reinterpret_cast<const uint4*>(&s.group_bits[tile0 >> 5]);
             uint32_t m = g.x | g.y | g.z | g.w;
-            if ((p & 127) == 0) job.tile_mask[(size_t)b * tiles_per_frame + ((w0 + p) >> 7)] = m;
+            if ((p & 127) == 0) {
+                job.tile_mask[(size_t)b * tiles_per_frame + ((w0 + p) >> 7)] = m;
+                *reinterpret_cast<uint4*>(job.nbr + nbr_runs_index(job.g.kvol, max_voxels, b, w0 + p)) = g;
+            }
             // a consumer that fetches `group` offsets at a time wants all of them as soon as it wants one
             if (job.group >= 2) m |= (m & 0x55555555u) << 1 | ((m >> 1) & 0x55555555u);
             if (job.group >= 4) m |= (m & 0x33333333u) << 2 | ((m >> 2) & 0x33333333u);
@@ -511,11 +514,13 @@ map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, 
         __syncthreads();
         if (lane == 0) s_mask[warp] = any;
         __syncthreads();
-        if (tid == 0) {
-            uint32_t m = 0;
+        if (warp == 0) {
+            uint32_t m = 0;                                  // of 32 rows: lane's quarter of the tile
 #pragma unroll
-            for (int w = 0; w < 4 * PLANES; ++w) m |= s_mask[w];
-            job.tile_mask[it] = m;
+            for (int p = 0; p < PLANES; ++p) m |= s_mask[4 * p + (lane & 3)];
+            if (lane < 4) job.nbr[nbr_runs_index(job.g.kvol, max_voxels, b, p0 + 32 * lane)] = (int32_t)m;
+            m = __reduce_or_sync(0xFFFFFFFFu, m);
+            if (lane == 0) job.tile_mask[it] = m;
         }
     }
 }

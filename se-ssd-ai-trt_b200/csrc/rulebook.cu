@@ -90,6 +90,7 @@ nbr_build_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__
             if (slot >= 0) row = in_table.vals[(size_t)b * in_table.cap + slot];
         }
         nbr[nbr_index(g.kvol, max_voxels, b, k, o)] = row;
+        if (k == 0 && (o & 31) == 0) nbr[nbr_runs_index(g.kvol, max_voxels, b, o)] = -1;
     }
 }
 
@@ -200,7 +201,7 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
 // more outputs than inputs.
 
 // Fills the map entries of the tiles that hold rows 0 .. out_num[b] with -1, 16 bytes per thread (a tile's kvol x kNbrRun words
-// are contiguous; the padding is written too), and zeroes the tails of the call's outputs.
+// are contiguous; the padding is written too: any offset for every 32 rows), and zeroes the tails of the call's outputs.
 __global__ void __launch_bounds__(kThreads)
 nbr_clear_kernel(int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num, int batch, int max_voxels, int kvol,
                  TailRows tails) {

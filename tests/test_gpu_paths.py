@@ -124,6 +124,81 @@ def test_fp32_rows_off_the_vector_alignment(gpu, skip_in, skip_out):
     w.close()
 
 
+@pytest.mark.parametrize("cin,dtype", [(4, 0), (4, 1), (16, 0)])
+@pytest.mark.parametrize("ks", [1, 2, 3])
+def test_narrow_layers_on_both_sides_of_the_line(gpu, oracle, cin, dtype, ks):
+    """4 -> 16 and fp32 16 -> 16 channels with room for more than 300,000 rows (64 positions to a warp) and for fewer: the same bits,
+    for the last rows of a run, kernels of 1, 8 and 27 offsets, more than 32 empty frames in a row, and the oracle's values."""
+    import torch
+
+    rs = np.random.RandomState(cin + ks)
+    layer = _layer(gpu, True, cin, 16, (ks,) * 3, (1, 1, 1), (ks // 2 if ks == 3 else 0,) * 3, (6, 20, 24))
+    W = (rs.randn(ks ** 3, cin, 16) / np.sqrt(cin * ks)).astype(np.float32)
+    sc, sh = (1 + 0.1 * rs.randn(16)).astype(np.float32), (0.1 * rs.randn(16)).astype(np.float32)
+    tdt = np.float16 if dtype else np.float32
+    rows = [0, 1, 31, 32, 33, 63, 64, 65, 127, 128, 129, 1500]
+    coors = [_random_coords(rs, n, layer.in_shape) for n in rows]
+    feats = [rs.randn(n, cin).astype(np.float32) for n in rows]
+    some = [(coors[i], feats[i]) for i in (1, 5, 9, 11)]
+    _check_layer(gpu, oracle, layer, some, W, sc, sh, True, dtype=dtype, maxV=80000)
+    _check_layer(gpu, oracle, layer, some, W, dtype=dtype, maxV=75001)
+    use = [0] * 35 + [int(v) for v in rs.randint(len(rows), size=160)] + [0]
+    names = []
+
+    def call(which, maxV):
+        p = gpu.conv_params(layer, maxV)
+        w = gpu.ConvWeights(p, W, sc, sh, True, dtype)
+        c, x = np.zeros((len(which), maxV, 4), np.int32), np.zeros((len(which), maxV, cin), tdt)
+        for b, i in enumerate(which):
+            c[b, :rows[i]], x[b, :rows[i]] = coors[i], feats[i]
+        args = (torch.from_numpy(x).cuda(), torch.from_numpy(c).cuda(), torch.tensor([rows[i] for i in which], dtype=torch.int32).cuda(), p, w)
+        r = gpu.subm_conv(*args, keep_workspace=True)
+        assert r["status"] == 0
+        names.append([n for n, _ in gpu.profile(lambda: gpu.subm_conv_into(*args, r["features"], r["workspace"]))][-1])
+        w.close()
+        return r["features"]
+
+    got, alone = call(use, 1537), [call([i], 1537)[0] for i in range(len(rows))]
+    assert names[0].startswith("conv_rows") and names[1].startswith("conv_narrow")
+    for b, i in enumerate(use):
+        assert torch.equal(got[b], alone[i]), b
+
+
+@pytest.mark.parametrize("cin,dtype", [(4, 0), (4, 1), (16, 0)])
+def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, cin, dtype):
+    """Weights that are no finite numbers go through the kernel of small calls whatever the room: such a weight reaches the rows with
+    its neighbour alone."""
+    import torch
+
+    rs = np.random.RandomState(6)
+    layer = _layer(gpu, True, cin, 16, (3, 3, 3), (1, 1, 1), (1, 1, 1), (6, 20, 30))
+    rows, maxV, tdt = 700, 300001, torch.float16 if dtype else torch.float32
+    c = _random_coords(rs, rows, layer.in_shape)
+    coors = torch.zeros((1, maxV, 4), dtype=torch.int32, device="cuda")
+    coors[0, :rows] = torch.from_numpy(c).cuda()
+    num = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, maxV)
+    W = (rs.randn(27, cin, 16) * 0.2).astype(np.float32)
+    x = torch.zeros((1, maxV, cin), dtype=tdt, device="cuda")
+    x[0, :rows] = torch.from_numpy(rs.randn(rows, cin)).to(tdt).cuda()
+    w = gpu.ConvWeights(p, W, None, None, False, dtype)
+    r = gpu.subm_conv(x, coors, num, p, w, keep_workspace=True)
+    names = [[n for n, _ in gpu.profile(lambda: gpu.subm_conv_into(x, coors, num, p, w, r["features"], r["workspace"]))][-1]]
+    w.close()
+    W[5, 1, 3] = 1e6 if dtype else np.inf
+    w = gpu.ConvWeights(p, W, None, None, False, dtype)
+    bad = gpu.subm_conv(x, coors, num, p, w, keep_workspace=True)
+    names.append([n for n, _ in gpu.profile(lambda: gpu.subm_conv_into(x, coors, num, p, w, bad["features"], bad["workspace"]))][-1])
+    pairs, pnum, _ = oracle.subm_rulebook(c, rows, layer.out_shape, rows)
+    hit = np.zeros(rows, bool)
+    hit[pairs[5, 1, :pnum[5]]] = True
+    f = bad["features"][0, :rows]
+    assert hit.any() and not hit.all()
+    assert (~torch.isfinite(f[:, 3]).cpu().numpy() == hit).all() and torch.isfinite(f[:, torch.arange(16) != 3]).all()
+    w.close()
+    assert names[0].startswith("conv_rows") and names[1].startswith("conv_narrow")
+
+
 @pytest.mark.parametrize("rows", [148 * 128, 148 * 128 + 1])
 def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     rs = np.random.RandomState(rows)
