@@ -105,6 +105,15 @@ __device__ __forceinline__ void cp_async_16_or_zero_once(uint32_t dst, const voi
         "l"(src), "r"(index), "r"(was_zero)
         : "memory");
 }
+// 16-byte copy that writes zeros instead when index < 0 (the source address is then not touched).
+__device__ __forceinline__ void cp_async_16_or_zero(uint32_t dst, const void* src, int index) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.lt.s32 p, %2, 0;\n\t"
+        "cp.async.cg.shared.global [%0], [%1], 16, p;\n\t}" ::"r"(dst),
+        "l"(src), "r"(index)
+        : "memory");
+}
 // Arrival on `bar` that fires when all cp.async copies this thread has issued so far have landed
 // (the barrier's expected count must include it).
 __device__ __forceinline__ void cp_async_arrive_noinc(uint32_t bar) {
@@ -422,6 +431,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 for (int i = 0; i < FEW_SLOTS; ++i) left &= left - 1u;
                 const uint32_t idx_base = smem_u32(s_idx + r * (FEW_IDX * TAP_WORDS) + (g * KG + koff) * TAP_WORDS + jrow);
                 const bool k_ok = g * KG + koff < kvol;
+                const bool plain = g * KG + KG <= kvol && row0 + TILE_M <= n;   // uniform over the warp
                 int vv[32];
 #pragma unroll
                 for (int w4 = 0; w4 < 8; ++w4) {
@@ -444,12 +454,15 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                     pdl_enter();
                     waited = true;
                 }
+                if (!plain) {
 #pragma unroll
-                for (int p = 0; p < 32; ++p) {
-                    const int id = (k_ok && 32 * (p >> 3) + (p & 7) < rows_left) ? vv[p] : -1;
-                    cp_async_16(a_base + (32 * (p >> 3) + (p & 7)) * ROW_BYTES + ((c ^ (p & 7)) << 4),
-                                lane_base + (size_t)(id < 0 ? 0 : id) * CIN, id < 0 ? 0u : 16u);
+                    for (int p = 0; p < 32; ++p)
+                        if (!(k_ok && 32 * (p >> 3) + (p & 7) < rows_left)) vv[p] = -1;
                 }
+#pragma unroll
+                for (int p = 0; p < 32; ++p)
+                    cp_async_16_or_zero(a_base + (32 * (p >> 3) + (p & 7)) * ROW_BYTES + ((c ^ (p & 7)) << 4),
+                                        lane_base + (ptrdiff_t)vv[p] * CIN, vv[p]);
                 cp_async_arrive_noinc(smem_u32(full + s));
             }
             items += (uint32_t)__popc(stages);
