@@ -15,10 +15,8 @@
 // One persistent CTA per SM; every role has warps of its own and walks the same sequence of groups:
 //   warps 0-3    epilogue (warp w reads tensor-memory lanes 32w .. 32w+31). The accumulators are double
 //                buffered (2 sets x 4 tiles x Cout columns), so the epilogue of one group runs while the
-//                other roles are already working on the next group. A thread holds one row; the rows go
-//                through a small staging area of the warp, so that a store instruction writes whole 32- or
-//                64-byte runs of 8 or 16 rows instead of one 16-byte piece of 32 rows (those piecemeal
-//                stores alone were an eighth of the kernel's time).
+//                other roles are already working on the next group. A thread holds one row and stores it 32 bytes
+//                at a time.
 //   warps 4-7    MMA issuers; issuer t owns tile t of every group. The warp works out the group's schedule
 //                once (lane g for stage g); it goes through it together, or with 64 input channels one elected lane alone,
 //                and that lane issues the tcgen05.mma and commit instructions (each costs its thread on the order of a
@@ -213,20 +211,13 @@ struct SharedCtl {
     uint32_t idx_uses[NIDX_MAX];             // bulk copies issued into index block j so far (for the abort path)
 };
 
-// Epilogue staging: every epilogue warp owns room for its 32 rows of one column block (up to 32 channels), so that
-// the rows leave for global memory as whole 32- or 64-byte runs instead of one 16-byte piece per row and store.
-template <int COUT>
-__host__ __device__ constexpr int stage_row_bytes() { return (COUT < 32 ? COUT : 32) * 2; }
 // Epilogue warps of the few-tiles path: with 64 channels a column block each for eight (warps 5-8 have nothing else to do there).
 template <int COUT>
 __host__ __device__ constexpr int few_epi_warps() { return COUT == 64 ? 2 * EPI_WARPS : EPI_WARPS; }
 template <int CIN, int COUT>
-__host__ __device__ constexpr int stage_bytes() { return (CIN == 64 ? few_epi_warps<COUT>() : EPI_WARPS) * 32 * stage_row_bytes<COUT>(); }
-
-template <int CIN, int COUT>
 constexpr int umma_smem_bytes() {
     return 1024 /*alignment slack*/ + Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES +
-           Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 + stage_bytes<CIN, COUT>() + (int)sizeof(SharedCtl);
+           Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 + (int)sizeof(SharedCtl);
 }
 
 // Offsets g*KG .. g*KG+KG-1 of a tile's 27-bit offset mask.
@@ -289,25 +280,18 @@ __device__ __forceinline__ int items_before_stage(uint32_t bits, int lane, int* 
     return items;
 }
 
-// Epilogue of channels FROM .. TO - 1 of a tile for one of four warps: rows 32 warp .. + 31 of the tile, lane = position `pos` of the map, output
-// row `row`, accumulators at tensor-memory address taddr (zeros instead when !have).
+// Epilogue of channels FROM .. TO - 1 of a tile for one of four warps: lane = position `pos` of the map, output row `row`, accumulators
+// at tensor-memory address taddr (zeros instead when !have). A lane stores its own row, 32 bytes to an instruction where the rows
+// start at multiples of 32 bytes (wide): whole sectors. (16 bytes at a time an instruction touches half of 32 sectors. Through
+// shared memory, so that a row leaves as one run, the warp's stores, reads and shuffles queue behind the gather warps' copies: a tile
+// of 64 channels took a warp 5,900 cycles, which bound every layer of few items to a tile.)
 template <int COUT, int FROM = 0, int TO = COUT>
-__device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiConst& epi, int relu, uint8_t* s_stage, int warp,
-                                           int lane, int pos, int row, int n, int b, int max_voxels, __half* __restrict__ out,
-                                           __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
-                                           int W) {
+__device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiConst& epi, int relu, int pos, int row, int n, int b,
+                                           int max_voxels, __half* __restrict__ out, bool wide, __half* __restrict__ dense,
+                                           const int4* __restrict__ out_coors, int D, int H, int W) {
     // Column blocks of CB channels keep the register footprint small.
     constexpr int CB = COUT < 32 ? COUT : 32;
-    constexpr int RB = stage_row_bytes<COUT>();   // bytes of a row's column block
-    constexpr int CPR = RB / 16;                  // 16-byte chunks per row and block: 4 or 2
-    uint8_t* stage = s_stage + warp * (32 * RB);
-    auto stage_swz = [](int r) { return RB == 64 ? (r >> 1) & 3 : (r >> 2) & 1; };
-    __half* d = nullptr;
-    if (dense && pos < n) {
-        // fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x)
-        const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + row]);
-        d = dense + (size_t)b * COUT * D * H * W + ((size_t)c4.y * H + c4.z) * W + c4.w;
-    }
+    __half* to = out + ((size_t)b * max_voxels + row) * COUT;
 #pragma unroll
     for (int cb = FROM; cb < TO; cb += CB) {
         float acc[CB];
@@ -315,57 +299,60 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
             if constexpr (CB == 32) {
                 uint32_t r32[32];
                 tmem_ld32(taddr + cb, r32);
+                tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 32; ++j) acc[j] = __uint_as_float(r32[j]);
             } else {
                 uint32_t r16[16];
                 tmem_ld16(taddr + cb, r16);
+                tmem_ld_wait();
 #pragma unroll
                 for (int j = 0; j < 16; ++j) acc[j] = __uint_as_float(r16[j]);
             }
-            tmem_ld_wait();
         } else {
 #pragma unroll
             for (int j = 0; j < CB; ++j) acc[j] = 0.f;
         }
-        // Every lane packs its row's block into the warp's staging area (16-byte chunks XOR-swizzled by
-        // row so that neither the writes nor the reads below meet in a bank) ...
+        uint32_t pk[CB / 2];
 #pragma unroll
-        for (int c0 = 0; c0 < CB; c0 += 8) {
-            uint4 pk;
-            __half2* h = reinterpret_cast<__half2*>(&pk);
+        for (int j = 0; j < CB / 2; ++j) {
+            const int ch = cb + 2 * j;        // a constant after unrolling
+            const __half2 h =
+                __floats2half2_rn(fmaf(acc[2 * j], epi.scale[ch], epi.shift[ch]), fmaf(acc[2 * j + 1], epi.scale[ch + 1], epi.shift[ch + 1]));
+            pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        if (relu) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int ch = cb + c0 + 2 * j;   // a constant after unrolling
-                float v0 = fmaf(acc[c0 + 2 * j], epi.scale[ch], epi.shift[ch]);
-                float v1 = fmaf(acc[c0 + 2 * j + 1], epi.scale[ch + 1], epi.shift[ch + 1]);
-                if (relu) {
-                    v0 = v0 > 0.f ? v0 : 0.f;
-                    v1 = v1 > 0.f ? v1 : 0.f;
-                }
-                h[j] = __floats2half2_rn(v0, v1);
+            for (int j = 0; j < CB / 2; ++j) {
+                const __half2 h = __hmax2(*reinterpret_cast<const __half2*>(&pk[j]), __half2(__half(0.f), __half(0.f)));   // (a NaN becomes 0)
+                pk[j] = *reinterpret_cast<const uint32_t*>(&h);
             }
-            *reinterpret_cast<uint4*>(stage + lane * RB + (((c0 >> 3) ^ stage_swz(lane)) << 4)) = pk;
-            if (d) {
+        }
+        if (pos < n) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    d[(size_t)(cb + c0 + 2 * j) * D * H * W] = __low2half(h[j]);
-                    d[(size_t)(cb + c0 + 2 * j + 1) * D * H * W] = __high2half(h[j]);
+            for (int j = 0; j < CB / 2; j += 8) {
+                if (wide) {
+                    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(to + cb + 2 * j), "r"(pk[j]), "r"(pk[j + 1]),
+                                 "r"(pk[j + 2]), "r"(pk[j + 3]), "r"(pk[j + 4]), "r"(pk[j + 5]), "r"(pk[j + 6]), "r"(pk[j + 7])
+                                 : "memory");
+                } else {
+                    *reinterpret_cast<uint4*>(to + cb + 2 * j) = make_uint4(pk[j], pk[j + 1], pk[j + 2], pk[j + 3]);
+                    *reinterpret_cast<uint4*>(to + cb + 2 * j + 8) = make_uint4(pk[j + 4], pk[j + 5], pk[j + 6], pk[j + 7]);
+                }
+            }
+            if (dense) {
+                // fused BEV scatter (sparse2Dense.cu:201-206): channel c*D + z, pixel (y, x)
+                const int4 c4 = __ldg(&out_coors[(size_t)b * max_voxels + row]);
+                const size_t plane = (size_t)D * H * W;
+                __half* d = dense + ((size_t)b * COUT + cb) * plane + ((size_t)c4.y * H + c4.z) * W + c4.w;
+#pragma unroll
+                for (int j = 0; j < CB / 2; ++j, d += 2 * plane) {
+                    const __half2 h = *reinterpret_cast<const __half2*>(&pk[j]);
+                    d[0] = __low2half(h);
+                    d[plane] = __high2half(h);
                 }
             }
         }
-        __syncwarp();
-        // ... and the warp copies the block out with CPR lanes per row: each store instruction writes
-        // 32 / CPR rows as whole runs of RB bytes.
-#pragma unroll
-        for (int i = 0; i < CPR; ++i) {
-            const int rr = lane / CPR + i * (32 / CPR), cc = lane % CPR;
-            const uint4 v = *reinterpret_cast<const uint4*>(stage + rr * RB + ((cc ^ stage_swz(rr)) << 4));
-            const int grow = __shfl_sync(0xFFFFFFFFu, row, rr);
-            if (pos - lane + rr < n)
-                *reinterpret_cast<uint4*>(out + ((size_t)b * max_voxels + grow) * COUT + cb + cc * 8) = v;
-        }
-        __syncwarp();
     }
 }
 
@@ -381,7 +368,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
 // SM, leaves the tiles to the others. A tile's offsets are added up in the same order as in the other path, so the results are
 // the same bits.
 template <int CIN, int COUT>
-__device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_t* s_idx, uint8_t* s_stage, uint32_t tmem,
+__device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_t* s_idx, bool wide, uint32_t tmem,
                                          bool leader, const __half* __restrict__ in, __half* __restrict__ out,
                                          const int32_t* __restrict__ nbr, const int32_t* __restrict__ order,
                                          const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
@@ -475,7 +462,6 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     } else if (warp < EPI_WARPS || (COUT == 64 && warp > EPI_WARPS && warp <= WEIGHT_WARP)) {
         // epilogue: a warp reads the tensor-memory lanes of its number modulo four
         const int quarter = warp & 3, part = warp < EPI_WARPS ? 0 : 1;
-        uint8_t* stage = s_stage + part * (EPI_WARPS * 32 * stage_row_bytes<COUT>());
         for (uint32_t round = 0;; ++round) {
             const uint32_t r = round & 1u;
             bool ok = mbar_wait(smem_u32(tile_full + r), (round >> 1) & 1u, abort_flag, 3 | (int)(round << 4));
@@ -500,14 +486,12 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             }
             const uint32_t taddr = tmem + ((uint32_t)(quarter * 32) << 16) + set * COUT;
             if constexpr (COUT < 64) {
-                store_tile<COUT>(taddr, have, epi, relu, stage, quarter, lane, pos, row, n, b, max_voxels, out, dense, out_coors, D, H, W);
+                store_tile<COUT>(taddr, have, epi, relu, pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
             } else {
                 if (part == 0)
-                    store_tile<COUT, 0, COUT / 2>(taddr, have, epi, relu, stage, quarter, lane, pos, row, n, b, max_voxels, out, dense,
-                                                  out_coors, D, H, W);
+                    store_tile<COUT, 0, COUT / 2>(taddr, have, epi, relu, pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
                 else
-                    store_tile<COUT, COUT / 2, COUT>(taddr, have, epi, relu, stage, quarter, lane, pos, row, n, b, max_voxels, out, dense,
-                                                     out_coors, D, H, W);
+                    store_tile<COUT, COUT / 2, COUT>(taddr, have, epi, relu, pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
             }
             if (have) {
                 tc_fence_before();
@@ -648,8 +632,8 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     uint8_t* sA = smem;
     uint8_t* sB = sA + NSLOT * A_BYTES;
     int32_t* s_idx = reinterpret_cast<int32_t*>(sB + B_STAGES * B_BYTES);
-    uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_idx + NIDX * IDX_WORDS);
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(s_stage + stage_bytes<CIN, COUT>());
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(s_idx + NIDX * IDX_WORDS);
+    const bool wide = reinterpret_cast<uintptr_t>(out) % 32 == 0;   // (rows are 32, 64 or 128 bytes)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = (kvol + KG - 1) / KG;
@@ -749,16 +733,12 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     }
     const bool few = tile_counter != nullptr && total_tiles <= FEW_TILES * (int)gridDim.x;
     if (few) {
-        // eight warps' staging areas: where s_stage has room for four only, they lie behind the index blocks
-        constexpr int FEW_STAGE = few_epi_warps<COUT>() * 32 * stage_row_bytes<COUT>();
-        constexpr int FEW_BYTES = FEW_SLOTS * (A_BYTES + B_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4;
-        constexpr bool BEHIND = FEW_STAGE > stage_bytes<CIN, COUT>();
-        uint8_t* few_stage = BEHIND ? sA + FEW_BYTES : s_stage;
-        static_assert(FEW_BYTES + (BEHIND ? FEW_STAGE : 0) <= NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
+        static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4 <=
+                              NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
                           FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX,
                       "the few-tiles path lives in the other path's buffers");
         int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));
-        few_uses = umma_few<CIN, COUT>(ctl, sA, few_idx, few_stage, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi,
+        few_uses = umma_few<CIN, COUT>(ctl, sA, few_idx, wide, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi,
                                        relu, batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter,
                                        total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
     }
@@ -1015,7 +995,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 const uint32_t m_t2 = t2 == 0 ? m[0] : (t2 == 1 ? m[1] : (t2 == 2 ? m[2] : m[3]));
                 if (got)
                     store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + set * SET_COLS + t2 * COUT, any && m_t2, epi, relu,
-                                     s_stage, warp, lane, pos, row, n, b, max_voxels, out, dense, out_coors, D, H, W);
+                                     pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
             }
             if (any && got) {
                 tc_fence_before();
