@@ -66,7 +66,7 @@ constexpr int KVOL_MAX = 27;
 // with the path 84.5, 16 tiles 151.0 and 154.4. (Groups have become faster since: four, seven, ten: 3 x 20,000 369, 354, 354; 5 x 77,000
 // 698, 690, 693; 64 -> 64 with 8 tiles per CTA 84.7, 84.7, 83.2.)
 constexpr int FEW_TILES = 10;
-constexpr int FEW_SLOTS = 7;                 // few-tiles path: stages in flight, an A slot and a weight block each
+constexpr int FEW_SLOTS = 8;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
 // instructions, with the issuer.
 __host__ __device__ constexpr int few_slot(int warp) {
@@ -214,11 +214,15 @@ struct SharedCtl {
 // Epilogue warps of the few-tiles path: with 64 channels a column block each for eight (warps 5-8 have nothing else to do there).
 template <int COUT>
 __host__ __device__ constexpr int few_epi_warps() { return COUT == 64 ? 2 * EPI_WARPS : EPI_WARPS; }
+// Buffers of the two paths, which share their place.
 template <int CIN, int COUT>
-constexpr int umma_smem_bytes() {
-    return 1024 /*alignment slack*/ + Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES +
-           Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 + (int)sizeof(SharedCtl);
+__host__ __device__ constexpr int ring_bytes() {
+    constexpr int groups = Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES + Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4;
+    constexpr int few = FEW_SLOTS * (A_BYTES + COUT * ROW_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4;
+    return groups > few ? groups : few;
 }
+template <int CIN, int COUT>
+constexpr int umma_smem_bytes() { return 1024 /*alignment slack*/ + ring_bytes<CIN, COUT>() + (int)sizeof(SharedCtl); }
 
 // Offsets g*KG .. g*KG+KG-1 of a tile's 27-bit offset mask.
 template <int KG>
@@ -360,7 +364,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
 // With few tiles per CTA the pipeline below is latency in good part: a group of one or two tiles uses a weight block once or
 // twice, so that three of them in flight bound it (390 ns per item on a single 20,000-point frame), everything before
 // the first gather (5.8 us: work split, masks, index copy) comes on top of every launch, and whole groups divide badly. This path
-// takes one tile at a time, with seven slots in flight that hold a stage's rows and its weight block, and all of a tile's indices in one
+// takes one tile at a time, with eight slots in flight that hold a stage's rows and its weight block, and all of a tile's indices in one
 // copy. What does not
 // depend on the preceding kernel comes before the wait for that kernel: barriers, tensor memory, tile, indices and the
 // first weight blocks. Tiles are handed out by a counter, one ahead of the tile in work (two index blocks, two accumulators: the
@@ -502,9 +506,10 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     } else if (warp == EPI_WARPS) {
         // Issuer. One thread, so that nothing holds the lanes together, and one barrier per slot for both operands. (As a warp, with
         // a barrier for each, an item took some 500 cycles and the issuer was what bound the chain of a tile's items: front end of a
-        // 20,000-point frame 250 us, then 240. Looking at the next item's barrier ahead of time gave nothing.) An item now takes 270
-        // cycles where some SMs are idle and 300 where all work, and what it takes is a slot's round trip, some 1,900 cycles, over the
-        // slots in flight: 320 with six of them, 372 with five, while half of the tcgen05.mma (270) or of the copies (303) change nothing.
+        // 20,000-point frame 250 us, then 240. Looking at the next item's barrier ahead of time gave nothing.) What an item takes is a
+        // slot's round trip over the slots in flight: of 2,200 cycles with seven slots a gather warp's copies were 1,100, their landing
+        // 950, the MMAs and their commit 430. Seven and eight slots: front end of 1 x 20,000 points 198.5 and 193.5 us, 1 x 120,000
+        // 363.6 and 353 to 360; nine and ten where narrower layers leave room 194.5 and 361.
         if (leader) {
             if (!waited) {
                 pdl_enter();
@@ -632,7 +637,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     uint8_t* sA = smem;
     uint8_t* sB = sA + NSLOT * A_BYTES;
     int32_t* s_idx = reinterpret_cast<int32_t*>(sB + B_STAGES * B_BYTES);
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(s_idx + NIDX * IDX_WORDS);
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + ring_bytes<CIN, COUT>());
     const bool wide = reinterpret_cast<uintptr_t>(out) % 32 == 0;   // (rows are 32, 64 or 128 bytes)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -735,10 +740,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     // to a channel and row, are what it does; there eight warps share them. (32 frames of 120,000 points: four warps 190 us, eight 139.)
     const bool few = tile_counter != nullptr && (dense != nullptr || total_tiles <= FEW_TILES * (int)gridDim.x);
     if (few) {
-        static_assert(FEW_SLOTS * (A_BYTES + B_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4 <=
-                              NSLOT * A_BYTES + B_STAGES * B_BYTES + NIDX * IDX_WORDS * 4 &&
-                          FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX,
-                      "the few-tiles path lives in the other path's buffers");
+        static_assert(FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX, "whole stages of indices");
         int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));
         few_uses = umma_few<CIN, COUT>(ctl, sA, few_idx, wide, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi,
                                        relu, batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter,
