@@ -369,7 +369,7 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
 // depend on the preceding kernel comes before the wait for that kernel: barriers, tensor memory, tile, indices and the
 // first weight blocks. Tiles are handed out by a counter, one ahead of the tile in work (two index blocks, two accumulators: the
 // next tile's gathers run while this one is stored): a CTA that starts late, because the preceding kernel still held its
-// SM, leaves the tiles to the others. A tile's offsets are added up in the same order as in the other path, so the results are
+// SM, leaves the further tiles to the others. A tile's offsets are added up in the same order as in the other path, so the results are
 // the same bits.
 template <int CIN, int COUT>
 __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_t* s_idx, bool wide, uint32_t tmem,
@@ -378,7 +378,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                                          const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
                                          const uint8_t* __restrict__ wtiles, const EpiConst& epi, int relu, int batch,
                                          int max_voxels, int kvol, __half* __restrict__ dense,
-                                         const int4* __restrict__ out_coors, int D, int H, int W, int* tile_counter,
+                                         const int4* __restrict__ out_coors, int D, int H, int W, int* tile_counter, uint32_t first_mask,
                                          bool ahead, bool wait_first, int withhold_weights) {   // returns a gather warp's uses of its slot
     constexpr int KG = 64 / CIN, CPO = CIN / 8, B_BYTES = COUT * ROW_BYTES;
     constexpr uint32_t IDESC = umma_idesc(COUT);
@@ -550,23 +550,22 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
         }
         __syncwarp();
     } else if (warp == INDEX_WARP) {
-        // the CTA's tiles and their indices. ahead: the next tile is taken while the last one is in work; where there is no more
-        // than a tile per CTA, those that start first would take two.
+        // the CTA's tiles and their indices. ahead: there are more tiles than CTAs, and the next one is taken while the last one is in
+        // work.
         for (uint32_t round = 0;; ++round) {
             const uint32_t r = round & 1u;
-            if (!waited && round >= (ahead ? 2u : 1u)) {
+            if (!waited && round >= 2u) {
                 pdl_enter();
                 waited = true;
             }
-            if (!ahead && round > 0) {
-                const bool ok = mbar_wait(smem_u32(tile_free + (r ^ 1u)), ((round - 1u) >> 1) & 1u, abort_flag, 7 | (int)(round << 4));
-                if (!__all_sync(0xFFFFFFFFu, ok)) break;
+            // the first tile is that of the CTA's number, the others are handed out
+            int t = blockIdx.x;
+            if (round > 0 && ahead) {
+                if (lane == 0) t = (int)gridDim.x + atomicAdd(tile_counter, 1);
+                t = __shfl_sync(0xFFFFFFFFu, t, 0);
             }
-            int t = 0;
-            if (lane == 0) t = atomicAdd(tile_counter, 1);
-            t = __shfl_sync(0xFFFFFFFFu, t, 0);
             int frame = -1, first = 0, rows = 0;
-            for (int f0 = 0; f0 < batch && frame < 0; f0 += 32) {
+            for (int f0 = 0; f0 < batch && frame < 0 && (round == 0 || ahead); f0 += 32) {
                 int n = f0 + lane < batch ? __ldg(out_num + f0 + lane) : 0;
                 n = n > max_voxels ? max_voxels : (n < 0 ? 0 : n);
                 const int tiles = (n + TILE_M - 1) / TILE_M;
@@ -585,7 +584,9 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 }
                 t -= __shfl_sync(0xFFFFFFFFu, incl, 31);
             }
-            const int mask = frame < 0 ? 0 : (int)__ldg(tile_mask + (size_t)frame * tiles_per_frame + first / TILE_M);
+            int mask = (int)first_mask;
+            if (round > 0 || batch > 1) mask = (int)__ldg(tile_mask + (size_t)(frame < 0 ? 0 : frame) * tiles_per_frame + first / TILE_M);
+            if (frame < 0) mask = 0;
             bool ok = mbar_wait(smem_u32(tile_free + r), ((round >> 1) & 1u) ^ 1u, abort_flag, 7 | (int)(round << 4));
             ok = __all_sync(0xFFFFFFFFu, ok);
             if (!ok) break;
@@ -642,6 +643,11 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int nstages = (kvol + KG - 1) / KG;
+    const int tiles_per_frame = (max_voxels + TILE_M - 1) / TILE_M;
+    // few-tiles path, a single frame: the mask of the CTA's first tile, requested before anything else
+    uint32_t first_mask = 0;
+    if (warp == INDEX_WARP && batch == 1 && (int)blockIdx.x < tiles_per_frame)   // (volatile: not ahead of the wait above)
+        asm volatile("ld.global.u32 %0, [%1];" : "=r"(first_mask) : "l"(tile_mask + blockIdx.x) : "memory");
 
     if (tid < THREADS / 2) {   // side by side: one thread would take half a microsecond for the hundred and more barriers
         if (tid < NSLOT) {
@@ -672,7 +678,6 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    const int tiles_per_frame = (max_voxels + TILE_M - 1) / TILE_M;
     if (warp == EPI_WARPS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&ctl->tmem_base)),
                      "r"(TMEM_COLS)
@@ -744,7 +749,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));
         few_uses = umma_few<CIN, COUT>(ctl, sA, few_idx, wide, tmem, leader, in, out, nbr, order, tile_mask, out_num, wtiles, epi,
                                        relu, batch, max_voxels, kvol, dense, out_coors, D, H, W, tile_counter,
-                                       total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
+                                       first_mask, total_tiles > (int)gridDim.x, !maps_ready, withhold_weights);
     }
     if (!few) {
         if (tid == 0) ctl->range_lo = 0, ctl->range_hi = total_tiles;   // (the next barrier comes before anyone's cut point)
