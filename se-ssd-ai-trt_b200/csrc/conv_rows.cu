@@ -119,6 +119,13 @@ struct Row<float, CIN> {
     }
 };
 
+// A read that stays behind the wait for the preceding kernel (the compiler may move one that is said to be constant ahead of it).
+__device__ __forceinline__ int load_late(const int32_t* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 __device__ __forceinline__ float weight_as_float(float w) { return w; }
 __device__ __forceinline__ float weight_as_float(__half w) { return __half2float(w); }
 
@@ -159,7 +166,7 @@ conv_rows_kernel(const __grid_constant__ RowsArgs a) {
     const int tiles_per_frame = (a.max_voxels + 127) / 128, stride = (int)gridDim.x * (R::WARPS / R::PARTS);
     int f0 = 0, before = 0, rows = 0, incl = 0;
     auto load_frames = [&]() {
-        rows = f0 + lane < a.batch ? __ldg(a.out_num + f0 + lane) : 0;
+        rows = f0 + lane < a.batch ? load_late(a.out_num + f0 + lane) : 0;
         rows = rows > a.max_voxels ? a.max_voxels : (rows < 0 ? 0 : rows);
         incl = (rows + R::RUN - 1) / R::RUN;
 #pragma unroll
@@ -182,9 +189,10 @@ conv_rows_kernel(const __grid_constant__ RowsArgs a) {
         const int src = __ffs((int)__ballot_sync(0xFFFFFFFFu, it < before + incl)) - 1;
         const int n = __shfl_sync(0xFFFFFFFFu, rows, src);
         const int pos = (it - before - (__shfl_sync(0xFFFFFFFFu, incl, src) - (n + R::RUN - 1) / R::RUN)) * R::RUN;
-        const int2 runs = __ldg(reinterpret_cast<const int2*>(a.nbr + nbr_runs_index(a.kvol, a.max_voxels, f0 + src, pos)));
-        return Run{f0 + src, pos, n, __ldg(a.tile_mask + (size_t)(f0 + src) * tiles_per_frame + (pos >> 7)) &
-                                         (uint32_t)(runs.x | (pos + 32 < n ? runs.y : 0))};
+        const int32_t* runs = a.nbr + nbr_runs_index(a.kvol, a.max_voxels, f0 + src, pos);
+        const int offsets = load_late(runs) | (pos + 32 < n ? load_late(runs + 1) : 0);
+        return Run{f0 + src, pos, n,
+                   (uint32_t)(load_late(reinterpret_cast<const int32_t*>(a.tile_mask) + (size_t)(f0 + src) * tiles_per_frame + (pos >> 7)) & offsets)};
     };
     // Offsets go through a run's buffer up to ROUND at a time: `more` gets those that are left.
     auto split = [&](uint32_t mask, uint32_t* more) {
