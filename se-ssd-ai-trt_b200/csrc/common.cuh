@@ -184,6 +184,8 @@ __host__ __device__ inline size_t nbr_index(int kvol, int max_voxels, int b, int
 }
 // The padding behind a tile's first offset holds four words, for each 32 of its rows a mask of offsets: at least those that any of
 // the 32 has a neighbour under (all ones where a map's builder does not say; bits that the tile's mask lacks mean nothing).
+// (map_tiles_kernel writes them where a call has room for more than kRunRows rows: conv_rows.cu, which reads them, takes no others.)
+constexpr int kRunRows = 300000;
 __host__ __device__ inline size_t nbr_runs_index(int kvol, int max_voxels, int b, int o) {
     return nbr_index(kvol, max_voxels, b, 0, o & ~127) + 128 + ((o >> 5) & 3);
 }

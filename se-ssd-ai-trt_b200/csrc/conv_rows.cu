@@ -374,7 +374,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
 // A weight that is no finite number must not reach the rows without its neighbour, which multiply it by zero here. Rows are read in
 // pieces of 8 (halves) or 16 bytes and written in pieces of 16.
 bool conv_rows_takes(const ConvLaunch& c) {
-    if ((int64_t)c.batch * c.max_voxels <= 300000 || !c.weights_finite || !c.tile_mask || c.kvol > ROWS_KVOL_MAX) return false;
+    if ((int64_t)c.batch * c.max_voxels <= kRunRows || !c.weights_finite || !c.tile_mask || c.kvol > ROWS_KVOL_MAX) return false;
     const bool half = c.dtype == SESSD_F16;
     if (c.cout != 16 || !(c.cin == 4 || (c.cin == 16 && !half))) return false;
     return reinterpret_cast<uintptr_t>(c.in) % (half ? 8 : 16) == 0 && reinterpret_cast<uintptr_t>(c.out) % 16 == 0;

@@ -495,7 +495,7 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
 // kernel's planes each: the launch's choice. Also zeroes the tails of the call's outputs, whose row counts are known by now.
 template <int PLANES>
 __global__ void __launch_bounds__(128 * PLANES)
-map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, int tiles_per_frame, TailRows tails) {
+map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, int tiles_per_frame, TailRows tails, int runs) {
     pdl_enter();
     zero_tails(tails);
     __shared__ uint32_t s_mask[4 * PLANES];
@@ -514,13 +514,17 @@ map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, 
         __syncthreads();
         if (lane == 0) s_mask[warp] = any;
         __syncthreads();
-        if (warp == 0) {
-            uint32_t m = 0;                                  // of 32 rows: lane's quarter of the tile
+        if (tid == 0) {
+            uint32_t m = 0;
 #pragma unroll
-            for (int p = 0; p < PLANES; ++p) m |= s_mask[4 * p + (lane & 3)];
-            if (lane < 4) job.nbr[nbr_runs_index(job.g.kvol, max_voxels, b, p0 + 32 * lane)] = (int32_t)m;
-            m = __reduce_or_sync(0xFFFFFFFFu, m);
-            if (lane == 0) job.tile_mask[it] = m;
+            for (int w = 0; w < 4 * PLANES; ++w) m |= s_mask[w];
+            job.tile_mask[it] = m;
+        }
+        if (runs && tid < 4) {                               // of 32 rows each
+            uint32_t m = 0;
+#pragma unroll
+            for (int p = 0; p < PLANES; ++p) m |= s_mask[4 * p + tid];
+            job.nbr[nbr_runs_index(job.g.kvol, max_voxels, b, p0 + 32 * tid)] = (int32_t)m;
         }
     }
 }
@@ -571,6 +575,7 @@ int launch_map_windows(const MapJobs& jobs, int batch, int max_voxels, const Row
 int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRows& tails, cudaStream_t stream) {
     const int tiles = (max_voxels + 127) / 128;
     const int64_t items = (int64_t)batch * tiles;
+    const int runs = (int64_t)batch * max_voxels > kRunRows ? 1 : 0;
     // A thread per plane up to room for twelve tiles per SM: the planes of a row one after the other are what a small call waits for.
     // Beyond that the reads bound the SMs, and three times the threads read coordinates and row counts. (This kernel in us, a thread
     // per row and three, 4 -> 16, 32 -> 32 and 64 -> 64 channels: room for 469 tiles, 1 x 20,000 points 17.1 and 11.3, 19.1 and 13.0,
@@ -579,14 +584,14 @@ int launch_map_tiles(const MapJob& job, int batch, int max_voxels, const TailRow
     // 13.2; 2,814, 3 x 60,000 28.5 and 31.7, 41.4 and 44.8, 13.1 and 14.2; 3,126, 2 x 120,000 36.2 and 44.0, 55.0 and 62.3, 12.6 and
     // 13.2; 5,628, 12 x 20,000 45.4 and 51.0, 62.4 and 74.1, 25.2 and 30.0.)
     if (items <= persistent_grid(12)) {
-        SESSD_LAUNCH(map_tiles_kernel<3>, (int)items, 384, 0, stream, job, batch, max_voxels, tiles, tails);
+        SESSD_LAUNCH(map_tiles_kernel<3>, (int)items, 384, 0, stream, job, batch, max_voxels, tiles, tails, runs);
         return SESSD_OK;
     }
     // four rounds of the nine blocks that are resident: with six per SM the reads in flight did not cover their latency, and in few
     // rounds the blocks whose tiles are empty leave SMs idle (calls of 8 x 120,000 points, 4 -> 16 channels: six 334 us, nine 318,
     // eighteen 307, thirty-six 304; 4 x 20,000 points, 16 -> 16: 54, 53, 44, 44)
     const int most = persistent_grid(36);
-    SESSD_LAUNCH(map_tiles_kernel<1>, (int)(items < most ? items : most), 128, 0, stream, job, batch, max_voxels, tiles, tails);
+    SESSD_LAUNCH(map_tiles_kernel<1>, (int)(items < most ? items : most), 128, 0, stream, job, batch, max_voxels, tiles, tails, runs);
     return SESSD_OK;
 }
 
