@@ -1,5 +1,5 @@
 // C ABI of the library: parameter validation, workspace layout and launch sequencing.
-// No kernel lives here; see voxelize.cu, rulebook.cu, conv_simt.cu, conv_f32.cu, conv_umma.cu,
+// No kernel lives here; see voxelize.cu, rulebook.cu, conv_simt.cu, conv_rows.cu, conv_f32.cu, conv_umma.cu,
 // sparse2dense.cu.
 #include <cmath>
 #include <cstdio>

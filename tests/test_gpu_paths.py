@@ -199,6 +199,29 @@ def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, cin, d
     assert names[0].startswith("conv_rows") and names[1].startswith("conv_narrow")
 
 
+@pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 64), (64, 64)])
+@pytest.mark.parametrize("rows", [1, 700, 148 * 128 * 10 + 200])
+def test_fp16_rows_at_16_but_not_32_byte_boundaries(gpu, cin, cout, rows):
+    """Output rows leave 32 bytes at a time, or 16 where they start at odd multiples of 16 bytes: the same bits, in the few-tiles path
+    and in groups (more than ten tiles per SM). (All rows are in use.)"""
+    import torch
+
+    rs = np.random.RandomState(cin + rows)
+    shape = (6, 20, 30) if rows < 1000 else (12, 200, 160)
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
+    coors = torch.from_numpy(_random_coords(rs, rows, shape))[None].cuda()
+    num = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, rows)
+    w = gpu.ConvWeights(p, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), None, None, True, 1)
+    x = torch.randn((1, rows, cin), device="cuda").half()
+    r = gpu.subm_conv(x, coors, num, p, w, keep_workspace=True)
+    assert r["status"] == 0 and r["features"].data_ptr() % 32 == 0
+    out = torch.empty(rows * cout + 8, dtype=torch.float16, device="cuda")[8:].view(1, rows, cout)
+    gpu.subm_conv_into(x, coors, num, p, w, out, r["workspace"])
+    assert torch.equal(out, r["features"])
+    w.close()
+
+
 @pytest.mark.parametrize("rows", [148 * 128, 148 * 128 + 1])
 def test_fp16_tiles_around_one_per_sm(gpu, oracle, rows):
     rs = np.random.RandomState(rows)
