@@ -60,12 +60,14 @@ constexpr int ROW_BYTES = 128;               // 64 halves per A/B row
 constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
 // Few-tiles path: up to this many tiles per CTA. It fetches a weight block per item instead of one for up to four tiles, but is
-// through sooner and shares the tiles out by a counter. In us, without the path / with one tile per CTA, three, six, ten, any number:
-// front end of 1 x 20,000 points 250 (239 at one), 227 from three on; 3 x 20,000 389, 385, 369, 365, 365; 5 x 77,000 721, 725, 705, 708,
-// 714; 3 x 120,000 824, -, 805, 805, 840; 8 x 120,000 1858, -, 1857, 1856, 1933. Calls of 64 -> 64 channels: 8 tiles per CTA 87.2 and
-// with the path 84.5, 16 tiles 151.0 and 154.4. (Groups have become faster since: four, seven, ten: 3 x 20,000 369, 354, 354; 5 x 77,000
-// 698, 690, 693; 64 -> 64 with 8 tiles per CTA 84.7, 84.7, 83.2.)
-constexpr int FEW_TILES = 10;
+// through sooner, shares the tiles out by a counter and pays nothing for a group's boundary. Layers in us (events around the launch),
+// groups and this path: 64 -> 64 with 11 tiles per CTA (8 x 20,000 points) 63.6 and 59.5, 14 (10 x 20,000) 74.0 and 70.1, 20 (5 x 77,000)
+// 80.0 and 74.1, 33 (8 x 120,000) 150.0 and 144.0, 45 (32 x 20,000)
+// 201 and 191, 131 (32 x 120,000) 575 and 578; 32 -> 64 with 45 117 and 113; 32 -> 32 with 20 (10 x 20,000) 59.6 and 55.5, 32 84.2 and 82.3; with 16 channels, whose items are few, 16 -> 32 with 12
+// (6 x 20,000) 26.9 and 27.0, 16 (8 x 20,000) 31.0 and 35.1, 20 35.1 and 39.1. Lower lines than ten are slower everywhere (front end of 3 x
+// 20,000 points at four, six, eight and ten 338, 326, 319, 319).
+template <int CIN>
+__host__ __device__ constexpr int few_tiles() { return CIN == 16 ? 14 : 50; }
 constexpr int FEW_SLOTS = 8;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
 // instructions, with the issuer.
@@ -743,7 +745,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     }
     // A layer with the BEV scatter takes the few-tiles path whatever its size: it has three offsets, and the scatter's stores, two bytes
     // to a channel and row, are what it does; there eight warps share them. (32 frames of 120,000 points: four warps 190 us, eight 139.)
-    const bool few = tile_counter != nullptr && (dense != nullptr || total_tiles <= FEW_TILES * (int)gridDim.x);
+    const bool few = tile_counter != nullptr && (dense != nullptr || total_tiles <= few_tiles<CIN>() * (int)gridDim.x);
     if (few) {
         static_assert(FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX, "whole stages of indices");
         int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));

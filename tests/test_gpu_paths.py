@@ -200,14 +200,14 @@ def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, cin, d
 
 
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 64), (64, 64)])
-@pytest.mark.parametrize("rows", [1, 700, 148 * 128 * 10 + 200])
+@pytest.mark.parametrize("rows", [1, 700, 148 * 128 * 50 + 200])
 def test_fp16_rows_at_16_but_not_32_byte_boundaries(gpu, cin, cout, rows):
     """Output rows leave 32 bytes at a time, or 16 where they start at odd multiples of 16 bytes: the same bits, in the few-tiles path
-    and in groups (more than ten tiles per SM). (All rows are in use.)"""
+    and in groups (more than 50 tiles per SM). (All rows are in use.)"""
     import torch
 
     rs = np.random.RandomState(cin + rows)
-    shape = (6, 20, 30) if rows < 1000 else (12, 200, 160)
+    shape = (6, 20, 30) if rows < 1000 else (20, 250, 210)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
     coors = torch.from_numpy(_random_coords(rs, rows, shape))[None].cuda()
     num = torch.tensor([rows], dtype=torch.int32, device="cuda")
@@ -293,6 +293,59 @@ def test_fp16_tiles_on_both_sides_of_the_few(gpu, oracle, cin, cout, extra):
     for b in range(frames):
         alone = gpu.subm_conv(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
         assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
+
+
+@pytest.mark.parametrize("cin,cout,line", [(16, 16, 14), (16, 32, 14), (32, 32, 50), (32, 64, 50), (64, 64, 50)])
+@pytest.mark.parametrize("extra", [0, 1])
+def test_fp16_tiles_on_both_sides_of_the_line_between_the_paths(gpu, cin, cout, line, extra):
+    """The most tiles that the few-tiles path takes (14 per SM with 16 input channels, 50 with more), and one more, which goes through
+    groups of four. Frames have the bits of calls on them alone (which are few tiles)."""
+    import torch
+
+    rs = np.random.RandomState(cin + cout + extra)
+    frames, total = 11, line * torch.cuda.get_device_properties(0).multi_processor_count + extra
+    tiles = [total // frames + (1 if b < total % frames else 0) for b in range(frames)]
+    rows = [128 * t - 7 * b for b, t in enumerate(tiles)]
+    V = max(rows) + 3
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (20, 120, 110))
+    coors = torch.from_numpy(_random_coords(rs, V, layer.in_shape)).cuda().expand(frames, V, 4).contiguous()
+    feat = torch.randn((frames, V, cin), device="cuda").half()
+    num = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, V)
+    w = gpu.ConvWeights(p, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), None, None, True, 1)
+    r = gpu.subm_conv(feat, coors, num, p, w)
+    assert r["status"] == 0
+    for b in (0, 4, 10):
+        alone = gpu.subm_conv(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
+        assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
+    w.close()
+
+
+@pytest.mark.parametrize("cin", [32, 64])
+def test_groups_that_wait_for_weights_in_vain_report_it(gpu, cin):
+    """More than 50 tiles per SM, with either kind of issuer, and the test hook that keeps the weights back: the issuers' waits run out
+    and are reported, and the same call without the hook gives what it gave before."""
+    import torch
+
+    rs = np.random.RandomState(cin)
+    n = 128 * 50 * torch.cuda.get_device_properties(0).multi_processor_count + 100
+    layer = _layer(gpu, True, cin, cin, (3, 3, 3), (1, 1, 1), (1, 1, 1), (20, 250, 210))
+    coors = torch.from_numpy(_random_coords(rs, n, layer.in_shape))[None].cuda()
+    num = torch.tensor([n], dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, n)
+    w = gpu.ConvWeights(p, (rs.randn(27, cin, cin) * 0.05).astype(np.float32), None, None, False, 1)
+    x = torch.randn((1, n, cin), device="cuda").half()
+    want = gpu.subm_conv(x, coors, num, p, w)
+    assert want["status"] == 0
+    assert gpu.lib().sessd_conv_weights_debug_withhold(w.handle, 1) == 0
+    try:
+        r = gpu.subm_conv(x, coors, num, p, w, keep_workspace=True)
+    finally:
+        gpu.lib().sessd_conv_weights_debug_withhold(w.handle, 0)
+    assert r["status"] & gpu.STATUS_TIMEOUT and int(r["workspace"][4:8].view(torch.int32)[0]) & 15 == 5
+    again = gpu.subm_conv(x, coors, num, p, w)
+    assert again["status"] == 0 and torch.equal(again["features"], want["features"])
+    w.close()
 
 
 def test_few_fp16_tiles_some_without_neighbours(gpu):
