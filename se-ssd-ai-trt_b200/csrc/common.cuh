@@ -207,11 +207,33 @@ struct ConvGeom {
 // the stream's previous kernel has finished. pdl_wait() returns when that kernel has completed and its writes can be
 // seen; pdl_release() allows the next kernel to start. A kernel releases only after its own wait: when a kernel runs,
 // everything before its predecessor is therefore complete, and it may read that even before its own wait.
+// What the predecessor itself has written (and, in a call's first kernel, any input) must not be read as a constant right behind the
+// wait: __ldg and reads through const __restrict__ parameters may be moved ahead of it by the compiler (seen with a tile's mask, which
+// came back as the call before had left it). Such a read is a load_late, unless what it reads or whether it is made depends on a
+// value that came from one.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_enter() {
     pdl_wait();
     pdl_release();
+}
+
+__device__ __forceinline__ int load_late(const int32_t* p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint32_t load_late(const uint32_t* p) { return (uint32_t)load_late(reinterpret_cast<const int32_t*>(p)); }
+__device__ __forceinline__ float load_late(const float* p) { return __int_as_float(load_late(reinterpret_cast<const int32_t*>(p))); }
+__device__ __forceinline__ __half load_late(const __half* p) {
+    unsigned short v;
+    asm volatile("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p) : "memory");
+    return __ushort_as_half(v);
+}
+__device__ __forceinline__ uint4 load_late(const uint4* p) {
+    uint4 v;
+    asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
 }
 
 __device__ __forceinline__ uint32_t hash_slot(uint32_t key, int shift) {

@@ -100,7 +100,7 @@ __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long
 }
 
 __device__ __forceinline__ int f32_frame_rows(const F32Args& a, int f) {
-    const int n = f < a.batch ? __ldg(a.out_num + f) : 0;
+    const int n = f < a.batch ? load_late(a.out_num + f) : 0;
     return n > a.max_voxels ? a.max_voxels : (n < 0 ? 0 : n);
 }
 

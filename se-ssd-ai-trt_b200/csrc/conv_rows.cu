@@ -119,13 +119,6 @@ struct Row<float, CIN> {
     }
 };
 
-// A read that stays behind the wait for the preceding kernel (the compiler may move one that is said to be constant ahead of it).
-__device__ __forceinline__ int load_late(const int32_t* p) {
-    int v;
-    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
 __device__ __forceinline__ float weight_as_float(float w) { return w; }
 __device__ __forceinline__ float weight_as_float(__half w) { return __half2float(w); }
 
@@ -192,7 +185,7 @@ conv_rows_kernel(const __grid_constant__ RowsArgs a) {
         const int32_t* runs = a.nbr + nbr_runs_index(a.kvol, a.max_voxels, f0 + src, pos);
         const int offsets = load_late(runs) | (pos + 32 < n ? load_late(runs + 1) : 0);
         return Run{f0 + src, pos, n,
-                   (uint32_t)(load_late(reinterpret_cast<const int32_t*>(a.tile_mask) + (size_t)(f0 + src) * tiles_per_frame + (pos >> 7)) & offsets)};
+                   load_late(a.tile_mask + (size_t)(f0 + src) * tiles_per_frame + (pos >> 7)) & (uint32_t)offsets};
     };
     // Offsets go through a run's buffer up to ROUND at a time: `more` gets those that are left.
     auto split = [&](uint32_t mask, uint32_t* more) {

@@ -180,7 +180,7 @@ conv_narrow_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t*
         for (; next < items; next += gridDim.x) {
             b_next = next / chunks;
             o_next = (next - b_next * chunks) * ROWS;
-            n_next = __ldg(out_num + b_next);
+            n_next = load_late(out_num + b_next);
             n_next = n_next > max_voxels ? max_voxels : n_next;
             if (o_next < n_next) break;
         }
@@ -293,7 +293,7 @@ conv_generic_kernel(const T* __restrict__ in, T* __restrict__ out, const int32_t
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
         const int p = (it - b * chunks) * ROWS + wrow;
-        int n = out_num[b];
+        int n = load_late(out_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (p >= n) continue;
         const int32_t* nb = nbr + nbr_index(kvol, max_voxels, b, 0, p);

@@ -568,7 +568,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
             }
             int frame = -1, first = 0, rows = 0;
             for (int f0 = 0; f0 < batch && frame < 0 && (round == 0 || ahead); f0 += 32) {
-                int n = f0 + lane < batch ? __ldg(out_num + f0 + lane) : 0;
+                int n = f0 + lane < batch ? load_late(out_num + f0 + lane) : 0;
                 n = n > max_voxels ? max_voxels : (n < 0 ? 0 : n);
                 const int tiles = (n + TILE_M - 1) / TILE_M;
                 int incl = tiles;
@@ -587,7 +587,7 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
                 t -= __shfl_sync(0xFFFFFFFFu, incl, 31);
             }
             int mask = (int)first_mask;
-            if (round > 0 || batch > 1) mask = (int)__ldg(tile_mask + (size_t)(frame < 0 ? 0 : frame) * tiles_per_frame + first / TILE_M);
+            if (round > 0 || batch > 1) mask = (int)load_late(tile_mask + (size_t)(frame < 0 ? 0 : frame) * tiles_per_frame + first / TILE_M);
             if (frame < 0) mask = 0;
             bool ok = mbar_wait(smem_u32(tile_free + r), ((round >> 1) & 1u) ^ 1u, abort_flag, 7 | (int)(round << 4));
             ok = __all_sync(0xFFFFFFFFu, ok);
@@ -648,8 +648,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     const int tiles_per_frame = (max_voxels + TILE_M - 1) / TILE_M;
     // few-tiles path, a single frame: the mask of the CTA's first tile, requested before anything else
     uint32_t first_mask = 0;
-    if (warp == INDEX_WARP && batch == 1 && (int)blockIdx.x < tiles_per_frame)   // (volatile: not ahead of the wait above)
-        asm volatile("ld.global.u32 %0, [%1];" : "=r"(first_mask) : "l"(tile_mask + blockIdx.x) : "memory");
+    if (warp == INDEX_WARP && batch == 1 && (int)blockIdx.x < tiles_per_frame) first_mask = load_late(tile_mask + blockIdx.x);
 
     if (tid < THREADS / 2) {   // side by side: one thread would take half a microsecond for the hundred and more barriers
         if (tid < NSLOT) {
@@ -708,7 +707,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     // tile sequence, a block scan turns the sums into running totals, and the threads whose slice holds cut
     // point blockIdx.x or blockIdx.x + 1 walk the slice to the tile where the running total passes the target.
     auto frame_rows = [&](int f) {
-        const int v = __ldg(out_num + f);
+        const int v = load_late(out_num + f);
         return v > max_voxels ? max_voxels : (v < 0 ? 0 : v);
     };
     // Tiles before every frame, in shared memory that nothing uses yet. (Row counts and masks are read side by side: one

@@ -29,7 +29,7 @@ __device__ __forceinline__ void zero_rows(void* tensor, int units, const TailRow
     memset(&zero, 0, sizeof(V));
     for (int64_t it = blockIdx.x; it < (int64_t)t.batch * chunks; it += gridDim.x) {
         const int b = (int)(it / chunks), c = (int)(it - (int64_t)b * chunks);
-        const int most = min(t.most, t.max_rows), n = max(0, min(__ldg(t.counts + b), most));
+        const int most = min(t.most, t.max_rows), n = max(0, min(load_late(t.counts + b), most));
         const int64_t low = (int64_t)n * units, at = (int64_t)c * threads * PER;
         if (at + threads * PER <= low) continue;       // uniform over the block
         V* base = static_cast<V*>(tensor) + (int64_t)b * per_frame;

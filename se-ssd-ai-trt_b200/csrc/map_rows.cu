@@ -322,7 +322,7 @@ __device__ __forceinline__ void row_means(const RowMeans& m, T* voxels, int batc
     for (int it = block; it < batch * chunks; it += blocks) {
         const int b = it / chunks;
         const int row = (it - b * chunks) * kMapThreads + threadIdx.x;
-        if (row >= __ldg(m.voxel_num + b)) continue;
+        if (row >= load_late(m.voxel_num + b)) continue;
         uint32_t pi[kMaxPointsPerVoxel];
         list_load(m.lists + ((size_t)b * m.max_points + row) * m.max_pts, m.max_pts, pi);
         int cnt;
@@ -343,7 +343,7 @@ map_windows_kernel(const __grid_constant__ MapJobs jobs, int batch, int max_voxe
     auto pair_rows = [&](int p) {
         if (p >= pairs) return 0;
         const int j = p / batch;
-        const int v = __ldg(jobs.job[j].out_num + (p - j * batch));
+        const int v = load_late(jobs.job[j].out_num + (p - j * batch));
         return v > max_voxels ? max_voxels : (v < 0 ? 0 : v);
     };
     int pair0 = 0, before = 0, my_rows = pair_rows(lane), incl = 0;
@@ -502,7 +502,7 @@ map_tiles_kernel(const __grid_constant__ MapJob job, int batch, int max_voxels, 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, plane = tid >> 7, row = tid & 127;
     for (int it = blockIdx.x; it < batch * tiles_per_frame; it += gridDim.x) {
         const int b = it / tiles_per_frame, p0 = (it - b * tiles_per_frame) * 128;
-        int n = __ldg(job.out_num + b);
+        int n = load_late(job.out_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (p0 >= n) continue;
         const bool live = p0 + row < n;

@@ -42,7 +42,7 @@ channels_last_kernel(const __half* __restrict__ in, __half* __restrict__ out, in
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
             const int c = c0 + warp + 8 * (i >> 1), p = p0 + lane + 32 * (i & 1);
-            v[i] = c < channels && p < pixels ? src[(size_t)c * pixels + p] : __half(0.f);
+            v[i] = c < channels && p < pixels ? load_late(src + (size_t)c * pixels + p) : __half(0.f);
         }
         __syncthreads();                       // the previous tile has been written out
 #pragma unroll
@@ -66,7 +66,7 @@ bias_relu_kernel(__half* __restrict__ y, const __half* __restrict__ bias, const 
                  int channels) {
     pdl_enter();                               // (the bias, too, may be the preceding kernel's work)
     float bv[8];
-    unpack8(__ldg(reinterpret_cast<const uint4*>(bias) + threadIdx.x % (channels / 8)), bv);
+    unpack8(load_late(reinterpret_cast<const uint4*>(bias) + threadIdx.x % (channels / 8)), bv);
     const int64_t stride = (int64_t)gridDim.x * kThreads;
     for (int64_t e = (int64_t)blockIdx.x * kThreads + threadIdx.x; e < vectors; e += 2 * stride) {
         uint4 v[2], a[2];
@@ -74,7 +74,7 @@ bias_relu_kernel(__half* __restrict__ y, const __half* __restrict__ bias, const 
         for (int i = 0; i < 2; ++i) {
             if (e + i * stride >= vectors) break;
             v[i] = reinterpret_cast<const uint4*>(y)[e + i * stride];
-            if (add) a[i] = __ldg(reinterpret_cast<const uint4*>(add) + e + i * stride);
+            if (add) a[i] = load_late(reinterpret_cast<const uint4*>(add) + e + i * stride);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -120,14 +120,14 @@ neck_tail_kernel(const __half* __restrict__ o0, const __half* __restrict__ o1, c
     const bool want_heads = heads.out[0] != nullptr;
     pdl_enter();                               // (the weights are arguments: they, too, may be the preceding kernel's work)
     float g0[8], g1[8];
-    unpack8(__ldg(reinterpret_cast<const uint4*>(gate_w) + l16), g0);
-    unpack8(__ldg(reinterpret_cast<const uint4*>(gate_w + C) + l16), g1);
-    const float b0 = __half2float(gate_b[0]), b1 = __half2float(gate_b[1]);
+    unpack8(load_late(reinterpret_cast<const uint4*>(gate_w) + l16), g0);
+    unpack8(load_late(reinterpret_cast<const uint4*>(gate_w + C) + l16), g1);
+    const float b0 = __half2float(load_late(gate_b)), b1 = __half2float(load_late(gate_b + 1));
     if (want_heads)
         for (int e = tid; e < NT * 8 * (C / 8); e += kThreads) {
             const int o = e / (C / 8), c = e % (C / 8) * 8;
             *reinterpret_cast<uint4*>(s_w + o * STRIDE + c) =
-                o < kHeadChannels ? __ldg(reinterpret_cast<const uint4*>(head_w + o * C + c)) : make_uint4(0u, 0u, 0u, 0u);
+                o < kHeadChannels ? load_late(reinterpret_cast<const uint4*>(head_w + o * C + c)) : make_uint4(0u, 0u, 0u, 0u);
         }
     const int64_t tiles = (pixels + kTilePixels - 1) / kTilePixels;
     for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
@@ -139,8 +139,8 @@ neck_tail_kernel(const __half* __restrict__ o0, const __half* __restrict__ o1, c
             const int p = (tid >> 4) + 16 * i;
             v0[i] = v1[i] = make_uint4(0u, 0u, 0u, 0u);
             if (p < rows) {
-                v0[i] = __ldg(reinterpret_cast<const uint4*>(o0 + (p0 + p) * C) + l16);
-                v1[i] = __ldg(reinterpret_cast<const uint4*>(o1 + (p0 + p) * C) + l16);
+                v0[i] = load_late(reinterpret_cast<const uint4*>(o0 + (p0 + p) * C) + l16);
+                v1[i] = load_late(reinterpret_cast<const uint4*>(o1 + (p0 + p) * C) + l16);
             }
         }
         __syncthreads();                       // the previous tile's rows and outputs have been used
@@ -196,7 +196,7 @@ neck_tail_kernel(const __half* __restrict__ o0, const __half* __restrict__ o1, c
                 for (int i = 0; i < 4; ++i) {
                     const int o = nt * 8 + (lane & 3) * 2 + (i & 1), p = warp * 16 + lane / 4 + (i >> 1) * 8;
                     if (o >= kHeadChannels) continue;
-                    const float v = round_half(round_half(acc[nt][i]) + __half2float(__ldg(head_b + o)));
+                    const float v = round_half(round_half(acc[nt][i]) + __half2float(load_late(head_b + o)));
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         const int ch = o - heads.first[q];

@@ -71,7 +71,7 @@ anchor_decode_kernel(const float* __restrict__ box_preds, float* __restrict__ ou
         const int i = (int)(e % g.anchors);
         float t[7], o[7];
 #pragma unroll
-        for (int j = 0; j < 7; ++j) t[j] = __ldg(box_preds + e * 7 + j);
+        for (int j = 0; j < 7; ++j) t[j] = load_late(box_preds + e * 7 + j);
         decode_box(g, i, t, o);
 #pragma unroll
         for (int j = 0; j < 7; ++j) out[e * 7 + j] = o[j];
@@ -150,7 +150,7 @@ box_count_kernel(FilterArgs a) {
         const int b = it / a.chunks, chunk = it - b * a.chunks;
         const int i = chunk * kThreads + threadIdx.x;
         int keep = 0;
-        if (i < a.anchors) keep = sigmoid(__ldg(a.cls + (size_t)b * a.anchors + i)) >= a.threshold ? 1 : 0;
+        if (i < a.anchors) keep = sigmoid(load_late(a.cls + (size_t)b * a.anchors + i)) >= a.threshold ? 1 : 0;
         const int n = block_sum(keep);
         if (threadIdx.x == 0) a.chunk_counts[it] = n;
     }
@@ -215,7 +215,7 @@ box_filter_kernel(FilterArgs a, AnchorGeom g) {
 #pragma unroll
     for (int i = 0; i < kFilterSteps; ++i) {
         const int e = first + i * 32 + lane;
-        logit[i] = i * 32 < per_warp && e < a.anchors ? __ldg(cls + e) : 0.0f;
+        logit[i] = i * 32 < per_warp && e < a.anchors ? load_late(cls + e) : 0.0f;
     }
     int count = 0;
 #pragma unroll

@@ -40,7 +40,7 @@ table_build_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ v
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
         const int i = (it - b * chunks) * kThreads + threadIdx.x;
-        int n = voxel_num[b];
+        int n = load_late(voxel_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (i >= n) continue;
         const int4 c = __ldg(&coors[(size_t)b * max_voxels + i]);  // (b, z, y, x)
@@ -74,7 +74,7 @@ nbr_build_kernel(const int4* __restrict__ out_coors, const int32_t* __restrict__
         const int r = it - b * (g.kvol * chunks);
         const int k = r / chunks;
         const int o = (r - k * chunks) * kThreads + threadIdx.x;
-        int n = out_num[b];
+        int n = load_late(out_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (o >= n) continue;
         const int4 c = __ldg(&out_coors[(size_t)b * max_voxels + o]);
@@ -102,7 +102,7 @@ rulebook_export_kernel(const int32_t* __restrict__ nbr, const uint32_t* __restri
                        uint32_t* __restrict__ pair_num) {
     pdl_enter();
     const int k = blockIdx.x;
-    int n = out_num[frame];
+    int n = load_late(out_num + frame);
     n = n > max_voxels ? max_voxels : n;
     const int32_t* col = nbr + nbr_index(kvol, max_voxels, frame, k, 0);   // entry o of the column: col[(o >> 7) * kvol * kNbrRun + (o & 127)]
     const uint32_t* mask = tile_mask + (size_t)frame * ((max_voxels + 127) / 128);
@@ -136,7 +136,7 @@ count_pairs_kernel(const int32_t* __restrict__ nbr, const uint32_t* __restrict__
         const int r = it - b * (kvol * chunks);
         const int k = r / chunks;
         const int p = (r - k * chunks) * kThreads + threadIdx.x;
-        int n = out_num[b];
+        int n = load_late(out_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (p < n && ((tile_mask[(size_t)b * tiles + (p >> 7)] >> k) & 1u) && nbr[nbr_index(kvol, max_voxels, b, k, p)] >= 0)
             ++local;
@@ -162,7 +162,7 @@ bucket_build_kernel(const int4* __restrict__ coors, const int32_t* __restrict__ 
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
         const int i = (it - b * chunks) * kThreads + threadIdx.x;
-        int n = voxel_num[b];
+        int n = load_late(voxel_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (i >= n) continue;
         const int4 c = __ldg(&coors[(size_t)b * max_voxels + i]);
@@ -188,7 +188,7 @@ mark_outputs_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
         const int i = (it - b * chunks) * kThreads + threadIdx.x;
-        int n = in_num[b];
+        int n = load_late(in_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (i >= n) continue;
         mark_row(__ldg(&in_coors[(size_t)b * max_voxels + i]), b, g, out);
@@ -212,7 +212,7 @@ nbr_clear_kernel(int32_t* __restrict__ nbr, const int32_t* __restrict__ out_num,
     const int64_t items = (int64_t)batch * chunks;
     for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = (int)(it / chunks);
-        const int n = min(__ldg(out_num + b), max_voxels);
+        const int n = min(load_late(out_num + b), max_voxels);
         const size_t w = ((size_t)(it - (int64_t)b * chunks) * kThreads + threadIdx.x) * 4;
         if (w < (size_t)((n + 127) / 128) * kvol * kNbrRun)
             *reinterpret_cast<int4*>(nbr + (size_t)b * frame_words + w) = make_int4(-1, -1, -1, -1);
@@ -231,7 +231,7 @@ scatter_rows_kernel(const int4* __restrict__ in_coors, const int32_t* __restrict
     for (int64_t it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = (int)(it / chunks);
         const int t = (int)(it - (int64_t)b * chunks) * kThreads + threadIdx.x;
-        const int n = min(__ldg(in_num + b), max_voxels);
+        const int n = min(load_late(in_num + b), max_voxels);
         if (t >= n * g.ncand) continue;
         int i, e[3], rest;
         split_small(t, g.span_max[2], &rest, &e[2]);
@@ -491,7 +491,7 @@ tile_mask_kernel(const int32_t* __restrict__ nbr, const int32_t* __restrict__ ou
         const int k = (int)(it % kvol);
         const int64_t bt = it / kvol;
         const int tile = (int)(bt % tiles_per_frame), b = (int)(bt / tiles_per_frame);
-        int n = out_num[b];
+        int n = load_late(out_num + b);
         n = n > max_voxels ? max_voxels : n;
         bool any = false;
         for (int q = 0; q < 4; ++q) {

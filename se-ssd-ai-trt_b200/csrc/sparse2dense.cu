@@ -23,7 +23,7 @@ sparse2dense_kernel(const T* __restrict__ feat, const int4* __restrict__ coors, 
     for (int it = blockIdx.x; it < items; it += gridDim.x) {
         const int b = it / chunks;
         const int64_t t = (int64_t)(it - b * chunks) * kThreads + threadIdx.x;
-        int n = voxel_num[b];
+        int n = load_late(voxel_num + b);
         n = n > max_voxels ? max_voxels : n;
         if (t >= (int64_t)n * C) continue;
         const int i = (int)(t / C), c = (int)(t - (int64_t)i * C);

@@ -98,7 +98,7 @@ __device__ __forceinline__ void for_points(const int32_t* __restrict__ points_si
 
 // Number of the record of an occupied word of a two-level grid.
 __device__ __forceinline__ int word_id(const BitGrid& grid, int b, uint32_t word) {
-    const uint4 t = __ldg(grid.top + (size_t)b * grid.top_words + (word >> 6));
+    const uint4 t = load_late(grid.top + (size_t)b * grid.top_words + (word >> 6));
     const unsigned long long bits = (unsigned long long)t.x | ((unsigned long long)t.y << 32);
     return (int)t.z + __popcll(bits & ((1ull << (word & 63)) - 1ull));
 }
@@ -108,7 +108,7 @@ __device__ __forceinline__ void push_points(const PointLists& l, int batch, int 
     for_points(l.points_size, batch, l.max_points, block, blocks, [&](int b, int p) {
         const uint32_t key = __ldg(l.pt_key + (size_t)b * l.max_points + p);
         if (key == kEmpty) return;
-        const uint4 r = __ldg(l.grid.rec + (size_t)b * l.grid.words + word_id(l.grid, b, key >> 6));
+        const uint4 r = load_late(l.grid.rec + (size_t)b * l.grid.words + word_id(l.grid, b, key >> 6));
         const unsigned long long bits = (unsigned long long)r.x | ((unsigned long long)r.y << 32);
         const int row = (int)r.z + __popcll(bits & ((1ull << (key & 63)) - 1ull));
         list_push(l.lists + ((size_t)b * l.max_points + row) * l.max_pts, l.max_pts, (uint32_t)p);

@@ -98,7 +98,7 @@ voxel_emit_kernel(const float4* __restrict__ points, const int32_t* __restrict__
 #pragma unroll
         for (int i = 0; i < STEPS; ++i) {
             const int e = e0 + i * kThreads;
-            claim[i] = e < n ? pt_claim[(size_t)b * max_points + e] : -1;
+            claim[i] = e < n ? load_late(pt_claim + (size_t)b * max_points + e) : -1;
         }
         uint32_t owner = 0;                        // bit i
         uint32_t mine = 0u;                        // counts of the steps, 16 bits each

@@ -1,5 +1,7 @@
 """GPU: the sizes at which a kernel changes its way of working, against the oracle (same tolerances as the tests whose helpers
 are used here: fp32 identical, fp16 1e-2 per layer)."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -729,4 +731,108 @@ def test_repeated_passes_give_the_same_bits(gpu):
             assert num.tolist() == n
             assert all(torch.equal(f[b, :n[b]], layer[b]) for b in range(4))
     assert gpu.read_status(ws) == 0
+    bb.close()
+
+
+def test_calls_in_turn_on_frames_of_other_sizes(gpu):
+    """Every kernel starts while the one before it runs, on buffers that still hold what the call before left there: calls on a large
+    and on a small frame in turn, in the same workspace and with nothing between them, give what each gives alone. (Voxeliser, the
+    submanifold layers of every kernel on its rows, a strided layer, and whole front ends.)"""
+    import torch
+
+    sizes = (12000, 700)
+    clouds = [torch.zeros((1, 12000, 4), device="cuda") for _ in sizes]
+    for x, n in zip(clouds, sizes):
+        x[0, :n] = torch.from_numpy(gpu.synth.lidar_frame(70 + n, n_points=n, n_boxes=9)).cuda()
+    nums = [torch.tensor([n], dtype=torch.int32, device="cuda") for n in sizes]
+    V, shape = 12000, (41, 1600, 1408)
+    vp = gpu.voxel_params(V)
+    L = gpu.schedule.ConvLayer
+    layers = []
+    rs = np.random.RandomState(70)
+    for cin, cout, dtype, subm in ((4, 16, 0, True), (4, 16, 1, True), (16, 16, 0, True), (16, 16, 1, True), (32, 32, 0, True),
+                                   (32, 64, 1, True), (8, 24, 0, True), (16, 32, 1, False), (32, 32, 0, False)):
+        l = L("l", subm, cin, cout, (3,) * 3, (1,) * 3, (1,) * 3, shape, shape) if subm else \
+            L("l", subm, cin, cout, (3,) * 3, (2,) * 3, (1,) * 3, shape, (21, 800, 704))
+        p = gpu.conv_params(l, V)
+        feat = torch.from_numpy(rs.randn(1, V, cin).astype(np.float16 if dtype else np.float32)).cuda()
+        layers.append((subm, p, gpu.ConvWeights(p, (rs.randn(27, cin, cout) * 0.1).astype(np.float32), None, None, True, dtype), feat))
+    vox = torch.empty((1, V, 4), device="cuda")
+    coors, num = torch.empty((1, V, 4), dtype=torch.int32, device="cuda"), torch.empty((1,), dtype=torch.int32, device="cuda")
+    ws = torch.empty(gpu.lib().sessd_voxelize_workspace_bytes(C.byref(vp), 1, 12000), dtype=torch.uint8, device="cuda")
+    conv_ws = [gpu._conv_workspace(p, 1, feat.device) for _subm, p, _w, feat in layers]
+
+    def run(which, apart):
+        outs = []
+        for i in which:
+            for (subm, p, w, feat), (cws, nbytes) in zip(layers, conv_ws):
+                o = (torch.empty((1, V, p.out_channel), dtype=feat.dtype, device="cuda"),
+                     torch.empty((1, V, 4), dtype=torch.int32, device="cuda"), torch.empty((1,), dtype=torch.int32, device="cuda"))
+                outs.append(o[:1] if subm else o)
+        torch.cuda.synchronize()
+        it = iter(outs)
+        for i in which:
+            for (subm, p, w, feat), (cws, nbytes) in zip(layers, conv_ws):
+                gpu.voxelize_into(clouds[i], nums[i], vp, vox, coors, num, ws, 0)
+                if apart:
+                    torch.cuda.synchronize()
+                args = (C.byref(p), w.handle, 1, gpu._vp(feat, coors, num), gpu._vp(*next(it)), cws.data_ptr(), nbytes, gpu._stream())
+                call = gpu.lib().sessd_subm_conv_enqueue if subm else gpu.lib().sessd_sparse_conv_enqueue
+                assert call(*args) == 0
+                if apart:
+                    torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return outs
+
+    turns = (0, 1, 0, 1, 1, 0, 0, 1)
+    alone = [run((i,), True) for i in (0, 1)]
+    rows = [int((a[0][0].abs().sum(2) > 0).sum()) for a in alone]
+    assert rows[0] > 10 * rows[1] > 0
+    got = run(turns, False)
+    for t, i in enumerate(turns):
+        for j, want in enumerate(alone[i]):
+            assert all(torch.equal(a, b) for a, b in zip(got[t * len(layers) + j], want)), (t, i, j)
+    for dtype in (0, 1):
+        w, sc, sh = gpu.random_weights()
+        bb = gpu.Backbone(20000, w, sc, sh, dtype=dtype)
+        bws = torch.empty(bb.workspace_bytes(1, 12000), dtype=torch.uint8, device="cuda")
+        want = [bb.run(clouds[i], nums[i])[0] for i in (0, 1)]
+        maps = [torch.empty_like(want[0]) for _ in turns]
+        torch.cuda.synchronize()
+        for m, i in zip(maps, turns):
+            bb.run(clouds[i], nums[i], bws, m)
+        torch.cuda.synchronize()
+        assert all(torch.equal(m, want[i]) for m, i in zip(maps, turns)), dtype
+        bb.close()
+
+
+def test_heads_and_filter_on_two_frames_in_turn(gpu):
+    """The layout kernel reads the map that the last convolution has written, the head kernel the branches, the filter the heads:
+    a captured detector on two frames in turn, and on each of them after itself."""
+    import torch
+
+    w, sc, sh = gpu.random_weights()
+    bb = gpu.Backbone(20000, w, sc, sh, dtype=1)
+    D = gpu.detector
+    blobs = D.random_neck_weights()
+    det = D.Detector(bb, D.Neck2D(blobs)).capture(12000)
+    pts, sizes = [], []
+    for n in (12000, 3000):
+        x = torch.zeros((1, 12000, 4), device="cuda")
+        x[0, :n] = torch.from_numpy(gpu.synth.lidar_frame(80 + n, n_points=n, n_boxes=9)).cuda()
+        pts.append(x)
+        sizes.append(torch.tensor([n], dtype=torch.int32, device="cuda"))
+
+    def replay(i):
+        out = det.replay(pts[i], sizes[i])
+        return [out["boxes"].clone(), out["num"].clone(), *(out["filtered"][k].clone() for k in ("box", "score", "valid")),
+                *(v.clone() for v in out["heads"].values())]
+
+    want = []
+    for i in (0, 1):
+        replay(i)
+        want.append(replay(i))
+    assert not torch.equal(want[0][5], want[1][5])
+    for i in (0, 1, 0, 1):
+        assert all(torch.equal(a, b) for a, b in zip(replay(i), want[i])), i
     bb.close()

@@ -120,3 +120,23 @@ def test_reference_arm_prints_the_contract_line():
     base = line["cpu_baseline"]
     assert base["kind"] == "port" and base["cores"] >= 1 and base["value"] == line["value"] and base["sample"]
     assert line["e2e"] == dict(value=line["value"], unit=line["unit"], h2d_bytes_per_step=0, d2h_bytes_per_step=0)
+
+
+def test_what_the_preceding_kernel_wrote_is_not_read_as_a_constant():
+    """Kernels start while their predecessor runs. A read that is said to be constant (__ldg, or a plain one through a const
+    __restrict__ parameter) may be moved ahead of the wait for it, so that row counts, which everything else depends on, and the
+    inputs that a kernel reads first go through load_late."""
+    import re
+
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "se-ssd-ai-trt_b200", "csrc")
+    read = {f: open(os.path.join(csrc, f)).read() for f in sorted(os.listdir(csrc)) if f.endswith((".cu", ".cuh"))}
+    counts = r"(?:out_num|in_num|voxel_num|counts)"
+    for name, text in read.items():
+        found = re.findall(r"__ldg\([\w.\[\]>-]*\b" + counts + r"\b[^;]*;", text)
+        found += re.findall(r"(?:=|\() *" + counts + r"\[[^\]]*\];", text)        # int n = out_num[b];
+        assert not found, (name, found)
+    # the first reads of kernels without row counts
+    for name, late in (("postprocess.cu", "load_late(cls + e)"), ("postprocess.cu", "load_late(box_preds +"), ("neck.cu", "load_late(src +"),
+                       ("voxelize.cu", "load_late(pt_claim +")):
+        assert late in read[name], (name, late)
+    assert "__ldg" not in read["neck.cu"]
