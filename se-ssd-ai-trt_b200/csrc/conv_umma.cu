@@ -16,7 +16,7 @@
 //   warps 0-3    epilogue (warp w reads tensor-memory lanes 32w .. 32w+31). The accumulators are double
 //                buffered (2 sets x 4 tiles x Cout columns), so the epilogue of one group runs while the
 //                other roles are already working on the next group. A thread holds one row and stores it 32 bytes
-//                at a time.
+//                at a time; 64 -> 64 channels go through a small staging area of the warp.
 //   warps 4-7    MMA issuers; issuer t owns tile t of every group. The warp works out the group's schedule
 //                once (lane g for stage g); it goes through it together, or with 64 input channels one elected lane alone,
 //                and that lane issues the tcgen05.mma and commit instructions (each costs its thread on the order of a
@@ -81,7 +81,8 @@ constexpr int FEW_IDX = 28;                  // offsets of a tile's index block 
 constexpr int TAP_WORDS = kNbrRun;
 static_assert(kNbrRun == TILE_M + 4, "the map's spacing between offsets is the index block's");
 
-// Gather slots (= gather warps): as many as fit beside the weight ring, the index blocks and the epilogue's staging area.
+// Gather slots (= gather warps): as many as fit beside the weight ring, the index blocks and, with 64 -> 64 channels, the epilogue's
+// staging area.
 // The index ring is deeper than the A ring (index rows come from DRAM, several microseconds away under load):
 // block j = q % NIDX, with NIDX a multiple of NSLOT so that block j is always read by gather warp j % NSLOT.
 template <int CIN>
@@ -216,10 +217,15 @@ struct SharedCtl {
 // Epilogue warps of the few-tiles path: with 64 channels a column block each for eight (warps 5-8 have nothing else to do there).
 template <int COUT>
 __host__ __device__ constexpr int few_epi_warps() { return COUT == 64 ? 2 * EPI_WARPS : EPI_WARPS; }
+// Groups: whether output rows go through shared memory (store_tile_staged), and an epilogue warp's room for it.
+template <int CIN, int COUT>
+__host__ __device__ constexpr bool groups_staged() { return CIN == 64 && COUT == 64; }
+constexpr int STAGE_BYTES = 32 * 64;
 // Buffers of the two paths, which share their place.
 template <int CIN, int COUT>
 __host__ __device__ constexpr int ring_bytes() {
-    constexpr int groups = Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES + Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4;
+    constexpr int groups = Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES + Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 +
+                           (groups_staged<CIN, COUT>() ? EPI_WARPS * STAGE_BYTES : 0);
     constexpr int few = FEW_SLOTS * (A_BYTES + COUT * ROW_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4;
     return groups > few ? groups : few;
 }
@@ -295,8 +301,8 @@ template <int COUT, int FROM = 0, int TO = COUT>
 __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiConst& epi, int relu, int pos, int row, int n, int b,
                                            int max_voxels, __half* __restrict__ out, bool wide, __half* __restrict__ dense,
                                            const int4* __restrict__ out_coors, int D, int H, int W) {
-    // Column blocks of CB channels keep the register footprint small.
-    constexpr int CB = COUT < 32 ? COUT : 32;
+    // Column blocks of CB channels keep the register footprint small (of 64 channels 32 at a time: these kernels spill).
+    constexpr int CB = COUT == 32 ? 32 : 16;
     __half* to = out + ((size_t)b * max_voxels + row) * COUT;
 #pragma unroll
     for (int cb = FROM; cb < TO; cb += CB) {
@@ -359,6 +365,53 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
                 }
             }
         }
+    }
+}
+
+// The same through the warp's staging area (32 rows of 64 bytes), four lanes to a row, without the scatter: groups of 64 -> 64 channels.
+// Where a tile has twenty items the epilogue has time, and what counts is how often it looks into L1, whose tags the gather warps' copies
+// keep busy: 64 lines of 128 bytes per 32 rows, where stores by row look 128 times. (In us, 64 -> 64 at 1/4 resolution, stores by row and
+// through here: 16 x 120,000 points 326 and 322, 24 477 and 473, 32 639 and 631, 40 798 and 789; 64 x 20,000 432 and 428. The other layers
+// have fewer items to a tile and are faster by row: 32 -> 64, 32 x 120,000, 445 and, by row, 396; 32 -> 32, 16 x 120,000, 380 and 379.)
+template <int COUT>
+__device__ __forceinline__ void store_tile_staged(uint32_t taddr, bool have, const EpiConst& epi, int relu, uint8_t* stage, int lane,
+                                                  int pos, int row, int n, int b, int max_voxels, __half* __restrict__ out) {
+    constexpr int CB = 32, RB = CB * 2, CPR = RB / 16;   // channels and bytes of a row's column block, its 16-byte pieces
+    static_assert(COUT % CB == 0, "whole column blocks");
+    // pieces XOR-swizzled by row, so that neither the writes nor the reads below meet in a bank
+    auto swizzled = [](int r, int piece) { return r * RB + ((piece ^ ((r >> 1) & 3)) << 4); };
+#pragma unroll
+    for (int cb = 0; cb < COUT; cb += CB) {
+#pragma unroll
+        for (int p0 = 0; p0 < CPR; p0 += 2) {            // sixteen columns
+            uint32_t acc[16] = {};
+            if (have) {
+                tmem_ld16(taddr + cb + 8 * p0, acc);
+                tmem_ld_wait();
+            }
+#pragma unroll
+            for (int p = 0; p < 2; ++p) {
+                uint32_t pk[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const int a = 8 * p + 2 * j, ch = cb + 8 * p0 + a;   // constants after unrolling
+                    __half2 h = __floats2half2_rn(fmaf(__uint_as_float(acc[a]), epi.scale[ch], epi.shift[ch]),
+                                                  fmaf(__uint_as_float(acc[a + 1]), epi.scale[ch + 1], epi.shift[ch + 1]));
+                    if (relu) h = __hmax2(h, __half2(__half(0.f), __half(0.f)));
+                    pk[j] = *reinterpret_cast<const uint32_t*>(&h);
+                }
+                *reinterpret_cast<uint4*>(stage + swizzled(lane, p0 + p)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < CPR; ++i) {
+            const int r = lane / CPR + i * (32 / CPR), p = lane % CPR;
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + swizzled(r, p));
+            const int to = __shfl_sync(0xFFFFFFFFu, row, r);
+            if (pos - lane + r < n) *reinterpret_cast<uint4*>(out + ((size_t)b * max_voxels + to) * COUT + cb + p * 8) = v;
+        }
+        __syncwarp();
     }
 }
 
@@ -640,6 +693,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     uint8_t* sA = smem;
     uint8_t* sB = sA + NSLOT * A_BYTES;
     int32_t* s_idx = reinterpret_cast<int32_t*>(sB + B_STAGES * B_BYTES);
+    uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_idx + NIDX * IDX_WORDS);   // (groups that are staged)
     SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + ring_bytes<CIN, COUT>());
     const bool wide = reinterpret_cast<uintptr_t>(out) % 32 == 0;   // (rows are 32, 64 or 128 bytes)
 
@@ -1003,9 +1057,12 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 const int pos = row0 + t2 * TILE_M + tid;
                 const int row = t2 == 0 ? out_row[0] : (t2 == 1 ? out_row[1] : (t2 == 2 ? out_row[2] : out_row[3]));
                 const uint32_t m_t2 = t2 == 0 ? m[0] : (t2 == 1 ? m[1] : (t2 == 2 ? m[2] : m[3]));
-                if (got)
-                    store_tile<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + set * SET_COLS + t2 * COUT, any && m_t2, epi, relu,
-                                     pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
+                if (!got) continue;
+                const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + set * SET_COLS + t2 * COUT;
+                if constexpr (groups_staged<CIN, COUT>())
+                    store_tile_staged<COUT>(taddr, any && m_t2, epi, relu, s_stage + warp * STAGE_BYTES, lane, pos, row, n, b, max_voxels, out);
+                else
+                    store_tile<COUT>(taddr, any && m_t2, epi, relu, pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
             }
             if (any && got) {
                 tc_fence_before();
