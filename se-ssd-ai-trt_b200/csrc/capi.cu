@@ -675,6 +675,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     c.cin = p->in_channel;
     c.cout = p->out_channel;
     c.dtype = w->impl.dtype;
+    c.subm = p->subm;
     c.status = ws.status;
     c.tile_counter = ws.tile_counter;
     c.debug_withhold_weights = w->impl.debug_withhold;
@@ -965,6 +966,7 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         c.cin = L.p.in_channel;
         c.cout = L.p.out_channel;
         c.dtype = bb->dtype;
+        c.subm = L.p.subm;
         c.status = w.status;
         c.tile_counter = w.tile_counter + i;
         c.maps_ready = i > 0 ? 1 : 0;   // the first layer follows the launch that builds the maps

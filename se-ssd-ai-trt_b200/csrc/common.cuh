@@ -426,7 +426,7 @@ struct ConvLaunch {
     const float* scale;    // [Cout] or null
     const float* shift;    // [Cout] or null
     int relu;
-    int batch, max_voxels, kvol, cin, cout, dtype;
+    int batch, max_voxels, kvol, cin, cout, dtype, subm;
     // Optional fused BEV scatter (last layer): when dense != null the result row is also written to
     // dense[b][c*D + z][y][x] using out_coors.
     void* dense;

@@ -61,13 +61,19 @@ constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
 // Few-tiles path: up to this many tiles per CTA. It fetches a weight block per item instead of one for up to four tiles, but is
 // through sooner, shares the tiles out by a counter and pays nothing for a group's boundary. Layers in us (events around the launch),
-// groups and this path: 64 -> 64 with 11 tiles per CTA (8 x 20,000 points) 63.6 and 59.5, 14 (10 x 20,000) 74.0 and 70.1, 20 (5 x 77,000)
-// 80.0 and 74.1, 33 (8 x 120,000) 150.0 and 144.0, 45 (32 x 20,000)
-// 201 and 191, 131 (32 x 120,000) 575 and 578; 32 -> 64 with 45 117 and 113; 32 -> 32 with 20 (10 x 20,000) 59.6 and 55.5, 32 84.2 and 82.3; with 16 channels, whose items are few, 16 -> 32 with 12
-// (6 x 20,000) 26.9 and 27.0, 16 (8 x 20,000) 31.0 and 35.1, 20 35.1 and 39.1. Lower lines than ten are slower everywhere (front end of 3 x
-// 20,000 points at four, six, eight and ten 338, 326, 319, 319).
-template <int CIN>
-__host__ __device__ constexpr int few_tiles() { return CIN == 16 ? 14 : 50; }
+// groups and this path, by tiles per CTA:
+//   64 -> 64 submanifold  11 (8 x 20,000 points) 72 and 66, 22 121 and 118, 33 (8 x 120,000) 170 and 166, 45 224 and 218, 50 248 and 242,
+//                         66 322 and 320, 131 (32 x 120,000) 633 and 621
+//   64 -> 64 strided      12 (8 x 120,000) 78 and 74, 25 131.5 and 130.6, 31 158 and 159, 37 185 and 187, 43 209 and 216, 49 240 and 246:
+//                         half of an item's rows are missing neighbours (submanifold: a fifth), and groups leave zeros out that are
+//                         still there
+//   32 -> 32              16 (8 x 20,000) 58 and 54, 40 119 and 115, 51 147 and 150, 69 193 and 195
+//   32 -> 64              11 (8 x 20,000) 47.5 and 45.6, 33 109 and 109, 45 136 and 140, 66 203 and 203
+//   16 -> 16              11 (12 x 20,000) 33 and 29, 14 37 and 32 to 33, 16 39 and 35, 19 43.5 and 39.4
+//   16 -> 32              12 (6 x 20,000) 31 and 29, 14 35 and 33, 16 37 and 35, 20 43.5 and 41.4
+// (With 16 channels the line could lie higher.) Lower lines than ten are slower everywhere (front end of 3 x 20,000 points at four, six,
+// eight and ten 338, 326, 319, 319).
+__host__ __device__ constexpr int few_tiles(int cin, bool subm) { return cin == 16 ? 14 : (cin == 64 && !subm ? 30 : 50); }
 constexpr int FEW_SLOTS = 8;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
 // instructions, with the issuer.
@@ -669,7 +675,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                  const int32_t* __restrict__ order, const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
                  const uint8_t* __restrict__ wtiles, const __grid_constant__ EpiConst epi, int relu, int batch,
                  int max_voxels, int kvol, __half* __restrict__ dense, const int4* __restrict__ out_coors, int D, int H,
-                 int W, int32_t* status, int* tile_counter, int maps_ready, int withhold_weights) {
+                 int W, int32_t* status, int* tile_counter, int few_line, int maps_ready, int withhold_weights) {
     // Whatever does not depend on the preceding kernel comes before the wait for it. maps_ready: neighbour map, masks and
     // row counts are older than that kernel.
     if (!maps_ready) pdl_enter();
@@ -798,7 +804,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     }
     // A layer with the BEV scatter takes the few-tiles path whatever its size: it has three offsets, and the scatter's stores, two bytes
     // to a channel and row, are what it does; there eight warps share them. (32 frames of 120,000 points: four warps 190 us, eight 139.)
-    const bool few = tile_counter != nullptr && (dense != nullptr || total_tiles <= few_tiles<CIN>() * (int)gridDim.x);
+    const bool few = tile_counter != nullptr && (dense != nullptr || total_tiles <= few_line * (int)gridDim.x);
     if (few) {
         static_assert(FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX, "whole stages of indices");
         int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));
@@ -1319,7 +1325,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
                        static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                        static_cast<const uint8_t*>(c.umma_weights), epi, c.relu, c.batch, c.max_voxels,
                        c.kvol, static_cast<__half*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W,
-                       c.status, c.tile_counter, c.maps_ready, c.debug_withhold_weights);
+                       c.status, c.tile_counter, few_tiles(CIN, c.subm != 0), c.maps_ready, c.debug_withhold_weights);
     return SESSD_OK;
 }
 

@@ -297,11 +297,12 @@ def test_fp16_tiles_on_both_sides_of_the_few(gpu, oracle, cin, cout, extra):
         assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
 
 
-@pytest.mark.parametrize("cin,cout,line", [(16, 16, 14), (16, 32, 14), (32, 32, 50), (32, 64, 50), (64, 64, 50)])
+@pytest.mark.parametrize("cin,cout,line,subm", [(16, 16, 14, True), (16, 32, 14, True), (32, 32, 50, True), (32, 64, 50, True),
+                                                (64, 64, 50, True), (64, 64, 30, False)])
 @pytest.mark.parametrize("extra", [0, 1])
-def test_fp16_tiles_on_both_sides_of_the_line_between_the_paths(gpu, cin, cout, line, extra):
-    """The most tiles that the few-tiles path takes (14 per SM with 16 input channels, 50 with more), and one more, which goes through
-    groups of four. Frames have the bits of calls on them alone (which are few tiles)."""
+def test_fp16_tiles_on_both_sides_of_the_line_between_the_paths(gpu, cin, cout, line, subm, extra):
+    """The most tiles that the few-tiles path takes (14 per SM with 16 input channels, 50 with more, 30 in strided layers with 64), and
+    one more, which goes through groups of four. Frames have the bits of calls on them alone (which are few tiles)."""
     import torch
 
     rs = np.random.RandomState(cin + cout + extra)
@@ -309,16 +310,29 @@ def test_fp16_tiles_on_both_sides_of_the_line_between_the_paths(gpu, cin, cout, 
     tiles = [total // frames + (1 if b < total % frames else 0) for b in range(frames)]
     rows = [128 * t - 7 * b for b, t in enumerate(tiles)]
     V = max(rows) + 3
-    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (20, 120, 110))
-    coors = torch.from_numpy(_random_coords(rs, V, layer.in_shape)).cuda().expand(frames, V, 4).contiguous()
+    shape = (20, 120, 110)
+    c = _random_coords(rs, V, shape)
+    if subm:
+        layer, call = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape), gpu.subm_conv
+    else:
+        # every cell on its even plane, and of the first frames' ones the cell behind it: as many outputs as cells
+        layer, call = _layer(gpu, False, cin, cout, (2, 1, 1), (2, 1, 1), (0, 0, 0), (40, 120, 110)), gpu.sparse_conv
+        c[:, 1] *= 2
+        behind = c[:rows[-1]] + np.array([0, 1, 0, 0], np.int32)
+        c = np.concatenate([c[:rows[-1]], behind, c[rows[-1]:]])
+        V += len(behind)
+        rows = [n + len(behind) for n in rows]
+    coors = torch.from_numpy(c).cuda().expand(frames, V, 4).contiguous()
     feat = torch.randn((frames, V, cin), device="cuda").half()
     num = torch.tensor(rows, dtype=torch.int32, device="cuda")
     p = gpu.conv_params(layer, V)
-    w = gpu.ConvWeights(p, (rs.randn(27, cin, cout) * 0.05).astype(np.float32), None, None, True, 1)
-    r = gpu.subm_conv(feat, coors, num, p, w)
-    assert r["status"] == 0
+    w = gpu.ConvWeights(p, (rs.randn(layer.kvol, cin, cout) * 0.05).astype(np.float32), None, None, True, 1)
+    r = call(feat, coors, num, p, w)
+    assert r["status"] == 0 and r["features"].any()
+    if not subm:
+        assert int(((r["voxel_num"] + 127) // 128).sum()) == total
     for b in (0, 4, 10):
-        alone = gpu.subm_conv(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
+        alone = call(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
         assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
     w.close()
 
