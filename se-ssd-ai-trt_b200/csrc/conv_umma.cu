@@ -16,7 +16,7 @@
 //   warps 0-3    epilogue (warp w reads tensor-memory lanes 32w .. 32w+31). The accumulators are double
 //                buffered (2 sets x 4 tiles x Cout columns), so the epilogue of one group runs while the
 //                other roles are already working on the next group. A thread holds one row and stores it 32 bytes
-//                at a time; 64 -> 64 channels go through a small staging area of the warp.
+//                at a time; 64 -> 64 channels with many offsets go through a small staging area of the warp.
 //   warps 4-7    MMA issuers; issuer t owns tile t of every group. The warp works out the group's schedule
 //                once (lane g for stage g); it goes through it together, or with 64 input channels one elected lane alone,
 //                and that lane issues the tcgen05.mma and commit instructions (each costs its thread on the order of a
@@ -66,7 +66,7 @@ constexpr int KVOL_MAX = 27;
 //                         66 322 and 320, 131 (32 x 120,000) 633 and 621
 //   64 -> 64 strided      12 (8 x 120,000) 78 and 74, 25 131.5 and 130.6, 31 158 and 159, 37 185 and 187, 43 209 and 216, 49 240 and 246:
 //                         half of an item's rows are missing neighbours (submanifold: a fifth), and groups leave zeros out that are
-//                         still there
+//                         still there; three offsets: 10 (8 x 120,000) 31 and 29, 42 70 and 78
 //   32 -> 32              16 (8 x 20,000) 58 and 54, 40 119 and 115, 51 147 and 150, 69 193 and 195
 //   32 -> 64              11 (8 x 20,000) 47.5 and 45.6, 33 109 and 109, 45 136 and 140, 66 203 and 203
 //   16 -> 16              11 (12 x 20,000) 33 and 29, 14 37 and 32 to 33, 16 39 and 35, 19 43.5 and 39.4
@@ -223,20 +223,17 @@ struct SharedCtl {
 // Epilogue warps of the few-tiles path: with 64 channels a column block each for eight (warps 5-8 have nothing else to do there).
 template <int COUT>
 __host__ __device__ constexpr int few_epi_warps() { return COUT == 64 ? 2 * EPI_WARPS : EPI_WARPS; }
-// Groups: whether output rows go through shared memory (store_tile_staged), and an epilogue warp's room for it.
-template <int CIN, int COUT>
-__host__ __device__ constexpr bool groups_staged() { return CIN == 64 && COUT == 64; }
-constexpr int STAGE_BYTES = 32 * 64;
+constexpr int STAGE_BYTES = 32 * 64;         // room of an epilogue warp of groups that are staged (store_tile_staged)
 // Buffers of the two paths, which share their place.
-template <int CIN, int COUT>
+template <int CIN, int COUT, bool STAGED>
 __host__ __device__ constexpr int ring_bytes() {
     constexpr int groups = Ring<CIN>::NSLOT * A_BYTES + B_STAGES * COUT * ROW_BYTES + Ring<CIN>::NIDX * (64 / CIN) * TAP_WORDS * 4 +
-                           (groups_staged<CIN, COUT>() ? EPI_WARPS * STAGE_BYTES : 0);
+                           (STAGED ? EPI_WARPS * STAGE_BYTES : 0);
     constexpr int few = FEW_SLOTS * (A_BYTES + COUT * ROW_BYTES) + 2 * FEW_IDX * TAP_WORDS * 4;
     return groups > few ? groups : few;
 }
-template <int CIN, int COUT>
-constexpr int umma_smem_bytes() { return 1024 /*alignment slack*/ + ring_bytes<CIN, COUT>() + (int)sizeof(SharedCtl); }
+template <int CIN, int COUT, bool STAGED>
+constexpr int umma_smem_bytes() { return 1024 /*alignment slack*/ + ring_bytes<CIN, COUT, STAGED>() + (int)sizeof(SharedCtl); }
 
 // Offsets g*KG .. g*KG+KG-1 of a tile's 27-bit offset mask.
 template <int KG>
@@ -374,11 +371,13 @@ __device__ __forceinline__ void store_tile(uint32_t taddr, bool have, const EpiC
     }
 }
 
-// The same through the warp's staging area (32 rows of 64 bytes), four lanes to a row, without the scatter: groups of 64 -> 64 channels.
-// Where a tile has twenty items the epilogue has time, and what counts is how often it looks into L1, whose tags the gather warps' copies
-// keep busy: 64 lines of 128 bytes per 32 rows, where stores by row look 128 times. (In us, 64 -> 64 at 1/4 resolution, stores by row and
-// through here: 16 x 120,000 points 326 and 322, 24 477 and 473, 32 639 and 631, 40 798 and 789; 64 x 20,000 432 and 428. The other layers
-// have fewer items to a tile and are faster by row: 32 -> 64, 32 x 120,000, 445 and, by row, 396; 32 -> 32, 16 x 120,000, 380 and 379.)
+// The same through the warp's staging area (32 rows of 64 bytes), four lanes to a row, without the scatter: groups of 64 -> 64 channels
+// with more than 18 offsets. Where a tile has twenty items the epilogue has time, and what counts is how often it looks into L1, whose
+// tags the gather warps' copies keep busy: 64 lines of 128 bytes per 32 rows, where stores by row look 128 times. (In us, stores by row
+// and through here: 27 offsets at 1/4 resolution, 16 x 120,000 points 326 and 322, 24 477 and 473, 32 639 and 631, 40 798 and 789, 64 x
+// 20,000 432 and 428; 18 offsets, 20 x 120,000, 299 and 299; nine 191 and 203, six 154 and 173, three 125 and 150. The other layers have
+// fewer items to a tile: 32 -> 64, 32 x 120,000, 396 and 445; 32 -> 32, 16 x 120,000, 379 and 380.)
+constexpr int STAGED_KVOL = 18;
 template <int COUT>
 __device__ __forceinline__ void store_tile_staged(uint32_t taddr, bool have, const EpiConst& epi, int relu, uint8_t* stage, int lane,
                                                   int pos, int row, int n, int b, int max_voxels, __half* __restrict__ out) {
@@ -669,7 +668,8 @@ __device__ __forceinline__ uint32_t umma_few(SharedCtl* ctl, uint8_t* sA, int32_
     return uses;
 }
 
-template <int CIN, int COUT>
+// STAGED: groups store their rows through shared memory. (A kernel of its own: with the choice made inside, 64 -> 64 groups are 8 % slower.)
+template <int CIN, int COUT, bool STAGED>
 __global__ void __launch_bounds__(Ring<CIN>::THREADS, 1)
 conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const int32_t* __restrict__ nbr,
                  const int32_t* __restrict__ order, const uint32_t* __restrict__ tile_mask, const int32_t* __restrict__ out_num,
@@ -700,7 +700,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     uint8_t* sB = sA + NSLOT * A_BYTES;
     int32_t* s_idx = reinterpret_cast<int32_t*>(sB + B_STAGES * B_BYTES);
     uint8_t* s_stage = reinterpret_cast<uint8_t*>(s_idx + NIDX * IDX_WORDS);   // (groups that are staged)
-    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + ring_bytes<CIN, COUT>());
+    SharedCtl* ctl = reinterpret_cast<SharedCtl*>(smem + ring_bytes<CIN, COUT, STAGED>());
     const bool wide = reinterpret_cast<uintptr_t>(out) % 32 == 0;   // (rows are 32, 64 or 128 bytes)
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1065,7 +1065,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 const uint32_t m_t2 = t2 == 0 ? m[0] : (t2 == 1 ? m[1] : (t2 == 2 ? m[2] : m[3]));
                 if (!got) continue;
                 const uint32_t taddr = tmem + ((uint32_t)(warp * 32) << 16) + set * SET_COLS + t2 * COUT;
-                if constexpr (groups_staged<CIN, COUT>())
+                if constexpr (STAGED)
                     store_tile_staged<COUT>(taddr, any && m_t2, epi, relu, s_stage + warp * STAGE_BYTES, lane, pos, row, n, b, max_voxels, out);
                 else
                     store_tile<COUT>(taddr, any && m_t2, epi, relu, pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
@@ -1302,11 +1302,11 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
     }
 }
 
-template <int CIN, int COUT>
+template <int CIN, int COUT, bool STAGED = false>
 int launch_one(const ConvLaunch& c, cudaStream_t stream) {
     static const std::string name = "conv_umma<f16," + std::to_string(CIN) + "," + std::to_string(COUT) + ">";
-    const int smem = umma_smem_bytes<CIN, COUT>();
-    static_assert(umma_smem_bytes<CIN, COUT>() <= 227 * 1024, "ring does not fit the shared memory of one SM");
+    const int smem = umma_smem_bytes<CIN, COUT, STAGED>();
+    static_assert(umma_smem_bytes<CIN, COUT, STAGED>() <= 227 * 1024, "ring does not fit the shared memory of one SM");
     // the attribute belongs to the device's context: set it once per device (repeating it is harmless, so a
     // race between two host threads only costs a second call)
     static std::atomic<uint64_t> configured{0};
@@ -1314,14 +1314,14 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
     SESSD_CUDA(cudaGetDevice(&dev));
     const uint64_t bit = 1ull << (dev & 63);
     if (!(configured.load(std::memory_order_acquire) & bit)) {
-        SESSD_CUDA(cudaFuncSetAttribute(conv_umma_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        SESSD_CUDA(cudaFuncSetAttribute(conv_umma_kernel<CIN, COUT, STAGED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         configured.fetch_or(bit, std::memory_order_release);
     }
     if (!c.scale_host || !c.shift_host) return SESSD_ERR_PARAM;
     EpiConst epi;
     memcpy(epi.scale, c.scale_host, sizeof epi.scale);
     memcpy(epi.shift, c.shift_host, sizeof epi.shift);
-    SESSD_LAUNCH_NAMED(name.c_str(), (conv_umma_kernel<CIN, COUT>), persistent_grid(1), Ring<CIN>::THREADS, smem, stream,
+    SESSD_LAUNCH_NAMED(name.c_str(), (conv_umma_kernel<CIN, COUT, STAGED>), persistent_grid(1), Ring<CIN>::THREADS, smem, stream,
                        static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                        static_cast<const uint8_t*>(c.umma_weights), epi, c.relu, c.batch, c.max_voxels,
                        c.kvol, static_cast<__half*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W,
@@ -1372,6 +1372,7 @@ int launch_conv_umma(const ConvLaunch& c, cudaStream_t stream) {
     SESSD_CASE(16, 32)
     SESSD_CASE(32, 32)
     SESSD_CASE(32, 64)
+    if (c.cin == 64 && c.cout == 64 && c.kvol > STAGED_KVOL) return launch_one<64, 64, true>(c, stream);
     SESSD_CASE(64, 64)
 #undef SESSD_CASE
     return SESSD_ERR_UNSUPPORTED;

@@ -158,4 +158,4 @@ def test_tensor_core_kernels_spill_no_registers(tmp_path):
                           os.path.join(csrc, "conv_umma.cu")], capture_output=True, text=True, timeout=600)
     assert out.returncode == 0, out.stderr[-2000:]
     spills = re.findall(r"Function properties for \S*conv_umma_kernel\S*\s+(\d+) bytes stack frame, (\d+) bytes spill stores", out.stderr)
-    assert len(spills) == 5 and set(spills) == {("0", "0")}, spills
+    assert len(spills) == 6 and set(spills) == {("0", "0")}, spills
