@@ -676,6 +676,7 @@ static int conv_enqueue_common(const sessd_conv_params* p, const sessd_conv_weig
     c.cout = p->out_channel;
     c.dtype = w->impl.dtype;
     c.subm = p->subm;
+    c.most_rows = (int64_t)batch * maxV;
     c.status = ws.status;
     c.tile_counter = ws.tile_counter;
     c.debug_withhold_weights = w->impl.debug_withhold;
@@ -967,6 +968,8 @@ static int backbone_enqueue_impl(const sessd_backbone* bb, int batch, int max_po
         c.cout = L.p.out_channel;
         c.dtype = bb->dtype;
         c.subm = L.p.subm;
+        // level 0 has a row per point at most, the others more than they have points
+        c.most_rows = (int64_t)batch * (L.level_out == 0 && max_points < maxV ? max_points : maxV);
         c.status = w.status;
         c.tile_counter = w.tile_counter + i;
         c.maps_ready = i > 0 ? 1 : 0;   // the first layer follows the launch that builds the maps

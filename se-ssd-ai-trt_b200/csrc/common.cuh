@@ -427,6 +427,7 @@ struct ConvLaunch {
     const float* shift;    // [Cout] or null
     int relu;
     int batch, max_voxels, kvol, cin, cout, dtype, subm;
+    int64_t most_rows;     // no more rows than this can be in use, all frames together
     // Optional fused BEV scatter (last layer): when dense != null the result row is also written to
     // dense[b][c*D + z][y][x] using out_coors.
     void* dense;

@@ -359,16 +359,27 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
 
 }  // namespace
 
-// Room for 300,000 rows is the line: below it the narrow kernel's rows, a few threads each, are through sooner than a lane with all of
-// a run's offsets. The front end's first layer in us, narrow and here: fp16 1 x 20,000 points (room for 60,000) 11 and 16, 1 x 120,000
-// (200,000) 18.8 and 18.7, 4 x 20,000 (240,000) 18.9 and 18.9, 5 x 20,000 (300,000) 20.9 and 20.6, 6 x 20,000 23.0 and 20.9, 2 x 60,000
-// (400,000) 20.9 and 19.0, 8 x 20,000 27 and 23; fp32 16 -> 16 4 x 20,000 39 and 41, 5 x 20,000 48 and 44. (The line is a capacity
-// because row counts are on the device.) fp32 16 -> 32 is no faster here at any size (4 x 120,000 236 and 246).
+// Where few rows are in use the narrow kernel's rows, a few threads each, are through sooner than a lane with all of a run's offsets;
+// beyond that a run's weights, read once for 64 rows, pay. Row counts are on the device, so the line goes by what the host knows: the
+// room, and in a front end the points, which level 0 has no more rows than.
+//   - Room for 300,000 rows or less: narrow. The front end's first layer in us, narrow and here: fp16 1 x 20,000 points (room for 60,000)
+//     11 and 16, 1 x 120,000 (200,000) 18.8 and 18.7, 4 x 20,000 (240,000) 18.9 and 18.9, 5 x 20,000 (300,000) 20.9 and 20.6.
+//   - Room for 300,000 to 800,000: narrow up to 80,000 points in fp16 and 40,000 in fp32. Front ends in us, narrow and here: fp16 8 x 3,000
+//     points (480,000) 304 and 310, 3 x 22,000 (600,000) 325 and 328, 8 x 9,000 436 and 438, 2 x 40,000 (400,000) 328 and 327, 4 x 22,000
+//     (800,000) 398 and 394, 8 x 20,000 621 and 611; fp32, two layers, 6 x 3,000 (360,000) 1153 and 1161, 8 x 4,000 1869 and 1869, 2 x 22,000
+//     1499 and 1495, 6 x 9,000 2373 and 2377, 2 x 30,000 1825 and 1808, 8 x 8,000 2963 and 2952.
+//   - More room: here (narrow blocks look at every row there is room for). fp16 14 x 3,000 points (840,000) 427 and 427, 32 x 1,000 531
+//     and 526; fp32 14 x 3,000 2556 and 2547.
+// A plugin call's room is all there is: with a third of it in use calls are faster here (4 -> 16 fp16, 8 x 20,000 points 39 and 27, 2 x 30,000
+// 23 and 21; fp32 16 -> 16 84 and 74, 46 and 35), with a tenth slower (fp16 8 x 3,000 15 and 17, 16 -> 16 21 and 29).
+// fp32 16 -> 32 is no faster here at any size (4 x 120,000 236 and 246).
 // A weight that is no finite number must not reach the rows without its neighbour, which multiply it by zero here. Rows are read in
 // pieces of 8 (halves) or 16 bytes and written in pieces of 16.
 bool conv_rows_takes(const ConvLaunch& c) {
-    if ((int64_t)c.batch * c.max_voxels <= kRunRows || !c.weights_finite || !c.tile_mask || c.kvol > ROWS_KVOL_MAX) return false;
+    if (!c.weights_finite || !c.tile_mask || c.kvol > ROWS_KVOL_MAX) return false;
     const bool half = c.dtype == SESSD_F16;
+    const int64_t room = (int64_t)c.batch * c.max_voxels;
+    if (room <= kRunRows || (room < 800000 && c.most_rows < (half ? 80000 : 40000))) return false;
     if (c.cout != 16 || !(c.cin == 4 || (c.cin == 16 && !half))) return false;
     return reinterpret_cast<uintptr_t>(c.in) % (half ? 8 : 16) == 0 && reinterpret_cast<uintptr_t>(c.out) % 16 == 0;
 }

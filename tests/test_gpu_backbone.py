@@ -543,3 +543,35 @@ def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dty
         assert torch.equal(dense, want), i
     assert delay(bb.handle, len(bb.layers), 1) < 0 and delay(None, 0, 1) < 0
     bb.close()
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+@pytest.mark.parametrize("frames,points,rows_kernel", [(8, 3000, False), (6, 10000, None), (14, 3000, True), (4, 21000, True)])
+def test_narrow_layers_of_front_ends_go_by_points(gpu, frames, points, rows_kernel, dtype):
+    """The narrow layers' kernel for many rows needs rows that are in use: a front end's level 0 has no more than points. 24,000
+    points in room for 480,000 rows take the kernel of small calls, 42,000 in room for 840,000 and 84,000 in room for 720,000 the other;
+    60,000 in room for 360,000 the one in fp16 and the other in fp32. Each frame's level-0 rows have the bits of a call on it alone."""
+    import torch
+
+    if points == 21000:
+        points, room = 21000, 180000
+    else:
+        room = 60000
+    w, sc, sh = gpu.random_weights()
+    bb = gpu.Backbone(room, w, sc, sh, dtype=dtype)
+    pts = torch.stack([torch.from_numpy(gpu.synth.lidar_frame(90 + i, n_points=points, n_boxes=9)) for i in range(frames)]).cuda()
+    sizes = torch.tensor([points - 37 * i for i in range(frames)], dtype=torch.int32, device="cuda")
+    dense, ws = bb.run(pts, sizes)
+    assert gpu.read_status(ws) == 0
+    names = [n for n, _ in gpu.profile(lambda: bb.run(pts, sizes, ws, dense)) if n.startswith("conv_")][:1 if dtype else 2]
+    want = (dtype == 0) if rows_kernel is None else rows_kernel
+    assert all(n.startswith("conv_rows" if want else "conv_narrow") for n in names), names
+    level0 = [[t.clone() for t in bb.layer_view(ws, frames, points, layer)] for layer in (0, 1)]
+    for b in (0, frames - 1):
+        _dense1, ws1 = bb.run(pts[b:b + 1], sizes[b:b + 1])
+        for layer in (0, 1):
+            feat, _coors, num = bb.layer_view(ws1, 1, points, layer)
+            n = int(num[0])
+            assert n > 0 and int(level0[layer][2][b]) == n
+            assert torch.equal(level0[layer][0][b, :n], feat[0, :n]), (b, layer)
+    bb.close()
