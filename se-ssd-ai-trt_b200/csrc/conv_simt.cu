@@ -365,12 +365,14 @@ int launch_narrow(const ConvLaunch& c, cudaStream_t stream) {
 template <typename T>
 int dispatch(const ConvLaunch& c, cudaStream_t stream) {
     // Half the channels per thread (a thread is through its row's neighbours sooner, and twice as many blocks share out the rows with
-    // the longest lists) is the faster way for the calls that conv_rows.cu leaves here: front end of 1 x 20,000 points, fp16 254 us
-    // and 258 with all of them, fp32 992 and 1000. fp32 16 -> 32 stays here at every size; with all the channels half as many threads
-    // walk a list, which a submanifold layer (the network has none of these) gains from between 4 and 8 x 20,000 points (4 x 120,000:
+    // the longest lists) is the faster way for small calls: front end of 1 x 20,000 points, fp16 254 us and 258 with all of them, fp32
+    // 992 and 1000. With all the channels half as many threads walk a list, which pays from a million rows on. 4 -> 16 in us, half and
+    // all: 32 x 20,000 points 125 and 113, 16 x 120,000 320 and 282, fp32 111 and 93, 275 and 230 (calls of that size are conv_rows.cu's
+    // where all weights are finite numbers). fp32 16 -> 16 is faster with half at any size (16 x 120,000 779 and 846). fp32 16 -> 32 stays
+    // here at every size: a submanifold layer (the network has none of these) gains from between 4 and 8 x 20,000 points (4 x 120,000:
     // 523 and 460), the network's strided one from a million rows on (8 x 120,000 18097 and 18062, the whole front end).
     const bool few = (int64_t)c.batch * c.max_voxels <= 1000000;
-    if (c.cin == 4 && c.cout == 16) return launch_narrow<T, 4, 16, 4>(c, stream);
+    if (c.cin == 4 && c.cout == 16) return few ? launch_narrow<T, 4, 16, 4>(c, stream) : launch_narrow<T, 4, 16, 8>(c, stream);
     if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these
         if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16, 2>(c, stream);
         if (c.cin == 16 && c.cout == 32) return few ? launch_narrow<float, 16, 32, 2>(c, stream) : launch_narrow<float, 16, 32, 4>(c, stream);

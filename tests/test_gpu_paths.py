@@ -167,14 +167,15 @@ def test_narrow_layers_on_both_sides_of_the_line(gpu, oracle, cin, dtype, ks):
 
 
 @pytest.mark.parametrize("cin,dtype", [(4, 0), (4, 1), (16, 0)])
-def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, cin, dtype):
+@pytest.mark.parametrize("maxV", [300001, 1000000, 1000001])
+def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, maxV, cin, dtype):
     """Weights that are no finite numbers go through the kernel of small calls whatever the room: such a weight reaches the rows with
-    its neighbour alone."""
+    its neighbour alone, and the other channels are the same bits. From a million rows on a thread has twice as many channels of 4 -> 16."""
     import torch
 
     rs = np.random.RandomState(6)
     layer = _layer(gpu, True, cin, 16, (3, 3, 3), (1, 1, 1), (1, 1, 1), (6, 20, 30))
-    rows, maxV, tdt = 700, 300001, torch.float16 if dtype else torch.float32
+    rows, tdt = 700, torch.float16 if dtype else torch.float32
     c = _random_coords(rs, rows, layer.in_shape)
     coors = torch.zeros((1, maxV, 4), dtype=torch.int32, device="cuda")
     coors[0, :rows] = torch.from_numpy(c).cuda()
@@ -196,7 +197,9 @@ def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, cin, d
     hit[pairs[5, 1, :pnum[5]]] = True
     f = bad["features"][0, :rows]
     assert hit.any() and not hit.all()
-    assert (~torch.isfinite(f[:, 3]).cpu().numpy() == hit).all() and torch.isfinite(f[:, torch.arange(16) != 3]).all()
+    others = torch.arange(16) != 3
+    assert (~torch.isfinite(f[:, 3]).cpu().numpy() == hit).all() and torch.isfinite(f[:, others]).all()
+    assert torch.equal(f[:, others], r["features"][0, :rows, others])
     w.close()
     assert names[0].startswith("conv_rows") and names[1].startswith("conv_narrow")
 
@@ -459,7 +462,8 @@ def test_fp16_work_split_over_frames(gpu, oracle, frames, most, cin, cout):
 @pytest.mark.parametrize("cin,cout,dtype", [(4, 16, 0), (4, 16, 1), (16, 16, 0), (16, 32, 0)])
 @pytest.mark.parametrize("max_voxels", [1000000, 1000001])
 def test_narrow_layers_around_a_million_rows(gpu, oracle, max_voxels, cin, cout, dtype):
-    """Room for a million rows is where the narrow kernels change their split; 129 rows: one more than a tile."""
+    """Room for a million rows is where fp32 16 -> 32 changes its split (4 -> 16, too, where another kernel does not take it); 129
+    rows: one more than a tile."""
     rs = np.random.RandomState(dtype)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (6, 9, 66))
     c = _random_coords(rs, 129, layer.in_shape)
