@@ -434,7 +434,7 @@ struct ConvLaunch {
     const int32_t* out_coors;
     int D, H, W;
     int32_t* status;       // device status word (tensor-core path reports wait timeouts there)
-    int* tile_counter;     // tensor-core path: zero before the launch; hands out the tiles of small layers (null: it never does)
+    int* tile_counter;     // tensor-core path: zero before the launch; hands out the tiles of the few-tiles path
     int maps_ready;        // neighbour map, masks and row counts are older than the kernel launched just before
     int debug_withhold_weights;   // tests only: whoever streams the weights stays silent (waits run out)
     int weights_finite;           // every weight is a finite number of the feature dtype

@@ -10,7 +10,8 @@
 // the offset loop outermost, so that a weight block is fetched once per four tiles; (tile, stage) pairs
 // without any neighbour are skipped using the per-tile offset masks the rulebook kernels produce. The
 // epilogue reads the accumulator with tcgen05.ld, applies the folded BatchNorm scale/shift and ReLU, and
-// stores fp16 rows (and, for the last layer, scatters them into the dense BEV map).
+// stores fp16 rows (and, for the last layer, scatters them into the dense BEV map). Layers of few tiles, and those with the scatter,
+// go through a path of their own (umma_few) instead of groups.
 //
 // One persistent CTA per SM; every role has warps of its own and walks the same sequence of groups:
 //   warps 0-3    epilogue (warp w reads tensor-memory lanes 32w .. 32w+31). The accumulators are double
@@ -802,9 +803,12 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
         __syncthreads();
         total_tiles = ctl->range_hi;
     }
-    // A layer with the BEV scatter takes the few-tiles path whatever its size: it has three offsets, and the scatter's stores, two bytes
-    // to a channel and row, are what it does; there eight warps share them. (32 frames of 120,000 points: four warps 190 us, eight 139.)
-    const bool few = tile_counter != nullptr && (dense != nullptr || total_tiles <= few_line * (int)gridDim.x);
+    // A layer with the BEV scatter takes the few-tiles path whatever its size. The scatter's stores, two bytes to a channel and row, are
+    // most of what it does, and a group's four tiles leave together, which the other roles wait for. (In us, groups and here, with up
+    // to 181 tiles per SM: 64 -> 64 of three offsets, 96 x 120,000 points, 535 and 390, of 27 1614 and 1029; 32 -> 32 of 27 756 and 560;
+    // 16 -> 16 of three 340 and 306, of 27 2835 and 852; 16 -> 32 of 27 414 and 351; at 14 to 18 tiles per SM 80 and 64, 245 and 154, 105
+    // and 84, 48 and 41, 76 and 66, 117 and 86.)
+    const bool few = dense != nullptr || total_tiles <= few_line * (int)gridDim.x;
     if (few) {
         static_assert(FEW_IDX % KG == 0 && FEW_IDX >= KVOL_MAX, "whole stages of indices");
         int32_t* few_idx = reinterpret_cast<int32_t*>(sA + FEW_SLOTS * (A_BYTES + B_BYTES));
@@ -1068,7 +1072,7 @@ conv_umma_kernel(const __half* __restrict__ in, __half* __restrict__ out, const 
                 if constexpr (STAGED)
                     store_tile_staged<COUT>(taddr, any && m_t2, epi, relu, s_stage + warp * STAGE_BYTES, lane, pos, row, n, b, max_voxels, out);
                 else
-                    store_tile<COUT>(taddr, any && m_t2, epi, relu, pos, row, n, b, max_voxels, out, wide, dense, out_coors, D, H, W);
+                    store_tile<COUT>(taddr, any && m_t2, epi, relu, pos, row, n, b, max_voxels, out, wide, nullptr, nullptr, 0, 0, 0);
             }
             if (any && got) {
                 tc_fence_before();
@@ -1365,14 +1369,16 @@ int conv_umma_pack_weights(const float* weights, int kvol, int cin, int cout, vo
 }
 
 int launch_conv_umma(const ConvLaunch& c, cudaStream_t stream) {
-    if (c.dtype != SESSD_F16 || !c.umma_weights || !c.tile_mask || c.kvol > KVOL_MAX) return SESSD_ERR_UNSUPPORTED;
+    if (c.dtype != SESSD_F16 || !c.umma_weights || !c.tile_mask || !c.tile_counter || c.kvol > KVOL_MAX) return SESSD_ERR_UNSUPPORTED;
 #define SESSD_CASE(CI, CO) \
     if (c.cin == CI && c.cout == CO) return launch_one<CI, CO>(c, stream);
     SESSD_CASE(16, 16)
     SESSD_CASE(16, 32)
     SESSD_CASE(32, 32)
     SESSD_CASE(32, 64)
-    if (c.cin == 64 && c.cout == 64 && c.kvol > STAGED_KVOL) return launch_one<64, 64, true>(c, stream);
+    // (a layer with the scatter has no groups: it takes the kernel whose code the layers before it have fetched, front end of 1 x 20,000
+    // points 190.2 and 188.8 us)
+    if (c.cin == 64 && c.cout == 64 && (c.kvol > STAGED_KVOL || c.dense)) return launch_one<64, 64, true>(c, stream);
     SESSD_CASE(64, 64)
 #undef SESSD_CASE
     return SESSD_ERR_UNSUPPORTED;
