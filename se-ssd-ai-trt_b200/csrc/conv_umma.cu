@@ -62,19 +62,22 @@ constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
 // Few-tiles path: up to this many tiles per CTA. It fetches a weight block per item instead of one for up to four tiles, but is
 // through sooner, shares the tiles out by a counter and pays nothing for a group's boundary. Layers in us (events around the launch),
-// groups and this path, by tiles per CTA:
-//   64 -> 64 submanifold  11 (8 x 20,000 points) 72 and 66, 22 121 and 118, 33 (8 x 120,000) 170 and 166, 45 224 and 218, 50 248 and 242,
-//                         66 322 and 320, 131 (32 x 120,000) 633 and 621
-//   64 -> 64 strided      12 (8 x 120,000) 78 and 74, 25 131.5 and 130.6, 31 158 and 159, 37 185 and 187, 43 209 and 216, 49 240 and 246:
-//                         half of an item's rows are missing neighbours (submanifold: a fifth), and groups leave zeros out that are
-//                         still there; three offsets: 10 (8 x 120,000) 31 and 29, 42 70 and 78
-//   32 -> 32              16 (8 x 20,000) 58 and 54, 40 119 and 115, 51 147 and 150, 69 193 and 195
-//   32 -> 64              11 (8 x 20,000) 47.5 and 45.6, 33 109 and 109, 45 136 and 140, 66 203 and 203
-//   16 -> 16              11 (12 x 20,000) 33 and 29, 14 37 and 32 to 33, 16 39 and 35, 19 43.5 and 39.4
-//   16 -> 32              12 (6 x 20,000) 31 and 29, 14 35 and 33, 16 37 and 35, 20 43.5 and 41.4
-// (With 16 channels the line could lie higher.) Lower lines than ten are slower everywhere (front end of 3 x 20,000 points at four, six,
-// eight and ten 338, 326, 319, 319).
-__host__ __device__ constexpr int few_tiles(int cin, bool subm) { return cin == 16 ? 14 : (cin == 64 && !subm ? 30 : 50); }
+// groups and this path, by tiles per CTA; the line lies where they cross:
+//   64 -> 64 submanifold  11 (8 x 20,000 points) 74 and 66, 22 125 and 119, 33 (8 x 120,000) 170 and 166, 45 224 and 220, 50 248 and 242 or,
+//                         at 1/8, 245 and 246, 66 322 and 318, 132 (32 x 120,000) 633 and 621
+//   64 -> 64 strided      12 (8 x 120,000) 77 and 74, 18 105 and 103, 25 131.5 and 131.5, 31 158 and 160, 37 185 and 189, 49 238 and 246 (half
+//                         of an item's rows are missing neighbours, submanifold a fifth, and groups leave zeros out that are still
+//                         there); three offsets: 10 29 and 29, 21 41.5 and 45.5, 42 66 and 78
+//   32 -> 32              10 (5 x 20,000) 41.5 and 37.4, 24 76 and 74, 40 119 and 115, 50 142 and 140 to 142, 64 177 and 177; frames of 120,000:
+//                         17 60 and 58, 26 80 and 82, 34 103 and 104, 43 125 and 127.5, 51 146 and 149.5
+//   32 -> 64              8 (6 x 20,000) 39.4 and 37.4, 17 62 and 61, 22 76 and 76, 25 84.5 and 84.5, 31 99 and 101, 41 129.5 and 133.5, 50 154 and 156
+//   16 -> 16              11 (12 x 20,000) 33 and 29, 18.5 43.5 and 39.4, 22 (5 x 120,000) 45.5 and 45.5, 24 50 and 48, 31 (7 x 120,000) 58 and 60,
+//                         37 70 and 70, 46 84.5 and 86.5, 70 117 and 119
+//   16 -> 32              12 (6 x 20,000) 31 and 29, 17 39.4 and 37.3, 20 43.5 and 41.4, 24 to 43 the same, 50 89 and 87, 64 107 and 109
+// Lower lines than ten are slower everywhere (front end of 3 x 20,000 points at four, six, eight and ten 338, 326, 319, 319).
+__host__ __device__ constexpr int few_tiles(int cin, int cout, bool subm) {
+    return cin == 16 ? 22 : (cin == 32 ? (cout == 32 ? 42 : 25) : (subm ? 50 : 20));
+}
 constexpr int FEW_SLOTS = 8;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
 // instructions, with the issuer.
@@ -1329,7 +1332,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
                        static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                        static_cast<const uint8_t*>(c.umma_weights), epi, c.relu, c.batch, c.max_voxels,
                        c.kvol, static_cast<__half*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W,
-                       c.status, c.tile_counter, few_tiles(CIN, c.subm != 0), c.maps_ready, c.debug_withhold_weights);
+                       c.status, c.tile_counter, few_tiles(CIN, COUT, c.subm != 0), c.maps_ready, c.debug_withhold_weights);
     return SESSD_OK;
 }
 
