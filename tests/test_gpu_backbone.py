@@ -6,6 +6,7 @@ import pytest
 
 import make_golden_inputs as mk
 from conftest import match_rows, rel_err
+from test_gpu_conv import FEW_TILES, _tiles_per_sm
 
 pytestmark = pytest.mark.gpu
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
@@ -518,12 +519,12 @@ def test_empty_and_out_of_range_frames_inside_a_batch(gpu):
     bb.close()
 
 
-@pytest.mark.parametrize("dtype", [0, 1])
-@pytest.mark.parametrize("frames", [1, 8])
+@pytest.mark.parametrize("dtype,frames", [(0, 1), (0, 8), (1, 1), (1, 40)])
 def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dtype):
     """Layers start while the kernel before them runs. One that takes twice the limit of their bounded waits (about 0.2 s) is put
     before one layer after the other: no wait runs out, and the outputs are those of a call without it. In fp16 one frame goes
-    through the few-tiles path, and eight through groups of tiles in the layers at 1/2 and 1/4 resolution."""
+    through the few-tiles path, and the layers of 40 down to 1/4 resolution through groups of tiles. In fp32 eight frames' second layer is
+    the narrow layers' kernel for many rows."""
     import torch
 
     w, sc, sh = gpu.random_weights()
@@ -535,7 +536,16 @@ def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dty
     want = dense.clone()
     delay = gpu.lib().sessd_backbone_debug_delay
     wide = [i for i, l in enumerate(bb.layers) if i > 0 and l.cin >= (32 if dtype == 0 else 16)]
-    for i in (wide[0], wide[2], wide[4], wide[-1]):
+    delayed = (wide[0], wide[2], wide[4], wide[-1]) if dtype == 0 else (1, 2, 3, 5, 6, 9, 13)
+    if frames == 40:
+        for i in (1, 2, 3, 5, 6, 9):
+            l = bb.layers[i]
+            line = FEW_TILES[l.cin, l.cout] if l.subm or l.cin < 64 else 20
+            assert _tiles_per_sm(bb.layer_view(ws, frames, pts.shape[1], i)[2].tolist()) > line, i
+    if (dtype, frames) == (0, 8):
+        delayed += (1,)
+        assert [n for n, _ in gpu.profile(lambda: bb.run(pts, sizes, ws, dense)) if n.startswith("conv_")][1].startswith("conv_rows")
+    for i in delayed:
         assert delay(bb.handle, i, 1) == 0
         bb.run(pts, sizes, ws, dense)
         assert delay(bb.handle, i, 0) == 0
@@ -546,11 +556,12 @@ def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dty
 
 
 @pytest.mark.parametrize("dtype", [0, 1])
-@pytest.mark.parametrize("frames,points,rows_kernel", [(8, 3000, False), (6, 10000, None), (14, 3000, True), (4, 21000, True)])
+@pytest.mark.parametrize("frames,points,rows_kernel", [(8, 3000, False), (6, 10000, None), (15, 3000, True), (4, 21000, True)])
 def test_narrow_layers_of_front_ends_go_by_points(gpu, frames, points, rows_kernel, dtype):
     """The narrow layers' kernel for many rows needs rows that are in use: a front end's level 0 has no more than points. 24,000
-    points in room for 480,000 rows take the kernel of small calls, 42,000 in room for 840,000 and 84,000 in room for 720,000 the other;
-    60,000 in room for 360,000 the one in fp16 and the other in fp32. Each frame's level-0 rows have the bits of a call on it alone."""
+    points in room for 480,000 rows take the kernel of small calls, 45,000 in room for 900,000 and 84,000 in room for 720,000 the other;
+    60,000 in room for 360,000 the one in fp16 and the other in fp32. Each frame's level-0 rows have the bits of a call on it alone,
+    also behind empty and nearly empty frames."""
     import torch
 
     if points == 21000:
@@ -561,17 +572,19 @@ def test_narrow_layers_of_front_ends_go_by_points(gpu, frames, points, rows_kern
     bb = gpu.Backbone(room, w, sc, sh, dtype=dtype)
     pts = torch.stack([torch.from_numpy(gpu.synth.lidar_frame(90 + i, n_points=points, n_boxes=9)) for i in range(frames)]).cuda()
     sizes = torch.tensor([points - 37 * i for i in range(frames)], dtype=torch.int32, device="cuda")
+    if frames == 15:
+        sizes[0], sizes[3], sizes[4] = 0, 1, 70
     dense, ws = bb.run(pts, sizes)
     assert gpu.read_status(ws) == 0
     names = [n for n, _ in gpu.profile(lambda: bb.run(pts, sizes, ws, dense)) if n.startswith("conv_")][:1 if dtype else 2]
     want = (dtype == 0) if rows_kernel is None else rows_kernel
     assert all(n.startswith("conv_rows" if want else "conv_narrow") for n in names), names
     level0 = [[t.clone() for t in bb.layer_view(ws, frames, points, layer)] for layer in (0, 1)]
-    for b in (0, frames - 1):
+    for b in range(frames) if frames == 15 else (0, frames - 1):
         _dense1, ws1 = bb.run(pts[b:b + 1], sizes[b:b + 1])
         for layer in (0, 1):
             feat, _coors, num = bb.layer_view(ws1, 1, points, layer)
             n = int(num[0])
-            assert n > 0 and int(level0[layer][2][b]) == n
+            assert (n > 0) == (int(sizes[b]) > 0) and int(level0[layer][2][b]) == n
             assert torch.equal(level0[layer][0][b, :n], feat[0, :n]), (b, layer)
     bb.close()

@@ -14,6 +14,17 @@ FP32_TOL = 1e-5
 FP16_TOL = 1e-2
 
 
+# The most tiles per SM that an fp16 layer of these channels takes through the tensor-core kernel's few-tiles path (strided
+# 64 -> 64: 20); beyond that it works in groups of four tiles.
+FEW_TILES = {(16, 16): 22, (16, 32): 22, (32, 32): 42, (32, 64): 25, (64, 64): 50}
+
+
+def _tiles_per_sm(rows):
+    import torch
+
+    return sum((int(n) + 127) // 128 for n in rows) / torch.cuda.get_device_properties(0).multi_processor_count
+
+
 def _layer(pkg, subm, cin, cout, K, S, P, in_shape):
     out_shape = in_shape if subm else tuple((in_shape[j] + 2 * P[j] - K[j]) // S[j] + 1 for j in range(3))
     return pkg.schedule.ConvLayer("t", subm, cin, cout, tuple(K), tuple(S), tuple(P), tuple(in_shape), out_shape)
@@ -250,20 +261,71 @@ def test_bad_coordinate_is_reported_not_dereferenced(gpu):
 
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 64), (64, 64)])
 def test_more_row_groups_than_resident_blocks_fp16(gpu, oracle, cin, cout):
-    """5 frames of 30,001 to 50,000 rows: more than ten tiles per SM, so that the kernel works in groups of four tiles; blocks walk
-    through several groups and their staging rings wrap many times."""
+    """5 frames, one of 30,001 rows and four of the same many: more tiles than the few-tiles path takes, so that the kernel works in
+    groups of four tiles; blocks walk through several groups and their staging rings wrap many times. The small frame has the oracle's
+    values and the others the bits of a call on one of them alone, which is few tiles."""
     import torch
 
     rs = np.random.RandomState(77 + cin)
-    shape = (10, 200, 176)
-    frames = []
-    for n in (50000, 44000, 45000, 30001, 45000):
-        c = _random_coords(rs, n, shape)
-        frames.append((c, rs.randn(len(c), cin).astype(np.float32)))
-    assert sum((len(c) + 127) // 128 for c, _ in frames) > 10 * torch.cuda.get_device_properties(0).multi_processor_count
+    shape = (20, 250, 250)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    many = 128 * (FEW_TILES[cin, cout] * sms // 4 + 1) - 50
+    assert _tiles_per_sm([many] * 4 + [30001]) > FEW_TILES[cin, cout] > _tiles_per_sm([many])
+    rows, maxV = [many, many, many, 30001, many], many + 3
+    c, x = _random_coords(rs, many, shape), torch.randn((many, cin), device="cuda").half()
+    small, xs = _random_coords(rs, 30001, shape), rs.randn(30001, cin).astype(np.float16)
+    coors = torch.zeros((5, maxV, 4), dtype=torch.int32, device="cuda")
+    feat = torch.zeros((5, maxV, cin), dtype=torch.float16, device="cuda")
+    for b, n in enumerate(rows):
+        coors[b, :n] = torch.from_numpy(c if n == many else small).cuda()
+        feat[b, :n] = x if n == many else torch.from_numpy(xs).cuda()
+        coors[b, :n, 0] = b
     W = (rs.randn(27, cin, cout) / np.sqrt(5 * cin)).astype(np.float32)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
-    _check_layer(gpu, oracle, layer, frames, W, dtype=gpu.F16, maxV=50048)
+    p = gpu.conv_params(layer, maxV)
+    w = gpu.ConvWeights(p, W, None, None, False, gpu.F16)
+    num = torch.tensor(rows, dtype=torch.int32, device="cuda")
+    r = gpu.subm_conv(feat, coors, num, p, w)
+    assert r["status"] == 0
+    alone = gpu.subm_conv(feat[:1], coors[:1], num[:1], p, w)
+    assert alone["status"] == 0 and alone["features"].any()
+    for b in (0, 1, 2, 4):
+        assert torch.equal(r["features"][b], alone["features"][0]), b
+    pairs, pnum, st = oracle.subm_rulebook(small, 30001, shape, 30001)
+    want = oracle.conv_apply(xs.astype(np.float32), pairs, pnum, W, 30001, half_inputs=True)
+    got = r["features"][3].float().cpu().numpy()
+    assert st == 0 and rel_err(got[:30001], want) <= FP16_TOL and not got[30001:].any()
+    w.close()
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 32), (32, 32), (32, 64), (64, 64)])
+def test_one_fp16_frame_through_groups(gpu, cin, cout):
+    """A single frame of more tiles than the few-tiles path takes: five slabs of rows without neighbours among each other, each of
+    which has the bits of a call on it alone, through the few-tiles path."""
+    import torch
+
+    rs = np.random.RandomState(cin + cout)
+    n = 128 * (FEW_TILES[cin, cout] * torch.cuda.get_device_properties(0).multi_processor_count // 5 + 1)
+    assert _tiles_per_sm([5 * n]) > FEW_TILES[cin, cout] > _tiles_per_sm([n])
+    slab = _random_coords(rs, n, (8, 200, 200))
+    c = np.concatenate([slab + np.array([0, 10 * i, 0, 0], np.int32) for i in range(5)])
+    coors = torch.from_numpy(c)[None].cuda()
+    x = torch.randn((1, 5 * n, cin), device="cuda").half()
+    W = (rs.randn(27, cin, cout) / np.sqrt(5 * cin)).astype(np.float32)
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (50, 200, 200))
+
+    def call(coors, x):
+        p = gpu.conv_params(layer, x.shape[1])
+        w = gpu.ConvWeights(p, W, None, None, True, gpu.F16)
+        r = gpu.subm_conv(x, coors, torch.tensor([x.shape[1]], dtype=torch.int32, device="cuda"), p, w)
+        w.close()
+        assert r["status"] == 0
+        return r["features"][0]
+
+    got = call(coors, x)
+    for i in range(5):
+        alone = call(coors[:, i * n:(i + 1) * n].contiguous(), x[:, i * n:(i + 1) * n].contiguous())
+        assert torch.equal(got[i * n:(i + 1) * n], alone) and alone.any(), i
 
 
 @pytest.mark.parametrize("dtype,cin,cout,n", [(1, 32, 32, 3000), (1, 32, 32, 195000), (1, 64, 64, 195000), (0, 32, 32, 3000), (0, 64, 64, 60000)])
@@ -271,8 +333,8 @@ def test_bounded_waits_run_out_report_and_leave_the_context_usable(gpu, dtype, c
     """Time-out path of the kernels that stream their weights, made on the host: with the library's test hook on, nobody asks
     for weights, the bounded waits for the first block run out, every block leaves through its abort path and the call
     reports SESSD_STATUS_TIMEOUT with the code of that wait. Nothing faults; the same call with the hook off then gives the
-    result it gave before. fp16: the few-tiles path, and groups (more than ten tiles per SM) with either kind of issuer; fp32: one
-    round of rows, and three."""
+    result it gave before. fp16: the few-tiles path with fewer tiles than SMs and with ten per SM (groups have a test of their own);
+    fp32: one round of rows, and three."""
     import torch
 
     rs = np.random.RandomState(5)

@@ -7,7 +7,7 @@ import pytest
 
 import make_golden_inputs as mk
 from test_gpu_backbone import _check_fp32_layers, _gpu_run, _oracle_layers
-from test_gpu_conv import _check_layer, _layer, _random_coords
+from test_gpu_conv import FEW_TILES, _check_layer, _layer, _random_coords, _tiles_per_sm
 from test_gpu_postprocess import _check_filter
 from test_gpu_voxelize import _compare
 
@@ -273,9 +273,9 @@ def test_strided_maps_through_a_table_and_by_input_rows(gpu, fp16):
 
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 32), (32, 64), (64, 64)])
 @pytest.mark.parametrize("extra", [0, 1])
-def test_fp16_tiles_on_both_sides_of_the_few(gpu, oracle, cin, cout, extra):
-    """Ten tiles per SM are the most that the few-tiles path takes, one more goes through groups of four. Every frame has the bits of
-    a call on it alone (211 or 212 tiles, through the few-tiles path), and the first of those has the oracle's values."""
+def test_fp16_ten_tiles_per_sm(gpu, oracle, cin, cout, extra):
+    """Ten tiles per SM, and one more, handed out one at a time. Every frame has the bits of a call on it alone (211 or 212 tiles), and
+    the first of those has the oracle's values."""
     import torch
 
     rs = np.random.RandomState(cin + cout)
@@ -298,10 +298,6 @@ def test_fp16_tiles_on_both_sides_of_the_few(gpu, oracle, cin, cout, extra):
     for b in range(frames):
         alone = gpu.subm_conv(feat[b:b + 1], coors[b:b + 1], num[b:b + 1], p, w)
         assert alone["status"] == 0 and torch.equal(r["features"][b], alone["features"][0]), b
-
-
-# The most tiles per SM that a layer of these channels takes through the few-tiles path (strided 64 -> 64: 20).
-FEW_TILES = {(16, 16): 22, (16, 32): 22, (32, 32): 42, (32, 64): 25, (64, 64): 50}
 
 
 @pytest.mark.parametrize("cin,cout,line,subm", [(*c, n, True) for c, n in FEW_TILES.items()] + [(64, 64, 20, False)])
@@ -424,22 +420,24 @@ def test_few_fp16_tiles_some_without_neighbours(gpu):
     args[-1].close(), bw.close()
 
 
-@pytest.mark.parametrize("cin,cout", [(16, 32), (64, 64)])
-@pytest.mark.parametrize("frames,most", [(8, 56301), (9, 56301), (40, 9301), (130, 6301)])
-def test_fp16_work_split_over_frames(gpu, oracle, frames, most, cin, cout):
-    """More than ten tiles per SM in up to eight frames, and in more (the work is then cut with the frames' first tiles in shared
-    memory): three to seven tiles per thread of the cut, with empty frames at the ends and in between. Every frame has the
-    bits of a call on it alone, and the first has the oracle's values."""
+@pytest.mark.parametrize("cin,cout", [(16, 32), (32, 32), (64, 64)])
+@pytest.mark.parametrize("frames", [8, 9, 40, 130])
+def test_fp16_work_split_over_frames(gpu, oracle, frames, cin, cout):
+    """More tiles than the few-tiles path takes in up to eight frames, and in more (the work is then cut with the frames' first tiles in
+    shared memory): five to twelve tiles per thread of the cut, with empty frames at the ends and in between. Every frame has the
+    bits of a call on it alone, through the few-tiles path, and a frame of rows of the first has the oracle's values."""
     import torch
 
     rs = np.random.RandomState(frames + cin)
-    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70))
-    W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
+    use = [None if f in (0, 3, frames - 1) else f % 6 for f in range(frames)]
+    large = sum(i in (0, 2, 4, 5) for i in use)
+    most = 128 * (FEW_TILES[cin, cout] * torch.cuda.get_device_properties(0).multi_processor_count // large + 5) + 45
     rows, maxV = [most - 301, 1, most - 301, 128, most - 501, most], most
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70) if most < 60000 else (12, 200, 180))
+    W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
     coors = [_random_coords(rs, n, layer.in_shape) for n in rows]
     feats = [rs.randn(n, cin).astype(np.float32) for n in rows]
-    _check_layer(gpu, oracle, layer, [(coors[0], feats[0])], W, dtype=1, maxV=maxV)
-    use = [None if f in (0, 3, frames - 1) else f % len(rows) for f in range(frames)]
+    _check_layer(gpu, oracle, layer, [(coors[0][:20000], feats[0][:20000])], W, dtype=1, maxV=maxV)
     p = gpu.conv_params(layer, maxV)
     w = gpu.ConvWeights(p, W, None, None, False, 1)
 
@@ -452,10 +450,10 @@ def test_fp16_work_split_over_frames(gpu, oracle, frames, most, cin, cout):
                 c[b, :rows[i], 0] = b
         r = gpu.subm_conv(torch.from_numpy(x).cuda(), torch.from_numpy(c).cuda(), torch.tensor(n, dtype=torch.int32).cuda(), p, w)
         assert r["status"] == 0
-        return r["features"], sum((v + 127) // 128 for v in n)
+        return r["features"], _tiles_per_sm(n)
 
     got, tiles = call(use)
-    assert tiles > 10 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert tiles > FEW_TILES[cin, cout] > _tiles_per_sm([most])
     alone = [call([i])[0][0] for i in range(len(rows))]
     for b, i in enumerate(use):
         assert not got[b].any() if i is None else torch.equal(got[b], alone[i]), b
@@ -857,3 +855,24 @@ def test_heads_and_filter_on_two_frames_in_turn(gpu):
     for i in (0, 1, 0, 1):
         assert all(torch.equal(a, b) for a, b in zip(replay(i), want[i])), i
     bb.close()
+
+
+@pytest.mark.parametrize("dtype", [0, 1])
+def test_narrow_strided_layer_whose_map_names_no_runs(gpu, oracle, dtype):
+    """4 -> 16 channels, strided, on a fine grid with room for more than 500,000 rows: the map is written by input rows, which name no
+    offsets for 32 rows at a time, and the contraction is the kernel for many rows."""
+    import torch
+
+    rs = np.random.RandomState(17)
+    layer = _layer(gpu, False, 4, 16, (3, 3, 3), (2, 2, 2), (1, 1, 1), (41, 1000, 1000))
+    c = _random_coords(rs, 9000, (10, 60, 60))
+    f = rs.randn(len(c), 4).astype(np.float32)
+    W = (rs.randn(27, 4, 16) * 0.2).astype(np.float32)
+    _check_layer(gpu, oracle, layer, [(c, f)], W, dtype=dtype, maxV=500001)
+    p = gpu.conv_params(layer, 500001)
+    w = gpu.ConvWeights(p, W, None, None, False, dtype)
+    x = torch.zeros((1, 500001, 4), dtype=torch.float16 if dtype else torch.float32, device="cuda")
+    coors = torch.zeros((1, 500001, 4), dtype=torch.int32, device="cuda")
+    names = [n for n, _ in gpu.profile(lambda: gpu.sparse_conv(x, coors, torch.tensor([1], dtype=torch.int32, device="cuda"), p, w))]
+    assert any("scatter_rows" in n for n in names) and names[-1].startswith("conv_rows"), names
+    w.close()
