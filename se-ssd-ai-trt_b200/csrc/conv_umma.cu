@@ -61,22 +61,28 @@ constexpr int ROW_BYTES = 128;               // 64 halves per A/B row
 constexpr int A_BYTES = TILE_M * ROW_BYTES;  // 16 KB
 constexpr int KVOL_MAX = 27;
 // Few-tiles path: up to this many tiles per CTA. It fetches a weight block per item instead of one for up to four tiles, but is
-// through sooner, shares the tiles out by a counter and pays nothing for a group's boundary. Layers in us (events around the launch),
-// groups and this path, by tiles per CTA; the line lies where they cross:
-//   64 -> 64 submanifold  11 (8 x 20,000 points) 74 and 66, 22 125 and 119, 33 (8 x 120,000) 170 and 166, 45 224 and 220, 50 248 and 242 or,
-//                         at 1/8, 245 and 246, 66 322 and 318, 132 (32 x 120,000) 633 and 621
-//   64 -> 64 strided      12 (8 x 120,000) 77 and 74, 18 105 and 103, 25 131.5 and 131.5, 31 158 and 160, 37 185 and 189, 49 238 and 246 (half
-//                         of an item's rows are missing neighbours, submanifold a fifth, and groups leave zeros out that are still
-//                         there); three offsets: 10 29 and 29, 21 41.5 and 45.5, 42 66 and 78
-//   32 -> 32              10 (5 x 20,000) 41.5 and 37.4, 24 76 and 74, 40 119 and 115, 50 142 and 140 to 142, 64 177 and 177; frames of 120,000:
-//                         17 60 and 58, 26 80 and 82, 34 103 and 104, 43 125 and 127.5, 51 146 and 149.5
-//   32 -> 64              8 (6 x 20,000) 39.4 and 37.4, 17 62 and 61, 22 76 and 76, 25 84.5 and 84.5, 31 99 and 101, 41 129.5 and 133.5, 50 154 and 156
-//   16 -> 16              11 (12 x 20,000) 33 and 29, 18.5 43.5 and 39.4, 22 (5 x 120,000) 45.5 and 45.5, 24 50 and 48, 31 (7 x 120,000) 58 and 60,
-//                         37 70 and 70, 46 84.5 and 86.5, 70 117 and 119
-//   16 -> 32              12 (6 x 20,000) 31 and 29, 17 39.4 and 37.3, 20 43.5 and 41.4, 24 to 43 the same, 50 89 and 87, 64 107 and 109
-// Lower lines than ten are slower everywhere (front end of 3 x 20,000 points at four, six, eight and ten 338, 326, 319, 319).
-__host__ __device__ constexpr int few_tiles(int cin, int cout, bool subm) {
-    return cin == 16 ? 22 : (cin == 32 ? (cout == 32 ? 42 : 25) : (subm ? 50 : 20));
+// through sooner, shares the tiles out by a counter and pays nothing for a group's boundary. The line lies where they cross, which
+// depends on whether the rows of the map are ordered by their neighbours (a front end's) or not (a plugin call's: more items, and more of
+// their rows missing neighbours, whose zeros groups leave out where they are still there). Layers in us (events around the launch),
+// groups and this path, by tiles per CTA. Front ends:
+//   16 -> 16  13 (3 x 120,000 points) 29 and 27, 17 33 and 33, 18 (20 x 20,000) 33 and 35, 26 43.5 and 45.5, 35 52 and 58
+//   16 -> 32  8 23 and 23, 10 (5 x 20,000) 25 and 25, 12 27 and 29, 17 (2 x 120,000) 33 and 36, 26 41.5 and 48, 50 68 and 84
+//   32 -> 32  20 (10 x 20,000) 60 and 57, 40 105 and 101, 64 158 and 152, 129 306 and 296, 193 453 and 458, 257 600 and 637; frames of 120,000:
+//             17 56 and 54, 34 93 and 97, 51 136 and 138, 69 179 and 179, 103 265 and 261, 137 353 and 342
+//   32 -> 64  14 (10 x 20,000) 48 and 45.5, 28 80 and 76, 45 115 and 112, 67 161 and 165, 90 210 and 218; frames of 120,000: 25 74 and 72, 58 152
+//             and 148, 132 332 and 318
+//   64 -> 64  11 (8 x 20,000) 66 and 58, 33 (8 x 120,000) 152 and 144, 67 293 and 277, 132 (32 x 120,000) 567 and 532, 197 842 and 791; strided 12 58 and
+//             54, 25 99 and 92, 49 180 and 170, 77 269 and 257
+// Plugin calls:
+//   16 -> 16  11 (12 x 20,000) 33 and 29, 18.5 43.5 and 39.4, 22 45.5 and 45.5, 31 58 and 60, 46 84.5 and 86.5
+//   16 -> 32  12 (6 x 20,000) 31 and 29, 20 43.5 and 41.4, 24 to 43 the same, 64 107 and 109
+//   32 -> 32  10 (5 x 20,000) 41.5 and 37.4, 24 76 and 74, 40 119 and 115, 64 177 and 177; frames of 120,000: 17 60 and 58, 34 103 and 104, 51 146 and 149.5
+//   32 -> 64  8 (6 x 20,000) 39.4 and 37.4, 17 62 and 61, 25 84.5 and 84.5, 41 129.5 and 133.5
+//   64 -> 64  11 (8 x 20,000) 74 and 66, 33 (8 x 120,000) 170 and 166, 66 322 and 318, 83 400 and 396, 132 633 and 621; strided 12 77 and 74, 25 131.5
+//             and 131.5, 37 185 and 189, 49 238 and 246; strided, three offsets, 10 29 and 29, 21 41.5 and 45.5, 42 66 and 78
+__host__ __device__ constexpr int few_tiles(int cin, int cout, bool subm, bool ordered) {
+    if (ordered) return cin == 16 ? (cout == 16 ? 17 : 10) : (cin == 32 ? (cout == 32 ? 150 : 60) : 200);
+    return cin == 16 ? 22 : (cin == 32 ? (cout == 32 ? 42 : 25) : (subm ? 130 : 20));
 }
 constexpr int FEW_SLOTS = 8;                 // few-tiles path: stages in flight, an A slot and a weight block each
 // The slot of a gather warp there (-1: none). Warps 12 and 16 stay out: they share a scheduler, and its queue for shared-memory
@@ -1332,7 +1338,7 @@ int launch_one(const ConvLaunch& c, cudaStream_t stream) {
                        static_cast<const __half*>(c.in), static_cast<__half*>(c.out), c.nbr, c.order, c.tile_mask, c.out_num,
                        static_cast<const uint8_t*>(c.umma_weights), epi, c.relu, c.batch, c.max_voxels,
                        c.kvol, static_cast<__half*>(c.dense), reinterpret_cast<const int4*>(c.out_coors), c.D, c.H, c.W,
-                       c.status, c.tile_counter, few_tiles(CIN, COUT, c.subm != 0), c.maps_ready, c.debug_withhold_weights);
+                       c.status, c.tile_counter, few_tiles(CIN, COUT, c.subm != 0, c.order != nullptr), c.maps_ready, c.debug_withhold_weights);
     return SESSD_OK;
 }
 

@@ -6,7 +6,7 @@ import pytest
 
 import make_golden_inputs as mk
 from conftest import match_rows, rel_err
-from test_gpu_conv import FEW_TILES, _tiles_per_sm
+from test_gpu_conv import FEW_TILES_FRONT_END, _tiles_per_sm
 
 pytestmark = pytest.mark.gpu
 GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
@@ -519,17 +519,18 @@ def test_empty_and_out_of_range_frames_inside_a_batch(gpu):
     bb.close()
 
 
-@pytest.mark.parametrize("dtype,frames", [(0, 1), (0, 8), (1, 1), (1, 40)])
+@pytest.mark.parametrize("dtype,frames", [(0, 1), (0, 8), (1, 1), (1, 150)])
 def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dtype):
     """Layers start while the kernel before them runs. One that takes twice the limit of their bounded waits (about 0.2 s) is put
     before one layer after the other: no wait runs out, and the outputs are those of a call without it. In fp16 one frame goes
-    through the few-tiles path, and the layers of 40 down to 1/4 resolution through groups of tiles. In fp32 eight frames' second layer is
+    through the few-tiles path, and the layers of 150 down to 1/4 resolution through groups of tiles. In fp32 eight frames' second layer is
     the narrow layers' kernel for many rows."""
     import torch
 
     w, sc, sh = gpu.random_weights()
     bb = gpu.Backbone(60000, w, sc, sh, dtype=dtype)
-    pts = torch.stack([torch.from_numpy(gpu.synth.lidar_frame(40 + i, n_points=20000, n_boxes=15)) for i in range(frames)]).cuda()
+    pts = torch.stack([torch.from_numpy(gpu.synth.lidar_frame(40 + i, n_points=20000, n_boxes=15)) for i in range(min(frames, 15))])
+    pts = pts.repeat((frames + 14) // 15 if frames > 15 else 1, 1, 1).cuda()
     sizes = torch.full((frames,), pts.shape[1], dtype=torch.int32, device="cuda")
     dense, ws = bb.run(pts, sizes)
     assert gpu.read_status(ws) == 0
@@ -537,11 +538,10 @@ def test_layers_behind_a_kernel_that_outlasts_the_bounded_waits(gpu, frames, dty
     delay = gpu.lib().sessd_backbone_debug_delay
     wide = [i for i, l in enumerate(bb.layers) if i > 0 and l.cin >= (32 if dtype == 0 else 16)]
     delayed = (wide[0], wide[2], wide[4], wide[-1]) if dtype == 0 else (1, 2, 3, 5, 6, 9, 13)
-    if frames == 40:
-        for i in (1, 2, 3, 5, 6, 9):
+    if frames == 150:
+        for i in (1, 2, 3, 5, 6):
             l = bb.layers[i]
-            line = FEW_TILES[l.cin, l.cout] if l.subm or l.cin < 64 else 20
-            assert _tiles_per_sm(bb.layer_view(ws, frames, pts.shape[1], i)[2].tolist()) > line, i
+            assert _tiles_per_sm(bb.layer_view(ws, frames, pts.shape[1], i)[2].tolist()) > FEW_TILES_FRONT_END[l.cin, l.cout], i
     if (dtype, frames) == (0, 8):
         delayed += (1,)
         assert [n for n, _ in gpu.profile(lambda: bb.run(pts, sizes, ws, dense)) if n.startswith("conv_")][1].startswith("conv_rows")

@@ -205,14 +205,16 @@ def test_narrow_layers_of_many_rows_through_the_other_kernel(gpu, oracle, maxV, 
 
 
 @pytest.mark.parametrize("cin,cout", [(16, 16), (16, 32), (32, 64), (64, 64)])
-@pytest.mark.parametrize("rows", [1, 700, 148 * 128 * 50 + 200])
+@pytest.mark.parametrize("rows", [1, 700, None])
 def test_fp16_rows_at_16_but_not_32_byte_boundaries(gpu, cin, cout, rows):
     """Output rows leave 32 bytes at a time, or 16 where they start at odd multiples of 16 bytes: the same bits, in the few-tiles path
-    and in groups (more than 50 tiles per SM). (All rows are in use.)"""
+    and in groups (rows None). (All rows are in use.)"""
     import torch
 
+    if rows is None:
+        rows = 128 * FEW_TILES[cin, cout] * torch.cuda.get_device_properties(0).multi_processor_count + 200
     rs = np.random.RandomState(cin + rows)
-    shape = (6, 20, 30) if rows < 1000 else (20, 250, 210)
+    shape = (6, 20, 30) if rows < 1000 else (20, 400, 400)
     layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
     coors = torch.from_numpy(_random_coords(rs, rows, shape))[None].cuda()
     num = torch.tensor([rows], dtype=torch.int32, device="cuda")
@@ -341,13 +343,13 @@ def test_fp16_tiles_on_both_sides_of_the_line_between_the_paths(gpu, cin, cout, 
 
 @pytest.mark.parametrize("cin", [32, 64])
 def test_groups_that_wait_for_weights_in_vain_report_it(gpu, cin):
-    """More than 50 tiles per SM, with either kind of issuer, and the test hook that keeps the weights back: the issuers' waits run out
+    """More than the few tiles, with either kind of issuer, and the test hook that keeps the weights back: the issuers' waits run out
     and are reported, and the same call without the hook gives what it gave before."""
     import torch
 
     rs = np.random.RandomState(cin)
-    n = 128 * 50 * torch.cuda.get_device_properties(0).multi_processor_count + 100
-    layer = _layer(gpu, True, cin, cin, (3, 3, 3), (1, 1, 1), (1, 1, 1), (20, 250, 210))
+    n = 128 * FEW_TILES[cin, cin] * torch.cuda.get_device_properties(0).multi_processor_count + 100
+    layer = _layer(gpu, True, cin, cin, (3, 3, 3), (1, 1, 1), (1, 1, 1), (20, 400, 400))
     coors = torch.from_numpy(_random_coords(rs, n, layer.in_shape))[None].cuda()
     num = torch.tensor([n], dtype=torch.int32, device="cuda")
     p = gpu.conv_params(layer, n)
@@ -433,10 +435,11 @@ def test_fp16_work_split_over_frames(gpu, oracle, frames, cin, cout):
     large = sum(i in (0, 2, 4, 5) for i in use)
     most = 128 * (FEW_TILES[cin, cout] * torch.cuda.get_device_properties(0).multi_processor_count // large + 5) + 45
     rows, maxV = [most - 301, 1, most - 301, 128, most - 501, most], most
-    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70) if most < 60000 else (12, 200, 180))
+    layer = _layer(gpu, True, cin, cout, (3, 3, 3), (1, 1, 1), (1, 1, 1), (12, 96, 70) if most < 60000 else (20, 300, 240))
     W = (rs.randn(27, cin, cout) * 0.05).astype(np.float32)
     coors = [_random_coords(rs, n, layer.in_shape) for n in rows]
-    feats = [rs.randn(n, cin).astype(np.float32) for n in rows]
+    rng = np.random.default_rng(frames)
+    feats = [rng.standard_normal((n, cin), dtype=np.float32) for n in rows]
     _check_layer(gpu, oracle, layer, [(coors[0][:20000], feats[0][:20000])], W, dtype=1, maxV=maxV)
     p = gpu.conv_params(layer, maxV)
     w = gpu.ConvWeights(p, W, None, None, False, 1)
