@@ -444,7 +444,7 @@ struct ConvLaunch {
 int launch_conv_simt(const ConvLaunch& c, cudaStream_t stream);
 bool conv_simt_supported(int cin, int cout);
 
-// conv_rows.cu (narrow layers: a warp per 32 rows)
+// conv_rows.cu (narrow layers of calls with many rows: a warp per 64 positions of the map)
 bool conv_rows_takes(const ConvLaunch& c);
 int launch_conv_rows(const ConvLaunch& c, cudaStream_t stream);
 

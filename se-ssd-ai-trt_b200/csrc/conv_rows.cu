@@ -12,8 +12,8 @@
 //   - Multiply-adds go two channels per instruction (each rounded like fmaf).
 //   - The map's entries of the next run are copied in (cp.async) while the present one is worked on, and the mask of the one after
 //     that is read; input rows are requested DEPTH offsets ahead.
-// What bounds it is latency, with sixteen warps per SM (128 registers: with one position per lane, twenty warps and twice the reads of
-// weights 176 us instead of 164). 4 -> 16 in fp16, 32 frames of 120,000 points (2.6 M rows with 4.8 neighbours; 230 MB, 35 us): 289 us
+// What bounds it is latency, with sixteen warps per SM (twelve with 16 input channels; 128 registers: with one position per lane, twenty
+// warps and twice the reads of weights 176 us instead of 164). 4 -> 16 in fp16, 32 frames of 120,000 points (2.6 M rows with 4.8 neighbours; 230 MB, 35 us): 289 us
 // before, now 164; of 20,000 points 74 and 50. fp32, 4 x 120,000 points: 4 -> 16 52 and 37, 16 -> 16 144 and 101.
 #include <string>
 

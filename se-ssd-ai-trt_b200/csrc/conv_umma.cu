@@ -71,12 +71,13 @@ constexpr int KVOL_MAX = 27;
 //             17 56 and 54, 34 93 and 97, 51 136 and 138, 69 179 and 179, 103 265 and 261, 137 353 and 342
 //   32 -> 64  14 (10 x 20,000) 48 and 45.5, 28 80 and 76, 45 115 and 112, 67 161 and 165, 90 210 and 218; frames of 120,000: 25 74 and 72, 58 152
 //             and 148, 132 332 and 318
-//   64 -> 64  11 (8 x 20,000) 66 and 58, 33 (8 x 120,000) 152 and 144, 67 293 and 277, 132 (32 x 120,000) 567 and 532, 197 842 and 791; strided 12 58 and
-//             54, 25 99 and 92, 49 180 and 170, 77 269 and 257
+//   64 -> 64  11 (8 x 20,000) 66 and 58, 33 (8 x 120,000) 152 and 144, 67 293 and 277, 132 (32 x 120,000) 567 and 532, 197 842 and 791;
+//             strided 12 58 and 54, 25 99 and 92, 49 180 and 170, 77 269 and 257
 // Plugin calls:
 //   16 -> 16  11 (12 x 20,000) 33 and 29, 18.5 43.5 and 39.4, 22 45.5 and 45.5, 31 58 and 60, 46 84.5 and 86.5
 //   16 -> 32  12 (6 x 20,000) 31 and 29, 20 43.5 and 41.4, 24 to 43 the same, 64 107 and 109
-//   32 -> 32  10 (5 x 20,000) 41.5 and 37.4, 24 76 and 74, 40 119 and 115, 64 177 and 177; frames of 120,000: 17 60 and 58, 34 103 and 104, 51 146 and 149.5
+//   32 -> 32  10 (5 x 20,000) 41.5 and 37.4, 24 76 and 74, 40 119 and 115, 64 177 and 177; frames of 120,000: 17 60 and 58, 34 103 and 104,
+//             51 146 and 149.5
 //   32 -> 64  8 (6 x 20,000) 39.4 and 37.4, 17 62 and 61, 25 84.5 and 84.5, 41 129.5 and 133.5
 //   64 -> 64  11 (8 x 20,000) 74 and 66, 33 (8 x 120,000) 170 and 166, 66 322 and 318, 83 400 and 396, 132 633 and 621; strided 12 77 and 74, 25 131.5
 //             and 131.5, 37 185 and 189, 49 238 and 246; strided, three offsets, 10 29 and 29, 21 41.5 and 45.5, 42 66 and 78
