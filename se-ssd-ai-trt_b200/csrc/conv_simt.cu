@@ -372,7 +372,11 @@ int dispatch(const ConvLaunch& c, cudaStream_t stream) {
     // here at every size: a submanifold layer (the network has none of these) gains from between 4 and 8 x 20,000 points (4 x 120,000:
     // 523 and 460), the network's strided one from a million rows on (8 x 120,000 18097 and 18062, the whole front end).
     const bool few = (int64_t)c.batch * c.max_voxels <= 1000000;
-    if (c.cin == 4 && c.cout == 16) return few ? launch_narrow<T, 4, 16, 4>(c, stream) : launch_narrow<T, 4, 16, 8>(c, stream);
+    if (c.cin == 4 && c.cout == 16) {
+        // (eight halves leave in 16 bytes; rows that start at other multiples of eight are taken, too, where all of them are in use)
+        const bool wide = !few && reinterpret_cast<uintptr_t>(c.out) % 16 == 0;
+        return wide ? launch_narrow<T, 4, 16, 8>(c, stream) : launch_narrow<T, 4, 16, 4>(c, stream);
+    }
     if (sizeof(T) == 4) {   // in fp16 the tensor-core kernel takes these
         if (c.cin == 16 && c.cout == 16) return launch_narrow<float, 16, 16, 2>(c, stream);
         if (c.cin == 16 && c.cout == 32) return few ? launch_narrow<float, 16, 32, 2>(c, stream) : launch_narrow<float, 16, 32, 4>(c, stream);

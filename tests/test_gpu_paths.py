@@ -879,3 +879,25 @@ def test_narrow_strided_layer_whose_map_names_no_runs(gpu, oracle, dtype):
     names = [n for n, _ in gpu.profile(lambda: gpu.sparse_conv(x, coors, torch.tensor([1], dtype=torch.int32, device="cuda"), p, w))]
     assert any("scatter_rows" in n for n in names) and names[-1].startswith("conv_rows"), names
     w.close()
+
+
+@pytest.mark.parametrize("rows", [300, 1000001])
+def test_fp16_narrow_rows_at_8_but_not_16_byte_boundaries(gpu, rows):
+    """4 -> 16 channels into rows at odd multiples of 8 bytes, all of them in use (rows past the count would be zeroed 16 bytes at a
+    time): the bits of a call with aligned rows."""
+    import torch
+
+    rs = np.random.RandomState(rows)
+    shape = (6, 20, 30) if rows < 1000 else (20, 400, 400)
+    layer = _layer(gpu, True, 4, 16, (3, 3, 3), (1, 1, 1), (1, 1, 1), shape)
+    coors = torch.from_numpy(_random_coords(rs, rows, shape))[None].cuda()
+    num = torch.tensor([rows], dtype=torch.int32, device="cuda")
+    p = gpu.conv_params(layer, rows)
+    w = gpu.ConvWeights(p, (rs.randn(27, 4, 16) * 0.2).astype(np.float32), None, None, True, 1)
+    x = torch.randn((1, rows, 4), device="cuda").half()
+    r = gpu.subm_conv(x, coors, num, p, w, keep_workspace=True)
+    out = torch.empty(rows * 16 + 8, dtype=torch.float16, device="cuda")[4:-4].view(1, rows, 16)
+    assert r["status"] == 0 and out.data_ptr() % 16 == 8
+    gpu.subm_conv_into(x, coors, num, p, w, out, r["workspace"])
+    assert torch.equal(out, r["features"])
+    w.close()
